@@ -6,9 +6,10 @@
  *   - Plain pointers and sizes only.  Every pointer is a DEVICE pointer unless
  *     the parameter comment says "host".  The caller allocates every input and
  *     output and keeps it alive until the work queued on `stream` has run.
- *   - The library never allocates, frees or synchronises; every launch goes to
- *     the `stream` argument (a cudaStream_t passed as void*; NULL = default
- *     stream).
+ *   - The library never synchronises; every launch goes to the `stream` argument (a
+ *     cudaStream_t passed as void*; NULL = default stream).  Calls that are split over
+ *     several launches take scratch memory from a stream-ordered pool of the library
+ *     (at most 256 MiB kept between calls) and give it back behind their work.
  *   - Return value: MEGA_OK or one of the MEGA_ERR_* codes below; nothing is
  *     launched when an argument is rejected.  No exception crosses the ABI and
  *     no kernel traps or asserts.
