@@ -1,6 +1,9 @@
 // Process-wide bookkeeping of the C ABI: status strings, launch counter, last CUDA error.
+#include <array>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
+#include <unordered_map>
 
 #include "common.cuh"
 
@@ -10,6 +13,21 @@ std::atomic<uint64_t> g_launches{0};
 thread_local char g_cuda_err[256] = "";
 std::atomic<int> g_options[8];
 std::atomic<const char*> g_last_kernel{"none"};
+
+void allow_smem(const void* kernel, size_t bytes) {
+  static std::mutex mutex;
+  static std::unordered_map<const void*, std::array<size_t, 16>> set;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return;
+  if (dev < 0 || dev >= 16) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    return;
+  }
+  std::lock_guard<std::mutex> lock(mutex);
+  size_t& have = set[kernel][dev];
+  if (have >= bytes) return;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess) have = bytes;
+}
 
 int check_launch(const char* what) {
   cudaError_t e = cudaGetLastError();

@@ -9,6 +9,7 @@
 // computation on the reversed sequence, delayed by one step when the kernel is shifted.
 // Four lanes share a (batch, channel) row and split its poles; sums over the batch are atomic adds.
 #include "common.cuh"
+#include "scan_ema.cuh"
 #include "stream_bwd.cuh"
 
 namespace mega {
@@ -560,13 +561,15 @@ extern "C" int mega_ema_bwd(const void* dy, const void* x, void* dx, int dtype, 
       cudaMemsetAsync(dgamma_hat, 0, K * N * sizeof(float), s) != cudaSuccess ||
       cudaMemsetAsync(domega, 0, (size_t)D * sizeof(float), s) != cudaSuccess)
     return check_launch("ema_bwd(memset)");
-  if (!bidir) {  // channel-contiguous activations: the streamed TMA kernel
-    EmaBwdStreamArgs sa{};
-    sa.B = B; sa.L = L; sa.D = D; sa.N = N;
-    sa.p = p; sa.q = q; sa.g = gamma_hat; sa.omega = omega; sa.mask = pad_mask; sa.h_in = h_in; sa.dh_out = dh_out;
-    sa.dp = dp; sa.dq = dq; sa.dg = dgamma_hat; sa.domega = domega; sa.dh_in = dh_in;
-    if (ema_bwd_stream_try(dtype, dy, x, dx, gsb, gsl, gsd, xsb, xsl, xsd, dsb, dsl, dsd, sa, s))
-      return check_launch("ema_bwd(stream)");
+  if (!trunc && !h_in && !dh_out && !dh_in && dx != dy && dx != x) {
+    ScanArgs ca{};
+    ca.x = x; ca.y = dx; ca.dy = dy; ca.B = B; ca.D = D; ca.L = L; ca.N = N;
+    ca.xsb = xsb; ca.xsl = xsl; ca.ysb = dsb; ca.ysl = dsl; ca.gsb = gsb; ca.gsl = gsl;
+    ca.p = p; ca.q = q; ca.g = gamma_hat; ca.omega = omega; ca.mask = pad_mask;
+    ca.bidir = bidir ? 1 : 0;
+    ca.shift = (flags & MEGA_EMA_NO_SHIFT) ? 0 : 1;
+    ca.dp = dp; ca.dq = dq; ca.dg = dgamma_hat; ca.domega = domega;
+    if (scan_ema_bwd_try(dtype, ca, xsd, dsd, gsd, s)) return check_launch("ema_bwd(scan)");
   }
   EmaBwdArgs a{};
   a.dy = dy; a.x = x; a.dx = dx; a.B = B; a.D = D; a.L = L; a.N = N;

@@ -6,6 +6,7 @@
 #include "common.cuh"
 #include "stream_bwd.cuh"
 #include "stream_cl.cuh"
+#include "scan_ema.cuh"
 
 namespace mega {
 
@@ -618,7 +619,6 @@ extern "C" int mega_cema_fwd(const void* x, void* y, int dtype, int B, int D, in
   if (!bidir && trunc) return MEGA_ERR_UNSUPPORTED;
   if (x == y && (bidir || trunc || xsb != ysb || xsd != ysd || xsl != ysl)) return MEGA_ERR_STRIDE;
   if (!bidir && !trunc && x != y && N <= 16) {
-    // channel-contiguous activations: the streamed TMA kernel (one thread per channel, poles in registers)
     StreamArgs sa{};
     sa.B = B; sa.L = L; sa.D = D; sa.N = N;
     sa.p = p; sa.q = q; sa.g = gamma_hat; sa.omega = omega; sa.h_in = h_in; sa.h_out = h_out; sa.mask = pad_mask;
@@ -626,8 +626,17 @@ extern "C" int mega_cema_fwd(const void* x, void* y, int dtype, int B, int D, in
     sa.cplx = 1;
     if (mma_cl_try(dtype, x, y, nullptr, xsb, xsl, xsd, ysb, ysl, ysd, false, sa, (cudaStream_t)stream))
       return check_launch("cema_fwd(mma)");
-    if (stream_cl_try(dtype, x, y, nullptr, xsb, xsl, xsd, ysb, ysl, ysd, false, true, sa, (cudaStream_t)stream))
-      return check_launch("cema_fwd(stream)");
+  }
+  if (!trunc && x != y) {
+    ScanArgs ca{};
+    ca.x = x; ca.y = y; ca.B = B; ca.D = D; ca.L = L; ca.N = N;
+    ca.xsb = xsb; ca.xsl = xsl; ca.ysb = ysb; ca.ysl = ysl;
+    ca.p = p; ca.q = q; ca.g = gamma_hat; ca.omega = omega; ca.mask = pad_mask; ca.h_in = h_in; ca.h_out = h_out;
+    ca.cplx = 1;
+    ca.bidir = bidir ? 1 : 0;
+    ca.shift = (flags & MEGA_EMA_NO_SHIFT) ? 0 : 1;
+    ca.silu = (flags & MEGA_EMA_SILU) ? 1 : 0;
+    if (scan_ema_fwd_try(dtype, ca, xsd, ysd, (cudaStream_t)stream)) return check_launch("cema_fwd(scan)");
   }
   CemaArgs a{};
   a.x = x; a.y = y; a.B = B; a.D = D; a.L = L; a.N = N;
@@ -759,13 +768,16 @@ extern "C" int mega_cema_bwd(const void* dy, const void* x, void* dx, int dtype,
       cudaMemsetAsync(dgamma_hat, 0, K * N * 2 * sizeof(float), s) != cudaSuccess ||
       cudaMemsetAsync(domega, 0, (size_t)D * sizeof(float), s) != cudaSuccess)
     return check_launch("cema_bwd(memset)");
-  if (!bidir) {  // channel-contiguous activations: the streamed TMA kernel
-    EmaBwdStreamArgs sa{};
-    sa.B = B; sa.L = L; sa.D = D; sa.N = N;
-    sa.p = p; sa.q = q; sa.g = gamma_hat; sa.omega = omega; sa.mask = pad_mask;
-    sa.dp = dp; sa.dq = dq; sa.dg = dgamma_hat; sa.domega = domega;
-    if (cema_bwd_stream_try(dtype, dy, x, dx, gsb, gsl, gsd, xsb, xsl, xsd, dsb, dsl, dsd, sa, s))
-      return check_launch("cema_bwd(stream)");
+  if (!trunc && dx != dy && dx != x) {
+    ScanArgs ca{};
+    ca.x = x; ca.y = dx; ca.dy = dy; ca.B = B; ca.D = D; ca.L = L; ca.N = N;
+    ca.xsb = xsb; ca.xsl = xsl; ca.ysb = dsb; ca.ysl = dsl; ca.gsb = gsb; ca.gsl = gsl;
+    ca.p = p; ca.q = q; ca.g = gamma_hat; ca.omega = omega; ca.mask = pad_mask;
+    ca.cplx = 1;
+    ca.bidir = bidir ? 1 : 0;
+    ca.shift = (flags & MEGA_EMA_NO_SHIFT) ? 0 : 1;
+    ca.dp = dp; ca.dq = dq; ca.dg = dgamma_hat; ca.domega = domega;
+    if (scan_ema_bwd_try(dtype, ca, xsd, dsd, gsd, s)) return check_launch("cema_bwd(scan)");
   }
   CemaBwdArgs a{};
   a.dy = dy; a.x = x; a.dx = dx; a.B = B; a.D = D; a.L = L; a.N = N;

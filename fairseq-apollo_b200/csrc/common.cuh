@@ -30,14 +30,14 @@ bool step_lanes_try(int dtype, const void* x, void* y, void* xn_out, int B, int 
                     const float* q, const float* g, const float* omega, const float* h_in, float* h_out, int silu,
                     void* stream, long long* count_next = nullptr);
 
+// Above the default 48 KB the dynamic shared-memory size is an opt-in attribute of the kernel ON THE CURRENT
+// DEVICE; it is raised once per kernel and device (abi.cu), as setting it costs a microsecond or two of every launch.
+void allow_smem(const void* kernel, size_t bytes);
+
 template <typename... KArgs, typename... Args>
 static inline void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, void* stream,
                           Args... args) {
-  // Above the default 48 KB the dynamic shared-memory size is an opt-in attribute of the kernel ON
-  // THE CURRENT DEVICE; setting it at every such launch (microseconds, these launches run for
-  // hundreds) keeps a process that drives several GPUs correct.
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (smem > 48 * 1024) allow_smem(reinterpret_cast<const void*>(kernel), smem);
   kernel<<<grid, block, smem, (cudaStream_t)stream>>>(static_cast<KArgs>(args)...);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   g_last_kernel.store("other", std::memory_order_relaxed);

@@ -9,6 +9,7 @@
 #include "common.cuh"
 #include "stream_cl.cuh"
 #include "rowres.cuh"
+#include "scan_ema.cuh"
 
 namespace mega {
 
@@ -431,7 +432,7 @@ extern "C" int mega_ema_fwd(const void* x, void* y, int dtype, int B, int D, int
     sa.p = p; sa.q = q; sa.g = gamma_hat; sa.omega = omega; sa.h_in = h_in; sa.h_out = h_out; sa.mask = pad_mask;
     sa.silu = (flags & MEGA_EMA_SILU) ? 1 : 0;
     // (a state is exported and L is not a multiple of the tensor-core step of 32: head on the
-    // tensor-core kernel, ragged tail on the streamed kernel, continuing from the head's state in place)
+    // tensor-core kernel, ragged tail on the generic kernel, continuing from the head's state in place)
     const int Lh = L - L % 32;
     if (h_out && Lh > 0 && Lh < L && !pad_mask) {
       StreamArgs head = sa;
@@ -440,19 +441,22 @@ extern "C" int mega_ema_fwd(const void* x, void* y, int dtype, int B, int D, int
         const size_t es = (size_t)elem_size(dtype);
         const void* xt = (const char*)x + (size_t)Lh * xsl * es;
         void* yt = (char*)y + (size_t)Lh * ysl * es;
-        StreamArgs tail = sa;
-        tail.L = L - Lh;
-        tail.h_in = h_out;
-        if (stream_cl_try(dtype, xt, yt, nullptr, xsb, xsl, xsd, ysb, ysl, ysd, false, true, tail, (cudaStream_t)stream))
-          return check_launch("ema_fwd(mma head + stream tail)");
         a.x = xt; a.y = yt; a.L = L - Lh; a.h_in = h_out;
         return ema_fwd_simt(a, flags, truncation, dtype, (cudaStream_t)stream);
       }
     }
     if (mma_cl_try(dtype, x, y, nullptr, xsb, xsl, xsd, ysb, ysl, ysd, false, sa, (cudaStream_t)stream))
       return check_launch("ema_fwd(mma)");
-    if (stream_cl_try(dtype, x, y, nullptr, xsb, xsl, xsd, ysb, ysl, ysd, false, true, sa, (cudaStream_t)stream))
-      return check_launch("ema_fwd(stream)");
+  }
+  if (!(truncation > 0 && truncation < L) && x != y) {
+    ScanArgs ca{};
+    ca.x = x; ca.y = y; ca.B = B; ca.D = D; ca.L = L; ca.N = N;
+    ca.xsb = xsb; ca.xsl = xsl; ca.ysb = ysb; ca.ysl = ysl;
+    ca.p = p; ca.q = q; ca.g = gamma_hat; ca.omega = omega; ca.mask = pad_mask; ca.h_in = h_in; ca.h_out = h_out;
+    ca.bidir = bidir ? 1 : 0;
+    ca.shift = (flags & MEGA_EMA_NO_SHIFT) ? 0 : 1;
+    ca.silu = (flags & MEGA_EMA_SILU) ? 1 : 0;
+    if (scan_ema_fwd_try(dtype, ca, xsd, ysd, (cudaStream_t)stream)) return check_launch("ema_fwd(scan)");
   }
   return ema_fwd_simt(a, flags, truncation, dtype, (cudaStream_t)stream);
 }

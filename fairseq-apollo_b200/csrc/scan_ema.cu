@@ -1,0 +1,780 @@
+// The EMA layer and its backward, parallel over time: real or complex poles, causal or bidirectional, any
+// activation type, any strides along batch and time, channels contiguous.
+//
+// A pole state is a linear recurrence, so the sequence is cut into segments that run at the same time.
+// (1) every segment folds its inputs into a state of its own, from zero; (2) a small launch carries the
+// states over the segments (H <- q^T H + h); (3) every segment runs again from the state it really starts
+// with and emits its outputs.  A warp owns 32 adjacent channels of one segment, a lane one channel with
+// its 16 poles in registers (ndim < 16: the rest are inert), so memory is read in whole rows and nothing is
+// exchanged between lanes.  Work per element and direction: 16 + 32 FMA real, twice to three times that
+// complex (the walk of one segment per sequence needs no first pass: 32).
+// Bound: the FMA pipe, when segments x channels fill the SMs; a sequence walked as one chain is bound by its
+// own latency instead (B = 8, L = 1024, D = 512 fp32: 103 us as 128 chains of 1024 steps).
+//
+// Backward.  With h the states for unit input gain, s = dh/dq and lambda the adjoint scaled by 1 / (p g):
+//   h_t = q h_{t-1} + x~_t,  s_t = q s_{t-1} + h_{t-1},  lambda_t = q lambda_{t+1} + dy_t,
+//   dx~_t = sum_n p g lambda_t,  dg = p sum dy h,  dp = g sum dy h,  dq = p g sum dy s,
+// with real parts taken for complex poles; the anti-causal half runs the same in reversed time.  The same
+// three steps: local (h, s, lambda) per segment, carried over the segments, then the sums and dx.
+#include <cmath>
+
+#include "common.cuh"
+#include "scan_ema.cuh"
+#include "scratch.cuh"
+#include "tma.cuh"
+#include "walk.cuh"
+
+namespace mega {
+
+namespace {
+
+constexpr int kP2 = 8;      // pole pairs of a lane (16 poles)
+
+struct SegArgs {
+  ScanArgs a;
+  int T, S;          // steps per segment, segments
+  int wide;          // one segment: the warps of a block own adjacent channel groups instead of segments
+  int parts;         // values per (batch, direction, segment, pole, channel) in the carry array
+  float* carry;      // [B][dirs][S][parts][16][D]
+};
+
+// One pole-state vector: real parts, and imaginary parts for complex poles.
+template <bool kC>
+struct State {
+  f32x2 r[kP2];
+  f32x2 i[kC ? kP2 : 1];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int j = 0; j < kP2; ++j) {
+      r[j] = pack2(0.f, 0.f);
+      if (kC) i[j] = pack2(0.f, 0.f);
+    }
+  }
+};
+
+// Poles of a lane's channel.  q; ni = -Im q; c (and nc = -Im c): output weight.
+template <bool kC>
+struct Poles {
+  f32x2 q[kP2];
+  f32x2 qi[kC ? kP2 : 1], ni[kC ? kP2 : 1];
+};
+
+template <bool kC>
+__device__ __forceinline__ void load_poles(Poles<kC>& P, const ScanArgs& a, int row) {
+#pragma unroll
+  for (int j = 0; j < kP2; ++j) {
+    float qr[2], qi[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int n = 2 * j + k;
+      const size_t c = (size_t)row * a.N + n;
+      qr[k] = qi[k] = 0.f;
+      if (n < a.N) {
+        qr[k] = kC ? __ldg(a.q + 2 * c) : __ldg(a.q + c);
+        if (kC) qi[k] = __ldg(a.q + 2 * c + 1);
+      }
+    }
+    P.q[j] = pack2(qr[0], qr[1]);
+    if (kC) {
+      P.qi[j] = pack2(qi[0], qi[1]);
+      P.ni[j] = pack2(-qi[0], -qi[1]);
+    }
+  }
+}
+
+// Output weights p gamma (kGain) or gamma alone; the imaginary part negated (y = Re(c h) = cr hr - ci hi).
+template <bool kC>
+__device__ __forceinline__ void load_weights(State<kC>& C, const ScanArgs& a, int row, bool gain) {
+#pragma unroll
+  for (int j = 0; j < kP2; ++j) {
+    float cr[2], ci[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int n = 2 * j + k;
+      const size_t c = (size_t)row * a.N + n;
+      cr[k] = ci[k] = 0.f;
+      if (n < a.N) {
+        const float p = gain ? __ldg(a.p + c) : 1.f;
+        cr[k] = p * (kC ? __ldg(a.g + 2 * c) : __ldg(a.g + c));
+        if (kC) ci[k] = -p * __ldg(a.g + 2 * c + 1);
+      }
+    }
+    C.r[j] = pack2(cr[0], cr[1]);
+    if (kC) C.i[j] = pack2(ci[0], ci[1]);
+  }
+}
+
+// h <- q h + x
+template <bool kC>
+__device__ __forceinline__ void advance(State<kC>& h, const Poles<kC>& P, f32x2 x2) {
+#pragma unroll
+  for (int j = 0; j < kP2; ++j) {
+    if (kC) {
+      const f32x2 nr = fma2(P.q[j], h.r[j], fma2(P.ni[j], h.i[j], x2));
+      h.i[j] = fma2(P.qi[j], h.r[j], mul2(P.q[j], h.i[j]));
+      h.r[j] = nr;
+    } else {
+      h.r[j] = fma2(P.q[j], h.r[j], x2);
+    }
+  }
+}
+// h <- q h + p x
+template <bool kC>
+__device__ __forceinline__ void advance_gain(State<kC>& h, const Poles<kC>& P, const f32x2 (&p)[kP2], f32x2 x2) {
+#pragma unroll
+  for (int j = 0; j < kP2; ++j) {
+    const f32x2 in = mul2(p[j], x2);
+    if (kC) {
+      const f32x2 nr = fma2(P.q[j], h.r[j], fma2(P.ni[j], h.i[j], in));
+      h.i[j] = fma2(P.qi[j], h.r[j], mul2(P.q[j], h.i[j]));
+      h.r[j] = nr;
+    } else {
+      h.r[j] = fma2(P.q[j], h.r[j], in);
+    }
+  }
+}
+// s <- q s + h (h before its own step)
+template <bool kC>
+__device__ __forceinline__ void advance_sens(State<kC>& s, const State<kC>& h, const Poles<kC>& P) {
+#pragma unroll
+  for (int j = 0; j < kP2; ++j) {
+    if (kC) {
+      const f32x2 nr = fma2(P.q[j], s.r[j], fma2(P.ni[j], s.i[j], h.r[j]));
+      s.i[j] = fma2(P.qi[j], s.r[j], fma2(P.q[j], s.i[j], h.i[j]));
+      s.r[j] = nr;
+    } else {
+      s.r[j] = fma2(P.q[j], s.r[j], h.r[j]);
+    }
+  }
+}
+// Re(sum c h)
+template <bool kC>
+__device__ __forceinline__ float dot(const State<kC>& c, const State<kC>& h) {
+  f32x2 a0 = pack2(0.f, 0.f), a1 = pack2(0.f, 0.f);
+#pragma unroll
+  for (int j = 0; j < kP2; j += 2) {
+    a0 = fma2(c.r[j], h.r[j], a0);
+    a1 = fma2(c.r[j + 1], h.r[j + 1], a1);
+    if (kC) {
+      a0 = fma2(c.i[j], h.i[j], a0);
+      a1 = fma2(c.i[j + 1], h.i[j + 1], a1);
+    }
+  }
+  float lo, hi;
+  unpack2(add2(a0, a1), lo, hi);
+  return lo + hi;
+}
+// acc += dy h
+template <bool kC>
+__device__ __forceinline__ void accumulate(State<kC>& acc, const State<kC>& h, f32x2 g2) {
+#pragma unroll
+  for (int j = 0; j < kP2; ++j) {
+    acc.r[j] = fma2(g2, h.r[j], acc.r[j]);
+    if (kC) acc.i[j] = fma2(g2, h.i[j], acc.i[j]);
+  }
+}
+
+// Entry of a state in the carry array: lanes are adjacent channels.
+template <bool kC>
+__device__ __forceinline__ void store_state(const State<kC>& h, float* dst, int D, bool ok) {
+  if (!ok) return;
+#pragma unroll
+  for (int j = 0; j < kP2; ++j) {
+    float lo, hi;
+    unpack2(h.r[j], lo, hi);
+    dst[(size_t)(2 * j) * D] = lo;
+    dst[(size_t)(2 * j + 1) * D] = hi;
+    if (kC) {
+      unpack2(h.i[j], lo, hi);
+      dst[(size_t)(16 + 2 * j) * D] = lo;
+      dst[(size_t)(16 + 2 * j + 1) * D] = hi;
+    }
+  }
+}
+template <bool kC>
+__device__ __forceinline__ void load_state(State<kC>& h, const float* src, int D) {
+#pragma unroll
+  for (int j = 0; j < kP2; ++j) {
+    h.r[j] = pack2(__ldg(src + (size_t)(2 * j) * D), __ldg(src + (size_t)(2 * j + 1) * D));
+    if (kC) h.i[j] = pack2(__ldg(src + (size_t)(16 + 2 * j) * D), __ldg(src + (size_t)(16 + 2 * j + 1) * D));
+  }
+}
+
+__device__ __forceinline__ f32x2 splat(float v) { return pack2(v, v); }
+
+// (batch, direction, segment) entry of the carry array
+__device__ __forceinline__ float* carry_at(const SegArgs& s, int b, int dir, int seg, int part, int d) {
+  const int dirs = s.a.bidir ? 2 : 1;
+  return s.carry + ((((size_t)b * dirs + dir) * s.S + seg) * s.parts + part) * 16 * s.a.D + d;
+}
+
+struct Lane {
+  int lane, warp, d, dc, b, seg, t0, t1, d0, left;   // d0: first channel of the warp, left: channels from there
+  bool ok;
+};
+__device__ __forceinline__ Lane lane_of(const SegArgs& s) {
+  Lane l;
+  l.lane = threadIdx.x & 31;
+  l.warp = threadIdx.x >> 5;
+  l.d = (s.wide ? blockIdx.x * kWarps + l.warp : blockIdx.x) * 32 + l.lane;
+  l.d0 = l.d - l.lane < s.a.D ? l.d - l.lane : 0;
+  l.left = s.a.D - (l.d - l.lane);
+  l.ok = l.d < s.a.D;
+  l.dc = l.ok ? l.d : s.a.D - 1;
+  l.seg = s.wide ? 0 : blockIdx.y * kWarps + l.warp;
+  l.b = blockIdx.z;
+  l.t0 = min(s.a.L, l.seg * s.T);
+  l.t1 = min(s.a.L, l.t0 + s.T);
+  return l;
+}
+
+// ---- (1) local states ---------------------------------------------------------------------------
+// forward: h of each direction.  backward: (h, s) of each direction and the adjoint, which runs the other way.
+template <typename T, bool kC, bool kMask, bool kBwd>
+__global__ void __launch_bounds__(kWarps * 32) scan_local_kernel(SegArgs s) {
+  const ScanArgs& a = s.a;
+  const int dirs = a.bidir ? 2 : 1;
+  SegArgs ss = s;
+  Lane l = lane_of(ss);
+  const int dir = l.b % dirs;
+  l.b /= dirs;
+  if (l.seg >= s.S) return;
+  const T* x = reinterpret_cast<const T*>(a.x) + l.b * a.xsb + l.d0;
+  const unsigned char* m = kMask ? a.mask + (size_t)l.b * a.L : nullptr;
+  Poles<kC> P;
+  load_poles<kC>(P, a, l.dc + dir * a.D);
+  extern __shared__ __align__(16) unsigned char rings[];
+  unsigned char* ring = rings + (size_t)l.warp * kRing * kTileBytes;
+  State<kC> h;
+  h.zero();
+  constexpr int kOne = kC ? 2 : 1;   // parts of a state
+  if (kBwd) {
+    State<kC> sn;
+    sn.zero();
+    auto step = [&](int, float xv, float, bool pad) {
+      advance_sens<kC>(sn, h, P);
+      advance<kC>(h, P, splat(kMask && pad ? 0.f : xv));
+    };
+    if (dir == 0) walk<T, 1, false, kMask>(x, a.xsl, x, 0, m, l.t0, l.t1, l.left, ring, step);
+    else walk<T, -1, false, kMask>(x, a.xsl, x, 0, m, l.t0, l.t1, l.left, ring, step);
+    store_state<kC>(h, carry_at(s, l.b, dir, l.seg, 0, l.dc), a.D, l.ok);
+    store_state<kC>(sn, carry_at(s, l.b, dir, l.seg, kOne, l.dc), a.D, l.ok);
+    h.zero();
+    const T* g = reinterpret_cast<const T*>(a.dy) + l.b * a.gsb + l.d0;
+    auto adj = [&](int, float gv, float, bool) { advance<kC>(h, P, splat(gv)); };
+    if (dir == 0) walk<T, -1, false, false>(g, a.gsl, g, 0, m, l.t0, l.t1, l.left, ring, adj);
+    else walk<T, 1, false, false>(g, a.gsl, g, 0, m, l.t0, l.t1, l.left, ring, adj);
+    store_state<kC>(h, carry_at(s, l.b, dir, l.seg, 2 * kOne, l.dc), a.D, l.ok);
+  } else {
+    auto step = [&](int, float xv, float, bool pad) { advance<kC>(h, P, splat(kMask && pad ? 0.f : xv)); };
+    if (dir == 0) walk<T, 1, false, kMask>(x, a.xsl, x, 0, m, l.t0, l.t1, l.left, ring, step);
+    else walk<T, -1, false, kMask>(x, a.xsl, x, 0, m, l.t0, l.t1, l.left, ring, step);
+    store_state<kC>(h, carry_at(s, l.b, dir, l.seg, 0, l.dc), a.D, l.ok);
+  }
+}
+
+// ---- (2) carry over the segments -----------------------------------------------------------------
+__device__ __forceinline__ float2 cmul(float2 a, float2 b) { return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
+__device__ __forceinline__ float2 ipow(float2 q, int n) {
+  float2 r = make_float2(1.f, 0.f);
+  for (; n > 0; n >>= 1) {
+    if (n & 1) r = cmul(r, q);
+    q = cmul(q, q);
+  }
+  return r;
+}
+
+// One thread per (channel, pole, direction, batch): replaces each segment's local values by the values the
+// segment starts from.  kGain: true states (input gain applied), from h_in, the last one to h_out.
+template <bool kC, bool kBwd>
+__global__ void __launch_bounds__(128) scan_carry_kernel(SegArgs s, int gain) {
+  const ScanArgs& a = s.a;
+  const int dirs = a.bidir ? 2 : 1;
+  const int d = blockIdx.x * 128 + threadIdx.x;
+  const int n = blockIdx.y;
+  const int dir = blockIdx.z % dirs, b = blockIdx.z / dirs;
+  if (d >= a.D) return;
+  const bool live = n < a.N;
+  const size_t c = (size_t)(d + dir * a.D) * a.N + n;
+  float2 q = make_float2(0.f, 0.f);
+  if (live) q = kC ? make_float2(__ldg(a.q + 2 * c), __ldg(a.q + 2 * c + 1)) : make_float2(__ldg(a.q + c), 0.f);
+  const int last = a.L - (s.S - 1) * s.T;   // steps of the last segment
+  float2 qT, qLast, qT1 = make_float2(0.f, 0.f), qLast1 = make_float2(0.f, 0.f);
+  if (kC) {
+    qT = ipow(q, s.T);
+    qLast = ipow(q, last);
+    if (kBwd) {
+      qT1 = ipow(q, s.T - 1);
+      qLast1 = ipow(q, last - 1);
+    }
+  } else {
+    qT = make_float2(powf(q.x, (float)s.T), 0.f);
+    qLast = make_float2(powf(q.x, (float)last), 0.f);
+    if (kBwd) {
+      qT1 = make_float2(powf(q.x, (float)(s.T - 1)), 0.f);
+      qLast1 = make_float2(powf(q.x, (float)(last - 1)), 0.f);
+    }
+  }
+  constexpr int kOne = kC ? 2 : 1;
+  const size_t step = (size_t)s.parts * 16 * a.D;
+  float* base = carry_at(s, b, dir, 0, 0, d) + (size_t)n * a.D;
+  const size_t im = (size_t)16 * a.D;   // imaginary part of the same value
+  const size_t part = (size_t)kOne * 16 * a.D;
+  float2 H = make_float2(0.f, 0.f), Sn = make_float2(0.f, 0.f);
+  const float pg = (gain && live) ? __ldg(a.p + c) : 1.f;
+  const size_t sidx = ((size_t)b * a.D + d) * a.N + n;
+  if (gain && a.h_in && live) H = kC ? make_float2(a.h_in[2 * sidx], a.h_in[2 * sidx + 1]) : make_float2(a.h_in[sidx], 0.f);
+  // (the loads of kB segments go out together: a load that follows the store of the segment before would wait
+  // for the whole round trip of every segment)
+  constexpr int kB = 8;
+  for (int k0 = 0; k0 < s.S; k0 += kB) {
+    float2 loc[kB], ls[kBwd ? kB : 1];
+#pragma unroll
+    for (int u = 0; u < kB; ++u) {
+      const int k = min(k0 + u, s.S - 1);
+      const float* v = base + (size_t)(dir == 0 ? k : s.S - 1 - k) * step;
+      loc[u] = make_float2(__ldcg(v), kC ? __ldcg(v + im) : 0.f);
+      if (kBwd) ls[kBwd ? u : 0] = make_float2(__ldcg(v + part), kC ? __ldcg(v + part + im) : 0.f);
+    }
+#pragma unroll
+    for (int u = 0; u < kB; ++u) {
+      if (k0 + u < s.S) {
+        const int seg = dir == 0 ? k0 + u : s.S - 1 - (k0 + u);
+        float* v = base + (size_t)seg * step;
+        const bool lst = seg == s.S - 1;
+        const float2 w = lst ? qLast : qT;
+        v[0] = H.x;
+        if (kC) v[im] = H.y;
+        if (kBwd) {
+          float* uu = v + part;
+          const float2 w1 = lst ? qLast1 : qT1;
+          const float len = lst ? (float)last : (float)s.T;
+          const float2 l2 = ls[kBwd ? u : 0];
+          uu[0] = Sn.x;
+          if (kC) {
+            uu[im] = Sn.y;
+            const float2 a1 = cmul(w, Sn), a2 = cmul(w1, H);
+            Sn = make_float2(a1.x + fmaf(len, a2.x, l2.x), a1.y + fmaf(len, a2.y, l2.y));
+          } else {
+            Sn.x = fmaf(w.x, Sn.x, fmaf(len * w1.x, H.x, l2.x));
+          }
+        }
+        if (kC) {
+          const float2 a1 = cmul(w, H);
+          H = make_float2(fmaf(pg, loc[u].x, a1.x), fmaf(pg, loc[u].y, a1.y));
+        } else {
+          H.x = fmaf(w.x, H.x, pg * loc[u].x);
+        }
+      }
+    }
+  }
+  if (gain && a.h_out && live) {
+    if (kC) {
+      a.h_out[2 * sidx] = H.x;
+      a.h_out[2 * sidx + 1] = H.y;
+    } else {
+      a.h_out[sidx] = H.x;
+    }
+  }
+  if (kBwd) {   // the adjoint, against the direction
+    float2 A = make_float2(0.f, 0.f);
+    for (int k0 = s.S - 1; k0 >= 0; k0 -= kB) {
+      float2 loc[kB];
+#pragma unroll
+      for (int u = 0; u < kB; ++u) {
+        const int k = max(k0 - u, 0);
+        const float* v = base + (size_t)(dir == 0 ? k : s.S - 1 - k) * step + 2 * part;
+        loc[u] = make_float2(__ldcg(v), kC ? __ldcg(v + im) : 0.f);
+      }
+#pragma unroll
+      for (int u = 0; u < kB; ++u) {
+        if (k0 - u >= 0) {
+          const int seg = dir == 0 ? k0 - u : s.S - 1 - (k0 - u);
+          float* v = base + (size_t)seg * step + 2 * part;
+          const float2 w = seg == s.S - 1 ? qLast : qT;
+          v[0] = A.x;
+          if (kC) {
+            v[im] = A.y;
+            const float2 a1 = cmul(w, A);
+            A = make_float2(a1.x + loc[u].x, a1.y + loc[u].y);
+          } else {
+            A.x = fmaf(w.x, A.x, loc[u].x);
+          }
+        }
+      }
+    }
+  }
+}
+
+// ---- (3) outputs -----------------------------------------------------------------------------------
+template <typename T, bool kC, bool kMask, bool kState>
+__global__ void __launch_bounds__(kWarps * 32, kC ? 3 : 4) scan_emit_kernel(SegArgs s) {
+  const ScanArgs& a = s.a;
+  const Lane l = lane_of(s);
+  if (l.seg >= s.S) return;
+  const T* x = reinterpret_cast<const T*>(a.x) + l.b * a.xsb + l.d0;
+  T* y = reinterpret_cast<T*>(a.y) + l.b * a.ysb + l.dc;
+  const unsigned char* m = kMask ? a.mask + (size_t)l.b * a.L : nullptr;
+  const float om = __ldg(a.omega + l.dc);
+  extern __shared__ __align__(16) unsigned char rings[];
+  unsigned char* ring = rings + (size_t)l.warp * kRing * kTileBytes;
+  Poles<kC> P;
+  State<kC> c, h;
+  f32x2 p[kState ? kP2 : 1];
+  load_poles<kC>(P, a, l.dc);
+  load_weights<kC>(c, a, l.dc, !kState);
+  if (kState) {
+#pragma unroll
+    for (int j = 0; j < kP2; ++j) {
+      const size_t n = (size_t)l.dc * a.N + 2 * j;
+      p[kState ? j : 0] = pack2(2 * j < a.N ? __ldg(a.p + n) : 0.f, 2 * j + 1 < a.N ? __ldg(a.p + n + 1) : 0.f);
+    }
+  }
+  h.zero();
+  if (s.carry) {
+    load_state<kC>(h, carry_at(s, l.b, 0, l.seg, 0, l.dc), a.D);
+  } else if (kState && a.h_in) {
+#pragma unroll
+    for (int j = 0; j < kP2; ++j) {
+      const size_t n = ((size_t)l.b * a.D + l.dc) * a.N + 2 * j;
+      float r[2] = {0.f, 0.f}, i[2] = {0.f, 0.f};
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        if (2 * j + k < a.N) {
+          r[k] = kC ? __ldg(a.h_in + 2 * (n + k)) : __ldg(a.h_in + n + k);
+          if (kC) i[k] = __ldg(a.h_in + 2 * (n + k) + 1);
+        }
+      h.r[j] = pack2(r[0], r[1]);
+      if (kC) h.i[j] = pack2(i[0], i[1]);
+    }
+  }
+  if (a.bidir) {   // the causal half leaves its share of the outputs in shared memory
+    float* part = reinterpret_cast<float*>(rings + kWarps * kRing * kTileBytes);
+    float* mine = part + (size_t)l.warp * s.T * 32 + l.lane;
+    walk<T, 1, false, kMask>(x, a.xsl, x, 0, m, l.t0, l.t1, l.left, ring, [&](int k, float xv, float, bool pad) {
+      advance<kC>(h, P, splat(kMask && pad ? 0.f : xv));
+      mine[k * 32] = fmaf(om, xv, dot<kC>(c, h));
+    });
+    load_poles<kC>(P, a, l.dc + a.D);
+    load_weights<kC>(c, a, l.dc + a.D, true);
+    load_state<kC>(h, carry_at(s, l.b, 1, l.seg, 0, l.dc), a.D);
+    const bool shift = a.shift != 0;
+    const float* last = mine + (l.t1 - l.t0 - 1) * 32;
+    T* py = y + (long long)(l.t1 - 1) * a.ysl;
+    walk<T, -1, false, kMask>(x, a.xsl, x, 0, m, l.t0, l.t1, l.left, ring, [&](int k, float xv, float, bool pad) {
+      float v = last[-k * 32];
+      if (shift) v += dot<kC>(c, h);
+      advance<kC>(h, P, splat(kMask && pad ? 0.f : xv));
+      if (!shift) v += dot<kC>(c, h);
+      if (a.silu) v = siluf_(v);
+      if (l.ok) Elem<T>::st(py, v);
+      py -= a.ysl;
+    });
+    return;
+  }
+  T* py = y + (long long)l.t0 * a.ysl;
+  walk<T, 1, false, kMask>(x, a.xsl, x, 0, m, l.t0, l.t1, l.left, ring, [&](int k, float xv, float, bool pad) {
+    const f32x2 x2 = splat(kMask && pad ? 0.f : xv);
+    if constexpr (kState) advance_gain<kC>(h, P, p, x2);
+    else advance<kC>(h, P, x2);
+    float v = fmaf(om, xv, dot<kC>(c, h));
+    if (a.silu) v = siluf_(v);
+    if (l.ok) Elem<T>::st(py, v);
+    py += a.ysl;
+  });
+  if (kState && !s.carry && a.h_out && l.ok) {
+#pragma unroll
+    for (int j = 0; j < kP2; ++j) {
+      const size_t n = ((size_t)l.b * a.D + l.d) * a.N + 2 * j;
+      float r[2], i[2] = {0.f, 0.f};
+      unpack2(h.r[j], r[0], r[1]);
+      if (kC) unpack2(h.i[j], i[0], i[1]);
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        if (2 * j + k < a.N) {
+          if (kC) {
+            a.h_out[2 * (n + k)] = r[k];
+            a.h_out[2 * (n + k) + 1] = i[k];
+          } else {
+            a.h_out[n + k] = r[k];
+          }
+        }
+    }
+  }
+}
+
+// Sums of a block's segments, then one atomic add per parameter.  red: [kWarps][32][32] floats.
+template <bool kC>
+__device__ __forceinline__ void reduce_grads(const State<kC>& ah, const State<kC>& as, const ScanArgs& a, int row, bool ok,
+                                             bool active, float* red) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kV = kC ? 64 : 32;   // sums per channel: dy h, dy s
+  for (int r0 = 0; r0 < kV; r0 += 32) {
+    // kV values of every lane go through shared memory, 32 at a time
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kP2; ++j) {
+      float v0, v1;
+      if (r0 == 0) {
+        unpack2(ah.r[j], v0, v1);
+        red[(warp * 32 + 2 * j) * 32 + lane] = active ? v0 : 0.f;
+        red[(warp * 32 + 2 * j + 1) * 32 + lane] = active ? v1 : 0.f;
+        unpack2(as.r[j], v0, v1);
+        red[(warp * 32 + 16 + 2 * j) * 32 + lane] = active ? v0 : 0.f;
+        red[(warp * 32 + 16 + 2 * j + 1) * 32 + lane] = active ? v1 : 0.f;
+      } else if (kC) {
+        unpack2(ah.i[kC ? j : 0], v0, v1);
+        red[(warp * 32 + 2 * j) * 32 + lane] = active ? v0 : 0.f;
+        red[(warp * 32 + 2 * j + 1) * 32 + lane] = active ? v1 : 0.f;
+        unpack2(as.i[kC ? j : 0], v0, v1);
+        red[(warp * 32 + 16 + 2 * j) * 32 + lane] = active ? v0 : 0.f;
+        red[(warp * 32 + 16 + 2 * j + 1) * 32 + lane] = active ? v1 : 0.f;
+      }
+    }
+    __syncthreads();
+    // warp w finishes poles 4w .. 4w + 3
+    for (int n = warp * 4; ok && n < warp * 4 + 4 && n < a.N; ++n) {
+      float vh = 0.f, vs = 0.f;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) {
+        vh += red[(w * 32 + n) * 32 + lane];
+        vs += red[(w * 32 + 16 + n) * 32 + lane];
+      }
+      const size_t c = (size_t)row * a.N + n;
+      const float p = __ldg(a.p + c);
+      if (kC) {
+        const float gr = __ldg(a.g + 2 * c), gi = __ldg(a.g + 2 * c + 1);
+        if (r0 == 0) {   // real parts
+          atomicAdd(a.dp + c, gr * vh);
+          atomicAdd(a.dg + 2 * c, p * vh);
+          atomicAdd(a.dq + 2 * c, p * gr * vs);
+          atomicAdd(a.dq + 2 * c + 1, -p * gi * vs);
+        } else {
+          atomicAdd(a.dp + c, -gi * vh);
+          atomicAdd(a.dg + 2 * c + 1, -p * vh);
+          atomicAdd(a.dq + 2 * c, -p * gi * vs);
+          atomicAdd(a.dq + 2 * c + 1, -p * gr * vs);
+        }
+      } else {
+        const float g = __ldg(a.g + c);
+        atomicAdd(a.dp + c, g * vh);
+        atomicAdd(a.dg + c, p * vh);
+        atomicAdd(a.dq + c, p * g * vs);
+      }
+    }
+  }
+}
+
+template <typename T, bool kC, bool kMask>
+__global__ void __launch_bounds__(kWarps * 32, kC ? 2 : 3) scan_bwd_kernel(SegArgs s) {
+  // rings; bidirectional: [kWarps][T][32] share of dx.  The sums of the block go through the rings' memory.
+  extern __shared__ __align__(16) unsigned char rings[];
+  const ScanArgs& a = s.a;
+  const Lane l = lane_of(s);
+  unsigned char* ring = rings + (size_t)l.warp * 2 * kRing * kTileBytes;
+  float* part = reinterpret_cast<float*>(rings + kWarps * 2 * kRing * kTileBytes);
+  float* red = reinterpret_cast<float*>(rings);
+  const bool active = l.seg < s.S;
+  const T* x = reinterpret_cast<const T*>(a.x) + l.b * a.xsb + l.d0;
+  const T* g = reinterpret_cast<const T*>(a.dy) + l.b * a.gsb + l.d0;
+  T* dx = reinterpret_cast<T*>(a.y) + l.b * a.ysb + l.dc;
+  const unsigned char* m = kMask ? a.mask + (size_t)l.b * a.L : nullptr;
+  const float om = __ldg(a.omega + l.dc);
+  constexpr int kOne = kC ? 2 : 1;
+  float dom = 0.f;
+  for (int dir = 0; dir < (a.bidir ? 2 : 1); ++dir) {
+    State<kC> ah, as;
+    ah.zero();
+    as.zero();
+    if (active) {
+      Poles<kC> P;
+      load_poles<kC>(P, a, l.dc + dir * a.D);
+      State<kC> h, sn;
+      h.zero();
+      sn.zero();
+      if (s.carry) {
+        load_state<kC>(h, carry_at(s, l.b, dir, l.seg, 0, l.dc), a.D);
+        load_state<kC>(sn, carry_at(s, l.b, dir, l.seg, kOne, l.dc), a.D);
+      }
+      if (dir == 0) {
+        walk<T, 1, true, kMask>(x, a.xsl, g, a.gsl, m, l.t0, l.t1, l.left, ring, [&](int, float xv, float gv, bool pad) {
+          dom = fmaf(gv, xv, dom);
+          advance_sens<kC>(sn, h, P);
+          advance<kC>(h, P, splat(kMask && pad ? 0.f : xv));
+          accumulate<kC>(ah, h, splat(gv));
+          accumulate<kC>(as, sn, splat(gv));
+        });
+      } else {
+        const bool shift = a.shift != 0;
+        walk<T, -1, true, kMask>(x, a.xsl, g, a.gsl, m, l.t0, l.t1, l.left, ring, [&](int, float xv, float gv, bool pad) {
+          if (shift) {
+            accumulate<kC>(ah, h, splat(gv));
+            accumulate<kC>(as, sn, splat(gv));
+          }
+          advance_sens<kC>(sn, h, P);
+          advance<kC>(h, P, splat(kMask && pad ? 0.f : xv));
+          if (!shift) {
+            accumulate<kC>(ah, h, splat(gv));
+            accumulate<kC>(as, sn, splat(gv));
+          }
+        });
+      }
+      // the adjoint
+      State<kC> c;
+      load_weights<kC>(c, a, l.dc + dir * a.D, true);
+      h.zero();
+      if (s.carry) load_state<kC>(h, carry_at(s, l.b, dir, l.seg, 2 * kOne, l.dc), a.D);
+      float* mine = part + (size_t)l.warp * s.T * 32 + l.lane;
+      if (dir == 0) {
+        const bool bidir = a.bidir != 0;
+        float* last = mine + (l.t1 - l.t0 - 1) * 32;
+        T* pd = dx + (long long)(l.t1 - 1) * a.ysl;
+        walk<T, -1, false, kMask>(g, a.gsl, g, 0, m, l.t0, l.t1, l.left, ring, [&](int k, float gv, float, bool pad) {
+          advance<kC>(h, P, splat(gv));
+          const float v = fmaf(om, gv, kMask && pad ? 0.f : dot<kC>(c, h));
+          if (bidir) last[-k * 32] = v;
+          else if (l.ok) Elem<T>::st(pd, v);
+          pd -= a.ysl;
+        });
+      } else {
+        const bool shift = a.shift != 0;
+        T* pd = dx + (long long)l.t0 * a.ysl;
+        walk<T, 1, false, kMask>(g, a.gsl, g, 0, m, l.t0, l.t1, l.left, ring, [&](int k, float gv, float, bool pad) {
+          float v = 0.f;
+          if (shift) v = dot<kC>(c, h);
+          advance<kC>(h, P, splat(gv));
+          if (!shift) v = dot<kC>(c, h);
+          v = mine[k * 32] + (kMask && pad ? 0.f : v);
+          if (l.ok) Elem<T>::st(pd, v);
+          pd += a.ysl;
+        });
+      }
+    }
+    reduce_grads<kC>(ah, as, a, l.dc + dir * a.D, l.ok, active, red);
+    __syncthreads();   // (the rings are free again)
+  }
+  // domega: the block's four segments
+  __syncthreads();
+  red[l.warp * 32 + l.lane] = dom;
+  __syncthreads();
+  if (l.warp == 0 && l.ok) {
+    float v = 0.f;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) v += red[w * 32 + l.lane];
+    atomicAdd(a.domega + l.d, v);
+  }
+}
+
+// Segments of a call.  A block takes four segments of 32 channels; `resident` blocks of the last kernel fit an SM.
+// The choice minimises (rounds of blocks over the 148 SMs) x (steps of a segment + what its states cost beside
+// them: written, carried and read, 64 steps' worth backward and 40 forward), so that neither a nearly empty last round nor short segments dominate.  Segments
+// are at least 32 steps; a bidirectional one keeps its share of the outputs in shared memory, so at most 64.
+// One segment per sequence when the channels alone fill the device: no first pass then.
+static void pick_segments(const ScanArgs& a, int resident, bool bwd, SegArgs& s) {
+  const long long strips = (long long)((a.D + 31) / 32) * a.B;
+  const double slots = 148.0 * resident;
+  double best = 1e30;
+  s.wide = 0;
+  if (!a.bidir && !bwd) {
+    s.T = a.L;
+    s.S = 1;
+    s.wide = 1;
+    const long long blocks = (long long)((a.D + 32 * kWarps - 1) / (32 * kWarps)) * a.B;
+    // (2/3: without the first pass; few warps on an SM still leave its pipes idle: at least half of the slots)
+    best = ceil(blocks / slots) * a.L * (2.0 / 3.0) * (blocks * 2 < slots ? 2.0 : 1.0);
+  }
+  for (int S = kWarps; S <= 4096; S += kWarps) {
+    int t = ((a.L + S - 1) / S + kU - 1) / kU * kU;
+    if (t < 32) t = 32;
+    if (a.bidir && t > 64) continue;
+    const int n = (a.L + t - 1) / t;
+    const long long blocks = strips * ((n + kWarps - 1) / kWarps);
+    const double cost = ceil(blocks / slots) * (t + (bwd ? 64 : 40));
+    if (cost < best) {
+      best = cost;
+      s.T = t;
+      s.S = n;
+      s.wide = 0;
+    }
+    if (t == 32) break;
+  }
+}
+
+template <typename T, bool kC, bool kMask>
+static bool fwd_launch(const SegArgs& s, cudaStream_t st) {
+  const ScanArgs& a = s.a;
+  const int dirs = a.bidir ? 2 : 1;
+  const dim3 block(kWarps * 32);
+  const dim3 grid(s.wide ? (a.D + 32 * kWarps - 1) / (32 * kWarps) : (a.D + 31) / 32, (s.S + kWarps - 1) / kWarps, a.B);
+  const bool state = a.h_in || a.h_out;
+  const size_t rings = (size_t)kWarps * kRing * kTileBytes;
+  if (s.carry) {
+    launch(scan_local_kernel<T, kC, kMask, false>, dim3(grid.x, grid.y, a.B * dirs), block, rings, (void*)st, s);
+    launch(scan_carry_kernel<kC, false>, dim3((a.D + 127) / 128, 16, a.B * dirs), 128, 0, (void*)st, s, state ? 1 : 0);
+  }
+  const size_t smem = rings + (a.bidir ? (size_t)kWarps * s.T * 32 * 4 : 0);
+  if (state) launch(scan_emit_kernel<T, kC, kMask, true>, grid, block, smem, (void*)st, s);
+  else launch(scan_emit_kernel<T, kC, kMask, false>, grid, block, smem, (void*)st, s);
+  return true;
+}
+
+template <typename T, bool kC, bool kMask>
+static bool bwd_launch(const SegArgs& s, cudaStream_t st) {
+  const ScanArgs& a = s.a;
+  const int dirs = a.bidir ? 2 : 1;
+  const dim3 block(kWarps * 32);
+  const dim3 grid((a.D + 31) / 32, (s.S + kWarps - 1) / kWarps, a.B);
+  const size_t rings = (size_t)kWarps * kRing * kTileBytes;
+  if (s.carry) {
+    launch(scan_local_kernel<T, kC, kMask, true>, dim3(grid.x, grid.y, a.B * dirs), block, rings, (void*)st, s);
+    launch(scan_carry_kernel<kC, true>, dim3((a.D + 127) / 128, 16, a.B * dirs), 128, 0, (void*)st, s, 0);
+  }
+  const size_t smem = 2 * rings + (a.bidir ? (size_t)kWarps * s.T * 32 * 4 : 0);
+  launch(scan_bwd_kernel<T, kC, kMask>, grid, block, smem, (void*)st, s);
+  return true;
+}
+
+template <bool kBwd>
+static bool dispatch(int dtype, const ScanArgs& a, cudaStream_t st) {
+  if (g_options[OPT_DISABLE_STREAM].load() != 0) return false;
+  const int dirs = a.bidir ? 2 : 1;
+  if (a.N > 16 || (long long)a.B * dirs > 65535 || a.L < 1) return false;
+  SegArgs s{};
+  s.a = a;
+  // blocks per SM by registers
+  pick_segments(a, kBwd ? (a.cplx ? 2 : 3) : (a.cplx ? 3 : 4), kBwd, s);
+  if ((s.S + kWarps - 1) / kWarps > 65535) return false;
+  s.parts = (kBwd ? 3 : 1) * (a.cplx ? 2 : 1);
+  const size_t floats = (!s.wide) ? (size_t)a.B * dirs * s.S * s.parts * 16 * a.D : 0;
+  Scratch sc(floats ? Scratch::padded(floats * 4) : 256, st);
+  if (!sc) return false;
+  s.carry = floats ? sc.take<float>(floats) : nullptr;
+#define MEGA_SCAN(TY)                                                                                           \
+  (a.cplx ? (a.mask ? (kBwd ? bwd_launch<TY, true, true>(s, st) : fwd_launch<TY, true, true>(s, st))             \
+                    : (kBwd ? bwd_launch<TY, true, false>(s, st) : fwd_launch<TY, true, false>(s, st)))          \
+          : (a.mask ? (kBwd ? bwd_launch<TY, false, true>(s, st) : fwd_launch<TY, false, true>(s, st))           \
+                    : (kBwd ? bwd_launch<TY, false, false>(s, st) : fwd_launch<TY, false, false>(s, st))))
+  switch (dtype) {
+    case MEGA_F32: return MEGA_SCAN(float);
+    case MEGA_BF16: return MEGA_SCAN(__nv_bfloat16);
+    case MEGA_F16: return MEGA_SCAN(__half);
+    default: return false;
+  }
+#undef MEGA_SCAN
+}
+
+}  // namespace
+
+bool scan_ema_fwd_try(int dtype, const ScanArgs& a, long long xsd, long long ysd, cudaStream_t s) {
+  if (!rows_ok(dtype, a.x, a.xsb, a.xsl, xsd, a.D) || ysd != 1 || a.x == a.y) return false;
+  return dispatch<false>(dtype, a, s);
+}
+
+bool scan_ema_bwd_try(int dtype, const ScanArgs& a, long long xsd, long long ysd, long long gsd, cudaStream_t s) {
+  if (!rows_ok(dtype, a.x, a.xsb, a.xsl, xsd, a.D) || !rows_ok(dtype, a.dy, a.gsb, a.gsl, gsd, a.D) || ysd != 1 || a.h_in ||
+      a.h_out)
+    return false;
+  return dispatch<true>(dtype, a, s);
+}
+
+}  // namespace mega

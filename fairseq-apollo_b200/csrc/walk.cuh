@@ -1,0 +1,105 @@
+// How the kernels that are parallel over time (scan_ema.cu, scan_norm.cu) read their inputs: a warp walks one
+// segment of 32 adjacent channels, a lane one channel.
+#pragma once
+#include "common.cuh"
+#include "tma.cuh"
+
+namespace mega {
+
+namespace {
+
+constexpr int kWarps = 4;   // warps (segments) per block
+constexpr int kU = 8;       // steps of an unrolled group
+
+// ---- the inputs of a walk ----------------------------------------------------------------------------
+// A warp fetches its 32 channels in tiles of 2 KB (32 steps of a 16-bit type, 16 of fp32) with 16-byte
+// asynchronous copies into a ring of its own, kRing - 1 tiles ahead of their use: loads straight into registers,
+// eight steps ahead, kept too few bytes in flight (0.6 TB/s on B = 8, L = 4096, D = 1024 bf16).  No barrier
+// beyond the warp's is involved.
+constexpr int kTileBytes = 2048;
+constexpr int kRing = 4;
+
+template <typename T>
+__device__ __forceinline__ void fetch_tile(uint32_t dst, const T* row, long long stride, int rows, int d_left, int lane) {
+  constexpr int kPer = 32 * (int)sizeof(T) / 16;   // 16-byte pieces of a row
+#pragma unroll
+  for (int i = 0; i < kTileBytes / 16 / 32; ++i) {
+    const int id = lane + 32 * i;
+    const int r = id / kPer, c = (id % kPer) * (16 / (int)sizeof(T));
+    const bool in = r < rows && c < d_left;
+    const T* src = in ? row + (long long)r * stride + c : row;
+    asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16, %2;" ::"r"(dst + id * 16), "l"(src), "r"(in ? 16 : 0)
+                 : "memory");
+  }
+}
+__device__ __forceinline__ void tile_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void tile_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// Walks the steps [t0, t1) of 32 channels in time order (kDir = 1) or reversed (-1); f(k, v, g, pad) sees step
+// k = 0, 1, ... of that order.  x, g: first channel of the warp; ring: the warp's (two of them with kTwo).
+template <typename T, int kDir, bool kTwo, bool kMask, typename F>
+__device__ __forceinline__ void walk(const T* x, long long xsl, const T* g, long long gsl, const unsigned char* m, int t0,
+                                     int t1, int d_left, unsigned char* ring, F&& f) {
+  constexpr int kR = kTileBytes / (32 * (int)sizeof(T));
+  const int lane = threadIdx.x & 31;
+  const int n = t1 - t0;
+  const int first = kDir > 0 ? t0 : t1 - 1;
+  const T* px = x + (long long)first * xsl;
+  const T* pg = kTwo ? g + (long long)first * gsl : nullptr;
+  const long long dx = kDir > 0 ? xsl : -xsl, dg = kDir > 0 ? gsl : -gsl;
+  const int tiles = (n + kR - 1) / kR;
+  const uint32_t rs = smem_u32(ring);
+  auto issue = [&](int j) {
+    if (j < tiles) {
+      const int slot = j % kRing;
+      fetch_tile<T>(rs + slot * kTileBytes, px + (long long)(j * kR) * dx, dx, n - j * kR, d_left, lane);
+      if (kTwo)
+        fetch_tile<T>(rs + (kRing + slot) * kTileBytes, pg + (long long)(j * kR) * dg, dg, n - j * kR, d_left, lane);
+    }
+    tile_commit();
+  };
+  auto flags = [&](int j) -> unsigned {   // bit r: step r of tile j is padded
+    if (!kMask) return 0u;
+    const int k = j * kR + lane;
+    const bool pad = lane < kR && k < n && __ldg(m + first + kDir * k) != 0;
+    return __ballot_sync(0xffffffffu, pad);
+  };
+  __syncwarp();   // (the walk before has read the last tiles of the ring)
+#pragma unroll
+  for (int j = 0; j < kRing - 1; ++j) issue(j);
+  unsigned next = flags(0);
+  for (int j = 0; j < tiles; ++j) {
+    tile_wait<kRing - 2>();
+    __syncwarp();
+    issue(j + kRing - 1);
+    const unsigned bits = next;
+    if (j + 1 < tiles) next = flags(j + 1);
+    const T* tx = reinterpret_cast<const T*>(ring + (j % kRing) * kTileBytes) + lane;
+    const T* tg = reinterpret_cast<const T*>(ring + (kRing + j % kRing) * kTileBytes) + lane;
+    const int rows = min(kR, n - j * kR);
+    int r0 = 0;
+    for (; r0 + kU <= rows; r0 += kU) {
+#pragma unroll
+      for (int u = 0; u < kU; ++u)
+        f(j * kR + r0 + u, Elem<T>::ld_shared(tx + (r0 + u) * 32), kTwo ? Elem<T>::ld_shared(tg + (r0 + u) * 32) : 0.f,
+          kMask && ((bits >> (r0 + u)) & 1u) != 0);
+    }
+    for (; r0 < rows; ++r0)
+      f(j * kR + r0, Elem<T>::ld_shared(tx + r0 * 32), kTwo ? Elem<T>::ld_shared(tg + r0 * 32) : 0.f,
+        kMask && ((bits >> r0) & 1u) != 0);
+  }
+  tile_wait<0>();
+}
+
+}  // namespace
+
+// channels contiguous, rows in whole 16-byte pieces
+static inline bool rows_ok(int dtype, const void* p, long long sb, long long sl, long long sd, int D) {
+  const long long es = elem_size(dtype);
+  return sd == 1 && aligned_to(p, 16) && (sb * es) % 16 == 0 && (sl * es) % 16 == 0 && (D * es) % 16 == 0;
+}
+
+}  // namespace mega
