@@ -45,6 +45,7 @@ SIGNATURES = {
     "mega_timestep_norm_fwd_train": [c_p, c_p, c_i, c_i, c_i, c_i, c_l, c_l, c_l, c_l, c_l, c_l, c_p, c_p, c_p,
                                      c_p, c_p, c_p, c_i, c_d, c_p, c_p, c_p, c_p, c_p, c_p, c_p],
     "mega_timestep_norm_bwd": [c_p, c_p, c_p, c_i, c_i, c_i, c_i] + [c_l] * 9 + [c_p] * 9 + [c_i] + [c_p] * 5,
+    "mega_timestep_norm_bwd_stats": [c_p, c_p, c_p, c_i, c_i, c_i, c_i] + [c_l] * 9 + [c_p] * 7 + [c_d] + [c_p] * 5,
     "mega_sequence_norm_bwd": [c_p, c_p, c_p, c_i, c_i, c_i, c_i] + [c_l] * 9 + [c_p] * 5 + [c_i] + [c_p] * 3,
     "mega_ema_bwd": [c_p, c_p, c_p, c_i, c_i, c_i, c_i] + [c_l] * 9 + [c_p] * 4 + [c_i] + [c_p] * 3 + [c_u, c_i]
                     + [c_p] * 6,

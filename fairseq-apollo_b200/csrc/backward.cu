@@ -10,6 +10,7 @@
 // Four lanes share a (batch, channel) row and split its poles; sums over the batch are atomic adds.
 #include "common.cuh"
 #include "scan_ema.cuh"
+#include "scan_norm.cuh"
 #include "stream_bwd.cuh"
 
 namespace mega {
@@ -665,6 +666,31 @@ extern "C" int mega_timestep_norm_bwd(const void* dy, const void* x, void* dx, i
     MEGA_DISPATCH_DTYPE(dtype, launch(tsn_bwd_group_kernel<T>, grid, 128, 0, stream, a));
   }
   return check_launch("timestep_norm_bwd");
+}
+
+extern "C" int mega_timestep_norm_bwd_stats(const void* dy, const void* x, void* dx, int dtype, int B, int L, int D,
+                                            int64_t gsb, int64_t gsl, int64_t gsd, int64_t xsb, int64_t xsl, int64_t xsd,
+                                            int64_t dsb, int64_t dsl, int64_t dsd, const float* dmean, const float* dvar,
+                                            const int64_t* prev_count, const float* prev_mean, const float* prev_var,
+                                            const float* gamma, const uint8_t* pad_mask, double eps, float* dprev_mean,
+                                            float* dprev_var, float* dgamma, float* dbeta, mega_stream_t stream) {
+  if (!dy || !x || !dx || !prev_count || !prev_mean || !prev_var || !gamma || !dprev_mean || !dprev_var || !dgamma ||
+      !dbeta)
+    return MEGA_ERR_NULL;
+  if (!valid_dtype(dtype)) return MEGA_ERR_DTYPE;
+  if (B <= 0 || L <= 0 || D <= 0) return MEGA_ERR_SHAPE;
+  cudaStream_t s = (cudaStream_t)stream;
+  ScanNormArgs na{};
+  na.x = x; na.y = dx; na.dy = dy; na.B = B; na.D = D; na.L = L;
+  na.xsb = xsb; na.xsl = xsl; na.ysb = dsb; na.ysl = dsl; na.gsb = gsb; na.gsl = gsl;
+  na.prev_count = (const long long*)prev_count; na.prev_mean = prev_mean; na.prev_var = prev_var; na.gamma = gamma;
+  na.mask = pad_mask; na.eps = (float)eps; na.dmean = dmean; na.dvar = dvar;
+  na.dprev_mean = dprev_mean; na.dprev_var = dprev_var; na.dgamma = dgamma; na.dbeta = dbeta;
+  if (cudaMemsetAsync(dgamma, 0, (size_t)D * sizeof(float), s) != cudaSuccess ||
+      cudaMemsetAsync(dbeta, 0, (size_t)D * sizeof(float), s) != cudaSuccess)
+    return check_launch("timestep_norm_bwd_stats(memset)");
+  if (!scan_norm_bwd_try(dtype, na, xsd, dsd, gsd, s)) return MEGA_ERR_UNSUPPORTED;
+  return check_launch("timestep_norm_bwd_stats");
 }
 
 extern "C" int mega_sequence_norm_bwd(const void* dy, const void* x, void* dx, int dtype, int B, int D, int L,

@@ -6,6 +6,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "scan_norm.cuh"
 #include "stream_bwd.cuh"
 #include "stream_cl.cuh"
 
@@ -486,7 +487,15 @@ static int tsn_fwd_common(const void* x, void* y, int dtype, int B, int L, int D
       sa.beta = beta; sa.eps = (float)eps; sa.count_out = a.count_out; sa.mean_out = mean_out; sa.var_out = var_out;
       sa.mask = pad_mask;
       sa.cummean = cummean; sa.cumrstd = cumrstd;
-      // bf16 without a mask and without the saves for backward: the tensor-core kernel's prefix sums
+      if (!cummean && g_options[OPT_MMA_TILE].load() == 0 && g_options[OPT_DISABLE_MMA].load() == 0) {
+        ScanNormArgs na{};
+        na.x = x; na.y = y; na.B = B; na.D = D; na.L = L;
+        na.xsb = xsb; na.xsl = xsl; na.ysb = ysb; na.ysl = ysl;
+        na.prev_count = a.prev_count; na.prev_mean = prev_mean; na.prev_var = prev_var; na.gamma = gamma; na.beta = beta;
+        na.mask = pad_mask; na.eps = (float)eps; na.count_out = a.count_out; na.mean_out = mean_out; na.var_out = var_out;
+        if (scan_norm_fwd_try(dtype, na, xsd, ysd, (cudaStream_t)stream)) return check_launch("timestep_norm_fwd(scan)");
+      }
+      // (a form of the tensor-core kernel asked for by name, or the streamed kernel)
       if (!cummean && mma_cl_try(dtype, x, y, nullptr, xsb, xsl, xsd, ysb, ysl, ysd, true, sa, (cudaStream_t)stream))
         return check_launch("timestep_norm_fwd(mma)");
       if (stream_cl_try(dtype, x, y, nullptr, xsb, xsl, xsd, ysb, ysl, ysd, true, false, sa, (cudaStream_t)stream))

@@ -1,0 +1,29 @@
+// Interface of the per-feature TimestepNorm that is parallel over time (scan_norm.cu).
+#pragma once
+#include <cuda_runtime.h>
+
+namespace mega {
+
+struct ScanNormArgs {
+  const void* x;
+  void* y;          // forward: output; backward: input gradient
+  const void* dy;
+  int B, D, L;
+  long long xsb, xsl, ysb, ysl, gsb, gsl;
+  const long long* prev_count;
+  const float *prev_mean, *prev_var;   // (B, D)
+  const float *gamma, *beta;
+  const unsigned char* mask;           // (B, L) or null
+  float eps;
+  long long* count_out;                // forward
+  float *mean_out, *var_out;
+  const float *dmean, *dvar;           // backward: gradients of the returned statistics, or null
+  float *dprev_mean, *dprev_var, *dgamma, *dbeta;
+};
+
+// Each returns false, having launched nothing, outside its envelope (channels not contiguous, rows that are not
+// whole 16-byte pieces, too many sequences for the grid) or when there is no scratch memory.
+bool scan_norm_fwd_try(int dtype, const ScanNormArgs& a, long long xsd, long long ysd, cudaStream_t s);
+bool scan_norm_bwd_try(int dtype, const ScanNormArgs& a, long long xsd, long long ysd, long long gsd, cudaStream_t s);
+
+}  // namespace mega

@@ -62,24 +62,41 @@ class ComplexEMAFunction(torch.autograd.Function):
 
 
 class TimestepNormFunction(torch.autograd.Function):
-    """(y, count, mean, var) = TimestepNorm(x (B, L, D)); gamma is the effective scale."""
+    """(y, count, mean, var) = TimestepNorm(x (B, L, D)); gamma is the effective scale.  Per-feature statistics
+    (channels contiguous) are taken again in the backward, so only the arguments are kept; otherwise the
+    statistics of every step are."""
 
     @staticmethod
     def forward(ctx, x, prev_count, prev_mean, prev_var, gamma, beta, padding_mask, num_groups, eps):
-        y, count, mean, var, cummean, cumrstd, group_mean = ops.timestep_norm_fwd_train(
-            x, prev_count, prev_mean, prev_var, gamma, beta, padding_mask, eps, num_groups)
-        ctx.save_for_backward(x, prev_mean, count, cummean, cumrstd, group_mean, gamma, padding_mask)
-        ctx.num_groups = num_groups
+        ctx.recompute = num_groups is None and ops.timestep_norm_keeps_nothing(x)
+        if ctx.recompute:
+            prev_count = prev_count.to(torch.int64).contiguous()
+            y, count, mean, var = ops.timestep_norm_fwd(x, prev_count, prev_mean, prev_var, gamma, beta, padding_mask, eps)
+            ctx.save_for_backward(x, prev_count, prev_mean, prev_var, gamma, padding_mask)
+        else:
+            y, count, mean, var, cummean, cumrstd, group_mean = ops.timestep_norm_fwd_train(
+                x, prev_count, prev_mean, prev_var, gamma, beta, padding_mask, eps, num_groups)
+            ctx.save_for_backward(x, prev_mean, count, cummean, cumrstd, group_mean, gamma, padding_mask)
+        ctx.num_groups, ctx.eps = num_groups, eps
         ctx.dtypes = (prev_mean.dtype, prev_var.dtype, gamma.dtype, beta.dtype)
         ctx.mark_non_differentiable(count)
+        ctx.set_materialize_grads(False)
         return y, count, mean, var
 
     @staticmethod
     def backward(ctx, dy, _, dmean, dvar):
-        x, prev_mean, count, cummean, cumrstd, group_mean, gamma, padding_mask = ctx.saved_tensors
-        dx, dpm, dpv, dgamma, dbeta = ops.timestep_norm_bwd(dy, dmean, dvar, x, prev_mean, count, cummean,
-                                                            cumrstd, group_mean, gamma, padding_mask,
-                                                            ctx.num_groups)
+        x = ctx.saved_tensors[0]
+        if dy is None:
+            dy = torch.zeros_like(x)
+        if ctx.recompute:
+            x, prev_count, prev_mean, prev_var, gamma, padding_mask = ctx.saved_tensors
+            dx, dpm, dpv, dgamma, dbeta = ops.timestep_norm_bwd_stats(dy, dmean, dvar, x, prev_count, prev_mean, prev_var,
+                                                                      gamma, padding_mask, ctx.eps)
+        else:
+            x, prev_mean, count, cummean, cumrstd, group_mean, gamma, padding_mask = ctx.saved_tensors
+            dx, dpm, dpv, dgamma, dbeta = ops.timestep_norm_bwd(dy, dmean, dvar, x, prev_mean, count, cummean,
+                                                                cumrstd, group_mean, gamma, padding_mask,
+                                                                ctx.num_groups)
         t = ctx.dtypes
         return dx, None, dpm.to(t[0]), dpv.to(t[1]), dgamma.to(t[2]), dbeta.to(t[3]), None, None, None
 

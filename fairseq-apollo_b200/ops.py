@@ -482,6 +482,38 @@ def timestep_norm_bwd(dy, dmean, dvar, x, prev_mean, count, cummean, cumrstd, gr
     return dx, dpm, dpv, dgamma, dbeta
 
 
+def timestep_norm_keeps_nothing(x):
+    """Whether timestep_norm_bwd_stats takes x (B, L, D): contiguous channels in whole 16-byte pieces."""
+    es = x.element_size()
+    return (x.stride(2) == 1 and x.shape[2] * es % 16 == 0 and x.stride(0) * es % 16 == 0
+            and x.stride(1) * es % 16 == 0 and x.data_ptr() % 16 == 0)
+
+
+def timestep_norm_bwd_stats(dy, dmean, dvar, x, prev_count, prev_mean, prev_var, gamma, padding_mask=None, eps=1e-5):
+    """Gradients of the per-feature TimestepNorm from the statistics its forward started with:
+    (dx, dprev_mean, dprev_var, dgamma, dbeta)."""
+    _cuda(dy, dmean, dvar, x, prev_count, prev_mean, prev_var, gamma, padding_mask)
+    bsz, length, dim = x.shape
+    if dy.dtype != x.dtype:
+        dy = dy.to(x.dtype)
+    if not timestep_norm_keeps_nothing(dy):
+        dy = dy.contiguous()
+    dmean, dvar, prev_mean, prev_var, gamma = _f32c(dmean), _f32c(dvar), _f32c(prev_mean), _f32c(prev_var), _f32c(gamma)
+    mask = _mask_u8(padding_mask, bsz, length)
+    dx = _like(x)
+    dpm = torch.empty(bsz, dim, device=x.device, dtype=torch.float32)
+    dpv = torch.empty_like(dpm)
+    dgamma = torch.empty(dim, device=x.device, dtype=torch.float32)
+    dbeta = torch.empty_like(dgamma)
+    with torch.cuda.device(x.device):
+        _lib.check(_lib.lib().mega_timestep_norm_bwd_stats(
+            dy.data_ptr(), x.data_ptr(), dx.data_ptr(), _dt(x), bsz, length, dim, *dy.stride(), *x.stride(),
+            *dx.stride(), _ptr(dmean), _ptr(dvar), prev_count.data_ptr(), prev_mean.data_ptr(), prev_var.data_ptr(),
+            gamma.data_ptr(), _ptr(mask), float(eps), dpm.data_ptr(), dpv.data_ptr(), dgamma.data_ptr(),
+            dbeta.data_ptr(), _stream()), "timestep_norm_bwd_stats")
+    return dx, dpm, dpv, dgamma, dbeta
+
+
 def sequence_norm_bwd(dy, x, count, mean, rstd, gamma, padding_mask=None, length_last=True, num_groups=None):
     """Gradients of SequenceNorm (per channel, or per group with ``num_groups``): (dx, dgamma, dbeta)."""
     _cuda(dy, x, count, mean, rstd, gamma, padding_mask)

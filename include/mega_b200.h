@@ -342,6 +342,20 @@ MEGA_API int mega_timestep_norm_bwd(const void* dy, const void* x, void* dx, int
                            float* dgamma, float* dbeta, mega_stream_t stream);
 
 /*
+ * mega_timestep_norm_bwd_stats: the same gradients for the per-feature form, from the statistics the forward
+ * STARTED with (prev_count, prev_mean, prev_var) instead of saves of every step: nothing has to be kept from
+ * mega_timestep_norm_fwd but its arguments.  Channels contiguous (stride 1) in all three tensors, base
+ * addresses and the strides of x and dy multiples of 16 bytes, D whole 16-byte pieces, dx distinct from both;
+ * MEGA_ERR_UNSUPPORTED otherwise.
+ */
+MEGA_API int mega_timestep_norm_bwd_stats(const void* dy, const void* x, void* dx, int dtype, int B, int L, int D,
+                           int64_t gsb, int64_t gsl, int64_t gsd, int64_t xsb, int64_t xsl, int64_t xsd,
+                           int64_t dsb, int64_t dsl, int64_t dsd, const float* dmean, const float* dvar,
+                           const int64_t* prev_count, const float* prev_mean, const float* prev_var,
+                           const float* gamma, const uint8_t* pad_mask, double eps, float* dprev_mean,
+                           float* dprev_var, float* dgamma, float* dbeta, mega_stream_t stream);
+
+/*
  * mega_sequence_norm_bwd: gradients of SequenceNorm (per-channel and grouped forms; mean, rstd are (B, G)).  dy, x, dx are (B, D, L)
  * with strides in elements (the length-major order of a (B, L, D) tensor is a stride pattern);
  * count (B), mean, rstd (B, D) are the forward's outputs.  dgamma, dbeta (D) are zeroed on the
