@@ -15,6 +15,16 @@ c_u = ctypes.c_uint
 c_l = ctypes.c_int64
 c_d = ctypes.c_double
 
+class BlockStepArgs(ctypes.Structure):
+    """mega_block_step_args of include/mega_b200.h."""
+    _fields_ = ([(n, ctypes.c_int32) for n in ("dtype", "batch", "embed", "zdim", "hdim", "ndim", "complex_poles",
+                                               "positions")]
+                + [(n, c_p) for n in ("x", "out", "count", "count_next", "mean", "var", "h", "norm_gamma", "norm_beta", "p",
+                                      "q", "gamma_hat", "omega", "v_weight", "v_bias", "mx_weight", "mx_bias", "h_weight",
+                                      "qk_gamma", "qk_beta", "rot", "keys", "keys_rot", "values", "work")]
+                + [("norm_eps", c_d), ("qk_eps", c_d), ("cap", c_l), ("pos", ctypes.c_int32)])
+
+
 # name -> argument types, in the order of include/mega_b200.h
 SIGNATURES = {
     "mega_ema_coeffs": [c_p, c_p, c_p, c_p, c_i, c_i, c_i, c_p, c_p, c_p, c_p],
@@ -63,6 +73,8 @@ SIGNATURES = {
                                            c_p],
     "mega_tsn_cema_fwd": [c_p, c_p, c_p, c_i, c_i, c_i, c_i, c_l, c_l, c_l, c_l, c_l, c_l, c_p, c_p, c_p,
                           c_p, c_p, c_d, c_p, c_p, c_p, c_p, c_p, c_p, c_p, c_i, c_p, c_p, c_p, c_u, c_p],
+    "mega_block_step": [c_p, c_p],
+    "mega_block_cache_fill": [c_p, c_l, c_l, c_p, c_l, c_l, c_p, c_i, c_i, c_i, c_i, c_i, c_i, c_p, c_p, c_p, c_l, c_p],
     "mega_set_option": [c_i, c_i],
     "mega_debug_device_error": [ctypes.POINTER(c_i), c_i],
 }
@@ -70,6 +82,7 @@ OTHER = {
     "mega_status_string": ([c_i], ctypes.c_char_p),
     "mega_last_cuda_error": ([], ctypes.c_char_p),
     "mega_abi_version": ([], c_i),
+    "mega_block_step_work": ([c_i, c_i, c_i, c_i, c_i, c_l], c_l),
     "mega_launch_count": ([], ctypes.c_uint64),
     "mega_debug_last_kernel": ([], ctypes.c_char_p),
 }

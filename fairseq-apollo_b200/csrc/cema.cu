@@ -6,6 +6,7 @@
 #include "common.cuh"
 #include "stream_bwd.cuh"
 #include "stream_cl.cuh"
+#include "block_step.cuh"
 #include "scan_ema.cuh"
 
 namespace mega {
@@ -343,6 +344,23 @@ static bool launch_cema_step_lanes(const T* x, T* y, T* xn_out, int B, int D, in
   else MEGA_CEMA_STEP_LANES(16);
 #undef MEGA_CEMA_STEP_LANES
   return true;
+}
+
+bool cema_step_lanes_try(int dtype, const void* x, void* y, void* xn_out, int B, int D, int N, const long long* count,
+                         float* mean, float* var, const float* gamma, const float* beta, float eps, const float* p,
+                         const float* q, const float* g, const float* omega, const float* h_in, float* h_out, int silu,
+                         void* stream, long long* count_next) {
+  switch (dtype) {
+#define MEGA_CEMA_STEP_CASE(DT, TY)                                                                                    \
+  case DT:                                                                                                             \
+    return launch_cema_step_lanes<TY>((const TY*)x, (TY*)y, (TY*)xn_out, B, D, N, count, mean, var, gamma, beta, eps,  \
+                                      p, q, g, omega, h_in, h_out, silu, stream, count_next);
+    MEGA_CEMA_STEP_CASE(MEGA_F32, float)
+    MEGA_CEMA_STEP_CASE(MEGA_BF16, __nv_bfloat16)
+    MEGA_CEMA_STEP_CASE(MEGA_F16, __half)
+#undef MEGA_CEMA_STEP_CASE
+    default: return false;
+  }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -693,13 +711,10 @@ extern "C" int mega_tsn_cema_step(const void* x, void* y, void* xn_out, int dtyp
   if (B <= 0 || D <= 0) return MEGA_ERR_SHAPE;
   if (N < 1 || N > MEGA_MAX_NDIM) return MEGA_ERR_NDIM;
   const int silu = (flags & MEGA_EMA_SILU) ? 1 : 0;
-  bool lanes = false;
   // a distinct count_next array takes the bumped counts from the element kernel itself
   long long* next = (count_next && count_next != count) ? (long long*)count_next : nullptr;
-  MEGA_DISPATCH_DTYPE(dtype, lanes = launch_cema_step_lanes<T>((const T*)x, (T*)y, (T*)xn_out, B, D, N,
-                                                              (const long long*)count, mean, var, gamma, beta,
-                                                              (float)eps, p, q, gamma_hat, omega, h, h, silu, stream,
-                                                              next));
+  const bool lanes = cema_step_lanes_try(dtype, x, y, xn_out, B, D, N, (const long long*)count, mean, var, gamma, beta,
+                                         (float)eps, p, q, gamma_hat, omega, h, h, silu, stream, next);
   if (!lanes) return MEGA_ERR_UNSUPPORTED;  // pole counts other than 2, 4, 8, 16, 32, or unaligned states
   if (!next) launch(cema_count_step_kernel, (unsigned)((B + 127) / 128), 128, 0, stream, (long long*)count, B);
   return check_launch("tsn_cema_step");

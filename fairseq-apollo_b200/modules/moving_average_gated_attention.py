@@ -31,6 +31,7 @@ from torch.nn import Parameter
 from .. import ops
 from ..functions import needs_grad
 from ..incremental_state import IncrementalStateMixin
+from . import block_decode
 from .attention_softmax import AttentionSoftmax
 from .complex_exponential_moving_average import MultiHeadComplexEMA
 from .efficient_attention import EfficientAttention
@@ -243,6 +244,13 @@ class MovingAverageGatedAttention(IncrementalStateMixin, nn.Module):
                 need_weights: bool = False, attn_mask: Optional[Tensor] = None,
                 before_attn_fn: bool = False) -> Tuple[Tensor, Optional[Tensor]]:
         """x: (B, L, D) -> (out (B, L, D), attention weights or None)."""
+        if (incremental_state is not None and padding_mask is None and x.size(1) == 1 and x.is_cuda
+                and not torch.is_grad_enabled() and attn_mask is None and not need_weights and not before_attn_fn
+                and not (self.training and (self.dropout_p or self.hidden_dropout_p or self.attention_dropout_p))
+                and x.is_contiguous() and x.size(2) == self.embed_dim):
+            out = block_decode.step(self, x, incremental_state)   # decoding: one call for the whole block
+            if out is not None:
+                return out, None
         bsz, seq_len, embed_dim = x.size()
         assert embed_dim == self.embed_dim
         saved_state = self._get_input_buffer(incremental_state) if incremental_state is not None else None

@@ -501,6 +501,45 @@ MEGA_API int mega_attention_dropkey_softmax_fwd(const void* x, void* y, int dtyp
                                        int inner, int causal, double dropout, uint64_t seed, uint64_t offset,
                                        mega_stream_t stream);
 
+/*
+ * ---- One decoding step of the causal Mega block ----------------------------------------------
+ * For x (batch, embed) contiguous: the running state (count / mean / var / h as in mega_tsn_ema_step,
+ * mega_tsn_cema_step with complex_poles; count -> count_next, two arrays), mx = SiLU(EMA(TimestepNorm(x))),
+ * v = SiLU(v_proj(xn)), [u, z, r, hx] = mx_proj(mx), query and key from z (mega_gate_qk_rotary's definition,
+ * position `pos` of the chunk), softmax over the pos + 1 keys of the chunk, and
+ * out = x + sigmoid(u) * (SiLU(hx + h_proj(attn * SiLU(r))) - x).
+ * keys (batch, cap, zdim) receives the key before the rotary embedding, keys_rot after it, values
+ * (batch, cap, hdim) SiLU(v), each at row `pos`; rows 0 .. pos - 1 are read.  Weights are row-major (out, in) in
+ * `dtype` (bf16 or fp16), biases too, the rest fp32; rot as in mega_gate_qk_rotary with `positions` rows.
+ * work: mega_block_step_work bytes, 16-byte aligned like every activation and weight pointer.
+ * MEGA_ERR_UNSUPPORTED: batch > 64, embed or hdim not a multiple of 32, zdim other than 64, 128, 256, pole counts
+ * mega_tsn_ema_step's fast form does not take, activations beyond a block's shared memory.
+ * Replaces: MovingAverageGatedAttention.forward with one position and an incremental state
+ * (fairseq/modules/moving_average_gated_attention.py:282-414).
+ *
+ * mega_block_cache_fill: keys k (batch, n, zdim) before the rotary embedding and values v (batch, n, hdim) of a
+ * prompt (strides of batch and position in elements) into the step's buffers.
+ */
+typedef struct mega_block_step_args {
+  int32_t dtype, batch, embed, zdim, hdim, ndim, complex_poles, positions;
+  const void* x;
+  void* out;
+  int64_t *count, *count_next;
+  float *mean, *var, *h;
+  const float *norm_gamma, *norm_beta, *p, *q, *gamma_hat, *omega;
+  const void *v_weight, *v_bias, *mx_weight, *mx_bias, *h_weight;
+  const float *qk_gamma, *qk_beta, *rot;
+  void *keys, *keys_rot, *values, *work;
+  double norm_eps, qk_eps;
+  int64_t cap;
+  int32_t pos;
+} mega_block_step_args;
+MEGA_API int64_t mega_block_step_work(int dtype, int batch, int embed, int zdim, int hdim, int64_t cap);
+MEGA_API int mega_block_step(const mega_block_step_args* args, mega_stream_t stream);
+MEGA_API int mega_block_cache_fill(const void* k, int64_t ksb, int64_t ksl, const void* v, int64_t vsb, int64_t vsl,
+                          const float* rot, int positions, int dtype, int batch, int n, int zdim, int hdim, void* keys,
+                          void* keys_rot, void* values, int64_t cap, mega_stream_t stream);
+
 #ifdef __cplusplus
 }
 #endif
