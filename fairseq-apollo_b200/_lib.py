@@ -73,6 +73,12 @@ SIGNATURES = {
                                            c_p],
     "mega_tsn_cema_fwd": [c_p, c_p, c_p, c_i, c_i, c_i, c_i, c_l, c_l, c_l, c_l, c_l, c_l, c_p, c_p, c_p,
                           c_p, c_p, c_d, c_p, c_p, c_p, c_p, c_p, c_p, c_p, c_i, c_p, c_p, c_p, c_u, c_p],
+    "mega_gate_silu_bwd": [c_p, c_l] * 3 + [c_p, c_i, c_l, c_i, c_p],
+    "mega_gate_mul_silu_bwd": [c_p, c_l] * 5 + [c_p, c_i, c_l, c_i, c_p],
+    "mega_gate_output_bwd": [c_p, c_l] * 8 + [c_p, c_p, c_i, c_l, c_i, c_p],
+    "mega_gate_qk_bwd": [c_p, c_l, c_p, c_p, c_i, c_i, c_i, c_p, c_l, c_p, c_l, c_p, c_l, c_p, c_p, c_p, c_i, c_l, c_i, c_d, c_p],
+    "mega_attention_bias_softmax_fwd": [c_p, c_p, c_p, c_i, c_p, c_i, c_l, c_i, c_i, c_p],
+    "mega_attention_bias_grad": [c_p, c_p, c_i, c_i, c_l, c_i, c_i, c_p],
     "mega_block_step": [c_p, c_p],
     "mega_block_cache_fill": [c_p, c_l, c_l, c_p, c_l, c_l, c_p, c_i, c_i, c_i, c_i, c_i, c_i, c_p, c_p, c_p, c_l, c_p],
     "mega_set_option": [c_i, c_i],

@@ -17,8 +17,9 @@ reference):
 * causal chunked softmax attention             ``EfficientAttention`` (scores GEMM, this library's
   causal softmax, values GEMM) when ``efficient_attn`` is set, else the reference's explicit path.
 
-Training (autograd enabled) takes the reference's own sequence of torch operations on top of the
-differentiable modules; the fused elementwise kernels are inference paths.
+Training without dropout runs everything behind the moving average as one autograd Function on the same kernels and
+their backward (``block_function``); with dropout, or in the branches it does not take, the reference's own sequence of
+torch operations runs on top of the differentiable modules.
 """
 import math
 from typing import Dict, Optional, Tuple
@@ -28,7 +29,7 @@ import torch.nn.functional as F
 from torch import Tensor, nn
 from torch.nn import Parameter
 
-from .. import ops
+from .. import block_function, ops
 from ..functions import needs_grad
 from ..incremental_state import IncrementalStateMixin
 from . import block_decode
@@ -276,6 +277,10 @@ class MovingAverageGatedAttention(IncrementalStateMixin, nn.Module):
                                        activation='silu' if silu_act else None, return_normed=True)
         if not silu_act:
             mx = self.move_act(mx)
+        if train and saved_state is None:
+            mode = block_function.mode_of(self, x, padding_mask, attn_mask, need_weights, before_attn_fn)
+            if mode is not None:
+                return block_function.run(self, mode, x, xn, mx, padding_mask), None
         mx = F.dropout(mx, self.hidden_dropout_p, self.training)
 
         # ---- projections and gates

@@ -422,6 +422,45 @@ def gate_qk_rotary(z, gamma, beta, rot, period, q_offset=0, eps=1e-5):
     return q, k
 
 
+def gate_silu_bwd(dy, a, da, colsum=None):
+    """da = dy * silu'(a) for row-major matrices (da may be dy); colsum (cols) fp32 gets da's column sums added."""
+    rows, cols = a.shape
+    with torch.cuda.device(a.device):
+        _lib.check(_lib.lib().mega_gate_silu_bwd(dy.data_ptr(), dy.stride(0), a.data_ptr(), a.stride(0), da.data_ptr(),
+                                                 da.stride(0), _ptr(colsum), _dt(a), rows, cols, _stream()), "gate_silu_bwd")
+
+
+def gate_mul_silu_bwd(dy, a, r, da, dr, colsum_r=None):
+    """Gradients of a * silu(r) into da (may be dy) and dr; colsum_r gets dr's column sums added."""
+    rows, cols = a.shape
+    with torch.cuda.device(a.device):
+        _lib.check(_lib.lib().mega_gate_mul_silu_bwd(
+            dy.data_ptr(), dy.stride(0), a.data_ptr(), a.stride(0), r.data_ptr(), r.stride(0), da.data_ptr(), da.stride(0),
+            dr.data_ptr(), dr.stride(0), _ptr(colsum_r), _dt(a), rows, cols, _stream()), "gate_mul_silu_bwd")
+
+
+def gate_output_bwd(dout, residual, u, hx, h_lin, dres, du, dhx, colsum_u=None, colsum_hx=None):
+    """Gradients of gate_output into dres, du and dhx (= that of h_lin), with column sums of the latter two."""
+    rows, cols = residual.shape
+    with torch.cuda.device(residual.device):
+        _lib.check(_lib.lib().mega_gate_output_bwd(
+            dout.data_ptr(), dout.stride(0), residual.data_ptr(), residual.stride(0), u.data_ptr(), u.stride(0),
+            hx.data_ptr(), hx.stride(0), h_lin.data_ptr(), h_lin.stride(0), dres.data_ptr(), dres.stride(0),
+            du.data_ptr(), du.stride(0), dhx.data_ptr(), dhx.stride(0), _ptr(colsum_u), _ptr(colsum_hx), _dt(residual),
+            rows, cols, _stream()), "gate_output_bwd")
+
+
+def gate_qk_bwd(z, gamma, rot, period, dq, dk, dz, dgamma, dbeta, colsum=None, eps=1e-5):
+    """Gradients of gate_qk (rot None) or gate_qk_rotary: dz, and dgamma, dbeta (2 S) fp32 added to."""
+    rows, cols = z.shape
+    g = _f32c(gamma)
+    with torch.cuda.device(z.device):
+        _lib.check(_lib.lib().mega_gate_qk_bwd(
+            z.data_ptr(), z.stride(0), g.data_ptr(), _ptr(rot), 0 if rot is None else rot.shape[0], int(period), 0,
+            dq.data_ptr(), dq.stride(0), dk.data_ptr(), dk.stride(0), dz.data_ptr(), dz.stride(0), dgamma.data_ptr(),
+            dbeta.data_ptr(), _ptr(colsum), _dt(z), rows, cols, float(eps), _stream()), "gate_qk_bwd")
+
+
 # ------------------------------------------------------------------------ training
 def _like(x):
     return torch.empty_strided(x.shape, x.stride(), dtype=x.dtype, device=x.device) \
@@ -750,3 +789,25 @@ def attention_softmax_bwd(dy, y, causal=True):
                                                          outer, inner, 1 if causal else 0, _stream()),
                    "attention_softmax_bwd")
     return dx
+
+
+def attention_bias_softmax_fwd(x, bias, padding_mask=None):
+    """softmax of scores x (batch, rows, cols) + bias[column - row + span - 1] over the last axis, without the columns
+    of padding_mask (batch, cols) uint8; bias (2 span - 1)."""
+    _cuda(x, bias, padding_mask)
+    xc = x.contiguous()
+    b = bias.to(xc.dtype).contiguous()
+    y = torch.empty_like(xc)
+    with torch.cuda.device(x.device):
+        _lib.check(_lib.lib().mega_attention_bias_softmax_fwd(
+            xc.data_ptr(), y.data_ptr(), b.data_ptr(), (b.shape[0] + 1) // 2, _ptr(padding_mask), _dt(xc), xc.shape[0],
+            xc.shape[1], xc.shape[2], _stream()), "attention_bias_softmax_fwd")
+    return y
+
+
+def attention_bias_grad(ds, dbias):
+    """Adds the sums of ds (batch, rows, cols) along its diagonals to dbias (2 span - 1) fp32."""
+    with torch.cuda.device(ds.device):
+        _lib.check(_lib.lib().mega_attention_bias_grad(ds.data_ptr(), dbias.data_ptr(), (dbias.shape[0] + 1) // 2, _dt(ds),
+                                                       ds.shape[0], ds.shape[1], ds.shape[2], _stream()),
+                   "attention_bias_grad")

@@ -502,6 +502,40 @@ MEGA_API int mega_attention_dropkey_softmax_fwd(const void* x, void* y, int dtyp
                                        mega_stream_t stream);
 
 /*
+ * Gradients of the gates (dy / dout: gradient of the result; operands as in the forward).  16-byte aligned operands,
+ * row pitches and column counts in whole 16-byte pieces (MEGA_ERR_ALIGN / MEGA_ERR_STRIDE).  colsum*: column sums of
+ * the gradient they are named after, ADDED to fp32 arrays of `cols` values (bias gradients of the projection that
+ * produced the operand), or NULL.  mega_gate_output_bwd: dhx is also the gradient of h_lin.
+ * mega_gate_qk_bwd: dq, dk in, dz out; dgamma, dbeta (2, cols) fp32 are added to; rot NULL: mega_gate_qk, else
+ * mega_gate_qk_rotary; cols <= 512.
+ * Replaces: the autograd of moving_average_gated_attention.py:308,322-330,407-412.
+ */
+MEGA_API int mega_gate_silu_bwd(const void* dy, int64_t ld_dy, const void* a, int64_t ld_a, void* da, int64_t ld_da,
+                       float* colsum, int dtype, int64_t rows, int cols, mega_stream_t stream);
+MEGA_API int mega_gate_mul_silu_bwd(const void* dy, int64_t ld_dy, const void* a, int64_t ld_a, const void* r, int64_t ld_r,
+                           void* da, int64_t ld_da, void* dr, int64_t ld_dr, float* colsum_r, int dtype,
+                           int64_t rows, int cols, mega_stream_t stream);
+MEGA_API int mega_gate_output_bwd(const void* dout, int64_t ld_do, const void* residual, int64_t ld_res, const void* u,
+                         int64_t ld_u, const void* hx, int64_t ld_hx, const void* h_lin, int64_t ld_h, void* dres,
+                         int64_t ld_dres, void* du, int64_t ld_du, void* dhx, int64_t ld_dhx, float* colsum_u,
+                         float* colsum_hx, int dtype, int64_t rows, int cols, mega_stream_t stream);
+MEGA_API int mega_gate_qk_bwd(const void* z, int64_t ld_z, const float* gamma, const float* rot, int positions, int period,
+                     int q_offset, const void* dq, int64_t ld_dq, const void* dk, int64_t ld_dk, void* dz,
+                     int64_t ld_dz, float* dgamma, float* dbeta, float* colsum, int dtype, int64_t rows, int cols,
+                     double eps, mega_stream_t stream);
+/*
+ * Softmax of scores x (batch, rows, cols) + bias[column - row + span - 1] with the columns of pad_mask (batch, cols)
+ * left out (a sequence that is padded throughout: no mask); bias (2 span - 1) in `dtype`; cols <= 49152.  Backward:
+ * mega_attention_softmax_bwd without the causal mask, and mega_attention_bias_grad, which ADDS the sums of ds along
+ * its diagonals to dbias (2 span - 1) fp32.
+ * Replaces: SimpleRelativePositionalBias + the softmax of moving_average_gated_attention.py:223-280.
+ */
+MEGA_API int mega_attention_bias_softmax_fwd(const void* x, void* y, const void* bias, int span, const uint8_t* pad_mask,
+                                    int dtype, int64_t batch, int rows, int cols, mega_stream_t stream);
+MEGA_API int mega_attention_bias_grad(const void* ds, float* dbias, int span, int dtype, int64_t batch, int rows, int cols,
+                             mega_stream_t stream);
+
+/*
  * ---- One decoding step of the causal Mega block ----------------------------------------------
  * For x (batch, embed) contiguous: the running state (count / mean / var / h as in mega_tsn_ema_step,
  * mega_tsn_cema_step with complex_poles; count -> count_next, two arrays), mx = SiLU(EMA(TimestepNorm(x))),
