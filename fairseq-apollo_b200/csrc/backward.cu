@@ -723,6 +723,14 @@ extern "C" int mega_sequence_norm_bwd(const void* dy, const void* x, void* dx, i
     MEGA_DISPATCH_DTYPE(dtype, launch(sqn_bwd_group_kernel<T>, (unsigned)((long long)B * G), 256, smem, stream, ga));
     return check_launch("sequence_norm_bwd(group)");
   }
+  {
+    ScanNormArgs na{};
+    na.x = x; na.y = dx; na.dy = dy; na.B = B; na.D = D; na.L = L;
+    na.xsb = xsb; na.xsl = xsl; na.ysb = dsb; na.ysl = dsl; na.gsb = gsb; na.gsl = gsl;
+    na.prev_count = a.count; na.prev_mean = mean; na.prev_var = rstd; na.gamma = gamma; na.mask = pad_mask;
+    na.dgamma = dgamma; na.dbeta = dbeta;
+    if (xsl != 1 && scan_sqn_bwd_try(dtype, na, xsd, dsd, gsd, s)) return check_launch("sequence_norm_bwd(scan)");
+  }
   MEGA_DISPATCH_DTYPE(dtype, launch(sqn_bwd_kernel<T>, (unsigned)((long long)B * D), 256, 0, stream, a));
   return check_launch("sequence_norm_bwd");
 }

@@ -1,0 +1,84 @@
+// TimestepNorm -> causal EMA in forms that are parallel over time (norm_ema_split.cuh).
+//
+// The fused kernels move every element once, but a sequence is one chain of steps to them: with few sequences and
+// channels they leave the SMs idle.  Two ways fill the SMs whatever the shape: the scan (scan_ema.cu), whose walks
+// normalise their inputs as they read them, and, for bf16, TimestepNorm by itself (scan_norm.cu) followed by the
+// tensor-core kernel alone, which runs in half the time of the fused one; the normalised activations then go to their
+// own output, or through y in place.
+#include "common.cuh"
+#include "norm_ema_split.cuh"
+#include "scan_ema.cuh"
+#include "scan_norm.cuh"
+
+namespace mega {
+
+namespace {
+
+// Times in us from a grid of shapes on one B200 (L in positions, n in elements): a chain costs so much per position
+// until the channels fill the device, then so much per element.
+double longer(double chain_ns, double per_us, double L, double n) {
+  const double a = L * chain_ns * 1e-3, b = n / per_us;
+  return a > b ? a : b;
+}
+
+bool mma_takes(int dtype, const StreamArgs& a, bool want_xn) {
+  const bool pipes = !want_xn && !a.cplx && a.mask == nullptr;   // forms pipelined along the sequence: any batch
+  return dtype == MEGA_BF16 && g_options[OPT_DISABLE_MMA].load() == 0 && !(a.mask && a.cplx) && (a.B >= 4 || pipes);
+}
+
+double fused_us(int dtype, const StreamArgs& a, bool want_xn) {
+  const double L = a.L, n = (double)a.B * a.D * a.L;
+  if (mma_takes(dtype, a, want_xn)) {
+    if (a.cplx) return longer(want_xn ? 75.0 : 62.0, want_xn ? 480e3 : 570e3, L, n);
+    return longer(want_xn ? 56.0 : a.mask ? 50.0 : 35.0, want_xn ? 700e3 : 820e3, L, n);
+  }
+  return a.cplx ? longer(240.0, 168e3, L, n) : longer(want_xn ? 190.0 : 130.0, want_xn ? 160e3 : 260e3, L, n);
+}
+
+// TimestepNorm, then the tensor-core kernel alone: where the fused call would run on it too (both round the normalised
+// activations to bf16), without a mask (that form gains little) and at lengths that it can stop at
+double mma_us(int dtype, const StreamArgs& a, bool want_xn) {
+  if (!mma_takes(dtype, a, want_xn) || a.mask || (a.h_out && a.L % 32 != 0)) return 1e30;
+  const double L = a.L, n = (double)a.B * a.D * a.L;
+  return 10.0 + n / 600e3 + (a.cplx ? longer(48.0, 600e3, L, n) : longer(24.0, 1300e3, L, n));
+}
+
+double scan_us(const StreamArgs& a, bool want_xn) {
+  const double n = (double)a.B * a.D * a.L;
+  return 20.0 + n / (a.cplx ? (want_xn ? 78e3 : 88e3) : (want_xn ? 145e3 : 165e3));
+}
+
+}  // namespace
+
+bool norm_ema_split_try(int dtype, const void* x, void* y, void* xn, long long xsb, long long xsl, long long xsd,
+                        long long ysb, long long ysl, long long ysd, const StreamArgs& a, cudaStream_t s) {
+  const int forced = g_options[OPT_SPLIT].load();
+  if (forced == 1 || g_options[OPT_DISABLE_STREAM].load() != 0 || g_options[OPT_DISABLE_MMA].load() != 0 ||
+      g_options[OPT_MMA_TILE].load() != 0)   // (a kernel asked for by name)
+    return false;
+  if (x == y || xn == y || xn == x || a.N < 1 || a.N > 16 || a.count_offset != 0) return false;
+  const double fused = fused_us(dtype, a, xn != nullptr), scan = scan_us(a, xn != nullptr), mma = mma_us(dtype, a, xn != nullptr);
+  // (the margin: two to four more launches, on a host that is not ahead of the device)
+  if (forced == 0 && (scan < mma ? scan : mma) + 25.0 > fused) return false;
+  if (mma < scan && forced != 3) {
+    void* mid = xn ? xn : y;
+    ScanNormArgs na{};
+    na.x = x; na.y = mid; na.B = a.B; na.D = a.D; na.L = a.L;
+    na.xsb = xsb; na.xsl = xsl; na.ysb = ysb; na.ysl = ysl;
+    na.prev_count = a.prev_count; na.prev_mean = a.prev_mean; na.prev_var = a.prev_var; na.gamma = a.gamma;
+    na.beta = a.beta; na.eps = a.eps; na.count_out = a.count_out; na.mean_out = a.mean_out; na.var_out = a.var_out;
+    if (scan_norm_fwd_try(dtype, na, xsd, ysd, s) &&
+        mma_cl_try(dtype, mid, y, nullptr, ysb, ysl, ysd, ysb, ysl, ysd, false, a, s))
+      return true;   // (were the second one refused, the next form starts from x again)
+  }
+  ScanArgs ea{};
+  ea.x = x; ea.y = y; ea.xn = xn; ea.B = a.B; ea.D = a.D; ea.L = a.L; ea.N = a.N;
+  ea.xsb = xsb; ea.xsl = xsl; ea.ysb = ysb; ea.ysl = ysl;
+  ea.p = a.p; ea.q = a.q; ea.g = a.g; ea.omega = a.omega; ea.mask = a.mask; ea.h_in = a.h_in; ea.h_out = a.h_out;
+  ea.cplx = a.cplx; ea.silu = a.silu;
+  ea.prev_count = a.prev_count; ea.prev_mean = a.prev_mean; ea.prev_var = a.prev_var; ea.gamma = a.gamma; ea.beta = a.beta;
+  ea.eps = a.eps; ea.count_out = a.count_out; ea.mean_out = a.mean_out; ea.var_out = a.var_out;
+  return scan_ema_fwd_try(dtype, ea, xsd, ysd, s);
+}
+
+}  // namespace mega

@@ -565,6 +565,14 @@ extern "C" int mega_sequence_norm_fwd(const void* x, void* y, int dtype, int B, 
   a.xsb = xsb; a.xsd = xsd; a.xsl = xsl; a.ysb = ysb; a.ysd = ysd; a.ysl = ysl;
   a.gamma = gamma; a.beta = beta; a.mask = pad_mask; a.eps = (float)eps;
   a.count_out = (long long*)count_out; a.mean_out = mean_out; a.rstd_out = rstd_out;
+  if (G == D && xsd == 1 && xsl != 1 && x != y) {
+    ScanNormArgs na{};
+    na.x = x; na.y = y; na.B = B; na.D = D; na.L = L;
+    na.xsb = xsb; na.xsl = xsl; na.ysb = ysb; na.ysl = ysl;
+    na.gamma = gamma; na.beta = beta; na.mask = pad_mask; na.eps = (float)eps;
+    na.count_out = a.count_out; na.mean_out = mean_out; na.var_out = rstd_out;
+    if (scan_sqn_fwd_try(dtype, na, xsd, ysd, (cudaStream_t)stream)) return check_launch("sequence_norm_fwd(scan)");
+  }
   if (G == D && xsd == 1 && xsl != 1) {
     const unsigned grid = (unsigned)(((long long)B * D + 127) / 128);
     MEGA_DISPATCH_DTYPE(dtype, launch(sqn_column_kernel<T>, grid, 128, 0, stream, a));

@@ -11,6 +11,9 @@
 // Bound: the FMA pipe, when segments x channels fill the SMs; a sequence walked as one chain is bound by its
 // own latency instead (B = 8, L = 1024, D = 512 fp32: 103 us as 128 chains of 1024 steps).
 //
+// TimestepNorm in front (norm_run.cuh): two small launches give every segment the statistics it starts from, and the
+// walks normalise their inputs as they read them, in fp32, so nothing but x is read and nothing but y written.
+//
 // Backward.  With h the states for unit input gain, s = dh/dq and lambda the adjoint scaled by 1 / (p g):
 //   h_t = q h_{t-1} + x~_t,  s_t = q s_{t-1} + h_{t-1},  lambda_t = q lambda_{t+1} + dy_t,
 //   dx~_t = sum_n p g lambda_t,  dg = p sum dy h,  dp = g sum dy h,  dq = p g sum dy s,
@@ -19,6 +22,7 @@
 #include <cmath>
 
 #include "common.cuh"
+#include "norm_run.cuh"
 #include "scan_ema.cuh"
 #include "scratch.cuh"
 #include "tma.cuh"
@@ -34,6 +38,7 @@ struct SegArgs {
   ScanArgs a;
   int T, S;          // steps per segment, segments
   int wide;          // one segment: the warps of a block own adjacent channel groups instead of segments
+  float *rn, *rm, *rs;   // TimestepNorm in front: what every segment starts from (count; mean, squared deviations)
   int parts;         // values per (batch, direction, segment, pole, channel) in the carry array
   float* carry;      // [B][dirs][S][parts][16][D]
 };
@@ -228,10 +233,64 @@ __device__ __forceinline__ Lane lane_of(const SegArgs& s) {
   return l;
 }
 
+// ---- TimestepNorm in front --------------------------------------------------------------------------
+// Moments of the segments -> what each segment starts from, and the statistics after the last.
+__global__ void __launch_bounds__(128) scan_stats_kernel(SegArgs s) {
+  const ScanArgs& a = s.a;
+  const int d = blockIdx.x * 128 + threadIdx.x, b = blockIdx.y;
+  const long long cnt0 = a.prev_count[b];
+  const float n0 = (float)cnt0;
+  const bool ok = d < a.D;
+  const size_t i = (size_t)b * a.D + (ok ? d : 0);
+  Run r{n0, a.prev_mean[i], a.prev_var[i] * n0};
+  const float* pn = s.rn + (size_t)b * s.S;
+  float *pm = s.rm + (size_t)b * s.S * a.D + (ok ? d : 0), *ps = s.rs + (size_t)b * s.S * a.D + (ok ? d : 0);
+  constexpr int kB = 8;
+  for (int k0 = 0; k0 < s.S; k0 += kB) {
+    Run seg[kB];
+#pragma unroll
+    for (int u = 0; u < kB; ++u) {
+      const int k = min(k0 + u, s.S - 1);
+      seg[u] = Run{__ldg(pn + k), __ldcg(pm + (size_t)k * a.D), __ldcg(ps + (size_t)k * a.D)};
+    }
+#pragma unroll
+    for (int u = 0; u < kB; ++u) {
+      if (k0 + u < s.S) {
+        if (ok) {
+          pm[(size_t)(k0 + u) * a.D] = r.m;
+          ps[(size_t)(k0 + u) * a.D] = r.s;
+        }
+        r = combine(r, seg[u]);
+      }
+    }
+  }
+  if (ok) {
+    a.mean_out[i] = r.n > 0.f ? r.m : a.prev_mean[i];
+    a.var_out[i] = r.n > 0.f ? r.s / r.n : a.prev_var[i];
+    if (d == 0) a.count_out[b] = cnt0 + (long long)(r.n - n0 + 0.5f);
+  }
+}
+
+// The statistics a segment starts from.
+__device__ __forceinline__ Run stats_of(const SegArgs& s, int b, int seg, int d) {
+  float n = (float)s.a.prev_count[b];
+  for (int k = 0; k < seg; ++k) n += __ldg(s.rn + (size_t)b * s.S + k);
+  const size_t i = ((size_t)b * s.S + seg) * s.a.D + d;
+  return Run{n, __ldg(s.rm + i), __ldg(s.rs + i)};
+}
+// the normalised input (0 at a padded position)
+__device__ __forceinline__ float normed(Running& st, float x, bool pad, float w, float bb, float eps) {
+  if (pad) return 0.f;
+  float inv, r;
+  const float d = st.step(x, eps, inv, r);
+  return fmaf((d - st.u) * r, w, bb);
+}
+
 // ---- (1) local states ---------------------------------------------------------------------------
 // forward: h of each direction.  backward: (h, s) of each direction and the adjoint, which runs the other way.
-template <typename T, bool kC, bool kMask, bool kBwd>
+template <typename T, bool kC, bool kMask, bool kBwd, bool kNorm = false>
 __global__ void __launch_bounds__(kWarps * 32) scan_local_kernel(SegArgs s) {
+  static_assert(!kNorm || !kBwd, "the norm in front is a forward form");
   const ScanArgs& a = s.a;
   const int dirs = a.bidir ? 2 : 1;
   SegArgs ss = s;
@@ -265,6 +324,14 @@ __global__ void __launch_bounds__(kWarps * 32) scan_local_kernel(SegArgs s) {
     if (dir == 0) walk<T, -1, false, false>(g, a.gsl, g, 0, m, l.t0, l.t1, l.left, ring, adj);
     else walk<T, 1, false, false>(g, a.gsl, g, 0, m, l.t0, l.t1, l.left, ring, adj);
     store_state<kC>(h, carry_at(s, l.b, dir, l.seg, 2 * kOne, l.dc), a.D, l.ok);
+  } else if constexpr (kNorm) {
+    Running st;
+    st.start(stats_of(s, l.b, l.seg, l.dc));
+    const float w = __ldg(a.gamma + l.dc), bb = __ldg(a.beta + l.dc), eps = a.eps;
+    walk<T, 1, false, kMask>(x, a.xsl, x, 0, m, l.t0, l.t1, l.left, ring, [&](int, float xv, float, bool pad) {
+      advance<kC>(h, P, splat(normed(st, xv, kMask && pad, w, bb, eps)));
+    });
+    store_state<kC>(h, carry_at(s, l.b, dir, l.seg, 0, l.dc), a.D, l.ok);
   } else {
     auto step = [&](int, float xv, float, bool pad) { advance<kC>(h, P, splat(kMask && pad ? 0.f : xv)); };
     if (dir == 0) walk<T, 1, false, kMask>(x, a.xsl, x, 0, m, l.t0, l.t1, l.left, ring, step);
@@ -407,8 +474,8 @@ __global__ void __launch_bounds__(128) scan_carry_kernel(SegArgs s, int gain) {
 }
 
 // ---- (3) outputs -----------------------------------------------------------------------------------
-template <typename T, bool kC, bool kMask, bool kState>
-__global__ void __launch_bounds__(kWarps * 32, kC ? 3 : 4) scan_emit_kernel(SegArgs s) {
+template <typename T, bool kC, bool kMask, bool kState, bool kNorm = false>
+__global__ void __launch_bounds__(kWarps * 32, kC || kNorm ? 3 : 4) scan_emit_kernel(SegArgs s) {
   const ScanArgs& a = s.a;
   const Lane l = lane_of(s);
   if (l.seg >= s.S) return;
@@ -473,7 +540,26 @@ __global__ void __launch_bounds__(kWarps * 32, kC ? 3 : 4) scan_emit_kernel(SegA
     return;
   }
   T* py = y + (long long)l.t0 * a.ysl;
-  walk<T, 1, false, kMask>(x, a.xsl, x, 0, m, l.t0, l.t1, l.left, ring, [&](int k, float xv, float, bool pad) {
+  if constexpr (kNorm) {
+    Running st;
+    st.start(stats_of(s, l.b, l.seg, l.dc));
+    const float w = __ldg(a.gamma + l.dc), bb = __ldg(a.beta + l.dc), eps = a.eps;
+    T* pn = a.xn ? reinterpret_cast<T*>(a.xn) + (py - reinterpret_cast<T*>(a.y)) : nullptr;   // (strided like y)
+    walk<T, 1, false, kMask>(x, a.xsl, x, 0, m, l.t0, l.t1, l.left, ring, [&](int, float xv, float, bool pad) {
+      const float xn = normed(st, xv, kMask && pad, w, bb, eps);
+      const f32x2 x2 = splat(xn);
+      if constexpr (kState) advance_gain<kC>(h, P, p, x2);
+      else advance<kC>(h, P, x2);
+      float v = fmaf(om, xn, dot<kC>(c, h));
+      if (a.silu) v = siluf_(v);
+      if (l.ok) Elem<T>::st(py, v);
+      py += a.ysl;
+      if (pn) {
+        if (l.ok) Elem<T>::st(pn, xn);
+        pn += a.ysl;
+      }
+    });
+  } else walk<T, 1, false, kMask>(x, a.xsl, x, 0, m, l.t0, l.t1, l.left, ring, [&](int k, float xv, float, bool pad) {
     const f32x2 x2 = splat(kMask && pad ? 0.f : xv);
     if constexpr (kState) advance_gain<kC>(h, P, p, x2);
     else advance<kC>(h, P, x2);
@@ -675,7 +761,7 @@ static void pick_segments(const ScanArgs& a, int resident, bool bwd, SegArgs& s)
   const double slots = 148.0 * resident;
   double best = 1e30;
   s.wide = 0;
-  if (!a.bidir && !bwd) {
+  if (!a.bidir && !bwd && !a.prev_count) {
     s.T = a.L;
     s.S = 1;
     s.wide = 1;
@@ -700,7 +786,7 @@ static void pick_segments(const ScanArgs& a, int resident, bool bwd, SegArgs& s)
   }
 }
 
-template <typename T, bool kC, bool kMask>
+template <typename T, bool kC, bool kMask, bool kNorm>
 static bool fwd_launch(const SegArgs& s, cudaStream_t st) {
   const ScanArgs& a = s.a;
   const int dirs = a.bidir ? 2 : 1;
@@ -708,13 +794,18 @@ static bool fwd_launch(const SegArgs& s, cudaStream_t st) {
   const dim3 grid(s.wide ? (a.D + 32 * kWarps - 1) / (32 * kWarps) : (a.D + 31) / 32, (s.S + kWarps - 1) / kWarps, a.B);
   const bool state = a.h_in || a.h_out;
   const size_t rings = (size_t)kWarps * kRing * kTileBytes;
+  if (kNorm) {
+    const MomentArgs m{a.x, a.xsb, a.xsl, a.mask, a.L, a.D, s.T, s.S, s.rn, s.rm, s.rs};
+    launch(norm_moments_kernel<T, kMask>, grid, block, rings, (void*)st, m);
+    launch(scan_stats_kernel, dim3((a.D + 127) / 128, a.B), 128, 0, (void*)st, s);
+  }
   if (s.carry) {
-    launch(scan_local_kernel<T, kC, kMask, false>, dim3(grid.x, grid.y, a.B * dirs), block, rings, (void*)st, s);
+    launch(scan_local_kernel<T, kC, kMask, false, kNorm>, dim3(grid.x, grid.y, a.B * dirs), block, rings, (void*)st, s);
     launch(scan_carry_kernel<kC, false>, dim3((a.D + 127) / 128, 16, a.B * dirs), 128, 0, (void*)st, s, state ? 1 : 0);
   }
   const size_t smem = rings + (a.bidir ? (size_t)kWarps * s.T * 32 * 4 : 0);
-  if (state) launch(scan_emit_kernel<T, kC, kMask, true>, grid, block, smem, (void*)st, s);
-  else launch(scan_emit_kernel<T, kC, kMask, false>, grid, block, smem, (void*)st, s);
+  if (state) launch(scan_emit_kernel<T, kC, kMask, true, kNorm>, grid, block, smem, (void*)st, s);
+  else launch(scan_emit_kernel<T, kC, kMask, false, kNorm>, grid, block, smem, (void*)st, s);
   return true;
 }
 
@@ -742,18 +833,26 @@ static bool dispatch(int dtype, const ScanArgs& a, cudaStream_t st) {
   SegArgs s{};
   s.a = a;
   // blocks per SM by registers
-  pick_segments(a, kBwd ? (a.cplx ? 2 : 3) : (a.cplx ? 3 : 4), kBwd, s);
+  pick_segments(a, kBwd ? (a.cplx ? 2 : 3) : (a.cplx || a.prev_count ? 3 : 4), kBwd, s);
   if ((s.S + kWarps - 1) / kWarps > 65535) return false;
   s.parts = (kBwd ? 3 : 1) * (a.cplx ? 2 : 1);
   const size_t floats = (!s.wide) ? (size_t)a.B * dirs * s.S * s.parts * 16 * a.D : 0;
-  Scratch sc(floats ? Scratch::padded(floats * 4) : 256, st);
+  const bool norm = !kBwd && a.prev_count != nullptr;
+  const size_t stats = norm ? (size_t)a.B * s.S * a.D : 0;
+  Scratch sc(Scratch::padded(floats * 4) + 2 * Scratch::padded(stats * 4) + Scratch::padded((size_t)a.B * s.S * 4), st);
   if (!sc) return false;
+  if (norm) {
+    s.rn = sc.take<float>((size_t)a.B * s.S);
+    s.rm = sc.take<float>(stats);
+    s.rs = sc.take<float>(stats);
+  }
   s.carry = floats ? sc.take<float>(floats) : nullptr;
-#define MEGA_SCAN(TY)                                                                                           \
-  (a.cplx ? (a.mask ? (kBwd ? bwd_launch<TY, true, true>(s, st) : fwd_launch<TY, true, true>(s, st))             \
-                    : (kBwd ? bwd_launch<TY, true, false>(s, st) : fwd_launch<TY, true, false>(s, st)))          \
-          : (a.mask ? (kBwd ? bwd_launch<TY, false, true>(s, st) : fwd_launch<TY, false, true>(s, st))           \
-                    : (kBwd ? bwd_launch<TY, false, false>(s, st) : fwd_launch<TY, false, false>(s, st))))
+#define MEGA_SCAN_FORM(TY, CPLX, MASK)                                             \
+  (kBwd ? bwd_launch<TY, CPLX, MASK>(s, st)                                        \
+        : norm ? fwd_launch<TY, CPLX, MASK, true>(s, st) : fwd_launch<TY, CPLX, MASK, false>(s, st))
+#define MEGA_SCAN(TY)                                                              \
+  (a.cplx ? (a.mask ? MEGA_SCAN_FORM(TY, true, true) : MEGA_SCAN_FORM(TY, true, false)) \
+          : (a.mask ? MEGA_SCAN_FORM(TY, false, true) : MEGA_SCAN_FORM(TY, false, false)))
   switch (dtype) {
     case MEGA_F32: return MEGA_SCAN(float);
     case MEGA_BF16: return MEGA_SCAN(__nv_bfloat16);
@@ -761,12 +860,18 @@ static bool dispatch(int dtype, const ScanArgs& a, cudaStream_t st) {
     default: return false;
   }
 #undef MEGA_SCAN
+#undef MEGA_SCAN_FORM
 }
 
 }  // namespace
 
+bool scan_ema_fwd_ok(int dtype, const ScanArgs& a, long long xsd, long long ysd) {
+  return g_options[OPT_DISABLE_STREAM].load() == 0 && rows_ok(dtype, a.x, a.xsb, a.xsl, xsd, a.D) && ysd == 1 && a.N <= 16 &&
+         (long long)a.B * (a.bidir ? 2 : 1) <= 65535 && (a.x != a.y || (a.xsb == a.ysb && a.xsl == a.ysl));
+}
+
 bool scan_ema_fwd_try(int dtype, const ScanArgs& a, long long xsd, long long ysd, cudaStream_t s) {
-  if (!rows_ok(dtype, a.x, a.xsb, a.xsl, xsd, a.D) || ysd != 1 || a.x == a.y) return false;
+  if (!scan_ema_fwd_ok(dtype, a, xsd, ysd)) return false;
   return dispatch<false>(dtype, a, s);
 }
 

@@ -1,4 +1,5 @@
-// Per-feature TimestepNorm and its backward, parallel over time (channels contiguous, any activation type).
+// Per-feature TimestepNorm and SequenceNorm with their backward, parallel over time (channels contiguous, any
+// activation type).
 //
 // The running statistics are counts, means and squared deviations, which combine associatively, so the sequence
 // is cut into segments: (1) the moments of every segment; (2) every segment combines those of the segments
@@ -13,10 +14,12 @@
 // Bound: the issue slots, about 20 instructions per element and pass forward and 30 backward; HBM moves x twice
 // and y once forward, x three times, dy twice and dx once backward.  B = 16, L = 4096, D = 1024, bf16: the
 // walk of whole sequences (16384 chains of 4096 steps, statistics of every step saved in fp32) took 370 us
-// forward and 365 us backward.
+// forward and 365 us backward.  SequenceNorm needs the moments of the whole sequence only (B = 16, L = 1024, D = 256
+// bf16: 403 us as one thread per column, its backward 99 us as one strided block per column).
 #include <cmath>
 
 #include "common.cuh"
+#include "norm_run.cuh"
 #include "scan_norm.cuh"
 #include "scratch.cuh"
 #include "walk.cuh"
@@ -33,15 +36,8 @@ struct SegNorm {
   float *sv, *su, *sw;     // [B][S][D] backward: the segment's map
 };
 
-struct Run {
-  float n, m, s;
-};
-__device__ __forceinline__ Run combine(Run a, Run b) {
-  const float n = a.n + b.n;
-  if (b.n == 0.f) return a;
-  if (a.n == 0.f) return b;
-  const float w = b.n * rcp_approx(n), d = b.m - a.m;
-  return {n, fmaf(d, w, a.m), a.s + b.s + d * d * a.n * w};
+static MomentArgs moments_of(const SegNorm& s) {
+  return {s.a.x, s.a.xsb, s.a.xsl, s.a.mask, s.a.L, s.a.D, s.T, s.S, s.rn, s.rm, s.rs};
 }
 
 struct NormLane {
@@ -77,66 +73,6 @@ __device__ __forceinline__ Run run_before(const SegNorm& s, const NormLane& l) {
     r = combine(r, Run{__ldg(pn + k), __ldg(pm + (size_t)k * s.a.D), __ldg(ps + (size_t)k * s.a.D)});
   return r;
 }
-
-template <typename T, bool kMask>
-__global__ void __launch_bounds__(kWarps * 32) norm_moments_kernel(SegNorm s) {
-  extern __shared__ __align__(16) unsigned char rings[];
-  const ScanNormArgs& a = s.a;
-  const NormLane l = norm_lane(s);
-  if (!l.active) return;
-  const T* x = reinterpret_cast<const T*>(a.x) + l.b * a.xsb + l.d0;
-  const unsigned char* m = kMask ? a.mask + (size_t)l.b * a.L : nullptr;
-  float c = 0.f, s1 = 0.f, s2 = 0.f, n = 0.f;
-  walk<T, 1, false, kMask>(x, a.xsl, x, 0, m, l.t0, l.t1, l.left, rings + (size_t)l.warp * kRing * kTileBytes,
-                           [&](int k, float xv, float, bool pad) {
-                             if (kMask) {
-                               if (!pad) {
-                                 if (n == 0.f) c = xv;
-                                 const float d = xv - c;
-                                 s1 += d;
-                                 s2 = fmaf(d, d, s2);
-                                 n += 1.f;
-                               }
-                             } else {
-                               if (k == 0) c = xv;
-                               const float d = xv - c;
-                               s1 += d;
-                               s2 = fmaf(d, d, s2);
-                             }
-                           });
-  if (!kMask) n = (float)(l.t1 - l.t0);
-  const float inv = n > 0.f ? 1.f / n : 0.f;
-  const size_t i = ((size_t)l.b * s.S + l.seg) * a.D + l.d;
-  if (l.ok) {
-    s.rm[i] = fmaf(s1, inv, c);
-    s.rs[i] = fmaxf(fmaf(-s1 * inv, s1, s2), 0.f);
-  }
-  if (blockIdx.x == 0 && l.lane == 0) s.rn[(size_t)l.b * s.S + l.seg] = n;
-}
-
-// The statistics of a walk, advanced by one unmasked input.
-struct Running {
-  float c, s1, s2, n, in_s;   // centre, sums about it, count, squared deviations that came in
-  float u;                    // mean - c
-  __device__ __forceinline__ void start(const Run& r) {
-    c = r.m;
-    s1 = s2 = u = 0.f;
-    n = r.n;
-    in_s = r.s;
-  }
-  // returns x - c; inv = 1 / n, r = 1 / sqrt(var + eps)
-  __device__ __forceinline__ float step(float x, float eps, float& inv, float& r) {
-    if (n == 0.f) c = x;
-    const float d = x - c;
-    s1 += d;
-    s2 = fmaf(d, d, s2);
-    n += 1.f;
-    inv = rcp_approx(n);
-    u = s1 * inv;
-    r = rsqrt_approx(fmaxf(fmaf(-u, u, (in_s + s2) * inv), 0.f) + eps);
-    return d;
-  }
-};
 
 template <typename T, bool kMask>
 __global__ void __launch_bounds__(kWarps * 32) norm_emit_kernel(SegNorm s) {
@@ -277,6 +213,95 @@ __global__ void __launch_bounds__(kWarps * 32) norm_bwd_emit_kernel(SegNorm s) {
                           });
 }
 
+// ---- SequenceNorm, per channel -----------------------------------------------------------------
+// The moments of the whole sequence: those of every segment (norm_moments_kernel), combined by each block.
+template <typename T, bool kMask>
+__global__ void __launch_bounds__(kWarps * 32) sqn_emit_kernel(SegNorm s) {
+  extern __shared__ __align__(16) unsigned char rings[];
+  const ScanNormArgs& a = s.a;
+  const NormLane l = norm_lane(s);
+  if (!l.active) return;
+  Run r{0.f, 0.f, 0.f};
+  const float* pn = s.rn + (size_t)l.b * s.S;
+  const float *pm = s.rm + (size_t)l.b * s.S * a.D + l.dc, *ps = s.rs + (size_t)l.b * s.S * a.D + l.dc;
+#pragma unroll 4
+  for (int k = 0; k < s.S; ++k) r = combine(r, Run{__ldg(pn + k), __ldg(pm + (size_t)k * a.D), __ldg(ps + (size_t)k * a.D)});
+  const float rstd = rsqrtf((r.n > 0.f ? r.s / r.n : 0.f) + a.eps), mean = r.m;
+  if (l.seg == 0 && l.ok) {
+    a.mean_out[(size_t)l.b * a.D + l.d] = mean;
+    a.var_out[(size_t)l.b * a.D + l.d] = rstd;
+    if (l.d == 0) a.count_out[l.b] = (long long)(r.n + 0.5f);
+  }
+  const T* x = reinterpret_cast<const T*>(a.x) + l.b * a.xsb + l.d0;
+  T* py = reinterpret_cast<T*>(a.y) + l.b * a.ysb + (long long)l.t0 * a.ysl + l.dc;
+  const unsigned char* m = kMask ? a.mask + (size_t)l.b * a.L : nullptr;
+  const float w = __ldg(a.gamma + l.dc), bb = __ldg(a.beta + l.dc);
+  walk<T, 1, false, kMask>(x, a.xsl, x, 0, m, l.t0, l.t1, l.left, rings + (size_t)l.warp * kRing * kTileBytes,
+                           [&](int, float xv, float, bool pad) {
+                             if (l.ok) Elem<T>::st(py, kMask && pad ? 0.f : fmaf((xv - mean) * rstd, w, bb));
+                             py += a.ysl;
+                           });
+}
+
+// Backward: every segment's sums of dy and dy (x - mean) ...
+template <typename T, bool kMask>
+__global__ void __launch_bounds__(kWarps * 32) sqn_bwd_sums_kernel(SegNorm s) {
+  extern __shared__ __align__(16) unsigned char rings[];
+  const ScanNormArgs& a = s.a;
+  const NormLane l = norm_lane(s);
+  if (!l.active) return;
+  const T* x = reinterpret_cast<const T*>(a.x) + l.b * a.xsb + l.d0;
+  const T* g = reinterpret_cast<const T*>(a.dy) + l.b * a.gsb + l.d0;
+  const unsigned char* m = kMask ? a.mask + (size_t)l.b * a.L : nullptr;
+  const float u = a.prev_mean[(size_t)l.b * a.D + l.dc];
+  float ds = 0.f, db = 0.f;
+  walk<T, 1, true, kMask>(x, a.xsl, g, a.gsl, m, l.t0, l.t1, l.left, rings + (size_t)l.warp * 2 * kRing * kTileBytes,
+                          [&](int, float xv, float gv, bool pad) {
+                            const float v = kMask && pad ? 0.f : gv;
+                            ds = fmaf(v, xv - u, ds);
+                            db += v;
+                          });
+  if (l.ok) {
+    const size_t i = ((size_t)l.b * s.S + l.seg) * a.D + l.d;
+    s.rm[i] = ds;
+    s.rs[i] = db;
+  }
+}
+
+// ... and the input gradient from their totals (fairseq/csrc/ops/sequence_norm.cc:374-529).
+template <typename T, bool kMask>
+__global__ void __launch_bounds__(kWarps * 32) sqn_bwd_emit_kernel(SegNorm s) {
+  extern __shared__ __align__(16) unsigned char rings[];
+  const ScanNormArgs& a = s.a;
+  const NormLane l = norm_lane(s);
+  if (!l.active) return;
+  const float *pm = s.rm + (size_t)l.b * s.S * a.D + l.dc, *ps = s.rs + (size_t)l.b * s.S * a.D + l.dc;
+  float ds = 0.f, db = 0.f;
+#pragma unroll 4
+  for (int k = 0; k < s.S; ++k) {
+    ds += __ldg(pm + (size_t)k * a.D);
+    db += __ldg(ps + (size_t)k * a.D);
+  }
+  const size_t row = (size_t)l.b * a.D + l.dc;
+  const float u = a.prev_mean[row], r = a.prev_var[row], w = __ldg(a.gamma + l.dc);   // (mean and rstd of the forward)
+  const long long cnt = a.prev_count[l.b];
+  const float coef = cnt > 0 ? 1.f / (float)cnt : 0.f;
+  if (l.seg == 0 && l.ok) {
+    atomicAdd(a.dgamma + l.d, r * ds);
+    atomicAdd(a.dbeta + l.d, db);
+  }
+  const float rw = r * w, kv = -coef * (r * r * rw) * ds, ku = -coef * rw * db;
+  const T* x = reinterpret_cast<const T*>(a.x) + l.b * a.xsb + l.d0;
+  const T* g = reinterpret_cast<const T*>(a.dy) + l.b * a.gsb + l.d0;
+  T* pd = reinterpret_cast<T*>(a.y) + l.b * a.ysb + (long long)l.t0 * a.ysl + l.dc;
+  const unsigned char* m = kMask ? a.mask + (size_t)l.b * a.L : nullptr;
+  walk<T, 1, true, kMask>(x, a.xsl, g, a.gsl, m, l.t0, l.t1, l.left, rings + (size_t)l.warp * 2 * kRing * kTileBytes,
+                          [&](int, float xv, float gv, bool pad) {
+                            if (l.ok) Elem<T>::st(pd, kMask && pad ? 0.f : fmaf(rw, gv, fmaf(kv, xv - u, ku)));
+                            pd += a.ysl;
+                          });
+}
+
 // Segments: enough blocks of four for the SMs (about six of them resident each) in few rounds, at least 64 steps
 // each and at most 64 of them, since every segment combines those before it.
 static void pick_segments(const ScanNormArgs& a, int resident, SegNorm& s) {
@@ -301,16 +326,53 @@ template <typename T, bool kMask>
 static void fwd_launch(const SegNorm& s, cudaStream_t st) {
   const dim3 grid((s.a.D + 31) / 32, (s.S + kWarps - 1) / kWarps, s.a.B), block(kWarps * 32);
   const size_t rings = (size_t)kWarps * kRing * kTileBytes;
-  launch(norm_moments_kernel<T, kMask>, grid, block, rings, (void*)st, s);
+  launch(norm_moments_kernel<T, kMask>, grid, block, rings, (void*)st, moments_of(s));
   launch(norm_emit_kernel<T, kMask>, grid, block, rings, (void*)st, s);
 }
 template <typename T, bool kMask>
 static void bwd_launch(const SegNorm& s, cudaStream_t st) {
   const dim3 grid((s.a.D + 31) / 32, (s.S + kWarps - 1) / kWarps, s.a.B), block(kWarps * 32);
   const size_t rings = (size_t)kWarps * kRing * kTileBytes;
-  launch(norm_moments_kernel<T, kMask>, grid, block, rings, (void*)st, s);
+  launch(norm_moments_kernel<T, kMask>, grid, block, rings, (void*)st, moments_of(s));
   launch(norm_bwd_map_kernel<T, kMask>, grid, block, 2 * rings, (void*)st, s);
   launch(norm_bwd_emit_kernel<T, kMask>, grid, block, 2 * rings, (void*)st, s);
+}
+
+template <typename T, bool kMask>
+static void sqn_launch(const SegNorm& s, bool bwd, cudaStream_t st) {
+  const dim3 grid((s.a.D + 31) / 32, (s.S + kWarps - 1) / kWarps, s.a.B), block(kWarps * 32);
+  const size_t rings = (size_t)kWarps * kRing * kTileBytes;
+  if (bwd) {
+    launch(sqn_bwd_sums_kernel<T, kMask>, grid, block, 2 * rings, (void*)st, s);
+    launch(sqn_bwd_emit_kernel<T, kMask>, grid, block, 2 * rings, (void*)st, s);
+  } else {
+    launch(norm_moments_kernel<T, kMask>, grid, block, rings, (void*)st, moments_of(s));
+    launch(sqn_emit_kernel<T, kMask>, grid, block, rings, (void*)st, s);
+  }
+}
+
+static bool sqn_dispatch(int dtype, const ScanNormArgs& a, bool bwd, cudaStream_t st) {
+  if (g_options[OPT_DISABLE_STREAM].load() != 0 || a.B > 65535) return false;
+  SegNorm s{};
+  s.a = a;
+  pick_segments(a, bwd ? 3 : 6, s);
+  const size_t n = (size_t)a.B * s.S * a.D;
+  Scratch sc(Scratch::padded(n * 4) * 2 + Scratch::padded((size_t)a.B * s.S * 4), st);
+  if (!sc) return false;
+  s.rn = sc.take<float>((size_t)a.B * s.S);
+  s.rm = sc.take<float>(n);
+  s.rs = sc.take<float>(n);
+#define MEGA_SCAN_SQN(TY)                          \
+  if (a.mask) sqn_launch<TY, true>(s, bwd, st);    \
+  else sqn_launch<TY, false>(s, bwd, st);          \
+  return true
+  switch (dtype) {
+    case MEGA_F32: MEGA_SCAN_SQN(float);
+    case MEGA_BF16: MEGA_SCAN_SQN(__nv_bfloat16);
+    case MEGA_F16: MEGA_SCAN_SQN(__half);
+    default: return false;
+  }
+#undef MEGA_SCAN_SQN
 }
 
 template <bool kBwd>
@@ -360,6 +422,18 @@ bool scan_norm_bwd_try(int dtype, const ScanNormArgs& a, long long xsd, long lon
       a.y == a.x || a.y == a.dy)
     return false;
   return dispatch<true>(dtype, a, s);
+}
+
+bool scan_sqn_fwd_try(int dtype, const ScanNormArgs& a, long long xsd, long long ysd, cudaStream_t s) {
+  if (!rows_ok(dtype, a.x, a.xsb, a.xsl, xsd, a.D) || ysd != 1) return false;
+  return sqn_dispatch(dtype, a, false, s);
+}
+
+bool scan_sqn_bwd_try(int dtype, const ScanNormArgs& a, long long xsd, long long ysd, long long gsd, cudaStream_t s) {
+  if (!rows_ok(dtype, a.x, a.xsb, a.xsl, xsd, a.D) || !rows_ok(dtype, a.dy, a.gsb, a.gsl, gsd, a.D) || ysd != 1 ||
+      a.y == a.x || a.y == a.dy)
+    return false;
+  return sqn_dispatch(dtype, a, true, s);
 }
 
 }  // namespace mega

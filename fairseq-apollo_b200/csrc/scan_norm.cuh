@@ -1,4 +1,4 @@
-// Interface of the per-feature TimestepNorm that is parallel over time (scan_norm.cu).
+// Interface of the per-feature norms that are parallel over time (scan_norm.cu).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -25,5 +25,10 @@ struct ScanNormArgs {
 // whole 16-byte pieces, too many sequences for the grid) or when there is no scratch memory.
 bool scan_norm_fwd_try(int dtype, const ScanNormArgs& a, long long xsd, long long ysd, cudaStream_t s);
 bool scan_norm_bwd_try(int dtype, const ScanNormArgs& a, long long xsd, long long ysd, long long gsd, cudaStream_t s);
+
+// Per-channel SequenceNorm: var_out receives rstd; the backward takes the forward's count, mean and rstd as
+// prev_count, prev_mean and prev_var.
+bool scan_sqn_fwd_try(int dtype, const ScanNormArgs& a, long long xsd, long long ysd, cudaStream_t s);
+bool scan_sqn_bwd_try(int dtype, const ScanNormArgs& a, long long xsd, long long ysd, long long gsd, cudaStream_t s);
 
 }  // namespace mega

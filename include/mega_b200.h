@@ -90,6 +90,9 @@ MEGA_API uint64_t mega_launch_count(void);
                                     step k (the barrier keeps expecting its bytes), so that every waiter of that
                                     stage runs into the wait limit, the kernel returns early without its final
                                     stores and raises the device error word; nothing faults or traps */
+#define MEGA_OPT_SPLIT 5 /* TimestepNorm -> EMA calls: 1: only the kernels that walk a sequence as one chain, 2: the forms
+                            parallel over time wherever they apply (3: the scan among them), 0: whichever is estimated
+                            to be faster */
 MEGA_API int mega_set_option(int key, int value);
 /*
  * Test aid: name of the kernel family of this process's most recent launch ("tsn_ema_mma tile=7 pipe=1",
