@@ -121,6 +121,7 @@ class BlockFunction(torch.autograd.Function):
         dwv = torch.mm(dv.t(), xn) if need[3] else None
         dmx = torch.mm(dbase, wm).view(bsz, seq, d) if need[2] else None
         dwm = torch.mm(dbase.t(), mx) if need[5] else None
+        dbv, dbm, dgamma, dbeta, dbias = torch.split(sums.to(wv.dtype), (e, f, 2 * s, 2 * s, nbias))
         t = ctx.dtypes
         return (dx.view(bsz, seq, d), dxn, dmx, dwv, dbv.to(t[0]), dwm, dbm.to(t[1]), dwh, dgamma.view(2, s).to(t[2]),
                 dbeta.view(2, s).to(t[3]), None if bias is None else dbias.to(bias.dtype), None, None, None)

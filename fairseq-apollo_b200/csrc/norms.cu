@@ -281,6 +281,49 @@ __global__ void __launch_bounds__(128) sqn_column_kernel(SqnArgs a) {
 }
 
 // ---------------------------------------------------------------------------
+// parameters of a norm module in one launch each way (as torch operations: a dozen launches of a few values)
+// ---------------------------------------------------------------------------
+// fp32 effective scale (weight + 1) and bias; with B > 0 also the priors as running statistics of B sequences
+template <typename T>
+__global__ void norm_prepare_kernel(const long long* prior_count, const T* prior_mean, const T* prior_logv, const T* weight,
+                                    const T* bias, int B, int G, int D, long long* count, float* mean, float* var,
+                                    float* gamma, float* beta) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < D) {
+    gamma[i] = Elem<T>::ld(weight + i) + 1.f;
+    beta[i] = Elem<T>::ld(bias + i);
+  }
+  if (i < G) {
+    const float m = Elem<T>::ld(prior_mean + i), v = expf(Elem<T>::ld(prior_logv + i));
+    for (int b = 0; b < B; ++b) {
+      mean[(size_t)b * G + i] = m;
+      var[(size_t)b * G + i] = v;
+    }
+  }
+  if (i < B) count[i] = prior_count[0];
+}
+// their gradients in the parameters' type: the affine pair converted, the priors' summed over the batch
+template <typename T>
+__global__ void norm_finish_kernel(const float* dprev_mean, const float* dprev_var, const T* prior_logv, const float* dgamma,
+                                   const float* dbeta, int B, int G, int D, T* dprior_mean, T* dprior_logv, T* dweight,
+                                   T* dbias) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < D) {
+    Elem<T>::st(dweight + i, dgamma[i]);
+    Elem<T>::st(dbias + i, dbeta[i]);
+  }
+  if (i < G && B > 0) {
+    float m = 0.f, v = 0.f;
+    for (int b = 0; b < B; ++b) {
+      m += dprev_mean[(size_t)b * G + i];
+      v += dprev_var[(size_t)b * G + i];
+    }
+    Elem<T>::st(dprior_mean + i, m);
+    Elem<T>::st(dprior_logv + i, v * expf(Elem<T>::ld(prior_logv + i)));
+  }
+}
+
+// ---------------------------------------------------------------------------
 // gates
 // ---------------------------------------------------------------------------
 template <typename T, int OP>
@@ -693,4 +736,32 @@ extern "C" int mega_gate_qk_rotary(const void* z, int64_t ld_z, const float* gam
                                     beta, rot, period, q_offset, (T*)q, (long long)ld_q, (T*)k, (long long)ld_k,
                                     (long long)rows, cols, (float)eps));
   return check_launch("gate_qk_rotary");
+}
+
+extern "C" int mega_norm_prepare(const int64_t* prior_count, const void* prior_mean, const void* prior_logv, const void* weight,
+                                 const void* bias, int dtype, int B, int G, int D, int64_t* count, float* mean, float* var,
+                                 float* gamma, float* beta, mega_stream_t stream) {
+  if (!weight || !bias || !gamma || !beta) return MEGA_ERR_NULL;
+  if (B > 0 && (!prior_count || !prior_mean || !prior_logv || !count || !mean || !var)) return MEGA_ERR_NULL;
+  if (!valid_dtype(dtype)) return MEGA_ERR_DTYPE;
+  if (D <= 0 || B < 0 || (B > 0 && G <= 0)) return MEGA_ERR_SHAPE;
+  const int n = D > B ? D : B;   // (G <= D)
+  MEGA_DISPATCH_DTYPE(dtype, launch(norm_prepare_kernel<T>, (unsigned)((n + 127) / 128), 128, 0, stream,
+                                    (const long long*)prior_count, (const T*)prior_mean, (const T*)prior_logv,
+                                    (const T*)weight, (const T*)bias, B, B > 0 ? G : 0, D, (long long*)count, mean, var, gamma,
+                                    beta));
+  return check_launch("norm_prepare");
+}
+
+extern "C" int mega_norm_finish(const float* dprev_mean, const float* dprev_var, const void* prior_logv, const float* dgamma,
+                                const float* dbeta, int dtype, int B, int G, int D, void* dprior_mean, void* dprior_logv,
+                                void* dweight, void* dbias, mega_stream_t stream) {
+  if (!dgamma || !dbeta || !dweight || !dbias) return MEGA_ERR_NULL;
+  if (B > 0 && (!dprev_mean || !dprev_var || !prior_logv || !dprior_mean || !dprior_logv)) return MEGA_ERR_NULL;
+  if (!valid_dtype(dtype)) return MEGA_ERR_DTYPE;
+  if (D <= 0 || B < 0 || (B > 0 && (G <= 0 || G > D))) return MEGA_ERR_SHAPE;
+  MEGA_DISPATCH_DTYPE(dtype, launch(norm_finish_kernel<T>, (unsigned)((D + 127) / 128), 128, 0, stream, dprev_mean, dprev_var,
+                                    (const T*)prior_logv, dgamma, dbeta, B, B > 0 ? G : 0, D, (T*)dprior_mean,
+                                    (T*)dprior_logv, (T*)dweight, (T*)dbias));
+  return check_launch("norm_finish");
 }

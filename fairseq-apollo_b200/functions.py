@@ -31,9 +31,8 @@ class EMAFunction(torch.autograd.Function):
         dx, dp, dq, dg, dom, _ = ops.ema_backward(dy, x, p, q, g, omega, padding_mask,
                                                   bidirectional=ctx.bidirectional, shift=ctx.shift,
                                                   truncation=ctx.truncation)
-        da, dd, db, dgm = ops.ema_coeffs_bwd(alpha, delta, beta, dp, dq, dg)
-        return (dx, da.to(alpha.dtype), dd.to(delta.dtype), db.to(beta.dtype), dgm.to(alpha.dtype),
-                dom.to(omega.dtype), None, None, None, None)
+        da, dd, db, dgm = ops.ema_coeffs_bwd(alpha, delta, beta, dp, dq, dg, alpha.dtype)
+        return (dx, da, dd.to(delta.dtype), db.to(beta.dtype), dgm, dom.to(omega.dtype), None, None, None, None)
 
 
 class ComplexEMAFunction(torch.autograd.Function):
@@ -56,66 +55,61 @@ class ComplexEMAFunction(torch.autograd.Function):
         dx, dp, dq, dg, dom = ops.cema_backward(dy, x, p, q, g, omega, padding_mask,
                                                 bidirectional=ctx.bidirectional, shift=ctx.shift,
                                                 truncation=ctx.truncation)
-        da, dd, dt, dgm = ops.cema_coeffs_bwd(alpha, delta, theta, q, dp, dq, dg)
-        return (dx, da.to(alpha.dtype), dd.to(delta.dtype), dt.to(theta.dtype), dgm.to(ctx.gamma_dtype),
+        da, dd, dt, dgm = ops.cema_coeffs_bwd(alpha, delta, theta, q, dp, dq, dg, alpha.dtype)
+        return (dx, da, dd.to(delta.dtype), dt.to(theta.dtype), dgm.to(ctx.gamma_dtype),
                 dom.view_as(omega).to(omega.dtype), None, None, None, None)
 
 
 class TimestepNormFunction(torch.autograd.Function):
-    """(y, count, mean, var) = TimestepNorm(x (B, L, D)); gamma is the effective scale.  Per-feature statistics
-    (channels contiguous) are taken again in the backward, so only the arguments are kept; otherwise the
-    statistics of every step are."""
+    """y = TimestepNorm(x (B, L, D)) from the module's own parameters.  Per-feature statistics (channels contiguous)
+    are taken again in the backward, so only the arguments are kept; otherwise the statistics of every step are."""
 
     @staticmethod
-    def forward(ctx, x, prev_count, prev_mean, prev_var, gamma, beta, padding_mask, num_groups, eps):
+    def forward(ctx, x, prior_count, prior_mean, prior_logv, weight, bias, padding_mask, num_groups, eps):
+        gamma, beta, prev_count, prev_mean, prev_var = ops.norm_prepare(weight, bias, (prior_count, prior_mean, prior_logv),
+                                                                        x.shape[0])
         ctx.recompute = num_groups is None and ops.timestep_norm_keeps_nothing(x)
         if ctx.recompute:
-            prev_count = prev_count.to(torch.int64).contiguous()
-            y, count, mean, var = ops.timestep_norm_fwd(x, prev_count, prev_mean, prev_var, gamma, beta, padding_mask, eps)
-            ctx.save_for_backward(x, prev_count, prev_mean, prev_var, gamma, padding_mask)
+            y, _, _, _ = ops.timestep_norm_fwd(x, prev_count, prev_mean, prev_var, gamma, beta, padding_mask, eps)
+            ctx.save_for_backward(x, prior_logv, prev_count, prev_mean, prev_var, gamma, padding_mask)
         else:
-            y, count, mean, var, cummean, cumrstd, group_mean = ops.timestep_norm_fwd_train(
+            y, count, _, _, cummean, cumrstd, group_mean = ops.timestep_norm_fwd_train(
                 x, prev_count, prev_mean, prev_var, gamma, beta, padding_mask, eps, num_groups)
-            ctx.save_for_backward(x, prev_mean, count, cummean, cumrstd, group_mean, gamma, padding_mask)
+            ctx.save_for_backward(x, prior_logv, prev_mean, count, cummean, cumrstd, group_mean, gamma, padding_mask)
         ctx.num_groups, ctx.eps = num_groups, eps
-        ctx.dtypes = (prev_mean.dtype, prev_var.dtype, gamma.dtype, beta.dtype)
-        ctx.mark_non_differentiable(count)
-        ctx.set_materialize_grads(False)
-        return y, count, mean, var
-
-    @staticmethod
-    def backward(ctx, dy, _, dmean, dvar):
-        x = ctx.saved_tensors[0]
-        if dy is None:
-            dy = torch.zeros_like(x)
-        if ctx.recompute:
-            x, prev_count, prev_mean, prev_var, gamma, padding_mask = ctx.saved_tensors
-            dx, dpm, dpv, dgamma, dbeta = ops.timestep_norm_bwd_stats(dy, dmean, dvar, x, prev_count, prev_mean, prev_var,
-                                                                      gamma, padding_mask, ctx.eps)
-        else:
-            x, prev_mean, count, cummean, cumrstd, group_mean, gamma, padding_mask = ctx.saved_tensors
-            dx, dpm, dpv, dgamma, dbeta = ops.timestep_norm_bwd(dy, dmean, dvar, x, prev_mean, count, cummean,
-                                                                cumrstd, group_mean, gamma, padding_mask,
-                                                                ctx.num_groups)
-        t = ctx.dtypes
-        return dx, None, dpm.to(t[0]), dpv.to(t[1]), dgamma.to(t[2]), dbeta.to(t[3]), None, None, None
-
-
-class SequenceNormFunction(torch.autograd.Function):
-    """y = SequenceNorm(x), per channel or per channel group; gamma is the effective scale."""
-
-    @staticmethod
-    def forward(ctx, x, gamma, beta, padding_mask, eps, length_last, num_groups=None):
-        y, count, mean, rstd = ops.sequence_norm_fwd(x, gamma, beta, padding_mask, eps, length_last, num_groups)
-        ctx.save_for_backward(x, count, mean, rstd, gamma, padding_mask)
-        ctx.length_last = length_last
-        ctx.num_groups = num_groups
-        ctx.dtypes = (gamma.dtype, beta.dtype)
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        x, count, mean, rstd, gamma, padding_mask = ctx.saved_tensors
+        if ctx.recompute:
+            x, prior_logv, prev_count, prev_mean, prev_var, gamma, padding_mask = ctx.saved_tensors
+            dx, dpm, dpv, dgamma, dbeta = ops.timestep_norm_bwd_stats(dy, None, None, x, prev_count, prev_mean, prev_var,
+                                                                      gamma, padding_mask, ctx.eps)
+        else:
+            x, prior_logv, prev_mean, count, cummean, cumrstd, group_mean, gamma, padding_mask = ctx.saved_tensors
+            dx, dpm, dpv, dgamma, dbeta = ops.timestep_norm_bwd(dy, None, None, x, prev_mean, count, cummean, cumrstd,
+                                                                group_mean, gamma, padding_mask, ctx.num_groups)
+        need = ctx.needs_input_grad
+        dw, db, dm, dl = ops.norm_finish(prior_logv, dgamma, dbeta, dpm, dpv, prior_logv)
+        return dx, None, dm if need[2] else None, dl if need[3] else None, dw, db, None, None, None
+
+
+class SequenceNormFunction(torch.autograd.Function):
+    """y = SequenceNorm(x), per channel or per channel group, from the module's own parameters."""
+
+    @staticmethod
+    def forward(ctx, x, weight, bias, padding_mask, eps, length_last, num_groups=None):
+        gamma, beta = ops.norm_prepare(weight, bias)
+        y, count, mean, rstd = ops.sequence_norm_fwd(x, gamma, beta, padding_mask, eps, length_last, num_groups)
+        ctx.save_for_backward(x, weight, count, mean, rstd, gamma, padding_mask)
+        ctx.length_last = length_last
+        ctx.num_groups = num_groups
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, weight, count, mean, rstd, gamma, padding_mask = ctx.saved_tensors
         dx, dgamma, dbeta = ops.sequence_norm_bwd(dy, x, count, mean, rstd, gamma, padding_mask, ctx.length_last,
                                                   ctx.num_groups)
-        return dx, dgamma.to(ctx.dtypes[0]), dbeta.to(ctx.dtypes[1]), None, None, None, None
+        dw, db = ops.norm_finish(weight, dgamma, dbeta)
+        return dx, dw, db, None, None, None, None

@@ -23,6 +23,12 @@ class _BlockPlan:
     """What a step passes to the library, converted once, with everything it keeps alive.  Valid for the same
     parameters (identity and version counters), state tensors, batch, dtype, device and stream."""
 
+    def __deepcopy__(self, memo):   # (a copied or pickled block builds its own)
+        return None
+
+    def __reduce__(self):
+        return (type(None), ())
+
     __slots__ = ("args", "addr", "fn", "key", "dev", "params", "versions", "nkey", "ekey", "akey", "mean", "var", "h",
                  "count", "count_next", "last_key", "last_value", "keys", "values", "pos", "cap", "chunk", "keep")
 

@@ -84,6 +84,7 @@ class MultiHeadComplexEMA(IncrementalStateMixin, nn.Module):
 
     def _apply(self, fn, *args, **kwargs):
         self._coeffs = None
+        self.__dict__.pop("_decode_cache", None)
         return super()._apply(fn, *args, **kwargs)
 
     # -- coefficients / kernel -----------------------------------------------------------

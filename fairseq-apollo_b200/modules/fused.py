@@ -40,14 +40,10 @@ def timestep_norm_ema(norm: TimestepNorm, move: MultiHeadEMA, x: Tensor,
     if (incremental_state is not None and x.size(1) == 1 and padding_mask is None and x.is_contiguous()
             and (not move.complex or move.ndim in (2, 4, 8, 16, 32))):
         return _decode_step(norm, move, x, incremental_state, activation, return_normed)
-    prev_count, prev_mean, prev_var, nstate = norm.initial_statistics(x.size(0), incremental_state)
-    if move.complex:
-        p, q, g = move.coeffs()
-        p, q, gamma_eff, beta, omega = p.squeeze(-1), q.squeeze(-1), norm.weight.detach().float() + 1.0, norm.bias, move.omega
-    else:
-        # inference: coefficients and the effective scale come from the cache that the single-token step
-        # uses too (rebuilt when a parameter's version counter moves), not from a kernel launch per call
-        gamma_eff, beta, p, q, g, omega = _fp32_params(norm, move)
+    # coefficients, effective scale and priors come from what the parameters were laid out to once (rebuilt when a
+    # version counter moves), not from kernel launches per call
+    gamma_eff, beta, p, q, g, omega = _fp32_params(norm, move)
+    _, _, prev_count, prev_mean, prev_var, nstate = norm.operands(x.size(0), incremental_state)
     h_in = None
     estate = None
     if incremental_state is not None:
@@ -70,11 +66,11 @@ def sequence_norm_ema(norm: SequenceNorm, move: MultiHeadEMA, x: Tensor, padding
     (moving_average_gated_attention.py:298-303, 313).  One kernel, one pass over x, when the norm
     is per channel and the rows fit the row-resident kernel; otherwise the two modules in turn."""
     assert activation in (None, 'silu')
-    train = needs_grad(x, *norm.parameters(), *move.parameters())
+    train = torch.is_grad_enabled() and needs_grad(x, *norm.parameters(), *move.parameters())
     if not train and not move.complex and norm.num_groups is None and move.truncation is None:
         p, q, g = move.coeffs()
-        y = ops.sqn_ema_forward(x, norm.weight.detach().float() + 1.0, norm.bias, norm.eps, p.squeeze(-1),
-                                q.squeeze(-1), g, move.omega, padding_mask, move.bidirectional, move.shift,
+        gamma, beta = norm.operands()
+        y = ops.sqn_ema_forward(x, gamma, beta, norm.eps, p, q, g, move.omega, padding_mask, move.bidirectional, move.shift,
                                 silu=activation == 'silu')
         if y is not None:
             return y
@@ -104,13 +100,7 @@ def _fp32_params(norm: TimestepNorm, move: MultiHeadEMA):
     return cache[1:7]
 
 
-_current_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
-
-try:   # the raw handle of the current stream without building a torch.cuda.Stream object
-    _raw_stream = torch._C._cuda_getCurrentRawStream
-except AttributeError:   # pragma: no cover - older / newer torch
-    def _raw_stream(index):
-        return torch.cuda.current_stream(index).cuda_stream
+_current_device, _raw_stream = ops._current_device, ops._raw_stream
 
 
 class _StepPlan:
@@ -120,6 +110,12 @@ class _StepPlan:
     Valid for as long as the parameters (identity and version counters), the state tensors, the batch
     size, the dtype and the options stay the same; the caller rebuilds it otherwise (new generation,
     reordered beams, an optimiser step, ...)."""
+
+    def __deepcopy__(self, memo):   # (a copied or pickled module builds its own)
+        return None
+
+    def __reduce__(self):
+        return (type(None), ())
 
     __slots__ = ("key", "fn", "args", "count_ptr", "count_cur", "count_alt", "keep", "params", "pver", "nkey", "ekey",
                  "dev")

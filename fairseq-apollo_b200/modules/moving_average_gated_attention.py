@@ -256,7 +256,7 @@ class MovingAverageGatedAttention(IncrementalStateMixin, nn.Module):
         assert embed_dim == self.embed_dim
         saved_state = self._get_input_buffer(incremental_state) if incremental_state is not None else None
         residual = x
-        train = needs_grad(x, *self.parameters())
+        train = torch.is_grad_enabled() and (x.requires_grad or needs_grad(*self.parameters()))
         silu_act = isinstance(self.move_act, nn.SiLU)
         fused_elementwise = not train and x.is_cuda
 

@@ -31,8 +31,31 @@ def _cuda(*ts):
             raise RuntimeError("mega_b200 ops run on CUDA tensors only (there is no CPU fallback)")
 
 
-def _stream():
-    return torch.cuda.current_stream().cuda_stream
+_current_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
+
+try:   # the raw handle of the current stream without building a torch.cuda.Stream object
+    _raw_stream = torch._C._cuda_getCurrentRawStream
+except AttributeError:   # pragma: no cover - older / newer torch
+    def _raw_stream(index):
+        return torch.cuda.current_stream(index).cuda_stream
+
+
+def _status(like, fn, *args):
+    """fn(*args, stream) on the device of ``like`` and its current stream."""
+    dev = like.get_device()
+    if dev < 0:
+        _cuda(like)
+    if _current_device() == dev:
+        return fn(*args, _raw_stream(dev))
+    with torch.cuda.device(dev):
+        return fn(*args, _raw_stream(dev))
+
+
+def _run(what, like, fn, *args):
+    """_status, raising on anything but OK."""
+    rc = _status(like, fn, *args)
+    if rc != 0:
+        _lib.check(rc, what)
 
 
 def _ptr(t):
@@ -41,12 +64,9 @@ def _ptr(t):
 
 def _f32c(t):
     """fp32, contiguous (parameters, statistics, states are tiny)."""
-    if t is None:
-        return None
-    t = t.detach()
-    if t.dtype != torch.float32:
-        t = t.float()
-    return t.contiguous()
+    if t is None or (t.dtype is torch.float32 and t.is_contiguous()):   # (only its memory is used)
+        return t
+    return t.detach().float().contiguous()
 
 
 def _mask_u8(mask, bsz, length):
@@ -54,8 +74,8 @@ def _mask_u8(mask, bsz, length):
         return None
     if mask.shape != (bsz, length):
         raise ValueError("padding_mask must be (batch, length) = (%d, %d), got %s" % (bsz, length, tuple(mask.shape)))
-    if mask.dtype == torch.bool:
-        return mask.contiguous().view(torch.uint8)
+    if mask.dtype is torch.bool:
+        return mask.contiguous()   # (a byte per value, 0 or 1: only its memory is used)
     return (mask != 0).contiguous().view(torch.uint8)
 
 
@@ -69,9 +89,8 @@ def ema_coeffs(alpha, delta, beta, gamma):
     p = torch.empty(k, n, device=alpha.device, dtype=torch.float32)
     q = torch.empty_like(p)
     g = torch.empty_like(p)
-    with torch.cuda.device(alpha.device):
-        _lib.check(_lib.lib().mega_ema_coeffs(*[a.data_ptr() for a in args], _dt(args[0]), k, n,
-                                              p.data_ptr(), q.data_ptr(), g.data_ptr(), _stream()), "ema_coeffs")
+    _run("ema_coeffs", alpha, _lib.lib().mega_ema_coeffs, *[a.data_ptr() for a in args], _dt(args[0]), k, n,
+         p.data_ptr(), q.data_ptr(), g.data_ptr())
     return p, q, g
 
 
@@ -81,9 +100,8 @@ def ema_kernel(p, q, g, length):
     p, q, g = _f32c(p), _f32c(q), _f32c(g)
     k, n = p.shape
     out = torch.empty(k, length, device=p.device, dtype=torch.float32)
-    with torch.cuda.device(p.device):
-        _lib.check(_lib.lib().mega_ema_kernel(p.data_ptr(), q.data_ptr(), g.data_ptr(), k, n, length,
-                                              out.data_ptr(), _stream()), "ema_kernel")
+    _run("ema_kernel", p, _lib.lib().mega_ema_kernel, p.data_ptr(), q.data_ptr(), g.data_ptr(), k, n, length,
+         out.data_ptr())
     return out
 
 
@@ -93,9 +111,8 @@ def ema_bias(q, g, h, length):
     q, g, h = _f32c(q), _f32c(g), _f32c(h)
     b, d, n = h.shape
     out = torch.empty(b, d, length, device=h.device, dtype=torch.float32)
-    with torch.cuda.device(h.device):
-        _lib.check(_lib.lib().mega_ema_bias(q.data_ptr(), g.data_ptr(), h.data_ptr(), b, d, n, length,
-                                            out.data_ptr(), _stream()), "ema_bias")
+    _run("ema_bias", h, _lib.lib().mega_ema_bias, q.data_ptr(), g.data_ptr(), h.data_ptr(), b, d, n, length,
+         out.data_ptr())
     return out
 
 
@@ -116,22 +133,21 @@ def ema_forward(x, p, q, g, omega, padding_mask=None, h_in=None, want_state=Fals
         raise ValueError("coefficient rows %d do not match embed_dim %d" % (p.shape[0], dim))
     mask = _mask_u8(padding_mask, bsz, length)
     if out is None:
-        out = torch.empty_strided(x.shape, x.stride(), dtype=x.dtype, device=x.device) \
-            if _dense(x) else torch.empty_like(x, memory_format=torch.contiguous_format)
+        out = _like(x)
     h_in = _f32c(h_in)
     h_out = torch.empty(bsz, dim, n, device=x.device, dtype=torch.float32) if want_state else None
     flags = (EMA_BIDIRECTIONAL if bidirectional else 0) | (0 if shift else EMA_NO_SHIFT) | (EMA_SILU if silu else 0)
     trunc = 0 if truncation is None or truncation < 1 else int(truncation)
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.lib().mega_ema_fwd(
-            x.data_ptr(), out.data_ptr(), _dt(x), bsz, dim, length, *x.stride(), *out.stride(),
-            p.data_ptr(), q.data_ptr(), g.data_ptr(), omega.data_ptr(), n,
-            _ptr(mask), _ptr(h_in), _ptr(h_out), flags, trunc, _stream()), "ema_fwd")
+    _run("ema_fwd", x, _lib.lib().mega_ema_fwd, x.data_ptr(), out.data_ptr(), _dt(x), bsz, dim, length, *x.stride(),
+         *out.stride(), p.data_ptr(), q.data_ptr(), g.data_ptr(), omega.data_ptr(), n, _ptr(mask), _ptr(h_in),
+         _ptr(h_out), flags, trunc)
     return (out, h_out) if want_state else out
 
 
 def _dense(t):
     """True when t's strides describe a permutation of a contiguous block."""
+    if t.is_contiguous():
+        return True
     exp = 1
     for size, stride in sorted(zip(t.shape, t.stride()), key=lambda v: v[1]):
         if size == 1:
@@ -153,14 +169,39 @@ def ema_step(x, p, q, g, omega, h=None, silu=False):
     h = _f32c(h)
     h_out = torch.empty(bsz, dim, n, device=x.device, dtype=torch.float32)
     y = torch.empty_like(x2)
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.lib().mega_ema_step(x2.data_ptr(), y.data_ptr(), _dt(x2), bsz, dim, p.data_ptr(),
-                                            q.data_ptr(), g.data_ptr(), omega.data_ptr(), n, _ptr(h),
-                                            h_out.data_ptr(), EMA_SILU if silu else 0, _stream()), "ema_step")
+    _run("ema_step", x, _lib.lib().mega_ema_step, x2.data_ptr(), y.data_ptr(), _dt(x2), bsz, dim, p.data_ptr(),
+         q.data_ptr(), g.data_ptr(), omega.data_ptr(), n, _ptr(h), h_out.data_ptr(), EMA_SILU if silu else 0)
     return y.view(shape), h_out
 
 
 # --------------------------------------------------------------------------- norms
+def norm_prepare(weight, bias, priors=None, bsz=0):
+    """A norm module's parameters for the operators: (gamma = weight + 1, beta) fp32, and with ``priors`` =
+    (prior_count, prior_mean, prior_logv) also (count, mean, var) of ``bsz`` sequences.  One launch."""
+    dev, dim = weight.device, weight.shape[0]
+    g = priors[1].shape[0] if priors else 0
+    f = torch.empty(2 * dim + 2 * bsz * g, device=dev, dtype=torch.float32)
+    gamma, beta, mean, var = f[:dim], f[dim:2 * dim], f[2 * dim:2 * dim + bsz * g], f[2 * dim + bsz * g:]
+    count = torch.empty(bsz, device=dev, dtype=torch.int64) if priors else None
+    pc, pm, pl = priors if priors else (None, None, None)
+    _run("norm_prepare", weight, _lib.lib().mega_norm_prepare, _ptr(pc), _ptr(pm), _ptr(pl), weight.data_ptr(),
+         bias.data_ptr(), _dt(weight), bsz, g, dim, _ptr(count), mean.data_ptr() if priors else None,
+         var.data_ptr() if priors else None, gamma.data_ptr(), beta.data_ptr())
+    return (gamma, beta, count, mean.view(bsz, g), var.view(bsz, g)) if priors else (gamma, beta)
+
+
+def norm_finish(like, dgamma, dbeta, dprev_mean=None, dprev_var=None, prior_logv=None):
+    """Gradients of norm_prepare's parameters in their type: (dweight, dbias[, dprior_mean, dprior_logv])."""
+    dim = dgamma.shape[0]
+    bsz, g = dprev_mean.shape if dprev_mean is not None else (0, 0)
+    out = torch.empty(2 * dim + 2 * g, device=like.device, dtype=like.dtype)
+    dw, db, dm, dl = torch.split(out, (dim, dim, g, g))
+    _run("norm_finish", like, _lib.lib().mega_norm_finish, _ptr(dprev_mean), _ptr(dprev_var), _ptr(prior_logv),
+         dgamma.data_ptr(), dbeta.data_ptr(), _dt(like), bsz, g, dim, dm.data_ptr() if g else None,
+         dl.data_ptr() if g else None, dw.data_ptr(), db.data_ptr())
+    return (dw, db, dm, dl) if g else (dw, db)
+
+
 def timestep_norm_fwd(x, prev_count, prev_mean, prev_var, gamma, beta, padding_mask=None,
                       eps=1e-5, num_groups=None, out=None):
     """x (B, L, D) any strides -> (y, count (B) int64, mean, var (B, G) fp32).
@@ -175,17 +216,14 @@ def timestep_norm_fwd(x, prev_count, prev_mean, prev_var, gamma, beta, padding_m
     gamma, beta = _f32c(gamma), _f32c(beta)
     mask = _mask_u8(padding_mask, bsz, length)
     if out is None:
-        out = torch.empty_strided(x.shape, x.stride(), dtype=x.dtype, device=x.device) \
-            if _dense(x) else torch.empty_like(x, memory_format=torch.contiguous_format)
+        out = _like(x)
     count = torch.empty(bsz, device=x.device, dtype=torch.int64)
     mean = torch.empty(bsz, groups, device=x.device, dtype=torch.float32)
     var = torch.empty_like(mean)
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.lib().mega_timestep_norm_fwd(
-            x.data_ptr(), out.data_ptr(), _dt(x), bsz, length, dim, *x.stride(), *out.stride(),
-            prev_count.data_ptr(), prev_mean.data_ptr(), prev_var.data_ptr(), gamma.data_ptr(), beta.data_ptr(),
-            _ptr(mask), groups, float(eps), count.data_ptr(), mean.data_ptr(), var.data_ptr(), _stream()),
-            "timestep_norm_fwd")
+    _run("timestep_norm_fwd", x, _lib.lib().mega_timestep_norm_fwd, x.data_ptr(), out.data_ptr(), _dt(x), bsz,
+         length, dim, *x.stride(), *out.stride(), prev_count.data_ptr(), prev_mean.data_ptr(), prev_var.data_ptr(),
+         gamma.data_ptr(), beta.data_ptr(), _ptr(mask), groups, float(eps), count.data_ptr(), mean.data_ptr(),
+         var.data_ptr())
     return out, count, mean, var
 
 
@@ -201,8 +239,7 @@ def sequence_norm_fwd(x, gamma, beta, padding_mask=None, eps=1e-5, length_last=T
     gamma, beta = _f32c(gamma), _f32c(beta)
     mask = _mask_u8(padding_mask, bsz, length)
     if out is None:
-        out = torch.empty_strided(x.shape, x.stride(), dtype=x.dtype, device=x.device) \
-            if _dense(x) else torch.empty_like(x, memory_format=torch.contiguous_format)
+        out = _like(x)
     xs, ys = x.stride(), out.stride()
     if not length_last:
         xs = (xs[0], xs[2], xs[1])
@@ -210,11 +247,9 @@ def sequence_norm_fwd(x, gamma, beta, padding_mask=None, eps=1e-5, length_last=T
     count = torch.empty(bsz, device=x.device, dtype=torch.int64)
     mean = torch.empty(bsz, groups, device=x.device, dtype=torch.float32)
     rstd = torch.empty_like(mean)
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.lib().mega_sequence_norm_fwd(
-            x.data_ptr(), out.data_ptr(), _dt(x), bsz, dim, length, *xs, *ys, gamma.data_ptr(), beta.data_ptr(),
-            _ptr(mask), groups, float(eps), count.data_ptr(), mean.data_ptr(), rstd.data_ptr(), _stream()),
-            "sequence_norm_fwd")
+    _run("sequence_norm_fwd", x, _lib.lib().mega_sequence_norm_fwd, x.data_ptr(), out.data_ptr(), _dt(x), bsz, dim,
+         length, *xs, *ys, gamma.data_ptr(), beta.data_ptr(), _ptr(mask), groups, float(eps), count.data_ptr(),
+         mean.data_ptr(), rstd.data_ptr())
     return out, count, mean, rstd
 
 
@@ -234,9 +269,8 @@ def tsn_ema_forward(x, prev_count, prev_mean, prev_var, gamma, beta, eps, p, q, 
         p, q, g, omega = _f32c(p), _f32c(q), _f32c(g), _f32c(omega)
     n = p.shape[1]
     mask = _mask_u8(padding_mask, bsz, length)
-    y = torch.empty_strided(x.shape, x.stride(), dtype=x.dtype, device=x.device) \
-        if _dense(x) else torch.empty_like(x, memory_format=torch.contiguous_format)
-    xn = torch.empty_strided(y.shape, y.stride(), dtype=x.dtype, device=x.device) if want_normed else None
+    y = _like(x)
+    xn = torch.empty_like(y) if want_normed else None
     count = torch.empty(bsz, device=x.device, dtype=torch.int64)
     mean = torch.empty(bsz, dim, device=x.device, dtype=torch.float32)
     var = torch.empty_like(mean)
@@ -247,13 +281,10 @@ def tsn_ema_forward(x, prev_count, prev_mean, prev_var, gamma, beta, eps, p, q, 
         h_in = _f32c(h_in)
         h_out = torch.empty(bsz, dim, n, device=x.device, dtype=torch.float32) if want_state else None
         entry, what = _lib.lib().mega_tsn_ema_fwd, "tsn_ema_fwd"
-    with torch.cuda.device(x.device):
-        _lib.check(entry(
-            x.data_ptr(), y.data_ptr(), _ptr(xn), _dt(x), bsz, length, dim, *x.stride(), *y.stride(),
-            prev_count.data_ptr(), prev_mean.data_ptr(), prev_var.data_ptr(), gamma.data_ptr(), beta.data_ptr(),
-            float(eps), count.data_ptr(), mean.data_ptr(), var.data_ptr(),
-            p.data_ptr(), q.data_ptr(), g.data_ptr(), omega.data_ptr(), n, _ptr(mask), _ptr(h_in), _ptr(h_out),
-            EMA_SILU if silu else 0, _stream()), what)
+    _run(what, x, entry, x.data_ptr(), y.data_ptr(), _ptr(xn), _dt(x), bsz, length, dim, *x.stride(), *y.stride(),
+         prev_count.data_ptr(), prev_mean.data_ptr(), prev_var.data_ptr(), gamma.data_ptr(), beta.data_ptr(),
+         float(eps), count.data_ptr(), mean.data_ptr(), var.data_ptr(), p.data_ptr(), q.data_ptr(), g.data_ptr(),
+         omega.data_ptr(), n, _ptr(mask), _ptr(h_in), _ptr(h_out), EMA_SILU if silu else 0)
     res = {"y": y, "count": count, "mean": mean, "var": var}
     if want_state:
         res["h"] = torch.view_as_complex(h_out) if complex_poles else h_out
@@ -274,11 +305,9 @@ def sqn_ema_forward(x, gamma, beta, eps, p, q, g, omega, padding_mask=None, bidi
     mask = _mask_u8(padding_mask, bsz, length)
     y = torch.empty_like(x, memory_format=torch.contiguous_format)
     flags = (EMA_BIDIRECTIONAL if bidirectional else 0) | (0 if shift else EMA_NO_SHIFT) | (EMA_SILU if silu else 0)
-    with torch.cuda.device(x.device):
-        rc = _lib.lib().mega_sqn_ema_fwd(x.data_ptr(), y.data_ptr(), _dt(x), bsz, dim, length, *x.stride(), *y.stride(),
-                                         gamma.data_ptr(), beta.data_ptr(), float(eps), None, None, None,
-                                         p.data_ptr(), q.data_ptr(), g.data_ptr(), omega.data_ptr(), p.shape[1],
-                                         _ptr(mask), flags, _stream())
+    rc = _status(x, _lib.lib().mega_sqn_ema_fwd, x.data_ptr(), y.data_ptr(), _dt(x), bsz, dim, length, *x.stride(),
+                 *y.stride(), gamma.data_ptr(), beta.data_ptr(), float(eps), None, None, None, p.data_ptr(), q.data_ptr(),
+                 g.data_ptr(), omega.data_ptr(), p.shape[1], _ptr(mask), flags)
     if rc == 7:  # MEGA_ERR_UNSUPPORTED: outside the envelope
         return None
     _lib.check(rc, "sqn_ema_fwd")
@@ -293,12 +322,9 @@ def tsn_ema_step_(x, y, count, mean, var, gamma, beta, eps, p, q, g, omega, h, s
     With ``count_next`` (a second (B) int64 tensor) the bumped counts go there from the same launch
     and ``count`` stays as it was; without it a second launch bumps ``count`` in place."""
     bsz, dim = x.shape
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.lib().mega_tsn_ema_step(
-            x.data_ptr(), y.data_ptr(), _ptr(xn_out), _dt(x), bsz, dim, _ptr(count), _ptr(count_next), _ptr(mean),
-            _ptr(var),
-            _ptr(gamma), _ptr(beta), float(eps), p.data_ptr(), q.data_ptr(), g.data_ptr(), omega.data_ptr(),
-            p.shape[1], h.data_ptr(), EMA_SILU if silu else 0, _stream()), "tsn_ema_step")
+    _run("tsn_ema_step", x, _lib.lib().mega_tsn_ema_step, x.data_ptr(), y.data_ptr(), _ptr(xn_out), _dt(x), bsz, dim,
+         _ptr(count), _ptr(count_next), _ptr(mean), _ptr(var), _ptr(gamma), _ptr(beta), float(eps), p.data_ptr(),
+         q.data_ptr(), g.data_ptr(), omega.data_ptr(), p.shape[1], h.data_ptr(), EMA_SILU if silu else 0)
     return y
 
 
@@ -307,12 +333,10 @@ def tsn_cema_step_(x, y, count, mean, var, gamma, beta, eps, p, q, g, omega, h, 
     """tsn_ema_step_ for the complex layer: q, g (K, N, 2) and h (B, D, N, 2) are fp32 views of the
     complex64 tensors; everything is updated in place, nothing is converted or allocated."""
     bsz, dim = x.shape
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.lib().mega_tsn_cema_step(
-            x.data_ptr(), y.data_ptr(), _ptr(xn_out), _dt(x), bsz, dim, count.data_ptr(), _ptr(count_next),
-            mean.data_ptr(),
-            var.data_ptr(), gamma.data_ptr(), beta.data_ptr(), float(eps), p.data_ptr(), q.data_ptr(), g.data_ptr(),
-            omega.data_ptr(), p.shape[1], h.data_ptr(), EMA_SILU if silu else 0, _stream()), "tsn_cema_step")
+    _run("tsn_cema_step", x, _lib.lib().mega_tsn_cema_step, x.data_ptr(), y.data_ptr(), _ptr(xn_out), _dt(x), bsz,
+         dim, count.data_ptr(), _ptr(count_next), mean.data_ptr(), var.data_ptr(), gamma.data_ptr(), beta.data_ptr(),
+         float(eps), p.data_ptr(), q.data_ptr(), g.data_ptr(), omega.data_ptr(), p.shape[1], h.data_ptr(),
+         EMA_SILU if silu else 0)
     return y
 
 
@@ -344,9 +368,8 @@ def gate_silu(a, b=None):
     if b is not None:
         b_, _, _, ldb = _rows(b)
     y = torch.empty(a.shape, dtype=a.dtype, device=a.device)
-    with torch.cuda.device(a.device):
-        _lib.check(_lib.lib().mega_gate_silu(a_.data_ptr(), lda, _ptr(b_), ldb, y.data_ptr(), cols, _dt(a),
-                                             rows, cols, _stream()), "gate_silu")
+    _run("gate_silu", a, _lib.lib().mega_gate_silu, a_.data_ptr(), lda, _ptr(b_), ldb, y.data_ptr(), cols, _dt(a),
+         rows, cols)
     return y
 
 
@@ -356,9 +379,8 @@ def gate_mul_silu(a, r):
     a_, rows, cols, lda = _rows(a)
     r_, _, _, ldr = _rows(r)
     y = torch.empty(a.shape, dtype=a.dtype, device=a.device)
-    with torch.cuda.device(a.device):
-        _lib.check(_lib.lib().mega_gate_mul_silu(a_.data_ptr(), lda, r_.data_ptr(), ldr, y.data_ptr(), cols,
-                                                 _dt(a), rows, cols, _stream()), "gate_mul_silu")
+    _run("gate_mul_silu", a, _lib.lib().mega_gate_mul_silu, a_.data_ptr(), lda, r_.data_ptr(), ldr, y.data_ptr(),
+         cols, _dt(a), rows, cols)
     return y
 
 
@@ -370,10 +392,8 @@ def gate_output(residual, u, hx, h_lin):
     x_, _, _, ldx = _rows(hx)
     h_, _, _, ldh = _rows(h_lin)
     y = torch.empty(residual.shape, dtype=residual.dtype, device=residual.device)
-    with torch.cuda.device(residual.device):
-        _lib.check(_lib.lib().mega_gate_output(r_.data_ptr(), ldr, u_.data_ptr(), ldu, x_.data_ptr(), ldx,
-                                               h_.data_ptr(), ldh, y.data_ptr(), cols, _dt(residual), rows, cols,
-                                               _stream()), "gate_output")
+    _run("gate_output", residual, _lib.lib().mega_gate_output, r_.data_ptr(), ldr, u_.data_ptr(), ldu, x_.data_ptr(),
+         ldx, h_.data_ptr(), ldh, y.data_ptr(), cols, _dt(residual), rows, cols)
     return y
 
 
@@ -390,10 +410,8 @@ def gate_qk(z, gamma, beta, eps=1e-5):
         raise ValueError("gate_qk: gamma and beta must be (2, %d)" % cols)
     q = torch.empty(z.shape, dtype=z.dtype, device=z.device)
     k = torch.empty(z.shape, dtype=z.dtype, device=z.device)
-    with torch.cuda.device(z.device):
-        _lib.check(_lib.lib().mega_gate_qk(z_.data_ptr(), ldz, g.data_ptr(), b.data_ptr(), q.data_ptr(), cols,
-                                           k.data_ptr(), cols, _dt(z), rows, cols, float(eps), _stream()),
-                   "gate_qk")
+    _run("gate_qk", z, _lib.lib().mega_gate_qk, z_.data_ptr(), ldz, g.data_ptr(), b.data_ptr(), q.data_ptr(), cols,
+         k.data_ptr(), cols, _dt(z), rows, cols, float(eps))
     return q, k
 
 
@@ -414,55 +432,51 @@ def gate_qk_rotary(z, gamma, beta, rot, period, q_offset=0, eps=1e-5):
         raise ValueError("gate_qk_rotary: rot must be (positions, %d) complex or (positions, %d, 2) float" % (cols // 2, cols // 2))
     q = torch.empty(z.shape, dtype=z.dtype, device=z.device)
     k = torch.empty(z.shape, dtype=z.dtype, device=z.device)
-    with torch.cuda.device(z.device):
-        _lib.check(_lib.lib().mega_gate_qk_rotary(z_.data_ptr(), ldz, g.data_ptr(), b.data_ptr(), r.data_ptr(),
-                                                  r.shape[0], int(period), int(q_offset), q.data_ptr(), cols,
-                                                  k.data_ptr(), cols, _dt(z), rows, cols, float(eps), _stream()),
-                   "gate_qk_rotary")
+    _run("gate_qk_rotary", z, _lib.lib().mega_gate_qk_rotary, z_.data_ptr(), ldz, g.data_ptr(), b.data_ptr(),
+         r.data_ptr(), r.shape[0], int(period), int(q_offset), q.data_ptr(), cols, k.data_ptr(), cols, _dt(z), rows,
+         cols, float(eps))
     return q, k
 
 
 def gate_silu_bwd(dy, a, da, colsum=None):
     """da = dy * silu'(a) for row-major matrices (da may be dy); colsum (cols) fp32 gets da's column sums added."""
     rows, cols = a.shape
-    with torch.cuda.device(a.device):
-        _lib.check(_lib.lib().mega_gate_silu_bwd(dy.data_ptr(), dy.stride(0), a.data_ptr(), a.stride(0), da.data_ptr(),
-                                                 da.stride(0), _ptr(colsum), _dt(a), rows, cols, _stream()), "gate_silu_bwd")
+    _run("gate_silu_bwd", a, _lib.lib().mega_gate_silu_bwd, dy.data_ptr(), dy.stride(0), a.data_ptr(), a.stride(0),
+         da.data_ptr(), da.stride(0), _ptr(colsum), _dt(a), rows, cols)
 
 
 def gate_mul_silu_bwd(dy, a, r, da, dr, colsum_r=None):
     """Gradients of a * silu(r) into da (may be dy) and dr; colsum_r gets dr's column sums added."""
     rows, cols = a.shape
-    with torch.cuda.device(a.device):
-        _lib.check(_lib.lib().mega_gate_mul_silu_bwd(
-            dy.data_ptr(), dy.stride(0), a.data_ptr(), a.stride(0), r.data_ptr(), r.stride(0), da.data_ptr(), da.stride(0),
-            dr.data_ptr(), dr.stride(0), _ptr(colsum_r), _dt(a), rows, cols, _stream()), "gate_mul_silu_bwd")
+    _run("gate_mul_silu_bwd", a, _lib.lib().mega_gate_mul_silu_bwd, dy.data_ptr(), dy.stride(0), a.data_ptr(),
+         a.stride(0), r.data_ptr(), r.stride(0), da.data_ptr(), da.stride(0), dr.data_ptr(), dr.stride(0),
+         _ptr(colsum_r), _dt(a), rows, cols)
 
 
 def gate_output_bwd(dout, residual, u, hx, h_lin, dres, du, dhx, colsum_u=None, colsum_hx=None):
     """Gradients of gate_output into dres, du and dhx (= that of h_lin), with column sums of the latter two."""
     rows, cols = residual.shape
-    with torch.cuda.device(residual.device):
-        _lib.check(_lib.lib().mega_gate_output_bwd(
-            dout.data_ptr(), dout.stride(0), residual.data_ptr(), residual.stride(0), u.data_ptr(), u.stride(0),
-            hx.data_ptr(), hx.stride(0), h_lin.data_ptr(), h_lin.stride(0), dres.data_ptr(), dres.stride(0),
-            du.data_ptr(), du.stride(0), dhx.data_ptr(), dhx.stride(0), _ptr(colsum_u), _ptr(colsum_hx), _dt(residual),
-            rows, cols, _stream()), "gate_output_bwd")
+    _run("gate_output_bwd", residual, _lib.lib().mega_gate_output_bwd, dout.data_ptr(), dout.stride(0),
+         residual.data_ptr(), residual.stride(0), u.data_ptr(), u.stride(0), hx.data_ptr(), hx.stride(0),
+         h_lin.data_ptr(), h_lin.stride(0), dres.data_ptr(), dres.stride(0), du.data_ptr(), du.stride(0),
+         dhx.data_ptr(), dhx.stride(0), _ptr(colsum_u), _ptr(colsum_hx), _dt(residual), rows, cols)
 
 
 def gate_qk_bwd(z, gamma, rot, period, dq, dk, dz, dgamma, dbeta, colsum=None, eps=1e-5):
     """Gradients of gate_qk (rot None) or gate_qk_rotary: dz, and dgamma, dbeta (2 S) fp32 added to."""
     rows, cols = z.shape
     g = _f32c(gamma)
-    with torch.cuda.device(z.device):
-        _lib.check(_lib.lib().mega_gate_qk_bwd(
-            z.data_ptr(), z.stride(0), g.data_ptr(), _ptr(rot), 0 if rot is None else rot.shape[0], int(period), 0,
-            dq.data_ptr(), dq.stride(0), dk.data_ptr(), dk.stride(0), dz.data_ptr(), dz.stride(0), dgamma.data_ptr(),
-            dbeta.data_ptr(), _ptr(colsum), _dt(z), rows, cols, float(eps), _stream()), "gate_qk_bwd")
+    _run("gate_qk_bwd", z, _lib.lib().mega_gate_qk_bwd, z.data_ptr(), z.stride(0), g.data_ptr(), _ptr(rot),
+         0 if rot is None else rot.shape[0], int(period), 0, dq.data_ptr(), dq.stride(0), dk.data_ptr(),
+         dk.stride(0), dz.data_ptr(), dz.stride(0), dgamma.data_ptr(), dbeta.data_ptr(), _ptr(colsum), _dt(z), rows,
+         cols, float(eps))
 
 
 # ------------------------------------------------------------------------ training
 def _like(x):
+    """Uninitialised, shaped and strided like x (contiguous when x's strides leave gaps)."""
+    if x.is_contiguous():
+        return torch.empty_like(x)
     return torch.empty_strided(x.shape, x.stride(), dtype=x.dtype, device=x.device) \
         if _dense(x) else torch.empty_like(x, memory_format=torch.contiguous_format)
 
@@ -487,12 +501,10 @@ def timestep_norm_fwd_train(x, prev_count, prev_mean, prev_var, gamma, beta, pad
     cummean = torch.empty(bsz, length, groups, device=x.device, dtype=torch.float32)
     cumrstd = torch.empty_like(cummean)
     group_mean = torch.empty_like(cummean) if groups != dim else None
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.lib().mega_timestep_norm_fwd_train(
-            x.data_ptr(), out.data_ptr(), _dt(x), bsz, length, dim, *x.stride(), *out.stride(),
-            prev_count.data_ptr(), prev_mean.data_ptr(), prev_var.data_ptr(), gamma.data_ptr(), beta.data_ptr(),
-            _ptr(mask), groups, float(eps), count.data_ptr(), mean.data_ptr(), var.data_ptr(),
-            cummean.data_ptr(), cumrstd.data_ptr(), _ptr(group_mean), _stream()), "timestep_norm_fwd_train")
+    _run("timestep_norm_fwd_train", x, _lib.lib().mega_timestep_norm_fwd_train, x.data_ptr(), out.data_ptr(), _dt(x),
+         bsz, length, dim, *x.stride(), *out.stride(), prev_count.data_ptr(), prev_mean.data_ptr(),
+         prev_var.data_ptr(), gamma.data_ptr(), beta.data_ptr(), _ptr(mask), groups, float(eps), count.data_ptr(),
+         mean.data_ptr(), var.data_ptr(), cummean.data_ptr(), cumrstd.data_ptr(), _ptr(group_mean))
     return out, count, mean, var, cummean, cumrstd, group_mean
 
 
@@ -512,12 +524,10 @@ def timestep_norm_bwd(dy, dmean, dvar, x, prev_mean, count, cummean, cumrstd, gr
     dpv = torch.empty_like(dpm)
     dgamma = torch.empty(dim, device=x.device, dtype=torch.float32)
     dbeta = torch.empty_like(dgamma)
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.lib().mega_timestep_norm_bwd(
-            dy.data_ptr(), x.data_ptr(), dx.data_ptr(), _dt(x), bsz, length, dim, *dy.stride(), *x.stride(),
-            *dx.stride(), _ptr(dmean), _ptr(dvar), prev_mean.data_ptr(), count.data_ptr(), cummean.data_ptr(),
-            cumrstd.data_ptr(), _ptr(group_mean), gamma.data_ptr(), _ptr(mask), groups, dpm.data_ptr(),
-            dpv.data_ptr(), dgamma.data_ptr(), dbeta.data_ptr(), _stream()), "timestep_norm_bwd")
+    _run("timestep_norm_bwd", x, _lib.lib().mega_timestep_norm_bwd, dy.data_ptr(), x.data_ptr(), dx.data_ptr(),
+         _dt(x), bsz, length, dim, *dy.stride(), *x.stride(), *dx.stride(), _ptr(dmean), _ptr(dvar),
+         prev_mean.data_ptr(), count.data_ptr(), cummean.data_ptr(), cumrstd.data_ptr(), _ptr(group_mean),
+         gamma.data_ptr(), _ptr(mask), groups, dpm.data_ptr(), dpv.data_ptr(), dgamma.data_ptr(), dbeta.data_ptr())
     return dx, dpm, dpv, dgamma, dbeta
 
 
@@ -544,12 +554,10 @@ def timestep_norm_bwd_stats(dy, dmean, dvar, x, prev_count, prev_mean, prev_var,
     dpv = torch.empty_like(dpm)
     dgamma = torch.empty(dim, device=x.device, dtype=torch.float32)
     dbeta = torch.empty_like(dgamma)
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.lib().mega_timestep_norm_bwd_stats(
-            dy.data_ptr(), x.data_ptr(), dx.data_ptr(), _dt(x), bsz, length, dim, *dy.stride(), *x.stride(),
-            *dx.stride(), _ptr(dmean), _ptr(dvar), prev_count.data_ptr(), prev_mean.data_ptr(), prev_var.data_ptr(),
-            gamma.data_ptr(), _ptr(mask), float(eps), dpm.data_ptr(), dpv.data_ptr(), dgamma.data_ptr(),
-            dbeta.data_ptr(), _stream()), "timestep_norm_bwd_stats")
+    _run("timestep_norm_bwd_stats", x, _lib.lib().mega_timestep_norm_bwd_stats, dy.data_ptr(), x.data_ptr(),
+         dx.data_ptr(), _dt(x), bsz, length, dim, *dy.stride(), *x.stride(), *dx.stride(), _ptr(dmean), _ptr(dvar),
+         prev_count.data_ptr(), prev_mean.data_ptr(), prev_var.data_ptr(), gamma.data_ptr(), _ptr(mask), float(eps),
+         dpm.data_ptr(), dpv.data_ptr(), dgamma.data_ptr(), dbeta.data_ptr())
     return dx, dpm, dpv, dgamma, dbeta
 
 
@@ -570,12 +578,10 @@ def sequence_norm_bwd(dy, x, count, mean, rstd, gamma, padding_mask=None, length
         gs, xs, ds = (gs[0], gs[2], gs[1]), (xs[0], xs[2], xs[1]), (ds[0], ds[2], ds[1])
     dgamma = torch.empty(dim, device=x.device, dtype=torch.float32)
     dbeta = torch.empty_like(dgamma)
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.lib().mega_sequence_norm_bwd(
-            dy.data_ptr(), x.data_ptr(), dx.data_ptr(), _dt(x), bsz, dim, length, *gs, *xs, *ds,
-            count.data_ptr(), mean.data_ptr(), rstd.data_ptr(), gamma.data_ptr(), _ptr(mask),
-            dim if num_groups is None else int(num_groups), dgamma.data_ptr(), dbeta.data_ptr(), _stream()),
-            "sequence_norm_bwd")
+    _run("sequence_norm_bwd", x, _lib.lib().mega_sequence_norm_bwd, dy.data_ptr(), x.data_ptr(), dx.data_ptr(),
+         _dt(x), bsz, dim, length, *gs, *xs, *ds, count.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
+         gamma.data_ptr(), _ptr(mask), dim if num_groups is None else int(num_groups), dgamma.data_ptr(),
+         dbeta.data_ptr())
     return dx, dgamma, dbeta
 
 
@@ -598,28 +604,25 @@ def ema_backward(dy, x, p, q, g, omega, padding_mask=None, h_in=None, dh_out=Non
     dom = torch.empty(dim, device=x.device, dtype=torch.float32)
     dh_in = torch.empty(bsz, dim, n, device=x.device, dtype=torch.float32) if want_dh_in else None
     flags = (EMA_BIDIRECTIONAL if bidirectional else 0) | (0 if shift else EMA_NO_SHIFT)
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.lib().mega_ema_bwd(
-            dy.data_ptr(), x.data_ptr(), dx.data_ptr(), _dt(x), bsz, dim, length, *dy.stride(), *x.stride(),
-            *dx.stride(), p.data_ptr(), q.data_ptr(), g.data_ptr(), omega.data_ptr(), n, _ptr(mask), _ptr(h_in),
-            _ptr(dh_out), flags, _trunc(truncation), dp.data_ptr(), dq.data_ptr(), dg.data_ptr(), dom.data_ptr(),
-            _ptr(dh_in),
-            _stream()), "ema_bwd")
+    _run("ema_bwd", x, _lib.lib().mega_ema_bwd, dy.data_ptr(), x.data_ptr(), dx.data_ptr(), _dt(x), bsz, dim, length,
+         *dy.stride(), *x.stride(), *dx.stride(), p.data_ptr(), q.data_ptr(), g.data_ptr(), omega.data_ptr(), n,
+         _ptr(mask), _ptr(h_in), _ptr(dh_out), flags, _trunc(truncation), dp.data_ptr(), dq.data_ptr(),
+         dg.data_ptr(), dom.data_ptr(), _ptr(dh_in))
     return dx, dp, dq, dg, dom, dh_in
 
 
-def ema_coeffs_bwd(alpha, delta, beta, dp, dq, dg):
-    """(dalpha, ddelta, dbeta (K, N, 1), dgamma (K, N)) from the coefficient gradients."""
+def ema_coeffs_bwd(alpha, delta, beta, dp, dq, dg, dtype=torch.float32):
+    """(dalpha, ddelta, dbeta (K, N, 1), dgamma (K, N)) in ``dtype`` from the coefficient gradients."""
     _cuda(alpha, delta, beta, dp, dq, dg)
     k, n = alpha.shape[0], alpha.shape[1]
     a, d, b = _f32c(alpha).view(k, n), _f32c(delta).view(k, n), _f32c(beta).view(k, n)
     dp, dq, dg = _f32c(dp), _f32c(dq), _f32c(dg)
-    outs = [torch.empty(k, n, device=alpha.device, dtype=torch.float32) for _ in range(4)]
-    with torch.cuda.device(alpha.device):
-        _lib.check(_lib.lib().mega_ema_coeffs_bwd(a.data_ptr(), d.data_ptr(), b.data_ptr(), dp.data_ptr(),
-                                                  dq.data_ptr(), dg.data_ptr(), k, n,
-                                                  *[o.data_ptr() for o in outs], _stream()), "ema_coeffs_bwd")
-    return outs[0].unsqueeze(-1), outs[1].unsqueeze(-1), outs[2].unsqueeze(-1), outs[3]
+    outs = torch.empty(4, k, n, device=alpha.device, dtype=torch.float32)
+    at, step = outs.data_ptr(), 4 * k * n
+    _run("ema_coeffs_bwd", alpha, _lib.lib().mega_ema_coeffs_bwd, a.data_ptr(), d.data_ptr(), b.data_ptr(), dp.data_ptr(),
+         dq.data_ptr(), dg.data_ptr(), k, n, at, at + step, at + 2 * step, at + 3 * step)
+    da, dd, db, dgm = outs.to(dtype).unbind(0)
+    return da.unsqueeze(-1), dd.unsqueeze(-1), db.unsqueeze(-1), dgm
 
 
 # --------------------------------------------------------------------- complex EMA
@@ -632,9 +635,8 @@ def cema_coeffs(alpha, delta, theta, gamma):
     p = torch.empty(k, n, device=alpha.device, dtype=torch.float32)
     q = torch.empty(k, n, 2, device=alpha.device, dtype=torch.float32)
     g = torch.empty_like(q)
-    with torch.cuda.device(alpha.device):
-        _lib.check(_lib.lib().mega_cema_coeffs(*[a.data_ptr() for a in args], _dt(args[0]), k, n,
-                                               p.data_ptr(), q.data_ptr(), g.data_ptr(), _stream()), "cema_coeffs")
+    _run("cema_coeffs", alpha, _lib.lib().mega_cema_coeffs, *[a.data_ptr() for a in args], _dt(args[0]), k, n,
+         p.data_ptr(), q.data_ptr(), g.data_ptr())
     return p, torch.view_as_complex(q), torch.view_as_complex(g)
 
 
@@ -643,9 +645,7 @@ def _c64(t):
     if t is None:
         return None
     t = t.detach()
-    if not t.is_complex():
-        t = t.to(torch.complex64)
-    elif t.dtype != torch.complex64:
+    if t.dtype is not torch.complex64:
         t = t.to(torch.complex64)
     return torch.view_as_real(t.contiguous())
 
@@ -656,9 +656,8 @@ def cema_kernel(p, q, g, length):
     p, q, g = _f32c(p), _c64(q), _c64(g)
     k, n = p.shape
     out = torch.empty(k, length, device=p.device, dtype=torch.float32)
-    with torch.cuda.device(p.device):
-        _lib.check(_lib.lib().mega_cema_kernel(p.data_ptr(), q.data_ptr(), g.data_ptr(), k, n, length,
-                                               out.data_ptr(), _stream()), "cema_kernel")
+    _run("cema_kernel", p, _lib.lib().mega_cema_kernel, p.data_ptr(), q.data_ptr(), g.data_ptr(), k, n, length,
+         out.data_ptr())
     return out
 
 
@@ -678,11 +677,9 @@ def cema_forward(x, p, q, g, omega, padding_mask=None, h_in=None, want_state=Fal
     h_out = torch.empty(bsz, dim, n, 2, device=x.device, dtype=torch.float32) if want_state else None
     flags = (EMA_BIDIRECTIONAL if bidirectional else 0) | (0 if shift else EMA_NO_SHIFT) | (EMA_SILU if silu else 0)
     trunc = 0 if truncation is None or truncation < 1 else int(truncation)
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.lib().mega_cema_fwd(
-            x.data_ptr(), out.data_ptr(), _dt(x), bsz, dim, length, *x.stride(), *out.stride(),
-            p.data_ptr(), q.data_ptr(), g.data_ptr(), omega.data_ptr(), n,
-            _ptr(mask), _ptr(h_in), _ptr(h_out), flags, trunc, _stream()), "cema_fwd")
+    _run("cema_fwd", x, _lib.lib().mega_cema_fwd, x.data_ptr(), out.data_ptr(), _dt(x), bsz, dim, length,
+         *x.stride(), *out.stride(), p.data_ptr(), q.data_ptr(), g.data_ptr(), omega.data_ptr(), n, _ptr(mask),
+         _ptr(h_in), _ptr(h_out), flags, trunc)
     return (out, torch.view_as_complex(h_out)) if want_state else out
 
 
@@ -697,10 +694,8 @@ def cema_step(x, p, q, g, omega, h=None, silu=False):
     h = _c64(h)
     h_out = torch.empty(bsz, dim, n, 2, device=x.device, dtype=torch.float32)
     y = torch.empty_like(x2)
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.lib().mega_cema_step(x2.data_ptr(), y.data_ptr(), _dt(x2), bsz, dim, p.data_ptr(),
-                                             q.data_ptr(), g.data_ptr(), omega.data_ptr(), n, _ptr(h),
-                                             h_out.data_ptr(), EMA_SILU if silu else 0, _stream()), "cema_step")
+    _run("cema_step", x, _lib.lib().mega_cema_step, x2.data_ptr(), y.data_ptr(), _dt(x2), bsz, dim, p.data_ptr(),
+         q.data_ptr(), g.data_ptr(), omega.data_ptr(), n, _ptr(h), h_out.data_ptr(), EMA_SILU if silu else 0)
     return y.view(shape), torch.view_as_complex(h_out)
 
 
@@ -720,30 +715,24 @@ def cema_backward(dy, x, p, q, g, omega, padding_mask=None, bidirectional=False,
     dg = torch.empty_like(g)
     dom = torch.empty(dim, device=x.device, dtype=torch.float32)
     flags = (EMA_BIDIRECTIONAL if bidirectional else 0) | (0 if shift else EMA_NO_SHIFT)
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.lib().mega_cema_bwd(
-            dy.data_ptr(), x.data_ptr(), dx.data_ptr(), _dt(x), bsz, dim, length, *dy.stride(), *x.stride(),
-            *dx.stride(), p.data_ptr(), q.data_ptr(), g.data_ptr(), omega.data_ptr(), n, _ptr(mask), flags,
-            _trunc(truncation), dp.data_ptr(), dq.data_ptr(), dg.data_ptr(), dom.data_ptr(), _stream()), "cema_bwd")
+    _run("cema_bwd", x, _lib.lib().mega_cema_bwd, dy.data_ptr(), x.data_ptr(), dx.data_ptr(), _dt(x), bsz, dim,
+         length, *dy.stride(), *x.stride(), *dx.stride(), p.data_ptr(), q.data_ptr(), g.data_ptr(), omega.data_ptr(),
+         n, _ptr(mask), flags, _trunc(truncation), dp.data_ptr(), dq.data_ptr(), dg.data_ptr(), dom.data_ptr())
     return dx, dp, torch.view_as_complex(dq), torch.view_as_complex(dg), dom
 
 
-def cema_coeffs_bwd(alpha, delta, theta, q, dp, dq, dg):
-    """(dalpha, ddelta (K, N, 1), dtheta (K, 1, 1), dgamma (K, N, 2)) from the coefficient gradients."""
+def cema_coeffs_bwd(alpha, delta, theta, q, dp, dq, dg, dtype=torch.float32):
+    """(dalpha, ddelta (K, N, 1), dtheta (K, 1, 1), dgamma (K, N, 2)) in ``dtype`` from the coefficient gradients."""
     _cuda(alpha, delta, theta, q, dp, dq, dg)
     k, n = alpha.shape[0], alpha.shape[1]
     a, d, t = _f32c(alpha).view(k, n), _f32c(delta).view(k, n), _f32c(theta).view(k)
     q, dp, dq, dg = _c64(q), _f32c(dp), _c64(dq), _c64(dg)
-    da = torch.empty(k, n, device=alpha.device, dtype=torch.float32)
-    dd = torch.empty_like(da)
-    dt = torch.empty(k, device=alpha.device, dtype=torch.float32)
-    dgm = torch.empty(k, n, 2, device=alpha.device, dtype=torch.float32)
-    with torch.cuda.device(alpha.device):
-        _lib.check(_lib.lib().mega_cema_coeffs_bwd(a.data_ptr(), d.data_ptr(), t.data_ptr(), q.data_ptr(),
-                                                   dp.data_ptr(), dq.data_ptr(), dg.data_ptr(), k, n, da.data_ptr(),
-                                                   dd.data_ptr(), dt.data_ptr(), dgm.data_ptr(), _stream()),
-                   "cema_coeffs_bwd")
-    return da.unsqueeze(-1), dd.unsqueeze(-1), dt.view(k, 1, 1), dgm
+    outs = torch.empty(4 * k * n + k, device=alpha.device, dtype=torch.float32)
+    at, step = outs.data_ptr(), 4 * k * n
+    _run("cema_coeffs_bwd", alpha, _lib.lib().mega_cema_coeffs_bwd, a.data_ptr(), d.data_ptr(), t.data_ptr(), q.data_ptr(),
+         dp.data_ptr(), dq.data_ptr(), dg.data_ptr(), k, n, at, at + step, at + 4 * step, at + 2 * step)
+    da, dd, dgm, dt = torch.split(outs.to(dtype), (k * n, k * n, 2 * k * n, k))
+    return da.view(k, n, 1), dd.view(k, n, 1), dt.view(k, 1, 1), dgm.view(k, n, 2)
 
 
 # ----------------------------------------------------------------------- attention
@@ -755,9 +744,8 @@ def attention_softmax_fwd(x, causal=True):
     outer, inner = xc.shape[-2], xc.shape[-1]
     batch = xc.numel() // (outer * inner)
     y = torch.empty_like(xc)
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.lib().mega_attention_softmax_fwd(xc.data_ptr(), y.data_ptr(), _dt(xc), batch, outer, inner,
-                                                         1 if causal else 0, _stream()), "attention_softmax_fwd")
+    _run("attention_softmax_fwd", x, _lib.lib().mega_attention_softmax_fwd, xc.data_ptr(), y.data_ptr(), _dt(xc),
+         batch, outer, inner, 1 if causal else 0)
     return y
 
 
@@ -769,10 +757,9 @@ def attention_dropkey_softmax_fwd(x, dropout, causal=True, seed=0, offset=0):
     outer, inner = xc.shape[-2], xc.shape[-1]
     batch = xc.numel() // (outer * inner)
     y = torch.empty_like(xc)
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.lib().mega_attention_dropkey_softmax_fwd(
-            xc.data_ptr(), y.data_ptr(), _dt(xc), batch, outer, inner, 1 if causal else 0, float(dropout),
-            int(seed) & 0xFFFFFFFFFFFFFFFF, int(offset) & 0xFFFFFFFFFFFFFFFF, _stream()), "attention_dropkey_softmax_fwd")
+    _run("attention_dropkey_softmax_fwd", x, _lib.lib().mega_attention_dropkey_softmax_fwd, xc.data_ptr(),
+         y.data_ptr(), _dt(xc), batch, outer, inner, 1 if causal else 0, float(dropout),
+         int(seed) & 0xFFFFFFFFFFFFFFFF, int(offset) & 0xFFFFFFFFFFFFFFFF)
     return y
 
 
@@ -784,10 +771,8 @@ def attention_softmax_bwd(dy, y, causal=True):
     outer, inner = yc.shape[-2], yc.shape[-1]
     batch = yc.numel() // (outer * inner)
     dx = torch.empty_like(yc)
-    with torch.cuda.device(y.device):
-        _lib.check(_lib.lib().mega_attention_softmax_bwd(dyc.data_ptr(), yc.data_ptr(), dx.data_ptr(), _dt(yc), batch,
-                                                         outer, inner, 1 if causal else 0, _stream()),
-                   "attention_softmax_bwd")
+    _run("attention_softmax_bwd", y, _lib.lib().mega_attention_softmax_bwd, dyc.data_ptr(), yc.data_ptr(),
+         dx.data_ptr(), _dt(yc), batch, outer, inner, 1 if causal else 0)
     return dx
 
 
@@ -798,16 +783,12 @@ def attention_bias_softmax_fwd(x, bias, padding_mask=None):
     xc = x.contiguous()
     b = bias.to(xc.dtype).contiguous()
     y = torch.empty_like(xc)
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.lib().mega_attention_bias_softmax_fwd(
-            xc.data_ptr(), y.data_ptr(), b.data_ptr(), (b.shape[0] + 1) // 2, _ptr(padding_mask), _dt(xc), xc.shape[0],
-            xc.shape[1], xc.shape[2], _stream()), "attention_bias_softmax_fwd")
+    _run("attention_bias_softmax_fwd", x, _lib.lib().mega_attention_bias_softmax_fwd, xc.data_ptr(), y.data_ptr(),
+         b.data_ptr(), (b.shape[0] + 1) // 2, _ptr(padding_mask), _dt(xc), xc.shape[0], xc.shape[1], xc.shape[2])
     return y
 
 
 def attention_bias_grad(ds, dbias):
     """Adds the sums of ds (batch, rows, cols) along its diagonals to dbias (2 span - 1) fp32."""
-    with torch.cuda.device(ds.device):
-        _lib.check(_lib.lib().mega_attention_bias_grad(ds.data_ptr(), dbias.data_ptr(), (dbias.shape[0] + 1) // 2, _dt(ds),
-                                                       ds.shape[0], ds.shape[1], ds.shape[2], _stream()),
-                   "attention_bias_grad")
+    _run("attention_bias_grad", ds, _lib.lib().mega_attention_bias_grad, ds.data_ptr(), dbias.data_ptr(),
+         (dbias.shape[0] + 1) // 2, _dt(ds), ds.shape[0], ds.shape[1], ds.shape[2])

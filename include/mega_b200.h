@@ -308,6 +308,20 @@ MEGA_API int mega_gate_qk_rotary(const void* z, int64_t ld_z, const float* gamma
                         int dtype, int64_t rows, int cols, double eps, mega_stream_t stream);
 
 /*
+ * A norm module's parameters (in `dtype`) as the entry points take them, in one launch: gamma = weight + 1, beta (D)
+ * fp32; with B > 0 also its priors as the running statistics of B sequences: count (B), mean = prior_mean, var =
+ * exp(prior_logv), (B, G).  mega_norm_finish: the way back for gradients, in `dtype`: dweight, dbias (D), and with
+ * B > 0 dprior_mean, dprior_logv (G), summed over the batch.
+ * Replaces: norm_layer/timestep_norm.py:110-139 and sequence_norm.py:66-72 around the operators.
+ */
+MEGA_API int mega_norm_prepare(const int64_t* prior_count, const void* prior_mean, const void* prior_logv, const void* weight,
+                      const void* bias, int dtype, int B, int G, int D, int64_t* count, float* mean, float* var,
+                      float* gamma, float* beta, mega_stream_t stream);
+MEGA_API int mega_norm_finish(const float* dprev_mean, const float* dprev_var, const void* prior_logv, const float* dgamma,
+                     const float* dbeta, int dtype, int B, int G, int D, void* dprior_mean, void* dprior_logv,
+                     void* dweight, void* dbias, mega_stream_t stream);
+
+/*
  * ---- Training: forward with saved statistics, and backward ---------------------------------
  *
  * mega_timestep_norm_fwd_train: mega_timestep_norm_fwd that also writes the per-step statistics
