@@ -4,10 +4,12 @@ There is no CPU or PyTorch fallback: if the shared library is missing, loading r
 every op raises when handed a non-CUDA tensor.
 """
 import ctypes
+import importlib.util
 import os
 
 _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "libmega_b200.so")
+HOST_PATH = os.path.join(_PKG, "_mega_host.so")
 
 c_p = ctypes.c_void_p
 c_i = ctypes.c_int
@@ -96,10 +98,28 @@ OTHER = {
 }
 
 _lib = None
+_host = None
 
 
 class MegaError(RuntimeError):
     pass
+
+
+def host():
+    """The native host side (host/host.cpp): operators on torch tensors and the training path's autograd Functions."""
+    global _host
+    if _host is None:
+        lib()
+        if not os.path.exists(HOST_PATH):
+            raise ImportError("_mega_host.so is missing at %s: build it with `python fairseq-apollo_b200/build.py` "
+                              "(there is no fallback)" % HOST_PATH)
+        import torch  # noqa: F401 - the extension's symbols come from torch's libraries
+        spec = importlib.util.spec_from_file_location("_mega_host", HOST_PATH)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        mod.set_error(MegaError)
+        _host = mod
+    return _host
 
 
 def lib():

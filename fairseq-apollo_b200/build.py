@@ -1,4 +1,5 @@
-"""Builds libmega_b200.so (the C-ABI CUDA library) in-tree with nvcc for sm_100a.
+"""Builds libmega_b200.so (the C-ABI CUDA library) in-tree with nvcc for sm_100a, and _mega_host.so (the native host
+side, a torch extension over it) with g++.
 
     python fairseq-apollo_b200/build.py [--force] [--verbose]
 
@@ -17,6 +18,8 @@ ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(PKG, "build")
 LIB = os.path.join(PKG, "libmega_b200.so")
+HOST = os.path.join(PKG, "_mega_host.so")
+HOST_SRC = os.path.join(PKG, "host", "host.cpp")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC",
@@ -46,7 +49,34 @@ def newest_dep():
     return max(os.path.getmtime(d) for d in deps)
 
 
+def build_host(force=False):
+    """The native host side, a torch extension linked against the library next to it."""
+    header = os.path.join(ROOT, "include", "mega_b200.h")
+    if not force and os.path.exists(HOST) and os.path.getmtime(HOST) >= max(os.path.getmtime(HOST_SRC), os.path.getmtime(header)):
+        return HOST
+    import sysconfig
+    import torch
+    base = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(nvcc()))
+    tlib = os.path.join(base, "lib")
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w",
+           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI), "-DTORCH_API_INCLUDE_EXTENSION_H",
+           "-DTORCH_EXTENSION_NAME=_mega_host", "-I", os.path.join(base, "include"),
+           "-I", os.path.join(base, "include", "torch", "csrc", "api", "include"), "-I", os.path.join(cuda, "include"),
+           "-I", sysconfig.get_paths()["include"], "-I", os.path.join(ROOT, "include"), HOST_SRC, "-o", HOST,
+           "-L", PKG, "-lmega_b200", "-Wl,-rpath,$ORIGIN", "-L", tlib, "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu",
+           "-ltorch_cuda", "-ltorch_python", "-Wl,-rpath," + tlib]
+    subprocess.run(cmd, check=True)
+    return HOST
+
+
 def build(force=False, verbose=False):
+    build_lib(force, verbose)
+    build_host(force)
+    return LIB
+
+
+def build_lib(force=False, verbose=False):
     if not force and os.path.exists(LIB) and os.path.getmtime(LIB) >= newest_dep():
         return LIB
     os.makedirs(OBJ, exist_ok=True)

@@ -557,10 +557,7 @@ extern "C" int mega_ema_bwd(const void* dy, const void* x, void* dx, int dtype, 
   if (!aligned_to(dy, es) || !aligned_to(x, es) || !aligned_to(dx, es)) return MEGA_ERR_ALIGN;
   const size_t K = (size_t)(bidir ? 2 : 1) * D;
   cudaStream_t s = (cudaStream_t)stream;
-  if (cudaMemsetAsync(dp, 0, K * N * sizeof(float), s) != cudaSuccess ||
-      cudaMemsetAsync(dq, 0, K * N * sizeof(float), s) != cudaSuccess ||
-      cudaMemsetAsync(dgamma_hat, 0, K * N * sizeof(float), s) != cudaSuccess ||
-      cudaMemsetAsync(domega, 0, (size_t)D * sizeof(float), s) != cudaSuccess)
+  if (!zero_arrays(s, {{dp, K * N}, {dq, K * N}, {dgamma_hat, K * N}, {domega, (size_t)D}}))
     return check_launch("ema_bwd(memset)");
   if (!trunc && !h_in && !dh_out && !dh_in && dx != dy && dx != x) {
     ScanArgs ca{};
@@ -632,8 +629,7 @@ extern "C" int mega_timestep_norm_bwd(const void* dy, const void* x, void* dx, i
   const size_t es = elem_size(dtype);
   if (!aligned_to(dy, es) || !aligned_to(x, es) || !aligned_to(dx, es)) return MEGA_ERR_ALIGN;
   cudaStream_t s = (cudaStream_t)stream;
-  if (cudaMemsetAsync(dgamma, 0, (size_t)D * sizeof(float), s) != cudaSuccess ||
-      cudaMemsetAsync(dbeta, 0, (size_t)D * sizeof(float), s) != cudaSuccess)
+  if (!zero_arrays(s, {{dgamma, (size_t)D}, {dbeta, (size_t)D}}))
     return check_launch("timestep_norm_bwd(memset)");
   TsnBwdArgs a{};
   a.dy = dy; a.x = x; a.dx = dx; a.B = B; a.L = L; a.D = D; a.G = G;
@@ -686,8 +682,7 @@ extern "C" int mega_timestep_norm_bwd_stats(const void* dy, const void* x, void*
   na.prev_count = (const long long*)prev_count; na.prev_mean = prev_mean; na.prev_var = prev_var; na.gamma = gamma;
   na.mask = pad_mask; na.eps = (float)eps; na.dmean = dmean; na.dvar = dvar;
   na.dprev_mean = dprev_mean; na.dprev_var = dprev_var; na.dgamma = dgamma; na.dbeta = dbeta;
-  if (cudaMemsetAsync(dgamma, 0, (size_t)D * sizeof(float), s) != cudaSuccess ||
-      cudaMemsetAsync(dbeta, 0, (size_t)D * sizeof(float), s) != cudaSuccess)
+  if (!zero_arrays(s, {{dgamma, (size_t)D}, {dbeta, (size_t)D}}))
     return check_launch("timestep_norm_bwd_stats(memset)");
   if (!scan_norm_bwd_try(dtype, na, xsd, dsd, gsd, s)) return MEGA_ERR_UNSUPPORTED;
   return check_launch("timestep_norm_bwd_stats");
@@ -707,8 +702,7 @@ extern "C" int mega_sequence_norm_bwd(const void* dy, const void* x, void* dx, i
   const size_t es = elem_size(dtype);
   if (!aligned_to(dy, es) || !aligned_to(x, es) || !aligned_to(dx, es)) return MEGA_ERR_ALIGN;
   cudaStream_t s = (cudaStream_t)stream;
-  if (cudaMemsetAsync(dgamma, 0, (size_t)D * sizeof(float), s) != cudaSuccess ||
-      cudaMemsetAsync(dbeta, 0, (size_t)D * sizeof(float), s) != cudaSuccess)
+  if (!zero_arrays(s, {{dgamma, (size_t)D}, {dbeta, (size_t)D}}))
     return check_launch("sequence_norm_bwd(memset)");
   SqnBwdArgs a{};
   a.dy = dy; a.x = x; a.dx = dx; a.B = B; a.D = D; a.L = L;

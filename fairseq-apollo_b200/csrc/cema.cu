@@ -800,10 +800,7 @@ extern "C" int mega_cema_bwd(const void* dy, const void* x, void* dx, int dtype,
   const bool bidir = (flags & MEGA_EMA_BIDIRECTIONAL) != 0;
   const size_t K = (size_t)(bidir ? 2 : 1) * D;
   cudaStream_t s = (cudaStream_t)stream;
-  if (cudaMemsetAsync(dp, 0, K * N * sizeof(float), s) != cudaSuccess ||
-      cudaMemsetAsync(dq, 0, K * N * 2 * sizeof(float), s) != cudaSuccess ||
-      cudaMemsetAsync(dgamma_hat, 0, K * N * 2 * sizeof(float), s) != cudaSuccess ||
-      cudaMemsetAsync(domega, 0, (size_t)D * sizeof(float), s) != cudaSuccess)
+  if (!zero_arrays(s, {{dp, K * N}, {dq, 2 * K * N}, {dgamma_hat, 2 * K * N}, {domega, (size_t)D}}))
     return check_launch("cema_bwd(memset)");
   if (!trunc && dx != dy && dx != x) {
     ScanArgs ca{};

@@ -7,6 +7,8 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <initializer_list>
+#include <utility>
 
 #include "mega_b200.h"
 
@@ -41,6 +43,22 @@ static inline void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_
   kernel<<<grid, block, smem, (cudaStream_t)stream>>>(static_cast<KArgs>(args)...);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   g_last_kernel.store("other", std::memory_order_relaxed);
+}
+
+// Zeroes `n` consecutive arrays of floats on the stream, as one piece where they lie side by side.
+static inline bool zero_arrays(cudaStream_t s, std::initializer_list<std::pair<float*, size_t>> arrays) {
+  float* at = nullptr;
+  size_t len = 0;
+  for (const auto& a : arrays) {
+    if (at && at + len == a.first) {
+      len += a.second;
+      continue;
+    }
+    if (at && cudaMemsetAsync(at, 0, len * sizeof(float), s) != cudaSuccess) return false;
+    at = a.first;
+    len = a.second;
+  }
+  return !at || cudaMemsetAsync(at, 0, len * sizeof(float), s) == cudaSuccess;
 }
 
 // ---- element I/O ------------------------------------------------------------

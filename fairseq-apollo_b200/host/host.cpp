@@ -1,0 +1,791 @@
+// Host side of the package in native code: operators on torch tensors and the autograd Functions of the training
+// path, each a few allocations and calls into libmega_b200.so on the current stream.
+//
+// At the small shapes of the path the host is what a call costs: an operator through Python (checks, allocations,
+// thirty converted arguments) takes 20 - 40 us, a Python autograd Function as much again each way, against 3 - 10 us
+// of device time per launch.  Here an operator takes 3 - 5 us and the backward of a training pass runs in the
+// autograd engine without the interpreter.
+//
+// fairseq/modules/norm_layer/{timestep_norm,sequence_norm}.py, fairseq/modules/fused_ops/*.py and
+// fairseq/modules/moving_average_gated_attention.py:317-414 of the reference are what the Functions stand in for.
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/extension.h>
+
+#include <tuple>
+#include <vector>
+
+#include "mega_b200.h"
+
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+using OptTensor = std::optional<Tensor>;
+
+namespace {
+
+PyObject* g_error = nullptr;   // the package's MegaError
+
+void check(int status, const char* what) {
+  if (status == MEGA_OK) return;
+  std::string msg = std::string(what) + ": " + mega_status_string(status);
+  if (status == MEGA_ERR_CUDA) msg += std::string(" (") + mega_last_cuda_error() + ")";
+  if (g_error && PyGILState_Check()) {
+    PyErr_SetString(g_error, msg.c_str());
+    throw py::error_already_set();
+  }
+  throw std::runtime_error(msg);   // (a backward in the autograd engine's threads)
+}
+
+void on_cuda(const Tensor& t) {
+  if (t.defined() && !t.is_cuda())
+    throw std::runtime_error("mega_b200 ops run on CUDA tensors only (there is no CPU fallback)");
+}
+template <typename... Ts>
+void on_cuda(const Tensor& t, const Ts&... rest) {
+  on_cuda(t);
+  on_cuda(rest...);
+}
+
+// device of the call and its current stream
+struct Where {
+  c10::cuda::CUDAGuard guard;
+  void* stream;
+  explicit Where(const Tensor& t) : guard(t.device()), stream(at::cuda::getCurrentCUDAStream(t.get_device()).stream()) {}
+};
+
+int dtype_of(const Tensor& t) {
+  switch (t.scalar_type()) {
+    case at::kFloat: return MEGA_F32;
+    case at::kBFloat16: return MEGA_BF16;
+    case at::kHalf: return MEGA_F16;
+    default: throw py::type_error("mega_b200 supports float32, bfloat16 and float16 activations");
+  }
+}
+
+Tensor none() { return Tensor(); }
+Tensor given(const OptTensor& t) { return t.has_value() ? *t : Tensor(); }
+
+template <typename T = void>
+T* ptr(const Tensor& t) {
+  return t.defined() ? static_cast<T*>(t.data_ptr()) : nullptr;
+}
+float* fptr(const Tensor& t) { return ptr<float>(t); }
+
+// fp32, contiguous (parameters, statistics, states are small)
+Tensor f32c(const Tensor& t) {
+  if (!t.defined() || (t.scalar_type() == at::kFloat && t.is_contiguous())) return t;
+  return t.detach().to(at::kFloat).contiguous();
+}
+// complex64 as its interleaved floats
+Tensor c64(const Tensor& t) {
+  if (!t.defined()) return t;
+  Tensor d = t.detach();
+  if (d.scalar_type() == at::kFloat) return d.contiguous();   // already interleaved
+  if (d.scalar_type() != at::kComplexFloat) d = d.to(at::kComplexFloat);
+  return at::view_as_real(d.contiguous());
+}
+
+Tensor mask_u8(const Tensor& mask, int64_t bsz, int64_t length) {
+  if (!mask.defined()) return mask;
+  if (mask.dim() != 2 || mask.size(0) != bsz || mask.size(1) != length)
+    throw py::value_error("padding_mask must be (batch, length) = (" + std::to_string(bsz) + ", " + std::to_string(length) + ")");
+  return mask.scalar_type() == at::kBool ? mask.contiguous() : mask.ne(0).contiguous();
+}
+
+// uninitialised, strided like t (contiguous when t's strides leave gaps)
+Tensor like(const Tensor& t) {
+  if (t.is_contiguous()) return at::empty(t.sizes(), t.options().requires_grad(false));
+  if (t.is_non_overlapping_and_dense()) return at::empty_strided(t.sizes(), t.strides(), t.options().requires_grad(false));
+  return at::empty(t.sizes(), t.options().requires_grad(false));
+}
+Tensor floats(at::IntArrayRef size, const Tensor& t) {
+  return at::empty(size, at::TensorOptions().dtype(at::kFloat).device(t.device()));
+}
+Tensor counts(int64_t n, const Tensor& t) { return at::empty({n}, at::TensorOptions().dtype(at::kLong).device(t.device())); }
+
+#define STRIDES3(t) (t).stride(0), (t).stride(1), (t).stride(2)
+
+// ------------------------------------------------------------------------------------------------ EMA
+struct Coeffs {
+  Tensor p, q, g;
+};
+
+Coeffs coeffs(const Tensor& alpha, const Tensor& delta, const Tensor& third, const Tensor& gamma, bool cplx, const Where& w) {
+  const int64_t k = alpha.size(0), n = alpha.size(1);
+  const auto st = alpha.scalar_type();
+  auto prep = [&](const Tensor& t) { return (t.scalar_type() == st ? t.detach() : t.detach().to(st)).contiguous(); };
+  const Tensor a = prep(alpha), d = prep(delta), t = prep(third), g = prep(gamma);
+  Tensor f = floats({(cplx ? 5 : 3) * k * n}, alpha);
+  Coeffs c;
+  c.p = f.narrow(0, 0, k * n).view({k, n});
+  if (cplx) {
+    c.q = f.narrow(0, k * n, 2 * k * n).view({k, n, 2});
+    c.g = f.narrow(0, 3 * k * n, 2 * k * n).view({k, n, 2});
+    check(mega_cema_coeffs(a.data_ptr(), d.data_ptr(), t.data_ptr(), g.data_ptr(), dtype_of(a), (int)k, (int)n, fptr(c.p),
+                           fptr(c.q), fptr(c.g), w.stream), "cema_coeffs");
+  } else {
+    c.q = f.narrow(0, k * n, k * n).view({k, n});
+    c.g = f.narrow(0, 2 * k * n, k * n).view({k, n});
+    check(mega_ema_coeffs(a.data_ptr(), d.data_ptr(), t.data_ptr(), g.data_ptr(), dtype_of(a), (int)k, (int)n, fptr(c.p),
+                          fptr(c.q), fptr(c.g), w.stream), "ema_coeffs");
+  }
+  return c;
+}
+
+// x (B, D, L); p (K, N), q / g (K, N) or interleaved (K, N, 2); states likewise
+void run_ema(const Tensor& x, const Tensor& y, const Tensor& p, const Tensor& q, const Tensor& g, const Tensor& omega,
+             const Tensor& mask, const Tensor& h_in, const Tensor& h_out, unsigned flags, int trunc, bool cplx, const Where& w) {
+  const int B = (int)x.size(0), D = (int)x.size(1), L = (int)x.size(2), N = (int)p.size(1);
+  auto fn = cplx ? mega_cema_fwd : mega_ema_fwd;
+  check(fn(x.data_ptr(), y.data_ptr(), dtype_of(x), B, D, L, STRIDES3(x), STRIDES3(y), fptr(p), fptr(q), fptr(g), fptr(omega),
+           N, ptr<uint8_t>(mask), fptr(h_in), fptr(h_out), flags, trunc, w.stream), cplx ? "cema_fwd" : "ema_fwd");
+}
+
+std::tuple<Tensor, OptTensor> ema_forward(const Tensor& x, const Tensor& p_, const Tensor& q_, const Tensor& g_,
+                                          const Tensor& omega_, const OptTensor& mask_, const OptTensor& h_in_, bool want_state,
+                                          int64_t flags, int64_t trunc, bool cplx, const OptTensor& out_) {
+  on_cuda(x, p_, q_, g_, omega_, given(mask_), given(h_in_));
+  const Where w(x);
+  const int64_t bsz = x.size(0), dim = x.size(1);
+  const Tensor p = f32c(p_), q = cplx ? c64(q_) : f32c(q_), g = cplx ? c64(g_) : f32c(g_), omega = f32c(omega_);
+  const int64_t n = p.size(1);
+  if (p.size(0) != ((flags & MEGA_EMA_BIDIRECTIONAL) ? 2 * dim : dim))
+    throw py::value_error("coefficient rows " + std::to_string(p.size(0)) + " do not match embed_dim " + std::to_string(dim));
+  const Tensor mask = mask_u8(given(mask_), bsz, x.size(2));
+  const Tensor h_in = cplx ? c64(given(h_in_)) : f32c(given(h_in_));
+  const Tensor y = out_.has_value() ? *out_ : like(x);
+  Tensor h_out = want_state ? (cplx ? floats({bsz, dim, n, 2}, x) : floats({bsz, dim, n}, x)) : Tensor();
+  run_ema(x, y, p, q, g, omega, mask, h_in, h_out, (unsigned)flags, (int)trunc, cplx, w);
+  if (!want_state) return {y, std::nullopt};
+  return {y, cplx ? at::view_as_complex(h_out) : h_out};
+}
+
+// y = silu(a) / its gradient over a dense tensor's memory
+bool rows_of(const Tensor& t, int64_t cols, int64_t& rows) {
+  const int64_t vec = 16 / t.element_size();
+  if (!t.is_non_overlapping_and_dense() || t.numel() % cols != 0 || cols % vec != 0) return false;
+  rows = t.numel() / cols;
+  return true;
+}
+
+class EmaFn : public torch::autograd::Function<EmaFn> {
+ public:
+  static Tensor forward(AutogradContext* ctx, Tensor x, Tensor alpha, Tensor delta, Tensor third, Tensor gamma, Tensor omega,
+                        OptTensor mask_, int64_t flags, int64_t trunc, bool cplx, bool silu) {
+    on_cuda(x, alpha, omega, given(mask_));
+    const Where w(x);
+    const Tensor mask = mask_u8(given(mask_), x.size(0), x.size(2));
+    const Coeffs c = coeffs(alpha, delta, third, gamma, cplx, w);
+    Tensor y = like(x);
+    run_ema(x, y, c.p, c.q, c.g, f32c(omega), mask, none(), none(), (unsigned)flags, (int)trunc, cplx, w);
+    Tensor out = y;
+    if (silu) {
+      int64_t rows;
+      if (rows_of(y, x.size(1), rows)) {
+        out = like(y);
+        check(mega_gate_silu(y.data_ptr(), x.size(1), nullptr, 0, out.data_ptr(), x.size(1), dtype_of(y), rows, (int)x.size(1),
+                             w.stream), "gate_silu");
+      } else {
+        out = at::silu(y);
+      }
+    }
+    ctx->save_for_backward({x, alpha, delta, third, omega, mask, c.p, c.q, c.g, silu ? y : Tensor()});
+    ctx->saved_data["flags"] = flags;
+    ctx->saved_data["trunc"] = trunc;
+    ctx->saved_data["cplx"] = cplx;
+    ctx->saved_data["gamma"] = (int64_t)gamma.scalar_type();
+    return out;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto s = ctx->get_saved_variables();
+    const Tensor &x = s[0], &alpha = s[1], &delta = s[2], &third = s[3], &omega = s[4], &mask = s[5], &p = s[6], &q = s[7], &g = s[8],
+                 &y = s[9];
+    const unsigned flags = (unsigned)ctx->saved_data["flags"].toInt();
+    const int trunc = (int)ctx->saved_data["trunc"].toInt();
+    const bool cplx = ctx->saved_data["cplx"].toBool();
+    const auto gamma_type = (at::ScalarType)ctx->saved_data["gamma"].toInt();
+    const Where w(x);
+    Tensor dy = grads[0];
+    if (dy.scalar_type() != x.scalar_type()) dy = dy.to(x.scalar_type());
+    if (y.defined()) {   // through the SiLU, in y's memory order
+      if (dy.strides() != y.strides()) {
+        Tensor t = like(y);
+        t.copy_(dy);
+        dy = t;
+      }
+      int64_t rows;
+      if (rows_of(y, x.size(1), rows)) {
+        Tensor d = like(y);
+        const int64_t c = x.size(1);
+        check(mega_gate_silu_bwd(dy.data_ptr(), c, y.data_ptr(), c, d.data_ptr(), c, nullptr, dtype_of(y), rows, (int)c, w.stream),
+              "gate_silu_bwd");
+        dy = d;
+      } else {
+        dy = at::silu_backward(dy, y);
+      }
+    }
+    const int B = (int)x.size(0), D = (int)x.size(1), L = (int)x.size(2);
+    const int64_t k = p.size(0), n = p.size(1), kn = k * n, m = cplx ? 2 : 1;
+    Tensor dx = like(x);
+    // dp, dq, dgamma_hat and domega in one piece (the library zeroes them together), the raw parameters' behind them
+    const int64_t sums = kn * (1 + 2 * m), raw = cplx ? 4 * kn + k : 4 * kn;
+    Tensor f = floats({sums + D + raw}, x);
+    float* at_ = f.data_ptr<float>();
+    float *dp = at_, *dq = at_ + kn, *dg = at_ + kn * (1 + m), *dom = at_ + sums, *da = dom + D, *dd = da + kn;
+    const Tensor om = f32c(omega);
+    const Tensor a = f32c(alpha), d = f32c(delta), t = f32c(third);
+    if (cplx) {
+      float *dgm = dd + kn, *dt = dgm + 2 * kn;
+      check(mega_cema_bwd(dy.data_ptr(), x.data_ptr(), dx.data_ptr(), dtype_of(x), B, D, L, STRIDES3(dy), STRIDES3(x), STRIDES3(dx),
+                          fptr(p), fptr(q), fptr(g), fptr(om), (int)n, ptr<uint8_t>(mask), flags, trunc, dp, dq, dg, dom, w.stream),
+            "cema_bwd");
+      check(mega_cema_coeffs_bwd(fptr(a), fptr(d), fptr(t), fptr(q), dp, dq, dg, (int)k, (int)n, da, dd, dt, dgm, w.stream),
+            "cema_coeffs_bwd");
+    } else {
+      float *db = dd + kn, *dgm = db + kn;
+      check(mega_ema_bwd(dy.data_ptr(), x.data_ptr(), dx.data_ptr(), dtype_of(x), B, D, L, STRIDES3(dy), STRIDES3(x), STRIDES3(dx),
+                         fptr(p), fptr(q), fptr(g), fptr(om), (int)n, ptr<uint8_t>(mask), nullptr, nullptr, flags, trunc, dp, dq, dg,
+                         dom, nullptr, w.stream), "ema_bwd");
+      check(mega_ema_coeffs_bwd(fptr(a), fptr(d), fptr(t), dp, dq, dg, (int)k, (int)n, da, dd, db, dgm, w.stream), "ema_coeffs_bwd");
+    }
+    Tensor out = f.narrow(0, sums, D + raw);
+    if (alpha.scalar_type() != at::kFloat) out = out.to(alpha.scalar_type());
+    auto part = [&](int64_t from, int64_t count, at::IntArrayRef size, at::ScalarType st) {
+      Tensor v = out.narrow(0, from, count).view(size);
+      return v.scalar_type() == st ? v : v.to(st);
+    };
+    const Tensor g_om = part(0, D, omega.sizes(), omega.scalar_type());
+    const Tensor g_a = part(D, kn, alpha.sizes(), alpha.scalar_type()), g_d = part(D + kn, kn, delta.sizes(), delta.scalar_type());
+    const Tensor g_3 = cplx ? part(D + 4 * kn, k, third.sizes(), third.scalar_type())
+                            : part(D + 2 * kn, kn, third.sizes(), third.scalar_type());
+    const Tensor g_g = cplx ? part(D + 2 * kn, 2 * kn, {k, n, 2}, gamma_type) : part(D + 3 * kn, kn, {k, n}, gamma_type);
+    return {dx, g_a, g_d, g_3, g_g, g_om, Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+Tensor ema_train(const Tensor& x, const Tensor& alpha, const Tensor& delta, const Tensor& third, const Tensor& gamma,
+                 const Tensor& omega, const OptTensor& mask, int64_t flags, int64_t trunc, bool cplx, bool silu) {
+  return EmaFn::apply(x, alpha, delta, third, gamma, omega, mask, flags, trunc, cplx, silu);
+}
+
+// ------------------------------------------------------------------------------------------------ norms
+struct NormParams {
+  Tensor gamma, beta, count, mean, var;
+};
+
+NormParams prepare(const Tensor& weight, const Tensor& bias, const Tensor& pc, const Tensor& pm, const Tensor& pl, int64_t bsz,
+                   const Where& w) {
+  const int64_t d = weight.size(0), g = pm.defined() ? pm.size(0) : 0;
+  const Tensor b = bias.scalar_type() == weight.scalar_type() ? bias : bias.detach().to(weight.scalar_type());
+  Tensor m = pm, l = pl;
+  if (g && m.scalar_type() != weight.scalar_type()) {
+    m = m.detach().to(weight.scalar_type());
+    l = l.detach().to(weight.scalar_type());
+  }
+  Tensor f = floats({2 * d + 2 * bsz * g}, weight);
+  NormParams r;
+  r.gamma = f.narrow(0, 0, d);
+  r.beta = f.narrow(0, d, d);
+  if (g) {
+    r.mean = f.narrow(0, 2 * d, bsz * g).view({bsz, g});
+    r.var = f.narrow(0, 2 * d + bsz * g, bsz * g).view({bsz, g});
+    r.count = counts(bsz, weight);
+  }
+  check(mega_norm_prepare(ptr<int64_t>(pc), ptr(m), ptr(l), weight.data_ptr(), b.data_ptr(), dtype_of(weight),
+                          (int)(g ? bsz : 0), (int)g, (int)d, ptr<int64_t>(r.count), fptr(r.mean), fptr(r.var), fptr(r.gamma),
+                          fptr(r.beta), w.stream), "norm_prepare");
+  return r;
+}
+
+py::tuple norm_prepare(const Tensor& weight, const Tensor& bias, const OptTensor& pc, const OptTensor& pm, const OptTensor& pl,
+                       int64_t bsz) {
+  on_cuda(weight, bias, given(pm));
+  const Where w(weight);
+  const NormParams r = prepare(weight, bias, given(pc), given(pm), given(pl), bsz, w);
+  if (!pm.has_value()) return py::make_tuple(r.gamma, r.beta);
+  return py::make_tuple(r.gamma, r.beta, r.count, r.mean, r.var);
+}
+
+// (dweight, dbias, dprior_mean, dprior_logv) in the parameters' type
+std::vector<Tensor> finish(const Tensor& weight, const Tensor& logv, const float* dgamma, const float* dbeta, const float* dpm,
+                           const float* dpv, int64_t bsz, int64_t g, const Where& w) {
+  const int64_t d = weight.size(0);
+  Tensor out = at::empty({2 * d + 2 * g}, weight.options().requires_grad(false));
+  const Tensor l = g && logv.scalar_type() != weight.scalar_type() ? logv.detach().to(weight.scalar_type()) : logv;
+  char* at_ = static_cast<char*>(out.data_ptr());
+  const int64_t es = out.element_size();
+  check(mega_norm_finish(dpm, dpv, ptr(l), dgamma, dbeta, dtype_of(weight), (int)(g ? bsz : 0), (int)g, (int)d,
+                         g ? at_ + 2 * d * es : nullptr, g ? at_ + (2 * d + g) * es : nullptr, at_, at_ + d * es, w.stream),
+        "norm_finish");
+  std::vector<Tensor> r = {out.narrow(0, 0, d), out.narrow(0, d, d)};
+  if (g) {
+    r.push_back(out.narrow(0, 2 * d, g));
+    r.push_back(out.narrow(0, 2 * d + g, g));
+    if (logv.scalar_type() != weight.scalar_type()) {
+      r[2] = r[2].to(logv.scalar_type());
+      r[3] = r[3].to(logv.scalar_type());
+    }
+  }
+  return r;
+}
+
+bool whole_rows(const Tensor& x) {   // contiguous channels in whole 16-byte pieces
+  const int64_t es = x.element_size();
+  return x.stride(2) == 1 && x.size(2) * es % 16 == 0 && x.stride(0) * es % 16 == 0 && x.stride(1) * es % 16 == 0 &&
+         reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0;
+}
+
+std::tuple<Tensor, Tensor, Tensor, Tensor> timestep_norm_fwd(const Tensor& x, const Tensor& pc_, const Tensor& pm_, const Tensor& pv_,
+                                                             const Tensor& gamma_, const Tensor& beta_, const OptTensor& mask_,
+                                                             double eps, int64_t groups, const OptTensor& out_) {
+  on_cuda(x, pc_, pm_, pv_, gamma_, beta_, given(mask_));
+  const Where w(x);
+  const int64_t bsz = x.size(0), length = x.size(1), dim = x.size(2), g = groups > 0 ? groups : dim;
+  const Tensor pc = pc_.to(at::kLong).contiguous(), pm = f32c(pm_), pv = f32c(pv_), gamma = f32c(gamma_), beta = f32c(beta_);
+  if (pm.dim() != 2 || pm.size(0) != bsz || pm.size(1) != g || pv.sizes() != pm.sizes())
+    throw py::value_error("prev_mean/prev_var must be (batch, groups) = (" + std::to_string(bsz) + ", " + std::to_string(g) + ")");
+  const Tensor mask = mask_u8(given(mask_), bsz, length);
+  const Tensor y = out_.has_value() ? *out_ : like(x);
+  Tensor count = counts(bsz, x), st = floats({2, bsz, g}, x);
+  Tensor mean = st.select(0, 0), var = st.select(0, 1);
+  check(mega_timestep_norm_fwd(x.data_ptr(), y.data_ptr(), dtype_of(x), (int)bsz, (int)length, (int)dim, STRIDES3(x), STRIDES3(y),
+                               ptr<int64_t>(pc), fptr(pm), fptr(pv), fptr(gamma), fptr(beta), ptr<uint8_t>(mask), (int)g, eps,
+                               ptr<int64_t>(count), fptr(mean), fptr(var), w.stream), "timestep_norm_fwd");
+  return {y, count, mean, var};
+}
+
+class TsnFn : public torch::autograd::Function<TsnFn> {
+ public:
+  static Tensor forward(AutogradContext* ctx, Tensor x, Tensor pcount, Tensor pmean, Tensor plogv, Tensor weight, Tensor bias,
+                        OptTensor mask_, int64_t groups, double eps) {
+    on_cuda(x, pmean, weight, given(mask_));
+    const Where w(x);
+    const int64_t bsz = x.size(0), length = x.size(1), dim = x.size(2), g = groups > 0 ? groups : dim;
+    const NormParams r = prepare(weight, bias, pcount, pmean, plogv, bsz, w);
+    const Tensor mask = mask_u8(given(mask_), bsz, length);
+    const bool again = groups <= 0 && whole_rows(x);
+    Tensor y = like(x), count = counts(bsz, x);
+    if (again) {   // the backward takes the statistics again: nothing is kept but the arguments
+      Tensor st = floats({2, bsz, g}, x);
+      check(mega_timestep_norm_fwd(x.data_ptr(), y.data_ptr(), dtype_of(x), (int)bsz, (int)length, (int)dim, STRIDES3(x), STRIDES3(y),
+                                   ptr<int64_t>(r.count), fptr(r.mean), fptr(r.var), fptr(r.gamma), fptr(r.beta),
+                                   ptr<uint8_t>(mask), (int)g, eps, ptr<int64_t>(count), fptr(st), fptr(st) + bsz * g, w.stream),
+            "timestep_norm_fwd");
+      ctx->save_for_backward({x, weight, plogv, r.gamma, mask, r.count, r.mean, r.var});
+    } else {
+      Tensor st = floats({2, bsz, g}, x), cm = floats({bsz, length, g}, x), cr = floats({bsz, length, g}, x);
+      Tensor gm = g != dim ? floats({bsz, length, g}, x) : Tensor();
+      check(mega_timestep_norm_fwd_train(x.data_ptr(), y.data_ptr(), dtype_of(x), (int)bsz, (int)length, (int)dim, STRIDES3(x),
+                                         STRIDES3(y), ptr<int64_t>(r.count), fptr(r.mean), fptr(r.var), fptr(r.gamma),
+                                         fptr(r.beta), ptr<uint8_t>(mask), (int)g, eps, ptr<int64_t>(count), fptr(st),
+                                         fptr(st) + bsz * g, fptr(cm), fptr(cr), fptr(gm), w.stream), "timestep_norm_fwd_train");
+      ctx->save_for_backward({x, weight, plogv, r.gamma, mask, count, r.mean, Tensor(), cm, cr, gm});
+    }
+    ctx->saved_data["again"] = again;
+    ctx->saved_data["g"] = g;
+    ctx->saved_data["eps"] = eps;
+    return y;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto s = ctx->get_saved_variables();
+    const Tensor &x = s[0], &weight = s[1], &plogv = s[2], &gamma = s[3], &mask = s[4];
+    const int64_t g = ctx->saved_data["g"].toInt();
+    const Where w(x);
+    const int64_t bsz = x.size(0), dim = x.size(2);
+    Tensor dy = grads[0];
+    if (dy.scalar_type() != x.scalar_type()) dy = dy.to(x.scalar_type());
+    const bool again = ctx->saved_data["again"].toBool();
+    if (again && !whole_rows(dy)) dy = dy.contiguous();
+    Tensor dx = like(x);
+    Tensor f = floats({2 * dim + 2 * bsz * g}, x);
+    float *dgamma = fptr(f), *dbeta = dgamma + dim, *dpm = dbeta + dim, *dpv = dpm + bsz * g;
+    if (again)
+      check(mega_timestep_norm_bwd_stats(dy.data_ptr(), x.data_ptr(), dx.data_ptr(), dtype_of(x), (int)bsz, (int)x.size(1), (int)dim,
+                                         STRIDES3(dy), STRIDES3(x), STRIDES3(dx), nullptr, nullptr, ptr<int64_t>(s[5]),
+                                         fptr(s[6]), fptr(s[7]), fptr(gamma), ptr<uint8_t>(mask),
+                                         ctx->saved_data["eps"].toDouble(), dpm, dpv, dgamma, dbeta, w.stream),
+            "timestep_norm_bwd_stats");
+    else
+      check(mega_timestep_norm_bwd(dy.data_ptr(), x.data_ptr(), dx.data_ptr(), dtype_of(x), (int)bsz, (int)x.size(1), (int)dim,
+                                   STRIDES3(dy), STRIDES3(x), STRIDES3(dx), nullptr, nullptr, fptr(s[6]), ptr<int64_t>(s[5]),
+                                   fptr(s[8]), fptr(s[9]), fptr(s[10]), fptr(gamma), ptr<uint8_t>(mask), (int)g, dpm, dpv,
+                                   dgamma, dbeta, w.stream), "timestep_norm_bwd");
+    auto r = finish(weight, plogv, dgamma, dbeta, dpm, dpv, bsz, g, w);
+    return {dx, Tensor(), r[2], r[3], r[0], r[1], Tensor(), Tensor(), Tensor()};
+  }
+};
+
+Tensor timestep_norm_train(const Tensor& x, const Tensor& pc, const Tensor& pm, const Tensor& pl, const Tensor& weight,
+                           const Tensor& bias, const OptTensor& mask, int64_t groups, double eps) {
+  return TsnFn::apply(x, pc, pm, pl, weight, bias, mask, groups, eps);
+}
+
+// x (B, D, L), or (B, L, D) with length_last = false
+struct Sqn {
+  int64_t bsz, dim, length, sb, sd, sl;
+};
+Sqn sqn_view(const Tensor& x, bool length_last) {
+  if (length_last) return {x.size(0), x.size(1), x.size(2), x.stride(0), x.stride(1), x.stride(2)};
+  return {x.size(0), x.size(2), x.size(1), x.stride(0), x.stride(2), x.stride(1)};
+}
+
+void run_sqn(const Tensor& x, const Tensor& y, const Tensor& gamma, const Tensor& beta, const Tensor& mask, double eps,
+             bool length_last, int64_t g, const Tensor& count, const Tensor& mean, const Tensor& rstd, const Where& w) {
+  const Sqn a = sqn_view(x, length_last), o = sqn_view(y, length_last);
+  check(mega_sequence_norm_fwd(x.data_ptr(), y.data_ptr(), dtype_of(x), (int)a.bsz, (int)a.dim, (int)a.length, a.sb, a.sd, a.sl, o.sb,
+                               o.sd, o.sl, fptr(gamma), fptr(beta), ptr<uint8_t>(mask), (int)g, eps, ptr<int64_t>(count),
+                               fptr(mean), fptr(rstd), w.stream), "sequence_norm_fwd");
+}
+
+std::tuple<Tensor, Tensor, Tensor, Tensor> sequence_norm_fwd(const Tensor& x, const Tensor& gamma_, const Tensor& beta_,
+                                                             const OptTensor& mask_, double eps, bool length_last, int64_t groups,
+                                                             const OptTensor& out_) {
+  on_cuda(x, gamma_, beta_, given(mask_));
+  const Where w(x);
+  const Sqn a = sqn_view(x, length_last);
+  const int64_t g = groups > 0 ? groups : a.dim;
+  const Tensor mask = mask_u8(given(mask_), a.bsz, a.length);
+  const Tensor y = out_.has_value() ? *out_ : like(x);
+  Tensor count = counts(a.bsz, x), st = floats({2, a.bsz, g}, x);
+  Tensor mean = st.select(0, 0), rstd = st.select(0, 1);
+  run_sqn(x, y, f32c(gamma_), f32c(beta_), mask, eps, length_last, g, count, mean, rstd, w);
+  return {y, count, mean, rstd};
+}
+
+class SqnFn : public torch::autograd::Function<SqnFn> {
+ public:
+  static Tensor forward(AutogradContext* ctx, Tensor x, Tensor weight, Tensor bias, OptTensor mask_, double eps, bool length_last,
+                        int64_t groups) {
+    on_cuda(x, weight, given(mask_));
+    const Where w(x);
+    const Sqn a = sqn_view(x, length_last);
+    const int64_t g = groups > 0 ? groups : a.dim;
+    const NormParams r = prepare(weight, bias, none(), none(), none(), 0, w);
+    const Tensor mask = mask_u8(given(mask_), a.bsz, a.length);
+    Tensor y = like(x), count = counts(a.bsz, x), st = floats({2, a.bsz, g}, x);
+    Tensor mean = st.select(0, 0), rstd = st.select(0, 1);
+    run_sqn(x, y, r.gamma, r.beta, mask, eps, length_last, g, count, mean, rstd, w);
+    ctx->save_for_backward({x, weight, r.gamma, mask, count, mean, rstd});
+    ctx->saved_data["ll"] = length_last;
+    ctx->saved_data["g"] = g;
+    return y;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto s = ctx->get_saved_variables();
+    const Tensor &x = s[0], &weight = s[1];
+    const bool ll = ctx->saved_data["ll"].toBool();
+    const Where w(x);
+    Tensor dy = grads[0];
+    if (dy.scalar_type() != x.scalar_type()) dy = dy.to(x.scalar_type());
+    Tensor dx = like(x);
+    const Sqn a = sqn_view(x, ll), q = sqn_view(dy, ll), o = sqn_view(dx, ll);
+    Tensor f = floats({2 * a.dim}, x);
+    check(mega_sequence_norm_bwd(dy.data_ptr(), x.data_ptr(), dx.data_ptr(), dtype_of(x), (int)a.bsz, (int)a.dim, (int)a.length, q.sb,
+                                 q.sd, q.sl, a.sb, a.sd, a.sl, o.sb, o.sd, o.sl, ptr<int64_t>(s[4]), fptr(s[5]), fptr(s[6]),
+                                 fptr(s[2]), ptr<uint8_t>(s[3]), (int)ctx->saved_data["g"].toInt(), fptr(f), fptr(f) + a.dim,
+                                 w.stream), "sequence_norm_bwd");
+    auto r = finish(weight, none(), fptr(f), fptr(f) + a.dim, nullptr, nullptr, 0, 0, w);
+    return {dx, r[0], r[1], Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+Tensor sequence_norm_train(const Tensor& x, const Tensor& weight, const Tensor& bias, const OptTensor& mask, double eps,
+                           bool length_last, int64_t groups) {
+  return SqnFn::apply(x, weight, bias, mask, eps, length_last, groups);
+}
+
+// ---------------------------------------------------------------------------------------- fused norm -> EMA
+// (y, count, mean, var, h or None, xn or None)
+py::tuple tsn_ema_forward(const Tensor& x, const Tensor& pc_, const Tensor& pm_, const Tensor& pv_, const Tensor& gamma_,
+                          const Tensor& beta_, double eps, const Tensor& p_, const Tensor& q_, const Tensor& g_,
+                          const Tensor& omega_, const OptTensor& mask_, const OptTensor& h_in_, bool want_state, bool silu,
+                          bool want_normed, bool cplx) {
+  on_cuda(x, pc_, pm_, pv_, gamma_, beta_, p_, q_, g_, omega_, given(mask_), given(h_in_));
+  const Where w(x);
+  const int64_t bsz = x.size(0), length = x.size(1), dim = x.size(2);
+  const Tensor pc = pc_.to(at::kLong).contiguous(), pm = f32c(pm_), pv = f32c(pv_), gamma = f32c(gamma_), beta = f32c(beta_);
+  const Tensor p = f32c(p_), q = cplx ? c64(q_) : f32c(q_), g = cplx ? c64(g_) : f32c(g_), omega = f32c(omega_);
+  const Tensor h_in = cplx ? c64(given(h_in_)) : f32c(given(h_in_));
+  const int64_t n = p.size(1);
+  const Tensor mask = mask_u8(given(mask_), bsz, length);
+  Tensor y = like(x), xn = want_normed ? like(y) : Tensor();
+  Tensor count = counts(bsz, x), st = floats({2, bsz, dim}, x);
+  Tensor mean = st.select(0, 0), var = st.select(0, 1);
+  Tensor h_out = want_state ? (cplx ? floats({bsz, dim, n, 2}, x) : floats({bsz, dim, n}, x)) : Tensor();
+  auto fn = cplx ? mega_tsn_cema_fwd : mega_tsn_ema_fwd;
+  check(fn(x.data_ptr(), y.data_ptr(), ptr(xn), dtype_of(x), (int)bsz, (int)length, (int)dim, STRIDES3(x), STRIDES3(y),
+           ptr<int64_t>(pc), fptr(pm), fptr(pv), fptr(gamma), fptr(beta), eps, ptr<int64_t>(count), fptr(mean), fptr(var), fptr(p),
+           fptr(q), fptr(g), fptr(omega), (int)n, ptr<uint8_t>(mask), fptr(h_in), fptr(h_out), silu ? MEGA_EMA_SILU : 0u,
+           w.stream), cplx ? "tsn_cema_fwd" : "tsn_ema_fwd");
+  py::object h = py::none(), nx = py::none();
+  if (want_state) h = py::cast(cplx ? at::view_as_complex(h_out) : h_out);
+  if (want_normed) nx = py::cast(xn);
+  return py::make_tuple(y, count, mean, var, h, nx);
+}
+
+// y, or None outside the fused kernel's envelope
+OptTensor sqn_ema_forward(const Tensor& x, const Tensor& gamma, const Tensor& beta, double eps, const Tensor& p_, const Tensor& q_,
+                          const Tensor& g_, const Tensor& omega_, const OptTensor& mask_, int64_t flags) {
+  on_cuda(x, gamma, beta, p_, q_, g_, omega_, given(mask_));
+  if (x.stride(2) != 1) return std::nullopt;
+  const Where w(x);
+  const Tensor p = f32c(p_), q = f32c(q_), g = f32c(g_), omega = f32c(omega_), ga = f32c(gamma), be = f32c(beta);
+  const Tensor mask = mask_u8(given(mask_), x.size(0), x.size(2));
+  Tensor y = at::empty(x.sizes(), x.options().requires_grad(false));
+  const int rc = mega_sqn_ema_fwd(x.data_ptr(), y.data_ptr(), dtype_of(x), (int)x.size(0), (int)x.size(1), (int)x.size(2), STRIDES3(x),
+                                  STRIDES3(y), fptr(ga), fptr(be), eps, nullptr, nullptr, nullptr, fptr(p), fptr(q), fptr(g),
+                                  fptr(omega), (int)p.size(1), ptr<uint8_t>(mask), (unsigned)flags, w.stream);
+  if (rc == MEGA_ERR_UNSUPPORTED) return std::nullopt;
+  check(rc, "sqn_ema_fwd");
+  return y;
+}
+
+// ------------------------------------------------------------------------------------------------ the block
+// Row-major matrix view of a tensor's last dimension with one row pitch; copied when it is none.
+struct Rows {
+  Tensor t;
+  int64_t rows, cols, ld;
+};
+Rows rows_view(const Tensor& t) {
+  const int64_t cols = t.size(-1);
+  bool ok = t.dim() >= 2 && (t.stride(-1) == 1 || cols == 1);
+  int64_t ld = cols;
+  if (ok) {
+    ld = t.size(-2) > 1 ? t.stride(-2) : std::max(cols, t.stride(-2));
+    int64_t exp = ld;
+    for (int64_t i = t.dim() - 2; i >= 0; --i) {
+      if (t.size(i) != 1 && t.stride(i) != exp) ok = false;
+      exp *= t.size(i);
+    }
+  }
+  if (!ok || ld < cols) return {t.contiguous(), t.numel() / cols, cols, cols};
+  return {t, t.numel() / cols, cols, ld};
+}
+Tensor fresh(const Tensor& t) { return at::empty(t.sizes(), t.options().requires_grad(false)); }
+
+Tensor gate_silu(const Tensor& a, const OptTensor& b) {
+  on_cuda(a, given(b));
+  const Where w(a);
+  const Rows ra = rows_view(a);
+  Tensor y = fresh(a);
+  Rows rb{Tensor(), 0, 0, 0};
+  if (b.has_value()) rb = rows_view(*b);
+  check(mega_gate_silu(ra.t.data_ptr(), ra.ld, ptr(rb.t), rb.ld, y.data_ptr(), ra.cols, dtype_of(a), ra.rows, (int)ra.cols, w.stream),
+        "gate_silu");
+  return y;
+}
+
+Tensor gate_mul_silu(const Tensor& a, const Tensor& r) {
+  on_cuda(a, r);
+  const Where w(a);
+  const Rows ra = rows_view(a), rr = rows_view(r);
+  Tensor y = fresh(a);
+  check(mega_gate_mul_silu(ra.t.data_ptr(), ra.ld, rr.t.data_ptr(), rr.ld, y.data_ptr(), ra.cols, dtype_of(a), ra.rows, (int)ra.cols,
+                           w.stream), "gate_mul_silu");
+  return y;
+}
+
+Tensor gate_output(const Tensor& residual, const Tensor& u, const Tensor& hx, const Tensor& h_lin) {
+  on_cuda(residual, u, hx, h_lin);
+  const Where w(residual);
+  const Rows r = rows_view(residual), ru = rows_view(u), rx = rows_view(hx), rh = rows_view(h_lin);
+  Tensor y = fresh(residual);
+  check(mega_gate_output(r.t.data_ptr(), r.ld, ru.t.data_ptr(), ru.ld, rx.t.data_ptr(), rx.ld, rh.t.data_ptr(), rh.ld, y.data_ptr(),
+                         r.cols, dtype_of(residual), r.rows, (int)r.cols, w.stream), "gate_output");
+  return y;
+}
+
+// rot: fp32 (positions, S / 2, 2), or None
+std::tuple<Tensor, Tensor> gate_qk(const Tensor& z, const Tensor& gamma, const Tensor& beta, const OptTensor& rot, int64_t period,
+                                   int64_t q_offset, double eps) {
+  on_cuda(z, gamma, beta, given(rot));
+  const Where w(z);
+  const Rows r = rows_view(z);
+  const Tensor g = f32c(gamma), b = f32c(beta);
+  if (g.dim() != 2 || g.size(0) != 2 || g.size(1) != r.cols || b.sizes() != g.sizes())
+    throw py::value_error("gate_qk: gamma and beta must be (2, " + std::to_string(r.cols) + ")");
+  Tensor q = fresh(z), k = fresh(z);
+  if (!rot.has_value()) {
+    check(mega_gate_qk(r.t.data_ptr(), r.ld, fptr(g), fptr(b), q.data_ptr(), r.cols, k.data_ptr(), r.cols, dtype_of(z), r.rows,
+                       (int)r.cols, eps, w.stream), "gate_qk");
+    return {q, k};
+  }
+  Tensor t = rot->is_complex() ? at::view_as_real(*rot) : *rot;
+  t = f32c(t);
+  if (t.dim() != 3 || t.size(1) * 2 != r.cols || t.size(2) != 2)
+    throw py::value_error("gate_qk_rotary: rot must be (positions, S / 2) complex or (positions, S / 2, 2) float");
+  check(mega_gate_qk_rotary(r.t.data_ptr(), r.ld, fptr(g), fptr(b), fptr(t), (int)t.size(0), (int)period, (int)q_offset, q.data_ptr(),
+                            r.cols, k.data_ptr(), r.cols, dtype_of(z), r.rows, (int)r.cols, eps, w.stream), "gate_qk_rotary");
+  return {q, k};
+}
+
+Tensor softmax_fwd(const Tensor& x, bool causal) {
+  on_cuda(x);
+  const Where w(x);
+  const Tensor xc = x.contiguous();
+  const int64_t outer = xc.size(-2), inner = xc.size(-1);
+  Tensor y = fresh(xc);
+  check(mega_attention_softmax_fwd(xc.data_ptr(), y.data_ptr(), dtype_of(xc), xc.numel() / (outer * inner), outer, (int)inner, causal,
+                                   w.stream), "attention_softmax_fwd");
+  return y;
+}
+
+// Training pass from the moving average to the output.  bias: learned relative bias (2 P - 1), or rot: rotary table
+// (positions, S / 2, 2) with the causal mask; rows (b, t) sit at position t % period of their chunk.
+class BlockFn : public torch::autograd::Function<BlockFn> {
+ public:
+  static Tensor forward(AutogradContext* ctx, Tensor x, Tensor xn, Tensor mx, Tensor wv, Tensor bv, Tensor wm, Tensor bm, Tensor wh,
+                        Tensor gamma, Tensor beta, OptTensor bias_, OptTensor rot_, OptTensor mask_, int64_t period) {
+    on_cuda(x, xn, mx, wv, wm, wh, given(mask_));
+    const Where w(x);
+    const int64_t bsz = x.size(0), seq = x.size(1), d = x.size(2), rows = bsz * seq, s = gamma.size(1), e = wv.size(0);
+    const int64_t f = 2 * d + s + e, nb = rows / period;
+    const int dt = dtype_of(x);
+    const int64_t es = x.element_size();
+    const Tensor bias = given(bias_), rot = given(rot_);
+    x = x.contiguous();
+    xn = xn.contiguous().view({rows, d});
+    mx = mx.contiguous().view({rows, d});
+    Tensor v_lin = at::addmm(bv, xn, wv.t());
+    Tensor base = at::addmm(bm, mx, wm.t());
+    char* bp = static_cast<char*>(base.data_ptr());
+    char *u = bp, *z = bp + d * es, *r = z + s * es, *hx = r + e * es;
+    Tensor v = fresh(v_lin);
+    check(mega_gate_silu(v_lin.data_ptr(), e, nullptr, 0, v.data_ptr(), e, dt, rows, (int)e, w.stream), "gate_silu");
+    const Tensor ga = f32c(gamma), be = f32c(beta);
+    Tensor q = at::empty({nb, period, s}, x.options().requires_grad(false)), k = fresh(q);
+    if (rot.defined())
+      check(mega_gate_qk_rotary(z, f, fptr(ga), fptr(be), fptr(rot), (int)rot.size(0), (int)period, 0, q.data_ptr(), s, k.data_ptr(), s,
+                                dt, rows, (int)s, 1e-5, w.stream), "gate_qk_rotary");
+    else
+      check(mega_gate_qk(z, f, fptr(ga), fptr(be), q.data_ptr(), s, k.data_ptr(), s, dt, rows, (int)s, 1e-5, w.stream), "gate_qk");
+    Tensor v3 = v.view({nb, period, e});
+    Tensor wgt;
+    {
+      Tensor scores = at::bmm(q, k.transpose(1, 2));
+      wgt = fresh(scores);
+      if (rot.defined()) {
+        check(mega_attention_softmax_fwd(scores.data_ptr(), wgt.data_ptr(), dt, nb, period, (int)period, 1, w.stream),
+              "attention_softmax_fwd");
+      } else {
+        const Tensor mask = mask_u8(given(mask_), bsz, seq);
+        const Tensor b = bias.scalar_type() == x.scalar_type() ? bias.detach().contiguous() : bias.detach().to(x.scalar_type()).contiguous();
+        check(mega_attention_bias_softmax_fwd(scores.data_ptr(), wgt.data_ptr(), b.data_ptr(), (int)((b.size(0) + 1) / 2),
+                                              ptr<uint8_t>(mask), dt, nb, (int)period, (int)period, w.stream),
+              "attention_bias_softmax_fwd");
+      }
+    }
+    Tensor attn = at::bmm(wgt, v3).view({rows, e});
+    Tensor gated = fresh(attn);
+    check(mega_gate_mul_silu(attn.data_ptr(), e, r, f, gated.data_ptr(), e, dt, rows, (int)e, w.stream), "gate_mul_silu");
+    Tensor h_lin = at::mm(gated, wh.t());
+    Tensor out = at::empty({bsz, seq, d}, x.options().requires_grad(false));
+    check(mega_gate_output(x.data_ptr(), d, u, f, hx, f, h_lin.data_ptr(), d, out.data_ptr(), d, dt, rows, (int)d, w.stream), "gate_output");
+    ctx->save_for_backward({x, xn, mx, wv, wm, wh, ga, bias, rot, v_lin, base, q, k, v3, wgt, attn, gated, h_lin});
+    ctx->saved_data["period"] = period;
+    ctx->saved_data["types"] = std::vector<int64_t>{(int64_t)bv.scalar_type(), (int64_t)bm.scalar_type(), (int64_t)gamma.scalar_type(),
+                                                    (int64_t)beta.scalar_type()};
+    ctx->saved_data["need"] = std::vector<int64_t>{xn.requires_grad(), mx.requires_grad(), wv.requires_grad(), wm.requires_grad(),
+                                                   wh.requires_grad()};
+    return out;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto sv = ctx->get_saved_variables();
+    const Tensor &x = sv[0], &xn = sv[1], &mx = sv[2], &wv = sv[3], &wm = sv[4], &wh = sv[5], &ga = sv[6], &bias = sv[7], &rot = sv[8],
+                 &v_lin = sv[9], &base = sv[10], &q = sv[11], &k = sv[12], &v3 = sv[13], &wgt = sv[14], &attn = sv[15], &gated = sv[16],
+                 &h_lin = sv[17];
+    const Where w(x);
+    const int64_t period = ctx->saved_data["period"].toInt();
+    const auto types = ctx->saved_data["types"].toIntVector();
+    const int64_t bsz = x.size(0), seq = x.size(1), d = x.size(2), rows = bsz * seq, s = ga.size(1), e = wv.size(0), nb = rows / period;
+    const int64_t f = base.size(1), nbias = bias.defined() ? bias.size(0) : 0;
+    const int dt = dtype_of(x);
+    const int64_t es = x.element_size();
+    Tensor dout = grads[0];
+    if (dout.scalar_type() != x.scalar_type()) dout = dout.to(x.scalar_type());
+    dout = dout.contiguous();
+    // every sum in one zeroed piece: bias gradients of v_proj and mx_proj, the (2, s) affine, the relative bias
+    Tensor sums = at::zeros({e + f + 4 * s + nbias}, at::TensorOptions().dtype(at::kFloat).device(x.device()));
+    float *sbv = fptr(sums), *sbm = sbv + e, *sg = sbm + f, *sb = sg + 2 * s, *srel = sb + 2 * s;
+    Tensor dbase = fresh(base), dx = fresh(x);
+    auto cut = [&](const Tensor& t, char*& u, char*& z, char*& r, char*& hx) {
+      u = static_cast<char*>(t.data_ptr());
+      z = u + d * es;
+      r = z + s * es;
+      hx = r + e * es;
+    };
+    char *u, *z, *r, *hx, *du, *dz, *dr, *dhx;
+    cut(base, u, z, r, hx);
+    cut(dbase, du, dz, dr, dhx);
+    check(mega_gate_output_bwd(dout.data_ptr(), d, x.data_ptr(), d, u, f, hx, f, h_lin.data_ptr(), d, dx.data_ptr(), d, du, f, dhx, f, sbm,
+                               sbm + d + s + e, dt, rows, (int)d, w.stream), "gate_output_bwd");
+    const Tensor dh = dbase.narrow(1, d + s + e, d);
+    Tensor dgated = at::mm(dh, wh);
+    const bool need_xn = ctx->needs_input_grad(1), need_mx = ctx->needs_input_grad(2), need_wv = ctx->needs_input_grad(3),
+               need_wm = ctx->needs_input_grad(5), need_wh = ctx->needs_input_grad(7);
+    Tensor dwh = need_wh ? at::mm(dh.t(), gated) : Tensor();
+    check(mega_gate_mul_silu_bwd(dgated.data_ptr(), e, attn.data_ptr(), e, r, f, dgated.data_ptr(), e, dr, f, sbm + d + s, dt, rows, (int)e,
+                                 w.stream), "gate_mul_silu_bwd");
+    const Tensor dattn = dgated.view({nb, period, e});
+    Tensor dv = at::bmm(wgt.transpose(1, 2), dattn).view({rows, e});
+    Tensor ds;
+    {
+      Tensor dw = at::bmm(dattn, v3.transpose(1, 2));
+      ds = fresh(dw);
+      check(mega_attention_softmax_bwd(dw.data_ptr(), wgt.data_ptr(), ds.data_ptr(), dt, nb, period, (int)period, rot.defined() ? 1 : 0,
+                                       w.stream), "attention_softmax_bwd");
+    }
+    if (nbias)
+      check(mega_attention_bias_grad(ds.data_ptr(), srel, (int)((nbias + 1) / 2), dt, nb, (int)period, (int)period, w.stream),
+            "attention_bias_grad");
+    Tensor dq = at::bmm(ds, k), dk = at::bmm(ds.transpose(1, 2), q);
+    check(mega_gate_qk_bwd(z, f, fptr(ga), fptr(rot), rot.defined() ? (int)rot.size(0) : 0, (int)period, 0, dq.data_ptr(), s, dk.data_ptr(),
+                           s, dz, f, sg, sb, sbm + d, dt, rows, (int)s, 1e-5, w.stream), "gate_qk_bwd");
+    check(mega_gate_silu_bwd(dv.data_ptr(), e, v_lin.data_ptr(), e, dv.data_ptr(), e, sbv, dt, rows, (int)e, w.stream), "gate_silu_bwd");
+    Tensor dxn = need_xn ? at::mm(dv, wv).view({bsz, seq, d}) : Tensor();
+    Tensor dwv = need_wv ? at::mm(dv.t(), xn) : Tensor();
+    Tensor dmx = need_mx ? at::mm(dbase, wm).view({bsz, seq, d}) : Tensor();
+    Tensor dwm = need_wm ? at::mm(dbase.t(), mx) : Tensor();
+    Tensor flat = wv.scalar_type() == at::kFloat ? sums : sums.to(wv.scalar_type());
+    auto part = [&](int64_t from, int64_t count, int64_t type) {
+      Tensor t = flat.narrow(0, from, count);
+      return t.scalar_type() == (at::ScalarType)type ? t : t.to((at::ScalarType)type);
+    };
+    return {dx, dxn, dmx, dwv, part(0, e, types[0]), dwm, part(e, f, types[1]), dwh, part(e + f, 2 * s, types[2]).view({2, s}),
+            part(e + f + 2 * s, 2 * s, types[3]).view({2, s}),
+            nbias ? part(e + f + 4 * s, nbias, (int64_t)bias.scalar_type()) : Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+Tensor block_train(const Tensor& x, const Tensor& xn, const Tensor& mx, const Tensor& wv, const Tensor& bv, const Tensor& wm,
+                   const Tensor& bm, const Tensor& wh, const Tensor& gamma, const Tensor& beta, const OptTensor& bias,
+                   const OptTensor& rot, const OptTensor& mask, int64_t period) {
+  return BlockFn::apply(x, xn, mx, wv, bv, wm, bm, wh, gamma, beta, bias, rot, mask, period);
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_mega_host, m) {
+  m.def("set_error", [](py::object e) { g_error = e.release().ptr(); });
+  m.def("ema_forward", &ema_forward);
+  m.def("ema_train", &ema_train);
+  m.def("norm_prepare", &norm_prepare);
+  m.def("timestep_norm_fwd", &timestep_norm_fwd);
+  m.def("timestep_norm_train", &timestep_norm_train);
+  m.def("sequence_norm_fwd", &sequence_norm_fwd);
+  m.def("sequence_norm_train", &sequence_norm_train);
+  m.def("tsn_ema_forward", &tsn_ema_forward);
+  m.def("sqn_ema_forward", &sqn_ema_forward);
+  m.def("gate_silu", &gate_silu);
+  m.def("gate_mul_silu", &gate_mul_silu);
+  m.def("gate_output", &gate_output);
+  m.def("gate_qk", &gate_qk);
+  m.def("attention_softmax_fwd", &softmax_fwd);
+  m.def("block_train", &block_train);
+}

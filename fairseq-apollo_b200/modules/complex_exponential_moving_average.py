@@ -17,7 +17,7 @@ import torch
 from torch import Tensor, nn
 
 from .. import ops
-from ..functions import ComplexEMAFunction, needs_grad
+from ..functions import ema, needs_grad
 from ..incremental_state import IncrementalStateMixin, require_no_grad
 
 
@@ -146,13 +146,11 @@ class MultiHeadComplexEMA(IncrementalStateMixin, nn.Module):
         assert not self.bidirectional or incremental_state is None, \
             'Bidirectional EMA does not support incremental state'
         if needs_grad(x, self.alpha, self.delta, self.theta, self.gamma, self.omega):
-            # differentiable path: forward and backward kernels behind an autograd Function; the
-            # activation is applied by torch on the result, as the reference's caller does
+            # differentiable path: forward and backward kernels behind an autograd Function
             if incremental_state is not None:
                 raise NotImplementedError("the incremental state is an inference feature: use torch.no_grad()")
-            y = ComplexEMAFunction.apply(x, self.alpha, self.delta, self.theta, self.gamma, self.omega,
-                                         padding_mask, self.bidirectional, self.shift, self.truncation)
-            return torch.nn.functional.silu(y) if activation == 'silu' else y
+            return ema(x, self.alpha, self.delta, self.theta, self.gamma, self.omega, padding_mask, self.bidirectional,
+                       self.shift, self.truncation, True, activation == 'silu')
         p, q, g = self.coeffs()
         p, q = p.squeeze(-1), q.squeeze(-1)
         silu = activation == 'silu'

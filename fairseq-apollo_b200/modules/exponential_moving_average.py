@@ -20,7 +20,7 @@ import torch
 from torch import Tensor, nn
 
 from .. import ops
-from ..functions import EMAFunction, needs_grad
+from ..functions import ema, needs_grad
 from ..incremental_state import IncrementalStateMixin, require_no_grad
 
 
@@ -160,13 +160,11 @@ class MultiHeadEMA(IncrementalStateMixin, nn.Module):
                                truncation=self.truncation, silu=silu)
 
     def _forward_train(self, x, padding_mask, incremental_state, activation):
-        """Differentiable path: forward and backward kernels behind an autograd Function; the
-        activation is applied by torch on the result, as the reference's caller does."""
+        """Differentiable path: forward and backward kernels behind an autograd Function."""
         if incremental_state is not None:
             raise NotImplementedError("the incremental state is an inference feature: use torch.no_grad()")
-        y = EMAFunction.apply(x, self.alpha, self.delta, self.beta, self.gamma, self.omega, padding_mask,
-                              self.bidirectional, self.shift, self.truncation)
-        return torch.nn.functional.silu(y) if activation == 'silu' else y
+        return ema(x, self.alpha, self.delta, self.beta, self.gamma, self.omega, padding_mask, self.bidirectional, self.shift,
+                   self.truncation, False, activation == 'silu')
 
     def forward_time_major(self, x, padding_mask=None, incremental_state=None, activation=None):
         """x: (L, B, D) time-major; returns (L, B, D).  A strided view, no copy."""

@@ -264,14 +264,10 @@ class MovingAverageGatedAttention(IncrementalStateMixin, nn.Module):
         if self.bidirectional:
             xn_t = self.norm(x.transpose(1, 2), padding_mask)
             xn = xn_t.transpose(1, 2)
-            mx = self.move(xn_t, padding_mask, None, 'silu' if (silu_act and not train) else None).transpose(1, 2)
-            if silu_act and train:
-                mx = F.silu(mx)
+            mx = self.move(xn_t, padding_mask, None, 'silu' if silu_act else None).transpose(1, 2)
         elif train:
             xn = self.norm(x, padding_mask=padding_mask, incremental_state=incremental_state)
-            mx = self.move(xn.transpose(1, 2), padding_mask, incremental_state).transpose(1, 2)
-            if silu_act:
-                mx = F.silu(mx)
+            mx = self.move(xn.transpose(1, 2), padding_mask, incremental_state, 'silu' if silu_act else None).transpose(1, 2)
         else:
             mx, xn = timestep_norm_ema(self.norm, self.move, x, padding_mask, incremental_state,
                                        activation='silu' if silu_act else None, return_normed=True)

@@ -9,7 +9,7 @@ import torch.nn as nn
 from torch.nn.parameter import Parameter
 
 from .. import ops
-from ..functions import SequenceNormFunction, needs_grad
+from ..functions import needs_grad, sequence_norm
 from ..incremental_state import require_no_grad
 
 
@@ -26,8 +26,7 @@ class SequenceNorm(nn.Module):
     def forward(self, x: torch.Tensor, padding_mask: Optional[torch.Tensor] = None,
                 length_last: bool = True) -> torch.Tensor:
         if needs_grad(x, self.weight, self.bias):
-            return SequenceNormFunction.apply(x, self.weight, self.bias, padding_mask, self.eps, length_last,
-                                              self.num_groups)
+            return sequence_norm(x, self.weight, self.bias, padding_mask, self.eps, length_last, self.num_groups)
         gamma, beta = ops.norm_prepare(self.weight, self.bias)
         y, _, _, _ = ops.sequence_norm_fwd(x, gamma, beta, padding_mask, self.eps, length_last, self.num_groups)
         return y

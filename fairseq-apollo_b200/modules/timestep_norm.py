@@ -18,7 +18,7 @@ from torch import Tensor
 from torch.nn.parameter import Parameter
 
 from .. import ops
-from ..functions import TimestepNormFunction, needs_grad
+from ..functions import needs_grad, timestep_norm
 from ..incremental_state import IncrementalStateMixin
 
 
@@ -81,8 +81,8 @@ class TimestepNorm(IncrementalStateMixin, nn.Module):
             # differentiable path (norm_layer/timestep_norm.py:100-139 with the autograd Function)
             if incremental_state is not None:
                 raise NotImplementedError("the incremental state is an inference feature: use torch.no_grad()")
-            return TimestepNormFunction.apply(x, self.prior_count, self.prior_mean, self.prior_logv, self.weight, self.bias,
-                                              padding_mask, groups, self.eps)
+            return timestep_norm(x, self.prior_count, self.prior_mean, self.prior_logv, self.weight, self.bias, padding_mask,
+                                 groups, self.eps)
         gamma, beta, prev_count, prev_mean, prev_var, saved_state = self.operands(x.size(0), incremental_state, keep=False)
         out, count, mean, var = ops.timestep_norm_fwd(x, prev_count, prev_mean, prev_var, gamma, beta,
                                                       padding_mask, self.eps, groups)

@@ -116,6 +116,10 @@ def ema_bias(q, g, h, length):
     return out
 
 
+def _flags(bidirectional, shift, silu):
+    return (EMA_BIDIRECTIONAL if bidirectional else 0) | (0 if shift else EMA_NO_SHIFT) | (EMA_SILU if silu else 0)
+
+
 def _trunc(truncation):
     return 0 if truncation is None or truncation < 1 else int(truncation)
 
@@ -125,23 +129,9 @@ def ema_forward(x, p, q, g, omega, padding_mask=None, h_in=None, want_state=Fals
     """EMA layer forward on x (B, D, L) with any strides (a transposed view of (B, L, D)
     memory is addressed in place).  Returns y shaped and strided like x, and the new state
     (B, D, N) when ``want_state``."""
-    _cuda(x, p, q, g, omega, padding_mask, h_in)
-    bsz, dim, length = x.shape
-    p, q, g, omega = _f32c(p), _f32c(q), _f32c(g), _f32c(omega)
-    n = p.shape[1]
-    if p.shape[0] != (2 * dim if bidirectional else dim):
-        raise ValueError("coefficient rows %d do not match embed_dim %d" % (p.shape[0], dim))
-    mask = _mask_u8(padding_mask, bsz, length)
-    if out is None:
-        out = _like(x)
-    h_in = _f32c(h_in)
-    h_out = torch.empty(bsz, dim, n, device=x.device, dtype=torch.float32) if want_state else None
-    flags = (EMA_BIDIRECTIONAL if bidirectional else 0) | (0 if shift else EMA_NO_SHIFT) | (EMA_SILU if silu else 0)
-    trunc = 0 if truncation is None or truncation < 1 else int(truncation)
-    _run("ema_fwd", x, _lib.lib().mega_ema_fwd, x.data_ptr(), out.data_ptr(), _dt(x), bsz, dim, length, *x.stride(),
-         *out.stride(), p.data_ptr(), q.data_ptr(), g.data_ptr(), omega.data_ptr(), n, _ptr(mask), _ptr(h_in),
-         _ptr(h_out), flags, trunc)
-    return (out, h_out) if want_state else out
+    y, h = _lib.host().ema_forward(x, p, q, g, omega, padding_mask, h_in, want_state, _flags(bidirectional, shift, silu),
+                                   _trunc(truncation), False, out)
+    return (y, h) if want_state else y
 
 
 def _dense(t):
@@ -178,79 +168,23 @@ def ema_step(x, p, q, g, omega, h=None, silu=False):
 def norm_prepare(weight, bias, priors=None, bsz=0):
     """A norm module's parameters for the operators: (gamma = weight + 1, beta) fp32, and with ``priors`` =
     (prior_count, prior_mean, prior_logv) also (count, mean, var) of ``bsz`` sequences.  One launch."""
-    dev, dim = weight.device, weight.shape[0]
-    g = priors[1].shape[0] if priors else 0
-    f = torch.empty(2 * dim + 2 * bsz * g, device=dev, dtype=torch.float32)
-    gamma, beta, mean, var = f[:dim], f[dim:2 * dim], f[2 * dim:2 * dim + bsz * g], f[2 * dim + bsz * g:]
-    count = torch.empty(bsz, device=dev, dtype=torch.int64) if priors else None
     pc, pm, pl = priors if priors else (None, None, None)
-    _run("norm_prepare", weight, _lib.lib().mega_norm_prepare, _ptr(pc), _ptr(pm), _ptr(pl), weight.data_ptr(),
-         bias.data_ptr(), _dt(weight), bsz, g, dim, _ptr(count), mean.data_ptr() if priors else None,
-         var.data_ptr() if priors else None, gamma.data_ptr(), beta.data_ptr())
-    return (gamma, beta, count, mean.view(bsz, g), var.view(bsz, g)) if priors else (gamma, beta)
-
-
-def norm_finish(like, dgamma, dbeta, dprev_mean=None, dprev_var=None, prior_logv=None):
-    """Gradients of norm_prepare's parameters in their type: (dweight, dbias[, dprior_mean, dprior_logv])."""
-    dim = dgamma.shape[0]
-    bsz, g = dprev_mean.shape if dprev_mean is not None else (0, 0)
-    out = torch.empty(2 * dim + 2 * g, device=like.device, dtype=like.dtype)
-    dw, db, dm, dl = torch.split(out, (dim, dim, g, g))
-    _run("norm_finish", like, _lib.lib().mega_norm_finish, _ptr(dprev_mean), _ptr(dprev_var), _ptr(prior_logv),
-         dgamma.data_ptr(), dbeta.data_ptr(), _dt(like), bsz, g, dim, dm.data_ptr() if g else None,
-         dl.data_ptr() if g else None, dw.data_ptr(), db.data_ptr())
-    return (dw, db, dm, dl) if g else (dw, db)
+    return _lib.host().norm_prepare(weight, bias, pc, pm, pl, bsz)
 
 
 def timestep_norm_fwd(x, prev_count, prev_mean, prev_var, gamma, beta, padding_mask=None,
                       eps=1e-5, num_groups=None, out=None):
     """x (B, L, D) any strides -> (y, count (B) int64, mean, var (B, G) fp32).
     gamma is the effective scale (module weight + 1)."""
-    _cuda(x, prev_count, prev_mean, prev_var, gamma, beta, padding_mask)
-    bsz, length, dim = x.shape
-    groups = dim if num_groups is None else int(num_groups)
-    prev_count = prev_count.detach().to(torch.int64).contiguous()
-    prev_mean, prev_var = _f32c(prev_mean), _f32c(prev_var)
-    if prev_mean.shape != (bsz, groups) or prev_var.shape != (bsz, groups):
-        raise ValueError("prev_mean/prev_var must be (batch, groups) = (%d, %d)" % (bsz, groups))
-    gamma, beta = _f32c(gamma), _f32c(beta)
-    mask = _mask_u8(padding_mask, bsz, length)
-    if out is None:
-        out = _like(x)
-    count = torch.empty(bsz, device=x.device, dtype=torch.int64)
-    mean = torch.empty(bsz, groups, device=x.device, dtype=torch.float32)
-    var = torch.empty_like(mean)
-    _run("timestep_norm_fwd", x, _lib.lib().mega_timestep_norm_fwd, x.data_ptr(), out.data_ptr(), _dt(x), bsz,
-         length, dim, *x.stride(), *out.stride(), prev_count.data_ptr(), prev_mean.data_ptr(), prev_var.data_ptr(),
-         gamma.data_ptr(), beta.data_ptr(), _ptr(mask), groups, float(eps), count.data_ptr(), mean.data_ptr(),
-         var.data_ptr())
-    return out, count, mean, var
+    return _lib.host().timestep_norm_fwd(x, prev_count, prev_mean, prev_var, gamma, beta, padding_mask, eps,
+                                         0 if num_groups is None else int(num_groups), out)
 
 
 def sequence_norm_fwd(x, gamma, beta, padding_mask=None, eps=1e-5, length_last=True, num_groups=None, out=None):
     """x (B, D, L) when ``length_last`` else (B, L, D); any strides.
     Returns (y, count (B) int64, mean, rstd (B, G) fp32)."""
-    _cuda(x, gamma, beta, padding_mask)
-    if length_last:
-        bsz, dim, length = x.shape
-    else:
-        bsz, length, dim = x.shape
-    groups = dim if num_groups is None else int(num_groups)
-    gamma, beta = _f32c(gamma), _f32c(beta)
-    mask = _mask_u8(padding_mask, bsz, length)
-    if out is None:
-        out = _like(x)
-    xs, ys = x.stride(), out.stride()
-    if not length_last:
-        xs = (xs[0], xs[2], xs[1])
-        ys = (ys[0], ys[2], ys[1])
-    count = torch.empty(bsz, device=x.device, dtype=torch.int64)
-    mean = torch.empty(bsz, groups, device=x.device, dtype=torch.float32)
-    rstd = torch.empty_like(mean)
-    _run("sequence_norm_fwd", x, _lib.lib().mega_sequence_norm_fwd, x.data_ptr(), out.data_ptr(), _dt(x), bsz, dim,
-         length, *xs, *ys, gamma.data_ptr(), beta.data_ptr(), _ptr(mask), groups, float(eps), count.data_ptr(),
-         mean.data_ptr(), rstd.data_ptr())
-    return out, count, mean, rstd
+    return _lib.host().sequence_norm_fwd(x, gamma, beta, padding_mask, eps, length_last,
+                                         0 if num_groups is None else int(num_groups), out)
 
 
 def tsn_ema_forward(x, prev_count, prev_mean, prev_var, gamma, beta, eps, p, q, g, omega,
@@ -259,35 +193,12 @@ def tsn_ema_forward(x, prev_count, prev_mean, prev_var, gamma, beta, eps, p, q, 
     """Fused per-feature TimestepNorm -> causal EMA on x (B, L, D).
     Returns dict(y, count, mean, var[, h][, xn]); y and xn are (B, L, D) like x.
     ``complex_poles``: q, g (and the states) are complex64, the layer is MultiHeadComplexEMA's."""
-    _cuda(x, prev_count, prev_mean, prev_var, gamma, beta, p, q, g, omega, padding_mask, h_in)
-    bsz, length, dim = x.shape
-    prev_count = prev_count.detach().to(torch.int64).contiguous()
-    prev_mean, prev_var, gamma, beta = _f32c(prev_mean), _f32c(prev_var), _f32c(gamma), _f32c(beta)
-    if complex_poles:
-        p, q, g, omega, h_in = _f32c(p), _c64(q), _c64(g), _f32c(omega).reshape(-1), _c64(h_in)
-    else:
-        p, q, g, omega = _f32c(p), _f32c(q), _f32c(g), _f32c(omega)
-    n = p.shape[1]
-    mask = _mask_u8(padding_mask, bsz, length)
-    y = _like(x)
-    xn = torch.empty_like(y) if want_normed else None
-    count = torch.empty(bsz, device=x.device, dtype=torch.int64)
-    mean = torch.empty(bsz, dim, device=x.device, dtype=torch.float32)
-    var = torch.empty_like(mean)
-    if complex_poles:
-        h_out = torch.empty(bsz, dim, n, 2, device=x.device, dtype=torch.float32) if want_state else None
-        entry, what = _lib.lib().mega_tsn_cema_fwd, "tsn_cema_fwd"
-    else:
-        h_in = _f32c(h_in)
-        h_out = torch.empty(bsz, dim, n, device=x.device, dtype=torch.float32) if want_state else None
-        entry, what = _lib.lib().mega_tsn_ema_fwd, "tsn_ema_fwd"
-    _run(what, x, entry, x.data_ptr(), y.data_ptr(), _ptr(xn), _dt(x), bsz, length, dim, *x.stride(), *y.stride(),
-         prev_count.data_ptr(), prev_mean.data_ptr(), prev_var.data_ptr(), gamma.data_ptr(), beta.data_ptr(),
-         float(eps), count.data_ptr(), mean.data_ptr(), var.data_ptr(), p.data_ptr(), q.data_ptr(), g.data_ptr(),
-         omega.data_ptr(), n, _ptr(mask), _ptr(h_in), _ptr(h_out), EMA_SILU if silu else 0)
+    y, count, mean, var, h, xn = _lib.host().tsn_ema_forward(
+        x, prev_count, prev_mean, prev_var, gamma, beta, eps, p, q, g, omega, padding_mask, h_in, want_state, silu, want_normed,
+        complex_poles)
     res = {"y": y, "count": count, "mean": mean, "var": var}
     if want_state:
-        res["h"] = torch.view_as_complex(h_out) if complex_poles else h_out
+        res["h"] = h
     if want_normed:
         res["xn"] = xn
     return res
@@ -297,21 +208,7 @@ def sqn_ema_forward(x, gamma, beta, eps, p, q, g, omega, padding_mask=None, bidi
                     silu=False):
     """Fused per-channel SequenceNorm -> EMA on x (B, D, L) with contiguous length.  Returns y, or
     None when the call is outside the fused kernel's envelope (the caller then runs the two ops)."""
-    _cuda(x, gamma, beta, p, q, g, omega, padding_mask)
-    bsz, dim, length = x.shape
-    if x.stride(2) != 1:
-        return None
-    gamma, beta, p, q, g, omega = _f32c(gamma), _f32c(beta), _f32c(p), _f32c(q), _f32c(g), _f32c(omega)
-    mask = _mask_u8(padding_mask, bsz, length)
-    y = torch.empty_like(x, memory_format=torch.contiguous_format)
-    flags = (EMA_BIDIRECTIONAL if bidirectional else 0) | (0 if shift else EMA_NO_SHIFT) | (EMA_SILU if silu else 0)
-    rc = _status(x, _lib.lib().mega_sqn_ema_fwd, x.data_ptr(), y.data_ptr(), _dt(x), bsz, dim, length, *x.stride(),
-                 *y.stride(), gamma.data_ptr(), beta.data_ptr(), float(eps), None, None, None, p.data_ptr(), q.data_ptr(),
-                 g.data_ptr(), omega.data_ptr(), p.shape[1], _ptr(mask), flags)
-    if rc == 7:  # MEGA_ERR_UNSUPPORTED: outside the envelope
-        return None
-    _lib.check(rc, "sqn_ema_fwd")
-    return y
+    return _lib.host().sqn_ema_forward(x, gamma, beta, eps, p, q, g, omega, padding_mask, _flags(bidirectional, shift, silu))
 
 
 def tsn_ema_step_(x, y, count, mean, var, gamma, beta, eps, p, q, g, omega, h, silu=False, xn_out=None,
@@ -362,39 +259,17 @@ def _rows(t):
 
 def gate_silu(a, b=None):
     """silu(a [+ b]) elementwise; a, b may be column slices of wider row-major matrices."""
-    _cuda(a, b)
-    a_, rows, cols, lda = _rows(a)
-    ldb, b_ = 0, None
-    if b is not None:
-        b_, _, _, ldb = _rows(b)
-    y = torch.empty(a.shape, dtype=a.dtype, device=a.device)
-    _run("gate_silu", a, _lib.lib().mega_gate_silu, a_.data_ptr(), lda, _ptr(b_), ldb, y.data_ptr(), cols, _dt(a),
-         rows, cols)
-    return y
+    return _lib.host().gate_silu(a, b)
 
 
 def gate_mul_silu(a, r):
     """a * silu(r)."""
-    _cuda(a, r)
-    a_, rows, cols, lda = _rows(a)
-    r_, _, _, ldr = _rows(r)
-    y = torch.empty(a.shape, dtype=a.dtype, device=a.device)
-    _run("gate_mul_silu", a, _lib.lib().mega_gate_mul_silu, a_.data_ptr(), lda, r_.data_ptr(), ldr, y.data_ptr(),
-         cols, _dt(a), rows, cols)
-    return y
+    return _lib.host().gate_mul_silu(a, r)
 
 
 def gate_output(residual, u, hx, h_lin):
     """residual + sigmoid(u) * (silu(hx + h_lin) - residual); u is the PRE-sigmoid gate."""
-    _cuda(residual, u, hx, h_lin)
-    r_, rows, cols, ldr = _rows(residual)
-    u_, _, _, ldu = _rows(u)
-    x_, _, _, ldx = _rows(hx)
-    h_, _, _, ldh = _rows(h_lin)
-    y = torch.empty(residual.shape, dtype=residual.dtype, device=residual.device)
-    _run("gate_output", residual, _lib.lib().mega_gate_output, r_.data_ptr(), ldr, u_.data_ptr(), ldu, x_.data_ptr(),
-         ldx, h_.data_ptr(), ldh, y.data_ptr(), cols, _dt(residual), rows, cols)
-    return y
+    return _lib.host().gate_output(residual, u, hx, h_lin)
 
 
 def gate_qk(z, gamma, beta, eps=1e-5):
@@ -402,17 +277,7 @@ def gate_qk(z, gamma, beta, eps=1e-5):
     zn = z / max(||z||_2, eps); returns (zn * (gamma[0] + 1) + beta[0], zn * (gamma[1] + 1) + beta[1]).
     gamma, beta are (2, S); z may be a column slice of the mx_proj output.
     Mirrors fairseq/modules/moving_average_gated_attention.py:324-328."""
-    _cuda(z, gamma, beta)
-    z_, rows, cols, ldz = _rows(z)
-    g = gamma.detach().to(torch.float32).contiguous()
-    b = beta.detach().to(torch.float32).contiguous()
-    if g.shape != (2, cols) or b.shape != (2, cols):
-        raise ValueError("gate_qk: gamma and beta must be (2, %d)" % cols)
-    q = torch.empty(z.shape, dtype=z.dtype, device=z.device)
-    k = torch.empty(z.shape, dtype=z.dtype, device=z.device)
-    _run("gate_qk", z, _lib.lib().mega_gate_qk, z_.data_ptr(), ldz, g.data_ptr(), b.data_ptr(), q.data_ptr(), cols,
-         k.data_ptr(), cols, _dt(z), rows, cols, float(eps))
-    return q, k
+    return _lib.host().gate_qk(z, gamma, beta, None, 1, 0, eps)
 
 
 def gate_qk_rotary(z, gamma, beta, rot, period, q_offset=0, eps=1e-5):
@@ -420,56 +285,7 @@ def gate_qk_rotary(z, gamma, beta, rot, period, q_offset=0, eps=1e-5):
     rot: complex64 (positions, S / 2) unit phasors (the table RotaryEmbedding keeps) or their float32
     (positions, S / 2, 2) view; row r of the flattened z is position r % period (+ q_offset for the query).
     Returns (q, k) in z's dtype."""
-    _cuda(z, gamma, beta, rot)
-    z_, rows, cols, ldz = _rows(z)
-    g = gamma.detach().to(torch.float32).contiguous()
-    b = beta.detach().to(torch.float32).contiguous()
-    if g.shape != (2, cols) or b.shape != (2, cols):
-        raise ValueError("gate_qk_rotary: gamma and beta must be (2, %d)" % cols)
-    r = torch.view_as_real(rot) if rot.is_complex() else rot
-    r = r.to(torch.float32).contiguous()
-    if r.dim() != 3 or r.shape[1] * 2 != cols or r.shape[2] != 2:
-        raise ValueError("gate_qk_rotary: rot must be (positions, %d) complex or (positions, %d, 2) float" % (cols // 2, cols // 2))
-    q = torch.empty(z.shape, dtype=z.dtype, device=z.device)
-    k = torch.empty(z.shape, dtype=z.dtype, device=z.device)
-    _run("gate_qk_rotary", z, _lib.lib().mega_gate_qk_rotary, z_.data_ptr(), ldz, g.data_ptr(), b.data_ptr(),
-         r.data_ptr(), r.shape[0], int(period), int(q_offset), q.data_ptr(), cols, k.data_ptr(), cols, _dt(z), rows,
-         cols, float(eps))
-    return q, k
-
-
-def gate_silu_bwd(dy, a, da, colsum=None):
-    """da = dy * silu'(a) for row-major matrices (da may be dy); colsum (cols) fp32 gets da's column sums added."""
-    rows, cols = a.shape
-    _run("gate_silu_bwd", a, _lib.lib().mega_gate_silu_bwd, dy.data_ptr(), dy.stride(0), a.data_ptr(), a.stride(0),
-         da.data_ptr(), da.stride(0), _ptr(colsum), _dt(a), rows, cols)
-
-
-def gate_mul_silu_bwd(dy, a, r, da, dr, colsum_r=None):
-    """Gradients of a * silu(r) into da (may be dy) and dr; colsum_r gets dr's column sums added."""
-    rows, cols = a.shape
-    _run("gate_mul_silu_bwd", a, _lib.lib().mega_gate_mul_silu_bwd, dy.data_ptr(), dy.stride(0), a.data_ptr(),
-         a.stride(0), r.data_ptr(), r.stride(0), da.data_ptr(), da.stride(0), dr.data_ptr(), dr.stride(0),
-         _ptr(colsum_r), _dt(a), rows, cols)
-
-
-def gate_output_bwd(dout, residual, u, hx, h_lin, dres, du, dhx, colsum_u=None, colsum_hx=None):
-    """Gradients of gate_output into dres, du and dhx (= that of h_lin), with column sums of the latter two."""
-    rows, cols = residual.shape
-    _run("gate_output_bwd", residual, _lib.lib().mega_gate_output_bwd, dout.data_ptr(), dout.stride(0),
-         residual.data_ptr(), residual.stride(0), u.data_ptr(), u.stride(0), hx.data_ptr(), hx.stride(0),
-         h_lin.data_ptr(), h_lin.stride(0), dres.data_ptr(), dres.stride(0), du.data_ptr(), du.stride(0),
-         dhx.data_ptr(), dhx.stride(0), _ptr(colsum_u), _ptr(colsum_hx), _dt(residual), rows, cols)
-
-
-def gate_qk_bwd(z, gamma, rot, period, dq, dk, dz, dgamma, dbeta, colsum=None, eps=1e-5):
-    """Gradients of gate_qk (rot None) or gate_qk_rotary: dz, and dgamma, dbeta (2 S) fp32 added to."""
-    rows, cols = z.shape
-    g = _f32c(gamma)
-    _run("gate_qk_bwd", z, _lib.lib().mega_gate_qk_bwd, z.data_ptr(), z.stride(0), g.data_ptr(), _ptr(rot),
-         0 if rot is None else rot.shape[0], int(period), 0, dq.data_ptr(), dq.stride(0), dk.data_ptr(),
-         dk.stride(0), dz.data_ptr(), dz.stride(0), dgamma.data_ptr(), dbeta.data_ptr(), _ptr(colsum), _dt(z), rows,
-         cols, float(eps))
+    return _lib.host().gate_qk(z, gamma, beta, rot, int(period), int(q_offset), eps)
 
 
 # ------------------------------------------------------------------------ training
@@ -531,13 +347,6 @@ def timestep_norm_bwd(dy, dmean, dvar, x, prev_mean, count, cummean, cumrstd, gr
     return dx, dpm, dpv, dgamma, dbeta
 
 
-def timestep_norm_keeps_nothing(x):
-    """Whether timestep_norm_bwd_stats takes x (B, L, D): contiguous channels in whole 16-byte pieces."""
-    es = x.element_size()
-    return (x.stride(2) == 1 and x.shape[2] * es % 16 == 0 and x.stride(0) * es % 16 == 0
-            and x.stride(1) * es % 16 == 0 and x.data_ptr() % 16 == 0)
-
-
 def timestep_norm_bwd_stats(dy, dmean, dvar, x, prev_count, prev_mean, prev_var, gamma, padding_mask=None, eps=1e-5):
     """Gradients of the per-feature TimestepNorm from the statistics its forward started with:
     (dx, dprev_mean, dprev_var, dgamma, dbeta)."""
@@ -545,7 +354,7 @@ def timestep_norm_bwd_stats(dy, dmean, dvar, x, prev_count, prev_mean, prev_var,
     bsz, length, dim = x.shape
     if dy.dtype != x.dtype:
         dy = dy.to(x.dtype)
-    if not timestep_norm_keeps_nothing(dy):
+    if dy.stride(2) != 1:
         dy = dy.contiguous()
     dmean, dvar, prev_mean, prev_var, gamma = _f32c(dmean), _f32c(dvar), _f32c(prev_mean), _f32c(prev_var), _f32c(gamma)
     mask = _mask_u8(padding_mask, bsz, length)
@@ -665,22 +474,9 @@ def cema_forward(x, p, q, g, omega, padding_mask=None, h_in=None, want_state=Fal
                  shift=True, truncation=None, silu=False):
     """Complex EMA layer forward on x (B, D, L) with any strides; q, g complex64 (K, N); the state
     is complex64 (B, D, N).  Returns y like x, and the new state when ``want_state``."""
-    _cuda(x, p, q, g, omega, padding_mask, h_in)
-    bsz, dim, length = x.shape
-    p, q, g, omega = _f32c(p), _c64(q), _c64(g), _f32c(omega).reshape(-1)
-    n = p.shape[1]
-    if p.shape[0] != (2 * dim if bidirectional else dim):
-        raise ValueError("coefficient rows %d do not match embed_dim %d" % (p.shape[0], dim))
-    mask = _mask_u8(padding_mask, bsz, length)
-    out = _like(x)
-    h_in = _c64(h_in)
-    h_out = torch.empty(bsz, dim, n, 2, device=x.device, dtype=torch.float32) if want_state else None
-    flags = (EMA_BIDIRECTIONAL if bidirectional else 0) | (0 if shift else EMA_NO_SHIFT) | (EMA_SILU if silu else 0)
-    trunc = 0 if truncation is None or truncation < 1 else int(truncation)
-    _run("cema_fwd", x, _lib.lib().mega_cema_fwd, x.data_ptr(), out.data_ptr(), _dt(x), bsz, dim, length,
-         *x.stride(), *out.stride(), p.data_ptr(), q.data_ptr(), g.data_ptr(), omega.data_ptr(), n, _ptr(mask),
-         _ptr(h_in), _ptr(h_out), flags, trunc)
-    return (out, torch.view_as_complex(h_out)) if want_state else out
+    y, h = _lib.host().ema_forward(x, p, q, g, omega, padding_mask, h_in, want_state, _flags(bidirectional, shift, silu),
+                                   _trunc(truncation), True, None)
+    return (y, h) if want_state else y
 
 
 def cema_step(x, p, q, g, omega, h=None, silu=False):
@@ -739,14 +535,7 @@ def cema_coeffs_bwd(alpha, delta, theta, q, dp, dq, dg, dtype=torch.float32):
 def attention_softmax_fwd(x, causal=True):
     """softmax over the last axis of the score tensor x (..., C_q, C_k); with ``causal`` row r keeps
     its first C_k - C_q + r + 1 columns (the rest is 0).  A row of -inf scores gives zeros."""
-    _cuda(x)
-    xc = x.contiguous()
-    outer, inner = xc.shape[-2], xc.shape[-1]
-    batch = xc.numel() // (outer * inner)
-    y = torch.empty_like(xc)
-    _run("attention_softmax_fwd", x, _lib.lib().mega_attention_softmax_fwd, xc.data_ptr(), y.data_ptr(), _dt(xc),
-         batch, outer, inner, 1 if causal else 0)
-    return y
+    return _lib.host().attention_softmax_fwd(x, causal)
 
 
 def attention_dropkey_softmax_fwd(x, dropout, causal=True, seed=0, offset=0):
@@ -774,21 +563,3 @@ def attention_softmax_bwd(dy, y, causal=True):
     _run("attention_softmax_bwd", y, _lib.lib().mega_attention_softmax_bwd, dyc.data_ptr(), yc.data_ptr(),
          dx.data_ptr(), _dt(yc), batch, outer, inner, 1 if causal else 0)
     return dx
-
-
-def attention_bias_softmax_fwd(x, bias, padding_mask=None):
-    """softmax of scores x (batch, rows, cols) + bias[column - row + span - 1] over the last axis, without the columns
-    of padding_mask (batch, cols) uint8; bias (2 span - 1)."""
-    _cuda(x, bias, padding_mask)
-    xc = x.contiguous()
-    b = bias.to(xc.dtype).contiguous()
-    y = torch.empty_like(xc)
-    _run("attention_bias_softmax_fwd", x, _lib.lib().mega_attention_bias_softmax_fwd, xc.data_ptr(), y.data_ptr(),
-         b.data_ptr(), (b.shape[0] + 1) // 2, _ptr(padding_mask), _dt(xc), xc.shape[0], xc.shape[1], xc.shape[2])
-    return y
-
-
-def attention_bias_grad(ds, dbias):
-    """Adds the sums of ds (batch, rows, cols) along its diagonals to dbias (2 span - 1) fp32."""
-    _run("attention_bias_grad", ds, _lib.lib().mega_attention_bias_grad, ds.data_ptr(), dbias.data_ptr(),
-         (dbias.shape[0] + 1) // 2, _dt(ds), ds.shape[0], ds.shape[1], ds.shape[2])
