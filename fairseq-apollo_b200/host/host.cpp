@@ -9,7 +9,9 @@
 // fairseq/modules/norm_layer/{timestep_norm,sequence_norm}.py, fairseq/modules/fused_ops/*.py and
 // fairseq/modules/moving_average_gated_attention.py:317-414 of the reference are what the Functions stand in for.
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/extension.h>
 
@@ -769,9 +771,139 @@ Tensor block_train(const Tensor& x, const Tensor& xn, const Tensor& mx, const Te
   return BlockFn::apply(x, xn, mx, wv, bv, wm, bm, wh, gamma, beta, bias, rot, mask, period);
 }
 
+// ------------------------------------------------------------------------------------ single-token step
+// TimestepNorm -> EMA on one token is one launch of 3 us, so the call is as fast as its host path: the same checks
+// and the same library call took 6.6 us through the interpreter and ctypes, 2 us here.
+//
+// A plan is everything a step passes to the library, and what it was built from: it holds as long as the parameters
+// (identity and version counters), the state tensors, the batch, the dtype and the options stay what they were.  The
+// state tensors are updated in place, except the counts: one array is read, another written, and they alternate.
+struct Names {
+  PyObject *params, *groups, *bidirectional, *plan, *count, *mean, *var, *h;
+  Names() {
+    auto s = [](const char* t) { return PyUnicode_InternFromString(t); };
+    params = s("_parameters"); groups = s("num_groups"); bidirectional = s("bidirectional"); plan = s("_step_plan");
+    count = s("prev_count"); mean = s("prev_mean"); var = s("prev_var"); h = s("prev_state");
+  }
+};
+const Names& names() {
+  static const Names* n = new Names;
+  return *n;
+}
+
+struct StepPlan {
+  std::vector<py::object> names, params;   // two of the norm, five of the layer
+  std::vector<int64_t> versions;
+  py::object nkey, ekey, groups, activation;
+  py::object count, count_next, mean, var, h;
+  std::vector<Tensor> operands;            // gamma, beta, p, q, g, omega (fp32)
+  Tensor count_t, next_t, mean_t, var_t, h_t;
+  int dtype, device, ndim, cplx, normed;
+  int64_t batch, dim;
+  double eps;
+};
+
+int64_t version_of(const Tensor& t) { return (int64_t)t.unsafeGetTensorImpl()->version_counter().current_version(); }
+
+std::unique_ptr<StepPlan> step_plan(std::vector<py::object> names, std::vector<py::object> params, py::object nkey, py::object ekey,
+                                    py::object groups, py::object activation, std::vector<py::object> state,
+                                    std::vector<Tensor> operands, const Tensor& x, bool cplx, bool normed, double eps) {
+  auto p = std::make_unique<StepPlan>();
+  p->names = std::move(names);
+  p->params = std::move(params);
+  for (auto& t : p->params) p->versions.push_back(version_of(THPVariable_Unpack(t.ptr())));
+  p->nkey = std::move(nkey); p->ekey = std::move(ekey); p->groups = std::move(groups); p->activation = std::move(activation);
+  p->count = state[0]; p->count_next = state[1]; p->mean = state[2]; p->var = state[3]; p->h = state[4];
+  p->count_t = THPVariable_Unpack(p->count.ptr()); p->next_t = THPVariable_Unpack(p->count_next.ptr());
+  p->mean_t = THPVariable_Unpack(p->mean.ptr()); p->var_t = THPVariable_Unpack(p->var.ptr());
+  p->h_t = THPVariable_Unpack(p->h.ptr());
+  p->operands = std::move(operands);
+  p->dtype = dtype_of(x); p->device = (int)x.get_device(); p->ndim = (int)p->operands[2].size(1);
+  p->cplx = cplx; p->normed = normed; p->batch = x.size(0); p->dim = x.size(2); p->eps = eps;
+  return p;
+}
+
+bool params_match(const StepPlan& p, PyObject* dict, size_t from, size_t to) {
+  for (size_t i = from; i < to; ++i) {
+    PyObject* t = PyDict_GetItemWithError(dict, p.names[i].ptr());
+    if (t != p.params[i].ptr() || version_of(THPVariable_Unpack(t)) != p.versions[i]) return false;
+  }
+  return true;
+}
+
+// norm_ema_step(norm, move, x, incremental_state, activation, return_normed): the outputs, or None when the layer has
+// no plan for this call
+PyObject* norm_ema_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  try {
+    if (n != 6) throw py::type_error("norm_ema_step takes 6 arguments");
+    if (!THPVariable_Check(a[2]) || !PyDict_Check(a[3]) || at::GradMode::is_enabled()) Py_RETURN_NONE;
+    const Names& k = names();
+    const auto norm = py::reinterpret_steal<py::object>(PyObject_GenericGetDict(a[0], nullptr));
+    const auto move = py::reinterpret_steal<py::object>(PyObject_GenericGetDict(a[1], nullptr));
+    PyObject* held = move ? PyDict_GetItemWithError(move.ptr(), k.plan) : nullptr;
+    if (!held || held == Py_None || !norm) {
+      PyErr_Clear();
+      Py_RETURN_NONE;
+    }
+    StepPlan& p = *py::cast<StepPlan*>(py::handle(held));
+    const Tensor& x = THPVariable_Unpack(a[2]);
+    PyObject* ns = PyDict_GetItemWithError(a[3], p.nkey.ptr());
+    PyObject* es = PyDict_GetItemWithError(a[3], p.ekey.ptr());
+    PyObject* np = PyDict_GetItemWithError(norm.ptr(), k.params);
+    PyObject* mp = PyDict_GetItemWithError(move.ptr(), k.params);
+    const bool same = ns && es && np && mp && PyDict_Check(ns) && PyDict_Check(es) &&
+                      PyDict_GetItemWithError(ns, k.mean) == p.mean.ptr() && PyDict_GetItemWithError(ns, k.var) == p.var.ptr() &&
+                      PyDict_GetItemWithError(ns, k.count) == p.count.ptr() && PyDict_GetItemWithError(es, k.h) == p.h.ptr() &&
+                      PyDict_GetItemWithError(norm.ptr(), k.groups) == p.groups.ptr() &&
+                      PyDict_GetItemWithError(move.ptr(), k.bidirectional) == Py_False &&
+                      PyObject_RichCompareBool(a[4], p.activation.ptr(), Py_EQ) == 1 && PyObject_IsTrue(a[5]) == p.normed &&
+                      x.is_cuda() && x.get_device() == p.device && x.dim() == 3 && x.size(1) == 1 && x.size(0) == p.batch &&
+                      x.size(2) == p.dim && x.is_contiguous() && x.scalar_type() != at::kDouble && x.is_floating_point() &&
+                      dtype_of(x) == p.dtype && params_match(p, np, 0, 2) && params_match(p, mp, 2, p.params.size());
+    if (!same) {
+      PyErr_Clear();
+      Py_RETURN_NONE;
+    }
+    const c10::cuda::CUDAGuard guard((c10::DeviceIndex)p.device);
+    void* stream = at::cuda::getCurrentCUDAStream((c10::DeviceIndex)p.device).stream();
+    auto like = [&] { return Tensor(at::detail::empty_cuda(x.sizes(), x.scalar_type(), x.device(), std::nullopt)); };
+    Tensor y = like(), xn = p.normed ? like() : Tensor();
+    const auto& o = p.operands;
+    const unsigned flags = p.activation.is_none() ? 0u : MEGA_EMA_SILU;
+    const auto step = p.cplx ? mega_tsn_cema_step : mega_tsn_ema_step;
+    check(step(x.data_ptr(), y.data_ptr(), ptr(xn), p.dtype, (int)p.batch, (int)p.dim, ptr<int64_t>(p.count_t), ptr<int64_t>(p.next_t),
+               fptr(p.mean_t), fptr(p.var_t), fptr(o[0]), fptr(o[1]), p.eps, fptr(o[2]), fptr(o[3]), fptr(o[4]), fptr(o[5]), p.ndim,
+               (float*)p.h_t.data_ptr(), flags, stream), "tsn_ema_step");
+    std::swap(p.count, p.count_next);
+    std::swap(p.count_t, p.next_t);
+    if (PyDict_SetItem(ns, k.count, p.count.ptr()) != 0) return nullptr;
+    PyObject* out = THPVariable_Wrap(std::move(y));
+    if (!p.normed) return out;
+    PyObject* second = THPVariable_Wrap(std::move(xn));
+    PyObject* both = PyTuple_Pack(2, out, second);
+    Py_XDECREF(out);
+    Py_XDECREF(second);
+    return both;
+  } catch (py::error_already_set& e) {
+    e.restore();
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+  }
+  return nullptr;
+}
+
+PyMethodDef g_raw[] = {{"norm_ema_step", (PyCFunction)(void (*)())norm_ema_step, METH_FASTCALL, nullptr}, {nullptr, nullptr, 0, nullptr}};
+
 }  // namespace
 
 PYBIND11_MODULE(_mega_host, m) {
+  py::class_<StepPlan>(m, "StepPlan")
+      .def(py::init(&step_plan))
+      .def("__deepcopy__", [](StepPlan&, py::object) { return py::none(); })   // (a copied or pickled layer builds its own)
+      .def("__reduce__", [](StepPlan&) {
+        return py::make_tuple(py::reinterpret_borrow<py::object>((PyObject*)Py_TYPE(Py_None)), py::tuple());
+      });
+  PyModule_AddFunctions(m.ptr(), g_raw);
   m.def("set_error", [](py::object e) { g_error = e.release().ptr(); });
   m.def("ema_forward", &ema_forward);
   m.def("ema_train", &ema_train);

@@ -14,7 +14,8 @@ import torch
 from torch import Tensor
 
 from .. import _lib, ops
-from .fused import _current_device, _fp32_params, _param_tensors, _raw_stream, _seed_decode_state
+from ..ops import _current_device, _raw_stream
+from .fused import _fp32_params, _param_tensors, _seed_decode_state
 
 _POLES = {False: (4, 8, 16, 32), True: (2, 4, 8, 16, 32)}
 
