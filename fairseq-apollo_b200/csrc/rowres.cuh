@@ -16,12 +16,11 @@ struct RowArgs {
   long long* count_out;                  // SequenceNorm outputs (optional)
   float *mean_out, *rstd_out;
   int shift, silu;
-  int seg;                               // elements per thread (multiple of 4)
-  unsigned magic;                        // ceil(2^32 / seg)
+  int warps;                             // of a row (set by the launch)
 };
 
-// Tries the row-resident path: length stride 1 on both tensors, ndim <= 16, the row (two copies
-// when bidirectional) fits in shared memory, at least 512 positions.  Returns false, launching
+// Tries the row-resident path: length stride 1 on both tensors, ndim <= 16, the row
+// fits in shared memory, at least 512 positions.  Returns false, launching
 // nothing, otherwise.  `norm` fuses a per-channel SequenceNorm in front of the EMA.
 bool rowres_try(int dtype, const RowArgs& a, long long xsl, long long ysl, bool bidir, bool norm, cudaStream_t s);
 
