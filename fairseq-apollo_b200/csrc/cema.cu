@@ -8,6 +8,7 @@
 #include "stream_cl.cuh"
 #include "block_step.cuh"
 #include "norm_ema_split.cuh"
+#include "scan_cluster.cuh"
 #include "scan_ema.cuh"
 
 namespace mega {
@@ -637,15 +638,6 @@ extern "C" int mega_cema_fwd(const void* x, void* y, int dtype, int B, int D, in
   if (bidir && (h_in || h_out)) return MEGA_ERR_UNSUPPORTED;
   if (!bidir && trunc) return MEGA_ERR_UNSUPPORTED;
   if (x == y && (bidir || trunc || xsb != ysb || xsd != ysd || xsl != ysl)) return MEGA_ERR_STRIDE;
-  if (!bidir && !trunc && x != y && N <= 16) {
-    StreamArgs sa{};
-    sa.B = B; sa.L = L; sa.D = D; sa.N = N;
-    sa.p = p; sa.q = q; sa.g = gamma_hat; sa.omega = omega; sa.h_in = h_in; sa.h_out = h_out; sa.mask = pad_mask;
-    sa.silu = (flags & MEGA_EMA_SILU) ? 1 : 0;
-    sa.cplx = 1;
-    if (mma_cl_try(dtype, x, y, nullptr, xsb, xsl, xsd, ysb, ysl, ysd, false, sa, (cudaStream_t)stream))
-      return check_launch("cema_fwd(mma)");
-  }
   if (!trunc && x != y) {
     ScanArgs ca{};
     ca.x = x; ca.y = y; ca.B = B; ca.D = D; ca.L = L; ca.N = N;
@@ -655,6 +647,15 @@ extern "C" int mega_cema_fwd(const void* x, void* y, int dtype, int B, int D, in
     ca.bidir = bidir ? 1 : 0;
     ca.shift = (flags & MEGA_EMA_NO_SHIFT) ? 0 : 1;
     ca.silu = (flags & MEGA_EMA_SILU) ? 1 : 0;
+    if (!bidir && N <= 16 && !scan_cluster_first(dtype, ca, xsd, ysd)) {
+      StreamArgs sa{};
+      sa.B = B; sa.L = L; sa.D = D; sa.N = N;
+      sa.p = p; sa.q = q; sa.g = gamma_hat; sa.omega = omega; sa.h_in = h_in; sa.h_out = h_out; sa.mask = pad_mask;
+      sa.silu = (flags & MEGA_EMA_SILU) ? 1 : 0;
+      sa.cplx = 1;
+      if (mma_cl_try(dtype, x, y, nullptr, xsb, xsl, xsd, ysb, ysl, ysd, false, sa, (cudaStream_t)stream))
+        return check_launch("cema_fwd(mma)");
+    }
     if (scan_ema_fwd_try(dtype, ca, xsd, ysd, (cudaStream_t)stream)) return check_launch("cema_fwd(scan)");
   }
   CemaArgs a{};

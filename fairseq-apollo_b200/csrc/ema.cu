@@ -9,6 +9,7 @@
 #include "common.cuh"
 #include "stream_cl.cuh"
 #include "rowres.cuh"
+#include "scan_cluster.cuh"
 #include "scan_ema.cuh"
 
 namespace mega {
@@ -426,7 +427,14 @@ extern "C" int mega_ema_fwd(const void* x, void* y, int dtype, int B, int D, int
     ra.silu = (flags & MEGA_EMA_SILU) ? 1 : 0;
     if (rowres_try(dtype, ra, xsl, ysl, bidir, false, (cudaStream_t)stream)) return check_launch("ema_fwd(rowres)");
   }
-  if (!bidir && x != y) {
+  ScanArgs ca{};
+  ca.x = x; ca.y = y; ca.B = B; ca.D = D; ca.L = L; ca.N = N;
+  ca.xsb = xsb; ca.xsl = xsl; ca.ysb = ysb; ca.ysl = ysl;
+  ca.p = p; ca.q = q; ca.g = gamma_hat; ca.omega = omega; ca.mask = pad_mask; ca.h_in = h_in; ca.h_out = h_out;
+  ca.bidir = bidir ? 1 : 0;
+  ca.shift = (flags & MEGA_EMA_NO_SHIFT) ? 0 : 1;
+  ca.silu = (flags & MEGA_EMA_SILU) ? 1 : 0;
+  if (!bidir && x != y && !scan_cluster_first(dtype, ca, xsd, ysd)) {
     StreamArgs sa{};
     sa.B = B; sa.L = L; sa.D = D; sa.N = N;
     sa.p = p; sa.q = q; sa.g = gamma_hat; sa.omega = omega; sa.h_in = h_in; sa.h_out = h_out; sa.mask = pad_mask;
@@ -448,16 +456,8 @@ extern "C" int mega_ema_fwd(const void* x, void* y, int dtype, int B, int D, int
     if (mma_cl_try(dtype, x, y, nullptr, xsb, xsl, xsd, ysb, ysl, ysd, false, sa, (cudaStream_t)stream))
       return check_launch("ema_fwd(mma)");
   }
-  if (!(truncation > 0 && truncation < L) && x != y) {
-    ScanArgs ca{};
-    ca.x = x; ca.y = y; ca.B = B; ca.D = D; ca.L = L; ca.N = N;
-    ca.xsb = xsb; ca.xsl = xsl; ca.ysb = ysb; ca.ysl = ysl;
-    ca.p = p; ca.q = q; ca.g = gamma_hat; ca.omega = omega; ca.mask = pad_mask; ca.h_in = h_in; ca.h_out = h_out;
-    ca.bidir = bidir ? 1 : 0;
-    ca.shift = (flags & MEGA_EMA_NO_SHIFT) ? 0 : 1;
-    ca.silu = (flags & MEGA_EMA_SILU) ? 1 : 0;
-    if (scan_ema_fwd_try(dtype, ca, xsd, ysd, (cudaStream_t)stream)) return check_launch("ema_fwd(scan)");
-  }
+  if (!(truncation > 0 && truncation < L) && x != y && scan_ema_fwd_try(dtype, ca, xsd, ysd, (cudaStream_t)stream))
+    return check_launch("ema_fwd(scan)");
   return ema_fwd_simt(a, flags, truncation, dtype, (cudaStream_t)stream);
 }
 

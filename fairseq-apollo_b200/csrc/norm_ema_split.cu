@@ -7,6 +7,7 @@
 // own output, or through y in place.
 #include "common.cuh"
 #include "norm_ema_split.cuh"
+#include "scan_cluster.cuh"
 #include "scan_ema.cuh"
 #include "scan_norm.cuh"
 
@@ -43,9 +44,10 @@ double mma_us(int dtype, const StreamArgs& a, bool want_xn) {
   return 10.0 + n / 600e3 + (a.cplx ? longer(48.0, 600e3, L, n) : longer(24.0, 1300e3, L, n));
 }
 
-double scan_us(const StreamArgs& a, bool want_xn) {
-  const double n = (double)a.B * a.D * a.L;
-  return 20.0 + n / (a.cplx ? (want_xn ? 78e3 : 88e3) : (want_xn ? 145e3 : 165e3));
+// (in one launch, or as the scan's five)
+double scan_us(int dtype, const ScanArgs& ea, bool want_xn) {
+  const double n = (double)ea.B * ea.D * ea.L, one = scan_cluster_us(dtype, ea);
+  return one < 1e29 ? one : 45.0 + n / (ea.cplx ? (want_xn ? 78e3 : 88e3) : (want_xn ? 145e3 : 165e3));
 }
 
 }  // namespace
@@ -57,9 +59,20 @@ bool norm_ema_split_try(int dtype, const void* x, void* y, void* xn, long long x
       g_options[OPT_MMA_TILE].load() != 0)   // (a kernel asked for by name)
     return false;
   if (x == y || xn == y || xn == x || a.N < 1 || a.N > 16 || a.count_offset != 0) return false;
-  const double fused = fused_us(dtype, a, xn != nullptr), scan = scan_us(a, xn != nullptr), mma = mma_us(dtype, a, xn != nullptr);
-  // (the margin: two to four more launches, on a host that is not ahead of the device)
-  if (forced == 0 && (scan < mma ? scan : mma) + 25.0 > fused) return false;
+  ScanArgs ea{};
+  ea.x = x; ea.y = y; ea.xn = xn; ea.B = a.B; ea.D = a.D; ea.L = a.L; ea.N = a.N;
+  ea.xsb = xsb; ea.xsl = xsl; ea.ysb = ysb; ea.ysl = ysl;
+  ea.p = a.p; ea.q = a.q; ea.g = a.g; ea.omega = a.omega; ea.mask = a.mask; ea.h_in = a.h_in; ea.h_out = a.h_out;
+  ea.cplx = a.cplx; ea.silu = a.silu;
+  ea.prev_count = a.prev_count; ea.prev_mean = a.prev_mean; ea.prev_var = a.prev_var; ea.gamma = a.gamma; ea.beta = a.beta;
+  ea.eps = a.eps; ea.count_out = a.count_out; ea.mean_out = a.mean_out; ea.var_out = a.var_out;
+  // (the margins: two more launches for the norm by itself, on a host that is not ahead of the device; the fixed 45 us of
+  // the scan's launches hold one; the models are good to a tenth)
+  // (a prompt that comes in chunks keeps to the tensor-core kernel, and its rounding, unless much is gained)
+  const bool chunk = dtype == MEGA_BF16 && a.h_out && !a.mask && !a.cplx;
+  const double fused = fused_us(dtype, a, xn != nullptr), scan = scan_us(dtype, ea, xn != nullptr) + (chunk ? 25.0 : 0.0),
+               mma = mma_us(dtype, a, xn != nullptr) + 25.0;
+  if (forced == 0 && (scan < mma ? scan : mma) > 0.9 * fused) return false;
   if (mma < scan && forced != 3) {
     void* mid = xn ? xn : y;
     ScanNormArgs na{};
@@ -71,13 +84,6 @@ bool norm_ema_split_try(int dtype, const void* x, void* y, void* xn, long long x
         mma_cl_try(dtype, mid, y, nullptr, ysb, ysl, ysd, ysb, ysl, ysd, false, a, s))
       return true;   // (were the second one refused, the next form starts from x again)
   }
-  ScanArgs ea{};
-  ea.x = x; ea.y = y; ea.xn = xn; ea.B = a.B; ea.D = a.D; ea.L = a.L; ea.N = a.N;
-  ea.xsb = xsb; ea.xsl = xsl; ea.ysb = ysb; ea.ysl = ysl;
-  ea.p = a.p; ea.q = a.q; ea.g = a.g; ea.omega = a.omega; ea.mask = a.mask; ea.h_in = a.h_in; ea.h_out = a.h_out;
-  ea.cplx = a.cplx; ea.silu = a.silu;
-  ea.prev_count = a.prev_count; ea.prev_mean = a.prev_mean; ea.prev_var = a.prev_var; ea.gamma = a.gamma; ea.beta = a.beta;
-  ea.eps = a.eps; ea.count_out = a.count_out; ea.mean_out = a.mean_out; ea.var_out = a.var_out;
   return scan_ema_fwd_try(dtype, ea, xsd, ysd, s);
 }
 
