@@ -779,10 +779,12 @@ Tensor block_train(const Tensor& x, const Tensor& xn, const Tensor& mx, const Te
 // (identity and version counters), the state tensors, the batch, the dtype and the options stay what they were.  The
 // state tensors are updated in place, except the counts: one array is read, another written, and they alternate.
 struct Names {
-  PyObject *params, *groups, *bidirectional, *plan, *count, *mean, *var, *h;
+  PyObject *params, *modules, *groups, *bidirectional, *plan, *block_plan, *count, *mean, *var, *h, *key, *value, *key_mask;
   Names() {
     auto s = [](const char* t) { return PyUnicode_InternFromString(t); };
     params = s("_parameters"); groups = s("num_groups"); bidirectional = s("bidirectional"); plan = s("_step_plan");
+    modules = s("_modules"); block_plan = s("_block_plan"); key = s("prev_key"); value = s("prev_value");
+    key_mask = s("prev_key_padding_mask");
     count = s("prev_count"); mean = s("prev_mean"); var = s("prev_var"); h = s("prev_state");
   }
 };
@@ -892,7 +894,152 @@ PyObject* norm_ema_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return nullptr;
 }
 
-PyMethodDef g_raw[] = {{"norm_ema_step", (PyCFunction)(void (*)())norm_ema_step, METH_FASTCALL, nullptr}, {nullptr, nullptr, 0, nullptr}};
+// ------------------------------------------------------------------------------------ single-token step of a block
+// Five launches of 3 - 6 us each: through the interpreter and ctypes a step took 31 us of host, more than the device.
+struct BlockPlan {
+  mega_block_step_args args;
+  PyObject* block;                         // (not owned: the plan lives in the block's dictionary)
+  py::object owners[5];                    // norm, move, v_proj, mx_proj, h_proj
+  std::vector<std::pair<int, py::object>> names;   // of a parameter: owner (0: the block, 1 ...: the above), key
+  std::vector<py::object> params;
+  std::vector<int64_t> versions;
+  py::object submodules[5];                // the owners' keys
+  py::object nkey, ekey, akey;
+  py::object count, count_next, mean, var, h, last_key, last_value;
+  Tensor keys, values;
+  std::vector<py::object> keep;
+  int64_t pos, chunk, batch, dim;
+  int device;
+  uintptr_t stream;
+  at::ScalarType type;
+};
+
+std::unique_ptr<BlockPlan> block_plan(py::bytes args, std::vector<py::object> owners, std::vector<std::string> submodules,
+                                      std::vector<std::pair<int, std::string>> names, std::vector<py::object> params,
+                                      std::vector<py::object> state_keys, std::vector<py::object> state, const Tensor& keys,
+                                      const Tensor& values, std::vector<py::object> keep, int64_t chunk, const Tensor& x,
+                                      uintptr_t stream) {
+  auto p = std::make_unique<BlockPlan>();
+  const std::string raw = args;
+  if (raw.size() != sizeof p->args || owners.size() != 6 || submodules.size() != 5) throw py::value_error("block_plan");
+  memcpy(&p->args, raw.data(), raw.size());
+  auto word = [](const std::string& t) { return py::reinterpret_steal<py::object>(PyUnicode_InternFromString(t.c_str())); };
+  p->block = owners[0].ptr();
+  for (int i = 0; i < 5; ++i) p->owners[i] = owners[i + 1];
+  for (int i = 0; i < 5; ++i) p->submodules[i] = word(submodules[i]);
+  for (auto& n : names) p->names.emplace_back(n.first, word(n.second));
+  p->params = std::move(params);
+  for (auto& t : p->params) p->versions.push_back(version_of(THPVariable_Unpack(t.ptr())));
+  p->nkey = state_keys[0]; p->ekey = state_keys[1]; p->akey = state_keys[2];
+  p->count = state[0]; p->count_next = state[1]; p->mean = state[2]; p->var = state[3]; p->h = state[4];
+  p->last_key = state[5]; p->last_value = state[6];
+  p->keys = keys; p->values = values;
+  p->keep = std::move(keep);
+  p->pos = p->args.pos; p->chunk = chunk;
+  p->batch = x.size(0); p->dim = x.size(2); p->device = (int)x.get_device(); p->stream = stream; p->type = x.scalar_type();
+  return p;
+}
+
+py::object dict_of(PyObject* o) { return py::reinterpret_steal<py::object>(PyObject_GenericGetDict(o, nullptr)); }
+
+// (an absent entry and None are the same)
+bool holds(PyObject* dict, PyObject* key, PyObject* want) {
+  PyObject* v = dict ? PyDict_GetItemWithError(dict, key) : nullptr;
+  return (v ? v : Py_None) == want;
+}
+
+// Whether the plan is one for this block, these inputs and this state.
+bool block_matches(const BlockPlan& p, PyObject* blk, PyObject* block_dict, const Tensor& x, PyObject* inc) {
+  const Names& k = names();
+  if (blk != p.block || p.pos >= p.args.cap) return false;
+  PyObject* ns = PyDict_GetItemWithError(inc, p.nkey.ptr());
+  PyObject* es = PyDict_GetItemWithError(inc, p.ekey.ptr());
+  PyObject* as = PyDict_GetItemWithError(inc, p.akey.ptr());
+  if (as == Py_None) as = nullptr;
+  if (!ns || !es || !PyDict_Check(ns) || !PyDict_Check(es) || (as && !PyDict_Check(as))) return false;
+  if (!holds(ns, k.mean, p.mean.ptr()) || !holds(ns, k.var, p.var.ptr()) || !holds(ns, k.count, p.count.ptr()) ||
+      !holds(es, k.h, p.h.ptr()) || !holds(as, k.key, p.last_key.ptr()) || !holds(as, k.value, p.last_value.ptr()) ||
+      !holds(as, k.key_mask, Py_None))
+    return false;
+  if (!x.is_cuda() || x.get_device() != p.device || x.dim() != 3 || x.size(1) != 1 || x.size(0) != p.batch || x.size(2) != p.dim ||
+      x.scalar_type() != p.type || !x.is_contiguous())
+    return false;
+  PyObject* subs = PyDict_GetItemWithError(block_dict, k.modules);
+  if (!subs) return false;
+  py::object dicts[6];   // the owners' parameters
+  for (int i = 0; i < 6; ++i) {
+    if (i && PyDict_GetItemWithError(subs, p.submodules[i - 1].ptr()) != p.owners[i - 1].ptr()) return false;
+    const py::object d = i ? dict_of(p.owners[i - 1].ptr()) : py::reinterpret_borrow<py::object>(block_dict);
+    dicts[i] = py::reinterpret_borrow<py::object>(d ? PyDict_GetItemWithError(d.ptr(), k.params) : nullptr);
+    if (!dicts[i]) return false;
+  }
+  for (size_t i = 0; i < p.params.size(); ++i) {
+    PyObject* t = PyDict_GetItemWithError(dicts[p.names[i].first].ptr(), p.names[i].second.ptr());
+    if (t != p.params[i].ptr() || version_of(THPVariable_Unpack(t)) != p.versions[i]) return false;
+  }
+  return true;
+}
+
+// block_step(block, x, incremental_state): the output, or None when the block has no plan for this call
+PyObject* block_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  try {
+    if (n != 3) throw py::type_error("block_step takes 3 arguments");
+    if (!THPVariable_Check(a[1]) || !PyDict_Check(a[2]) || at::GradMode::is_enabled()) Py_RETURN_NONE;
+    const Names& k = names();
+    const py::object dict = dict_of(a[0]);
+    PyObject* held = dict ? PyDict_GetItemWithError(dict.ptr(), k.block_plan) : nullptr;
+    if (!held || held == Py_None) {
+      PyErr_Clear();
+      Py_RETURN_NONE;
+    }
+    const py::object keep_plan = py::reinterpret_borrow<py::object>(held);
+    BlockPlan& p = *py::cast<BlockPlan*>(py::handle(held));
+    const Tensor& x = THPVariable_Unpack(a[1]);
+    if (!block_matches(p, a[0], dict.ptr(), x, a[2])) {
+      PyErr_Clear();
+      Py_RETURN_NONE;
+    }
+    const c10::cuda::CUDAGuard guard((c10::DeviceIndex)p.device);
+    void* stream = at::cuda::getCurrentCUDAStream((c10::DeviceIndex)p.device).stream();
+    if ((uintptr_t)stream != p.stream) Py_RETURN_NONE;
+    Tensor out(at::detail::empty_cuda(x.sizes(), x.scalar_type(), x.device(), std::nullopt));
+    p.args.x = x.data_ptr();
+    p.args.out = out.data_ptr();
+    p.args.pos = p.pos;
+    check(mega_block_step(&p.args, stream), "block_step");
+    // the counts alternate between two arrays, the step wrote the second one
+    std::swap(p.count, p.count_next);
+    std::swap(p.args.count, p.args.count_next);
+    if (PyDict_SetItem(PyDict_GetItemWithError(a[2], p.nkey.ptr()), k.count, p.count.ptr()) != 0) return nullptr;
+    PyObject* as = PyDict_GetItemWithError(a[2], p.akey.ptr());
+    if (!as || as == Py_None) {
+      const auto fresh = py::dict();
+      if (PyDict_SetItem(a[2], p.akey.ptr(), fresh.ptr()) != 0) return nullptr;
+      as = PyDict_GetItemWithError(a[2], p.akey.ptr());
+    }
+    const int64_t pos = ++p.pos;
+    if (p.chunk < 0 || pos % p.chunk != 0) {
+      p.last_key = py::reinterpret_steal<py::object>(THPVariable_Wrap(p.keys.narrow(1, 0, pos)));
+      p.last_value = py::reinterpret_steal<py::object>(THPVariable_Wrap(p.values.narrow(1, 0, pos)));
+      if (PyDict_SetItem(as, k.key, p.last_key.ptr()) != 0 || PyDict_SetItem(as, k.value, p.last_value.ptr()) != 0 ||
+          PyDict_SetItem(as, k.key_mask, Py_None) != 0)
+        return nullptr;
+    } else {   // the chunk is complete: the next token starts another one, in other buffers
+      for (PyObject* key : {k.key, k.value, k.key_mask})
+        if (PyDict_GetItemWithError(as, key) && PyDict_DelItem(as, key) != 0) return nullptr;
+      if (PyDict_SetItem(dict.ptr(), k.block_plan, Py_None) != 0) return nullptr;
+    }
+    return THPVariable_Wrap(std::move(out));
+  } catch (py::error_already_set& e) {
+    e.restore();
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+  }
+  return nullptr;
+}
+
+PyMethodDef g_raw[] = {{"norm_ema_step", (PyCFunction)(void (*)())norm_ema_step, METH_FASTCALL, nullptr},
+                       {"block_step", (PyCFunction)(void (*)())block_step, METH_FASTCALL, nullptr}, {nullptr, nullptr, 0, nullptr}};
 
 }  // namespace
 
@@ -901,6 +1048,12 @@ PYBIND11_MODULE(_mega_host, m) {
       .def(py::init(&step_plan))
       .def("__deepcopy__", [](StepPlan&, py::object) { return py::none(); })   // (a copied or pickled layer builds its own)
       .def("__reduce__", [](StepPlan&) {
+        return py::make_tuple(py::reinterpret_borrow<py::object>((PyObject*)Py_TYPE(Py_None)), py::tuple());
+      });
+  py::class_<BlockPlan>(m, "BlockPlan")
+      .def(py::init(&block_plan))
+      .def("__deepcopy__", [](BlockPlan&, py::object) { return py::none(); })
+      .def("__reduce__", [](BlockPlan&) {
         return py::make_tuple(py::reinterpret_borrow<py::object>((PyObject*)Py_TYPE(Py_None)), py::tuple());
       });
   PyModule_AddFunctions(m.ptr(), g_raw);
