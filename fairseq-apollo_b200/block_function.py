@@ -9,13 +9,12 @@ import torch
 
 from . import _lib
 
-_CAUSAL, _BIAS = 0, 1
+CAUSAL, _BIAS = 0, 1
 
 
 def mode_of(blk, x, padding_mask, attn_mask, need_weights, before_attn_fn):
-    """_CAUSAL (chunked causal softmax with rotary positions), _BIAS (softmax with the learned relative bias, with or
+    """CAUSAL (chunked causal softmax with rotary positions), _BIAS (softmax with the learned relative bias, with or
     without a padding mask), or None when the block's own sequence of operations has to run."""
-    from .modules.moving_average_gated_attention import RotaryEmbedding, SimpleRelativePositionalBias
     if (attn_mask is not None or need_weights or before_attn_fn or not x.is_cuda
             or (blk.training and (blk.dropout_p or blk.hidden_dropout_p or blk.attention_dropout_p))
             or x.dtype not in (torch.float32, torch.bfloat16, torch.float16) or torch.is_autocast_enabled()):
@@ -30,10 +29,10 @@ def mode_of(blk, x, padding_mask, attn_mask, need_weights, before_attn_fn):
     if seq % period:
         return None
     if blk.efficient_attn is not None:
-        ok = isinstance(blk.rel_pos_bias, RotaryEmbedding) and period <= 8192
-        return _CAUSAL if ok else None
+        ok = type(blk.rel_pos_bias).__name__ == "RotaryEmbedding" and period <= 8192
+        return CAUSAL if ok else None
     if (blk.attention_activation == 'softmax' and blk.attn_softmax is None and period <= 8192
-            and isinstance(blk.rel_pos_bias, SimpleRelativePositionalBias) and period <= blk.rel_pos_bias.max_positions):
+            and type(blk.rel_pos_bias).__name__ == "SimpleRelativePositionalBias" and period <= blk.rel_pos_bias.max_positions):
         return _BIAS
     return None
 
@@ -42,10 +41,29 @@ def run(blk, mode, x, xn, mx, padding_mask):
     seq = x.size(1)
     period = blk.chunk_size if 1 < blk.chunk_size < seq else seq
     rot = bias = None
-    if mode == _CAUSAL:
+    if mode == CAUSAL:
         rot = torch.view_as_real(blk.rel_pos_bias._angles(0, period))
         padding_mask = None      # (as EfficientAttention: the causal kernel takes none)
     else:
         bias = blk.rel_pos_bias.rel_pos_bias
     return _lib.host().block_train(x, xn, mx, blk.v_proj.weight, blk.v_proj.bias, blk.mx_proj.weight, blk.mx_proj.bias,
                                    blk.h_proj.weight, blk.gamma, blk.beta, bias, rot, padding_mask, period)
+
+
+def qk_affine(blk):
+    """gamma and beta of the queries and keys in fp32, kept until a parameter changes (identity, version counter, storage)."""
+    ver = (blk.gamma._version, blk.beta._version, blk.gamma.data_ptr(), blk.beta.data_ptr())
+    cache = blk.__dict__.get("_qk_fp32")
+    if cache is None or cache[0] is not blk.gamma or cache[1] is not blk.beta or cache[2] != ver:
+        cache = blk._qk_fp32 = (blk.gamma, blk.beta, ver, blk.gamma.detach().float().contiguous(),
+                                blk.beta.detach().float().contiguous())
+    return cache[3], cache[4]
+
+
+def infer(blk, x, xn, mx, cache):
+    """The same in inference, causal mode: the output, and with ``cache`` the keys (not rotated) and values."""
+    seq = x.size(1)
+    period = blk.chunk_size if 1 < blk.chunk_size < seq else seq
+    rot = torch.view_as_real(blk.rel_pos_bias._angles(0, period))
+    return _lib.host().block_infer(x, xn, mx, blk.v_proj.weight, blk.v_proj.bias, blk.mx_proj.weight, blk.mx_proj.bias,
+                                   blk.h_proj.weight, *qk_affine(blk), rot, period, cache)

@@ -261,6 +261,108 @@ __global__ void __launch_bounds__(kT) attn_softmax_bwd_kernel(const T* __restric
 using namespace mega;
 
 // vectors per thread for the vectorised kernels: rows up to kT * kN * kV elements
+// Short rows: a warp takes one, kN vectors per lane, nothing but shuffles between its lanes.  Memory-bound (the kept part
+// of x in, y out); a block of 128 threads per row of 1024 bf16 spends its time in two barriers: 65 us for 64 x 1024 x 1024
+// causal, 58 as warps.  Forward up to 2048 columns of 16 bits (fp32 1024), backward, which holds two values of each, a quarter
+// of that: at 1024 columns the block form was faster (16 us against 22 for 16 x 1024 x 1024).
+template <typename T, int kN>
+__global__ void __launch_bounds__(256) attn_softmax_fwd_warp_kernel(const T* __restrict__ x, T* __restrict__ y, long long rows,
+                                                                    long long outer, int inner, int causal) {
+  constexpr int kV = Vec<T>::kV;
+  const int lane = threadIdx.x & 31;
+  const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  const int n = causal ? (int)(inner - outer + row % outer + 1) : inner;
+  const T* xr = x + row * inner;
+  T* yr = y + row * inner;
+  float v[kN][kV], m = -INFINITY;
+#pragma unroll
+  for (int j = 0; j < kN; ++j) {
+    const int c = (lane + j * 32) * kV;
+    if (c < n) {  // vectors wholly past the kept columns are not read at all
+      Vec<T>::load(xr + c, v[j]);
+#pragma unroll
+      for (int k = 0; k < kV; ++k) {
+        if (c + k >= n) v[j][k] = -INFINITY;
+        m = fmaxf(m, v[j][k]);
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < kV; ++k) v[j][k] = -INFINITY;
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  const bool dead = m == -INFINITY;
+  float d = 0.f;
+#pragma unroll
+  for (int j = 0; j < kN; ++j)
+    if (32 * j * kV < n) {
+#pragma unroll
+      for (int k = 0; k < kV; ++k) {
+        v[j][k] = dead ? 0.f : __expf(v[j][k] - m);
+        d += v[j][k];
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < kV; ++k) v[j][k] = 0.f;
+    }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+  const float inv = d == 0.f ? 0.f : 1.f / d;
+#pragma unroll
+  for (int j = 0; j < kN; ++j) {
+    const int c = (lane + j * 32) * kV;
+    if (c < inner) {
+#pragma unroll
+      for (int k = 0; k < kV; ++k) v[j][k] *= inv;
+      Vec<T>::store(yr + c, v[j]);
+    }
+  }
+}
+
+template <typename T, int kN>
+__global__ void __launch_bounds__(256) attn_softmax_bwd_warp_kernel(const T* __restrict__ dy, const T* __restrict__ y,
+                                                                    T* __restrict__ dx, long long rows, long long outer, int inner,
+                                                                    int causal) {
+  constexpr int kV = Vec<T>::kV;
+  const int lane = threadIdx.x & 31;
+  const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  const int n = causal ? (int)(inner - outer + row % outer + 1) : inner;
+  const T *gr = dy + row * inner, *yr = y + row * inner;
+  T* dr = dx + row * inner;
+  float yv[kN][kV], gv[kN][kV], s = 0.f;
+#pragma unroll
+  for (int j = 0; j < kN; ++j) {
+    const int c = (lane + j * 32) * kV;
+    if (c < n) {
+      Vec<T>::load(yr + c, yv[j]);
+      Vec<T>::load(gr + c, gv[j]);
+#pragma unroll
+      for (int k = 0; k < kV; ++k) {
+        if (c + k >= n) yv[j][k] = 0.f;
+        s = fmaf(yv[j][k], gv[j][k], s);
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < kV; ++k) yv[j][k] = gv[j][k] = 0.f;
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+#pragma unroll
+  for (int j = 0; j < kN; ++j) {
+    const int c = (lane + j * 32) * kV;
+    if (c < inner) {
+      float o[kV];
+#pragma unroll
+      for (int k = 0; k < kV; ++k) o[k] = yv[j][k] * (gv[j][k] - s);
+      Vec<T>::store(dr + c, o);
+    }
+  }
+}
+
 #define MEGA_ATTN_DISPATCH_VEC(KERNEL, EXTRA, ...)                                                   \
   MEGA_DISPATCH_DTYPE(dtype, {                                                                       \
     constexpr int kV = Vec<T>::kV;                                                                   \
@@ -297,6 +399,18 @@ static int attention_softmax_fwd_impl(const void* x, void* y, int dtype, int64_t
     if (drop) {
       MEGA_ATTN_DISPATCH_VEC(attn_softmax_fwd_vec_kernel, MEGA_COMMA true, (const T*)x, (T*)y, (long long)outer, inner,
                              causal, dk);
+    } else if (inner <= 8 * 32 * 16 / elem_size(dtype)) {
+      const long long rows = batch * outer;
+      MEGA_DISPATCH_DTYPE(dtype, {
+        const int vecs = (inner / Vec<T>::kV + 31) / 32;
+        auto run = [&](auto kernel) {
+          launch(kernel, (unsigned)((rows + 7) / 8), 256, 0, stream, (const T*)x, (T*)y, rows, (long long)outer, inner, causal);
+        };
+        if (vecs <= 1) run(attn_softmax_fwd_warp_kernel<T, 1>);
+        else if (vecs <= 2) run(attn_softmax_fwd_warp_kernel<T, 2>);
+        else if (vecs <= 4) run(attn_softmax_fwd_warp_kernel<T, 4>);
+        else run(attn_softmax_fwd_warp_kernel<T, 8>);
+      });
     } else {
       MEGA_ATTN_DISPATCH_VEC(attn_softmax_fwd_vec_kernel, MEGA_COMMA false, (const T*)x, (T*)y, (long long)outer,
                              inner, causal, dk);
@@ -337,6 +451,19 @@ extern "C" int mega_attention_softmax_bwd(const void* dy, const void* y, void* d
   if (inner > 64 * kT) return MEGA_ERR_UNSUPPORTED;
   if (batch * outer > 2147483647LL) return MEGA_ERR_SHAPE;
   const unsigned grid = (unsigned)(batch * outer);
+  if (vec_ok(dtype, inner, dy, y, dx) && inner <= 2 * 32 * 16 / elem_size(dtype)) {
+    const long long rows = batch * outer;
+    MEGA_DISPATCH_DTYPE(dtype, {
+      const int vecs = (inner / Vec<T>::kV + 31) / 32;
+      auto run = [&](auto kernel) {
+        launch(kernel, (unsigned)((rows + 7) / 8), 256, 0, stream, (const T*)dy, (const T*)y, (T*)dx, rows, (long long)outer, inner,
+               causal);
+      };
+      if (vecs <= 1) run(attn_softmax_bwd_warp_kernel<T, 1>);
+      else run(attn_softmax_bwd_warp_kernel<T, 2>);
+    });
+    return check_launch("attention_softmax_bwd(warp)");
+  }
   if (vec_ok(dtype, inner, dy, y, dx)) {
     MEGA_ATTN_DISPATCH_VEC(attn_softmax_bwd_vec_kernel, , (const T*)dy, (const T*)y, (T*)dx, (long long)outer, inner,
                            causal);

@@ -22,27 +22,6 @@ namespace mega {
 
 namespace {
 
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-template <typename... KArgs, typename... Args>
-static void launch_after(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
-  if (smem > 48 * 1024) allow_smem(reinterpret_cast<const void*>(kernel), smem);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  g_last_kernel.store("other", std::memory_order_relaxed);
-}
-
 template <typename T>
 __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                           uint32_t b1);
@@ -97,6 +76,7 @@ __device__ __forceinline__ void rows_times(const T* w, const T* act, int B, int 
 #pragma unroll
   for (int i = 0; i < kAhead; ++i) fetch(i);
   pdl_wait();   // the activations are the launch before's
+  pdl_next();   // (after the wait: so the next launch may read, before its own, whatever earlier steps left in the caches)
   for (int i = threadIdx.x; i < B * (K / 8); i += kW * 32) {
     const int b = i / (K / 8), c = (i - b * (K / 8)) * 8;
     *reinterpret_cast<uint4*>(as + (size_t)b * pitch + c) = __ldg(reinterpret_cast<const uint4*>(act + (size_t)b * K + c));
@@ -162,7 +142,6 @@ __device__ __forceinline__ float round_to(float v) {
 template <typename T, int kNB>
 __global__ void __launch_bounds__(256) block_proj_kernel(BlockStep a) {
   extern __shared__ __align__(16) unsigned char smem[];
-  pdl_next();
   const int r0 = blockIdx.x * 16;
   const bool isv = r0 < a.E;
   const int F = 2 * a.D + a.S + a.E;
@@ -182,9 +161,22 @@ template <typename T>
 __global__ void __launch_bounds__(256) block_score_kernel(BlockStep a) {
   __shared__ float qs[512];
   __shared__ float red[8];
-  pdl_next();
-  pdl_wait();
   const int b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // the keys of earlier steps are read ahead of the wait
+  const int k0 = blockIdx.x * kKeys;
+  const int lanes = a.S / 8;           // lanes of a key (8, 16 or 32)
+  const int per = 32 / lanes;          // keys of a warp at once
+  const int sub = lane % lanes, first = k0 + warp * per + lane / lanes;
+  const T* key = reinterpret_cast<const T*>(a.krot) + (size_t)b * a.cap * a.S + 8 * sub;
+  uint4 early[kKeys / 8];
+#pragma unroll
+  for (int i = 0; i < kKeys / 8; ++i) {
+    const int k = first + i * 8 * per;
+    early[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (i * per < kKeys / 8 && k < a.pos) early[i] = __ldcg(reinterpret_cast<const uint4*>(key + (size_t)k * a.S));
+  }
+  pdl_wait();
+  pdl_next();
   const int S = a.S, F = 2 * a.D + S + a.E, n = a.pos + 1;
   const T* z = reinterpret_cast<const T*>(a.base) + (size_t)b * F + a.D;
   float ss = 0.f;
@@ -200,7 +192,6 @@ __global__ void __launch_bounds__(256) block_score_kernel(BlockStep a) {
 #pragma unroll
   for (int k = 0; k < 8; ++k) ss += red[k];
   const float inv = 1.f / fmaxf(sqrtf(ss), a.qk_eps);
-  const int k0 = blockIdx.x * kKeys;
   const bool owner = k0 <= a.pos && a.pos < k0 + kKeys;   // this block's keys include the new one
   const float2* rot = reinterpret_cast<const float2*>(a.rot) + (size_t)a.pos * (S / 2);
   for (int j = tid; j < S / 2; j += 256) {
@@ -221,16 +212,16 @@ __global__ void __launch_bounds__(256) block_score_kernel(BlockStep a) {
     }
   }
   __syncthreads();   // (also orders the new key's row before its read below)
-  const int lanes = S / 8;             // lanes of a key (8, 16 or 32)
-  const int per = 32 / lanes;          // keys of a warp at once
-  const int sub = lane % lanes;
-  for (int k = k0 + warp * per + lane / lanes; k < k0 + kKeys; k += 8 * per) {
+#pragma unroll
+  for (int i = 0; i < kKeys / 8; ++i) {
+    const int k = first + i * 8 * per;
+    if (i * per >= kKeys / 8) break;
     float s = 0.f;
     if (k < n) {
-      const uint4 v = *reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(a.krot) + ((size_t)b * a.cap + k) * S + 8 * sub);
+      const uint4 v = k < a.pos ? early[i] : *reinterpret_cast<const uint4*>(key + (size_t)k * S);
       const T* e = reinterpret_cast<const T*>(&v);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) s = fmaf(Elem<T>::ld_shared(e + i), qs[8 * sub + i], s);
+      for (int j = 0; j < 8; ++j) s = fmaf(Elem<T>::ld_shared(e + j), qs[8 * sub + j], s);
     }
     for (int o = lanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (sub == 0 && k < n) a.scores[(size_t)b * a.cap + k] = s;
@@ -244,9 +235,22 @@ __global__ void __launch_bounds__(256) block_attend_kernel(BlockStep a) {
   float* w = reinterpret_cast<float*>(smem);   // [n] weights, then [8][64] partial sums
   __shared__ float red[8];
   pdl_next();
-  pdl_wait();
   const int b = blockIdx.y, c0 = blockIdx.x * 64, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n = a.pos + 1;
+  const int cv = tid & 7, kr = tid >> 3;
+  const int col = c0 + 8 * cv;
+  const T* val = reinterpret_cast<const T*>(a.values) + (size_t)b * a.cap * a.E + col;
+  constexpr int kDeep = 8;
+  uint4 r[kDeep];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int u = 0; u < kDeep; ++u) {
+      const int k = k0 + 32 * u;
+      r[u] = k < n && col < a.E ? __ldcg(reinterpret_cast<const uint4*>(val + (size_t)k * a.E)) : make_uint4(0u, 0u, 0u, 0u);
+    }
+  };
+  fetch(kr);   // (the values are complete: the launch before this one waited for those that write them)
+  pdl_wait();
   const float* sc = a.scores + (size_t)b * a.cap;
   float m = -INFINITY;
   for (int k = tid; k < n; k += 256) {
@@ -275,29 +279,18 @@ __global__ void __launch_bounds__(256) block_attend_kernel(BlockStep a) {
 #pragma unroll
   for (int k = 0; k < 8; ++k) sum += red[k];
   const float inv = sum > 0.f ? 1.f / sum : 0.f;
-  const int cv = tid & 7, kr = tid >> 3;
-  const int col = c0 + 8 * cv;
   float acc[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-  if (col < a.E) {
-    const T* v = reinterpret_cast<const T*>(a.values) + (size_t)b * a.cap * a.E + col;
-    constexpr int kDeep = 8;
-    for (int k0 = kr; k0 < n; k0 += 32 * kDeep) {
-      uint4 r[kDeep];
+  for (int k0 = kr; k0 < n; k0 += 32 * kDeep) {
+    if (k0 != kr) fetch(k0);
 #pragma unroll
-      for (int u = 0; u < kDeep; ++u) {
-        const int k = k0 + 32 * u;
-        r[u] = k < n ? *reinterpret_cast<const uint4*>(v + (size_t)k * a.E) : make_uint4(0u, 0u, 0u, 0u);
-      }
+    for (int u = 0; u < kDeep; ++u) {
+      const int k = k0 + 32 * u;
+      const float wk = k < n ? w[k] : 0.f;
+      const T* e = reinterpret_cast<const T*>(&r[u]);
 #pragma unroll
-      for (int u = 0; u < kDeep; ++u) {
-        const int k = k0 + 32 * u;
-        const float wk = k < n ? w[k] : 0.f;
-        const T* e = reinterpret_cast<const T*>(&r[u]);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) acc[i] = fmaf(wk, Elem<T>::ld_shared(e + i), acc[i]);
-      }
+      for (int i = 0; i < 8; ++i) acc[i] = fmaf(wk, Elem<T>::ld_shared(e + i), acc[i]);
     }
   }
   // a warp holds four keys' partial sums of the 64 columns
@@ -427,10 +420,10 @@ extern "C" int mega_block_step(const mega_block_step_args* p, mega_stream_t stre
       p->complex_poles
           ? cema_step_lanes_try(p->dtype, p->x, mx, xn, B, D, p->ndim, (const long long*)p->count, p->mean, p->var,
                                 p->norm_gamma, p->norm_beta, (float)p->norm_eps, p->p, p->q, p->gamma_hat, p->omega, p->h,
-                                p->h, 1, stream, (long long*)p->count_next)
+                                p->h, 1, stream, (long long*)p->count_next, true)
           : step_lanes_try(p->dtype, p->x, mx, xn, B, D, p->ndim, (const long long*)p->count, p->mean, p->var, p->norm_gamma,
                            p->norm_beta, (float)p->norm_eps, p->p, p->q, p->gamma_hat, p->omega, p->h, p->h, 1, stream,
-                           (long long*)p->count_next);
+                           (long long*)p->count_next, true);
   if (!ok) return MEGA_ERR_UNSUPPORTED;
 #define MEGA_BLOCK_STEP(TY)                                \
   if (B <= 8) step_launches<TY, 1>(a, s);                  \

@@ -5,5 +5,5 @@ namespace mega {
 bool cema_step_lanes_try(int dtype, const void* x, void* y, void* xn_out, int B, int D, int N, const long long* count,
                          float* mean, float* var, const float* gamma, const float* beta, float eps, const float* p,
                          const float* q, const float* g, const float* omega, const float* h_in, float* h_out, int silu,
-                         void* stream, long long* count_next);
+                         void* stream, long long* count_next, bool after = false);
 }  // namespace mega

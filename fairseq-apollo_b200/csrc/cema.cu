@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(128) cema_step_kernel(const T* x, T* y, int B,
 // batch entries with its coefficients in registers.  h_in may be NULL and may alias h_out.
 // With use_norm the TimestepNorm update of the token runs first (redundantly in the LN lanes;
 // lane 0 stores the statistics), as in the real layer's step kernel.
-template <typename T, int LN, int BB>
+template <typename T, int LN, int BB, bool kAfter>
 __global__ void __launch_bounds__(128) cema_step_lanes_kernel(const T* __restrict__ x, T* __restrict__ y,
                                                               T* __restrict__ xn_out, int B, int D,
                                                               const long long* count, float* mean, float* var,
@@ -234,6 +234,10 @@ __global__ void __launch_bounds__(128) cema_step_lanes_kernel(const T* __restric
                                                               const float* __restrict__ omega, const float* h_in,
                                                               float* h_out, int silu, int use_norm,
                                                               long long* count_next) {
+  if (kAfter) {   // (in the step of a block; the next launch may begin once all that came before this one is done)
+    pdl_wait();
+    pdl_next();
+  }
   constexpr int N = LN * 2;
   const int sub = threadIdx.x % LN;
   const int d = blockIdx.x * (128 / LN) + threadIdx.x / LN;
@@ -326,7 +330,7 @@ static bool launch_cema_step_lanes(const T* x, T* y, T* xn_out, int B, int D, in
                                    float* mean, float* var, const float* gamma, const float* beta, float eps,
                                    const float* p, const float* q, const float* g, const float* omega,
                                    const float* h_in, float* h_out, int silu, void* stream,
-                                   long long* count_next = nullptr) {
+                                   long long* count_next = nullptr, bool after = false) {
   const int use_norm = count != nullptr;
   if (N != 2 && N != 4 && N != 8 && N != 16 && N != 32) return false;
   if (!aligned_to(h_out, 16) || (h_in && !aligned_to(h_in, 16)) || !aligned_to(p, 8) || !aligned_to(q, 16) ||
@@ -337,8 +341,14 @@ static bool launch_cema_step_lanes(const T* x, T* y, T* xn_out, int B, int D, in
   dim3 grid((unsigned)((D + 128 / ln - 1) / (128 / ln)), (unsigned)((B + BB - 1) / BB));
   if (grid.y > 65535) return false;
 #define MEGA_CEMA_STEP_LANES(LNV) \
-  launch(cema_step_lanes_kernel<T, LNV, BB>, grid, 128, 0, stream, x, y, xn_out, B, D, count, mean, var, gamma, \
-         beta, eps, p, q, g, omega, h_in, h_out, silu, use_norm, count_next)
+  do {                                                                                                    \
+    if (after)                                                                                            \
+      launch_after(cema_step_lanes_kernel<T, LNV, BB, true>, grid, 128, 0, stream, x, y, xn_out, B, D, count, mean, var, gamma, \
+         beta, eps, p, q, g, omega, h_in, h_out, silu, use_norm, count_next);   \
+    else                                                                                                  \
+      launch(cema_step_lanes_kernel<T, LNV, BB, false>, grid, 128, 0, stream, x, y, xn_out, B, D, count, mean, var, gamma, \
+         beta, eps, p, q, g, omega, h_in, h_out, silu, use_norm, count_next);        \
+  } while (0)
   if (ln == 1) MEGA_CEMA_STEP_LANES(1);
   else if (ln == 2) MEGA_CEMA_STEP_LANES(2);
   else if (ln == 4) MEGA_CEMA_STEP_LANES(4);
@@ -351,12 +361,12 @@ static bool launch_cema_step_lanes(const T* x, T* y, T* xn_out, int B, int D, in
 bool cema_step_lanes_try(int dtype, const void* x, void* y, void* xn_out, int B, int D, int N, const long long* count,
                          float* mean, float* var, const float* gamma, const float* beta, float eps, const float* p,
                          const float* q, const float* g, const float* omega, const float* h_in, float* h_out, int silu,
-                         void* stream, long long* count_next) {
+                         void* stream, long long* count_next, bool after) {
   switch (dtype) {
 #define MEGA_CEMA_STEP_CASE(DT, TY)                                                                                    \
   case DT:                                                                                                             \
     return launch_cema_step_lanes<TY>((const TY*)x, (TY*)y, (TY*)xn_out, B, D, N, count, mean, var, gamma, beta, eps,  \
-                                      p, q, g, omega, h_in, h_out, silu, stream, count_next);
+                                      p, q, g, omega, h_in, h_out, silu, stream, count_next, after);
     MEGA_CEMA_STEP_CASE(MEGA_F32, float)
     MEGA_CEMA_STEP_CASE(MEGA_BF16, __nv_bfloat16)
     MEGA_CEMA_STEP_CASE(MEGA_F16, __half)

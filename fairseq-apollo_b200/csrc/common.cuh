@@ -26,11 +26,11 @@ int check_launch(const char* what);
 
 // Single-token step with N / 4 lanes per (sequence, channel) (csrc/fused.cu): TimestepNorm update
 // when count is given, then the pole update; false (nothing launched) when N is not 4, 8, 16 or 32
-// or a state / coefficient pointer is not 16-byte aligned.
+// or a state / coefficient pointer is not 16-byte aligned.  `after`: launched as launch_after does.
 bool step_lanes_try(int dtype, const void* x, void* y, void* xn_out, int B, int D, int N, const long long* count,
                     float* mean, float* var, const float* gamma, const float* beta, float eps, const float* p,
                     const float* q, const float* g, const float* omega, const float* h_in, float* h_out, int silu,
-                    void* stream, long long* count_next = nullptr);
+                    void* stream, long long* count_next = nullptr, bool after = false);
 
 // Above the default 48 KB the dynamic shared-memory size is an opt-in attribute of the kernel ON THE CURRENT
 // DEVICE; it is raised once per kernel and device (abi.cu), as setting it costs a microsecond or two of every launch.
@@ -41,6 +41,29 @@ static inline void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_
                           Args... args) {
   if (smem > 48 * 1024) allow_smem(reinterpret_cast<const void*>(kernel), smem);
   kernel<<<grid, block, smem, (cudaStream_t)stream>>>(static_cast<KArgs>(args)...);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  g_last_kernel.store("other", std::memory_order_relaxed);
+}
+
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// A launch that may begin before the one before it on the stream has ended: its kernel waits (pdl_wait) before it reads
+// anything that launch, or any earlier one, writes, and lets its own successor begin (pdl_next) when that is safe.
+template <typename... KArgs, typename... Args>
+static inline void launch_after(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, void* stream, Args... args) {
+  if (smem > 48 * 1024) allow_smem(reinterpret_cast<const void*>(kernel), smem);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = (cudaStream_t)stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   g_last_kernel.store("other", std::memory_order_relaxed);
 }

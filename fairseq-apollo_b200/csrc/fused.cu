@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(128) tsn_ema_step_kernel(const T* __restrict__
 // the BB steps are issued before the arithmetic).  With use_norm the TimestepNorm update runs
 // redundantly in the LN lanes; lane 0 stores the statistics and the output.  h_in may be NULL
 // (zero state) and may alias h_out.
-template <typename T, int LN, int BB>
+template <typename T, int LN, int BB, bool kAfter>
 __global__ void __launch_bounds__(128) tsn_ema_step_lanes_kernel(const T* __restrict__ x, T* __restrict__ y,
                                                                  T* __restrict__ xn_out, int B, int D,
                                                                  const long long* count, float* mean, float* var,
@@ -204,6 +204,10 @@ __global__ void __launch_bounds__(128) tsn_ema_step_lanes_kernel(const T* __rest
                                                                  const float* __restrict__ omega, const float* h_in,
                                                                  float* h_out, int silu, int use_norm,
                                                                  long long* count_next) {
+  if (kAfter) {   // (in the step of a block; the next launch may begin once all that came before this one is done)
+    pdl_wait();
+    pdl_next();
+  }
   constexpr int N = LN * 4;
   const int sub = threadIdx.x % LN;
   const int d = blockIdx.x * (128 / LN) + threadIdx.x / LN;
@@ -289,7 +293,7 @@ template <typename T>
 static bool launch_step_lanes(const T* x, T* y, T* xn_out, int B, int D, int N, const long long* count, float* mean,
                               float* var, const float* gamma, const float* beta, float eps, const float* p,
                               const float* q, const float* g, const float* omega, const float* h_in, float* h_out,
-                              int silu, int use_norm, mega_stream_t stream, long long* count_next) {
+                              int silu, int use_norm, mega_stream_t stream, long long* count_next, bool after) {
   if (N != 4 && N != 8 && N != 16 && N != 32) return false;
   if (!aligned_to(h_out, 16) || (h_in && !aligned_to(h_in, 16)) || !aligned_to(p, 16) || !aligned_to(q, 16) ||
       !aligned_to(g, 16))
@@ -299,8 +303,14 @@ static bool launch_step_lanes(const T* x, T* y, T* xn_out, int B, int D, int N, 
   dim3 grid((unsigned)((D + 128 / ln - 1) / (128 / ln)), (unsigned)((B + BB - 1) / BB));
   if (grid.y > 65535) return false;
 #define MEGA_STEP_LANES(LNV)                                                                              \
-  launch(tsn_ema_step_lanes_kernel<T, LNV, BB>, grid, 128, 0, stream, x, y, xn_out, B, D, count, mean, var, \
-         gamma, beta, eps, p, q, g, omega, h_in, h_out, silu, use_norm, count_next)
+  do {                                                                                                    \
+    if (after)                                                                                            \
+      launch_after(tsn_ema_step_lanes_kernel<T, LNV, BB, true>, grid, 128, 0, stream, x, y, xn_out, B, D, count, mean, var, \
+         gamma, beta, eps, p, q, g, omega, h_in, h_out, silu, use_norm, count_next);   \
+    else                                                                                                  \
+      launch(tsn_ema_step_lanes_kernel<T, LNV, BB, false>, grid, 128, 0, stream, x, y, xn_out, B, D, count, mean, var, \
+         gamma, beta, eps, p, q, g, omega, h_in, h_out, silu, use_norm, count_next);        \
+  } while (0)
   if (ln == 1) MEGA_STEP_LANES(1);
   else if (ln == 2) MEGA_STEP_LANES(2);
   else if (ln == 4) MEGA_STEP_LANES(4);
@@ -312,20 +322,20 @@ static bool launch_step_lanes(const T* x, T* y, T* xn_out, int B, int D, int N, 
 bool step_lanes_try(int dtype, const void* x, void* y, void* xn_out, int B, int D, int N, const long long* count,
                     float* mean, float* var, const float* gamma, const float* beta, float eps, const float* p,
                     const float* q, const float* g, const float* omega, const float* h_in, float* h_out, int silu,
-                    void* stream, long long* count_next) {
+                    void* stream, long long* count_next, bool after) {
   const int use_norm = count != nullptr;
   switch (dtype) {
     case MEGA_F32:
       return launch_step_lanes<float>((const float*)x, (float*)y, (float*)xn_out, B, D, N, count, mean, var, gamma,
-                                      beta, eps, p, q, g, omega, h_in, h_out, silu, use_norm, stream, count_next);
+                                      beta, eps, p, q, g, omega, h_in, h_out, silu, use_norm, stream, count_next, after);
     case MEGA_BF16:
       return launch_step_lanes<__nv_bfloat16>((const __nv_bfloat16*)x, (__nv_bfloat16*)y, (__nv_bfloat16*)xn_out, B,
                                               D, N, count, mean, var, gamma, beta, eps, p, q, g, omega, h_in, h_out,
-                                              silu, use_norm, stream, count_next);
+                                              silu, use_norm, stream, count_next, after);
     case MEGA_F16:
       return launch_step_lanes<__half>((const __half*)x, (__half*)y, (__half*)xn_out, B, D, N, count, mean, var,
                                        gamma, beta, eps, p, q, g, omega, h_in, h_out, silu, use_norm, stream,
-                                       count_next);
+                                       count_next, after);
     default:
       return false;
   }

@@ -8,6 +8,8 @@
 // the four gradients of the mx_proj output land in one matrix without copies.
 // Bound: HBM, each operand once (16384 rows, embed 1024, hidden 2048: the torch operations they replace, with their
 // slice gradients zero-filled, copied and added, took 1.1 ms of a 3.5 ms training pass).
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace mega {
@@ -132,26 +134,51 @@ __global__ void __launch_bounds__(256) gate_bwd_kernel(GateBwd p) {
 // (2, S) parameter sums and of the column sums stay in registers.
 constexpr int kQkPairs = 8;   // at most 512 features
 
+// two adjacent values (rows and pairs start at even elements of aligned arrays)
 template <typename T>
+__device__ __forceinline__ void load_pair(const T* p, float& a, float& b) {
+  using P = typename std::conditional<sizeof(T) == 4, float2, uint32_t>::type;
+  const P v = __ldg(reinterpret_cast<const P*>(p));
+  a = Elem<T>::ld_shared(reinterpret_cast<const T*>(&v));
+  b = Elem<T>::ld_shared(reinterpret_cast<const T*>(&v) + 1);
+}
+template <typename T>
+__device__ __forceinline__ void store_pair(T* p, float a, float b) {
+  using P = typename std::conditional<sizeof(T) == 4, float2, uint32_t>::type;
+  P v;
+  Elem<T>::st(reinterpret_cast<T*>(&v), a);
+  Elem<T>::st(reinterpret_cast<T*>(&v) + 1, b);
+  *reinterpret_cast<P*>(p) = v;
+}
+
+// kP: pairs of a lane (1, 2, 4 or 8): the sums of 64 features are 10 registers, those of 512 are 80 and leave few warps.
+template <typename T, int kP>
 __global__ void __launch_bounds__(256) gate_qk_bwd_kernel(const T* z, long long ldz, const float* gamma, const float* rot,
                                                           int period, int q_offset, const T* dq, long long ldq, const T* dk,
                                                           long long ldk, T* dz, long long ldd, float* dgamma, float* dbeta,
                                                           float* colsum, long long rows, int cols, float eps) {
   __shared__ float red[8][128];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = cols >> 1;
-  float sg0[2 * kQkPairs], sg1[2 * kQkPairs], sb0[2 * kQkPairs], sb1[2 * kQkPairs], sz[2 * kQkPairs];
+  float sg0[2 * kP], sg1[2 * kP], sb0[2 * kP], sb1[2 * kP], sz[2 * kP];
 #pragma unroll
-  for (int i = 0; i < 2 * kQkPairs; ++i) sg0[i] = sg1[i] = sb0[i] = sb1[i] = sz[i] = 0.f;
+  for (int i = 0; i < 2 * kP; ++i) sg0[i] = sg1[i] = sb0[i] = sb1[i] = sz[i] = 0.f;
   for (long long r = (long long)blockIdx.x * 8 + warp; r < rows; r += (long long)gridDim.x * 8) {
-    float zn[2 * kQkPairs], d[2 * kQkPairs];
+    float zn[2 * kP], d[2 * kP], gq[2 * kP], gk[2 * kP];
     float ss = 0.f;
 #pragma unroll
-    for (int i = 0; i < kQkPairs; ++i) {
+    for (int i = 0; i < kP; ++i) {
+      const int j = lane + 32 * i;
+      if (j < half) {
+        load_pair(dq + r * ldq + 2 * j, gq[2 * i], gq[2 * i + 1]);
+        load_pair(dk + r * ldk + 2 * j, gk[2 * i], gk[2 * i + 1]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kP; ++i) {
       const int j = lane + 32 * i;
       zn[2 * i] = zn[2 * i + 1] = d[2 * i] = d[2 * i + 1] = 0.f;
       if (j < half) {
-        zn[2 * i] = Elem<T>::ld(z + r * ldz + 2 * j);
-        zn[2 * i + 1] = Elem<T>::ld(z + r * ldz + 2 * j + 1);
+        load_pair(z + r * ldz + 2 * j, zn[2 * i], zn[2 * i + 1]);
         ss = fmaf(zn[2 * i], zn[2 * i], fmaf(zn[2 * i + 1], zn[2 * i + 1], ss));
       }
     }
@@ -164,12 +191,11 @@ __global__ void __launch_bounds__(256) gate_qk_bwd_kernel(const T* z, long long 
     const float2* rq = reinterpret_cast<const float2*>(rot) + (size_t)(pos + q_offset) * half;
     float dots = 0.f;
 #pragma unroll
-    for (int i = 0; i < kQkPairs; ++i) {
+    for (int i = 0; i < kP; ++i) {
       const int j = lane + 32 * i;
       if (j < half) {
         const int c = 2 * j;
-        float qa = Elem<T>::ld(dq + r * ldq + c), qb = Elem<T>::ld(dq + r * ldq + c + 1);
-        float ka = Elem<T>::ld(dk + r * ldk + c), kb = Elem<T>::ld(dk + r * ldk + c + 1);
+        float qa = gq[2 * i], qb = gq[2 * i + 1], ka = gk[2 * i], kb = gk[2 * i + 1];
         if (rot) {   // the transposed rotations
           const float2 wq = __ldg(rq + j), wk = __ldg(rk + j);
           const float q0 = qa * wq.x + qb * wq.y, k0 = ka * wk.x + kb * wk.y;
@@ -197,22 +223,21 @@ __global__ void __launch_bounds__(256) gate_qk_bwd_kernel(const T* z, long long 
     for (int o = 16; o > 0; o >>= 1) dots += __shfl_xor_sync(0xffffffffu, dots, o);
     if (norm < eps) dots = 0.f;   // the divisor is eps itself
 #pragma unroll
-    for (int i = 0; i < kQkPairs; ++i) {
+    for (int i = 0; i < kP; ++i) {
       const int j = lane + 32 * i;
       if (j < half) {
         const float v0 = inv * (d[2 * i] - zn[2 * i] * dots), v1 = inv * (d[2 * i + 1] - zn[2 * i + 1] * dots);
-        Elem<T>::st(dz + r * ldd + 2 * j, v0);
-        Elem<T>::st(dz + r * ldd + 2 * j + 1, v1);
+        store_pair(dz + r * ldd + 2 * j, v0, v1);
         sz[2 * i] += v0;
         sz[2 * i + 1] += v1;
       }
     }
   }
   // the block's eight warps, two values of every lane at a time
-  auto flush = [&](const float(&s)[2 * kQkPairs], float* out) {
+  auto flush = [&](const float(&s)[2 * kP], float* out) {
     if (!out) return;
 #pragma unroll
-    for (int i = 0; i < kQkPairs; ++i) {
+    for (int i = 0; i < kP; ++i) {
       if (64 * i >= cols) break;
       __syncthreads();
       red[warp][2 * lane] = s[2 * i];
@@ -234,6 +259,75 @@ __global__ void __launch_bounds__(256) gate_qk_bwd_kernel(const T* z, long long 
 }
 
 // softmax over a row of scores + bias[column - row + span - 1], padded columns out; a fully padded row takes no mask
+// Rows of at most 2048 values of 16 bits (1024 fp32) in whole 16-byte pieces: a warp takes one, kN pieces per lane, in
+// registers.  Bound by the bias's unaligned loads (a diagonal per row) and the instructions around them.
+template <typename T, int kN>
+__global__ void __launch_bounds__(256) bias_softmax_warp_kernel(const T* x, T* y, const T* bias, const unsigned char* mask, int rows,
+                                                                int cols, int span) {
+  constexpr int kV = 16 / (int)sizeof(T);
+  using M = typename std::conditional<kV == 8, uint2, unsigned>::type;   // the mask of a piece
+  const int lane = threadIdx.x & 31, b = blockIdx.y, r = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (r >= rows) return;
+  const T* xr = x + ((size_t)b * rows + r) * cols;
+  T* yr = y + ((size_t)b * rows + r) * cols;
+  const T* br = bias + (span - 1 - r);
+  float v[kN][kV];
+  unsigned pad[kN];
+  bool live = mask == nullptr;
+#pragma unroll
+  for (int j = 0; j < kN; ++j) {
+    const int c = (lane + 32 * j) * kV;
+    pad[j] = 0u;
+    if (c < cols) {
+      const uint4 raw = *reinterpret_cast<const uint4*>(xr + c);
+      if (mask) {
+        const M m = __ldg(reinterpret_cast<const M*>(mask + (size_t)b * cols + c));
+        const unsigned char* e = reinterpret_cast<const unsigned char*>(&m);
+#pragma unroll
+        for (int k = 0; k < kV; ++k) pad[j] |= (e[k] != 0 ? 1u : 0u) << k;
+        live |= pad[j] != (1u << kV) - 1u;
+      }
+#pragma unroll
+      for (int k = 0; k < kV; ++k) v[j][k] = Elem<T>::ld_shared(reinterpret_cast<const T*>(&raw) + k) + Elem<T>::ld(br + c + k);
+    } else {
+#pragma unroll
+      for (int k = 0; k < kV; ++k) v[j][k] = -INFINITY;
+    }
+  }
+  const bool all = !__any_sync(0xffffffffu, live);   // (padded throughout: as without a mask)
+  float m = -INFINITY;
+#pragma unroll
+  for (int j = 0; j < kN; ++j)
+#pragma unroll
+    for (int k = 0; k < kV; ++k) {
+      if (!all && ((pad[j] >> k) & 1u)) v[j][k] = -INFINITY;
+      m = fmaxf(m, v[j][k]);
+    }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  float s = 0.f;
+#pragma unroll
+  for (int j = 0; j < kN; ++j)
+#pragma unroll
+    for (int k = 0; k < kV; ++k) {
+      v[j][k] = m == -INFINITY ? 0.f : __expf(v[j][k] - m);
+      s += v[j][k];
+    }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  const float inv = s > 0.f ? 1.f / s : 0.f;
+#pragma unroll
+  for (int j = 0; j < kN; ++j) {
+    const int c = (lane + 32 * j) * kV;
+    if (c < cols) {
+      uint4 raw;
+#pragma unroll
+      for (int k = 0; k < kV; ++k) Elem<T>::st(reinterpret_cast<T*>(&raw) + k, v[j][k] * inv);
+      *reinterpret_cast<uint4*>(yr + c) = raw;
+    }
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(128) bias_softmax_kernel(const T* x, T* y, const T* bias, const unsigned char* mask,
                                                            int rows, int cols, int span) {
@@ -379,10 +473,17 @@ extern "C" int mega_gate_qk_bwd(const void* z, int64_t ld_z, const float* gamma,
   if (cols > 64 * kQkPairs) return MEGA_ERR_UNSUPPORTED;
   const long long want = (rows + 31) / 32;   // four rows per warp at least
   const unsigned grid = (unsigned)(want > 148 * 4 ? 148 * 4 : want);
-  MEGA_DISPATCH_DTYPE(dtype, launch(gate_qk_bwd_kernel<T>, grid, 256, 0, stream, (const T*)z, (long long)ld_z, gamma, rot,
-                                    rot ? period : 1, q_offset, (const T*)dq, (long long)ld_dq, (const T*)dk,
-                                    (long long)ld_dk, (T*)dz, (long long)ld_dz, dgamma, dbeta, colsum, (long long)rows, cols,
-                                    (float)eps));
+  MEGA_DISPATCH_DTYPE(dtype, {
+    auto run = [&](auto kernel) {
+      launch(kernel, grid, 256, 0, stream, (const T*)z, (long long)ld_z, gamma, rot, rot ? period : 1, q_offset, (const T*)dq,
+             (long long)ld_dq, (const T*)dk, (long long)ld_dk, (T*)dz, (long long)ld_dz, dgamma, dbeta, colsum, (long long)rows, cols,
+             (float)eps);
+    };
+    if (cols <= 64) run(gate_qk_bwd_kernel<T, 1>);
+    else if (cols <= 128) run(gate_qk_bwd_kernel<T, 2>);
+    else if (cols <= 256) run(gate_qk_bwd_kernel<T, 4>);
+    else run(gate_qk_bwd_kernel<T, kQkPairs>);
+  });
   return check_launch("gate_qk_bwd");
 }
 
@@ -393,6 +494,21 @@ extern "C" int mega_attention_bias_softmax_fwd(const void* x, void* y, const voi
   if (batch <= 0 || batch > 65535 || rows <= 0 || cols <= 0 || span < rows || span < cols) return MEGA_ERR_SHAPE;
   if (cols > 48 * 1024) return MEGA_ERR_UNSUPPORTED;   // a row lives in shared memory
   const dim3 grid(rows, (unsigned)batch);
+  const int kv = 16 / elem_size(dtype);
+  if (cols % kv == 0 && cols <= 8 * 32 * kv && aligned_to(x, 16) && aligned_to(y, 16) && aligned_to(pad_mask, kv)) {
+    const dim3 gridw((rows + 7) / 8, (unsigned)batch);
+    const int vecs = (cols / kv + 31) / 32;
+    MEGA_DISPATCH_DTYPE(dtype, {
+      auto run = [&](auto kernel) {
+        launch(kernel, gridw, 256, 0, stream, (const T*)x, (T*)y, (const T*)bias, pad_mask, rows, cols, span);
+      };
+      if (vecs <= 1) run(bias_softmax_warp_kernel<T, 1>);
+      else if (vecs <= 2) run(bias_softmax_warp_kernel<T, 2>);
+      else if (vecs <= 4) run(bias_softmax_warp_kernel<T, 4>);
+      else run(bias_softmax_warp_kernel<T, 8>);
+    });
+    return check_launch("attention_bias_softmax_fwd");
+  }
   MEGA_DISPATCH_DTYPE(dtype, launch(bias_softmax_kernel<T>, grid, 128, (size_t)cols * 4, stream, (const T*)x, (T*)y,
                                     (const T*)bias, pad_mask, rows, cols, span));
   return check_launch("attention_bias_softmax_fwd");

@@ -351,84 +351,67 @@ __global__ void gate_kernel(const T* a, long long lda, const T* b, long long ldb
   }
 }
 
-// The same gates, 16 bytes per access (8 bf16 / fp16 or 4 fp32 values), for column counts, row
-// pitches and base addresses that are multiples of 16 bytes; a thread takes kU vectors a grid
-// stride apart, all loads first.  vpr = vectors per row.
-template <typename T>
-struct GateVec {
-  static constexpr int kN = 16 / (int)sizeof(T);
-  static __device__ __forceinline__ void load(const T* p, float (&f)[kN]) {
-    const uint4 v = __ldcs(reinterpret_cast<const uint4*>(p));   // read once: streaming
-    const T* e = reinterpret_cast<const T*>(&v);
-#pragma unroll
-    for (int k = 0; k < kN; ++k) f[k] = Elem<T>::ld_shared(e + k);
-  }
-  static __device__ __forceinline__ void store(T* p, const float (&f)[kN]) {
-    uint4 v;
-    T* e = reinterpret_cast<T*>(&v);
-#pragma unroll
-    for (int k = 0; k < kN; ++k) Elem<T>::st(e + k, f[k]);
-    __stcs(reinterpret_cast<uint4*>(p), v);
-  }
-};
-
+// The same gates, 16 bytes per access (8 bf16 / fp16 or 4 fp32 values), for column counts, row pitches and base
+// addresses that are multiples of 16 bytes.  A block is blockDim.x vectors of blockDim.y rows, kU times; all loads first,
+// and no division (with one per vector, and a grid-stride loop: 126 us where this takes 78 on (65536, 2048) bf16).
+// Memory-bound: 2, 3 and 5 streams.
 template <typename T, int OP, int kU>
 __global__ void __launch_bounds__(256) gate_vec_kernel(const T* a, long long lda, const T* b, long long ldb, const T* c,
                                                        long long ldc, const T* d, long long ldd, T* y, long long ldy,
-                                                       unsigned nvec, unsigned vpr) {
-  constexpr int kN = GateVec<T>::kN;
-  const unsigned stride = gridDim.x * blockDim.x;
-  for (unsigned v0 = blockIdx.x * blockDim.x + threadIdx.x; v0 < nvec; v0 += kU * stride) {
-    float fa[kU][kN], fb[kU][kN], fc[kU][kN], fd[kU][kN];
-    long long off[kU][5];
+                                                       long long rows, int cols) {
+  constexpr int kN = 16 / (int)sizeof(T);
+  const int col = (blockIdx.y * blockDim.x + threadIdx.x) * kN;
+  if (col >= cols) return;
+  const long long r0 = (long long)blockIdx.x * blockDim.y * kU + threadIdx.y;
+  uint4 va[kU], vb[kU], vc[OP == 2 ? kU : 1], vd[OP == 2 ? kU : 1];
 #pragma unroll
-    for (int u = 0; u < kU; ++u) {
-      const unsigned v = v0 + u * stride;
-      if (v < nvec) {
-        const unsigned r = v / vpr;
-        const long long col = (long long)(v - r * vpr) * kN;
-        off[u][0] = r * lda + col; off[u][1] = r * ldb + col; off[u][2] = r * ldc + col; off[u][3] = r * ldd + col;
-        off[u][4] = r * ldy + col;
-        GateVec<T>::load(a + off[u][0], fa[u]);
-        if (OP != 0 || b != nullptr) GateVec<T>::load(b + off[u][1], fb[u]);
-        if (OP == 2) {
-          GateVec<T>::load(c + off[u][2], fc[u]);
-          GateVec<T>::load(d + off[u][3], fd[u]);
-        }
+  for (int u = 0; u < kU; ++u) {
+    const long long r = r0 + u * blockDim.y;
+    if (r < rows) {
+      va[u] = *reinterpret_cast<const uint4*>(a + r * lda + col);
+      if (OP != 0 || b != nullptr) vb[u] = *reinterpret_cast<const uint4*>(b + r * ldb + col);
+      if (OP == 2) {
+        vc[OP == 2 ? u : 0] = *reinterpret_cast<const uint4*>(c + r * ldc + col);
+        vd[OP == 2 ? u : 0] = *reinterpret_cast<const uint4*>(d + r * ldd + col);
       }
     }
+  }
 #pragma unroll
-    for (int u = 0; u < kU; ++u) {
-      const unsigned v = v0 + u * stride;
-      if (v < nvec) {
-        float out[kN];
-        // 16-bit outputs: SiLU and the sigmoid from one tanh.approx each (relative error ~2^-11, below
-        // the rounding of the output); fp32 keeps the exponential forms
-        constexpr bool kFast = sizeof(T) == 2;
+  for (int u = 0; u < kU; ++u) {
+    const long long r = r0 + u * blockDim.y;
+    if (r >= rows) break;
+    const T *fa = reinterpret_cast<const T*>(&va[u]), *fb = reinterpret_cast<const T*>(&vb[u]),
+            *fc = reinterpret_cast<const T*>(&vc[OP == 2 ? u : 0]), *fd = reinterpret_cast<const T*>(&vd[OP == 2 ? u : 0]);
+    uint4 out;
+    T* o = reinterpret_cast<T*>(&out);
+    // 16-bit outputs: SiLU and the sigmoid from one tanh.approx each (relative error ~2^-11, below
+    // the rounding of the output); fp32 keeps the exponential forms
+    constexpr bool kFast = sizeof(T) == 2;
 #pragma unroll
-        for (int k = 0; k < kN; ++k) {
-          if (OP == 0) {  // silu(a [+ b])
-            const float v = b != nullptr ? fa[u][k] + fb[u][k] : fa[u][k];
-            out[k] = kFast ? silu_tanh(v) : siluf_(v);
-          } else if (OP == 1) {  // a * silu(b)
-            out[k] = fa[u][k] * (kFast ? silu_tanh(fb[u][k]) : siluf_(fb[u][k]));
-          } else {  // a = residual, b = u, c = hx, d = h_lin
-            float g;
-            if (kFast) {
-              float t;
-              asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(0.5f * fb[u][k]));
-              g = fmaf(0.5f, t, 0.5f);
-            } else {
-              g = sigmoidf_(fb[u][k]);
-            }
-            const float hs = fc[u][k] + fd[u][k];
-            const float h = kFast ? silu_tanh(hs) : siluf_(hs);
-            out[k] = fmaf(g, h - fa[u][k], fa[u][k]);
-          }
+    for (int k = 0; k < kN; ++k) {
+      const float x = Elem<T>::ld_shared(fa + k);
+      if (OP == 0) {  // silu(a [+ b])
+        const float v = b != nullptr ? x + Elem<T>::ld_shared(fb + k) : x;
+        Elem<T>::st(o + k, kFast ? silu_tanh(v) : siluf_(v));
+      } else if (OP == 1) {  // a * silu(b)
+        const float v = Elem<T>::ld_shared(fb + k);
+        Elem<T>::st(o + k, x * (kFast ? silu_tanh(v) : siluf_(v)));
+      } else {  // a = residual, b = u, c = hx, d = h_lin
+        const float v = Elem<T>::ld_shared(fb + k);
+        float g;
+        if (kFast) {
+          float t;
+          asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(0.5f * v));
+          g = fmaf(0.5f, t, 0.5f);
+        } else {
+          g = sigmoidf_(v);
         }
-        GateVec<T>::store(y + off[u][4], out);
+        const float hs = Elem<T>::ld_shared(fc + k) + Elem<T>::ld_shared(fd + k);
+        const float h = kFast ? silu_tanh(hs) : siluf_(hs);
+        Elem<T>::st(o + k, fmaf(g, h - x, x));
       }
     }
+    *reinterpret_cast<uint4*>(y + r * ldy + col) = out;
   }
 }
 
@@ -462,8 +445,8 @@ __global__ void gate_qk_kernel(const T* z, long long ldz, const float* gamma, co
 // on the unrounded affine results.
 template <typename T>
 __global__ void gate_qk_rotary_kernel(const T* z, long long ldz, const float* gamma, const float* beta,
-                                      const float* rot, int period, int q_offset, T* qo, long long ldq, T* ko,
-                                      long long ldk, long long rows, int cols, float eps) {
+                                      const float* rot, int period, int q_offset, int out_period, T* qo, long long ldq, T* ko,
+                                      long long ldk, T* kraw, long long rows, int cols, float eps) {
   const int lane = threadIdx.x & 31;
   const int half = cols >> 1;
   const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -478,6 +461,7 @@ __global__ void gate_qk_rotary_kernel(const T* z, long long ldz, const float* ga
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     const float inv = 1.f / fmaxf(sqrtf(ss), eps);
     const int pos = (int)(r % period);
+    const long long at = r / period * out_period + pos;
     const float2* rk = reinterpret_cast<const float2*>(rot) + (size_t)pos * half;
     const float2* rq = reinterpret_cast<const float2*>(rot) + (size_t)(pos + q_offset) * half;
     for (int j = lane; j < half; j += 32) {
@@ -487,11 +471,74 @@ __global__ void gate_qk_rotary_kernel(const T* z, long long ldz, const float* ga
       const float ka = fmaf(a, gamma[cols + c] + 1.f, beta[cols + c]);
       const float kb = fmaf(b, gamma[cols + c + 1] + 1.f, beta[cols + c + 1]);
       const float2 wq = __ldg(rq + j), wk = __ldg(rk + j);
-      Elem<T>::st(qo + r * ldq + c, qa * wq.x - qb * wq.y);
-      Elem<T>::st(qo + r * ldq + c + 1, qa * wq.y + qb * wq.x);
-      Elem<T>::st(ko + r * ldk + c, ka * wk.x - kb * wk.y);
-      Elem<T>::st(ko + r * ldk + c + 1, ka * wk.y + kb * wk.x);
+      Elem<T>::st(qo + at * ldq + c, qa * wq.x - qb * wq.y);
+      Elem<T>::st(qo + at * ldq + c + 1, qa * wq.y + qb * wq.x);
+      Elem<T>::st(ko + at * ldk + c, ka * wk.x - kb * wk.y);
+      Elem<T>::st(ko + at * ldk + c + 1, ka * wk.y + kb * wk.x);
+      if (kraw) {
+        Elem<T>::st(kraw + r * cols + c, ka);
+        Elem<T>::st(kraw + r * cols + c + 1, kb);
+      }
     }
+  }
+}
+
+// The same, 16 bytes per access, for 16-bit types and 64, 128 or 256 features: kLanes lanes take a row, eight features
+// each.  Rows of a chunk may be written at a pitch of their own (out_period >= period rows per chunk), and the keys also
+// as they are before the rotation (kraw, contiguous rows, or null), which is what a decoding cache keeps.  Memory-bound.
+template <typename T, int kLanes>
+__global__ void __launch_bounds__(256) gate_qk_rotary_vec_kernel(const T* z, long long ldz, const float* gamma, const float* beta,
+                                                                 const float* rot, int period, int q_offset, int out_period, T* qo,
+                                                                 long long ldq, T* ko, long long ldk, T* kraw, long long rows,
+                                                                 float eps) {
+  constexpr int kCols = kLanes * 8, kPer = 32 / kLanes;
+  const int lane = threadIdx.x & 31, sub = lane % kLanes, c = 8 * sub;
+  const long long first = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * (2 * kPer) + lane / kLanes;
+  uint4 in[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {   // (two rows at once: more bytes in flight)
+    const long long r = first + u * kPer;
+    in[u] = make_uint4(0u, 0u, 0u, 0u);
+    if (r < rows) in[u] = *reinterpret_cast<const uint4*>(z + r * ldz + c);
+  }
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const long long r = first + u * kPer;
+    const T* e = reinterpret_cast<const T*>(&in[u]);
+    float f[8], ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      f[i] = Elem<T>::ld_shared(e + i);
+      ss = fmaf(f[i], f[i], ss);
+    }
+#pragma unroll
+    for (int o = kLanes / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if (r >= rows) break;
+    const float inv = 1.f / fmaxf(sqrtf(ss), eps);
+    const long long chunk = r / period;
+    const int pos = (int)(r - chunk * period);
+    const float4* rk = reinterpret_cast<const float4*>(rot + (size_t)pos * kCols + c);
+    const float4* rq = reinterpret_cast<const float4*>(rot + (size_t)(pos + q_offset) * kCols + c);
+    uint4 qv, kv, kw;
+    T *qp = reinterpret_cast<T*>(&qv), *kp = reinterpret_cast<T*>(&kv), *wp = reinterpret_cast<T*>(&kw);
+#pragma unroll
+    for (int i = 0; i < 8; i += 4) {
+      const float4 g0 = __ldg(reinterpret_cast<const float4*>(gamma + c + i)), g1 = __ldg(reinterpret_cast<const float4*>(gamma + kCols + c + i));
+      const float4 b0 = __ldg(reinterpret_cast<const float4*>(beta + c + i)), b1 = __ldg(reinterpret_cast<const float4*>(beta + kCols + c + i));
+      const float4 wq = __ldg(rq + i / 4), wk = __ldg(rk + i / 4);
+      const float x0 = f[i] * inv, x1 = f[i + 1] * inv, x2 = f[i + 2] * inv, x3 = f[i + 3] * inv;
+      const float q0 = fmaf(x0, g0.x + 1.f, b0.x), q1 = fmaf(x1, g0.y + 1.f, b0.y), q2 = fmaf(x2, g0.z + 1.f, b0.z), q3 = fmaf(x3, g0.w + 1.f, b0.w);
+      const float k0 = fmaf(x0, g1.x + 1.f, b1.x), k1 = fmaf(x1, g1.y + 1.f, b1.y), k2 = fmaf(x2, g1.z + 1.f, b1.z), k3 = fmaf(x3, g1.w + 1.f, b1.w);
+      Elem<T>::st(qp + i, q0 * wq.x - q1 * wq.y); Elem<T>::st(qp + i + 1, q0 * wq.y + q1 * wq.x);
+      Elem<T>::st(qp + i + 2, q2 * wq.z - q3 * wq.w); Elem<T>::st(qp + i + 3, q2 * wq.w + q3 * wq.z);
+      Elem<T>::st(kp + i, k0 * wk.x - k1 * wk.y); Elem<T>::st(kp + i + 1, k0 * wk.y + k1 * wk.x);
+      Elem<T>::st(kp + i + 2, k2 * wk.z - k3 * wk.w); Elem<T>::st(kp + i + 3, k2 * wk.w + k3 * wk.z);
+      Elem<T>::st(wp + i, k0); Elem<T>::st(wp + i + 1, k1); Elem<T>::st(wp + i + 2, k2); Elem<T>::st(wp + i + 3, k3);
+    }
+    const long long at = chunk * out_period + pos;
+    *reinterpret_cast<uint4*>(qo + at * ldq + c) = qv;
+    *reinterpret_cast<uint4*>(ko + at * ldk + c) = kv;
+    if (kraw) *reinterpret_cast<uint4*>(kraw + r * kCols + c) = kw;
   }
 }
 
@@ -650,23 +697,22 @@ static int gate_common(int op, const void* a, int64_t lda, const void* b, int64_
     const int vn = 16 / elem_size(dtype);
     const long long es = elem_size(dtype);
     auto ok16 = [&](const void* p, long long ld) { return p == nullptr || (aligned_to(p, 16) && (ld * es) % 16 == 0); };
-    const long long nvec = n / vn;
-    if (cols % vn == 0 && ok16(a, lda) && ok16(b, ldb) && ok16(c, ldc) && ok16(d, ldd) && ok16(y, ldy) &&
-        nvec < 0xffffffffLL) {
-      constexpr int kU = 2;
-      const long long want = (nvec + 256 * kU - 1) / (256 * kU);
-      const unsigned gridv = (unsigned)(want > 148 * 32 ? 148 * 32 : want);
-      const unsigned vpr = (unsigned)(cols / vn);
+    const int vpr = cols / vn;
+    int bx = 32;
+    while (bx < vpr && bx < 256) bx *= 2;
+    constexpr int kU = 4;
+    const int by = 256 / bx;
+    const long long gx = (rows + by * kU - 1) / (by * kU);
+    if (cols % vn == 0 && ok16(a, lda) && ok16(b, ldb) && ok16(c, ldc) && ok16(d, ldd) && ok16(y, ldy) && gx < 0x7fffffffLL) {
+      const dim3 gridv((unsigned)gx, (unsigned)((vpr + bx - 1) / bx)), blockv(bx, by);
       MEGA_DISPATCH_DTYPE(dtype, {
-        if (op == 0)
-          launch(gate_vec_kernel<T, 0, kU>, gridv, 256, 0, stream, (const T*)a, lda, (const T*)b, ldb, (const T*)c, ldc,
-                 (const T*)d, ldd, (T*)y, ldy, (unsigned)nvec, vpr);
-        else if (op == 1)
-          launch(gate_vec_kernel<T, 1, kU>, gridv, 256, 0, stream, (const T*)a, lda, (const T*)b, ldb, (const T*)c, ldc,
-                 (const T*)d, ldd, (T*)y, ldy, (unsigned)nvec, vpr);
-        else
-          launch(gate_vec_kernel<T, 2, kU>, gridv, 256, 0, stream, (const T*)a, lda, (const T*)b, ldb, (const T*)c, ldc,
-                 (const T*)d, ldd, (T*)y, ldy, (unsigned)nvec, vpr);
+        auto run = [&](auto kernel) {
+          launch(kernel, gridv, blockv, 0, stream, (const T*)a, lda, (const T*)b, ldb, (const T*)c, ldc, (const T*)d, ldd, (T*)y, ldy,
+                 rows, cols);
+        };
+        if (op == 0) run(gate_vec_kernel<T, 0, kU>);
+        else if (op == 1) run(gate_vec_kernel<T, 1, kU>);
+        else run(gate_vec_kernel<T, 2, kU>);
       });
       return check_launch("gate");
     }
@@ -721,21 +767,49 @@ extern "C" int mega_gate_qk(const void* z, int64_t ld_z, const float* gamma, con
   return check_launch("gate_qk");
 }
 
-extern "C" int mega_gate_qk_rotary(const void* z, int64_t ld_z, const float* gamma, const float* beta, const float* rot,
-                                   int positions, int period, int q_offset, void* q, int64_t ld_q, void* k,
-                                   int64_t ld_k, int dtype, int64_t rows, int cols, double eps, mega_stream_t stream) {
+extern "C" int mega_gate_qk_rotary_cache(const void* z, int64_t ld_z, const float* gamma, const float* beta, const float* rot,
+                                         int positions, int period, int q_offset, int out_period, void* q, int64_t ld_q, void* k,
+                                         int64_t ld_k, void* k_raw, int dtype, int64_t rows, int cols, double eps,
+                                         mega_stream_t stream) {
   if (!z || !gamma || !beta || !rot || !q || !k) return MEGA_ERR_NULL;
   if (!valid_dtype(dtype)) return MEGA_ERR_DTYPE;
-  if (rows <= 0 || cols <= 0 || (cols & 1) || period <= 0 || q_offset < 0 || period + q_offset > positions)
+  if (rows <= 0 || cols <= 0 || (cols & 1) || period <= 0 || out_period < period || q_offset < 0 || period + q_offset > positions)
     return MEGA_ERR_SHAPE;
   if (ld_z < cols || ld_q < cols || ld_k < cols) return MEGA_ERR_STRIDE;
   if (!aligned_to(rot, 8)) return MEGA_ERR_ALIGN;
+  const bool vec = elem_size(dtype) == 2 && (cols == 64 || cols == 128 || cols == 256) && ld_z % 8 == 0 && ld_q % 8 == 0 &&
+                   ld_k % 8 == 0 && aligned_to(z, 16) && aligned_to(q, 16) && aligned_to(k, 16) && aligned_to(k_raw, 16) &&
+                   aligned_to(gamma, 16) && aligned_to(beta, 16) && aligned_to(rot, 16);
+  if (vec) {
+    const int per = 8 * 2 * (256 / cols);   // rows of a block: eight warps
+    const unsigned grid = (unsigned)((rows + per - 1) / per);
+#define MEGA_QK(T)                                                                                                        \
+  {                                                                                                                       \
+    auto run = [&](auto kernel) {                                                                                         \
+      launch(kernel, grid, 256, 0, stream, (const T*)z, (long long)ld_z, gamma, beta, rot, period, q_offset, out_period, (T*)q, \
+             (long long)ld_q, (T*)k, (long long)ld_k, (T*)k_raw, (long long)rows, (float)eps);                            \
+    };                                                                                                                    \
+    if (cols == 64) run(gate_qk_rotary_vec_kernel<T, 8>);                                                                 \
+    else if (cols == 128) run(gate_qk_rotary_vec_kernel<T, 16>);                                                          \
+    else run(gate_qk_rotary_vec_kernel<T, 32>);                                                                           \
+  }
+    if (dtype == MEGA_BF16) MEGA_QK(__nv_bfloat16) else MEGA_QK(__half)
+#undef MEGA_QK
+    return check_launch("gate_qk_rotary");
+  }
   const long long blocks = (rows + 7) / 8;  // 8 warps per block, one row per warp and pass
   const unsigned grid = (unsigned)(blocks > 148 * 8 ? 148 * 8 : blocks);
   MEGA_DISPATCH_DTYPE(dtype, launch(gate_qk_rotary_kernel<T>, grid, 256, 0, stream, (const T*)z, (long long)ld_z, gamma,
-                                    beta, rot, period, q_offset, (T*)q, (long long)ld_q, (T*)k, (long long)ld_k,
-                                    (long long)rows, cols, (float)eps));
+                                    beta, rot, period, q_offset, out_period, (T*)q, (long long)ld_q, (T*)k, (long long)ld_k,
+                                    (T*)k_raw, (long long)rows, cols, (float)eps));
   return check_launch("gate_qk_rotary");
+}
+
+extern "C" int mega_gate_qk_rotary(const void* z, int64_t ld_z, const float* gamma, const float* beta, const float* rot,
+                                   int positions, int period, int q_offset, void* q, int64_t ld_q, void* k,
+                                   int64_t ld_k, int dtype, int64_t rows, int cols, double eps, mega_stream_t stream) {
+  return mega_gate_qk_rotary_cache(z, ld_z, gamma, beta, rot, positions, period, q_offset, period, q, ld_q, k, ld_k, nullptr, dtype,
+                                   rows, cols, eps, stream);
 }
 
 extern "C" int mega_norm_prepare(const int64_t* prior_count, const void* prior_mean, const void* prior_logv, const void* weight,

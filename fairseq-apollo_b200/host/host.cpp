@@ -765,6 +765,51 @@ class BlockFn : public torch::autograd::Function<BlockFn> {
   }
 };
 
+// Inference from the moving average to the output, chunked causal attention with rotary positions.  cache: the keys
+// (before their rotation) and values come back too, as a decoding state keeps them.
+std::tuple<Tensor, Tensor, Tensor> block_infer(Tensor x, Tensor xn, Tensor mx, const Tensor& wv, const Tensor& bv, const Tensor& wm,
+                                               const Tensor& bm, const Tensor& wh, const Tensor& gamma, const Tensor& beta,
+                                               const Tensor& rot, int64_t period, bool cache) {
+  on_cuda(x, xn, mx, wv, wm, wh);
+  const Where w(x);
+  const int64_t bsz = x.size(0), seq = x.size(1), d = x.size(2), rows = bsz * seq, s = gamma.size(1), e = wv.size(0);
+  const int64_t f = 2 * d + s + e, nb = rows / period;
+  const int dt = dtype_of(x);
+  const int64_t es = x.element_size();
+  x = x.contiguous();
+  const Tensor xn2 = xn.contiguous().view({rows, d}), mx2 = mx.contiguous().view({rows, d});
+  // (score rows and reduction indices in whole 16-byte pieces: the library's products are several times faster on them;
+  // the positions in between are of no row's causal range, and their values zero)
+  const int64_t pitch = period % 8 && nb <= 32 ? (period + 7) / 8 * 8 : period;
+  Tensor v_lin = at::addmm(bv, xn2, wv.t()), v3 = v_lin.view({nb, period, e}), vp = v3;
+  if (pitch != period) {
+    vp = at::empty({nb, pitch, e}, x.options());
+    vp.narrow(1, period, pitch - period).zero_();
+    v3 = vp.narrow(1, 0, period);
+    for (int64_t i = 0; i < nb; ++i)
+      check(mega_gate_silu(static_cast<char*>(v_lin.data_ptr()) + i * period * e * es, e, nullptr, 0,
+                           static_cast<char*>(vp.data_ptr()) + i * pitch * e * es, e, dt, period, (int)e, w.stream), "gate_silu");
+  } else {
+    check(mega_gate_silu(v_lin.data_ptr(), e, nullptr, 0, v_lin.data_ptr(), e, dt, rows, (int)e, w.stream), "gate_silu");
+  }
+  const Tensor base = at::addmm(bm, mx2, wm.t());
+  char* bp = static_cast<char*>(base.data_ptr());
+  char *u = bp, *z = bp + d * es, *r = z + s * es, *hx = r + e * es;
+  const Tensor ga = f32c(gamma), be = f32c(beta);
+  Tensor q = at::empty({nb, pitch, s}, x.options()), k = fresh(q), raw;
+  if (cache) raw = at::empty({bsz, seq, s}, x.options());
+  check(mega_gate_qk_rotary_cache(z, f, fptr(ga), fptr(be), fptr(rot), (int)rot.size(0), (int)period, 0, (int)pitch, q.data_ptr(), s,
+                                  k.data_ptr(), s, ptr(raw), dt, rows, (int)s, 1e-5, w.stream), "gate_qk_rotary");
+  const Tensor scores = at::bmm(q, k.transpose(1, 2));
+  Tensor wgt = fresh(scores);
+  check(mega_attention_softmax_fwd(scores.data_ptr(), wgt.data_ptr(), dt, nb, pitch, (int)pitch, 1, w.stream), "attention_softmax_fwd");
+  Tensor attn = at::bmm(wgt.narrow(1, 0, period), vp).view({rows, e});
+  check(mega_gate_mul_silu(attn.data_ptr(), e, r, f, attn.data_ptr(), e, dt, rows, (int)e, w.stream), "gate_mul_silu");
+  Tensor out = at::mm(attn, wh.t()).view({bsz, seq, d});
+  check(mega_gate_output(x.data_ptr(), d, u, f, hx, f, out.data_ptr(), d, out.data_ptr(), d, dt, rows, (int)d, w.stream), "gate_output");
+  return {out, raw, cache ? v3.reshape({bsz, seq, e}) : Tensor()};
+}
+
 Tensor block_train(const Tensor& x, const Tensor& xn, const Tensor& mx, const Tensor& wv, const Tensor& bv, const Tensor& wm,
                    const Tensor& bm, const Tensor& wh, const Tensor& gamma, const Tensor& beta, const OptTensor& bias,
                    const OptTensor& rot, const OptTensor& mask, int64_t period) {
@@ -1073,4 +1118,5 @@ PYBIND11_MODULE(_mega_host, m) {
   m.def("gate_qk", &gate_qk);
   m.def("attention_softmax_fwd", &softmax_fwd);
   m.def("block_train", &block_train);
+  m.def("block_infer", &block_infer);
 }

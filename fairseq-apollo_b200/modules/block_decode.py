@@ -13,6 +13,7 @@ import torch
 from torch import Tensor
 
 from .. import _lib, ops
+from ..block_function import qk_affine
 from ..ops import _raw_stream
 from .fused import _fp32_params, _param_names, _seed_decode_state
 
@@ -101,11 +102,7 @@ def _build(blk, x, stream, incremental_state):
                 dt, bsz, n, blk.zdim, blk.hdim, keys.data_ptr(), keys_rot.data_ptr(), values.data_ptr(), cap,
                 stream), "block_cache_fill")
         work = torch.empty(lib.mega_block_step_work(dt, bsz, dim, blk.zdim, blk.hdim, cap), dtype=torch.uint8, device=dev)
-    cache = blk.__dict__.get("_qk_fp32")
-    gver = (blk.gamma._version, blk.beta._version)
-    if cache is None or cache[0] is not blk.gamma or cache[1] is not blk.beta or cache[2] != gver:
-        cache = blk._qk_fp32 = (blk.gamma, blk.beta, gver, blk.gamma.detach().float().contiguous(),
-                                blk.beta.detach().float().contiguous())
+    qk = qk_affine(blk)
     gamma_eff, beta, p, q, g, omega = _fp32_params(norm, move)
     args = _lib.BlockStepArgs(
         dtype=dt, batch=bsz, embed=dim, zdim=blk.zdim, hdim=blk.hdim, ndim=move.ndim, complex_poles=int(move.complex),
@@ -114,13 +111,13 @@ def _build(blk, x, stream, incremental_state):
         norm_beta=beta.data_ptr(), p=p.data_ptr(), q=q.data_ptr(), gamma_hat=g.data_ptr(), omega=omega.data_ptr(),
         v_weight=blk.v_proj.weight.data_ptr(), v_bias=blk.v_proj.bias.data_ptr(),
         mx_weight=blk.mx_proj.weight.data_ptr(), mx_bias=blk.mx_proj.bias.data_ptr(),
-        h_weight=blk.h_proj.weight.data_ptr(), qk_gamma=cache[3].data_ptr(), qk_beta=cache[4].data_ptr(),
+        h_weight=blk.h_proj.weight.data_ptr(), qk_gamma=qk[0].data_ptr(), qk_beta=qk[1].data_ptr(),
         rot=rot.data_ptr(), keys=keys.data_ptr(), keys_rot=keys_rot.data_ptr(), values=values.data_ptr(),
         work=work.data_ptr(), norm_eps=norm.eps, qk_eps=1e-5, cap=cap, pos=n)
     names = _names(blk)
     owners = [blk] + [blk._modules[m] for m in _SUBMODULES]
     blk._block_plan = _lib.host().BlockPlan(
         bytes(args), owners, list(_SUBMODULES), names, [owners[i]._parameters[name] for i, name in names], [nkey, ekey, akey],
-        [count, count_next, mean, var, h, k, v], keys, values, [keys_rot, work, rot, cache, gamma_eff, beta, p, q, g, omega],
+        [count, count_next, mean, var, h, k, v], keys, values, [keys_rot, work, rot, qk, gamma_eff, beta, p, q, g, omega],
         chunk, x, stream)
     return True

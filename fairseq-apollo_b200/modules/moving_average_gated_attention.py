@@ -277,6 +277,15 @@ class MovingAverageGatedAttention(IncrementalStateMixin, nn.Module):
             mode = block_function.mode_of(self, x, padding_mask, attn_mask, need_weights, before_attn_fn)
             if mode is not None:
                 return block_function.run(self, mode, x, xn, mx, padding_mask), None
+        fresh = not saved_state   # (no state, or the first call on it)
+        if (fused_elementwise and silu_act and fresh and padding_mask is None
+                and block_function.mode_of(self, x, None, attn_mask, need_weights, before_attn_fn) == block_function.CAUSAL):
+            out, k, v = block_function.infer(self, x, xn, mx, saved_state is not None)
+            if saved_state is not None:
+                if self.chunk_size < 0 or seq_len % self.chunk_size != 0:
+                    saved_state["prev_key"], saved_state["prev_value"], saved_state["prev_key_padding_mask"] = k, v, None
+                self._set_input_buffer(incremental_state, saved_state)
+            return out, None
         mx = F.dropout(mx, self.hidden_dropout_p, self.training)
 
         # ---- projections and gates

@@ -306,6 +306,15 @@ MEGA_API int mega_gate_qk_rotary(const void* z, int64_t ld_z, const float* gamma
                         const float* rot, int positions, int period, int q_offset,
                         void* q, int64_t ld_q, void* k, int64_t ld_k,
                         int dtype, int64_t rows, int cols, double eps, mega_stream_t stream);
+/*
+ * The same with what a prompt's decoding cache and an aligned product need: chunk i of `period` rows is written from row
+ * i * out_period of q and k (out_period >= period; the rows between are left alone), and k_raw, contiguous rows or NULL,
+ * receives the keys before the rotation.
+ */
+MEGA_API int mega_gate_qk_rotary_cache(const void* z, int64_t ld_z, const float* gamma, const float* beta,
+                              const float* rot, int positions, int period, int q_offset, int out_period, void* q,
+                              int64_t ld_q, void* k, int64_t ld_k, void* k_raw, int dtype, int64_t rows, int cols,
+                              double eps, mega_stream_t stream);
 
 /*
  * A norm module's parameters (in `dtype`) as the entry points take them, in one launch: gamma = weight + 1, beta (D)
