@@ -426,6 +426,18 @@ static int gate_bwd_common(int op, GateBwd p, int dtype, int64_t rows, int cols,
   return check_launch("gate_bwd");
 }
 
+struct ToFloat {
+  const void* src[8];
+  float* dst[8];
+  long long n[8];
+};
+template <typename T>
+__global__ void __launch_bounds__(256) to_float_kernel(ToFloat a) {
+  const int k = blockIdx.y;
+  const T* s = reinterpret_cast<const T*>(a.src[k]);
+  for (long long i = blockIdx.x * 256 + threadIdx.x; i < a.n[k]; i += (long long)gridDim.x * 256) a.dst[k][i] = Elem<T>::ld(s + i);
+}
+
 }  // namespace
 
 }  // namespace mega
@@ -523,4 +535,26 @@ extern "C" int mega_attention_bias_grad(const void* ds, float* dbias, int span, 
   if (grid.y > 65535) return MEGA_ERR_UNSUPPORTED;
   MEGA_DISPATCH_DTYPE(dtype, launch(bias_grad_kernel<T>, grid, 256, 0, stream, (const T*)ds, dbias, (int)batch, rows, cols, span));
   return check_launch("attention_bias_grad");
+}
+
+extern "C" int mega_to_float(const void* const* src, float* const* dst, const int64_t* n, int count, int dtype,
+                             mega_stream_t stream) {
+  if (!src || !dst || !n) return MEGA_ERR_NULL;
+  if (dtype != MEGA_BF16 && dtype != MEGA_F16) return MEGA_ERR_DTYPE;
+  if (count < 1 || count > 8) return MEGA_ERR_SHAPE;
+  ToFloat a{};
+  long long most = 0;
+  for (int i = 0; i < count; ++i) {
+    if (!src[i] || !dst[i]) return MEGA_ERR_NULL;
+    if (n[i] < 0) return MEGA_ERR_SHAPE;
+    a.src[i] = src[i];
+    a.dst[i] = dst[i];
+    a.n[i] = n[i];
+    if (n[i] > most) most = n[i];
+  }
+  const long long blocks = most / 256 + 1;
+  const dim3 grid((unsigned)(blocks > 256 ? 256 : blocks), count);
+  if (dtype == MEGA_BF16) launch(to_float_kernel<__nv_bfloat16>, grid, 256, 0, stream, a);
+  else launch(to_float_kernel<__half>, grid, 256, 0, stream, a);
+  return check_launch("to_float");
 }

@@ -12,11 +12,11 @@ def needs_grad(*tensors):
 
 
 def ema(x, alpha, delta, third, gamma, omega, padding_mask, bidirectional, shift, truncation=None, complex_poles=False,
-        silu=False):
-    """y = EMA(x) [then SiLU] for x (B, D, L) from the layer's raw parameters; ``third`` is beta (real poles) or
+        silu=False, channels_last=False):
+    """y = EMA(x) [then SiLU] for x (B, D, L), with ``channels_last`` (B, L, D), from the layer's raw parameters; ``third`` is beta (real poles) or
     theta (complex ones)."""
     return _lib.host().ema_train(x, alpha, delta, third, gamma, omega, padding_mask, ops._flags(bidirectional, shift, False),
-                                 ops._trunc(truncation), complex_poles, silu)
+                                 ops._trunc(truncation), complex_poles, silu, channels_last)
 
 
 def timestep_norm(x, prior_count, prior_mean, prior_logv, weight, bias, padding_mask, num_groups, eps):

@@ -80,6 +80,34 @@ Tensor f32c(const Tensor& t) {
   if (!t.defined() || (t.scalar_type() == at::kFloat && t.is_contiguous())) return t;
   return t.detach().to(at::kFloat).contiguous();
 }
+// Parameters in fp32, contiguous, side by side: one launch for all that are not so already
+std::vector<Tensor> f32_all(const std::vector<Tensor>& ts, void* stream) {
+  std::vector<Tensor> out(ts.size());
+  const void* src[8];
+  float* dst[8];
+  int64_t n[8], total = 0;
+  int count = 0;
+  for (const auto& t : ts) total += t.scalar_type() != at::kFloat ? (t.numel() + 3) / 4 * 4 : 0;
+  Tensor all;
+  if (total) all = at::empty({total}, at::TensorOptions().dtype(at::kFloat).device(ts[0].device()));
+  int64_t from = 0;
+  int dt = -1;
+  for (size_t i = 0; i < ts.size(); ++i) {
+    const Tensor& t = ts[i];
+    if (t.scalar_type() == at::kFloat || !t.is_contiguous() || (dt >= 0 && dtype_of(t) != dt) || count == 8) {
+      out[i] = f32c(t);
+      continue;
+    }
+    dt = dtype_of(t);
+    out[i] = all.narrow(0, from, t.numel()).view(t.sizes());
+    src[count] = t.data_ptr();
+    dst[count] = fptr(all) + from;
+    n[count++] = t.numel();
+    from += (t.numel() + 3) / 4 * 4;
+  }
+  if (count) check(mega_to_float(src, dst, n, count, dt, stream), "to_float");
+  return out;
+}
 // complex64 as its interleaved floats
 Tensor c64(const Tensor& t) {
   if (!t.defined()) return t;
@@ -174,14 +202,17 @@ bool rows_of(const Tensor& t, int64_t cols, int64_t& rows) {
 
 class EmaFn : public torch::autograd::Function<EmaFn> {
  public:
-  static Tensor forward(AutogradContext* ctx, Tensor x, Tensor alpha, Tensor delta, Tensor third, Tensor gamma, Tensor omega,
-                        OptTensor mask_, int64_t flags, int64_t trunc, bool cplx, bool silu) {
+  // chan: x and y are (B, L, D) instead of (B, D, L)
+  static Tensor forward(AutogradContext* ctx, Tensor x_, Tensor alpha, Tensor delta, Tensor third, Tensor gamma, Tensor omega,
+                        OptTensor mask_, int64_t flags, int64_t trunc, bool cplx, bool silu, bool chan) {
+    const Tensor x = chan ? x_.transpose(1, 2) : x_;
     on_cuda(x, alpha, omega, given(mask_));
     const Where w(x);
     const Tensor mask = mask_u8(given(mask_), x.size(0), x.size(2));
     const Coeffs c = coeffs(alpha, delta, third, gamma, cplx, w);
     Tensor y = like(x);
-    run_ema(x, y, c.p, c.q, c.g, f32c(omega), mask, none(), none(), (unsigned)flags, (int)trunc, cplx, w);
+    const auto f = f32_all({omega, alpha, delta, third}, w.stream);
+    run_ema(x, y, c.p, c.q, c.g, f[0], mask, none(), none(), (unsigned)flags, (int)trunc, cplx, w);
     Tensor out = y;
     if (silu) {
       int64_t rows;
@@ -193,24 +224,28 @@ class EmaFn : public torch::autograd::Function<EmaFn> {
         out = at::silu(y);
       }
     }
-    ctx->save_for_backward({x, alpha, delta, third, omega, mask, c.p, c.q, c.g, silu ? y : Tensor()});
+    ctx->save_for_backward({x_, f[1], f[2], f[3], f[0], mask, c.p, c.q, c.g, silu ? y : Tensor()});
     ctx->saved_data["flags"] = flags;
     ctx->saved_data["trunc"] = trunc;
     ctx->saved_data["cplx"] = cplx;
-    ctx->saved_data["gamma"] = (int64_t)gamma.scalar_type();
-    return out;
+    ctx->saved_data["chan"] = chan;
+    ctx->saved_data["types"] = std::vector<int64_t>{(int64_t)alpha.scalar_type(), (int64_t)delta.scalar_type(),
+                                                    (int64_t)third.scalar_type(), (int64_t)gamma.scalar_type(),
+                                                    (int64_t)omega.scalar_type()};
+    return chan ? out.transpose(1, 2) : out;
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto s = ctx->get_saved_variables();
-    const Tensor &x = s[0], &alpha = s[1], &delta = s[2], &third = s[3], &omega = s[4], &mask = s[5], &p = s[6], &q = s[7], &g = s[8],
-                 &y = s[9];
+    const bool chan = ctx->saved_data["chan"].toBool();
+    const Tensor x = chan ? s[0].transpose(1, 2) : s[0];
+    const Tensor &alpha = s[1], &delta = s[2], &third = s[3], &omega = s[4], &mask = s[5], &p = s[6], &q = s[7], &g = s[8], &y = s[9];
     const unsigned flags = (unsigned)ctx->saved_data["flags"].toInt();
     const int trunc = (int)ctx->saved_data["trunc"].toInt();
     const bool cplx = ctx->saved_data["cplx"].toBool();
-    const auto gamma_type = (at::ScalarType)ctx->saved_data["gamma"].toInt();
+    const auto types = ctx->saved_data["types"].toIntVector();
     const Where w(x);
-    Tensor dy = grads[0];
+    Tensor dy = chan ? grads[0].transpose(1, 2) : grads[0];
     if (dy.scalar_type() != x.scalar_type()) dy = dy.to(x.scalar_type());
     if (y.defined()) {   // through the SiLU, in y's memory order
       if (dy.strides() != y.strides()) {
@@ -237,40 +272,39 @@ class EmaFn : public torch::autograd::Function<EmaFn> {
     Tensor f = floats({sums + D + raw}, x);
     float* at_ = f.data_ptr<float>();
     float *dp = at_, *dq = at_ + kn, *dg = at_ + kn * (1 + m), *dom = at_ + sums, *da = dom + D, *dd = da + kn;
-    const Tensor om = f32c(omega);
-    const Tensor a = f32c(alpha), d = f32c(delta), t = f32c(third);
     if (cplx) {
       float *dgm = dd + kn, *dt = dgm + 2 * kn;
       check(mega_cema_bwd(dy.data_ptr(), x.data_ptr(), dx.data_ptr(), dtype_of(x), B, D, L, STRIDES3(dy), STRIDES3(x), STRIDES3(dx),
-                          fptr(p), fptr(q), fptr(g), fptr(om), (int)n, ptr<uint8_t>(mask), flags, trunc, dp, dq, dg, dom, w.stream),
+                          fptr(p), fptr(q), fptr(g), fptr(omega), (int)n, ptr<uint8_t>(mask), flags, trunc, dp, dq, dg, dom, w.stream),
             "cema_bwd");
-      check(mega_cema_coeffs_bwd(fptr(a), fptr(d), fptr(t), fptr(q), dp, dq, dg, (int)k, (int)n, da, dd, dt, dgm, w.stream),
+      check(mega_cema_coeffs_bwd(fptr(alpha), fptr(delta), fptr(third), fptr(q), dp, dq, dg, (int)k, (int)n, da, dd, dt, dgm, w.stream),
             "cema_coeffs_bwd");
     } else {
       float *db = dd + kn, *dgm = db + kn;
       check(mega_ema_bwd(dy.data_ptr(), x.data_ptr(), dx.data_ptr(), dtype_of(x), B, D, L, STRIDES3(dy), STRIDES3(x), STRIDES3(dx),
-                         fptr(p), fptr(q), fptr(g), fptr(om), (int)n, ptr<uint8_t>(mask), nullptr, nullptr, flags, trunc, dp, dq, dg,
+                         fptr(p), fptr(q), fptr(g), fptr(omega), (int)n, ptr<uint8_t>(mask), nullptr, nullptr, flags, trunc, dp, dq, dg,
                          dom, nullptr, w.stream), "ema_bwd");
-      check(mega_ema_coeffs_bwd(fptr(a), fptr(d), fptr(t), dp, dq, dg, (int)k, (int)n, da, dd, db, dgm, w.stream), "ema_coeffs_bwd");
+      check(mega_ema_coeffs_bwd(fptr(alpha), fptr(delta), fptr(third), dp, dq, dg, (int)k, (int)n, da, dd, db, dgm, w.stream), "ema_coeffs_bwd");
     }
     Tensor out = f.narrow(0, sums, D + raw);
-    if (alpha.scalar_type() != at::kFloat) out = out.to(alpha.scalar_type());
-    auto part = [&](int64_t from, int64_t count, at::IntArrayRef size, at::ScalarType st) {
-      Tensor v = out.narrow(0, from, count).view(size);
-      return v.scalar_type() == st ? v : v.to(st);
+    if ((at::ScalarType)types[0] != at::kFloat) out = out.to((at::ScalarType)types[0]);
+    const int64_t base = out.storage_offset();
+    auto part = [&](int64_t from, at::IntArrayRef size, at::IntArrayRef stride, int64_t type) {
+      Tensor v = out.as_strided(size, stride, base + from);
+      return v.scalar_type() == (at::ScalarType)type ? v : v.to((at::ScalarType)type);
     };
-    const Tensor g_om = part(0, D, omega.sizes(), omega.scalar_type());
-    const Tensor g_a = part(D, kn, alpha.sizes(), alpha.scalar_type()), g_d = part(D + kn, kn, delta.sizes(), delta.scalar_type());
-    const Tensor g_3 = cplx ? part(D + 4 * kn, k, third.sizes(), third.scalar_type())
-                            : part(D + 2 * kn, kn, third.sizes(), third.scalar_type());
-    const Tensor g_g = cplx ? part(D + 2 * kn, 2 * kn, {k, n, 2}, gamma_type) : part(D + 3 * kn, kn, {k, n}, gamma_type);
-    return {dx, g_a, g_d, g_3, g_g, g_om, Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+    auto like_param = [&](int64_t from, const Tensor& t, int64_t type) { return part(from, t.sizes(), t.strides(), type); };
+    const Tensor g_om = like_param(0, omega, types[4]), g_a = like_param(D, alpha, types[0]), g_d = like_param(D + kn, delta, types[1]);
+    const Tensor g_3 = like_param(D + (cplx ? 4 : 2) * kn, third, types[2]);
+    const Tensor g_g = cplx ? part(D + 2 * kn, {k, n, 2}, {2 * n, 2, 1}, types[3]) : part(D + 3 * kn, {k, n}, {n, 1}, types[3]);
+    return {chan ? dx.transpose(1, 2) : dx, g_a, g_d, g_3, g_g, g_om, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };
 
 Tensor ema_train(const Tensor& x, const Tensor& alpha, const Tensor& delta, const Tensor& third, const Tensor& gamma,
-                 const Tensor& omega, const OptTensor& mask, int64_t flags, int64_t trunc, bool cplx, bool silu) {
-  return EmaFn::apply(x, alpha, delta, third, gamma, omega, mask, flags, trunc, cplx, silu);
+                 const Tensor& omega, const OptTensor& mask, int64_t flags, int64_t trunc, bool cplx, bool silu,
+                 bool chan) {
+  return EmaFn::apply(x, alpha, delta, third, gamma, omega, mask, flags, trunc, cplx, silu, chan);
 }
 
 // ------------------------------------------------------------------------------------------------ norms
@@ -659,7 +693,8 @@ class BlockFn : public torch::autograd::Function<BlockFn> {
     char *u = bp, *z = bp + d * es, *r = z + s * es, *hx = r + e * es;
     Tensor v = fresh(v_lin);
     check(mega_gate_silu(v_lin.data_ptr(), e, nullptr, 0, v.data_ptr(), e, dt, rows, (int)e, w.stream), "gate_silu");
-    const Tensor ga = f32c(gamma), be = f32c(beta);
+    const auto affine = f32_all({gamma, beta}, w.stream);
+    const Tensor &ga = affine[0], &be = affine[1];
     Tensor q = at::empty({nb, period, s}, x.options().requires_grad(false)), k = fresh(q);
     if (rot.defined())
       check(mega_gate_qk_rotary(z, f, fptr(ga), fptr(be), fptr(rot), (int)rot.size(0), (int)period, 0, q.data_ptr(), s, k.data_ptr(), s,

@@ -135,6 +135,14 @@ class MultiHeadComplexEMA(IncrementalStateMixin, nn.Module):
         return ops.cema_forward(x, p.squeeze(-1), q.squeeze(-1), g, zero, None, hx, want_state=True)
 
     # -- forward ---------------------------------------------------------------------------
+    def _forward_train(self, x, padding_mask, incremental_state, activation, channels_last=False):
+        """Differentiable path: forward and backward kernels behind an autograd Function.  ``channels_last``: x and the
+        result are (B, L, D)."""
+        if incremental_state is not None:
+            raise NotImplementedError("the incremental state is an inference feature: use torch.no_grad()")
+        return ema(x, self.alpha, self.delta, self.theta, self.gamma, self.omega, padding_mask, self.bidirectional, self.shift,
+                   self.truncation, True, activation == 'silu', channels_last)
+
     def forward(self, x, padding_mask: Optional[Tensor] = None,
                 incremental_state: Optional[Dict[str, Dict[str, Optional[Tensor]]]] = None,
                 activation: Optional[str] = None) -> Tensor:
@@ -146,11 +154,7 @@ class MultiHeadComplexEMA(IncrementalStateMixin, nn.Module):
         assert not self.bidirectional or incremental_state is None, \
             'Bidirectional EMA does not support incremental state'
         if needs_grad(x, self.alpha, self.delta, self.theta, self.gamma, self.omega):
-            # differentiable path: forward and backward kernels behind an autograd Function
-            if incremental_state is not None:
-                raise NotImplementedError("the incremental state is an inference feature: use torch.no_grad()")
-            return ema(x, self.alpha, self.delta, self.theta, self.gamma, self.omega, padding_mask, self.bidirectional,
-                       self.shift, self.truncation, True, activation == 'silu')
+            return self._forward_train(x, padding_mask, incremental_state, activation)
         p, q, g = self.coeffs()
         p, q = p.squeeze(-1), q.squeeze(-1)
         silu = activation == 'silu'

@@ -159,12 +159,13 @@ class MultiHeadEMA(IncrementalStateMixin, nn.Module):
                                bidirectional=self.bidirectional, shift=self.shift,
                                truncation=self.truncation, silu=silu)
 
-    def _forward_train(self, x, padding_mask, incremental_state, activation):
-        """Differentiable path: forward and backward kernels behind an autograd Function."""
+    def _forward_train(self, x, padding_mask, incremental_state, activation, channels_last=False):
+        """Differentiable path: forward and backward kernels behind an autograd Function.  ``channels_last``: x and the
+        result are (B, L, D)."""
         if incremental_state is not None:
             raise NotImplementedError("the incremental state is an inference feature: use torch.no_grad()")
         return ema(x, self.alpha, self.delta, self.beta, self.gamma, self.omega, padding_mask, self.bidirectional, self.shift,
-                   self.truncation, False, activation == 'silu')
+                   self.truncation, False, activation == 'silu', channels_last)
 
     def forward_time_major(self, x, padding_mask=None, incremental_state=None, activation=None):
         """x: (L, B, D) time-major; returns (L, B, D).  A strided view, no copy."""

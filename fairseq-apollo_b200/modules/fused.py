@@ -39,7 +39,7 @@ def timestep_norm_ema(norm: TimestepNorm, move: MultiHeadEMA, x: Tensor,
     if train or not per_feature or move.bidirectional:
         # training, grouped statistics or a bidirectional layer: the two modules in turn
         xn = norm(x, padding_mask, incremental_state)
-        mx = move(xn.transpose(1, 2), padding_mask, incremental_state, activation).transpose(1, 2)
+        mx = ema_channels_last(move, xn, padding_mask, incremental_state, activation)
         return (mx, xn) if return_normed else mx
     if (incremental_state is not None and x.size(1) == 1 and padding_mask is None and x.is_contiguous()
             and (not move.complex or move.ndim in (2, 4, 8, 16, 32))):
@@ -63,6 +63,14 @@ def timestep_norm_ema(norm: TimestepNorm, move: MultiHeadEMA, x: Tensor,
         estate['prev_state'] = res["h"]
         move._set_input_buffer(incremental_state, estate)
     return (res["y"], res["xn"]) if return_normed else res["y"]
+
+
+def ema_channels_last(move, x, padding_mask, incremental_state, activation):
+    """move(x) for x (B, L, D).  In training without transposes around it, which cost the backward a node each (a module
+    with hooks is called as one)."""
+    if needs_grad(x, *move.parameters()) and not (move._forward_hooks or move._forward_pre_hooks or move._backward_hooks):
+        return move._forward_train(x, padding_mask, incremental_state, activation, channels_last=True)
+    return move(x.transpose(1, 2), padding_mask, incremental_state, activation).transpose(1, 2)
 
 
 def sequence_norm_ema(norm: SequenceNorm, move: MultiHeadEMA, x: Tensor, padding_mask: Optional[Tensor] = None,

@@ -37,7 +37,7 @@ from .attention_softmax import AttentionSoftmax
 from .complex_exponential_moving_average import MultiHeadComplexEMA
 from .efficient_attention import EfficientAttention
 from .exponential_moving_average import MultiHeadEMA
-from .fused import sequence_norm_ema, timestep_norm_ema
+from .fused import ema_channels_last, timestep_norm_ema
 from .sequence_norm import SequenceNorm
 from .timestep_norm import TimestepNorm
 
@@ -261,13 +261,18 @@ class MovingAverageGatedAttention(IncrementalStateMixin, nn.Module):
         fused_elementwise = not train and x.is_cuda
 
         # ---- norm -> EMA (-> SiLU): mx (B, L, D) and the normalised activations xn (B, L, D)
-        if self.bidirectional:
+        if train:
+            # (as (B, L, D) throughout: a transpose costs the backward a node of its own)
+            act = 'silu' if silu_act else None
+            if self.bidirectional:
+                xn = self.norm(x, padding_mask, length_last=False)
+            else:
+                xn = self.norm(x, padding_mask=padding_mask, incremental_state=incremental_state)
+            mx = ema_channels_last(self.move, xn, padding_mask, incremental_state, act)
+        elif self.bidirectional:
             xn_t = self.norm(x.transpose(1, 2), padding_mask)
             xn = xn_t.transpose(1, 2)
             mx = self.move(xn_t, padding_mask, None, 'silu' if silu_act else None).transpose(1, 2)
-        elif train:
-            xn = self.norm(x, padding_mask=padding_mask, incremental_state=incremental_state)
-            mx = self.move(xn.transpose(1, 2), padding_mask, incremental_state, 'silu' if silu_act else None).transpose(1, 2)
         else:
             mx, xn = timestep_norm_ema(self.norm, self.move, x, padding_mask, incremental_state,
                                        activation='silu' if silu_act else None, return_normed=True)

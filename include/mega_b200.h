@@ -528,6 +528,12 @@ MEGA_API int mega_attention_dropkey_softmax_fwd(const void* x, void* y, int dtyp
                                        mega_stream_t stream);
 
 /*
+ * Up to eight arrays of n[i] values of `dtype` (bf16 or fp16) as fp32, in one launch (parameters of a layer).
+ */
+MEGA_API int mega_to_float(const void* const* src, float* const* dst, const int64_t* n, int count, int dtype,
+                  mega_stream_t stream);
+
+/*
  * Gradients of the gates (dy / dout: gradient of the result; operands as in the forward).  16-byte aligned operands,
  * row pitches and column counts in whole 16-byte pieces (MEGA_ERR_ALIGN / MEGA_ERR_STRIDE).  colsum*: column sums of
  * the gradient they are named after, ADDED to fp32 arrays of `cols` values (bias gradients of the projection that
