@@ -11,8 +11,9 @@
 //   V_t = V + sum_{s >= t} b_s,  h_t = U + sum_{s > t} (a_s - e_s V_s) + a_t,  dx_t = dy r w + h_t + 2 (x - u) V_t,
 // and a suffix is a total minus a prefix: one launch takes every segment's totals, the next walks forward in
 // time from them.  A segment acts on (V, U) by an affine map, composed over the later segments.
-// Bound: the issue slots, about 20 instructions per element and pass forward and 30 backward; HBM moves x twice
-// and y once forward, x three times, dy twice and dx once backward.  B = 16, L = 4096, D = 1024, bf16: the
+// Bound: the issue slots and memory alike; a lane takes two channels in packed arithmetic (one channel per lane: 74 us
+// forward behind the moments, 109 and 129 us backward, at B = 16, L = 4096, D = 1024 bf16; in pairs 64, 104 and 106).
+// HBM moves x twice and y once forward, x three times, dy twice and dx once backward.  B = 16, L = 4096, D = 1024, bf16: the
 // walk of whole sequences (16384 chains of 4096 steps, statistics of every step saved in fp32) took 370 us
 // forward and 365 us backward.  SequenceNorm needs the moments of the whole sequence only (B = 16, L = 1024, D = 256
 // bf16: 403 us as one thread per column, its backward 99 us as one strided block per column).
@@ -61,50 +62,117 @@ __device__ __forceinline__ NormLane norm_lane(const SegNorm& s) {
   return l;
 }
 
-// What a segment starts from: the prior and the segments before it.
-__device__ __forceinline__ Run run_before(const SegNorm& s, const NormLane& l) {
+// ---- two channels per lane ----------------------------------------------------------------------
+struct PairLane {
+  int lane, warp, d, dc, d0, left, b, seg, t0, t1;   // d: first of the lane's two channels
+  bool ok, active;
+};
+__device__ __forceinline__ PairLane pair_lane(const SegNorm& s) {
+  PairLane l;
+  l.lane = threadIdx.x & 31;
+  l.warp = threadIdx.x >> 5;
+  l.d0 = blockIdx.x * 64;
+  l.left = s.a.D - l.d0;
+  l.d = l.d0 + 2 * l.lane;
+  l.ok = l.d < s.a.D;   // (rows are whole 16-byte pieces: channels come in pairs)
+  l.dc = l.ok ? l.d : s.a.D - 2;
+  l.seg = blockIdx.y * kWarps + l.warp;
+  l.b = blockIdx.z;
+  l.active = l.seg < s.S;
+  l.t0 = min(s.a.L, l.seg * s.T);
+  l.t1 = min(s.a.L, l.t0 + s.T);
+  return l;
+}
+__device__ __forceinline__ f32x2 ldg2(const float* p) { return pack2(__ldg(p), __ldg(p + 1)); }
+__device__ __forceinline__ f32x2 both(float v) { return pack2(v, v); }
+__device__ __forceinline__ f32x2 neg2(f32x2 v) { return mul2(v, both(-1.f)); }
+
+// What a segment starts from: the prior and the segments before it (for two channels).
+__device__ __forceinline__ void pair_before(const SegNorm& s, const PairLane& l, Run (&r)[2]) {
   const float n0 = (float)s.a.prev_count[l.b];
   const size_t i = (size_t)l.b * s.a.D + l.dc;
-  Run r{n0, s.a.prev_mean[i], s.a.prev_var[i] * n0};
   const float* pn = s.rn + (size_t)l.b * s.S;
-  const float *pm = s.rm + (size_t)l.b * s.S * s.a.D + l.dc, *ps = s.rs + (size_t)l.b * s.S * s.a.D + l.dc;
+  const size_t at = (size_t)l.b * s.S * s.a.D + l.dc;
+#pragma unroll
+  for (int c = 0; c < 2; ++c) r[c] = Run{n0, s.a.prev_mean[i + c], s.a.prev_var[i + c] * n0};
 #pragma unroll 4
-  for (int k = 0; k < l.seg; ++k)
-    r = combine(r, Run{__ldg(pn + k), __ldg(pm + (size_t)k * s.a.D), __ldg(ps + (size_t)k * s.a.D)});
-  return r;
+  for (int k = 0; k < l.seg; ++k) {
+    const float n = __ldg(pn + k);
+    const float2 m = __ldg(reinterpret_cast<const float2*>(s.rm + at + (size_t)k * s.a.D));
+    const float2 q = __ldg(reinterpret_cast<const float2*>(s.rs + at + (size_t)k * s.a.D));
+    r[0] = combine(r[0], Run{n, m.x, q.x});
+    r[1] = combine(r[1], Run{n, m.y, q.y});
+  }
 }
+
+// Running (norm_run.cuh) for two channels.
+struct PairRunning {
+  f32x2 c, s1, s2, in_s, u;
+  float n;
+  __device__ __forceinline__ void start(const Run (&r)[2]) {
+    c = pack2(r[0].m, r[1].m);
+    s1 = s2 = u = both(0.f);
+    n = r[0].n;
+    in_s = pack2(r[0].s, r[1].s);
+  }
+  // returns x - c; inv = 1 / n, r = 1 / sqrt(var + eps)
+  __device__ __forceinline__ f32x2 step(f32x2 x, float eps, f32x2& inv, f32x2& r) {
+    if (n == 0.f) c = x;
+    const f32x2 d = sub2(x, c);
+    s1 = add2(s1, d);
+    s2 = fma2(d, d, s2);
+    n += 1.f;
+    inv = both(rcp_approx(n));
+    u = mul2(s1, inv);
+    const f32x2 v = fma2(neg2(u), u, mul2(add2(in_s, s2), inv));
+    float a, b;
+    unpack2(v, a, b);
+    r = pack2(rsqrt_approx(fmaxf(a, 0.f) + eps), rsqrt_approx(fmaxf(b, 0.f) + eps));
+    return d;
+  }
+};
 
 template <typename T, bool kMask>
 __global__ void __launch_bounds__(kWarps * 32) norm_emit_kernel(SegNorm s) {
   extern __shared__ __align__(16) unsigned char rings[];
   const ScanNormArgs& a = s.a;
-  const NormLane l = norm_lane(s);
+  const PairLane l = pair_lane(s);
   if (!l.active) return;
   const T* x = reinterpret_cast<const T*>(a.x) + l.b * a.xsb + l.d0;
   T* py = reinterpret_cast<T*>(a.y) + l.b * a.ysb + (long long)l.t0 * a.ysl + l.dc;
   const unsigned char* m = kMask ? a.mask + (size_t)l.b * a.L : nullptr;
-  const float w = __ldg(a.gamma + l.dc), bb = __ldg(a.beta + l.dc), eps = a.eps;
-  const Run in = run_before(s, l);
-  Running st;
+  const f32x2 w = ldg2(a.gamma + l.dc), bb = ldg2(a.beta + l.dc);
+  const float eps = a.eps;
+  Run in[2];
+  pair_before(s, l, in);
+  PairRunning st;
   st.start(in);
-  walk<T, 1, false, kMask>(x, a.xsl, x, 0, m, l.t0, l.t1, l.left, rings + (size_t)l.warp * kRing * kTileBytes,
-                           [&](int, float xv, float, bool pad) {
-                             float out = 0.f;
-                             if (!(kMask && pad)) {
-                               float inv, r;
-                               const float d = st.step(xv, eps, inv, r);
-                               out = fmaf((d - st.u) * r, w, bb);
-                             }
-                             if (l.ok) Elem<T>::st(py, out);
-                             py += a.ysl;
-                           });
+  walk_pairs<T, false, kMask>(x, a.xsl, x, 0, m, l.t0, l.t1, l.left, rings + (size_t)l.warp * kRing * kTileBytes,
+                              [&](f32x2 xv, f32x2, bool pad) {
+                                f32x2 out = both(0.f);
+                                if (!(kMask && pad)) {
+                                  f32x2 inv, r;
+                                  const f32x2 d = st.step(xv, eps, inv, r);
+                                  out = fma2(mul2(sub2(d, st.u), r), w, bb);
+                                }
+                                if (l.ok) pair_st(py, out);
+                                py += a.ysl;
+                              });
   if (l.seg == s.S - 1 && l.ok) {
-    const size_t i = (size_t)l.b * a.D + l.d;
     const bool any = st.n > 0.f;
     const float inv = any ? 1.f / st.n : 0.f;
-    a.mean_out[i] = any ? fmaf(st.s1, inv, st.c) : a.prev_mean[i];
-    const float u = st.s1 * inv;
-    a.var_out[i] = any ? fmaxf(fmaf(-u, u, (st.in_s + st.s2) * inv), 0.f) : a.prev_var[i];
+    float c[2], s1[2], s2[2], q[2];
+    unpack2(st.c, c[0], c[1]);
+    unpack2(st.s1, s1[0], s1[1]);
+    unpack2(st.s2, s2[0], s2[1]);
+    unpack2(st.in_s, q[0], q[1]);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const size_t i = (size_t)l.b * a.D + l.d + k;
+      const float u = s1[k] * inv;
+      a.mean_out[i] = any ? c[k] + u : a.prev_mean[i];
+      a.var_out[i] = any ? fmaxf(fmaf(-u, u, (q[k] + s2[k]) * inv), 0.f) : a.prev_var[i];
+    }
     if (l.d == 0) a.count_out[l.b] = a.prev_count[l.b] + (long long)(st.n - (float)a.prev_count[l.b] + 0.5f);
   }
 }
@@ -114,48 +182,51 @@ template <typename T, bool kMask>
 __global__ void __launch_bounds__(kWarps * 32) norm_bwd_map_kernel(SegNorm s) {
   extern __shared__ __align__(16) unsigned char rings[];
   const ScanNormArgs& a = s.a;
-  const NormLane l = norm_lane(s);
-  float dg = 0.f, db = 0.f;
+  const PairLane l = pair_lane(s);
+  f32x2 dg = both(0.f), db = both(0.f);
   if (l.active) {
     const T* x = reinterpret_cast<const T*>(a.x) + l.b * a.xsb + l.d0;
     const T* g = reinterpret_cast<const T*>(a.dy) + l.b * a.gsb + l.d0;
     const unsigned char* m = kMask ? a.mask + (size_t)l.b * a.L : nullptr;
-    const float w = __ldg(a.gamma + l.dc), eps = a.eps;
-    Running st;
-    st.start(run_before(s, l));
-    float sv = 0.f, su = 0.f, se = 0.f;
-    walk<T, 1, true, kMask>(x, a.xsl, g, a.gsl, m, l.t0, l.t1, l.left, rings + (size_t)l.warp * 2 * kRing * kTileBytes,
-                            [&](int, float xv, float gv, bool pad) {
-                              if (kMask && pad) return;
-                              const float up = st.u;
-                              float inv, r;
-                              const float d = st.step(xv, eps, inv, r);
-                              const float xu = d - st.u, gr = gv * r, gx = gr * xu;
-                              se = fmaf(2.f * (d - up), inv, se);
-                              const float wi = w * inv;
-                              const float b = -0.5f * (gx * (r * r)) * wi;
-                              sv += b;
-                              su -= fmaf(b, se, gr * wi);
-                              dg += gx;
-                              db += gv;
-                            });
+    const f32x2 w = ldg2(a.gamma + l.dc), wh = mul2(w, both(-0.5f));
+    const float eps = a.eps;
+    Run in[2];
+    pair_before(s, l, in);
+    PairRunning st;
+    st.start(in);
+    f32x2 sv = both(0.f), su = sv, se = sv;   // (su with its sign turned)
+    walk_pairs<T, true, kMask>(x, a.xsl, g, a.gsl, m, l.t0, l.t1, l.left, rings + (size_t)l.warp * 2 * kRing * kTileBytes,
+                               [&](f32x2 xv, f32x2 gv, bool pad) {
+                                 if (kMask && pad) return;
+                                 const f32x2 up = st.u;
+                                 f32x2 inv, r;
+                                 const f32x2 d = st.step(xv, eps, inv, r);
+                                 const f32x2 gr = mul2(gv, r), gx = mul2(gr, sub2(d, st.u));
+                                 se = fma2(mul2(sub2(d, up), both(2.f)), inv, se);
+                                 const f32x2 b = mul2(mul2(gx, mul2(r, r)), mul2(wh, inv));
+                                 sv = add2(sv, b);
+                                 su = add2(su, fma2(b, se, mul2(gr, mul2(w, inv))));
+                                 dg = add2(dg, gx);
+                                 db = add2(db, gv);
+                               });
     if (l.ok) {
       const size_t i = ((size_t)l.b * s.S + l.seg) * a.D + l.d;
-      s.sv[i] = sv;
-      s.su[i] = su;
-      s.sw[i] = -se;
+      *reinterpret_cast<f32x2*>(s.sv + i) = sv;
+      *reinterpret_cast<f32x2*>(s.su + i) = neg2(su);
+      *reinterpret_cast<f32x2*>(s.sw + i) = neg2(se);
     }
   }
   __syncthreads();
-  float* red = reinterpret_cast<float*>(rings);   // [2][kWarps][32]
-  red[l.warp * 32 + l.lane] = dg;
-  red[(kWarps + l.warp) * 32 + l.lane] = db;
+  float* red = reinterpret_cast<float*>(rings);   // [2][kWarps][64]
+  *reinterpret_cast<f32x2*>(red + l.warp * 64 + 2 * l.lane) = dg;
+  *reinterpret_cast<f32x2*>(red + (kWarps + l.warp) * 64 + 2 * l.lane) = db;
   __syncthreads();
-  if (l.warp < 2 && l.ok) {
+  const int c = threadIdx.x & 63, which = threadIdx.x >> 6;   // (128 threads: the 64 channels of either sum)
+  if (l.d0 + c < a.D) {
     float v = 0.f;
 #pragma unroll
-    for (int k = 0; k < kWarps; ++k) v += red[(l.warp * kWarps + k) * 32 + l.lane];
-    atomicAdd((l.warp == 0 ? a.dgamma : a.dbeta) + l.d, v);
+    for (int k = 0; k < kWarps; ++k) v += red[(which * kWarps + k) * 64 + c];
+    atomicAdd((which == 0 ? a.dgamma : a.dbeta) + l.d0 + c, v);
   }
 }
 
@@ -163,54 +234,61 @@ template <typename T, bool kMask>
 __global__ void __launch_bounds__(kWarps * 32) norm_bwd_emit_kernel(SegNorm s) {
   extern __shared__ __align__(16) unsigned char rings[];
   const ScanNormArgs& a = s.a;
-  const NormLane l = norm_lane(s);
+  const PairLane l = pair_lane(s);
   if (!l.active) return;
   const T* x = reinterpret_cast<const T*>(a.x) + l.b * a.xsb + l.d0;
   const T* g = reinterpret_cast<const T*>(a.dy) + l.b * a.gsb + l.d0;
   T* pd = reinterpret_cast<T*>(a.y) + l.b * a.ysb + (long long)l.t0 * a.ysl + l.dc;
   const unsigned char* m = kMask ? a.mask + (size_t)l.b * a.L : nullptr;
-  const float w = __ldg(a.gamma + l.dc), eps = a.eps;
+  const f32x2 w = ldg2(a.gamma + l.dc), wh = mul2(w, both(0.5f));
+  const float eps = a.eps;
   const size_t row = (size_t)l.b * a.D + l.dc;
   const float n0 = (float)a.prev_count[l.b];
   float n_end = n0;
   for (int k = 0; k < s.S; ++k) n_end += __ldg(s.rn + (size_t)l.b * s.S + k);
-  const float inv_end = n_end > 0.f ? 1.f / n_end : 0.f;
-  float V = a.dvar ? a.dvar[row] * inv_end : 0.f, U = a.dmean ? a.dmean[row] * inv_end : 0.f;
+  const f32x2 inv_end = both(n_end > 0.f ? 1.f / n_end : 0.f);
+  f32x2 V = a.dvar ? mul2(pack2(a.dvar[row], a.dvar[row + 1]), inv_end) : both(0.f);
+  f32x2 U = a.dmean ? mul2(pack2(a.dmean[row], a.dmean[row + 1]), inv_end) : both(0.f);
   const size_t at = (size_t)l.b * s.S * a.D + l.dc;
+  auto map = [&](const float* p, int k) { return __ldg(reinterpret_cast<const unsigned long long*>(p + at + (size_t)k * a.D)); };
 #pragma unroll 4
   for (int k = s.S - 1; k > l.seg; --k) {
-    const size_t i = at + (size_t)k * a.D;
-    U = fmaf(__ldg(s.sw + i), V, U + __ldg(s.su + i));
-    V += __ldg(s.sv + i);
+    U = fma2(map(s.sw, k), V, add2(U, map(s.su, k)));
+    V = add2(V, map(s.sv, k));
   }
-  const size_t own = at + (size_t)l.seg * a.D;
-  float W = fmaf(__ldg(s.sw + own), V, U + __ldg(s.su + own));   // U as it leaves the segment's first step
-  V += __ldg(s.sv + own);
+  f32x2 W = fma2(map(s.sw, l.seg), V, add2(U, map(s.su, l.seg)));   // U as it leaves the segment's first step
+  V = add2(V, map(s.sv, l.seg));
   if (l.seg == 0 && l.ok) {
     const bool any = n_end > n0;   // (no unmasked step: the incoming gradients pass through)
-    a.dprev_mean[row] = any ? n0 * W : (a.dmean ? a.dmean[row] : 0.f);
-    a.dprev_var[row] = any ? n0 * V : (a.dvar ? a.dvar[row] : 0.f);
+    float wv[2], vv[2];
+    unpack2(W, wv[0], wv[1]);
+    unpack2(V, vv[0], vv[1]);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      a.dprev_mean[row + k] = any ? n0 * wv[k] : (a.dmean ? a.dmean[row + k] : 0.f);
+      a.dprev_var[row + k] = any ? n0 * vv[k] : (a.dvar ? a.dvar[row + k] : 0.f);
+    }
   }
-  Running st;
-  st.start(run_before(s, l));
-  walk<T, 1, true, kMask>(x, a.xsl, g, a.gsl, m, l.t0, l.t1, l.left, rings + (size_t)l.warp * 2 * kRing * kTileBytes,
-                          [&](int, float xv, float gv, bool pad) {
-                            float out = 0.f;
-                            if (!(kMask && pad)) {
-                              const float up = st.u;
-                              float inv, r;
-                              const float d = st.step(xv, eps, inv, r);
-                              const float xu = d - st.u, gr = gv * r, gx = gr * xu, wi = w * inv;
-                              const float b = -0.5f * (gx * (r * r)) * wi;
-                              const float ev = 2.f * (d - up) * inv * V;
-                              const float h = W + ev;
-                              out = fmaf(gr, w, fmaf(2.f * xu, V, h));
-                              W = fmaf(gr, wi, h);   // W - (a - e V) with a = -gr wi
-                              V -= b;
-                            }
-                            if (l.ok) Elem<T>::st(pd, out);
-                            pd += a.ysl;
-                          });
+  Run in[2];
+  pair_before(s, l, in);
+  PairRunning st;
+  st.start(in);
+  walk_pairs<T, true, kMask>(x, a.xsl, g, a.gsl, m, l.t0, l.t1, l.left, rings + (size_t)l.warp * 2 * kRing * kTileBytes,
+                             [&](f32x2 xv, f32x2 gv, bool pad) {
+                               f32x2 out = both(0.f);
+                               if (!(kMask && pad)) {
+                                 const f32x2 up = st.u;
+                                 f32x2 inv, r;
+                                 const f32x2 d = st.step(xv, eps, inv, r);
+                                 const f32x2 xu = sub2(d, st.u), gr = mul2(gv, r), gx = mul2(gr, xu), V2 = add2(V, V);
+                                 const f32x2 h = fma2(mul2(sub2(d, up), inv), V2, W);   // W + e V
+                                 out = fma2(gr, w, fma2(xu, V2, h));
+                                 W = fma2(gr, mul2(w, inv), h);                         // W - (a - e V) with a = -gr w / n
+                                 V = fma2(mul2(gx, mul2(r, r)), mul2(wh, inv), V);      // V - b
+                               }
+                               if (l.ok) pair_st(pd, out);
+                               pd += a.ysl;
+                             });
 }
 
 // ---- SequenceNorm, per channel -----------------------------------------------------------------
@@ -304,8 +382,8 @@ __global__ void __launch_bounds__(kWarps * 32) sqn_bwd_emit_kernel(SegNorm s) {
 
 // Segments: enough blocks of four for the SMs (about six of them resident each) in few rounds, at least 64 steps
 // each and at most 64 of them, since every segment combines those before it.
-static void pick_segments(const ScanNormArgs& a, int resident, SegNorm& s) {
-  const long long strips = (long long)((a.D + 31) / 32) * a.B;
+static void pick_segments(const ScanNormArgs& a, int resident, int width, SegNorm& s) {
+  const long long strips = (long long)((a.D + width - 1) / width) * a.B;
   const double slots = 148.0 * resident;
   double best = 1e30;
   for (int S = 1; S <= 64; ++S) {
@@ -325,17 +403,19 @@ static void pick_segments(const ScanNormArgs& a, int resident, SegNorm& s) {
 template <typename T, bool kMask>
 static void fwd_launch(const SegNorm& s, cudaStream_t st) {
   const dim3 grid((s.a.D + 31) / 32, (s.S + kWarps - 1) / kWarps, s.a.B), block(kWarps * 32);
+  const dim3 pairs((s.a.D + 63) / 64, grid.y, grid.z);
   const size_t rings = (size_t)kWarps * kRing * kTileBytes;
   launch(norm_moments_kernel<T, kMask>, grid, block, rings, (void*)st, moments_of(s));
-  launch(norm_emit_kernel<T, kMask>, grid, block, rings, (void*)st, s);
+  launch(norm_emit_kernel<T, kMask>, pairs, block, rings, (void*)st, s);
 }
 template <typename T, bool kMask>
 static void bwd_launch(const SegNorm& s, cudaStream_t st) {
   const dim3 grid((s.a.D + 31) / 32, (s.S + kWarps - 1) / kWarps, s.a.B), block(kWarps * 32);
+  const dim3 pairs((s.a.D + 63) / 64, grid.y, grid.z);
   const size_t rings = (size_t)kWarps * kRing * kTileBytes;
   launch(norm_moments_kernel<T, kMask>, grid, block, rings, (void*)st, moments_of(s));
-  launch(norm_bwd_map_kernel<T, kMask>, grid, block, 2 * rings, (void*)st, s);
-  launch(norm_bwd_emit_kernel<T, kMask>, grid, block, 2 * rings, (void*)st, s);
+  launch(norm_bwd_map_kernel<T, kMask>, pairs, block, 2 * rings, (void*)st, s);
+  launch(norm_bwd_emit_kernel<T, kMask>, pairs, block, 2 * rings, (void*)st, s);
 }
 
 template <typename T, bool kMask>
@@ -355,7 +435,7 @@ static bool sqn_dispatch(int dtype, const ScanNormArgs& a, bool bwd, cudaStream_
   if (g_options[OPT_DISABLE_STREAM].load() != 0 || a.B > 65535) return false;
   SegNorm s{};
   s.a = a;
-  pick_segments(a, bwd ? 3 : 6, s);
+  pick_segments(a, bwd ? 3 : 6, 32, s);
   const size_t n = (size_t)a.B * s.S * a.D;
   Scratch sc(Scratch::padded(n * 4) * 2 + Scratch::padded((size_t)a.B * s.S * 4), st);
   if (!sc) return false;
@@ -380,7 +460,7 @@ static bool dispatch(int dtype, const ScanNormArgs& a, cudaStream_t st) {
   if (g_options[OPT_DISABLE_STREAM].load() != 0 || a.B > 65535) return false;
   SegNorm s{};
   s.a = a;
-  pick_segments(a, kBwd ? 3 : 6, s);
+  pick_segments(a, kBwd ? 3 : 6, 64, s);
   const size_t n = (size_t)a.B * s.S * a.D;
   Scratch sc(Scratch::padded(n * 4) * (kBwd ? 5 : 2) + Scratch::padded((size_t)a.B * s.S * 4), st);
   if (!sc) return false;
@@ -412,14 +492,19 @@ static bool dispatch(int dtype, const ScanNormArgs& a, cudaStream_t st) {
 
 }  // namespace
 
+// outputs are stored two channels at a time
+static bool pairs_ok(int dtype, const ScanNormArgs& a, long long ysd) {
+  return ysd == 1 && aligned_to(a.y, 2 * elem_size(dtype)) && a.ysb % 2 == 0 && a.ysl % 2 == 0;
+}
+
 bool scan_norm_fwd_try(int dtype, const ScanNormArgs& a, long long xsd, long long ysd, cudaStream_t s) {
-  if (!rows_ok(dtype, a.x, a.xsb, a.xsl, xsd, a.D) || ysd != 1 || a.x == a.y) return false;
+  if (!rows_ok(dtype, a.x, a.xsb, a.xsl, xsd, a.D) || !pairs_ok(dtype, a, ysd) || a.x == a.y) return false;
   return dispatch<false>(dtype, a, s);
 }
 
 bool scan_norm_bwd_try(int dtype, const ScanNormArgs& a, long long xsd, long long ysd, long long gsd, cudaStream_t s) {
-  if (!rows_ok(dtype, a.x, a.xsb, a.xsl, xsd, a.D) || !rows_ok(dtype, a.dy, a.gsb, a.gsl, gsd, a.D) || ysd != 1 ||
-      a.y == a.x || a.y == a.dy)
+  if (!rows_ok(dtype, a.x, a.xsb, a.xsl, xsd, a.D) || !rows_ok(dtype, a.dy, a.gsb, a.gsl, gsd, a.D) ||
+      !pairs_ok(dtype, a, ysd) || a.y == a.x || a.y == a.dy)
     return false;
   return dispatch<true>(dtype, a, s);
 }

@@ -19,9 +19,9 @@ constexpr int kU = 8;       // steps of an unrolled group
 constexpr int kTileBytes = 2048;
 constexpr int kRing = 4;
 
-template <typename T>
+template <typename T, int kCh = 32>
 __device__ __forceinline__ void fetch_tile(uint32_t dst, const T* row, long long stride, int rows, int d_left, int lane) {
-  constexpr int kPer = 32 * (int)sizeof(T) / 16;   // 16-byte pieces of a row
+  constexpr int kPer = kCh * (int)sizeof(T) / 16;   // 16-byte pieces of a row
 #pragma unroll
   for (int i = 0; i < kTileBytes / 16 / 32; ++i) {
     const int id = lane + 32 * i;
@@ -90,6 +90,75 @@ __device__ __forceinline__ void walk(const T* x, long long xsl, const T* g, long
     for (; r0 < rows; ++r0)
       f(j * kR + r0, Elem<T>::ld_shared(tx + r0 * 32), kTwo ? Elem<T>::ld_shared(tg + r0 * 32) : 0.f,
         kMask && ((bits >> r0) & 1u) != 0);
+  }
+  tile_wait<0>();
+}
+
+// ---- two adjacent channels per lane, in packed fp32 arithmetic: half the instructions per element ------------
+template <typename T>
+__device__ __forceinline__ f32x2 pair_ld(const T* p) {   // (shared memory)
+  if constexpr (sizeof(T) == 4) {
+    return *reinterpret_cast<const f32x2*>(p);
+  } else {
+    const uint32_t v = *reinterpret_cast<const uint32_t*>(p);
+    return pack2(Elem<T>::ld_shared(reinterpret_cast<const T*>(&v)), Elem<T>::ld_shared(reinterpret_cast<const T*>(&v) + 1));
+  }
+}
+template <typename T>
+__device__ __forceinline__ void pair_st(T* p, f32x2 v) {
+  if constexpr (sizeof(T) == 4) {
+    *reinterpret_cast<f32x2*>(p) = v;
+  } else {
+    float lo, hi;
+    unpack2(v, lo, hi);
+    uint32_t w;
+    Elem<T>::st(reinterpret_cast<T*>(&w), lo);
+    Elem<T>::st(reinterpret_cast<T*>(&w) + 1, hi);
+    *reinterpret_cast<uint32_t*>(p) = w;
+  }
+}
+
+// walk() in time order for 64 channels: f(v, g, pad) sees the pairs of every step.
+template <typename T, bool kTwo, bool kMask, typename F>
+__device__ __forceinline__ void walk_pairs(const T* x, long long xsl, const T* g, long long gsl, const unsigned char* m, int t0, int t1,
+                                           int d_left, unsigned char* ring, F&& f) {
+  constexpr int kR = kTileBytes / (64 * (int)sizeof(T));
+  const int lane = threadIdx.x & 31, n = t1 - t0, tiles = (n + kR - 1) / kR;
+  const T* px = x + (long long)t0 * xsl;
+  const T* pg = kTwo ? g + (long long)t0 * gsl : nullptr;
+  const uint32_t rs = smem_u32(ring);
+  auto issue = [&](int j) {
+    if (j < tiles) {
+      const int slot = j % kRing;
+      fetch_tile<T, 64>(rs + slot * kTileBytes, px + (long long)(j * kR) * xsl, xsl, n - j * kR, d_left, lane);
+      if (kTwo) fetch_tile<T, 64>(rs + (kRing + slot) * kTileBytes, pg + (long long)(j * kR) * gsl, gsl, n - j * kR, d_left, lane);
+    }
+    tile_commit();
+  };
+  auto flags = [&](int j) -> unsigned {   // bit r: step r of tile j is padded
+    if (!kMask) return 0u;
+    const int k = j * kR + lane;
+    return __ballot_sync(0xffffffffu, lane < kR && k < n && __ldg(m + t0 + k) != 0);
+  };
+#pragma unroll
+  for (int j = 0; j < kRing - 1; ++j) issue(j);
+  unsigned next = flags(0);
+  for (int j = 0; j < tiles; ++j) {
+    tile_wait<kRing - 2>();
+    __syncwarp();
+    issue(j + kRing - 1);
+    const unsigned bits = next;
+    if (j + 1 < tiles) next = flags(j + 1);
+    const T* tx = reinterpret_cast<const T*>(ring + (j % kRing) * kTileBytes) + 2 * lane;
+    const T* tg = reinterpret_cast<const T*>(ring + (kRing + j % kRing) * kTileBytes) + 2 * lane;
+    const int rows = min(kR, n - j * kR);
+    int r0 = 0;
+    for (; r0 + kU <= rows; r0 += kU) {
+#pragma unroll
+      for (int u = 0; u < kU; ++u)
+        f(pair_ld(tx + (r0 + u) * 64), kTwo ? pair_ld(tg + (r0 + u) * 64) : 0ull, kMask && ((bits >> (r0 + u)) & 1u) != 0);
+    }
+    for (; r0 < rows; ++r0) f(pair_ld(tx + r0 * 64), kTwo ? pair_ld(tg + r0 * 64) : 0ull, kMask && ((bits >> r0) & 1u) != 0);
   }
   tile_wait<0>();
 }
