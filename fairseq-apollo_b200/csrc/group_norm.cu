@@ -112,18 +112,35 @@ __global__ void __launch_bounds__(kScanG* kScanT) group_scan_kernel(const float*
   const int t0 = min(L, ti * per), t1 = min(L, t0 + per);
   const unsigned char* mp = mask ? mask + (size_t)b * L : nullptr;
   const size_t base = (size_t)b * L * G + g;
+  // (the loads of several steps go out together: one at a time, each waited for the one before, 31 us at L = 4096 and
+  // 32 groups)
+  constexpr int kFwdB = 8;
+  float ms[kFwdB], vs[kFwdB];
+  bool skip[kFwdB];
+  auto fetch = [&](int k) {
+#pragma unroll
+    for (int j = 0; j < kFwdB; ++j) {
+      const int t = min(k + j, t1 - 1);
+      ms[j] = __ldg(gm + base + (size_t)t * G);
+      vs[j] = __ldg(gv + base + (size_t)t * G);
+      skip[j] = k + j >= t1 || (mp && mp[t]);
+    }
+  };
   // own run: sums about its first value
   Run r{0.f, 0.f, 0.f};
   if (ok) {
     float c = 0.f, s1 = 0.f, s2 = 0.f, n = 0.f;
-    for (int t = t0; t < t1; ++t) {
-      if (mp && mp[t]) continue;
-      const float m = __ldg(gm + base + (size_t)t * G), v = __ldg(gv + base + (size_t)t * G);
-      if (n == 0.f) c = m;
-      const float d = m - c;
-      s1 += d;
-      s2 += fmaf(d, d, v);
-      n += 1.f;
+    for (int k = t0; k < t1; k += kFwdB) {
+      fetch(k);
+#pragma unroll
+      for (int j = 0; j < kFwdB; ++j) {
+        if (skip[j]) continue;
+        if (n == 0.f) c = ms[j];
+        const float d = ms[j] - c;
+        s1 += d;
+        s2 += fmaf(d, d, vs[j]);
+        n += 1.f;
+      }
     }
     if (n > 0.f) r = {n, c + s1 / n, fmaxf(s2 - s1 * s1 / n, 0.f)};
   }
@@ -146,22 +163,26 @@ __global__ void __launch_bounds__(kScanG* kScanT) group_scan_kernel(const float*
   // second walk, sums about the mean that came in (or the first value when nothing did)
   float c = in.m, s1 = 0.f, s2 = 0.f, n = in.n;
   float mean = in.n > 0.f ? in.m : prior.m, var = in.n > 0.f ? in.s / in.n : prev_var[(size_t)b * G + g];
-  for (int t = t0; t < t1; ++t) {
-    const size_t i = base + (size_t)t * G;
-    const bool mk = mp && mp[t];
-    if (!mk) {
-      const float m = __ldg(gm + i), v = __ldg(gv + i);
-      if (n == 0.f) c = m;
-      const float d = m - c;
-      s1 += d;
-      s2 += fmaf(d, d, v);
-      n += 1.f;
-      const float inv = 1.f / n, u = s1 * inv;
-      mean = c + u;
-      var = fmaxf(fmaf(-u, u, (in.s + s2) * inv), 0.f);
+  for (int k = t0; k < t1; k += kFwdB) {
+    fetch(k);
+#pragma unroll
+    for (int j = 0; j < kFwdB; ++j) {
+      if (!skip[j]) {
+        if (n == 0.f) c = ms[j];
+        const float d = ms[j] - c;
+        s1 += d;
+        s2 += fmaf(d, d, vs[j]);
+        n += 1.f;
+        const float inv = 1.f / n, u = s1 * inv;
+        mean = c + u;
+        var = fmaxf(fmaf(-u, u, (in.s + s2) * inv), 0.f);
+      }
+      if (k + j < t1) {
+        const size_t i = base + (size_t)(k + j) * G;
+        cummean[i] = mean;
+        cumrstd[i] = rsqrtf(var + eps);
+      }
     }
-    cummean[i] = mean;
-    cumrstd[i] = rsqrtf(var + eps);
   }
   if (ti == kScanT - 1) {
     const Run all = part[ti][gi];
@@ -299,18 +320,35 @@ __global__ void __launch_bounds__(kScanG* kScanT) group_bwd_scan_kernel(const fl
   const float n_end = (float)count[b];
   const float n_in = n_end - later;   // count after this run's last step
   auto prev_u = [&](int t) -> float { return t > 0 ? __ldg(cummean + base + (size_t)(t - 1) * G) : prev_mean[(size_t)b * G + g]; };
+  constexpr int kBwdB = 4;   // (steps whose loads go out together)
+  float lr[kBwdB], le[kBwdB], ls[kBwdB], lb[kBwdB];
+  bool skip[kBwdB];
+  auto fetch = [&](int k) {   // steps k, k - 1, ...
+#pragma unroll
+    for (int j = 0; j < kBwdB; ++j) {
+      const int t = max(k - j, lo);
+      const size_t i = base + (size_t)t * G;
+      lr[j] = __ldg(cumrstd + i);
+      le[j] = 2.f * (__ldg(group_mean + i) - prev_u(t));
+      ls[j] = __ldg(ds + i);
+      lb[j] = __ldg(db + i);
+      skip[j] = k - j < lo || (mp && mp[t]);
+    }
+  };
   Map m{0.f, 0.f, 0.f, 0.f};
   if (ok) {
     float n = n_in;
-    for (int t = hi - 1; t >= lo; --t) {
-      if (mp && mp[t]) continue;
-      const size_t i = base + (size_t)t * G;
-      const float rs = __ldg(cumrstd + i), inv = 1.f / n;
-      const float e = 2.f * (__ldg(group_mean + i) - prev_u(t)) * inv;
-      m.sv -= 0.5f * (rs * rs * rs) * __ldg(ds + i) * inv;
-      m.su -= fmaf(e, m.sv, rs * __ldg(db + i) * inv);
-      m.sw -= e;
-      n -= 1.f;
+    for (int k = hi - 1; k >= lo; k -= kBwdB) {
+      fetch(k);
+#pragma unroll
+      for (int j = 0; j < kBwdB; ++j) {
+        if (skip[j]) continue;
+        const float rs = lr[j], inv = 1.f / n, e = le[j] * inv;
+        m.sv -= 0.5f * (rs * rs * rs) * ls[j] * inv;
+        m.su -= fmaf(e, m.sv, rs * lb[j] * inv);
+        m.sw -= e;
+        n -= 1.f;
+      }
     }
     m.n = n_in - n;
   }
@@ -334,21 +372,26 @@ __global__ void __launch_bounds__(kScanG* kScanT) group_bwd_scan_kernel(const fl
     U = u0 + p.su + p.sw * v0;
   }
   float n = n_in;
-  for (int t = hi - 1; t >= lo; --t) {
-    const size_t i = base + (size_t)t * G;
-    float ou = 0.f, ov = 0.f;
-    if (!(mp && mp[t])) {
-      const float rs = __ldg(cumrstd + i), inv = 1.f / n;
-      const float e = 2.f * (__ldg(group_mean + i) - prev_u(t));
-      V -= 0.5f * (rs * rs * rs) * __ldg(ds + i) * inv;
-      const float h = U - rs * __ldg(db + i) * inv;
-      ov = V;
-      ou = fmaf((n - 1.f) * inv * e, V, h);
-      U = fmaf(-e * inv, V, h);
-      n -= 1.f;
+  for (int k = hi - 1; k >= lo; k -= kBwdB) {
+    fetch(k);
+#pragma unroll
+    for (int j = 0; j < kBwdB; ++j) {
+      float ou = 0.f, ov = 0.f;
+      if (!skip[j]) {
+        const float rs = lr[j], inv = 1.f / n, e = le[j];
+        V -= 0.5f * (rs * rs * rs) * ls[j] * inv;
+        const float h = U - rs * lb[j] * inv;
+        ov = V;
+        ou = fmaf((n - 1.f) * inv * e, V, h);
+        U = fmaf(-e * inv, V, h);
+        n -= 1.f;
+      }
+      if (k - j >= lo) {
+        const size_t i = base + (size_t)(k - j) * G;
+        dux[i] = ou;
+        dvx[i] = ov;
+      }
     }
-    dux[i] = ou;
-    dvx[i] = ov;
   }
   if (ti == kScanT - 1) {
     const Map all = part[ti][gi];
