@@ -229,7 +229,13 @@ __global__ void __launch_bounds__(kW * 32, kC ? 1 : 2) scan_cluster_kernel(Clust
     }
     r = Run{(float)cnt0, __ldg(a.prev_mean + i), __ldg(a.prev_var + i) * (float)cnt0};
     const float* all = run + kW * 3 * 32 + lane;
-    for (int k = 0; k < rank; ++k) r = combine(r, Run{peer(all, k), peer(all + 32, k), peer(all + 64, k)});
+    Run before[7];   // (at most eight blocks; all reads of the others at once)
+#pragma unroll
+    for (int k = 0; k < 7; ++k)
+      if (k < rank) before[k] = Run{peer(all, k), peer(all + 32, k), peer(all + 64, k)};
+#pragma unroll
+    for (int k = 0; k < 7; ++k)
+      if (k < rank) r = combine(r, before[k]);
     for (int k = 0; k < warp; ++k)
       r = combine(r, Run{run[(k * 3) * 32 + lane], run[(k * 3 + 1) * 32 + lane], run[(k * 3 + 2) * 32 + lane]});
     rs.start(r);
@@ -318,12 +324,18 @@ __global__ void __launch_bounds__(kW * 32, kC ? 1 : 2) scan_cluster_kernel(Clust
         float2 whole = full[dir][k];   // q^(steps of a block)
 #pragma unroll
         for (int i = 0; i < 3; ++i) whole = kC ? cmul(whole, whole) : make_float2(whole.x * whole.x, 0.f);
-        for (int i = 0; i < (dir == 0 ? rank : ranks - 1 - rank); ++i) {
-          const int r = dir == 0 ? i : ranks - 1 - i;
-          const float2 v = make_float2(gain * peer(t, r), kC ? gain * peer(t + 16 * 32, r) : 0.f);
+        const int before = dir == 0 ? rank : ranks - 1 - rank;
+        float2 v[7];
+#pragma unroll
+        for (int i = 0; i < 7; ++i)
+          if (i < before) {
+            const int r = dir == 0 ? i : ranks - 1 - i;
+            v[i] = make_float2(gain * peer(t, r), kC ? gain * peer(t + 16 * 32, r) : 0.f);
+          }
+#pragma unroll
+        for (int i = 0; i < 7; ++i)
           // (blocks before one with steps are whole; against time, H is zero until the last of them)
-          H = onward<kC>(whole, H, v);
-        }
+          if (i < before) H = onward<kC>(whole, H, v[i]);
       }
       float* v = st + dir * kW * kState_ + pole * 32 + lane;
 #pragma unroll
@@ -434,19 +446,20 @@ namespace {
 // Steps of a segment and blocks of a cluster: the smallest product of rounds and steps (60 steps' worth of time pass
 // beside them: copies in, exchange of states).  False when the sequence does not fit, or is one of complex poles walked
 // both ways (its exchange costs more than the launches it saves).
-bool plan(int dtype, const ScanArgs& a, int& T, int& ranks, double& rounds) {
+bool plan(int dtype, const ScanArgs& a, int& T, int& ranks, double& rounds, double& best) {
   if ((a.cplx && a.bidir) || a.B > 65535 || a.N > 16) return false;
   const bool norm = a.prev_count != nullptr;
   const int dirs = a.bidir ? 2 : 1;
   const int row = (norm ? 128 : 32 * elem_size(dtype)) + (a.bidir ? 128 : 0);
   const double strips = (double)((a.D + 31) / 32) * a.B;
-  double best = 1e30;
+  best = 1e30;
   for (int c = 1; c <= 8; c *= 2) {
     const int t = std::max(16, ((a.L + c * kW - 1) / (c * kW) + kU - 1) / kU * kU);
     const int smem = kW * t * row + dirs * (kW + 1) * (a.cplx ? 2 : 1) * 2048 + (kW + 1) * 384 + kW * (t / 32 + 1) * 4;
     if (smem > 200 * 1024) continue;
     const int per_sm = std::max(1, std::min(227 * 1024 / (smem + 1024), a.cplx ? 1 : 2));
-    const double n = std::ceil(strips * c / (148.0 * per_sm));
+    // (a cluster stays within a group of 16 to 18 SMs: larger ones leave some of them over)
+    const double n = std::ceil(strips * c / ((c == 8 ? 112.0 : c == 4 ? 132.0 : 148.0) * per_sm));
     const double cost = n * (t + 60.0) * (strips * c > 148 ? std::min<double>(per_sm, strips * c / 148.0) : 1.0);
     if (cost < best) {
       best = cost;
@@ -465,34 +478,34 @@ bool plan(int dtype, const ScanArgs& a, int& T, int& ranks, double& rounds) {
 // take.  Beyond eight million elements, or in rounds of long segments, the three launches of scan_ema.cu are as fast.
 double scan_cluster_us(int dtype, const ScanArgs& a) {
   int T = 0, ranks = 1;
-  double rounds = 0;
+  double rounds = 0, steps = 0;
   const double n = (double)a.B * a.L * a.D;
-  if (!plan(dtype, a, T, ranks, rounds)) return 1e30;
-  if (n > (a.cplx ? 6.5e6 : a.bidir ? 4.3e6 : 8.5e6) || (rounds > 1 && T > 64)) return 1e30;
+  if (!plan(dtype, a, T, ranks, rounds, steps)) return 1e30;
+  if (n > (a.cplx && rounds > 1 ? 6.5e6 : a.bidir ? 4.3e6 : 8.5e6) || (rounds > 1 && T > 64)) return 1e30;
   const bool norm = a.prev_count != nullptr;
   const double fixed = a.cplx ? 14.0 : a.bidir ? 12.0 : norm ? 8.0 : 6.0;
-  const double step = a.cplx ? (norm ? 1.0 : 0.45) : a.bidir ? 0.5 : norm ? 0.4 : 0.3;
-  const double rate = a.cplx ? (norm ? 85e3 : 115e3) : a.bidir ? 100e3 : norm ? 140e3 : 195e3;
-  return fixed + std::max(T * step, n / rate);
+  const double step = a.cplx ? (norm ? 0.4 : 0.3) : a.bidir ? 0.4 : norm ? 0.22 : 0.14;
+  const double rate = a.cplx ? (norm ? 85e3 : 115e3) : a.bidir ? 100e3 : norm ? 165e3 : 195e3;
+  return std::max(fixed + std::max(T * step, n / rate), (a.cplx ? 0.27 : 0.08) * steps);   // (many short rounds: the latter)
 }
 
-// The chain costs 24 ns per position pipelined along the sequence, 44 with a mask and 48 complex, until all elements cost
-// more (1.3 and 0.6 per ns); a tenth in hand for the model.
+// The chain costs 24 ns per position pipelined along the sequence, 44 with a mask, and 28 complex beside 54 us of its own
+// (filling the pipeline of its tiles), until all elements cost more (1.3 and 0.6 per ns); a tenth in hand for the model.
 bool scan_cluster_first(int dtype, const ScanArgs& a, long long xsd, long long ysd) {
   if (dtype != MEGA_BF16 || a.bidir || g_options[OPT_SPLIT].load() == 1 || g_options[OPT_DISABLE_MMA].load() != 0 ||
       g_options[OPT_MMA_TILE].load() != 0 || !scan_ema_fwd_ok(dtype, a, xsd, ysd))
     return false;
   if (a.h_out && !a.mask && !a.cplx && a.L % 32 != 0) return false;   // (that kernel's head, then a tail of under 32 steps)
   const double n = (double)a.B * a.L * a.D;
-  const double chain = a.L * (a.cplx ? 48e-3 : a.mask ? 44e-3 : 24e-3), all = n / (a.cplx ? 600e3 : 1300e3);
+  const double chain = a.cplx ? 54.0 + a.L * 28e-3 : a.L * (a.mask ? 44e-3 : 24e-3), all = n / (a.cplx ? 600e3 : 1300e3);
   return scan_cluster_us(dtype, a) < 0.9 * (6.0 + std::max(chain, all));
 }
 
 bool scan_cluster_try(int dtype, const ScanArgs& a, cudaStream_t st) {
   ClusterArgs s{a, 0};
   int ranks = 1;
-  double rounds;
-  if (scan_cluster_us(dtype, a) > 1e29 || !plan(dtype, a, s.T, ranks, rounds)) return false;
+  double rounds, steps;
+  if (scan_cluster_us(dtype, a) > 1e29 || !plan(dtype, a, s.T, ranks, rounds, steps)) return false;
   switch (dtype) {
     case MEGA_F32: return a.cplx ? launch_form<float, true>(s, ranks, st) : launch_form<float, false>(s, ranks, st);
     case MEGA_BF16: return a.cplx ? launch_form<__nv_bfloat16, true>(s, ranks, st) : launch_form<__nv_bfloat16, false>(s, ranks, st);
