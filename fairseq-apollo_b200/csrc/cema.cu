@@ -773,15 +773,15 @@ extern "C" int mega_tsn_cema_fwd(const void* x, void* y, void* xn_out, int dtype
         tail.count_offset = Lh;
         tail.prev_mean = mean_out; tail.prev_var = var_out; tail.h_in = h_out;
         if (stream_cl_try(dtype, (const char*)x + (size_t)Lh * xsl * es, (char*)y + (size_t)Lh * ysl * es,
-                          xn_out ? (char*)xn_out + (size_t)Lh * ysl * es : nullptr, xsb, xsl, xsd, ysb, ysl, ysd, true, true,
-                          tail, (cudaStream_t)stream))
+                          xn_out ? (char*)xn_out + (size_t)Lh * ysl * es : nullptr, xsb, xsl, xsd, ysb, ysl, ysd, true, tail,
+                          (cudaStream_t)stream))
           return check_launch("tsn_cema_fwd(mma head + stream tail)");
         // (the streamed kernel refused, which its envelope rules out here: the whole call below)
       }
     }
     if (mma_cl_try(dtype, x, y, xn_out, xsb, xsl, xsd, ysb, ysl, ysd, true, sa, (cudaStream_t)stream))
       return check_launch("tsn_cema_fwd(mma)");
-    if (stream_cl_try(dtype, x, y, xn_out, xsb, xsl, xsd, ysb, ysl, ysd, true, true, sa, (cudaStream_t)stream))
+    if (stream_cl_try(dtype, x, y, xn_out, xsb, xsl, xsd, ysb, ysl, ysd, true, sa, (cudaStream_t)stream))
       return check_launch("tsn_cema_fwd(stream)");
   }
   // outside the streamed kernel's envelope: the two operators in turn (the EMA runs in place)

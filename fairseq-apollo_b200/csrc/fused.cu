@@ -476,7 +476,7 @@ extern "C" int mega_tsn_ema_fwd(const void* x, void* y, void* xn_out, int dtype,
         tail.L = L - Lh;
         tail.count_offset = Lh;
         tail.prev_mean = mean_out; tail.prev_var = var_out; tail.h_in = h_out;
-        if (stream_cl_try(dtype, xt, yt, nt, xsb, xsl, xsd, ysb, ysl, ysd, true, true, tail, (cudaStream_t)stream))
+        if (stream_cl_try(dtype, xt, yt, nt, xsb, xsl, xsd, ysb, ysl, ysd, true, tail, (cudaStream_t)stream))
           return check_launch("tsn_ema_fwd(mma head + stream tail)");
         a.x = xt; a.y = yt; a.xn = nt; a.L = L - Lh; a.count_offset = Lh;
         a.prev_mean = mean_out; a.prev_var = var_out; a.h_in = h_out;
@@ -490,7 +490,7 @@ extern "C" int mega_tsn_ema_fwd(const void* x, void* y, void* xn_out, int dtype,
     // (the tensor-core kernel writes the normalised activations too when xn_out is given)
     if (mma_cl_try(dtype, x, y, xn_out, xsb, xsl, xsd, ysb, ysl, ysd, true, sa, (cudaStream_t)stream))
       return check_launch("tsn_ema_fwd(mma)");
-    if (stream_cl_try(dtype, x, y, xn_out, xsb, xsl, xsd, ysb, ysl, ysd, true, true, sa, (cudaStream_t)stream))
+    if (stream_cl_try(dtype, x, y, xn_out, xsb, xsl, xsd, ysb, ysl, ysd, true, sa, (cudaStream_t)stream))
       return check_launch("tsn_ema_fwd(stream)");
   }
   const int np = next_pow2_ndim(N);

@@ -588,7 +588,7 @@ static int tsn_fwd_common(const void* x, void* y, int dtype, int B, int L, int D
       // (a form of the tensor-core kernel asked for by name, or the streamed kernel)
       if (!cummean && mma_cl_try(dtype, x, y, nullptr, xsb, xsl, xsd, ysb, ysl, ysd, true, sa, (cudaStream_t)stream))
         return check_launch("timestep_norm_fwd(mma)");
-      if (stream_cl_try(dtype, x, y, nullptr, xsb, xsl, xsd, ysb, ysl, ysd, true, false, sa, (cudaStream_t)stream))
+      if (stream_cl_try(dtype, x, y, nullptr, xsb, xsl, xsd, ysb, ysl, ysd, false, sa, (cudaStream_t)stream))
         return check_launch("timestep_norm_fwd(stream)");
     }
     const unsigned grid = (unsigned)(((long long)B * D + 127) / 128);

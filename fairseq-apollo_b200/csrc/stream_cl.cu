@@ -1,4 +1,4 @@
-// Streamed channel-contiguous kernels: TimestepNorm, causal EMA, or both fused, for activations
+// Streamed channel-contiguous kernels: TimestepNorm, alone or with the causal EMA behind it, for activations
 // whose channel stride is 1 ((B, L, D) and time-major (L, B, D) memory).
 //
 // One CTA owns kW adjacent channels of one sequence and walks the sequence in tiles of kR
@@ -78,7 +78,7 @@ struct StreamCfg {
   }
 };
 
-template <typename T, bool kNorm, bool kEma, bool kState, bool kCplx, bool kSave>
+template <typename T, bool kEma, bool kState, bool kCplx, bool kSave>
 __global__ void __launch_bounds__(kW) stream_cl_kernel(const __grid_constant__ CUtensorMap tmx,
                                                        const __grid_constant__ CUtensorMap tmy,
                                                        const __grid_constant__ CUtensorMap tmn,
@@ -196,16 +196,14 @@ __global__ void __launch_bounds__(kW) stream_cl_kernel(const __grid_constant__ C
     }
   }
   float mean = 0.f, var = 1.f, w = 1.f, bb = 0.f;
-  if (kNorm) {
-    mean = a.prev_mean[(size_t)b * a.D + dc];
-    var = a.prev_var[(size_t)b * a.D + dc];
-    w = __ldg(a.gamma + dc);
-    bb = __ldg(a.beta + dc);
-  }
+  mean = a.prev_mean[(size_t)b * a.D + dc];
+  var = a.prev_var[(size_t)b * a.D + dc];
+  w = __ldg(a.gamma + dc);
+  bb = __ldg(a.beta + dc);
 
   // warp 0 keeps the running count and publishes, per timestep of the next tile, the Welford
   // coefficient 1/count (negative = padded step)
-  long long cnt_run = kNorm ? a.prev_count[b] + a.count_offset : 0;
+  long long cnt_run = a.prev_count[b] + a.count_offset;
   const unsigned char* mrow = a.mask ? a.mask + (size_t)b * L : nullptr;
   auto publish = [&](int tile, unsigned char mk_byte) {
     // called by warp 0 (kR == 32 lanes); lane r handles timestep tile*kR + r
@@ -247,24 +245,20 @@ __global__ void __launch_bounds__(kW) stream_cl_kernel(const __grid_constant__ C
         const float coef = cf[r];
         const bool mk = coef < 0.f;
         float xn;
-        if (kNorm) {
-          const float d1 = xr - mean;
-          const float m1 = fmaf(coef, d1, mean);
-          const float dm = xr - m1;
-          const float d2 = fmaf(d1, dm, -var);
-          const float m2 = fmaf(coef, d2, var);
-          const float rstd = rsqrtf(m2 + a.eps);
-          xn = mk ? 0.f : fmaf(dm * rstd, w, bb);
-          mean = mk ? mean : m1;
-          var = mk ? var : m2;
-          if (kSave) {  // the running mean after this step (unchanged by a padded step)
-            cms[(o * kR + r) * kW + tid] = mean;
-            crs[(o * kR + r) * kW + tid] = rstd;
-          }
-          if (!kEma || a.has_xn) Elem<T>::st((kEma ? ntile : yt) + r * kW, xn);
-        } else {
-          xn = mk ? 0.f : xr;
+        const float d1 = xr - mean;
+        const float m1 = fmaf(coef, d1, mean);
+        const float dm = xr - m1;
+        const float d2 = fmaf(d1, dm, -var);
+        const float m2 = fmaf(coef, d2, var);
+        const float rstd = rsqrtf(m2 + a.eps);
+        xn = mk ? 0.f : fmaf(dm * rstd, w, bb);
+        mean = mk ? mean : m1;
+        var = mk ? var : m2;
+        if (kSave) {  // the running mean after this step (unchanged by a padded step)
+          cms[(o * kR + r) * kW + tid] = mean;
+          crs[(o * kR + r) * kW + tid] = rstd;
         }
+        if (!kEma || a.has_xn) Elem<T>::st((kEma ? ntile : yt) + r * kW, xn);
         if (kEma) {
           const f32x2 x2 = pack2(xn, xn);
           f32x2 acc0 = pack2(0.f, 0.f), acc1 = pack2(0.f, 0.f);
@@ -296,7 +290,7 @@ __global__ void __launch_bounds__(kW) stream_cl_kernel(const __grid_constant__ C
           }
           float lo, hi;
           unpack2(add2(acc0, acc1), lo, hi);
-          float v = fmaf(om, kNorm ? xn : xr, lo + hi);
+          float v = fmaf(om, xn, lo + hi);
           if (a.silu) v = siluf_(v);
           Elem<T>::st(yt + r * kW, v);
         }
@@ -308,7 +302,7 @@ __global__ void __launch_bounds__(kW) stream_cl_kernel(const __grid_constant__ C
     if (__syncthreads_or(!ok)) break;
     if (tid == 0) {
       tma_store_3d(&tmy, d0, i * kR, b, ys + (size_t)o * kR * kW);
-      if (kNorm && kEma && a.has_xn) tma_store_3d(&tmn, d0, i * kR, b, ns + (size_t)o * kR * kW);
+      if (kEma && a.has_xn) tma_store_3d(&tmn, d0, i * kR, b, ns + (size_t)o * kR * kW);
       if (kSave) {
         tma_store_3d(&tmm, d0, i * kR, b, cms + (size_t)o * kR * kW);
         tma_store_3d(&tmr, d0, i * kR, b, crs + (size_t)o * kR * kW);
@@ -323,10 +317,8 @@ __global__ void __launch_bounds__(kW) stream_cl_kernel(const __grid_constant__ C
   if (tid == 0) bulk_wait<0>();
 
   if (valid) {
-    if (kNorm) {
-      a.mean_out[(size_t)b * a.D + d] = mean;
-      a.var_out[(size_t)b * a.D + d] = var;
-    }
+    a.mean_out[(size_t)b * a.D + d] = mean;
+    a.var_out[(size_t)b * a.D + d] = var;
     if (kEma && kState && kCplx && a.h_out) {
 #pragma unroll
       for (int j = 0; j < kNP / 2; ++j) {
@@ -353,16 +345,16 @@ __global__ void __launch_bounds__(kW) stream_cl_kernel(const __grid_constant__ C
       }
     }
   }
-  if (kNorm && blockIdx.x == 0 && tid == 0) a.count_out[b] = cnt_run;
+  if (blockIdx.x == 0 && tid == 0) a.count_out[b] = cnt_run;
 }
 
 // ---------------------------------------------------------------------------
 // host launcher
 // ---------------------------------------------------------------------------
-template <typename T, bool kNorm, bool kEma, bool kState, bool kCplx = false, bool kSave = false>
+template <typename T, bool kEma, bool kState, bool kCplx = false, bool kSave = false>
 static bool launch_one(const CUtensorMap& tx, const CUtensorMap& ty, const CUtensorMap& tn, const StreamArgs& a,
                        cudaStream_t s, const CUtensorMap* tm = nullptr, const CUtensorMap* tr = nullptr) {
-  auto kern = stream_cl_kernel<T, kNorm, kEma, kState, kCplx, kSave>;
+  auto kern = stream_cl_kernel<T, kEma, kState, kCplx, kSave>;
   const int smem = StreamCfg<T>::smem_bytes(a.has_xn != 0, kSave);
   static std::once_flag once;
   static bool attr_ok = true;
@@ -383,14 +375,14 @@ static bool launch_one(const CUtensorMap& tx, const CUtensorMap& ty, const CUten
 // Tries the streamed path; returns false (nothing launched) when the call is outside its envelope:
 // channel stride must be 1, ndim <= 16, 16-byte aligned bases and strides, B <= 65535.
 bool stream_cl_try(int dtype, const void* x, void* y, void* xn, long long xsb, long long xsl, long long xsd,
-                   long long ysb, long long ysl, long long ysd, bool norm, bool ema, const StreamArgs& a_in,
+                   long long ysb, long long ysl, long long ysd, bool ema, const StreamArgs& a_in,
                    cudaStream_t s) {
   if (g_options[OPT_DISABLE_STREAM].load() != 0) return false;
   if (xsd != 1 || ysd != 1) return false;
   if (ema && a_in.N > kNP) return false;
   if (a_in.B > 65535 || a_in.D < 8) return false;
   StreamArgs a = a_in;
-  a.has_xn = (xn != nullptr && norm && ema) ? 1 : 0;
+  a.has_xn = (xn != nullptr && ema) ? 1 : 0;
   CUtensorMap tx, ty, tn;
   if (!make_tensor_map_3d(&tx, dtype, x, a.D, a.L, a.B, xsl, xsb, kW, kR, 1, CU_TENSOR_MAP_SWIZZLE_NONE))
     return false;
@@ -401,7 +393,7 @@ bool stream_cl_try(int dtype, const void* x, void* y, void* xn, long long xsb, l
       !make_tensor_map_3d(&tn, dtype, xn, a.D, a.L, a.B, ysl, ysb, kW, kR, 1, CU_TENSOR_MAP_SWIZZLE_NONE))
     return false;
   const bool state = ema && (a.h_in || a.h_out);
-  const bool save = norm && !ema && a.cummean != nullptr && a.cumrstd != nullptr;
+  const bool save = !ema && a.cummean != nullptr && a.cumrstd != nullptr;
   CUtensorMap tm, tr;
   if (save) {
     if (!make_tensor_map_3d(&tm, MEGA_F32, a.cummean, a.D, a.L, a.B, a.D, (long long)a.L * a.D, kW, kR, 1,
@@ -414,17 +406,12 @@ bool stream_cl_try(int dtype, const void* x, void* y, void* xn, long long xsb, l
   switch (dtype) {
 #define MEGA_STREAM_CASE(DT, TY)                                                        \
   case DT:                                                                              \
-    if (ema && a.cplx) {                                                                \
-      if (norm) ok = state ? launch_one<TY, true, true, true, true>(tx, ty, tn, a, s)   \
-                           : launch_one<TY, true, true, false, true>(tx, ty, tn, a, s); \
-      else ok = state ? launch_one<TY, false, true, true, true>(tx, ty, tn, a, s)       \
-                      : launch_one<TY, false, true, false, true>(tx, ty, tn, a, s);     \
-    } else if (norm && ema) ok = state ? launch_one<TY, true, true, true>(tx, ty, tn, a, s)    \
-                                : launch_one<TY, true, true, false>(tx, ty, tn, a, s);  \
-    else if (ema) ok = state ? launch_one<TY, false, true, true>(tx, ty, tn, a, s)      \
-                             : launch_one<TY, false, true, false>(tx, ty, tn, a, s);    \
-    else if (save) ok = launch_one<TY, true, false, false, false, true>(tx, ty, tn, a, s, &tm, &tr); \
-    else ok = launch_one<TY, true, false, false>(tx, ty, tn, a, s);                     \
+    if (ema && a.cplx) ok = state ? launch_one<TY, true, true, true>(tx, ty, tn, a, s)   \
+                                  : launch_one<TY, true, false, true>(tx, ty, tn, a, s); \
+    else if (ema) ok = state ? launch_one<TY, true, true>(tx, ty, tn, a, s)             \
+                             : launch_one<TY, true, false>(tx, ty, tn, a, s);           \
+    else if (save) ok = launch_one<TY, false, false, false, true>(tx, ty, tn, a, s, &tm, &tr); \
+    else ok = launch_one<TY, false, false>(tx, ty, tn, a, s);                           \
     break;
     MEGA_STREAM_CASE(MEGA_F32, float)
     MEGA_STREAM_CASE(MEGA_BF16, __nv_bfloat16)

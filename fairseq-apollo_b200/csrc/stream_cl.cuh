@@ -33,12 +33,11 @@ struct StreamArgs {
                      // [1 + n_items]: set when a wait of this launch ran out
 };
 
-// Tries the streamed TMA path for TimestepNorm (norm), causal EMA (ema) or both fused.  Returns
+// Tries the streamed TMA path for TimestepNorm, alone or (ema) with the causal EMA behind it.  Returns
 // false, having launched nothing, when the call is outside its envelope (channel stride != 1,
 // ndim > 16, bases or strides not 16-byte aligned, more than 65535 sequences).
 bool stream_cl_try(int dtype, const void* x, void* y, void* xn, long long xsb, long long xsl, long long xsd,
-                   long long ysb, long long ysl, long long ysd, bool norm, bool ema, const StreamArgs& a,
-                   cudaStream_t s);
+                   long long ysb, long long ysl, long long ysd, bool ema, const StreamArgs& a, cudaStream_t s);
 
 // Tries the tensor-core path (mma_cl.cu): bf16, channel stride 1, ndim <= 16 (its envelope is
 // stated at the definition).  Same contract as stream_cl_try.

@@ -4,8 +4,8 @@ libmega_b200.so on the current CUDA stream.
 The functions mirror the operator surface the reference's Python wrappers expect from
 ``fairseq.mega2_extension.ops`` (fairseq/modules/fused_ops/*.py,
 fairseq/modules/norm_layer/*.py), with the FFT convolution, its bias and the hidden-state
-update folded into one ``ema_forward``.  Outputs are allocated here with torch (device
-memory plumbing); the library itself allocates nothing.
+update folded into one ``ema_forward``.  Outputs are allocated with torch, by the
+native host side (host/host.cpp) where an operator is one of the package's own paths.
 """
 from typing import Optional, Tuple
 
@@ -238,25 +238,6 @@ def tsn_cema_step_(x, y, count, mean, var, gamma, beta, eps, p, q, g, omega, h, 
 
 
 # --------------------------------------------------------------------------- gates
-def _rows(t):
-    """View t (..., cols) as `rows` rows of `cols` elements with one row pitch; copies only
-    when the memory is not a uniform-pitch row-major matrix (e.g. after a transpose)."""
-    cols = t.shape[-1]
-    if t.dim() == 1:
-        t = t.unsqueeze(0)
-    ok = t.stride(-1) == 1 or cols == 1
-    ld = t.stride(-2) if t.shape[-2] > 1 else max(cols, t.stride(-2))
-    exp = ld
-    for size, stride in zip(reversed(t.shape[:-1]), reversed(t.stride()[:-1])):
-        if size != 1 and stride != exp:
-            ok = False
-        exp *= size
-    if not ok or ld < cols:
-        t = t.contiguous()
-        ld = cols
-    return t, t.numel() // cols, cols, ld
-
-
 def gate_silu(a, b=None):
     """silu(a [+ b]) elementwise; a, b may be column slices of wider row-major matrices."""
     return _lib.host().gate_silu(a, b)
