@@ -78,6 +78,7 @@ SIGNATURES = {
                           c_p, c_p, c_d, c_p, c_p, c_p, c_p, c_p, c_p, c_p, c_i, c_p, c_p, c_p, c_u, c_p],
     "mega_norm_prepare": [c_p] * 5 + [c_i] * 4 + [c_p] * 6,
     "mega_norm_finish": [c_p] * 5 + [c_i] * 4 + [c_p] * 5,
+    "mega_to_float": [c_p, c_p, c_p, c_i, c_i, c_p],
     "mega_gate_silu_bwd": [c_p, c_l] * 3 + [c_p, c_i, c_l, c_i, c_p],
     "mega_gate_mul_silu_bwd": [c_p, c_l] * 5 + [c_p, c_i, c_l, c_i, c_p],
     "mega_gate_output_bwd": [c_p, c_l] * 8 + [c_p, c_p, c_i, c_l, c_i, c_p],
