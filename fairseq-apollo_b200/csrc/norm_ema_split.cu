@@ -27,12 +27,17 @@ bool mma_takes(int dtype, const StreamArgs& a, bool want_xn) {
   return dtype == MEGA_BF16 && g_options[OPT_DISABLE_MMA].load() == 0 && !(a.mask && a.cplx) && (a.B >= 4 || pipes);
 }
 
-// (a part for the launch and, on the tensor-core kernel with complex poles, for filling the pipeline of its tiles)
+// (a part for the launch and, on the tensor-core kernel with complex poles, for filling the pipeline of its tiles; long
+// chains of the forms with a second output or a mask fall behind the short ones' rate)
 double fused_us(int dtype, const StreamArgs& a, bool want_xn) {
   const double L = a.L, n = (double)a.B * a.D * a.L;
   if (mma_takes(dtype, a, want_xn)) {
-    if (a.cplx) return 68.0 + longer(want_xn ? 46.0 : 36.0, want_xn ? 300e3 : 480e3, L, n);
-    return want_xn ? 15.0 + longer(44.0, 500e3, L, n) : a.mask ? 13.0 + longer(42.0, 520e3, L, n) : 11.0 + longer(30.0, 600e3, L, n);
+    const double fixed = a.cplx ? 68.0 : want_xn ? 15.0 : a.mask ? 13.0 : 11.0;
+    const double chain = a.cplx ? (want_xn ? 46.0 : 36.0) : want_xn ? 44.0 : a.mask ? 42.0 : 30.0;
+    const double rate = a.cplx ? (want_xn ? 300e3 : 480e3) : want_xn ? 500e3 : a.mask ? 520e3 : 600e3;
+    const double far = L * 1e-3 * (a.cplx ? (want_xn ? 75.0 : 62.0) : want_xn || a.mask ? 50.0 : 34.0);
+    const double near = fixed + longer(chain, rate, L, n);
+    return near > far ? near : far;
   }
   return a.cplx ? 8.0 + longer(171.0, 168e3, L, n) : 6.0 + longer(122.0, want_xn ? 160e3 : 260e3, L, n);
 }
@@ -42,7 +47,7 @@ double fused_us(int dtype, const StreamArgs& a, bool want_xn) {
 double mma_us(int dtype, const StreamArgs& a, bool want_xn) {
   if (!mma_takes(dtype, a, want_xn) || a.mask || (a.h_out && a.L % 32 != 0)) return 1e30;
   const double L = a.L, n = (double)a.B * a.D * a.L;
-  return 10.0 + n / 600e3 + (a.cplx ? 54.0 + longer(28.0, 600e3, L, n) : longer(24.0, 1300e3, L, n));
+  return 10.0 + n / 700e3 + (a.cplx ? 54.0 + longer(28.0, 600e3, L, n) : longer(22.0, 1300e3, L, n));
 }
 
 // (in one launch, or as the scan's five)
