@@ -24,7 +24,8 @@ double longer(double chain_ns, double per_us, double L, double n) {
 
 bool mma_takes(int dtype, const StreamArgs& a, bool want_xn) {
   const bool pipes = !want_xn && !a.cplx && a.mask == nullptr;   // forms pipelined along the sequence: any batch
-  return dtype == MEGA_BF16 && g_options[OPT_DISABLE_MMA].load() == 0 && !(a.mask && a.cplx) && (a.B >= 4 || pipes);
+  return dtype == MEGA_BF16 && g_options[OPT_DISABLE_MMA].load() == 0 && !(a.mask && a.cplx) && (a.B >= 4 || pipes) &&
+         !(a.cplx && a.h_out && a.L % 32 != 0);   // (it cannot stop a state in mid-step; a real layer's head still runs there)
 }
 
 // (a part for the launch and, on the tensor-core kernel with complex poles, for filling the pipeline of its tiles; long
