@@ -599,7 +599,8 @@ __global__ void __launch_bounds__(kWarps * 32, kC ? 2 : 3) scan_bwd_kernel(SegAr
 // Segments of a call.  A block takes four segments of 32 channels; `resident` blocks of the last kernel fit an SM.
 // The choice minimises (rounds of blocks over the 148 SMs) x (steps of a segment + what its states cost beside
 // them: written, carried and read, 64 steps' worth backward and 40 forward), so that neither a nearly empty last round nor short segments dominate.  Segments
-// are at least 32 steps; a bidirectional one keeps its share of the outputs in shared memory, so at most 64.
+// are at least 32 steps; a bidirectional one keeps its share of the outputs in shared memory, so at most 64: beyond 4096
+// of those the counts start from what the length asks for.
 // One segment per sequence when the channels alone fill the device: no first pass then.
 static void pick_segments(const ScanArgs& a, int resident, bool bwd, SegArgs& s) {
   const long long strips = (long long)((a.D + 31) / 32) * a.B;
@@ -614,7 +615,8 @@ static void pick_segments(const ScanArgs& a, int resident, bool bwd, SegArgs& s)
     // (2/3: without the first pass; few warps on an SM still leave its pipes idle: at least half of the slots)
     best = ceil(blocks / slots) * a.L * (2.0 / 3.0) * (blocks * 2 < slots ? 2.0 : 1.0);
   }
-  for (int S = kWarps; S <= 4096; S += kWarps) {
+  const int least = a.bidir ? (a.L + 63) / 64 : 1, from = (least + kWarps - 1) / kWarps * kWarps;
+  for (int S = from; S < from + 4096; S += kWarps) {
     int t = ((a.L + S - 1) / S + kU - 1) / kU * kU;
     if (t < 32) t = 32;
     if (a.bidir && t > 64) continue;
@@ -679,7 +681,7 @@ static bool dispatch(int dtype, const ScanArgs& a, cudaStream_t st) {
   s.a = a;
   // blocks per SM by registers
   pick_segments(a, kBwd ? (a.cplx ? 2 : 3) : (a.cplx || a.prev_count ? 3 : 4), kBwd, s);
-  if ((s.S + kWarps - 1) / kWarps > 65535) return false;
+  if (s.S < 1 || (s.S + kWarps - 1) / kWarps > 65535) return false;
   s.parts = (kBwd ? 3 : 1) * (a.cplx ? 2 : 1);
   const size_t floats = (!s.wide) ? (size_t)a.B * dirs * s.S * s.parts * 16 * a.D : 0;
   const bool norm = !kBwd && a.prev_count != nullptr;

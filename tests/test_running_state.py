@@ -41,3 +41,47 @@ def test_ragged_complex_prefill_state(split, normed, option):
     got = state["prev_state"].cpu().to(torch.complex128)
     assert float((got - h).norm() / h.norm()) < 1e-5
     assert rel_l2(state["prev_mean"], mean) < 1e-5 and rel_l2(state["prev_var"], var) < 1e-5
+
+
+def _taps(q, c, length, lag=0):
+    """sum_n c q^(t + lag) for t < length, (D, length) float64"""
+    t = torch.arange(lag, length + lag, dtype=torch.float64)
+    out = 0
+    for n in range(q.size(1)):
+        v = torch.exp(t * torch.log(q[:, n:n + 1])) * c[:, n:n + 1]
+        out = out + (v.real if v.is_complex() else v)
+    return out
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+def test_bidirectional_beyond_a_quarter_million(cplx):
+    """More segments of 64 positions than 4096; forward and input gradient against a convolution in float64."""
+    import math
+    from fairseq_apollo_b200 import functions, ops
+    gen = torch.Generator().manual_seed(3)
+    dim, ndim, length = 8, 4, 4096 * 64 + 1
+    alpha, delta = torch.randn(2 * dim, ndim, 1, generator=gen), torch.randn(2 * dim, ndim, 1, generator=gen)
+    third = torch.randn(2 * dim, 1 if cplx else ndim, 1, generator=gen)
+    gamma = torch.randn(2 * dim, ndim, 2, generator=gen) if cplx else torch.randn(2 * dim, ndim, generator=gen)
+    omega = torch.randn(dim, generator=gen)
+    from oracle import mega_oracle as O
+    p, q, g = (O.cema_coeffs if cplx else O.ema_coeffs)(alpha, delta, third, gamma, dtype=torch.float64)
+    x, dy = torch.randn(1, length, dim, generator=gen), torch.randn(1, length, dim, generator=gen)
+    xg = x.cuda().requires_grad_(True)
+    y = functions.ema(xg, *(t.cuda() for t in (alpha, delta, third, gamma, omega)), None, True, True, None, cplx, False, True)
+    y.backward(dy.cuda())
+    n = 2 * length
+    right, left = _taps(q[:dim], p[:dim] * g[:dim], length), _taps(q[dim:], p[dim:] * g[dim:], length)
+    kernel = torch.zeros(dim, n, dtype=torch.float64)
+    kernel[:, :length] = right
+    kernel[:, n - length + 1:] += left[:, :length - 1].flip(-1)    # lag -1 - k
+    kernel[:, 0] += omega.double()
+    kf = torch.fft.rfft(kernel)
+    conv = lambda t, k: torch.fft.irfft(torch.fft.rfft(t[0].t().double(), n=n) * k, n=n)[:, :length].t()
+    assert rel_l2(y[0], conv(x, kf)) < 5e-6
+    assert rel_l2(xg.grad[0], conv(dy, kf.conj())) < 5e-6
+    with torch.no_grad():
+        cf = ops.cema_coeffs if cplx else ops.ema_coeffs
+        out = (ops.cema_forward if cplx else ops.ema_forward)(
+            xg.transpose(1, 2), *cf(*(t.cuda() for t in (alpha, delta, third, gamma))), omega.cuda(), bidirectional=True)
+    assert rel_l2(out[0].t(), conv(x, kf)) < 5e-6
