@@ -161,6 +161,12 @@ static inline bool aligned_to(const void* p, size_t a) {
   return (reinterpret_cast<uintptr_t>(p) % a) == 0;
 }
 
+// Whether two arrays of n floats share memory (running statistics may be updated in place).
+static inline bool overlap(const float* a, const float* b, size_t n) {
+  const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b), bytes = n * sizeof(float);
+  return a != nullptr && b != nullptr && x < y + bytes && y < x + bytes;
+}
+
 static inline int next_pow2_ndim(int n) {
   int v = 2;
   while (v < n) v <<= 1;

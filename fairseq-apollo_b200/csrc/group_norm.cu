@@ -155,14 +155,17 @@ __global__ void __launch_bounds__(kScanG* kScanT) group_scan_kernel(const float*
     part[ti][gi] = mine;
     __syncthreads();
   }
-  if (!ok) return;
   const long long cnt0 = prev_count[b];
-  const Run prior{(float)cnt0, prev_mean[(size_t)b * G + g], prev_var[(size_t)b * G + g] * (float)cnt0};
+  const size_t at = (size_t)b * G + (ok ? g : 0);
+  const float mean0 = prev_mean[at], var0 = prev_var[at];
+  __syncthreads();   // (mean_out and var_out may be prev_mean and prev_var: all threads have read them)
+  if (!ok) return;
+  const Run prior{(float)cnt0, mean0, var0 * (float)cnt0};
   Run in = prior;
   if (ti > 0) in = combine(prior, part[ti - 1][gi]);
   // second walk, sums about the mean that came in (or the first value when nothing did)
   float c = in.m, s1 = 0.f, s2 = 0.f, n = in.n;
-  float mean = in.n > 0.f ? in.m : prior.m, var = in.n > 0.f ? in.s / in.n : prev_var[(size_t)b * G + g];
+  float mean = in.n > 0.f ? in.m : prior.m, var = in.n > 0.f ? in.s / in.n : var0;
   for (int k = t0; k < t1; k += kFwdB) {
     fetch(k);
 #pragma unroll
@@ -188,7 +191,7 @@ __global__ void __launch_bounds__(kScanG* kScanT) group_scan_kernel(const float*
     const Run all = part[ti][gi];
     const Run fin = combine(prior, all);
     mean_out[(size_t)b * G + g] = fin.n > 0.f ? fin.m : prior.m;
-    var_out[(size_t)b * G + g] = fin.n > 0.f ? fin.s / fin.n : prev_var[(size_t)b * G + g];
+    var_out[(size_t)b * G + g] = fin.n > 0.f ? fin.s / fin.n : var0;
     if (g == 0) count_out[b] = cnt0 + (long long)(all.n + 0.5f);
   }
 }

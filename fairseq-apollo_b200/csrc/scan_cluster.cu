@@ -444,11 +444,17 @@ bool launch_form(const ClusterArgs& s, int ranks, cudaStream_t st) {
 namespace {
 
 // Steps of a segment and blocks of a cluster: the smallest product of rounds and steps (60 steps' worth of time pass
-// beside them: copies in, exchange of states).  False when the sequence does not fit, or is one of complex poles walked
-// both ways (its exchange costs more than the launches it saves).
+// beside them: copies in, exchange of states).  False when the sequence does not fit, is one of complex poles walked both
+// ways (its exchange costs more than the launches it saves), or statistics or states are updated in place.
 bool plan(int dtype, const ScanArgs& a, int& T, int& ranks, double& rounds, double& best) {
   if ((a.cplx && a.bidir) || a.B > 65535 || a.N > 16) return false;
   const bool norm = a.prev_count != nullptr;
+  // (all blocks of a cluster read the incoming statistics and states, the last one writes the new ones)
+  const size_t stats = (size_t)a.B * a.D, states = stats * a.N * (a.cplx ? 2 : 1);
+  if (overlap(a.h_in, a.h_out, states)) return false;
+  if (norm)
+    for (const float* out : {a.mean_out, a.var_out})
+      if (overlap(out, a.prev_mean, stats) || overlap(out, a.prev_var, stats)) return false;
   const int dirs = a.bidir ? 2 : 1;
   const int row = (norm ? 128 : 32 * elem_size(dtype)) + (a.bidir ? 128 : 0);
   const double strips = (double)((a.D + 31) / 32) * a.B;

@@ -97,17 +97,18 @@ __device__ __forceinline__ Lane lane_of(const SegArgs& s) {
 }
 
 // ---- TimestepNorm in front --------------------------------------------------------------------------
-// Moments of the segments -> what each segment starts from, and the statistics after the last.
+// Moments of the segments -> what each segment starts from, and the statistics after the last (mean_out and var_out may
+// be prev_mean and prev_var: the thread that writes a channel's is the only one to read them).
 __global__ void __launch_bounds__(128) scan_stats_kernel(SegArgs s) {
   const ScanArgs& a = s.a;
   const int d = blockIdx.x * 128 + threadIdx.x, b = blockIdx.y;
+  if (d >= a.D) return;
   const long long cnt0 = a.prev_count[b];
   const float n0 = (float)cnt0;
-  const bool ok = d < a.D;
-  const size_t i = (size_t)b * a.D + (ok ? d : 0);
+  const size_t i = (size_t)b * a.D + d;
   Run r{n0, a.prev_mean[i], a.prev_var[i] * n0};
   const float* pn = s.rn + (size_t)b * s.S;
-  float *pm = s.rm + (size_t)b * s.S * a.D + (ok ? d : 0), *ps = s.rs + (size_t)b * s.S * a.D + (ok ? d : 0);
+  float *pm = s.rm + (size_t)b * s.S * a.D + d, *ps = s.rs + (size_t)b * s.S * a.D + d;
   constexpr int kB = 8;
   for (int k0 = 0; k0 < s.S; k0 += kB) {
     Run seg[kB];
@@ -119,19 +120,15 @@ __global__ void __launch_bounds__(128) scan_stats_kernel(SegArgs s) {
 #pragma unroll
     for (int u = 0; u < kB; ++u) {
       if (k0 + u < s.S) {
-        if (ok) {
-          pm[(size_t)(k0 + u) * a.D] = r.m;
-          ps[(size_t)(k0 + u) * a.D] = r.s;
-        }
+        pm[(size_t)(k0 + u) * a.D] = r.m;
+        ps[(size_t)(k0 + u) * a.D] = r.s;
         r = combine(r, seg[u]);
       }
     }
   }
-  if (ok) {
-    a.mean_out[i] = r.n > 0.f ? r.m : a.prev_mean[i];
-    a.var_out[i] = r.n > 0.f ? r.s / r.n : a.prev_var[i];
-    if (d == 0) a.count_out[b] = cnt0 + (long long)(r.n - n0 + 0.5f);
-  }
+  a.mean_out[i] = r.n > 0.f ? r.m : a.prev_mean[i];
+  a.var_out[i] = r.n > 0.f ? r.s / r.n : a.prev_var[i];
+  if (d == 0) a.count_out[b] = cnt0 + (long long)(r.n - n0 + 0.5f);
 }
 
 // The statistics a segment starts from.

@@ -499,6 +499,10 @@ static bool pairs_ok(int dtype, const ScanNormArgs& a, long long ysd) {
 
 bool scan_norm_fwd_try(int dtype, const ScanNormArgs& a, long long xsd, long long ysd, cudaStream_t s) {
   if (!rows_ok(dtype, a.x, a.xsb, a.xsl, xsd, a.D) || !pairs_ok(dtype, a, ysd) || a.x == a.y) return false;
+  // (every segment's block reads the incoming statistics, the last one's writes the new ones)
+  const size_t n = (size_t)a.B * a.D;
+  for (const float* out : {a.mean_out, a.var_out})
+    if (overlap(out, a.prev_mean, n) || overlap(out, a.prev_var, n)) return false;
   return dispatch<false>(dtype, a, s);
 }
 

@@ -22,7 +22,7 @@ struct ScanNormArgs {
 };
 
 // Each returns false, having launched nothing, outside its envelope (channels not contiguous, rows that are not
-// whole 16-byte pieces, too many sequences for the grid) or when there is no scratch memory.
+// whole 16-byte pieces, too many sequences for the grid, statistics updated in place) or when there is no scratch memory.
 bool scan_norm_fwd_try(int dtype, const ScanNormArgs& a, long long xsd, long long ysd, cudaStream_t s);
 bool scan_norm_bwd_try(int dtype, const ScanNormArgs& a, long long xsd, long long ysd, long long gsd, cudaStream_t s);
 

@@ -85,3 +85,60 @@ def test_bidirectional_beyond_a_quarter_million(cplx):
         out = (ops.cema_forward if cplx else ops.ema_forward)(
             xg.transpose(1, 2), *cf(*(t.cuda() for t in (alpha, delta, third, gamma))), omega.cuda(), bidirectional=True)
     assert rel_l2(out[0].t(), conv(x, kf)) < 5e-6
+
+
+def _norm_call(form, gen, bsz, length, dim, count):
+    """(run(mean_out, var_out) -> (y, count), prev_mean, prev_var, reference) of a TimestepNorm form of the C interface"""
+    from fairseq_apollo_b200 import _lib, ops
+    from oracle import mega_oracle as O
+    groups = 4 if form == "group" else dim
+    x = torch.randn(bsz, length, dim, generator=gen) * 1.1 + 0.2
+    mask = torch.zeros(bsz, length, dtype=torch.bool)
+    mask[0, 3:length - 4:5] = True
+    mask[-1, length - length // 3:] = True
+    pc = torch.full((bsz,), count)
+    pm, pv = torch.randn(bsz, groups, generator=gen) * 0.3, torch.rand(bsz, groups, generator=gen) + 0.5
+    gamma, beta = torch.rand(dim, generator=gen) + 0.5, torch.randn(dim, generator=gen)
+    if groups == dim:
+        want = O.timestep_norm(x.double(), pc, pm.double(), pv.double(), gamma.double(), beta.double(), mask, acc_dtype=torch.float64)
+    else:
+        want = O.group_timestep_norm(x.double(), pc, pm.double(), pv.double(), gamma.double(), beta.double(), mask, groups,
+                                     acc_dtype=torch.float64)
+    dev = [t.cuda() for t in (x, pc, pm, pv, gamma, beta, mask)]
+    prm = [t.cuda() for t in (torch.rand(dim, 16, generator=gen) * 0.2, torch.rand(dim, 16, generator=gen) * 0.5 + 0.4,
+                              torch.randn(dim, 16, generator=gen), torch.randn(dim, generator=gen))]
+
+    def run(mean_out, var_out):
+        xg, pcg, pmg, pvg, ga, be, mk = dev
+        y, xn, cnt = torch.empty_like(xg), torch.empty_like(xg), torch.empty_like(pcg)
+        s = xg.stride()
+        P = lambda t: t.data_ptr()
+        stream = torch.cuda.current_stream().cuda_stream
+        if form in ("group", "norm"):
+            rc = _lib.lib().mega_timestep_norm_fwd(P(xg), P(y), 0, bsz, length, dim, *s, *s, P(pcg), P(pmg), P(pvg), P(ga), P(be), P(mk),
+                                                   groups, 1e-5, P(cnt), P(mean_out), P(var_out), stream)
+            xn = y
+        else:
+            rc = _lib.lib().mega_tsn_ema_fwd(P(xg), P(y), P(xn), 0, bsz, length, dim, *s, *s, P(pcg), P(pmg), P(pvg), P(ga), P(be), 1e-5,
+                                             P(cnt), P(mean_out), P(var_out), *(P(t) for t in prm), 16, P(mk), None, None, 0, stream)
+        assert rc == 0
+        return xn, cnt
+    return run, dev[2], dev[3], want
+
+
+@pytest.mark.parametrize("form,length,bsz,dim,split", [
+    ("norm", 700, 2, 72, 0),          # several segments of at least 64 steps
+    ("group", 700, 2, 128, 0),        # 128 threads along time, the last ones without steps
+    ("fused", 700, 2, 72, 3),         # a cluster of blocks
+    ("fused", 100, 1, 32, 3),         # one block
+    ("fused", 2200, 64, 96, 3),       # the scan of several launches
+])
+def test_statistics_updated_in_place(form, length, bsz, dim, split, option):
+    """mean_out and var_out may be prev_mean and prev_var."""
+    gen = torch.Generator().manual_seed(length)
+    run, pm, pv, want = _norm_call(form, gen, bsz, length, dim, 5)
+    option(5, split)
+    y, cnt = run(pm, pv)
+    assert rel_l2(y, want[0]) < 1e-5
+    assert torch.equal(cnt.cpu(), want[1])
+    assert rel_l2(pm, want[2]) < 1e-5 and rel_l2(pv, want[3]) < 1e-5
