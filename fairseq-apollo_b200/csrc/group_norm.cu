@@ -164,7 +164,10 @@ __global__ void __launch_bounds__(kScanG* kScanT) group_scan_kernel(const float*
   Run in = prior;
   if (ti > 0) in = combine(prior, part[ti - 1][gi]);
   // second walk, sums about the mean that came in (or the first value when nothing did)
-  float c = in.m, s1 = 0.f, s2 = 0.f, n = in.n;
+  // (the thread's own steps counted from zero: one by one they would be lost on a count beyond 2^24)
+  float c = in.m, s1 = 0.f, s2 = 0.f, seen = 0.f;
+  const float n0 = in.n;
+  float n = n0;
   float mean = in.n > 0.f ? in.m : prior.m, var = in.n > 0.f ? in.s / in.n : var0;
   for (int k = t0; k < t1; k += kFwdB) {
     fetch(k);
@@ -175,7 +178,8 @@ __global__ void __launch_bounds__(kScanG* kScanT) group_scan_kernel(const float*
         const float d = ms[j] - c;
         s1 += d;
         s2 += fmaf(d, d, vs[j]);
-        n += 1.f;
+        seen += 1.f;
+        n = n0 + seen;
         const float inv = 1.f / n, u = s1 * inv;
         mean = c + u;
         var = fmaxf(fmaf(-u, u, (in.s + s2) * inv), 0.f);
@@ -321,7 +325,7 @@ __global__ void __launch_bounds__(kScanG* kScanT) group_bwd_scan_kernel(const fl
   float later = 0.f;
   for (int i = 0; i < ti; ++i) later += cnts[i];
   const float n_end = (float)count[b];
-  const float n_in = n_end - later;   // count after this run's last step
+  const float n_in = n_end - later;   // count after this run's last step (its own steps are counted apart: see the forward)
   auto prev_u = [&](int t) -> float { return t > 0 ? __ldg(cummean + base + (size_t)(t - 1) * G) : prev_mean[(size_t)b * G + g]; };
   constexpr int kBwdB = 4;   // (steps whose loads go out together)
   float lr[kBwdB], le[kBwdB], ls[kBwdB], lb[kBwdB];
@@ -340,20 +344,18 @@ __global__ void __launch_bounds__(kScanG* kScanT) group_bwd_scan_kernel(const fl
   };
   Map m{0.f, 0.f, 0.f, 0.f};
   if (ok) {
-    float n = n_in;
     for (int k = hi - 1; k >= lo; k -= kBwdB) {
       fetch(k);
 #pragma unroll
       for (int j = 0; j < kBwdB; ++j) {
         if (skip[j]) continue;
-        const float rs = lr[j], inv = 1.f / n, e = le[j] * inv;
+        const float rs = lr[j], inv = 1.f / (n_in - m.n), e = le[j] * inv;
         m.sv -= 0.5f * (rs * rs * rs) * ls[j] * inv;
         m.su -= fmaf(e, m.sv, rs * lb[j] * inv);
         m.sw -= e;
-        n -= 1.f;
+        m.n += 1.f;
       }
     }
-    m.n = n_in - n;
   }
   part[ti][gi] = m;
   __syncthreads();
@@ -374,20 +376,20 @@ __global__ void __launch_bounds__(kScanG* kScanT) group_bwd_scan_kernel(const fl
     V = v0 + p.sv;
     U = u0 + p.su + p.sw * v0;
   }
-  float n = n_in;
+  float done = 0.f;
   for (int k = hi - 1; k >= lo; k -= kBwdB) {
     fetch(k);
 #pragma unroll
     for (int j = 0; j < kBwdB; ++j) {
       float ou = 0.f, ov = 0.f;
       if (!skip[j]) {
-        const float rs = lr[j], inv = 1.f / n, e = le[j];
+        const float rs = lr[j], n = n_in - done, inv = 1.f / n, e = le[j];
         V -= 0.5f * (rs * rs * rs) * ls[j] * inv;
         const float h = U - rs * lb[j] * inv;
         ov = V;
         ou = fmaf((n - 1.f) * inv * e, V, h);
         U = fmaf(-e * inv, V, h);
-        n -= 1.f;
+        done += 1.f;
       }
       if (k - j >= lo) {
         const size_t i = base + (size_t)(k - j) * G;

@@ -20,14 +20,16 @@ __device__ __forceinline__ Run combine(Run a, Run b) {
   return {n, fmaf(d, w, a.m), a.s + b.s + d * d * a.n * w};
 }
 
-// The statistics of a walk, advanced by one unmasked input.
+// The statistics of a walk, advanced by one unmasked input.  The walk's own steps are counted from zero: added one by one
+// to a count beyond 2^24 they would be lost.
 struct Running {
-  float c, s1, s2, n, in_s;   // centre, sums about it, count, squared deviations that came in
-  float u;                    // mean - c
+  float c, s1, s2, n0, in_s;   // centre, sums about it, count and squared deviations that came in
+  float seen, n;               // steps of the walk, count
+  float u;                     // mean - c
   __device__ __forceinline__ void start(const Run& r) {
     c = r.m;
-    s1 = s2 = u = 0.f;
-    n = r.n;
+    s1 = s2 = u = seen = 0.f;
+    n0 = n = r.n;
     in_s = r.s;
   }
   // returns x - c; inv = 1 / n, r = 1 / sqrt(var + eps)
@@ -36,7 +38,8 @@ struct Running {
     const float d = x - c;
     s1 += d;
     s2 = fmaf(d, d, s2);
-    n += 1.f;
+    seen += 1.f;
+    n = n0 + seen;
     inv = rcp_approx(n);
     u = s1 * inv;
     r = rsqrt_approx(fmaxf(fmaf(-u, u, (in_s + s2) * inv), 0.f) + eps);

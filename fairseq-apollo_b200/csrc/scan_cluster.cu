@@ -236,14 +236,21 @@ __global__ void __launch_bounds__(kW * 32, kC ? 1 : 2) scan_cluster_kernel(Clust
 #pragma unroll
     for (int k = 0; k < 7; ++k)
       if (k < rank) r = combine(r, before[k]);
-    for (int k = 0; k < warp; ++k)
+    float seen = 0.f;   // unmasked steps of the call before the segment (a float count that starts beyond 2^24 would round them)
+#pragma unroll
+    for (int k = 0; k < 7; ++k)
+      if (k < rank) seen += before[k].n;
+    for (int k = 0; k < warp; ++k) {
       r = combine(r, Run{run[(k * 3) * 32 + lane], run[(k * 3 + 1) * 32 + lane], run[(k * 3 + 2) * 32 + lane]});
+      seen += run[(k * 3) * 32 + lane];
+    }
+    r.n = (float)cnt0 + seen;
     rs.start(r);
     if (rank == ranks - 1 && warp == kW - 1 && ok) {
       r = combine(r, Run{cnt, c, sq});
       a.mean_out[i] = r.n > 0.f ? r.m : a.prev_mean[i];
       a.var_out[i] = r.n > 0.f ? r.s / r.n : a.prev_var[i];
-      if (d == 0) a.count_out[b] = cnt0 + (long long)(r.n - (float)cnt0 + 0.5f);
+      if (d == 0) a.count_out[b] = cnt0 + (long long)(seen + cnt);
     }
   }
 

@@ -107,6 +107,7 @@ __global__ void __launch_bounds__(128) scan_stats_kernel(SegArgs s) {
   const float n0 = (float)cnt0;
   const size_t i = (size_t)b * a.D + d;
   Run r{n0, a.prev_mean[i], a.prev_var[i] * n0};
+  long long seen = 0;   // unmasked steps of the call (a float count that starts beyond 2^24 would round them)
   const float* pn = s.rn + (size_t)b * s.S;
   float *pm = s.rm + (size_t)b * s.S * a.D + d, *ps = s.rs + (size_t)b * s.S * a.D + d;
   constexpr int kB = 8;
@@ -123,18 +124,20 @@ __global__ void __launch_bounds__(128) scan_stats_kernel(SegArgs s) {
         pm[(size_t)(k0 + u) * a.D] = r.m;
         ps[(size_t)(k0 + u) * a.D] = r.s;
         r = combine(r, seg[u]);
+        seen += (long long)seg[u].n;
       }
     }
   }
   a.mean_out[i] = r.n > 0.f ? r.m : a.prev_mean[i];
   a.var_out[i] = r.n > 0.f ? r.s / r.n : a.prev_var[i];
-  if (d == 0) a.count_out[b] = cnt0 + (long long)(r.n - n0 + 0.5f);
+  if (d == 0) a.count_out[b] = cnt0 + seen;
 }
 
 // The statistics a segment starts from.
 __device__ __forceinline__ Run stats_of(const SegArgs& s, int b, int seg, int d) {
-  float n = (float)s.a.prev_count[b];
-  for (int k = 0; k < seg; ++k) n += __ldg(s.rn + (size_t)b * s.S + k);
+  float seen = 0.f;
+  for (int k = 0; k < seg; ++k) seen += __ldg(s.rn + (size_t)b * s.S + k);
+  const float n = (float)s.a.prev_count[b] + seen;
   const size_t i = ((size_t)b * s.S + seg) * s.a.D + d;
   return Run{n, __ldg(s.rm + i), __ldg(s.rs + i)};
 }

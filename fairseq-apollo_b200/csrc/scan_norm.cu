@@ -90,6 +90,7 @@ __device__ __forceinline__ f32x2 neg2(f32x2 v) { return mul2(v, both(-1.f)); }
 // What a segment starts from: the prior and the segments before it (for two channels).
 __device__ __forceinline__ void pair_before(const SegNorm& s, const PairLane& l, Run (&r)[2]) {
   const float n0 = (float)s.a.prev_count[l.b];
+  float seen = 0.f;   // (unmasked steps of the call: a float count that starts beyond 2^24 would round them)
   const size_t i = (size_t)l.b * s.a.D + l.dc;
   const float* pn = s.rn + (size_t)l.b * s.S;
   const size_t at = (size_t)l.b * s.S * s.a.D + l.dc;
@@ -102,17 +103,20 @@ __device__ __forceinline__ void pair_before(const SegNorm& s, const PairLane& l,
     const float2 q = __ldg(reinterpret_cast<const float2*>(s.rs + at + (size_t)k * s.a.D));
     r[0] = combine(r[0], Run{n, m.x, q.x});
     r[1] = combine(r[1], Run{n, m.y, q.y});
+    seen += n;
   }
+  r[0].n = r[1].n = n0 + seen;
 }
 
 // Running (norm_run.cuh) for two channels.
 struct PairRunning {
   f32x2 c, s1, s2, in_s, u;
-  float n;
+  float n0, seen, n;
   __device__ __forceinline__ void start(const Run (&r)[2]) {
     c = pack2(r[0].m, r[1].m);
     s1 = s2 = u = both(0.f);
-    n = r[0].n;
+    n0 = n = r[0].n;
+    seen = 0.f;
     in_s = pack2(r[0].s, r[1].s);
   }
   // returns x - c; inv = 1 / n, r = 1 / sqrt(var + eps)
@@ -121,7 +125,8 @@ struct PairRunning {
     const f32x2 d = sub2(x, c);
     s1 = add2(s1, d);
     s2 = fma2(d, d, s2);
-    n += 1.f;
+    seen += 1.f;
+    n = n0 + seen;
     inv = both(rcp_approx(n));
     u = mul2(s1, inv);
     const f32x2 v = fma2(neg2(u), u, mul2(add2(in_s, s2), inv));
@@ -173,7 +178,11 @@ __global__ void __launch_bounds__(kWarps * 32) norm_emit_kernel(SegNorm s) {
       a.mean_out[i] = any ? c[k] + u : a.prev_mean[i];
       a.var_out[i] = any ? fmaxf(fmaf(-u, u, (q[k] + s2[k]) * inv), 0.f) : a.prev_var[i];
     }
-    if (l.d == 0) a.count_out[l.b] = a.prev_count[l.b] + (long long)(st.n - (float)a.prev_count[l.b] + 0.5f);
+    if (l.d == 0) {
+      long long total = a.prev_count[l.b];
+      for (int k = 0; k < s.S; ++k) total += (long long)__ldg(s.rn + (size_t)l.b * s.S + k);
+      a.count_out[l.b] = total;
+    }
   }
 }
 
@@ -244,8 +253,9 @@ __global__ void __launch_bounds__(kWarps * 32) norm_bwd_emit_kernel(SegNorm s) {
   const float eps = a.eps;
   const size_t row = (size_t)l.b * a.D + l.dc;
   const float n0 = (float)a.prev_count[l.b];
-  float n_end = n0;
-  for (int k = 0; k < s.S; ++k) n_end += __ldg(s.rn + (size_t)l.b * s.S + k);
+  float total = 0.f;   // unmasked steps of the call
+  for (int k = 0; k < s.S; ++k) total += __ldg(s.rn + (size_t)l.b * s.S + k);
+  const float n_end = n0 + total;
   const f32x2 inv_end = both(n_end > 0.f ? 1.f / n_end : 0.f);
   f32x2 V = a.dvar ? mul2(pack2(a.dvar[row], a.dvar[row + 1]), inv_end) : both(0.f);
   f32x2 U = a.dmean ? mul2(pack2(a.dmean[row], a.dmean[row + 1]), inv_end) : both(0.f);
@@ -259,7 +269,7 @@ __global__ void __launch_bounds__(kWarps * 32) norm_bwd_emit_kernel(SegNorm s) {
   f32x2 W = fma2(map(s.sw, l.seg), V, add2(U, map(s.su, l.seg)));   // U as it leaves the segment's first step
   V = add2(V, map(s.sv, l.seg));
   if (l.seg == 0 && l.ok) {
-    const bool any = n_end > n0;   // (no unmasked step: the incoming gradients pass through)
+    const bool any = total > 0.f;   // (no unmasked step: the incoming gradients pass through)
     float wv[2], vv[2];
     unpack2(W, wv[0], wv[1]);
     unpack2(V, vv[0], vv[1]);

@@ -142,3 +142,35 @@ def test_statistics_updated_in_place(form, length, bsz, dim, split, option):
     assert rel_l2(y, want[0]) < 1e-5
     assert torch.equal(cnt.cpu(), want[1])
     assert rel_l2(pm, want[2]) < 1e-5 and rel_l2(pv, want[3]) < 1e-5
+
+
+@pytest.mark.parametrize("form,length,bsz,dim,split", [
+    ("norm", 700, 2, 72, 0), ("group", 700, 2, 128, 0), ("fused", 700, 2, 72, 3), ("fused", 1, 1, 32, 3), ("fused", 2200, 64, 96, 3),
+    ("norm", 1, 2, 64, 0),
+])
+@pytest.mark.parametrize("count", [2 ** 24 + 1, 2 ** 31 + 5])
+def test_counts_stay_whole_numbers(form, length, bsz, dim, split, count, option):
+    gen = torch.Generator().manual_seed(length)
+    run, pm, pv, want = _norm_call(form, gen, bsz, length, dim, count)
+    option(5, split)
+    mean, var = torch.empty_like(pm), torch.empty_like(pv)
+    y, cnt = run(mean, var)
+    assert torch.equal(cnt.cpu(), want[1])
+    assert rel_l2(y, want[0]) < 1e-5 and rel_l2(mean, want[2]) < 1e-5 and rel_l2(var, want[3]) < 1e-5
+
+
+@pytest.mark.parametrize("groups", [None, 4])
+def test_prior_gradients_of_a_long_stream(groups):
+    """Backward with an incoming count of 2^27: one more step has to be seen.  dprior = n0 / n times the output's share."""
+    import fairseq_apollo_b200 as M
+    torch.manual_seed(1)
+    dim = 64
+    norm = M.TimestepNorm(dim, num_groups=groups, prior_count=2 ** 27).cuda()
+    x = torch.randn(2, 3, dim, device="cuda")
+    norm(x).sum().backward()
+    # mean and variance stay at the prior's: dy/dmean = -rstd per channel, dy/dlogv = -(x - mean) rstd / 2 (prior variance 1)
+    per = dim // (groups or dim)
+    want = torch.full((dim // per,), -6.0 * per, device="cuda")
+    assert rel_l2(norm.prior_mean.grad, want) < 1e-4
+    dv = (-0.5 * x.sum((0, 1))).view(-1, per).sum(-1)
+    assert rel_l2(norm.prior_logv.grad, dv) < 1e-4
