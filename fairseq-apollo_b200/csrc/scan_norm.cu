@@ -345,9 +345,9 @@ __global__ void __launch_bounds__(kWarps * 32) sqn_bwd_sums_kernel(SegNorm s) {
   float ds = 0.f, db = 0.f;
   walk<T, 1, true, kMask>(x, a.xsl, g, a.gsl, m, l.t0, l.t1, l.left, rings + (size_t)l.warp * 2 * kRing * kTileBytes,
                           [&](int, float xv, float gv, bool pad) {
-                            const float v = kMask && pad ? 0.f : gv;
-                            ds = fmaf(v, xv - u, ds);
-                            db += v;
+                            if (kMask && pad) return;   // (whatever stands there, NaN included)
+                            ds = fmaf(gv, xv - u, ds);
+                            db += gv;
                           });
   if (l.ok) {
     const size_t i = ((size_t)l.b * s.S + l.seg) * a.D + l.d;

@@ -1,0 +1,26 @@
+"""Infinities and NaN: where they were an output's own business, they still are."""
+import pytest
+import torch
+
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_sequence_norm_backward_ignores_padding(dtype):
+    """(B, L, D): what stands at padded positions takes no part, NaN included."""
+    import fairseq_apollo_b200 as M
+    torch.manual_seed(2)
+    norm = M.SequenceNorm(64).cuda()
+    x = torch.randn(2, 200, 64, device="cuda").to(dtype)
+    mask = torch.zeros(2, 200, dtype=torch.bool, device="cuda")
+    mask[1, 150:] = True
+    grads = []
+    for fill in (0.0, float("nan"), float("inf")):
+        norm.zero_grad()
+        xx = x.masked_fill(mask.unsqueeze(-1), fill).requires_grad_(True)
+        norm(xx, mask, length_last=False).backward(torch.ones_like(x))
+        grads.append((xx.grad, norm.weight.grad.clone(), norm.bias.grad.clone()))
+    for other in grads[1:]:
+        for a, b in zip(grads[0], other):
+            torch.testing.assert_close(a, b, rtol=1e-5, atol=1e-5)
