@@ -129,6 +129,8 @@ struct Elem<__half> {
   static __device__ __forceinline__ void st(__half* p, float v) { *p = __float2half_rn(v); }
 };
 
+// v, 0 where rounding took it below; NaN stays NaN (fmaxf would drop it)
+__device__ __forceinline__ float not_negative(float v) { return v < 0.f ? 0.f : v; }
 // MUFU approximations (about 1 ulp): no slow path, no subroutine call in a serial loop
 __device__ __forceinline__ float rcp_approx(float v) {
   float r;

@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kScanG* kScanT) group_scan_kernel(const float*
         n += 1.f;
       }
     }
-    if (n > 0.f) r = {n, c + s1 / n, fmaxf(s2 - s1 * s1 / n, 0.f)};
+    if (n > 0.f) r = {n, c + s1 / n, not_negative(s2 - s1 * s1 / n)};
   }
   part[ti][gi] = r;
   __syncthreads();
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(kScanG* kScanT) group_scan_kernel(const float*
         n = n0 + seen;
         const float inv = 1.f / n, u = s1 * inv;
         mean = c + u;
-        var = fmaxf(fmaf(-u, u, (in.s + s2) * inv), 0.f);
+        var = not_negative(fmaf(-u, u, (in.s + s2) * inv));
       }
       if (k + j < t1) {
         const size_t i = base + (size_t)(k + j) * G;

@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(kWarps * 32) norm_moments_kernel(MomentArgs s)
   const size_t i = ((size_t)b * s.S + seg) * s.D + d;
   if (d < s.D) {
     s.rm[i] = fmaf(s1, inv, c);
-    s.rs[i] = fmaxf(fmaf(-s1 * inv, s1, s2), 0.f);
+    s.rs[i] = not_negative(fmaf(-s1 * inv, s1, s2));
   }
   if (blockIdx.x == 0 && lane == 0) s.rn[(size_t)b * s.S + seg] = n;
 }

@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(kWarps * 32) norm_emit_kernel(SegNorm s) {
       const size_t i = (size_t)l.b * a.D + l.d + k;
       const float u = s1[k] * inv;
       a.mean_out[i] = any ? c[k] + u : a.prev_mean[i];
-      a.var_out[i] = any ? fmaxf(fmaf(-u, u, (q[k] + s2[k]) * inv), 0.f) : a.prev_var[i];
+      a.var_out[i] = any ? not_negative(fmaf(-u, u, (q[k] + s2[k]) * inv)) : a.prev_var[i];
     }
     if (l.d == 0) {
       long long total = a.prev_count[l.b];

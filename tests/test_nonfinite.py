@@ -2,7 +2,6 @@
 import pytest
 import torch
 
-
 pytestmark = pytest.mark.gpu
 
 
@@ -24,3 +23,14 @@ def test_sequence_norm_backward_ignores_padding(dtype):
     for other in grads[1:]:
         for a, b in zip(grads[0], other):
             torch.testing.assert_close(a, b, rtol=1e-5, atol=1e-5)
+
+
+def test_running_variance_of_nan_is_nan():
+    from fairseq_apollo_b200 import ops
+    x = torch.randn(1, 300, 64, device="cuda")
+    x[0, 40, 5] = float("nan")
+    one = torch.ones(64, device="cuda")
+    _, _, mean, var = ops.timestep_norm_fwd(x, torch.full((1,), 2, device="cuda"), torch.zeros(1, 64, device="cuda"),
+                                            torch.ones(1, 64, device="cuda"), one, one)
+    assert mean[0, 5].isnan() and var[0, 5].isnan()
+    assert var.isnan().sum() == 1 and mean.isnan().sum() == 1
