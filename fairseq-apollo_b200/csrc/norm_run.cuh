@@ -48,6 +48,8 @@ struct Running {
 };
 
 // The moments of every segment of T steps: unmasked steps rn (B, S), mean rm and squared deviations rs (B, S, D).
+// Sums about the mean of the first 32 steps, 32 steps at a time: about the segment's first value, and one step after the
+// other, the variance of 5000 steps was 1.9e-6 off its own size, further than a step-by-step Welford update (1.2e-6).
 struct MomentArgs {
   const void* x;
   long long xsb, xsl;
@@ -65,24 +67,30 @@ __global__ void __launch_bounds__(kWarps * 32) norm_moments_kernel(MomentArgs s)
   const int t0 = min(s.L, seg * s.T), t1 = min(s.L, t0 + s.T);
   const T* x = reinterpret_cast<const T*>(s.x) + b * s.xsb + d0;
   const unsigned char* m = kMask ? s.mask + (size_t)b * s.L : nullptr;
-  float c = 0.f, s1 = 0.f, s2 = 0.f, n = 0.f;
+  float c = 0.f, s1 = 0.f, s2 = 0.f, n = 0.f, p1 = 0.f, p2 = 0.f;   // p1, p2: of the present 32 steps
   walk<T, 1, false, kMask>(x, s.xsl, x, 0, m, t0, t1, s.D - d0, rings + (size_t)warp * kRing * kTileBytes,
                            [&](int k, float xv, float, bool pad) {
-                             if (kMask) {
-                               if (!pad) {
-                                 if (n == 0.f) c = xv;
-                                 const float d = xv - c;
-                                 s1 += d;
-                                 s2 = fmaf(d, d, s2);
-                                 n += 1.f;
-                               }
-                             } else {
-                               if (k == 0) c = xv;
+                             if (!(kMask && pad)) {
+                               if (kMask ? n == 0.f : k == 0) c = xv;
                                const float d = xv - c;
-                               s1 += d;
-                               s2 = fmaf(d, d, s2);
+                               p1 += d;
+                               p2 = fmaf(d, d, p2);
+                               if (kMask) n += 1.f;
+                             }
+                             if ((k & 31) == 31) {
+                               if (k == 31) {   // (from here on about their mean)
+                                 const float n32 = kMask ? n : 32.f, to = n32 > 0.f ? c + p1 / n32 : c, e = to - c;
+                                 p2 = fmaf(e, fmaf(n32, e, -2.f * p1), p2);
+                                 p1 = fmaf(-n32, e, p1);
+                                 c = to;
+                               }
+                               s1 += p1;
+                               s2 += p2;
+                               p1 = p2 = 0.f;
                              }
                            });
+  s1 += p1;
+  s2 += p2;
   if (!kMask) n = (float)(t1 - t0);
   const float inv = n > 0.f ? 1.f / n : 0.f;
   const int d = d0 + lane;
