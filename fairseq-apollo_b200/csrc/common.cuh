@@ -144,6 +144,27 @@ __device__ __forceinline__ float rsqrt_approx(float v) {
 }
 __device__ __forceinline__ float sigmoidf_(float v) { return 1.0f / (1.0f + __expf(-v)); }
 __device__ __forceinline__ float siluf_(float v) { return v / (1.0f + __expf(-v)); }
+// sigmoid(v) to a few units of its last place, however nearly closed the gate: 0.5 + 0.5 tanh.approx(v / 2) is good to 2^-12
+// of 1, which at v = -8 is most of the value.  fp32 activations take the full-range exponential and division, 16-bit ones
+// two MUFU operations.
+template <typename T>
+__device__ __forceinline__ float exp_of(float v) {
+  return sizeof(T) == 4 ? expf(v) : __expf(v);
+}
+template <typename T>
+__device__ __forceinline__ float sigmoid_of(float v) {
+  const float e = 1.f + exp_of<T>(-v);
+  return sizeof(T) == 4 ? 1.f / e : rcp_approx(e);
+}
+// sigmoid(v) and sigmoid(-v)
+struct Gate {
+  float s, c;
+};
+template <typename T>
+__device__ __forceinline__ Gate gate_of(float v) {
+  const float e = exp_of<T>(-fabsf(v)), r = sizeof(T) == 4 ? 1.f / (1.f + e) : rcp_approx(1.f + e), l = e * r;
+  return v >= 0.f ? Gate{r, l} : Gate{l, r};
+}
 // silu(v) = v * sigmoid(v) = h + h * tanh(h), h = v / 2: one MUFU op (tanh.approx, relative error
 // about 2^-11) and two FP32 ops.  For kernels whose output is rounded to bf16 / fp16 anyway.
 __device__ __forceinline__ float silu_tanh(float v) {

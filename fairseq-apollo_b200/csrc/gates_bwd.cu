@@ -34,17 +34,7 @@ struct Row16 {
   }
 };
 
-// sigmoid; 16-bit types from one tanh.approx (relative error ~2^-11, below the rounding of the results)
-template <typename T>
-__device__ __forceinline__ float sig(float v) {
-  if (sizeof(T) == 2) {
-    float t;
-    asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(0.5f * v));
-    return fmaf(0.5f, t, 0.5f);
-  }
-  return sigmoidf_(v);
-}
-// d silu(v) / dv given s = sigmoid(v)
+// d silu(v) / dv given s = sigmoid(v)  (1 - s is small only where the term it is in is small beside s)
 __device__ __forceinline__ float dsilu(float v, float s) { return fmaf(v * s, 1.f - s, s); }
 
 // column sums of a block (32 vectors of columns x 8 rows of threads) into `out`
@@ -93,7 +83,7 @@ __global__ void __launch_bounds__(256) gate_bwd_kernel(GateBwd p) {
     if (OP == 0) {
 #pragma unroll
       for (int k = 0; k < kN; ++k) {
-        o0[k] = g[k] * dsilu(a[k], sig<T>(a[k]));
+        o0[k] = g[k] * dsilu(a[k], sigmoid_of<T>(a[k]));
         s0[k] += o0[k];
       }
     } else if (OP == 1) {
@@ -101,7 +91,7 @@ __global__ void __launch_bounds__(256) gate_bwd_kernel(GateBwd p) {
       Row16<T>::load(reinterpret_cast<const T*>(p.b) + r * p.ldb + col, b);
 #pragma unroll
       for (int k = 0; k < kN; ++k) {
-        const float s = sig<T>(b[k]);
+        const float s = sigmoid_of<T>(b[k]);
         o0[k] = g[k] * b[k] * s;
         o1[k] = g[k] * a[k] * dsilu(b[k], s);
         s0[k] += o1[k];
@@ -114,10 +104,12 @@ __global__ void __launch_bounds__(256) gate_bwd_kernel(GateBwd p) {
       Row16<T>::load(reinterpret_cast<const T*>(p.d) + r * p.ldd + col, d);
 #pragma unroll
       for (int k = 0; k < kN; ++k) {
-        const float u = sig<T>(b[k]), t = c[k] + d[k], s = sig<T>(t);
-        o0[k] = fmaf(-u, g[k], g[k]);
-        o1[k] = g[k] * (t * s - a[k]) * u * (1.f - u);
-        o2[k] = g[k] * u * dsilu(t, s);
+        const float t = c[k] + d[k];
+        const Gate u = gate_of<T>(b[k]);
+        const float s = sigmoid_of<T>(t);
+        o0[k] = g[k] * u.c;
+        o1[k] = g[k] * fmaf(t, s, -a[k]) * u.s * u.c;
+        o2[k] = g[k] * u.s * dsilu(t, s);
         s0[k] += o1[k];
         s1[k] += o2[k];
       }
@@ -310,7 +302,7 @@ __global__ void __launch_bounds__(256) bias_softmax_warp_kernel(const T* x, T* y
   for (int j = 0; j < kN; ++j)
 #pragma unroll
     for (int k = 0; k < kV; ++k) {
-      v[j][k] = m == -INFINITY ? 0.f : __expf(v[j][k] - m);
+      v[j][k] = m == -INFINITY ? 0.f : exp_of<T>(v[j][k] - m);
       s += v[j][k];
     }
 #pragma unroll
@@ -362,7 +354,7 @@ __global__ void __launch_bounds__(128) bias_softmax_kernel(const T* x, T* y, con
   __syncthreads();
   float s = 0.f;
   for (int c = tid; c < cols; c += 128) {
-    const float e = m == -INFINITY ? 0.f : __expf(row[c] - m);
+    const float e = m == -INFINITY ? 0.f : exp_of<T>(row[c] - m);
     row[c] = e;
     s += e;
   }

@@ -338,13 +338,14 @@ __global__ void gate_kernel(const T* a, long long lda, const T* b, long long ldb
     if (OP == 0) {  // silu(a [+ b])
       float v = Elem<T>::ld(a + r * lda + col);
       if (b) v += Elem<T>::ld(b + r * ldb + col);
-      out = siluf_(v);
+      out = v * sigmoid_of<T>(v);
     } else if (OP == 1) {  // a * silu(b)
-      out = Elem<T>::ld(a + r * lda + col) * siluf_(Elem<T>::ld(b + r * ldb + col));
+      const float v = Elem<T>::ld(b + r * ldb + col);
+      out = Elem<T>::ld(a + r * lda + col) * (v * sigmoid_of<T>(v));
     } else {  // a = residual, b = u, c = hx, d = h_lin
       const float res = Elem<T>::ld(a + r * lda + col);
-      const float u = sigmoidf_(Elem<T>::ld(b + r * ldb + col));
-      const float h = siluf_(Elem<T>::ld(c + r * ldc + col) + Elem<T>::ld(d + r * ldd + col));
+      const float u = sigmoid_of<T>(Elem<T>::ld(b + r * ldb + col));
+      const float v = Elem<T>::ld(c + r * ldc + col) + Elem<T>::ld(d + r * ldd + col), h = v * sigmoid_of<T>(v);
       out = fmaf(u, h - res, res);
     }
     Elem<T>::st(y + r * ldy + col, out);
@@ -384,30 +385,20 @@ __global__ void __launch_bounds__(256) gate_vec_kernel(const T* a, long long lda
             *fc = reinterpret_cast<const T*>(&vc[OP == 2 ? u : 0]), *fd = reinterpret_cast<const T*>(&vd[OP == 2 ? u : 0]);
     uint4 out;
     T* o = reinterpret_cast<T*>(&out);
-    // 16-bit outputs: SiLU and the sigmoid from one tanh.approx each (relative error ~2^-11, below
-    // the rounding of the output); fp32 keeps the exponential forms
-    constexpr bool kFast = sizeof(T) == 2;
 #pragma unroll
     for (int k = 0; k < kN; ++k) {
       const float x = Elem<T>::ld_shared(fa + k);
       if (OP == 0) {  // silu(a [+ b])
         const float v = b != nullptr ? x + Elem<T>::ld_shared(fb + k) : x;
-        Elem<T>::st(o + k, kFast ? silu_tanh(v) : siluf_(v));
+        Elem<T>::st(o + k, v * sigmoid_of<T>(v));
       } else if (OP == 1) {  // a * silu(b)
         const float v = Elem<T>::ld_shared(fb + k);
-        Elem<T>::st(o + k, x * (kFast ? silu_tanh(v) : siluf_(v)));
+        Elem<T>::st(o + k, x * (v * sigmoid_of<T>(v)));
       } else {  // a = residual, b = u, c = hx, d = h_lin
         const float v = Elem<T>::ld_shared(fb + k);
-        float g;
-        if (kFast) {
-          float t;
-          asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(0.5f * v));
-          g = fmaf(0.5f, t, 0.5f);
-        } else {
-          g = sigmoidf_(v);
-        }
+        const float g = sigmoid_of<T>(v);
         const float hs = Elem<T>::ld_shared(fc + k) + Elem<T>::ld_shared(fd + k);
-        const float h = kFast ? silu_tanh(hs) : siluf_(hs);
+        const float h = hs * sigmoid_of<T>(hs);
         Elem<T>::st(o + k, fmaf(g, h - x, x));
       }
     }
