@@ -40,7 +40,8 @@ double fused_us(int dtype, const StreamArgs& a, bool want_xn) {
     const double near = fixed + longer(chain, rate, L, n);
     return near > far ? near : far;
   }
-  return a.cplx ? 8.0 + longer(171.0, 168e3, L, n) : 6.0 + longer(122.0, want_xn ? 160e3 : 260e3, L, n);
+  // (complex: 254 ns a position with a state, which prompts of 700 to 4999 positions show alike)
+  return a.cplx ? 8.0 + longer(a.h_in || a.h_out ? 254.0 : 171.0, 168e3, L, n) : 6.0 + longer(122.0, want_xn ? 160e3 : 260e3, L, n);
 }
 
 // TimestepNorm, then the tensor-core kernel alone: where the fused call would run on it too (both round the normalised
