@@ -50,6 +50,15 @@ void on_cuda(const Tensor& t, const Ts&... rest) {
   on_cuda(rest...);
 }
 
+// The library takes pointers: what it reads behind one has to be there.
+void expect(bool ok, const char* what) {
+  if (!ok) throw py::value_error(what);
+}
+void expect_numel(const Tensor& t, int64_t n, const char* what) {
+  if (t.defined() && t.numel() != n)
+    throw py::value_error(std::string(what) + " has " + std::to_string(t.numel()) + " values, not " + std::to_string(n));
+}
+
 // device of the call and its current stream
 struct Where {
   c10::cuda::CUDAGuard guard;
@@ -142,8 +151,29 @@ struct Coeffs {
   Tensor p, q, g;
 };
 
+void check_rows(int64_t rows, int64_t dim, bool bidir) {
+  if (rows != (bidir ? 2 * dim : dim))
+    throw py::value_error("coefficient rows " + std::to_string(rows) + " do not match embed_dim " + std::to_string(dim));
+}
+// p (K, N); q, gamma (K, N), complex ones interleaved; omega (D); a state (B, D, N)
+void check_coeffs(const Tensor& p, const Tensor& q, const Tensor& g, const Tensor& omega, const Tensor& h, bool cplx, int64_t bsz,
+                  int64_t dim, bool bidir) {
+  expect(p.dim() >= 2, "coefficients must be (rows, ndim)");
+  check_rows(p.size(0), dim, bidir);
+  const int64_t m = cplx ? 2 : 1, n = p.size(1);
+  expect_numel(p, p.size(0) * n, "p");
+  expect_numel(q, p.numel() * m, "q");
+  expect_numel(g, p.numel() * m, "gamma");
+  expect_numel(omega, dim, "omega");
+  expect_numel(h, bsz * dim * n * m, "the state");
+}
+
 Coeffs coeffs(const Tensor& alpha, const Tensor& delta, const Tensor& third, const Tensor& gamma, bool cplx, const Where& w) {
   const int64_t k = alpha.size(0), n = alpha.size(1);
+  expect_numel(alpha, k * n, "alpha");
+  expect_numel(delta, k * n, "delta");
+  expect_numel(third, cplx ? k : k * n, cplx ? "theta" : "beta");
+  expect_numel(gamma, cplx ? 2 * k * n : k * n, "gamma");
   const auto st = alpha.scalar_type();
   auto prep = [&](const Tensor& t) { return (t.scalar_type() == st ? t.detach() : t.detach().to(st)).contiguous(); };
   const Tensor a = prep(alpha), d = prep(delta), t = prep(third), g = prep(gamma);
@@ -181,11 +211,11 @@ std::tuple<Tensor, OptTensor> ema_forward(const Tensor& x, const Tensor& p_, con
   const int64_t bsz = x.size(0), dim = x.size(1);
   const Tensor p = f32c(p_), q = cplx ? c64(q_) : f32c(q_), g = cplx ? c64(g_) : f32c(g_), omega = f32c(omega_);
   const int64_t n = p.size(1);
-  if (p.size(0) != ((flags & MEGA_EMA_BIDIRECTIONAL) ? 2 * dim : dim))
-    throw py::value_error("coefficient rows " + std::to_string(p.size(0)) + " do not match embed_dim " + std::to_string(dim));
   const Tensor mask = mask_u8(given(mask_), bsz, x.size(2));
   const Tensor h_in = cplx ? c64(given(h_in_)) : f32c(given(h_in_));
+  check_coeffs(p, q, g, omega, h_in, cplx, bsz, dim, flags & MEGA_EMA_BIDIRECTIONAL);
   const Tensor y = out_.has_value() ? *out_ : like(x);
+  expect(y.sizes() == x.sizes() && y.scalar_type() == x.scalar_type(), "out must be like x");
   Tensor h_out = want_state ? (cplx ? floats({bsz, dim, n, 2}, x) : floats({bsz, dim, n}, x)) : Tensor();
   run_ema(x, y, p, q, g, omega, mask, h_in, h_out, (unsigned)flags, (int)trunc, cplx, w);
   if (!want_state) return {y, std::nullopt};
@@ -206,7 +236,10 @@ class EmaFn : public torch::autograd::Function<EmaFn> {
   static Tensor forward(AutogradContext* ctx, Tensor x_, Tensor alpha, Tensor delta, Tensor third, Tensor gamma, Tensor omega,
                         OptTensor mask_, int64_t flags, int64_t trunc, bool cplx, bool silu, bool chan) {
     const Tensor x = chan ? x_.transpose(1, 2) : x_;
-    on_cuda(x, alpha, omega, given(mask_));
+    on_cuda(x, alpha, delta, third, gamma, omega, given(mask_));
+    expect(x.dim() == 3 && alpha.dim() >= 2, "x must have three dimensions, alpha (rows, ndim, 1)");
+    check_rows(alpha.size(0), x.size(1), flags & MEGA_EMA_BIDIRECTIONAL);
+    expect_numel(omega, x.size(1), "omega");
     const Where w(x);
     const Tensor mask = mask_u8(given(mask_), x.size(0), x.size(2));
     const Coeffs c = coeffs(alpha, delta, third, gamma, cplx, w);
@@ -315,6 +348,11 @@ struct NormParams {
 NormParams prepare(const Tensor& weight, const Tensor& bias, const Tensor& pc, const Tensor& pm, const Tensor& pl, int64_t bsz,
                    const Where& w) {
   const int64_t d = weight.size(0), g = pm.defined() ? pm.size(0) : 0;
+  expect_numel(weight, d, "weight");
+  expect_numel(bias, d, "bias");
+  expect_numel(pm, g, "prior_mean");
+  if (pm.defined()) expect_numel(pl, g, "prior_logv");
+  expect(g <= d, "more prior means than features");
   const Tensor b = bias.scalar_type() == weight.scalar_type() ? bias : bias.detach().to(weight.scalar_type());
   Tensor m = pm, l = pl;
   if (g && m.scalar_type() != weight.scalar_type()) {
@@ -338,7 +376,7 @@ NormParams prepare(const Tensor& weight, const Tensor& bias, const Tensor& pc, c
 
 py::tuple norm_prepare(const Tensor& weight, const Tensor& bias, const OptTensor& pc, const OptTensor& pm, const OptTensor& pl,
                        int64_t bsz) {
-  on_cuda(weight, bias, given(pm));
+  on_cuda(weight, bias, given(pc), given(pm), given(pl));
   const Where w(weight);
   const NormParams r = prepare(weight, bias, given(pc), given(pm), given(pl), bsz, w);
   if (!pm.has_value()) return py::make_tuple(r.gamma, r.beta);
@@ -384,7 +422,11 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> timestep_norm_fwd(const Tensor& x, co
   if (pm.dim() != 2 || pm.size(0) != bsz || pm.size(1) != g || pv.sizes() != pm.sizes())
     throw py::value_error("prev_mean/prev_var must be (batch, groups) = (" + std::to_string(bsz) + ", " + std::to_string(g) + ")");
   const Tensor mask = mask_u8(given(mask_), bsz, length);
+  expect_numel(pc, bsz, "prev_count");
+  expect_numel(gamma, dim, "gamma");
+  expect_numel(beta, dim, "beta");
   const Tensor y = out_.has_value() ? *out_ : like(x);
+  expect(y.sizes() == x.sizes() && y.scalar_type() == x.scalar_type(), "out must be like x");
   Tensor count = counts(bsz, x), st = floats({2, bsz, g}, x);
   Tensor mean = st.select(0, 0), var = st.select(0, 1);
   check(mega_timestep_norm_fwd(x.data_ptr(), y.data_ptr(), dtype_of(x), (int)bsz, (int)length, (int)dim, STRIDES3(x), STRIDES3(y),
@@ -397,9 +439,11 @@ class TsnFn : public torch::autograd::Function<TsnFn> {
  public:
   static Tensor forward(AutogradContext* ctx, Tensor x, Tensor pcount, Tensor pmean, Tensor plogv, Tensor weight, Tensor bias,
                         OptTensor mask_, int64_t groups, double eps) {
-    on_cuda(x, pmean, weight, given(mask_));
+    on_cuda(x, pcount, pmean, plogv, weight, bias, given(mask_));
     const Where w(x);
     const int64_t bsz = x.size(0), length = x.size(1), dim = x.size(2), g = groups > 0 ? groups : dim;
+    expect_numel(weight, dim, "weight");
+    expect_numel(pmean, g, "prior_mean");
     const NormParams r = prepare(weight, bias, pcount, pmean, plogv, bsz, w);
     const Tensor mask = mask_u8(given(mask_), bsz, length);
     const bool again = groups <= 0 && whole_rows(x);
@@ -485,7 +529,10 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> sequence_norm_fwd(const Tensor& x, co
   const Sqn a = sqn_view(x, length_last);
   const int64_t g = groups > 0 ? groups : a.dim;
   const Tensor mask = mask_u8(given(mask_), a.bsz, a.length);
+  expect_numel(gamma_, a.dim, "gamma");
+  expect_numel(beta_, a.dim, "beta");
   const Tensor y = out_.has_value() ? *out_ : like(x);
+  expect(y.sizes() == x.sizes() && y.scalar_type() == x.scalar_type(), "out must be like x");
   Tensor count = counts(a.bsz, x), st = floats({2, a.bsz, g}, x);
   Tensor mean = st.select(0, 0), rstd = st.select(0, 1);
   run_sqn(x, y, f32c(gamma_), f32c(beta_), mask, eps, length_last, g, count, mean, rstd, w);
@@ -496,10 +543,11 @@ class SqnFn : public torch::autograd::Function<SqnFn> {
  public:
   static Tensor forward(AutogradContext* ctx, Tensor x, Tensor weight, Tensor bias, OptTensor mask_, double eps, bool length_last,
                         int64_t groups) {
-    on_cuda(x, weight, given(mask_));
+    on_cuda(x, weight, bias, given(mask_));
     const Where w(x);
     const Sqn a = sqn_view(x, length_last);
     const int64_t g = groups > 0 ? groups : a.dim;
+    expect_numel(weight, a.dim, "weight");
     const NormParams r = prepare(weight, bias, none(), none(), none(), 0, w);
     const Tensor mask = mask_u8(given(mask_), a.bsz, a.length);
     Tensor y = like(x), count = counts(a.bsz, x), st = floats({2, a.bsz, g}, x);
@@ -548,6 +596,12 @@ py::tuple tsn_ema_forward(const Tensor& x, const Tensor& pc_, const Tensor& pm_,
   const Tensor p = f32c(p_), q = cplx ? c64(q_) : f32c(q_), g = cplx ? c64(g_) : f32c(g_), omega = f32c(omega_);
   const Tensor h_in = cplx ? c64(given(h_in_)) : f32c(given(h_in_));
   const int64_t n = p.size(1);
+  check_coeffs(p, q, g, omega, h_in, cplx, bsz, dim, false);
+  expect_numel(pc, bsz, "prev_count");
+  expect_numel(pm, bsz * dim, "prev_mean");
+  expect_numel(pv, bsz * dim, "prev_var");
+  expect_numel(gamma, dim, "gamma");
+  expect_numel(beta, dim, "beta");
   const Tensor mask = mask_u8(given(mask_), bsz, length);
   Tensor y = like(x), xn = want_normed ? like(y) : Tensor();
   Tensor count = counts(bsz, x), st = floats({2, bsz, dim}, x);
@@ -571,6 +625,9 @@ OptTensor sqn_ema_forward(const Tensor& x, const Tensor& gamma, const Tensor& be
   if (x.stride(2) != 1) return std::nullopt;
   const Where w(x);
   const Tensor p = f32c(p_), q = f32c(q_), g = f32c(g_), omega = f32c(omega_), ga = f32c(gamma), be = f32c(beta);
+  check_coeffs(p, q, g, omega, none(), false, x.size(0), x.size(1), flags & MEGA_EMA_BIDIRECTIONAL);
+  expect_numel(ga, x.size(1), "gamma");
+  expect_numel(be, x.size(1), "beta");
   const Tensor mask = mask_u8(given(mask_), x.size(0), x.size(2));
   Tensor y = at::empty(x.sizes(), x.options().requires_grad(false));
   const int rc = mega_sqn_ema_fwd(x.data_ptr(), y.data_ptr(), dtype_of(x), (int)x.size(0), (int)x.size(1), (int)x.size(2), STRIDES3(x),
@@ -671,16 +728,29 @@ Tensor softmax_fwd(const Tensor& x, bool causal) {
   return y;
 }
 
+// the shapes that pointers into the projections' outputs rely on
+void check_block(const Tensor& x, const Tensor& wv, const Tensor& wm, const Tensor& wh, const Tensor& gamma, const Tensor& beta,
+                 const Tensor& bias, const Tensor& rot, int64_t period) {
+  const int64_t d = x.size(2), s = gamma.size(1), e = wv.size(0);
+  expect(wv.dim() == 2 && wv.size(1) == d && wm.dim() == 2 && wm.size(0) == 2 * d + s + e && wm.size(1) == d && wh.dim() == 2 &&
+             wh.size(0) == d && wh.size(1) == e, "projections do not fit the block");
+  expect(gamma.numel() == 2 * s && beta.numel() == 2 * s, "gamma and beta must be (2, zdim)");
+  expect(period > 0 && x.size(0) * x.size(1) % period == 0, "chunks do not divide the sequence");
+  expect(!bias.defined() || bias.numel() >= 2 * period - 1, "relative bias too short");
+  expect(!rot.defined() || rot.numel() >= period * s, "rotary table too short");
+}
+
 // Training pass from the moving average to the output.  bias: learned relative bias (2 P - 1), or rot: rotary table
 // (positions, S / 2, 2) with the causal mask; rows (b, t) sit at position t % period of their chunk.
 class BlockFn : public torch::autograd::Function<BlockFn> {
  public:
   static Tensor forward(AutogradContext* ctx, Tensor x, Tensor xn, Tensor mx, Tensor wv, Tensor bv, Tensor wm, Tensor bm, Tensor wh,
                         Tensor gamma, Tensor beta, OptTensor bias_, OptTensor rot_, OptTensor mask_, int64_t period) {
-    on_cuda(x, xn, mx, wv, wm, wh, given(mask_));
+    on_cuda(x, xn, mx, wv, bv, wm, bm, wh, gamma, beta, given(bias_), given(rot_), given(mask_));
     const Where w(x);
     const int64_t bsz = x.size(0), seq = x.size(1), d = x.size(2), rows = bsz * seq, s = gamma.size(1), e = wv.size(0);
     const int64_t f = 2 * d + s + e, nb = rows / period;
+    check_block(x, wv, wm, wh, gamma, beta, given(bias_), given(rot_), period);
     const int dt = dtype_of(x);
     const int64_t es = x.element_size();
     const Tensor bias = given(bias_), rot = given(rot_);
@@ -805,7 +875,8 @@ class BlockFn : public torch::autograd::Function<BlockFn> {
 std::tuple<Tensor, Tensor, Tensor> block_infer(Tensor x, Tensor xn, Tensor mx, const Tensor& wv, const Tensor& bv, const Tensor& wm,
                                                const Tensor& bm, const Tensor& wh, const Tensor& gamma, const Tensor& beta,
                                                const Tensor& rot, int64_t period, bool cache) {
-  on_cuda(x, xn, mx, wv, wm, wh);
+  on_cuda(x, xn, mx, wv, bv, wm, bm, wh, gamma, beta, rot);
+  check_block(x, wv, wm, wh, gamma, beta, none(), rot, period);
   const Where w(x);
   const int64_t bsz = x.size(0), seq = x.size(1), d = x.size(2), rows = bsz * seq, s = gamma.size(1), e = wv.size(0);
   const int64_t f = 2 * d + s + e, nb = rows / period;

@@ -1,0 +1,87 @@
+"""The native host side: what it refuses, the precision of parameters of several types, autograd around its Functions."""
+import copy
+
+import pytest
+import torch
+
+from _util import make_ema_params, rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+def _cuda(*ts):
+    return [t.cuda() for t in ts]
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("wrong", ["rows", "bidirectional", "delta", "third", "gamma", "omega", "device"])
+def test_training_ema_checks_its_parameters(cplx, wrong):
+    from fairseq_apollo_b200 import functions
+    gen = torch.Generator().manual_seed(0)
+    dim, n = 16, 16
+    prm = make_ema_params(gen, dim, n, device="cuda")
+    if cplx:
+        prm[2], prm[3] = torch.randn(dim, 1, 1).cuda(), torch.randn(dim, n, 2).cuda()
+    x = torch.randn(2, 8, dim, device="cuda", requires_grad=True)
+    bidir, error = False, ValueError
+    if wrong == "rows":
+        x = torch.randn(2, 8, dim + 8, device="cuda", requires_grad=True)
+    elif wrong == "bidirectional":
+        bidir = True
+    elif wrong == "device":
+        prm[1], error = prm[1].cpu(), RuntimeError
+    else:
+        at = {"delta": 1, "third": 2, "gamma": 3, "omega": 4}[wrong]
+        prm[at] = prm[at][: dim // 2].contiguous()
+    with pytest.raises(error):
+        functions.ema(x, *prm, None, bidir, True, None, cplx, False, True)
+
+
+@pytest.mark.parametrize("wrong", ["bias", "prior", "logv", "features", "device"])
+def test_training_norms_checks_their_parameters(wrong):
+    from fairseq_apollo_b200 import functions
+    x = torch.randn(2, 8, 16, device="cuda", requires_grad=True)
+    w, b, m, v = (torch.randn(16, device="cuda") for _ in range(4))
+    count, error = torch.tensor(2, device="cuda"), ValueError
+    if wrong == "bias":
+        b = b[:8].contiguous()
+    elif wrong == "prior":
+        m, v = m[:8].contiguous(), v[:8].contiguous()
+    elif wrong == "logv":
+        v = v[:8].contiguous()
+    elif wrong == "features":
+        w, b = w[:8].contiguous(), b[:8].contiguous()
+    else:
+        b, error = b.cpu(), RuntimeError
+    with pytest.raises(error):
+        functions.timestep_norm(x, count, m, v, w, b, None, None, 1e-5)
+    if wrong in ("bias", "features", "device"):
+        with pytest.raises(error):
+            functions.sequence_norm(x, w, b, None, 1e-5, False)
+
+
+def test_fused_operators_checks_their_operands():
+    from fairseq_apollo_b200 import ops
+    x = torch.randn(2, 600, 16, device="cuda")
+    c = torch.full((2,), 2, device="cuda")
+    m, v = torch.zeros(2, 16, device="cuda"), torch.ones(2, 16, device="cuda")
+    one = torch.ones(16, device="cuda")
+    co = [torch.rand(16, 4, device="cuda") for _ in range(3)]
+    ops.tsn_ema_forward(x, c, m, v, one, one, 1e-5, *co, one)
+    bad = [dict(m=m[:1]), dict(v=v[:, :8]), dict(c=c[:1]), dict(ga=one[:8]), dict(be=one[:8]), dict(om=one[:8]),
+           dict(co=[t[:8] for t in co]), dict(co=[co[0], co[1][:8], co[2]]), dict(h=torch.zeros(2, 8, 4, device="cuda"))]
+    for b in bad:
+        with pytest.raises(ValueError):
+            ops.tsn_ema_forward(x, b.get("c", c), b.get("m", m), b.get("v", v), b.get("ga", one), b.get("be", one), 1e-5,
+                                *b.get("co", co), b.get("om", one), None, b.get("h"), True)
+    xt = x.transpose(1, 2).contiguous()
+    for ga, om, k in ((one[:8], one, co), (one, one[:8], co), (one, one, [t[:8] for t in co])):
+        with pytest.raises(ValueError):
+            ops.sqn_ema_forward(xt, ga, one, 1e-5, *k, om)
+    for ga, be in ((one[:8], one), (one, one[:8])):
+        with pytest.raises(ValueError):
+            ops.timestep_norm_fwd(x, c, m, v, ga, be)
+        with pytest.raises(ValueError):
+            ops.sequence_norm_fwd(x, ga, be, length_last=False)
+    with pytest.raises(ValueError):
+        ops.ema_forward(xt, *co, one[:8])
