@@ -117,11 +117,12 @@ std::vector<Tensor> f32_all(const std::vector<Tensor>& ts, void* stream) {
   if (count) check(mega_to_float(src, dst, n, count, dt, stream), "to_float");
   return out;
 }
-// complex64 as its interleaved floats
-Tensor c64(const Tensor& t) {
+// complex64 of `dims` dimensions as its interleaved floats; a real tensor has no imaginary part, unless it is (..., 2) fp32
+// and so interleaved already
+Tensor c64(const Tensor& t, int64_t dims) {
   if (!t.defined()) return t;
   Tensor d = t.detach();
-  if (d.scalar_type() == at::kFloat) return d.contiguous();   // already interleaved
+  if (d.scalar_type() == at::kFloat && d.dim() > dims && d.size(-1) == 2) return d.contiguous();
   if (d.scalar_type() != at::kComplexFloat) d = d.to(at::kComplexFloat);
   return at::view_as_real(d.contiguous());
 }
@@ -209,10 +210,10 @@ std::tuple<Tensor, OptTensor> ema_forward(const Tensor& x, const Tensor& p_, con
   on_cuda(x, p_, q_, g_, omega_, given(mask_), given(h_in_));
   const Where w(x);
   const int64_t bsz = x.size(0), dim = x.size(1);
-  const Tensor p = f32c(p_), q = cplx ? c64(q_) : f32c(q_), g = cplx ? c64(g_) : f32c(g_), omega = f32c(omega_);
+  const Tensor p = f32c(p_), q = cplx ? c64(q_, 2) : f32c(q_), g = cplx ? c64(g_, 2) : f32c(g_), omega = f32c(omega_);
   const int64_t n = p.size(1);
   const Tensor mask = mask_u8(given(mask_), bsz, x.size(2));
-  const Tensor h_in = cplx ? c64(given(h_in_)) : f32c(given(h_in_));
+  const Tensor h_in = cplx ? c64(given(h_in_), 3) : f32c(given(h_in_));
   check_coeffs(p, q, g, omega, h_in, cplx, bsz, dim, flags & MEGA_EMA_BIDIRECTIONAL);
   const Tensor y = out_.has_value() ? *out_ : like(x);
   expect(y.sizes() == x.sizes() && y.scalar_type() == x.scalar_type(), "out must be like x");
@@ -593,8 +594,8 @@ py::tuple tsn_ema_forward(const Tensor& x, const Tensor& pc_, const Tensor& pm_,
   const Where w(x);
   const int64_t bsz = x.size(0), length = x.size(1), dim = x.size(2);
   const Tensor pc = pc_.to(at::kLong).contiguous(), pm = f32c(pm_), pv = f32c(pv_), gamma = f32c(gamma_), beta = f32c(beta_);
-  const Tensor p = f32c(p_), q = cplx ? c64(q_) : f32c(q_), g = cplx ? c64(g_) : f32c(g_), omega = f32c(omega_);
-  const Tensor h_in = cplx ? c64(given(h_in_)) : f32c(given(h_in_));
+  const Tensor p = f32c(p_), q = cplx ? c64(q_, 2) : f32c(q_), g = cplx ? c64(g_, 2) : f32c(g_), omega = f32c(omega_);
+  const Tensor h_in = cplx ? c64(given(h_in_), 3) : f32c(given(h_in_));
   const int64_t n = p.size(1);
   check_coeffs(p, q, g, omega, h_in, cplx, bsz, dim, false);
   expect_numel(pc, bsz, "prev_count");

@@ -85,3 +85,15 @@ def test_fused_operators_checks_their_operands():
             ops.sequence_norm_fwd(x, ga, be, length_last=False)
     with pytest.raises(ValueError):
         ops.ema_forward(xt, *co, one[:8])
+
+
+def test_real_coefficients_of_the_complex_layer():
+    """q, gamma and the state given as real tensors are complex ones without an imaginary part."""
+    from fairseq_apollo_b200 import ops
+    gen = torch.Generator().manual_seed(0)
+    x = torch.randn(2, 16, 50, generator=gen).cuda()
+    p, q, g = (torch.rand(16, 4, generator=gen).cuda() for _ in range(3))
+    om, h = torch.randn(16, generator=gen).cuda(), torch.randn(2, 16, 4, generator=gen).cuda()
+    y, hn = ops.cema_forward(x, p, q, g, om, None, h, want_state=True)
+    want, hw = ops.ema_forward(x, p, q, g, om, None, h, want_state=True)
+    assert rel_l2(y, want) < 1e-5 and rel_l2(hn.real, hw) < 1e-5
