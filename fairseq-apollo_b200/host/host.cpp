@@ -15,6 +15,7 @@
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/extension.h>
 
+#include <algorithm>
 #include <tuple>
 #include <vector>
 
@@ -96,14 +97,15 @@ std::vector<Tensor> f32_all(const std::vector<Tensor>& ts, void* stream) {
   float* dst[8];
   int64_t n[8], total = 0;
   int count = 0;
-  for (const auto& t : ts) total += t.scalar_type() != at::kFloat ? (t.numel() + 3) / 4 * 4 : 0;
+  auto half = [](const Tensor& t) { return t.scalar_type() == at::kBFloat16 || t.scalar_type() == at::kHalf; };
+  for (const auto& t : ts) total += half(t) ? (t.numel() + 3) / 4 * 4 : 0;
   Tensor all;
   if (total) all = at::empty({total}, at::TensorOptions().dtype(at::kFloat).device(ts[0].device()));
   int64_t from = 0;
   int dt = -1;
   for (size_t i = 0; i < ts.size(); ++i) {
     const Tensor& t = ts[i];
-    if (t.scalar_type() == at::kFloat || !t.is_contiguous() || (dt >= 0 && dtype_of(t) != dt) || count == 8) {
+    if (!half(t) || !t.is_contiguous() || (dt >= 0 && dtype_of(t) != dt) || count == 8) {
       out[i] = f32c(t);
       continue;
     }
@@ -320,8 +322,9 @@ class EmaFn : public torch::autograd::Function<EmaFn> {
                          dom, nullptr, w.stream), "ema_bwd");
       check(mega_ema_coeffs_bwd(fptr(alpha), fptr(delta), fptr(third), dp, dq, dg, (int)k, (int)n, da, dd, db, dgm, w.stream), "ema_coeffs_bwd");
     }
+    // (one conversion where the parameters share a type; none passes through another's)
     Tensor out = f.narrow(0, sums, D + raw);
-    if ((at::ScalarType)types[0] != at::kFloat) out = out.to((at::ScalarType)types[0]);
+    if (std::all_of(types.begin(), types.end(), [&](int64_t t) { return t == types[0]; })) out = out.to((at::ScalarType)types[0]);
     const int64_t base = out.storage_offset();
     auto part = [&](int64_t from, at::IntArrayRef size, at::IntArrayRef stride, int64_t type) {
       Tensor v = out.as_strided(size, stride, base + from);
@@ -346,6 +349,24 @@ struct NormParams {
   Tensor gamma, beta, count, mean, var;
 };
 
+// The type that parameters share when the library reads it, else fp32: none of them passes through a narrower one.
+at::ScalarType common_type(std::initializer_list<Tensor> ts) {
+  at::ScalarType type = at::kFloat;
+  bool first = true;
+  for (const auto& t : ts) {
+    if (!t.defined()) continue;
+    const auto own = t.scalar_type();
+    if ((own != at::kFloat && own != at::kBFloat16 && own != at::kHalf) || (!first && own != type)) return at::kFloat;
+    type = own;
+    first = false;
+  }
+  return type;
+}
+Tensor as_type(const Tensor& t, at::ScalarType type) {
+  if (!t.defined()) return t;
+  return (t.scalar_type() == type ? t.detach() : t.detach().to(type)).contiguous();
+}
+
 NormParams prepare(const Tensor& weight, const Tensor& bias, const Tensor& pc, const Tensor& pm, const Tensor& pl, int64_t bsz,
                    const Where& w) {
   const int64_t d = weight.size(0), g = pm.defined() ? pm.size(0) : 0;
@@ -354,12 +375,9 @@ NormParams prepare(const Tensor& weight, const Tensor& bias, const Tensor& pc, c
   expect_numel(pm, g, "prior_mean");
   if (pm.defined()) expect_numel(pl, g, "prior_logv");
   expect(g <= d, "more prior means than features");
-  const Tensor b = bias.scalar_type() == weight.scalar_type() ? bias : bias.detach().to(weight.scalar_type());
-  Tensor m = pm, l = pl;
-  if (g && m.scalar_type() != weight.scalar_type()) {
-    m = m.detach().to(weight.scalar_type());
-    l = l.detach().to(weight.scalar_type());
-  }
+  const auto type = common_type({weight, bias, pm, pl});
+  const Tensor wt = as_type(weight, type), b = as_type(bias, type), m = as_type(pm, type), l = as_type(pl, type);
+  const Tensor c = pc.defined() ? pc.detach().to(at::kLong).contiguous() : pc;
   Tensor f = floats({2 * d + 2 * bsz * g}, weight);
   NormParams r;
   r.gamma = f.narrow(0, 0, d);
@@ -369,7 +387,7 @@ NormParams prepare(const Tensor& weight, const Tensor& bias, const Tensor& pc, c
     r.var = f.narrow(0, 2 * d + bsz * g, bsz * g).view({bsz, g});
     r.count = counts(bsz, weight);
   }
-  check(mega_norm_prepare(ptr<int64_t>(pc), ptr(m), ptr(l), weight.data_ptr(), b.data_ptr(), dtype_of(weight),
+  check(mega_norm_prepare(ptr<int64_t>(c), ptr(m), ptr(l), wt.data_ptr(), b.data_ptr(), dtype_of(wt),
                           (int)(g ? bsz : 0), (int)g, (int)d, ptr<int64_t>(r.count), fptr(r.mean), fptr(r.var), fptr(r.gamma),
                           fptr(r.beta), w.stream), "norm_prepare");
   return r;
@@ -384,25 +402,23 @@ py::tuple norm_prepare(const Tensor& weight, const Tensor& bias, const OptTensor
   return py::make_tuple(r.gamma, r.beta, r.count, r.mean, r.var);
 }
 
-// (dweight, dbias, dprior_mean, dprior_logv) in the parameters' type
-std::vector<Tensor> finish(const Tensor& weight, const Tensor& logv, const float* dgamma, const float* dbeta, const float* dpm,
-                           const float* dpv, int64_t bsz, int64_t g, const Where& w) {
+// (dweight, dbias, dprior_mean, dprior_logv), each in its parameter's type
+std::vector<Tensor> finish(const Tensor& weight, const Tensor& bias, const Tensor& pm, const Tensor& logv, const float* dgamma,
+                           const float* dbeta, const float* dpm, const float* dpv, int64_t bsz, int64_t g, const Where& w) {
   const int64_t d = weight.size(0);
-  Tensor out = at::empty({2 * d + 2 * g}, weight.options().requires_grad(false));
-  const Tensor l = g && logv.scalar_type() != weight.scalar_type() ? logv.detach().to(weight.scalar_type()) : logv;
+  const auto type = common_type({weight, bias, pm, logv});
+  Tensor out = at::empty({2 * d + 2 * g}, weight.options().requires_grad(false).dtype(type));
+  const Tensor l = as_type(logv, type);
   char* at_ = static_cast<char*>(out.data_ptr());
   const int64_t es = out.element_size();
-  check(mega_norm_finish(dpm, dpv, ptr(l), dgamma, dbeta, dtype_of(weight), (int)(g ? bsz : 0), (int)g, (int)d,
+  check(mega_norm_finish(dpm, dpv, ptr(l), dgamma, dbeta, dtype_of(out), (int)(g ? bsz : 0), (int)g, (int)d,
                          g ? at_ + 2 * d * es : nullptr, g ? at_ + (2 * d + g) * es : nullptr, at_, at_ + d * es, w.stream),
         "norm_finish");
-  std::vector<Tensor> r = {out.narrow(0, 0, d), out.narrow(0, d, d)};
+  auto own = [&](int64_t from, const Tensor& p) { return out.narrow(0, from, p.numel()).view(p.sizes()).to(p.scalar_type()); };
+  std::vector<Tensor> r = {own(0, weight), own(d, bias)};
   if (g) {
-    r.push_back(out.narrow(0, 2 * d, g));
-    r.push_back(out.narrow(0, 2 * d + g, g));
-    if (logv.scalar_type() != weight.scalar_type()) {
-      r[2] = r[2].to(logv.scalar_type());
-      r[3] = r[3].to(logv.scalar_type());
-    }
+    r.push_back(own(2 * d, pm));
+    r.push_back(own(2 * d + g, logv));
   }
   return r;
 }
@@ -455,7 +471,7 @@ class TsnFn : public torch::autograd::Function<TsnFn> {
                                    ptr<int64_t>(r.count), fptr(r.mean), fptr(r.var), fptr(r.gamma), fptr(r.beta),
                                    ptr<uint8_t>(mask), (int)g, eps, ptr<int64_t>(count), fptr(st), fptr(st) + bsz * g, w.stream),
             "timestep_norm_fwd");
-      ctx->save_for_backward({x, weight, plogv, r.gamma, mask, r.count, r.mean, r.var});
+      ctx->save_for_backward({x, weight, plogv, r.gamma, mask, r.count, r.mean, r.var, bias, pmean});
     } else {
       Tensor st = floats({2, bsz, g}, x), cm = floats({bsz, length, g}, x), cr = floats({bsz, length, g}, x);
       Tensor gm = g != dim ? floats({bsz, length, g}, x) : Tensor();
@@ -463,7 +479,7 @@ class TsnFn : public torch::autograd::Function<TsnFn> {
                                          STRIDES3(y), ptr<int64_t>(r.count), fptr(r.mean), fptr(r.var), fptr(r.gamma),
                                          fptr(r.beta), ptr<uint8_t>(mask), (int)g, eps, ptr<int64_t>(count), fptr(st),
                                          fptr(st) + bsz * g, fptr(cm), fptr(cr), fptr(gm), w.stream), "timestep_norm_fwd_train");
-      ctx->save_for_backward({x, weight, plogv, r.gamma, mask, count, r.mean, Tensor(), cm, cr, gm});
+      ctx->save_for_backward({x, weight, plogv, r.gamma, mask, count, r.mean, Tensor(), bias, pmean, cm, cr, gm});
     }
     ctx->saved_data["again"] = again;
     ctx->saved_data["g"] = g;
@@ -493,9 +509,9 @@ class TsnFn : public torch::autograd::Function<TsnFn> {
     else
       check(mega_timestep_norm_bwd(dy.data_ptr(), x.data_ptr(), dx.data_ptr(), dtype_of(x), (int)bsz, (int)x.size(1), (int)dim,
                                    STRIDES3(dy), STRIDES3(x), STRIDES3(dx), nullptr, nullptr, fptr(s[6]), ptr<int64_t>(s[5]),
-                                   fptr(s[8]), fptr(s[9]), fptr(s[10]), fptr(gamma), ptr<uint8_t>(mask), (int)g, dpm, dpv,
+                                   fptr(s[10]), fptr(s[11]), fptr(s[12]), fptr(gamma), ptr<uint8_t>(mask), (int)g, dpm, dpv,
                                    dgamma, dbeta, w.stream), "timestep_norm_bwd");
-    auto r = finish(weight, plogv, dgamma, dbeta, dpm, dpv, bsz, g, w);
+    auto r = finish(weight, s[8], s[9], plogv, dgamma, dbeta, dpm, dpv, bsz, g, w);
     return {dx, Tensor(), r[2], r[3], r[0], r[1], Tensor(), Tensor(), Tensor()};
   }
 };
@@ -554,7 +570,7 @@ class SqnFn : public torch::autograd::Function<SqnFn> {
     Tensor y = like(x), count = counts(a.bsz, x), st = floats({2, a.bsz, g}, x);
     Tensor mean = st.select(0, 0), rstd = st.select(0, 1);
     run_sqn(x, y, r.gamma, r.beta, mask, eps, length_last, g, count, mean, rstd, w);
-    ctx->save_for_backward({x, weight, r.gamma, mask, count, mean, rstd});
+    ctx->save_for_backward({x, weight, r.gamma, mask, count, mean, rstd, bias});
     ctx->saved_data["ll"] = length_last;
     ctx->saved_data["g"] = g;
     return y;
@@ -574,7 +590,7 @@ class SqnFn : public torch::autograd::Function<SqnFn> {
                                  q.sd, q.sl, a.sb, a.sd, a.sl, o.sb, o.sd, o.sl, ptr<int64_t>(s[4]), fptr(s[5]), fptr(s[6]),
                                  fptr(s[2]), ptr<uint8_t>(s[3]), (int)ctx->saved_data["g"].toInt(), fptr(f), fptr(f) + a.dim,
                                  w.stream), "sequence_norm_bwd");
-    auto r = finish(weight, none(), fptr(f), fptr(f) + a.dim, nullptr, nullptr, 0, 0, w);
+    auto r = finish(weight, s[7], none(), none(), fptr(f), fptr(f) + a.dim, nullptr, nullptr, 0, 0, w);
     return {dx, r[0], r[1], Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };
@@ -860,7 +876,10 @@ class BlockFn : public torch::autograd::Function<BlockFn> {
     Tensor dwv = need_wv ? at::mm(dv.t(), xn) : Tensor();
     Tensor dmx = need_mx ? at::mm(dbase, wm).view({bsz, seq, d}) : Tensor();
     Tensor dwm = need_wm ? at::mm(dbase.t(), mx) : Tensor();
-    Tensor flat = wv.scalar_type() == at::kFloat ? sums : sums.to(wv.scalar_type());
+    const auto own = wv.scalar_type();   // (one conversion where all share it; none passes through another's type)
+    const bool same = std::all_of(types.begin(), types.end(), [&](int64_t t) { return t == (int64_t)own; }) &&
+                      (!nbias || bias.scalar_type() == own);
+    Tensor flat = same ? sums.to(own) : sums;
     auto part = [&](int64_t from, int64_t count, int64_t type) {
       Tensor t = flat.narrow(0, from, count);
       return t.scalar_type() == (at::ScalarType)type ? t : t.to((at::ScalarType)type);

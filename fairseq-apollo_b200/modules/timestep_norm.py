@@ -107,13 +107,7 @@ class TimestepNorm(IncrementalStateMixin, nn.Module):
         key = [batch_size] + [p._version for p in ps] + [p.data_ptr() for p in ps] if keep else None
         cache = self.__dict__.get("_prep")
         if not keep or cache is None or cache[0] != key or any(a is not b for a, b in zip(cache[1], ps)):
-            if self.prior_mean.dtype == self.weight.dtype == self.bias.dtype:
-                prep = ops.norm_prepare(self.weight, self.bias, ps[:3], batch_size)
-            else:
-                prep = (self.weight.detach().float() + 1.0, self.bias.detach().float().contiguous(),
-                        self.prior_count.expand(batch_size).contiguous(),
-                        self.prior_mean.detach().float().expand(batch_size, -1).contiguous(),
-                        torch.exp(self.prior_logv.detach().float()).expand(batch_size, -1).contiguous())
+            prep = ops.norm_prepare(self.weight, self.bias, ps[:3], batch_size)
             if not keep:
                 return prep
             cache = self.__dict__["_prep"] = (key, ps, prep)

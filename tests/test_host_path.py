@@ -97,3 +97,70 @@ def test_real_coefficients_of_the_complex_layer():
     y, hn = ops.cema_forward(x, p, q, g, om, None, h, want_state=True)
     want, hw = ops.ema_forward(x, p, q, g, om, None, h, want_state=True)
     assert rel_l2(y, want) < 1e-5 and rel_l2(hn.real, hw) < 1e-5
+
+
+@pytest.mark.parametrize("wide", [torch.float32, torch.float64])
+def test_parameters_of_several_types(wide):
+    """bf16 scale and shift beside wider priors (and the other way round): no value passes through the narrower type."""
+    import fairseq_apollo_b200 as M
+    torch.manual_seed(3)
+    norm = M.TimestepNorm(64, prior_count=4).cuda()
+    with torch.no_grad():
+        for p in norm.parameters():
+            p.normal_(0, 0.3)
+    x, dy = torch.randn(2, 100, 64, device="cuda"), torch.randn(2, 100, 64, device="cuda")
+    for narrow in (("weight", "bias"), ("prior_mean", "prior_logv"), ("bias",), ("weight", "prior_logv"), ()):
+        mixed, ref = copy.deepcopy(norm), copy.deepcopy(norm)
+        for name, p in mixed.named_parameters():
+            p.data = p.data.to(torch.bfloat16 if name in narrow else wide)
+        for (name, p), q in zip(mixed.named_parameters(), ref.parameters()):
+            q.data = p.data.float()
+        out = []
+        for m in (mixed, ref):
+            xx = x.clone().requires_grad_(True)
+            y = m(xx)
+            y.backward(dy)
+            out.append([y, xx.grad] + [p.grad for p in m.parameters()])
+            with torch.no_grad():
+                out[-1].append(m(x))
+        for a, b in zip(*out):
+            assert rel_l2(a, b.to(a.dtype)) < 1e-6
+        for p in mixed.parameters():
+            assert p.grad.dtype == p.dtype
+
+
+def test_ema_parameters_of_several_types():
+    import fairseq_apollo_b200 as M
+    torch.manual_seed(4)
+    x, dy = torch.randn(2, 32, 200, device="cuda"), torch.randn(2, 32, 200, device="cuda")
+    for names in (("alpha",), ("omega",), ("gamma", "beta")):
+        mixed = M.MultiHeadEMA(32, ndim=16).cuda()
+        ref = copy.deepcopy(mixed)
+        for name, p in mixed.named_parameters():
+            if name in names:
+                p.data = p.data.bfloat16()
+        for p, q in zip(mixed.parameters(), ref.parameters()):
+            q.data = p.data.float()
+        if "alpha" in names:    # (the coefficients are made in alpha's type)
+            for q in (ref.delta, ref.beta, ref.gamma):
+                q.data = q.data.bfloat16().float()
+        for m in (mixed, ref):
+            m(x).backward(dy)
+        for (name, p), q in zip(mixed.named_parameters(), ref.named_parameters()):
+            assert rel_l2(p.grad.float(), q[1].grad) < (1e-2 if p.dtype == torch.bfloat16 or "alpha" in names else 1e-5), name
+
+
+def test_block_with_fp32_affine_in_a_16_bit_block():
+    """The query / key affine kept in fp32: its gradients are not rounded to the projections' type."""
+    import fairseq_apollo_b200 as M
+    torch.manual_seed(6)
+    blk = M.MovingAverageGatedAttention(64, 64, 128, 16, efficient_attn=True, rel_pos_bias='rotary', chunk_size=32,
+                                        moving_act='silu').cuda().bfloat16()
+    for name in ("gamma", "beta"):
+        p = getattr(blk, name)
+        p.data = torch.randn_like(p.data, dtype=torch.float32) * 0.3
+    x = torch.randn(2, 64, 64, device="cuda").bfloat16().requires_grad_(True)
+    blk(x)[0].sum().backward()
+    for p in (blk.gamma, blk.beta):
+        assert p.grad.dtype == torch.float32
+        assert (p.grad != p.grad.bfloat16().float()).float().mean() > 0.5
