@@ -246,18 +246,18 @@ class EmaFn : public torch::autograd::Function<EmaFn> {
     const Where w(x);
     const Tensor mask = mask_u8(given(mask_), x.size(0), x.size(2));
     const Coeffs c = coeffs(alpha, delta, third, gamma, cplx, w);
-    Tensor y = like(x);
+    // (the result is a tensor of its own, not a view of one: a view made in here could not be changed in place)
+    Tensor y_ = like(x_), y = chan ? y_.transpose(1, 2) : y_, out = y_;
     const auto f = f32_all({omega, alpha, delta, third}, w.stream);
     run_ema(x, y, c.p, c.q, c.g, f[0], mask, none(), none(), (unsigned)flags, (int)trunc, cplx, w);
-    Tensor out = y;
     if (silu) {
       int64_t rows;
-      if (rows_of(y, x.size(1), rows)) {
-        out = like(y);
-        check(mega_gate_silu(y.data_ptr(), x.size(1), nullptr, 0, out.data_ptr(), x.size(1), dtype_of(y), rows, (int)x.size(1),
+      if (rows_of(y_, x.size(1), rows)) {
+        out = like(y_);
+        check(mega_gate_silu(y_.data_ptr(), x.size(1), nullptr, 0, out.data_ptr(), x.size(1), dtype_of(y), rows, (int)x.size(1),
                              w.stream), "gate_silu");
       } else {
-        out = at::silu(y);
+        out = at::silu(y_);
       }
     }
     ctx->save_for_backward({x_, f[1], f[2], f[3], f[0], mask, c.p, c.q, c.g, silu ? y : Tensor()});
@@ -268,7 +268,7 @@ class EmaFn : public torch::autograd::Function<EmaFn> {
     ctx->saved_data["types"] = std::vector<int64_t>{(int64_t)alpha.scalar_type(), (int64_t)delta.scalar_type(),
                                                     (int64_t)third.scalar_type(), (int64_t)gamma.scalar_type(),
                                                     (int64_t)omega.scalar_type()};
-    return chan ? out.transpose(1, 2) : out;
+    return out;
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {

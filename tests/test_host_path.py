@@ -164,3 +164,19 @@ def test_block_with_fp32_affine_in_a_16_bit_block():
     for p in (blk.gamma, blk.beta):
         assert p.grad.dtype == torch.float32
         assert (p.grad != p.grad.bfloat16().float()).float().mean() > 0.5
+
+
+@pytest.mark.parametrize("silu", [None, "silu"])
+def test_result_may_be_changed_in_place(silu):
+    import fairseq_apollo_b200 as M
+    torch.manual_seed(8)
+    norm, move = M.TimestepNorm(64, prior_count=2).cuda(), M.MultiHeadEMA(64, ndim=16).cuda()
+    x = torch.randn(2, 40, 64, device="cuda", requires_grad=True)
+    grads = []
+    for inplace in (False, True):
+        x.grad = None
+        y = M.timestep_norm_ema(norm, move, x, None, None, silu)
+        y = y.mul_(2.0) if inplace else y * 2.0
+        y.sum().backward()
+        grads.append(x.grad.clone())
+    assert torch.equal(*grads)
