@@ -423,6 +423,8 @@ std::vector<Tensor> finish(const Tensor& weight, const Tensor& bias, const Tenso
   return r;
 }
 
+constexpr int64_t kGridSequences = 65535;   // sequences that the kernels over time take in a launch
+
 bool whole_rows(const Tensor& x) {   // contiguous channels in whole 16-byte pieces
   const int64_t es = x.element_size();
   return x.stride(2) == 1 && x.size(2) * es % 16 == 0 && x.stride(0) * es % 16 == 0 && x.stride(1) * es % 16 == 0 &&
@@ -463,7 +465,7 @@ class TsnFn : public torch::autograd::Function<TsnFn> {
     expect_numel(pmean, g, "prior_mean");
     const NormParams r = prepare(weight, bias, pcount, pmean, plogv, bsz, w);
     const Tensor mask = mask_u8(given(mask_), bsz, length);
-    const bool again = groups <= 0 && whole_rows(x);
+    const bool again = groups <= 0 && whole_rows(x) && bsz <= kGridSequences;
     Tensor y = like(x), count = counts(bsz, x);
     if (again) {   // the backward takes the statistics again: nothing is kept but the arguments
       Tensor st = floats({2, bsz, g}, x);
@@ -500,17 +502,38 @@ class TsnFn : public torch::autograd::Function<TsnFn> {
     Tensor dx = like(x);
     Tensor f = floats({2 * dim + 2 * bsz * g}, x);
     float *dgamma = fptr(f), *dbeta = dgamma + dim, *dpm = dbeta + dim, *dpv = dpm + bsz * g;
-    if (again)
-      check(mega_timestep_norm_bwd_stats(dy.data_ptr(), x.data_ptr(), dx.data_ptr(), dtype_of(x), (int)bsz, (int)x.size(1), (int)dim,
-                                         STRIDES3(dy), STRIDES3(x), STRIDES3(dx), nullptr, nullptr, ptr<int64_t>(s[5]),
-                                         fptr(s[6]), fptr(s[7]), fptr(gamma), ptr<uint8_t>(mask),
-                                         ctx->saved_data["eps"].toDouble(), dpm, dpv, dgamma, dbeta, w.stream),
-            "timestep_norm_bwd_stats");
-    else
+    bool done = false;
+    if (again) {
+      const int rc = mega_timestep_norm_bwd_stats(dy.data_ptr(), x.data_ptr(), dx.data_ptr(), dtype_of(x), (int)bsz, (int)x.size(1), (int)dim,
+                                                  STRIDES3(dy), STRIDES3(x), STRIDES3(dx), nullptr, nullptr, ptr<int64_t>(s[5]),
+                                                  fptr(s[6]), fptr(s[7]), fptr(gamma), ptr<uint8_t>(mask),
+                                                  ctx->saved_data["eps"].toDouble(), dpm, dpv, dgamma, dbeta, w.stream);
+      done = rc != MEGA_ERR_UNSUPPORTED;   // (the device had no scratch memory for it: with saves, as the other forms do)
+      if (done) check(rc, "timestep_norm_bwd_stats");
+    }
+    if (!done) {
+      Tensor count = s[5], cm, cr, gm;
+      if (again) {
+        const int64_t length = x.size(1);
+        Tensor y = like(x), st = floats({2, bsz, g}, x);
+        count = counts(bsz, x);
+        cm = floats({bsz, length, g}, x);
+        cr = floats({bsz, length, g}, x);
+        check(mega_timestep_norm_fwd_train(x.data_ptr(), y.data_ptr(), dtype_of(x), (int)bsz, (int)length, (int)dim, STRIDES3(x),
+                                           STRIDES3(y), ptr<int64_t>(s[5]), fptr(s[6]), fptr(s[7]), fptr(gamma), fptr(gamma),
+                                           ptr<uint8_t>(mask), (int)g, ctx->saved_data["eps"].toDouble(), ptr<int64_t>(count),
+                                           fptr(st), fptr(st) + bsz * g, fptr(cm), fptr(cr), nullptr, w.stream),
+              "timestep_norm_fwd_train");
+      } else {
+        cm = s[10];
+        cr = s[11];
+        gm = s[12];
+      }
       check(mega_timestep_norm_bwd(dy.data_ptr(), x.data_ptr(), dx.data_ptr(), dtype_of(x), (int)bsz, (int)x.size(1), (int)dim,
-                                   STRIDES3(dy), STRIDES3(x), STRIDES3(dx), nullptr, nullptr, fptr(s[6]), ptr<int64_t>(s[5]),
-                                   fptr(s[10]), fptr(s[11]), fptr(s[12]), fptr(gamma), ptr<uint8_t>(mask), (int)g, dpm, dpv,
-                                   dgamma, dbeta, w.stream), "timestep_norm_bwd");
+                                   STRIDES3(dy), STRIDES3(x), STRIDES3(dx), nullptr, nullptr, fptr(s[6]), ptr<int64_t>(count),
+                                   fptr(cm), fptr(cr), fptr(gm), fptr(gamma), ptr<uint8_t>(mask), (int)g, dpm, dpv, dgamma, dbeta,
+                                   w.stream), "timestep_norm_bwd");
+    }
     auto r = finish(weight, s[8], s[9], plogv, dgamma, dbeta, dpm, dpv, bsz, g, w);
     return {dx, Tensor(), r[2], r[3], r[0], r[1], Tensor(), Tensor(), Tensor()};
   }

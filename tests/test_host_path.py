@@ -180,3 +180,46 @@ def test_result_may_be_changed_in_place(silu):
         y.sum().backward()
         grads.append(x.grad.clone())
     assert torch.equal(*grads)
+
+
+def test_more_sequences_than_a_grid_axis():
+    """65537 sequences: the backward that takes the statistics again has no grid for them; the saved ones do."""
+    import fairseq_apollo_b200 as M
+    torch.manual_seed(9)
+    bsz = 65537
+    norm = M.TimestepNorm(8, prior_count=2).cuda()
+    x = torch.randn(bsz, 2, 8, device="cuda")
+    dy = torch.randn_like(x)
+    xx = x.clone().requires_grad_(True)
+    norm(xx).backward(dy)
+    w, dx = norm.weight.grad.clone(), []
+    norm.zero_grad()
+    for part in (slice(0, 40000), slice(40000, bsz)):
+        xp = x[part].clone().requires_grad_(True)
+        norm(xp).backward(dy[part])
+        dx.append(xp.grad)
+    assert rel_l2(xx.grad, torch.cat(dx)) < 1e-5
+    assert rel_l2(w, norm.weight.grad) < 1e-4
+
+
+def test_backward_without_the_form_over_time():
+    """The form that takes the statistics again refuses (no scratch memory; here: switched off between the passes)."""
+    import fairseq_apollo_b200 as M
+    from fairseq_apollo_b200 import _lib
+    torch.manual_seed(9)
+    norm = M.TimestepNorm(64, prior_count=2).cuda()
+    x, dy, grads = torch.randn(3, 200, 64, device="cuda"), torch.randn(3, 200, 64, device="cuda"), []
+    mask = torch.zeros(3, 200, dtype=torch.bool, device="cuda")
+    mask[1, 100:] = True
+    for off in (0, 1):
+        norm.zero_grad()
+        xx = x.clone().requires_grad_(True)
+        y = norm(xx, mask)
+        _lib.set_option(0, off)
+        try:
+            y.backward(dy)
+        finally:
+            _lib.set_option(0, 0)
+        grads.append([xx.grad] + [p.grad.clone() for p in norm.parameters()])
+    for a, b in zip(*grads):
+        assert rel_l2(a, b) < 1e-5
