@@ -794,6 +794,7 @@ class BlockFn : public torch::autograd::Function<BlockFn> {
     const int dt = dtype_of(x);
     const int64_t es = x.element_size();
     const Tensor bias = given(bias_), rot = given(rot_);
+    const Tensor x_ = x, xn_ = xn, mx_ = mx;
     x = x.contiguous();
     xn = xn.contiguous().view({rows, d});
     mx = mx.contiguous().view({rows, d});
@@ -833,17 +834,65 @@ class BlockFn : public torch::autograd::Function<BlockFn> {
     Tensor h_lin = at::mm(gated, wh.t());
     Tensor out = at::empty({bsz, seq, d}, x.options().requires_grad(false));
     check(mega_gate_output(x.data_ptr(), d, u, f, hx, f, h_lin.data_ptr(), d, out.data_ptr(), d, dt, rows, (int)d, w.stream), "gate_output");
-    ctx->save_for_backward({x, xn, mx, wv, wm, wh, ga, bias, rot, v_lin, base, q, k, v3, wgt, attn, gated, h_lin});
+    ctx->save_for_backward({x, xn, mx, wv, wm, wh, ga, bias, rot, v_lin, base, q, k, v3, wgt, attn, gated, h_lin, x_, xn_, mx_, bv, bm,
+                            gamma, beta, rot.defined() ? Tensor() : mask_u8(given(mask_), bsz, seq)});
     ctx->saved_data["period"] = period;
     ctx->saved_data["types"] = std::vector<int64_t>{(int64_t)bv.scalar_type(), (int64_t)bm.scalar_type(), (int64_t)gamma.scalar_type(),
                                                     (int64_t)beta.scalar_type()};
-    ctx->saved_data["need"] = std::vector<int64_t>{xn.requires_grad(), mx.requires_grad(), wv.requires_grad(), wm.requires_grad(),
-                                                   wh.requires_grad()};
     return out;
+  }
+
+  // The pass in torch operations, for a gradient that is to be differentiated again: the gradients of the inputs as
+  // functions of the inputs.  (Through aliases of them: an input that another one was computed from gets its own share.)
+  static variable_list differentiable(AutogradContext* ctx, const variable_list& sv, Tensor dout) {
+    const int64_t period = ctx->saved_data["period"].toInt();
+    std::vector<Tensor> in = {sv[18], sv[19], sv[20], sv[3], sv[21], sv[4], sv[22], sv[5], sv[23], sv[24], sv[7]};
+    for (auto& t : in)
+      if (t.defined()) t = t.view_as(t);
+    const Tensor &x = in[0], &xn = in[1], &mx = in[2], &wv = in[3], &bv = in[4], &wm = in[5], &bm = in[6], &wh = in[7], &gamma = in[8],
+                 &beta = in[9], &bias = in[10], &rot = sv[8], &mask = sv[25];
+    const int64_t bsz = x.size(0), seq = x.size(1), d = x.size(2), s = gamma.size(1), e = wv.size(0), nb = bsz * seq / period;
+    const auto type = x.scalar_type();
+    const Tensor v = at::silu(at::linear(xn, wv, bv)).reshape({nb, period, e}), base = at::linear(mx, wm, bm);
+    const Tensor u = base.narrow(2, 0, d), z = base.narrow(2, d, s), r = base.narrow(2, d + s, e), hx = base.narrow(2, d + s + e, d);
+    const Tensor zn = z / z.norm(2, {-1}, true).clamp_min(1e-5);
+    auto part = [&](int64_t i) {
+      Tensor t = (zn * (gamma[i] + 1.0) + beta[i]).reshape({nb, period, s});
+      if (!rot.defined()) return t.to(type);
+      const Tensor w = rot.narrow(0, 0, period), f = t.to(at::kFloat).reshape({nb, period, s / 2, 2});
+      const Tensor a = f.select(3, 0), b = f.select(3, 1), c = w.select(2, 0), i_ = w.select(2, 1);
+      return at::stack({a * c - b * i_, a * i_ + b * c}, -1).flatten(2).to(type);
+    };
+    Tensor scores = at::bmm(part(0), part(1).transpose(1, 2));
+    const auto where = scores.options().requires_grad(false);
+    if (rot.defined()) {
+      scores = scores.masked_fill(at::ones({period, period}, where.dtype(at::kBool)).triu(1), -INFINITY);
+    } else {
+      const Tensor at_ = at::arange(period, where.dtype(at::kLong));
+      scores = scores + bias.index({at_.unsqueeze(0) - at_.unsqueeze(1) + (bias.size(0) + 1) / 2 - 1});
+      if (mask.defined()) {
+        const Tensor m = mask.reshape({nb, period}).to(at::kBool);
+        scores = scores.masked_fill(m.logical_and(m.all(1, true).logical_not()).unsqueeze(1), -INFINITY);
+      }
+    }
+    const Tensor attn = at::bmm(scores.to(at::kFloat).softmax(-1).to(type), v).reshape({bsz, seq, e});
+    const Tensor h = at::silu(hx + at::linear(attn * at::silu(r), wh));
+    const Tensor out = at::addcmul(x, u.sigmoid(), h - x);
+    variable_list wanted, result(14);
+    std::vector<size_t> place;
+    for (size_t i = 0; i < in.size(); ++i)
+      if (in[i].defined() && in[i].requires_grad()) {
+        wanted.push_back(in[i]);
+        place.push_back(i);
+      }
+    const auto g = torch::autograd::grad({out}, wanted, {dout}, true, true, true);
+    for (size_t i = 0; i < place.size(); ++i) result[place[i]] = g[i];
+    return result;
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto sv = ctx->get_saved_variables();
+    if (at::GradMode::is_enabled()) return differentiable(ctx, sv, grads[0].to(sv[0].scalar_type()));
     const Tensor &x = sv[0], &xn = sv[1], &mx = sv[2], &wv = sv[3], &wm = sv[4], &wh = sv[5], &ga = sv[6], &bias = sv[7], &rot = sv[8],
                  &v_lin = sv[9], &base = sv[10], &q = sv[11], &k = sv[12], &v3 = sv[13], &wgt = sv[14], &attn = sv[15], &gated = sv[16],
                  &h_lin = sv[17];

@@ -223,3 +223,34 @@ def test_backward_without_the_form_over_time():
         grads.append([xx.grad] + [p.grad.clone() for p in norm.parameters()])
     for a, b in zip(*grads):
         assert rel_l2(a, b) < 1e-5
+
+
+@pytest.mark.parametrize("bidir", [False, True])
+def test_second_derivative_through_the_block(bidir):
+    """A gradient penalty on the projections' inputs: as the block's own sequence of operations gives it."""
+    import fairseq_apollo_b200 as M
+    from fairseq_apollo_b200 import block_function
+    torch.manual_seed(10)
+    kw = dict(bidirectional=True, rel_pos_bias='simple', max_positions=32) if bidir else \
+        dict(efficient_attn=True, rel_pos_bias='rotary')
+    blk = M.MovingAverageGatedAttention(32, 64, 64, 16, chunk_size=-1 if bidir else 16, moving_act='silu', **kw).cuda()
+    with torch.no_grad():
+        for lin in (blk.v_proj, blk.mx_proj, blk.h_proj):
+            lin.weight.normal_(0, 0.2)
+    x = torch.randn(2, 32, 32, device="cuda")
+    res = []
+    mode_of = block_function.mode_of
+    for own in (False, True):
+        block_function.mode_of = (lambda *a: None) if own else mode_of
+        try:
+            xx = x.clone().requires_grad_(True)
+            y = blk(xx)[0]
+            g, = torch.autograd.grad(y.square().sum(), xx, create_graph=True)
+            blk.zero_grad()
+            g.square().sum().backward()
+        finally:
+            block_function.mode_of = mode_of
+        res.append([g.detach()] + [p.grad.clone() for p in blk.parameters() if p.grad is not None])
+    assert len(res[0]) == len(res[1])
+    for a, b in zip(*res):
+        assert rel_l2(a, b) < 1e-4
