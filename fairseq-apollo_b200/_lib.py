@@ -24,7 +24,7 @@ class BlockStepArgs(ctypes.Structure):
                 + [(n, c_p) for n in ("x", "out", "count", "count_next", "mean", "var", "h", "norm_gamma", "norm_beta", "p",
                                       "q", "gamma_hat", "omega", "v_weight", "v_bias", "mx_weight", "mx_bias", "h_weight",
                                       "qk_gamma", "qk_beta", "rot", "keys", "keys_rot", "values", "work")]
-                + [("norm_eps", c_d), ("qk_eps", c_d), ("cap", c_l), ("pos", ctypes.c_int32)])
+                + [("norm_eps", c_d), ("qk_eps", c_d), ("cap", c_l), ("pos", ctypes.c_int32), ("qk_dtype", ctypes.c_int32)])
 
 
 # name -> argument types, in the order of include/mega_b200.h

@@ -50,20 +50,10 @@ def run(blk, mode, x, xn, mx, padding_mask):
                                    blk.h_proj.weight, blk.gamma, blk.beta, bias, rot, padding_mask, period)
 
 
-def qk_affine(blk):
-    """gamma and beta of the queries and keys in fp32, kept until a parameter changes (identity, version counter, storage)."""
-    ver = (blk.gamma._version, blk.beta._version, blk.gamma.data_ptr(), blk.beta.data_ptr())
-    cache = blk.__dict__.get("_qk_fp32")
-    if cache is None or cache[0] is not blk.gamma or cache[1] is not blk.beta or cache[2] != ver:
-        cache = blk._qk_fp32 = (blk.gamma, blk.beta, ver, blk.gamma.detach().float().contiguous(),
-                                blk.beta.detach().float().contiguous())
-    return cache[3], cache[4]
-
-
 def infer(blk, x, xn, mx, cache):
     """The same in inference, causal mode: the output, and with ``cache`` the keys (not rotated) and values."""
     seq = x.size(1)
     period = blk.chunk_size if 1 < blk.chunk_size < seq else seq
     rot = torch.view_as_real(blk.rel_pos_bias._angles(0, period))
     return _lib.host().block_infer(x, xn, mx, blk.v_proj.weight, blk.v_proj.bias, blk.mx_proj.weight, blk.mx_proj.bias,
-                                   blk.h_proj.weight, *qk_affine(blk), rot, period, cache)
+                                   blk.h_proj.weight, blk.gamma, blk.beta, rot, period, cache)

@@ -45,7 +45,9 @@ struct BlockStep {
   const void *x, *xn, *mx;
   void* out;
   const void *vw, *vb, *mw, *mb, *hw;
-  const float *qg, *qb, *rot;
+  const void *qg, *qb;
+  const float* rot;
+  int qk16;         // the query / key affine in the activations' type (else fp32)
   float qk_eps;
   void *keys, *krot, *values;
   long long cap;
@@ -198,12 +200,16 @@ __global__ void __launch_bounds__(256) block_score_kernel(BlockStep a) {
     const int c = 2 * j;
     const float u = Elem<T>::ld_shared(z + c) * inv, v = Elem<T>::ld_shared(z + c + 1) * inv;
     const float2 w = __ldg(rot + j);
-    const float qa = fmaf(u, __ldg(a.qg + c) + 1.f, __ldg(a.qb + c)), qb = fmaf(v, __ldg(a.qg + c + 1) + 1.f, __ldg(a.qb + c + 1));
+    auto affine = [&](float z, int i) {
+      const float g = a.qk16 ? Elem<T>::ld(reinterpret_cast<const T*>(a.qg) + i) : __ldg(reinterpret_cast<const float*>(a.qg) + i);
+      const float b = a.qk16 ? Elem<T>::ld(reinterpret_cast<const T*>(a.qb) + i) : __ldg(reinterpret_cast<const float*>(a.qb) + i);
+      return fmaf(z, g + 1.f, b);
+    };
+    const float qa = affine(u, c), qb = affine(v, c + 1);
     qs[c] = qa * w.x - qb * w.y;
     qs[c + 1] = qa * w.y + qb * w.x;
     if (owner) {
-      const float ka = round_to<T>(fmaf(u, __ldg(a.qg + S + c) + 1.f, __ldg(a.qb + S + c)));
-      const float kb = round_to<T>(fmaf(v, __ldg(a.qg + S + c + 1) + 1.f, __ldg(a.qb + S + c + 1)));
+      const float ka = round_to<T>(affine(u, S + c)), kb = round_to<T>(affine(v, S + c + 1));
       const size_t at = ((size_t)b * a.cap + a.pos) * S + c;
       Elem<T>::st(reinterpret_cast<T*>(a.keys) + at, ka);
       Elem<T>::st(reinterpret_cast<T*>(a.keys) + at + 1, kb);
@@ -388,7 +394,7 @@ extern "C" int mega_block_step(const mega_block_step_args* p, mega_stream_t stre
       !p->p || !p->q || !p->gamma_hat || !p->omega || !p->h || !p->v_weight || !p->v_bias || !p->mx_weight || !p->mx_bias ||
       !p->h_weight || !p->qk_gamma || !p->qk_beta || !p->rot || !p->keys || !p->keys_rot || !p->values || !p->work)
     return MEGA_ERR_NULL;
-  if (p->dtype != MEGA_BF16 && p->dtype != MEGA_F16) return MEGA_ERR_DTYPE;
+  if ((p->dtype != MEGA_BF16 && p->dtype != MEGA_F16) || (p->qk_dtype != MEGA_F32 && p->qk_dtype != p->dtype)) return MEGA_ERR_DTYPE;
   const int B = p->batch, D = p->embed, S = p->zdim, E = p->hdim;
   if (B <= 0 || D <= 0 || S <= 0 || E <= 0 || p->pos < 0 || p->pos >= p->cap || p->pos >= p->positions) return MEGA_ERR_SHAPE;
   // whole MMA tiles; a key is 8, 16 or 32 lanes of 16 bytes; the activations of a block fit its shared memory
@@ -414,7 +420,7 @@ extern "C" int mega_block_step(const mega_block_step_args* p, mega_stream_t stre
   a.scores = (float*)take((size_t)B * p->cap * 4);
   a.x = p->x; a.xn = xn; a.mx = mx; a.out = p->out;
   a.vw = p->v_weight; a.vb = p->v_bias; a.mw = p->mx_weight; a.mb = p->mx_bias; a.hw = p->h_weight;
-  a.qg = p->qk_gamma; a.qb = p->qk_beta; a.rot = p->rot; a.qk_eps = (float)p->qk_eps;
+  a.qg = p->qk_gamma; a.qb = p->qk_beta; a.qk16 = p->qk_dtype != MEGA_F32; a.rot = p->rot; a.qk_eps = (float)p->qk_eps;
   a.keys = p->keys; a.krot = p->keys_rot; a.values = p->values; a.cap = p->cap; a.pos = p->pos;
   const bool ok =
       p->complex_poles

@@ -993,7 +993,8 @@ std::tuple<Tensor, Tensor, Tensor> block_infer(Tensor x, Tensor xn, Tensor mx, c
   const Tensor base = at::addmm(bm, mx2, wm.t());
   char* bp = static_cast<char*>(base.data_ptr());
   char *u = bp, *z = bp + d * es, *r = z + s * es, *hx = r + e * es;
-  const Tensor ga = f32c(gamma), be = f32c(beta);
+  const auto affine = f32_all({gamma, beta}, w.stream);
+  const Tensor &ga = affine[0], &be = affine[1];
   Tensor q = at::empty({nb, pitch, s}, x.options()), k = fresh(q), raw;
   if (cache) raw = at::empty({bsz, seq, s}, x.options());
   check(mega_gate_qk_rotary_cache(z, f, fptr(ga), fptr(be), fptr(rot), (int)rot.size(0), (int)period, 0, (int)pitch, q.data_ptr(), s,

@@ -13,9 +13,8 @@ import torch
 from torch import Tensor
 
 from .. import _lib, ops
-from ..block_function import qk_affine
 from ..ops import _raw_stream
-from .fused import _fp32_params, _param_names, _seed_decode_state
+from .fused import _ema_params, _param_names, _seed_decode_state
 
 _POLES = {False: (4, 8, 16, 32), True: (2, 4, 8, 16, 32)}
 
@@ -41,6 +40,8 @@ def applicable(blk, x) -> bool:
             and (chunk < 0 or chunk > 1) and x.dtype in (torch.bfloat16, torch.float16)
             and all(w is not None and w.dtype == x.dtype and w.is_cuda and w.is_contiguous() and w.data_ptr() % 16 == 0
                     for w in weights)
+            and blk.gamma.dtype == blk.beta.dtype and blk.gamma.dtype in (torch.float32, x.dtype)
+            and blk.gamma.is_contiguous() and blk.beta.is_contiguous()
             and x.size(0) <= 64 and blk.zdim in (64, 128, 256) and blk.embed_dim % 32 == 0 and blk.hdim % 32 == 0
             and x.size(0) * (max(blk.embed_dim, blk.hdim) * 2 + 64) <= 200 * 1024)
 
@@ -102,8 +103,8 @@ def _build(blk, x, stream, incremental_state):
                 dt, bsz, n, blk.zdim, blk.hdim, keys.data_ptr(), keys_rot.data_ptr(), values.data_ptr(), cap,
                 stream), "block_cache_fill")
         work = torch.empty(lib.mega_block_step_work(dt, bsz, dim, blk.zdim, blk.hdim, cap), dtype=torch.uint8, device=dev)
-    qk = qk_affine(blk)
-    gamma_eff, beta, p, q, g, omega = _fp32_params(norm, move)
+    gamma_eff, beta = ops.norm_prepare(norm.weight, norm.bias)
+    p, q, g, omega = _ema_params(move)
     args = _lib.BlockStepArgs(
         dtype=dt, batch=bsz, embed=dim, zdim=blk.zdim, hdim=blk.hdim, ndim=move.ndim, complex_poles=int(move.complex),
         positions=rot.size(0), count=count.data_ptr(), count_next=count_next.data_ptr(),
@@ -111,13 +112,14 @@ def _build(blk, x, stream, incremental_state):
         norm_beta=beta.data_ptr(), p=p.data_ptr(), q=q.data_ptr(), gamma_hat=g.data_ptr(), omega=omega.data_ptr(),
         v_weight=blk.v_proj.weight.data_ptr(), v_bias=blk.v_proj.bias.data_ptr(),
         mx_weight=blk.mx_proj.weight.data_ptr(), mx_bias=blk.mx_proj.bias.data_ptr(),
-        h_weight=blk.h_proj.weight.data_ptr(), qk_gamma=qk[0].data_ptr(), qk_beta=qk[1].data_ptr(),
+        h_weight=blk.h_proj.weight.data_ptr(), qk_gamma=blk.gamma.data_ptr(), qk_beta=blk.beta.data_ptr(),
         rot=rot.data_ptr(), keys=keys.data_ptr(), keys_rot=keys_rot.data_ptr(), values=values.data_ptr(),
-        work=work.data_ptr(), norm_eps=norm.eps, qk_eps=1e-5, cap=cap, pos=n)
+        work=work.data_ptr(), norm_eps=norm.eps, qk_eps=1e-5, cap=cap, pos=n,
+        qk_dtype=ops._dt(blk.gamma))
     names = _names(blk)
     owners = [blk] + [blk._modules[m] for m in _SUBMODULES]
     blk._block_plan = _lib.host().BlockPlan(
         bytes(args), owners, list(_SUBMODULES), names, [owners[i]._parameters[name] for i, name in names], [nkey, ekey, akey],
-        [count, count_next, mean, var, h, k, v], keys, values, [keys_rot, work, rot, qk, gamma_eff, beta, p, q, g, omega],
+        [count, count_next, mean, var, h, k, v], keys, values, [keys_rot, work, rot, gamma_eff, beta, p, q, g, omega],
         chunk, x, stream)
     return True

@@ -78,13 +78,18 @@ class MultiHeadComplexEMA(IncrementalStateMixin, nn.Module):
             self.gamma[:, :, 1] = 0.
             nn.init.normal_(self.omega, mean=0.0, std=1.0)
 
-    def train(self, mode=True):
+    def _forget(self):
+        """What was made of the parameters: only valid while they are frozen."""
         self._coeffs = None
+        for name in ("_decode_cache", "_step_plan"):
+            self.__dict__.pop(name, None)
+
+    def train(self, mode=True):
+        self._forget()
         return super().train(mode)
 
     def _apply(self, fn, *args, **kwargs):
-        self._coeffs = None
-        self.__dict__.pop("_decode_cache", None)
+        self._forget()
         return super()._apply(fn, *args, **kwargs)
 
     # -- coefficients / kernel -----------------------------------------------------------

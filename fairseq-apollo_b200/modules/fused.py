@@ -9,6 +9,7 @@ from torch import Tensor
 
 from .. import _lib, ops
 from ..functions import needs_grad
+from ..ops import _raw_stream
 from .exponential_moving_average import MultiHeadEMA
 from .sequence_norm import SequenceNorm
 from .timestep_norm import TimestepNorm
@@ -45,10 +46,8 @@ def timestep_norm_ema(norm: TimestepNorm, move: MultiHeadEMA, x: Tensor,
             and (not move.complex or move.ndim in (2, 4, 8, 16, 32))):
         with torch.no_grad():
             return _decode_step(norm, move, x, incremental_state, activation, return_normed)
-    # coefficients, effective scale and priors come from what the parameters were laid out to once (rebuilt when a
-    # version counter moves), not from kernel launches per call
-    gamma_eff, beta, p, q, g, omega = _fp32_params(norm, move)
-    _, _, prev_count, prev_mean, prev_var, nstate = norm.operands(x.size(0), incremental_state)
+    p, q, g, omega = _ema_params(move)
+    gamma_eff, beta, prev_count, prev_mean, prev_var, nstate = norm.operands(x.size(0), incremental_state)
     h_in = None
     estate = None
     if incremental_state is not None:
@@ -90,27 +89,27 @@ def sequence_norm_ema(norm: SequenceNorm, move: MultiHeadEMA, x: Tensor, padding
     return move(norm(x, padding_mask), padding_mask, None, activation)
 
 
-def _fp32_params(norm: TimestepNorm, move: MultiHeadEMA):
-    """fp32, contiguous copies of everything the decode kernel reads, cached until a parameter
-    is modified (checked through the tensors' version counters)."""
+def _ema_params(move: MultiHeadEMA):
+    """(p, q, gamma, omega) of the layer, fp32 and contiguous.  Outside of training they are kept until a parameter
+    changes (identity, version counter, storage), the layer is moved or its mode is set; never across streams, nor from a
+    call that is only being captured."""
     third = move.theta if move.complex else move.beta
-    tensors = (norm.weight, norm.bias, move.alpha, move.delta, third, move.gamma, move.omega)
-    # (in-place updates bump the version counters; a parameter that was replaced has a new identity)
-    key = (norm.weight._version, norm.bias._version, move.alpha._version, move.delta._version, third._version,
-           move.gamma._version, move.omega._version)
-    cache = getattr(move, "_decode_cache", None)
-    if cache is not None and (cache[0] != key or any(a is not b for a, b in zip(cache[-1], tensors))):
-        cache = None
-    if cache is None:
-        if move.complex:   # q, g complex64 (K, N): the kernel reads them as interleaved (re, im) floats
-            p, q, g = ops.cema_coeffs(move.alpha, move.delta, move.theta, move.gamma)
-            p, q, g = p.reshape(p.shape[0], -1).contiguous(), q.reshape(q.shape[0], -1).contiguous(), g.contiguous()
-        else:
-            p, q, g = ops.ema_coeffs(move.alpha, move.delta, move.beta, move.gamma)
-        cache = (key, (norm.weight.detach().float() + 1.0).contiguous(), norm.bias.detach().float().contiguous(),
-                 p, q, g, move.omega.detach().float().reshape(-1).contiguous(), tensors)
-        move._decode_cache = cache
-    return cache[1:7]
+    tensors = (move.alpha, move.delta, third, move.gamma, move.omega)
+    key = None
+    if not move.training:
+        key = [_raw_stream(move.alpha.get_device())] + [t._version for t in tensors] + [t.data_ptr() for t in tensors]
+        cache = move.__dict__.get("_decode_cache")
+        if cache is not None and cache[0] == key and all(a is b for a, b in zip(cache[2], tensors)):
+            return cache[1]
+    if move.complex:   # q, g complex64 (K, N): the kernel reads them as interleaved (re, im) floats
+        p, q, g = ops.cema_coeffs(move.alpha, move.delta, move.theta, move.gamma)
+        p, q, g = p.reshape(p.shape[0], -1).contiguous(), q.reshape(q.shape[0], -1).contiguous(), g.contiguous()
+    else:
+        p, q, g = ops.ema_coeffs(move.alpha, move.delta, move.beta, move.gamma)
+    prm = (p, q, g, move.omega.detach().float().reshape(-1).contiguous())
+    if key is not None and not torch.cuda.is_current_stream_capturing():
+        move._decode_cache = (key, prm, tensors)
+    return prm
 
 
 def _param_names(move):
@@ -152,7 +151,8 @@ def _decode_step_plan(norm, move, x, incremental_state, activation, return_norme
         nstate['prev_count'] = count.long().contiguous()
         estate['prev_state'] = h.to(sdtype).contiguous()
         count, mean, var, h = nstate['prev_count'], nstate['prev_mean'], nstate['prev_var'], estate['prev_state']
-    gamma, beta, p, q, g, omega = _fp32_params(norm, move)
+    gamma, beta = ops.norm_prepare(norm.weight, norm.bias)
+    p, q, g, omega = _ema_params(move)
     move._step_plan = _lib.host().StepPlan(
         _param_names(move), _param_tensors(norm, move), nkey, ekey, norm.num_groups, activation,
         [count, torch.empty_like(count), mean, var, h], [gamma, beta, p, q, g, omega], x, move.complex, return_normed, norm.eps)

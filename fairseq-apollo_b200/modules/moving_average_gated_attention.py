@@ -178,6 +178,14 @@ class MovingAverageGatedAttention(IncrementalStateMixin, nn.Module):
         nn.init.constant_(self.gamma, 0.0)
         nn.init.constant_(self.beta, 0.0)
 
+    def train(self, mode=True):
+        self.__dict__.pop("_block_plan", None)
+        return super().train(mode)
+
+    def _apply(self, fn, *args, **kwargs):
+        self.__dict__.pop("_block_plan", None)
+        return super()._apply(fn, *args, **kwargs)
+
     # ------------------------------------------------------------------ attention weights
     def _scores(self, q, k):
         """Rotary positions or the learned relative bias applied, raw scores (B*K, Cq, Ck)."""

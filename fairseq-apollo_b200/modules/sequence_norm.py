@@ -27,27 +27,13 @@ class SequenceNorm(nn.Module):
                 length_last: bool = True) -> torch.Tensor:
         if needs_grad(x, self.weight, self.bias):
             return sequence_norm(x, self.weight, self.bias, padding_mask, self.eps, length_last, self.num_groups)
-        gamma, beta = ops.norm_prepare(self.weight, self.bias)
+        gamma, beta = self.operands()
         y, _, _, _ = ops.sequence_norm_fwd(x, gamma, beta, padding_mask, self.eps, length_last, self.num_groups)
         return y
 
     def operands(self):
-        """(gamma = weight + 1, beta) fp32 for the fused norm -> EMA path, laid out once until a parameter changes
-        (identity, storage, version counter)."""
-        ps = (self.weight, self.bias)
-        key = [p._version for p in ps] + [p.data_ptr() for p in ps]
-        cache = self.__dict__.get("_prep")
-        if cache is None or cache[0] != key or cache[1][0] is not ps[0] or cache[1][1] is not ps[1]:
-            cache = self.__dict__["_prep"] = (key, ps, ops.norm_prepare(*ps))
-        return cache[2]
-
-    def train(self, mode=True):
-        self.__dict__.pop("_prep", None)
-        return super().train(mode)
-
-    def _apply(self, fn, *args, **kwargs):
-        self.__dict__.pop("_prep", None)
-        return super()._apply(fn, *args, **kwargs)
+        """(gamma = weight + 1, beta) fp32 for the fused norm -> EMA path."""
+        return ops.norm_prepare(self.weight, self.bias)
 
     def extra_repr(self) -> str:
         return 'num_features={num_features}, num_groups={num_groups}, eps={eps}'.format(**self.__dict__)

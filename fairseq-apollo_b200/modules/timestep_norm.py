@@ -83,43 +83,26 @@ class TimestepNorm(IncrementalStateMixin, nn.Module):
                 raise NotImplementedError("the incremental state is an inference feature: use torch.no_grad()")
             return timestep_norm(x, self.prior_count, self.prior_mean, self.prior_logv, self.weight, self.bias, padding_mask,
                                  groups, self.eps)
-        gamma, beta, prev_count, prev_mean, prev_var, saved_state = self.operands(x.size(0), incremental_state, keep=False)
+        gamma, beta, prev_count, prev_mean, prev_var, saved_state = self.operands(x.size(0), incremental_state)
         out, count, mean, var = ops.timestep_norm_fwd(x, prev_count, prev_mean, prev_var, gamma, beta,
                                                       padding_mask, self.eps, groups)
         self.store_statistics(incremental_state, saved_state, count, mean, var)
         return out
 
-    def operands(self, batch_size, incremental_state=None, keep=True):
+    def operands(self, batch_size, incremental_state=None):
         """What an inference call hands to the operator: (gamma, beta) fp32, the incoming statistics and the saved
-        state or None.  With ``keep`` the parameters are laid out once until one of them changes (identity, storage,
-        version counter), as the fused norm -> EMA path does with the EMA's coefficients; what comes back may then be
-        shared with other calls: it is read, never written."""
+        state or None.  One launch on the parameters as they are: nothing is kept from call to call (a parameter written
+        through ``p.data`` moves no version counter)."""
         saved_state = None
         if incremental_state is not None:
             saved_state = self._get_input_buffer(incremental_state)
-        gamma, beta, count, mean, var = self._prepared(batch_size, keep)
         if saved_state is not None and 'prev_mean' in saved_state:
+            gamma, beta = ops.norm_prepare(self.weight, self.bias)
             count, mean, var = saved_state['prev_count'], saved_state['prev_mean'], saved_state['prev_var']
+        else:
+            gamma, beta, count, mean, var = ops.norm_prepare(self.weight, self.bias,
+                                                             (self.prior_count, self.prior_mean, self.prior_logv), batch_size)
         return gamma, beta, count, mean, var, saved_state
-
-    def _prepared(self, batch_size, keep):
-        ps = (self.prior_count, self.prior_mean, self.prior_logv, self.weight, self.bias)
-        key = [batch_size] + [p._version for p in ps] + [p.data_ptr() for p in ps] if keep else None
-        cache = self.__dict__.get("_prep")
-        if not keep or cache is None or cache[0] != key or any(a is not b for a, b in zip(cache[1], ps)):
-            prep = ops.norm_prepare(self.weight, self.bias, ps[:3], batch_size)
-            if not keep:
-                return prep
-            cache = self.__dict__["_prep"] = (key, ps, prep)
-        return cache[2]
-
-    def train(self, mode=True):
-        self.__dict__.pop("_prep", None)
-        return super().train(mode)
-
-    def _apply(self, fn, *args, **kwargs):
-        self.__dict__.pop("_prep", None)
-        return super()._apply(fn, *args, **kwargs)
 
     def _get_input_buffer(self, incremental_state):
         result = self.get_incremental_state(incremental_state, "norm_state")

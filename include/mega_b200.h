@@ -576,7 +576,7 @@ MEGA_API int mega_attention_bias_grad(const void* ds, float* dbias, int span, in
  * out = x + sigmoid(u) * (SiLU(hx + h_proj(attn * SiLU(r))) - x).
  * keys (batch, cap, zdim) receives the key before the rotary embedding, keys_rot after it, values
  * (batch, cap, hdim) SiLU(v), each at row `pos`; rows 0 .. pos - 1 are read.  Weights are row-major (out, in) in
- * `dtype` (bf16 or fp16), biases too, the rest fp32; rot as in mega_gate_qk_rotary with `positions` rows.
+ * `dtype` (bf16 or fp16), biases too, the query / key affine in qk_dtype, the rest fp32; rot as in mega_gate_qk_rotary with `positions` rows.
  * work: mega_block_step_work bytes, 16-byte aligned like every activation and weight pointer.
  * MEGA_ERR_UNSUPPORTED: batch > 64, embed or hdim not a multiple of 32, zdim other than 64, 128, 256, pole counts
  * mega_tsn_ema_step's fast form does not take, activations beyond a block's shared memory.
@@ -594,11 +594,12 @@ typedef struct mega_block_step_args {
   float *mean, *var, *h;
   const float *norm_gamma, *norm_beta, *p, *q, *gamma_hat, *omega;
   const void *v_weight, *v_bias, *mx_weight, *mx_bias, *h_weight;
-  const float *qk_gamma, *qk_beta, *rot;
+  const void *qk_gamma, *qk_beta; /* (2, zdim) in qk_dtype: MEGA_F32 or `dtype` */
+  const float* rot;
   void *keys, *keys_rot, *values, *work;
   double norm_eps, qk_eps;
   int64_t cap;
-  int32_t pos;
+  int32_t pos, qk_dtype;
 } mega_block_step_args;
 MEGA_API int64_t mega_block_step_work(int dtype, int batch, int embed, int zdim, int hdim, int64_t cap);
 MEGA_API int mega_block_step(const mega_block_step_args* args, mega_stream_t stream);

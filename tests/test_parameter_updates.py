@@ -1,0 +1,86 @@
+"""Parameters that change between calls: written through ``p.data`` (no version counter moves), given new storage, replaced;
+and what a generation keeps while it runs and after it."""
+import copy
+import gc
+
+import pytest
+import torch
+
+from _util import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+def _block(M, cplx=False, dim=64, chunk=64, **kw):
+    torch.manual_seed(11)
+    args = dict(efficient_attn=True, rel_pos_bias='rotary')
+    args.update(kw)
+    blk = M.MovingAverageGatedAttention(dim, 64, 2 * dim, 16, chunk_size=chunk, moving_layer='cema' if cplx else 'ema',
+                                        moving_act='silu', **args)
+    return _other(blk).cuda().bfloat16().eval()
+
+
+def _other(module, seed=12):
+    """New values for every parameter, written behind autograd's back."""
+    gen = torch.Generator().manual_seed(seed)
+    for p in module.parameters():
+        p.data.copy_((torch.randn(p.shape, generator=gen) * (0.5 if p.dim() != 2 else 0.1)).to(p.device))
+    return module
+
+
+def _fresh(module):
+    """The module with its present parameters and nothing else."""
+    new = copy.deepcopy(module)
+    for m in new.modules():
+        for name in ("_coeffs", "_decode_cache", "_step_plan", "_block_plan", "_qk_fp32", "_prep"):
+            if m.__dict__.get(name) is not None:
+                m.__dict__[name] = None
+    return new
+
+
+def _generate(blk, x, inc=None):
+    inc = {} if inc is None else inc
+    return torch.cat([blk(x[:, :5].contiguous(), incremental_state=inc)[0]]
+                     + [blk(x[:, t:t + 1].contiguous(), incremental_state=inc)[0] for t in range(5, x.size(1))], 1)
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("call", ["block", "generate", "norm_ema", "step"])
+def test_writes_between_evaluations(cplx, call):
+    """Evaluate, train with an optimiser that writes through p.data, evaluate again."""
+    import fairseq_apollo_b200 as M
+    blk = _block(M, cplx)
+    x = torch.randn(2, 12, 64, device="cuda").bfloat16()
+
+    def run(b):
+        with torch.no_grad():
+            if call == "block":
+                return b(x)[0]
+            if call == "generate":
+                return _generate(b, x)
+            if call == "norm_ema":
+                return torch.cat(M.timestep_norm_ema(b.norm, b.move, x, None, {}, "silu", True))
+            inc = {}
+            return torch.cat([M.timestep_norm_ema(b.norm, b.move, x[:, t:t + 1].contiguous(), None, inc) for t in range(3)])
+
+    first = run(blk)
+    blk.train()
+    _other(blk, 13)
+    blk.eval()
+    second = run(blk)
+    assert torch.equal(second, run(_fresh(blk)))
+    assert rel_l2(second, first) > 0.1
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+def test_query_key_affine_and_norm_are_read_on_each_call(cplx):
+    """Without train() in between: the block's own affine parameters are read when they are used."""
+    import fairseq_apollo_b200 as M
+    blk = _block(M, cplx)
+    x = torch.randn(2, 64, 64, device="cuda").bfloat16()
+    with torch.no_grad():
+        blk(x)
+        own = [blk.gamma, blk.beta] + ([blk.norm.weight] if cplx else [])
+        for p in own:
+            p.data.mul_(-1.5).add_(0.25)
+        assert torch.equal(blk(x)[0], _fresh(blk)(x)[0])
