@@ -4,15 +4,18 @@
 // A CTA keeps rows (batch, channel) in shared memory (fp32) and cuts each into segments of 32 positions, which turns the
 // layer into three products with matrices of the channel, S the number of segments:
 //   local pole states   H = X V      X (S, 32) the row, V (32, poles): q^(31-k), anti-causal q^k
-//   outputs             Y = X T + C E   T (32, 32) the taps between positions of a segment, both directions at once and
-//                                    omega on its diagonal; C (S, poles) the states that enter a segment, E (poles, 32)
+//   outputs             Y = X T + C E   T (32, 32) the taps between positions of a segment, both directions at once;
+//                                    C (S, poles) the states that enter a segment, E (poles, 32)
+// omega x is added in fp32 beside them.
 // and a scan of the S states per pole (C from H): the run that a lane holds, lanes by shuffles, warps through a table.
 // 96 multiply-adds per element bidirectional, 64 causal.  HBM sees the row once in, once out.
 //
 // fp32 on the bf16 tensor pipe: a float is exactly the sum of three bf16 values, and six of the nine products (all
-// but those below 2^-24 of the largest) are accumulated in fp32, the leading one last.  That is 576 bf16 products per
-// element where the packed FMA pipe, at an eleventh of the rate, would spend 96 slots.  Against the float64 recurrence
-// the result is as close as that of the fp32 walk it replaces (1e-7).
+// but those below 2^-24 of the largest) are accumulated in fp32.  That is 576 bf16 products per element where the packed
+// FMA pipe, at an eleventh of the rate, would spend 96 slots.  The tensor pipe truncates its sums, so what would be large
+// in them stays out: omega x, usually the larger part of an output, and every tile's leading products have fp32 additions
+// of their own.  Against the float64 recurrence: 1.0e-7 bidirectional, 6.1e-8 causal (the fp32 walk: 1.1e-7 and 6.7e-8;
+// omega on T's diagonal, one accumulator and taps summed in fp32: 1.3e-7 and 8.0e-8).
 //
 // B = 32, D = 256, L = 16384 fp32 bidirectional after the norm: 1310 us as a walk (FMA, one row per SM), 590 us now (650
 // padded by up to half): the tensor pipe is at 45 %, issue slots at 40 %, the rest is latency, 16 warps being what the
@@ -78,8 +81,8 @@ __device__ __forceinline__ Frag load_frag(const unsigned char* block) {
   const int lane = threadIdx.x & 31;
   return {*reinterpret_cast<const uint4*>(block + lane * 16), *reinterpret_cast<const uint2*>(block + 512 + lane * 8)};
 }
-// d = products of K reduction tiles, all but those of the leading parts, smallest first, then those: the tensor pipe
-// truncates its sums, and this leaves the large ones for the end.  Block of tile k at block + k * stride.
+// d = products of K reduction tiles, all but those of the leading parts, smallest first, then those, each tile's on its own:
+// the tensor pipe truncates its sums, the additions here round.  Block of tile k at block + k * stride.
 template <int K>
 __device__ __forceinline__ void products(float (&d)[4], const uint32_t (&a)[K][3][4], const unsigned char* block, int stride) {
   d[0] = d[1] = d[2] = d[3] = 0.f;
@@ -95,7 +98,10 @@ __device__ __forceinline__ void products(float (&d)[4], const uint32_t (&a)[K][3
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     const uint2 b = *reinterpret_cast<const uint2*>(block + k * stride + (threadIdx.x & 31) * 16);
-    mma(d, a[k][0], b.x, b.y);
+    float l[4] = {0.f, 0.f, 0.f, 0.f};
+    mma(l, a[k][0], b.x, b.y);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) d[i] += l[i];
   }
 }
 // zero where the mask's bits say so
@@ -148,13 +154,24 @@ __device__ __forceinline__ void prepare_channel(const RowArgs& a, int d, int per
   const bool live = n < a.N && (kBidir || lane < 16);
   const size_t at = (size_t)(d + (lane < 16 ? 0 : a.D)) * a.N + n;
   const float q = live ? __ldg(a.q + at) : 0.f;
-  const float c = live ? __ldg(a.p + at) * __ldg(a.g + at) : 0.f;
+  const double c = live ? (double)__ldg(a.p + at) * __ldg(a.g + at) : 0.;
+  for (int l = tid; l < 31; l += blockDim.x)
+    if (!kBidir) tap[l] = 0.f;
   {
-    double step = 1., v = 1.;   // (few enough to keep their roundings out of the result)
+    // (in double, rounded once: few enough to keep their roundings out of the result; the poles' shares of a tap alternate
+    // in sign.  Lanes 0 - 15 sum those of the causal half, the others those of the anti-causal one)
+    double step = 1., v = 1.;
     for (int i = 0; i < nw; ++i) step *= q;
     for (int i = 0; i < w; ++i) v *= q;
     for (int k = w; k <= 32; k += nw) {
       pw[k * 32 + lane] = (float)v;
+      double t = c * v;
+#pragma unroll
+      for (int s = 8; s > 0; s >>= 1) t += __shfl_xor_sync(0xffffffffu, t, s);
+      const int back = a.shift ? k + 1 : k;   // lag of the anti-causal half
+      if (kBidir && back == 0) t += __shfl_xor_sync(0xffffffffu, t, 16);
+      if (lane == 0 && k < 32) tap[31 + k] = (float)t;
+      if (kBidir && lane == 16 && back > 0 && back < 32) tap[31 - back] = (float)t;
       v *= step;
     }
   }
@@ -171,20 +188,6 @@ __device__ __forceinline__ void prepare_channel(const RowArgs& a, int d, int per
       v *= r;
     }
   }
-  // taps: one warp takes a lag, its lanes the poles
-  for (int l = w; l < 63; l += nw) {
-    const int lag = l - 31;
-    float v = 0.f;
-    if (lag >= 0) v = lane < 16 ? c * pw[lag * 32 + lane] : 0.f;
-    if (kBidir && lane >= 16) {
-      const int k = a.shift ? -lag - 1 : -lag;
-      if (k >= 0) v = c * pw[k * 32 + lane];
-    }
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) v += __shfl_xor_sync(0xffffffffu, v, s);
-    if (lane == 0) tap[l] = lag == 0 ? v + __ldg(a.omega + d) : v;
-  }
-  __syncthreads();
   constexpr int kStateTiles = kBidir ? 4 : 2, kStateK = kBidir ? 2 : 1;
   constexpr int kV = 2 * kStateTiles, kT = 8, kE = 4 * kStateK;
   for (int e = tid; e < (kV + kT + kE) * 32; e += blockDim.x) {
@@ -203,8 +206,8 @@ __device__ __forceinline__ void prepare_channel(const RowArgs& a, int d, int per
         const int kt = (blk - kV - kT) >> 2, nt = (blk - kV - kT) & 3, pole = 16 * kt + k, pos = column_pos(nt, g);
         const int m = pole & 15;
         const size_t row = (size_t)(d + (pole < 16 ? 0 : a.D)) * a.N + m;
-        const float cp = m < a.N ? __ldg(a.p + row) * __ldg(a.g + row) : 0.f;
-        v[i] = cp * pw[(pole < 16 ? pos + 1 : (a.shift ? 31 : 32) - pos) * 32 + pole];
+        const double cp = m < a.N ? (double)__ldg(a.p + row) * __ldg(a.g + row) : 0.;
+        v[i] = (float)(cp * pw[(pole < 16 ? pos + 1 : (a.shift ? 31 : 32) - pos) * 32 + pole]);
       }
     }
     uint32_t lo[3], hi[3];
@@ -518,6 +521,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) rowres_kernel(RowArgs a) {
     // ---- 16 segments at a time: local states (column tile nt, rows g (st[..][nt][0, 1]) and g + 8 (2, 3), columns
     // 8 nt + 2 t, + 1), and the outputs of the inputs themselves in the inputs' place
     float st[kGroups][kStateTiles][4];
+    const float om = __ldg(a.omega + d);
     if (live) {
 #pragma unroll
       for (int gr = 0; gr < kGroups; ++gr) {
@@ -531,9 +535,13 @@ __global__ void __launch_bounds__(kMaxThreads, 1) rowres_kernel(RowArgs a) {
           products<2>(y[0], f, ft + 2 * half * kBlockBytes, 4 * kBlockBytes);
           products<2>(y[1], f, ft + (2 * half + 1) * kBlockBytes, 4 * kBlockBytes);
 #pragma unroll
-          for (int h = 0; h < 2; ++h)
-            *reinterpret_cast<float4*>(xs + 4 * piece(seg_of(gr, h), 4 * half + t, rs)) =
-                make_float4(y[0][2 * h], y[0][2 * h + 1], y[1][2 * h], y[1][2 * h + 1]);
+          for (int h = 0; h < 2; ++h) {
+            float4* at = reinterpret_cast<float4*>(xs + 4 * piece(seg_of(gr, h), 4 * half + t, rs));
+            float4 v = *at;
+            if (kNorm) v = make_float4(fmaf(v.x, sc, sh), fmaf(v.y, sc, sh), fmaf(v.z, sc, sh), fmaf(v.w, sc, sh));
+            *at = make_float4(fmaf(om, v.x, y[0][2 * h]), fmaf(om, v.y, y[0][2 * h + 1]), fmaf(om, v.z, y[1][2 * h]),
+                              fmaf(om, v.w, y[1][2 * h + 1]));
+          }
         }
 #pragma unroll
         for (int nt = 0; nt < kStateTiles; ++nt) products<2>(st[gr][nt], f, fv + nt * kBlockBytes, kStateTiles * kBlockBytes);
@@ -623,7 +631,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) rowres_kernel(RowArgs a) {
       }
     }
     __syncwarp();
-    if (row) store_row<T, !kNorm, rs>(xs, mk, any, L, base, kNorm ? 0.f : __ldg(a.omega + d), a.silu, xg, yg);
+    if (row) store_row<T, !kNorm, rs>(xs, mk, any, L, base, om, a.silu, xg, yg);
   }
 }
 
