@@ -1020,7 +1020,7 @@ Tensor block_train(const Tensor& x, const Tensor& xn, const Tensor& mx, const Te
 // and the same library call took 6.6 us through the interpreter and ctypes, 2 us here.
 //
 // A plan is everything a step passes to the library, and what it was built from: it holds as long as the parameters
-// (identity and version counters), the state tensors, the batch, the dtype and the options stay what they were.  The
+// (identity, version counters and storage: p.data = t, which is also how a module is moved, leaves the first two alone), the state tensors, the batch, the dtype and the options stay what they were.  The
 // state tensors are updated in place, except the counts: one array is read, another written, and they alternate.
 struct Names {
   PyObject *params, *modules, *groups, *bidirectional, *plan, *block_plan, *count, *mean, *var, *h, *key, *value, *key_mask;
@@ -1037,9 +1037,20 @@ const Names& names() {
   return *n;
 }
 
+int64_t version_of(const Tensor& t) { return (int64_t)t.unsafeGetTensorImpl()->version_counter().current_version(); }
+
+// A parameter as it was when a plan was built; its storage stays as long as the plan, which may hold its address.
+struct Mark {
+  int64_t version;
+  const void* at;
+  c10::Storage storage;
+  explicit Mark(const Tensor& t) : version(version_of(t)), at(t.data_ptr()), storage(t.storage()) {}
+  bool holds(const Tensor& t) const { return version_of(t) == version && t.data_ptr() == at; }
+};
+
 struct StepPlan {
   std::vector<py::object> names, params;   // two of the norm, five of the layer
-  std::vector<int64_t> versions;
+  std::vector<Mark> marks;
   py::object nkey, ekey, groups, activation;
   py::object count, count_next, mean, var, h;
   std::vector<Tensor> operands;            // gamma, beta, p, q, g, omega (fp32)
@@ -1049,15 +1060,13 @@ struct StepPlan {
   double eps;
 };
 
-int64_t version_of(const Tensor& t) { return (int64_t)t.unsafeGetTensorImpl()->version_counter().current_version(); }
-
 std::unique_ptr<StepPlan> step_plan(std::vector<py::object> names, std::vector<py::object> params, py::object nkey, py::object ekey,
                                     py::object groups, py::object activation, std::vector<py::object> state,
                                     std::vector<Tensor> operands, const Tensor& x, bool cplx, bool normed, double eps) {
   auto p = std::make_unique<StepPlan>();
   p->names = std::move(names);
   p->params = std::move(params);
-  for (auto& t : p->params) p->versions.push_back(version_of(THPVariable_Unpack(t.ptr())));
+  for (auto& t : p->params) p->marks.emplace_back(THPVariable_Unpack(t.ptr()));
   p->nkey = std::move(nkey); p->ekey = std::move(ekey); p->groups = std::move(groups); p->activation = std::move(activation);
   p->count = state[0]; p->count_next = state[1]; p->mean = state[2]; p->var = state[3]; p->h = state[4];
   p->count_t = THPVariable_Unpack(p->count.ptr()); p->next_t = THPVariable_Unpack(p->count_next.ptr());
@@ -1072,7 +1081,7 @@ std::unique_ptr<StepPlan> step_plan(std::vector<py::object> names, std::vector<p
 bool params_match(const StepPlan& p, PyObject* dict, size_t from, size_t to) {
   for (size_t i = from; i < to; ++i) {
     PyObject* t = PyDict_GetItemWithError(dict, p.names[i].ptr());
-    if (t != p.params[i].ptr() || version_of(THPVariable_Unpack(t)) != p.versions[i]) return false;
+    if (t != p.params[i].ptr() || !p.marks[i].holds(THPVariable_Unpack(t))) return false;
   }
   return true;
 }
@@ -1146,7 +1155,7 @@ struct BlockPlan {
   py::object owners[5];                    // norm, move, v_proj, mx_proj, h_proj
   std::vector<std::pair<int, py::object>> names;   // of a parameter: owner (0: the block, 1 ...: the above), key
   std::vector<py::object> params;
-  std::vector<int64_t> versions;
+  std::vector<Mark> marks;
   py::object submodules[5];                // the owners' keys
   py::object nkey, ekey, akey;
   py::object count, count_next, mean, var, h, last_key, last_value;
@@ -1173,7 +1182,7 @@ std::unique_ptr<BlockPlan> block_plan(py::bytes args, std::vector<py::object> ow
   for (int i = 0; i < 5; ++i) p->submodules[i] = word(submodules[i]);
   for (auto& n : names) p->names.emplace_back(n.first, word(n.second));
   p->params = std::move(params);
-  for (auto& t : p->params) p->versions.push_back(version_of(THPVariable_Unpack(t.ptr())));
+  for (auto& t : p->params) p->marks.emplace_back(THPVariable_Unpack(t.ptr()));
   p->nkey = state_keys[0]; p->ekey = state_keys[1]; p->akey = state_keys[2];
   p->count = state[0]; p->count_next = state[1]; p->mean = state[2]; p->var = state[3]; p->h = state[4];
   p->last_key = state[5]; p->last_value = state[6];
@@ -1219,7 +1228,7 @@ bool block_matches(const BlockPlan& p, PyObject* blk, PyObject* block_dict, cons
   }
   for (size_t i = 0; i < p.params.size(); ++i) {
     PyObject* t = PyDict_GetItemWithError(dicts[p.names[i].first].ptr(), p.names[i].second.ptr());
-    if (t != p.params[i].ptr() || version_of(THPVariable_Unpack(t)) != p.versions[i]) return false;
+    if (t != p.params[i].ptr() || !p.marks[i].holds(THPVariable_Unpack(t))) return false;
   }
   return true;
 }

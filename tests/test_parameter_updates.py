@@ -84,3 +84,35 @@ def test_query_key_affine_and_norm_are_read_on_each_call(cplx):
         for p in own:
             p.data.mul_(-1.5).add_(0.25)
         assert torch.equal(blk(x)[0], _fresh(blk)(x)[0])
+
+
+@pytest.mark.parametrize("how", ["data", "moved", "assigned", "in place"])
+def test_storage_replaced_during_a_generation(how):
+    import fairseq_apollo_b200 as M
+    blk = _block(M)
+    x = torch.randn(2, 8, 64, device="cuda").bfloat16()
+    ref = copy.deepcopy(blk).float()
+    a, b = {}, {}
+    got, want = [], []
+    with torch.no_grad():
+        for t in range(8):
+            if t == 4:
+                for m in (blk, ref):
+                    if how == "data":
+                        for p in m.parameters():
+                            p.data = p.data.clone() * 1.5
+                    elif how == "moved":
+                        for p in m.parameters():
+                            p.mul_(1.5)
+                        m.cpu()
+                        m.cuda()
+                    elif how == "assigned":
+                        m.v_proj.weight = torch.nn.Parameter(m.v_proj.weight * 1.5)
+                        m.h_proj = copy.deepcopy(m.h_proj)
+                    else:
+                        m.v_proj.weight.mul_(1.5)
+                junk = [torch.full_like(p, float("nan")) for p in blk.parameters()]   # (takes what was given back)
+            got.append(blk(x[:, t:t + 1].contiguous(), incremental_state=a)[0])
+            want.append(ref(x[:, t:t + 1].float().contiguous(), incremental_state=b)[0])
+    del junk
+    assert rel_l2(torch.cat(got, 1).float(), torch.cat(want, 1)) < 2e-2
