@@ -17,6 +17,7 @@
 
 #include <algorithm>
 #include <tuple>
+#include <unordered_map>
 #include <vector>
 
 #include "mega_b200.h"
@@ -1149,16 +1150,21 @@ PyObject* norm_ema_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 // ------------------------------------------------------------------------------------ single-token step of a block
 // Five launches of 3 - 6 us each: through the interpreter and ctypes a step took 31 us of host, more than the device.
+//
+// A plan belongs to a generation: to its running mean, a tensor that the steps update in place and that the state keeps
+// from the first to the last of them.  The block's plans are found by it, so generations that are answered in turn keep
+// theirs, and a plan goes, with the buffers of keys and values it holds, when the tensor does.
 struct BlockPlan {
   mega_block_step_args args;
-  PyObject* block;                         // (not owned: the plan lives in the block's dictionary)
+  PyObject* block;                         // (not owned: the plans live in the block's dictionary)
   py::object owners[5];                    // norm, move, v_proj, mx_proj, h_proj
   std::vector<std::pair<int, py::object>> names;   // of a parameter: owner (0: the block, 1 ...: the above), key
   std::vector<py::object> params;
   std::vector<Mark> marks;
   py::object submodules[5];                // the owners' keys
   py::object nkey, ekey, akey;
-  py::object count, count_next, mean, var, h, last_key, last_value;
+  PyObject* mean;                          // (not owned: the plan goes with it)
+  py::object count, count_next, var, h, last_key, last_value;
   Tensor keys, values;
   std::vector<py::object> keep;
   int64_t pos, chunk, batch, dim;
@@ -1167,12 +1173,12 @@ struct BlockPlan {
   at::ScalarType type;
 };
 
-std::unique_ptr<BlockPlan> block_plan(py::bytes args, std::vector<py::object> owners, std::vector<std::string> submodules,
+std::shared_ptr<BlockPlan> block_plan(py::bytes args, std::vector<py::object> owners, std::vector<std::string> submodules,
                                       std::vector<std::pair<int, std::string>> names, std::vector<py::object> params,
                                       std::vector<py::object> state_keys, std::vector<py::object> state, const Tensor& keys,
                                       const Tensor& values, std::vector<py::object> keep, int64_t chunk, const Tensor& x,
                                       uintptr_t stream) {
-  auto p = std::make_unique<BlockPlan>();
+  auto p = std::make_shared<BlockPlan>();
   const std::string raw = args;
   if (raw.size() != sizeof p->args || owners.size() != 6 || submodules.size() != 5) throw py::value_error("block_plan");
   memcpy(&p->args, raw.data(), raw.size());
@@ -1184,7 +1190,7 @@ std::unique_ptr<BlockPlan> block_plan(py::bytes args, std::vector<py::object> ow
   p->params = std::move(params);
   for (auto& t : p->params) p->marks.emplace_back(THPVariable_Unpack(t.ptr()));
   p->nkey = state_keys[0]; p->ekey = state_keys[1]; p->akey = state_keys[2];
-  p->count = state[0]; p->count_next = state[1]; p->mean = state[2]; p->var = state[3]; p->h = state[4];
+  p->count = state[0]; p->count_next = state[1]; p->mean = state[2].ptr(); p->var = state[3]; p->h = state[4];
   p->last_key = state[5]; p->last_value = state[6];
   p->keys = keys; p->values = values;
   p->keep = std::move(keep);
@@ -1192,6 +1198,27 @@ std::unique_ptr<BlockPlan> block_plan(py::bytes args, std::vector<py::object> ow
   p->batch = x.size(0); p->dim = x.size(2); p->device = (int)x.get_device(); p->stream = stream; p->type = x.scalar_type();
   return p;
 }
+
+// A block's plans.
+struct BlockPlans {
+  struct Entry {
+    std::shared_ptr<BlockPlan> plan;
+    py::object watch;   // weak reference to the mean
+  };
+  using Map = std::unordered_map<PyObject*, Entry>;
+  std::shared_ptr<Map> plans = std::make_shared<Map>();
+  py::object nkey;      // the norm's key in a state
+
+  void add(std::shared_ptr<BlockPlan> p) {
+    PyObject* const mean = p->mean;
+    nkey = p->nkey;
+    std::weak_ptr<Map> all = plans;
+    py::object watch = py::weakref(mean, py::cpp_function([all, mean](py::handle) {
+      if (auto m = all.lock()) m->erase(mean);
+    }));
+    (*plans)[mean] = Entry{std::move(p), std::move(watch)};
+  }
+};
 
 py::object dict_of(PyObject* o) { return py::reinterpret_steal<py::object>(PyObject_GenericGetDict(o, nullptr)); }
 
@@ -1210,7 +1237,7 @@ bool block_matches(const BlockPlan& p, PyObject* blk, PyObject* block_dict, cons
   PyObject* as = PyDict_GetItemWithError(inc, p.akey.ptr());
   if (as == Py_None) as = nullptr;
   if (!ns || !es || !PyDict_Check(ns) || !PyDict_Check(es) || (as && !PyDict_Check(as))) return false;
-  if (!holds(ns, k.mean, p.mean.ptr()) || !holds(ns, k.var, p.var.ptr()) || !holds(ns, k.count, p.count.ptr()) ||
+  if (!holds(ns, k.mean, p.mean) || !holds(ns, k.var, p.var.ptr()) || !holds(ns, k.count, p.count.ptr()) ||
       !holds(es, k.h, p.h.ptr()) || !holds(as, k.key, p.last_key.ptr()) || !holds(as, k.value, p.last_value.ptr()) ||
       !holds(as, k.key_mask, Py_None))
     return false;
@@ -1245,8 +1272,16 @@ PyObject* block_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
       PyErr_Clear();
       Py_RETURN_NONE;
     }
-    const py::object keep_plan = py::reinterpret_borrow<py::object>(held);
-    BlockPlan& p = *py::cast<BlockPlan*>(py::handle(held));
+    const auto plans = py::cast<BlockPlans*>(py::handle(held))->plans;
+    PyObject* ns = PyDict_GetItemWithError(a[2], py::cast<BlockPlans*>(py::handle(held))->nkey.ptr());
+    PyObject* mean = ns && PyDict_Check(ns) ? PyDict_GetItemWithError(ns, k.mean) : nullptr;
+    const auto found = plans->find(mean);
+    if (found == plans->end()) {
+      PyErr_Clear();
+      Py_RETURN_NONE;
+    }
+    const std::shared_ptr<BlockPlan> keep_plan = found->second.plan;
+    BlockPlan& p = *keep_plan;
     const Tensor& x = THPVariable_Unpack(a[1]);
     if (!block_matches(p, a[0], dict.ptr(), x, a[2])) {
       PyErr_Clear();
@@ -1256,13 +1291,17 @@ PyObject* block_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
     void* stream = at::cuda::getCurrentCUDAStream((c10::DeviceIndex)p.device).stream();
     if ((uintptr_t)stream != p.stream) Py_RETURN_NONE;
     Tensor out(at::detail::empty_cuda(x.sizes(), x.scalar_type(), x.device(), std::nullopt));
+    auto at = [](PyObject* t) { return THPVariable_Unpack(t).data_ptr(); };
+    p.args.count = (int64_t*)at(p.count.ptr());
+    p.args.count_next = (int64_t*)at(p.count_next.ptr());
+    p.args.mean = (float*)at(p.mean);
+    p.args.var = (float*)at(p.var.ptr());
+    p.args.h = (float*)at(p.h.ptr());
     p.args.x = x.data_ptr();
     p.args.out = out.data_ptr();
     p.args.pos = p.pos;
     check(mega_block_step(&p.args, stream), "block_step");
-    // the counts alternate between two arrays, the step wrote the second one
-    std::swap(p.count, p.count_next);
-    std::swap(p.args.count, p.args.count_next);
+    std::swap(p.count, p.count_next);   // the counts alternate between two arrays, the step wrote the second one
     if (PyDict_SetItem(PyDict_GetItemWithError(a[2], p.nkey.ptr()), k.count, p.count.ptr()) != 0) return nullptr;
     PyObject* as = PyDict_GetItemWithError(a[2], p.akey.ptr());
     if (!as || as == Py_None) {
@@ -1280,7 +1319,7 @@ PyObject* block_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
     } else {   // the chunk is complete: the next token starts another one, in other buffers
       for (PyObject* key : {k.key, k.value, k.key_mask})
         if (PyDict_GetItemWithError(as, key) && PyDict_DelItem(as, key) != 0) return nullptr;
-      if (PyDict_SetItem(dict.ptr(), k.block_plan, Py_None) != 0) return nullptr;
+      plans->erase(p.mean);
     }
     return THPVariable_Wrap(std::move(out));
   } catch (py::error_already_set& e) {
@@ -1303,10 +1342,13 @@ PYBIND11_MODULE(_mega_host, m) {
       .def("__reduce__", [](StepPlan&) {
         return py::make_tuple(py::reinterpret_borrow<py::object>((PyObject*)Py_TYPE(Py_None)), py::tuple());
       });
-  py::class_<BlockPlan>(m, "BlockPlan")
-      .def(py::init(&block_plan))
-      .def("__deepcopy__", [](BlockPlan&, py::object) { return py::none(); })
-      .def("__reduce__", [](BlockPlan&) {
+  py::class_<BlockPlan, std::shared_ptr<BlockPlan>>(m, "BlockPlan").def(py::init(&block_plan));
+  py::class_<BlockPlans>(m, "BlockPlans")
+      .def(py::init<>())
+      .def("add", &BlockPlans::add)
+      .def("__len__", [](BlockPlans& b) { return b.plans->size(); })
+      .def("__deepcopy__", [](BlockPlans&, py::object) { return py::none(); })
+      .def("__reduce__", [](BlockPlans&) {
         return py::make_tuple(py::reinterpret_borrow<py::object>((PyObject*)Py_TYPE(Py_None)), py::tuple());
       });
   PyModule_AddFunctions(m.ptr(), g_raw);

@@ -5,7 +5,7 @@ MovingAverageGatedAttention.forward with an incremental state
 The keys and values of a chunk live in buffers with room for the whole chunk; the state's ``prev_key`` /
 ``prev_value`` are views of their first rows, so a step appends a row instead of copying the cache.  Rows that a
 view covers are never written again: a step appends only behind the views that the step before handed out, and
-any other state (a new generation, reordered beams, a copied state) gets buffers of its own.
+any other state (a new generation, reordered beams, a copied state) gets buffers of its own.  They go with the state.
 """
 from typing import Optional
 
@@ -107,9 +107,8 @@ def _build(blk, x, stream, incremental_state):
     p, q, g, omega = _ema_params(move)
     args = _lib.BlockStepArgs(
         dtype=dt, batch=bsz, embed=dim, zdim=blk.zdim, hdim=blk.hdim, ndim=move.ndim, complex_poles=int(move.complex),
-        positions=rot.size(0), count=count.data_ptr(), count_next=count_next.data_ptr(),
-        mean=mean.data_ptr(), var=var.data_ptr(), h=h.data_ptr(), norm_gamma=gamma_eff.data_ptr(),
-        norm_beta=beta.data_ptr(), p=p.data_ptr(), q=q.data_ptr(), gamma_hat=g.data_ptr(), omega=omega.data_ptr(),
+        positions=rot.size(0), norm_gamma=gamma_eff.data_ptr(), norm_beta=beta.data_ptr(),
+        p=p.data_ptr(), q=q.data_ptr(), gamma_hat=g.data_ptr(), omega=omega.data_ptr(),
         v_weight=blk.v_proj.weight.data_ptr(), v_bias=blk.v_proj.bias.data_ptr(),
         mx_weight=blk.mx_proj.weight.data_ptr(), mx_bias=blk.mx_proj.bias.data_ptr(),
         h_weight=blk.h_proj.weight.data_ptr(), qk_gamma=blk.gamma.data_ptr(), qk_beta=blk.beta.data_ptr(),
@@ -118,8 +117,11 @@ def _build(blk, x, stream, incremental_state):
         qk_dtype=ops._dt(blk.gamma))
     names = _names(blk)
     owners = [blk] + [blk._modules[m] for m in _SUBMODULES]
-    blk._block_plan = _lib.host().BlockPlan(
+    plans = blk.__dict__.get("_block_plan")   # (None in a copy of a block)
+    if plans is None:
+        plans = blk._block_plan = _lib.host().BlockPlans()
+    plans.add(_lib.host().BlockPlan(
         bytes(args), owners, list(_SUBMODULES), names, [owners[i]._parameters[name] for i, name in names], [nkey, ekey, akey],
         [count, count_next, mean, var, h, k, v], keys, values, [keys_rot, work, rot, gamma_eff, beta, p, q, g, omega],
-        chunk, x, stream)
+        chunk, x, stream))
     return True

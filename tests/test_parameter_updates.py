@@ -116,3 +116,58 @@ def test_storage_replaced_during_a_generation(how):
             want.append(ref(x[:, t:t + 1].float().contiguous(), incremental_state=b)[0])
     del junk
     assert rel_l2(torch.cat(got, 1).float(), torch.cat(want, 1)) < 2e-2
+
+
+def test_generation_gives_its_buffers_back():
+    import fairseq_apollo_b200 as M
+    blk = _block(M, chunk=1024)
+    x = torch.randn(8, 8, 64, device="cuda").bfloat16()
+    with torch.no_grad():
+        _generate(blk, x)
+        gc.collect()
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        inc = {}
+        _generate(blk, x, inc)
+        assert torch.cuda.memory_allocated() > before
+        del inc
+        assert torch.cuda.memory_allocated() - before < 1 << 16
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_two_generations_in_turn(dtype):
+    """Two requests answered token by token in turn: each as by itself, and neither sets the other's step up again."""
+    import fairseq_apollo_b200 as M
+    blk = _block(M).to(dtype)
+    xs = [torch.randn(2, 40, 64, device="cuda").to(dtype) for _ in range(2)]
+    with torch.no_grad():
+        want = [_generate(blk, x) for x in xs]
+        incs = [{}, {}]
+        got = [[blk(x[:, :5].contiguous(), incremental_state=i)[0]] for x, i in zip(xs, incs)]
+        for t in range(5, 40):
+            before = M.launch_count()
+            for k in range(2):
+                got[k].append(blk(xs[k][:, t:t + 1].contiguous(), incremental_state=incs[k])[0])
+            if t > 5:
+                assert M.launch_count() - before == 10
+    for k in range(2):
+        assert torch.equal(torch.cat(got[k], 1), want[k])
+
+
+def test_copies_and_files_of_a_block_in_the_middle_of_a_generation(tmp_path):
+    """A copied or loaded block and state go on as the original does; a state's file holds tensors alone."""
+    import fairseq_apollo_b200 as M
+    blk = _block(M)
+    x = torch.randn(2, 12, 64, device="cuda").bfloat16()
+    with torch.no_grad():
+        want = _generate(blk, x)[:, 8:]
+        inc = {}
+        _generate(blk, x[:, :8], inc)
+        torch.save(inc, tmp_path / "state.pt")
+        torch.save(blk, tmp_path / "block.pt")
+        copies = [(copy.deepcopy(blk), copy.deepcopy(inc)),
+                  (torch.load(tmp_path / "block.pt", weights_only=False), torch.load(tmp_path / "state.pt", weights_only=True)),
+                  (blk, {k: {n: t if t is None else t.clone() for n, t in v.items()} for k, v in inc.items()}), (blk, inc)]
+        for b, i in copies:
+            got = torch.cat([b(x[:, t:t + 1].contiguous(), incremental_state=i)[0] for t in range(8, 12)], 1)
+            assert torch.equal(got, want)
