@@ -8,8 +8,18 @@ are column sums taken while those matrices are written, so autograd has no slice
 import torch
 
 from . import _lib
+from .functions import plain
 
 CAUSAL, _BIAS = 0, 1
+
+
+def _own(module, name):
+    """A plain one of the package's classes (by name: their module imports this one)."""
+    return type(module).__name__ == name and plain(module, type(module))
+
+
+def projections_plain(blk):
+    return all(plain(m, torch.nn.Linear) for m in (blk.v_proj, blk.mx_proj, blk.h_proj))
 
 
 def mode_of(blk, x, padding_mask, attn_mask, need_weights, before_attn_fn):
@@ -22,6 +32,8 @@ def mode_of(blk, x, padding_mask, attn_mask, need_weights, before_attn_fn):
     n = 16 // x.element_size()
     if blk.embed_dim % n or blk.zdim % n or blk.hdim % n or blk.zdim > 512:
         return None
+    if not projections_plain(blk):
+        return None
     if any(w.dtype != x.dtype for w in (blk.v_proj.weight, blk.mx_proj.weight, blk.h_proj.weight)):
         return None
     seq = x.size(1)
@@ -29,10 +41,10 @@ def mode_of(blk, x, padding_mask, attn_mask, need_weights, before_attn_fn):
     if seq % period:
         return None
     if blk.efficient_attn is not None:
-        ok = type(blk.rel_pos_bias).__name__ == "RotaryEmbedding" and period <= 8192
+        ok = _own(blk.rel_pos_bias, "RotaryEmbedding") and _own(blk.efficient_attn, "EfficientAttention") and period <= 8192
         return CAUSAL if ok else None
     if (blk.attention_activation == 'softmax' and blk.attn_softmax is None and period <= 8192
-            and type(blk.rel_pos_bias).__name__ == "SimpleRelativePositionalBias" and period <= blk.rel_pos_bias.max_positions):
+            and _own(blk.rel_pos_bias, "SimpleRelativePositionalBias") and period <= blk.rel_pos_bias.max_positions):
         return _BIAS
     return None
 

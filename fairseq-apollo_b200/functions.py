@@ -3,12 +3,23 @@ backward run on the library's kernels, and the backward without the interpreter;
 the reference's Functions (fairseq/modules/norm_layer/timestep_norm.py:14-66, sequence_norm.py:12-52,
 fairseq/modules/fused_ops/{fftconv,ema_parameters,ema_hidden}.py)."""
 import torch
+from torch.nn.modules.module import _has_any_global_hook
 
 from . import _lib, ops
 
 
 def needs_grad(*tensors):
     return torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)
+
+
+def plain(module, *types):
+    """Whether calling the module is its class's forward and nothing else: one of these classes itself (an adapter, a
+    quantised or a sharded layer is another), no forward of its own, no hooks.  Only then may a path take the module's
+    parameters instead of calling it."""
+    d = module.__dict__
+    return (type(module) in types and "forward" not in d
+            and not (d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"])
+            and not _has_any_global_hook())
 
 
 def ema(x, alpha, delta, third, gamma, omega, padding_mask, bidirectional, shift, truncation=None, complex_poles=False,

@@ -1024,12 +1024,13 @@ Tensor block_train(const Tensor& x, const Tensor& xn, const Tensor& mx, const Te
 // (identity, version counters and storage: p.data = t, which is also how a module is moved, leaves the first two alone), the state tensors, the batch, the dtype and the options stay what they were.  The
 // state tensors are updated in place, except the counts: one array is read, another written, and they alternate.
 struct Names {
-  PyObject *params, *modules, *groups, *bidirectional, *plan, *block_plan, *count, *mean, *var, *h, *key, *value, *key_mask;
+  PyObject *params, *modules, *groups, *bidirectional, *plan, *block_plan, *count, *mean, *var, *h, *key, *value, *key_mask,
+      *forward, *hooks, *pre_hooks;
   Names() {
     auto s = [](const char* t) { return PyUnicode_InternFromString(t); };
     params = s("_parameters"); groups = s("num_groups"); bidirectional = s("bidirectional"); plan = s("_step_plan");
     modules = s("_modules"); block_plan = s("_block_plan"); key = s("prev_key"); value = s("prev_value");
-    key_mask = s("prev_key_padding_mask");
+    key_mask = s("prev_key_padding_mask"); forward = s("forward"); hooks = s("_forward_hooks"); pre_hooks = s("_forward_pre_hooks");
     count = s("prev_count"); mean = s("prev_mean"); var = s("prev_var"); h = s("prev_state");
   }
 };
@@ -1154,14 +1155,15 @@ PyObject* norm_ema_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // A plan belongs to a generation: to its running mean, a tensor that the steps update in place and that the state keeps
 // from the first to the last of them.  The block's plans are found by it, so generations that are answered in turn keep
 // theirs, and a plan goes, with the buffers of keys and values it holds, when the tensor does.
+constexpr int kOwners = 7;
 struct BlockPlan {
   mega_block_step_args args;
   PyObject* block;                         // (not owned: the plans live in the block's dictionary)
-  py::object owners[5];                    // norm, move, v_proj, mx_proj, h_proj
+  py::object owners[kOwners];              // norm, move, then those a step stands for: v_proj, mx_proj, h_proj, attention, positions
   std::vector<std::pair<int, py::object>> names;   // of a parameter: owner (0: the block, 1 ...: the above), key
   std::vector<py::object> params;
   std::vector<Mark> marks;
-  py::object submodules[5];                // the owners' keys
+  py::object submodules[kOwners];          // the owners' keys
   py::object nkey, ekey, akey;
   PyObject* mean;                          // (not owned: the plan goes with it)
   py::object count, count_next, var, h, last_key, last_value;
@@ -1180,12 +1182,12 @@ std::shared_ptr<BlockPlan> block_plan(py::bytes args, std::vector<py::object> ow
                                       uintptr_t stream) {
   auto p = std::make_shared<BlockPlan>();
   const std::string raw = args;
-  if (raw.size() != sizeof p->args || owners.size() != 6 || submodules.size() != 5) throw py::value_error("block_plan");
+  if (raw.size() != sizeof p->args || owners.size() != kOwners + 1 || submodules.size() != kOwners) throw py::value_error("block_plan");
   memcpy(&p->args, raw.data(), raw.size());
   auto word = [](const std::string& t) { return py::reinterpret_steal<py::object>(PyUnicode_InternFromString(t.c_str())); };
   p->block = owners[0].ptr();
-  for (int i = 0; i < 5; ++i) p->owners[i] = owners[i + 1];
-  for (int i = 0; i < 5; ++i) p->submodules[i] = word(submodules[i]);
+  for (int i = 0; i < kOwners; ++i) p->owners[i] = owners[i + 1];
+  for (int i = 0; i < kOwners; ++i) p->submodules[i] = word(submodules[i]);
   for (auto& n : names) p->names.emplace_back(n.first, word(n.second));
   p->params = std::move(params);
   for (auto& t : p->params) p->marks.emplace_back(THPVariable_Unpack(t.ptr()));
@@ -1228,6 +1230,12 @@ bool holds(PyObject* dict, PyObject* key, PyObject* want) {
   return (v ? v : Py_None) == want;
 }
 
+// whether a dictionary in a module's dictionary is empty
+bool empty(PyObject* dict, PyObject* key) {
+  PyObject* v = PyDict_GetItemWithError(dict, key);
+  return v && PyDict_Check(v) && PyDict_Size(v) == 0;
+}
+
 // Whether the plan is one for this block, these inputs and this state.
 bool block_matches(const BlockPlan& p, PyObject* blk, PyObject* block_dict, const Tensor& x, PyObject* inc) {
   const Names& k = names();
@@ -1246,12 +1254,13 @@ bool block_matches(const BlockPlan& p, PyObject* blk, PyObject* block_dict, cons
     return false;
   PyObject* subs = PyDict_GetItemWithError(block_dict, k.modules);
   if (!subs) return false;
-  py::object dicts[6];   // the owners' parameters
-  for (int i = 0; i < 6; ++i) {
+  py::object dicts[kOwners + 1];   // the owners' parameters
+  for (int i = 0; i <= kOwners; ++i) {
     if (i && PyDict_GetItemWithError(subs, p.submodules[i - 1].ptr()) != p.owners[i - 1].ptr()) return false;
     const py::object d = i ? dict_of(p.owners[i - 1].ptr()) : py::reinterpret_borrow<py::object>(block_dict);
     dicts[i] = py::reinterpret_borrow<py::object>(d ? PyDict_GetItemWithError(d.ptr(), k.params) : nullptr);
     if (!dicts[i]) return false;
+    if (i > 2 && (PyDict_Contains(d.ptr(), k.forward) != 0 || !empty(d.ptr(), k.hooks) || !empty(d.ptr(), k.pre_hooks))) return false;
   }
   for (size_t i = 0; i < p.params.size(); ++i) {
     PyObject* t = PyDict_GetItemWithError(dicts[p.names[i].first].ptr(), p.names[i].second.ptr());

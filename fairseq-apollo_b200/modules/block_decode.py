@@ -11,16 +11,19 @@ from typing import Optional
 
 import torch
 from torch import Tensor
+from torch.nn.modules.module import _has_any_global_hook
 
 from .. import _lib, ops
+from ..block_function import _own, projections_plain
 from ..ops import _raw_stream
 from .fused import _ema_params, _param_names, _seed_decode_state
 
 _POLES = {False: (4, 8, 16, 32), True: (2, 4, 8, 16, 32)}
 
 
-# submodules that hold parameters of a step, and those parameters: (owner, 0 the block itself, then in this order; name)
-_SUBMODULES = ("norm", "move", "v_proj", "mx_proj", "h_proj")
+# submodules that a step stands for (from the third on it stands for calling them, so they have to be without hooks and
+# forwards of their own, at every step), and the parameters it takes: (owner, 0 the block itself, then in this order; name)
+_SUBMODULES = ("norm", "move", "v_proj", "mx_proj", "h_proj", "efficient_attn", "rel_pos_bias")
 
 
 def _names(blk):
@@ -34,8 +37,8 @@ def applicable(blk, x) -> bool:
     norm, move = blk.norm, blk.move
     weights = (blk.v_proj.weight, blk.v_proj.bias, blk.mx_proj.weight, blk.mx_proj.bias, blk.h_proj.weight)
     chunk = blk.chunk_size
-    return (blk.efficient_attn is not None and isinstance(blk.move_act, torch.nn.SiLU)
-            and type(blk.rel_pos_bias).__name__ == "RotaryEmbedding" and not move.bidirectional
+    return (blk.efficient_attn is not None and _own(blk.efficient_attn, "EfficientAttention") and projections_plain(blk)
+            and isinstance(blk.move_act, torch.nn.SiLU) and _own(blk.rel_pos_bias, "RotaryEmbedding") and not move.bidirectional
             and norm.num_groups in (None, norm.num_features) and move.ndim in _POLES[move.complex]
             and (chunk < 0 or chunk > 1) and x.dtype in (torch.bfloat16, torch.float16)
             and all(w is not None and w.dtype == x.dtype and w.is_cuda and w.is_contiguous() and w.data_ptr() % 16 == 0
@@ -49,6 +52,8 @@ def applicable(blk, x) -> bool:
 def step(blk, x: Tensor, incremental_state) -> Optional[Tensor]:
     """One token through the block, or None when the call is not the library's (the caller then runs the
     block's own sequence of operations).  Called with gradients disabled, x (B, 1, D) contiguous, no masks."""
+    if _has_any_global_hook():
+        return None
     out = _lib.host().block_step(blk, x, incremental_state)
     if out is None and _build(blk, x, _raw_stream(x.device.index), incremental_state):
         out = _lib.host().block_step(blk, x, incremental_state)

@@ -8,8 +8,9 @@ import torch
 from torch import Tensor
 
 from .. import _lib, ops
-from ..functions import needs_grad
+from ..functions import needs_grad, plain
 from ..ops import _raw_stream
+from .complex_exponential_moving_average import MultiHeadComplexEMA
 from .exponential_moving_average import MultiHeadEMA
 from .sequence_norm import SequenceNorm
 from .timestep_norm import TimestepNorm
@@ -66,8 +67,8 @@ def timestep_norm_ema(norm: TimestepNorm, move: MultiHeadEMA, x: Tensor,
 
 def ema_channels_last(move, x, padding_mask, incremental_state, activation):
     """move(x) for x (B, L, D).  In training without transposes around it, which cost the backward a node each (a module
-    with hooks is called as one)."""
-    if needs_grad(x, *move.parameters()) and not (move._forward_hooks or move._forward_pre_hooks or move._backward_hooks):
+    with hooks or a forward of its own is called as one)."""
+    if needs_grad(x, *move.parameters()) and plain(move, MultiHeadEMA, MultiHeadComplexEMA):
         return move._forward_train(x, padding_mask, incremental_state, activation, channels_last=True)
     return move(x.transpose(1, 2), padding_mask, incremental_state, activation).transpose(1, 2)
 
