@@ -529,6 +529,43 @@ __global__ void __launch_bounds__(kMaxThreads, 1) rowres_kernel(RowArgs a) {
         uint32_t f[2][3][4];
         load_x(gr, 0, f[0]);
         load_x(gr, 1, f[1]);
+        auto states = [&] {
+#pragma unroll
+          for (int nt = 0; nt < kStateTiles; ++nt) products<2>(st[gr][nt], f, fv + nt * kBlockBytes, kStateTiles * kBlockBytes);
+        };
+        // Causal rows: T's zeros do not keep a NaN or an infinity from the positions before it, and the products would make
+        // up to 31 earlier outputs NaN.  A segment with one takes its outputs from the finite values alone, NaN from there
+        // on; its state is NaN, as are all later ones.
+        int bad[2] = {kSeg, kSeg};   // first such position of the lane's two segments
+        bool odd = false;
+        if constexpr (!kBidir && !kNorm) {
+          states();
+          unsigned e = 0u;   // bit 15 or 31: a leading part whose exponent is all ones
+#pragma unroll
+          for (int i = 0; i < 4; ++i) e |= ((f[0][0][i] & 0x7f807f80u) + 0x00800080u) | ((f[1][0][i] & 0x7f807f80u) + 0x00800080u);
+          odd = __any_sync(0xffffffffu, (e & 0x80008000u) != 0u);
+          if (odd) {
+#pragma unroll
+            for (int kt = 0; kt < 2; ++kt)
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                const float4 v = *reinterpret_cast<const float4*>(xs + 4 * piece(seg_of(gr, h), 4 * kt + t, rs));
+                float u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int c = 3; c >= 0; --c)
+                  if (!(fabsf(u[c]) < 0x1.FFp127f)) {   // (from there on the leading part is an infinity)
+                    bad[h] = min(bad[h], 16 * kt + 4 * t + c);
+                    u[c] = 0.f;
+                  }
+                split3(u[0], u[1], f[kt][0][h], f[kt][1][h], f[kt][2][h]);
+                split3(u[2], u[3], f[kt][0][2 + h], f[kt][1][2 + h], f[kt][2][2 + h]);
+              }
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+              for (int s = 1; s < 4; s <<= 1) bad[h] = min(bad[h], __shfl_xor_sync(0xffffffffu, bad[h], s));
+          }
+        }
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
           float y[2][4];
@@ -539,12 +576,17 @@ __global__ void __launch_bounds__(kMaxThreads, 1) rowres_kernel(RowArgs a) {
             float4* at = reinterpret_cast<float4*>(xs + 4 * piece(seg_of(gr, h), 4 * half + t, rs));
             float4 v = *at;
             if (kNorm) v = make_float4(fmaf(v.x, sc, sh), fmaf(v.y, sc, sh), fmaf(v.z, sc, sh), fmaf(v.w, sc, sh));
-            *at = make_float4(fmaf(om, v.x, y[0][2 * h]), fmaf(om, v.y, y[0][2 * h + 1]), fmaf(om, v.z, y[1][2 * h]),
-                              fmaf(om, v.w, y[1][2 * h + 1]));
+            float4 r = make_float4(fmaf(om, v.x, y[0][2 * h]), fmaf(om, v.y, y[0][2 * h + 1]), fmaf(om, v.z, y[1][2 * h]),
+                                   fmaf(om, v.w, y[1][2 * h + 1]));
+            if (!kBidir && !kNorm && odd) {
+              const int p = 16 * half + 4 * t;
+              const float nan = __int_as_float(0x7fffffff);
+              r = make_float4(p < bad[h] ? r.x : nan, p + 1 < bad[h] ? r.y : nan, p + 2 < bad[h] ? r.z : nan, p + 3 < bad[h] ? r.w : nan);
+            }
+            *at = r;
           }
         }
-#pragma unroll
-        for (int nt = 0; nt < kStateTiles; ++nt) products<2>(st[gr][nt], f, fv + nt * kBlockBytes, kStateTiles * kBlockBytes);
+        if constexpr (kBidir || kNorm) states();
       }
     } else {
 #pragma unroll
