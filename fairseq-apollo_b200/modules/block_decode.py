@@ -52,8 +52,10 @@ def applicable(blk, x) -> bool:
 def step(blk, x: Tensor, incremental_state) -> Optional[Tensor]:
     """One token through the block, or None when the call is not the library's (the caller then runs the
     block's own sequence of operations).  Called with gradients disabled, x (B, 1, D) contiguous, no masks."""
-    if _has_any_global_hook():
+    if _has_any_global_hook() or torch.is_autocast_enabled():
         return None
+    if x.data_ptr() % 16:   # (a slice of a larger tensor: the step reads whole 16-byte pieces)
+        x = x.clone()
     out = _lib.host().block_step(blk, x, incremental_state)
     if out is None and _build(blk, x, _raw_stream(x.device.index), incremental_state):
         out = _lib.host().block_step(blk, x, incremental_state)

@@ -171,3 +171,21 @@ def test_copies_and_files_of_a_block_in_the_middle_of_a_generation(tmp_path):
         for b, i in copies:
             got = torch.cat([b(x[:, t:t + 1].contiguous(), incremental_state=i)[0] for t in range(8, 12)], 1)
             assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("shift", [1, 4])
+def test_token_at_any_address(shift):
+    """A token that is a slice of a larger tensor, aligned to its elements only."""
+    import fairseq_apollo_b200 as M
+    blk = _block(M)
+    x = torch.randn(2, 12, 64, device="cuda").bfloat16()
+    with torch.no_grad():
+        want = _generate(blk, x)
+        inc = {}
+        got = [blk(x[:, :5].contiguous(), incremental_state=inc)[0]]
+        for t in range(5, 12):
+            buf = torch.empty(2 * 64 + 8, device="cuda", dtype=x.dtype)
+            tok = buf[shift:shift + 128].view(2, 1, 64)
+            tok.copy_(x[:, t:t + 1])
+            got.append(blk(tok, incremental_state=inc)[0])
+    assert torch.equal(torch.cat(got, 1), want)
