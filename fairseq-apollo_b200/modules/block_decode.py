@@ -2,7 +2,7 @@
 MovingAverageGatedAttention.forward with an incremental state
 (fairseq/modules/moving_average_gated_attention.py:282-414).
 
-The keys and values of a chunk live in buffers with room for the whole chunk; the state's ``prev_key`` /
+The keys and values of a chunk live in buffers with room for more than there are; the state's ``prev_key`` /
 ``prev_value`` are views of their first rows, so a step appends a row instead of copying the cache.  Rows that a
 view covers are never written again: a step appends only behind the views that the step before handed out, and
 any other state (a new generation, reordered beams, a copied state) gets buffers of its own.  They go with the state.
@@ -94,7 +94,10 @@ def _build(blk, x, stream, incremental_state):
             d[key] = d[key].to(dt).contiguous()
     mean, var, count, h = nstate['prev_mean'], nstate['prev_var'], nstate['prev_count'], estate['prev_state']
     count_next = torch.empty_like(count)
-    cap = chunk if chunk > 0 else max(256, 2 * n)
+    if chunk > 49152:
+        return False
+    cap = max(256, 2 * n)   # (a chunk is not laid out in full for its first tokens; the next plan has room for twice as many)
+    cap = min(cap, chunk) if chunk > 0 else cap
     if cap > 49152:
         return False
     keys = torch.empty(bsz, cap, blk.zdim, dtype=x.dtype, device=dev)

@@ -189,3 +189,20 @@ def test_token_at_any_address(shift):
             tok.copy_(x[:, t:t + 1])
             got.append(blk(tok, incremental_state=inc)[0])
     assert torch.equal(torch.cat(got, 1), want)
+
+
+def test_chunk_is_laid_out_as_it_fills():
+    """Buffers for at most 256 positions, or twice those there are; tokens across the doublings as without a chunk's end."""
+    import fairseq_apollo_b200 as M
+    blk = _block(M, chunk=4096)
+    x = torch.randn(8, 600, 64, device="cuda").bfloat16()
+    with torch.no_grad():
+        gc.collect()
+        _generate(blk, x[:, :8])
+        before = torch.cuda.memory_allocated()
+        inc = {}
+        got = [_generate(blk, x[:, :8], inc)]
+        assert torch.cuda.memory_allocated() - before < 8 * 300 * (64 + 64 + 128) * 2
+        got += [blk(x[:, t:t + 1].contiguous(), incremental_state=inc)[0] for t in range(8, 600)]
+        want = blk(x)[0]
+    assert rel_l2(torch.cat(got, 1), want) < 1e-2
