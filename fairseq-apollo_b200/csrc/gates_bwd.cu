@@ -475,6 +475,12 @@ extern "C" int mega_gate_qk_bwd(const void* z, int64_t ld_z, const float* gamma,
   if (rows <= 0 || cols <= 0 || (cols & 1)) return MEGA_ERR_SHAPE;
   if (rot && (period <= 0 || q_offset < 0 || period + q_offset > positions)) return MEGA_ERR_SHAPE;
   if (cols > 64 * kQkPairs) return MEGA_ERR_UNSUPPORTED;
+  // (pairs of values are read and written at once)
+  if (ld_z < cols || ld_dq < cols || ld_dk < cols || ld_dz < cols) return MEGA_ERR_STRIDE;
+  const size_t pair = 2 * elem_size(dtype);
+  if (!aligned_to(z, pair) || !aligned_to(dq, pair) || !aligned_to(dk, pair) || !aligned_to(dz, pair) || !aligned_to(rot, 8) ||
+      ((ld_z | ld_dq | ld_dk | ld_dz) & 1))
+    return MEGA_ERR_ALIGN;
   const long long want = (rows + 31) / 32;   // four rows per warp at least
   const unsigned grid = (unsigned)(want > 148 * 4 ? 148 * 4 : want);
   MEGA_DISPATCH_DTYPE(dtype, {

@@ -539,7 +539,7 @@ MEGA_API int mega_to_float(const void* const* src, float* const* dst, const int6
  * the gradient they are named after, ADDED to fp32 arrays of `cols` values (bias gradients of the projection that
  * produced the operand), or NULL.  mega_gate_output_bwd: dhx is also the gradient of h_lin.
  * mega_gate_qk_bwd: dq, dk in, dz out; dgamma, dbeta (2, cols) fp32 are added to; rot NULL: mega_gate_qk, else
- * mega_gate_qk_rotary; cols <= 512.
+ * mega_gate_qk_rotary; cols <= 512; operands at addresses and row pitches of whole pairs of values (MEGA_ERR_ALIGN).
  * Replaces: the autograd of moving_average_gated_attention.py:308,322-330,407-412.
  */
 MEGA_API int mega_gate_silu_bwd(const void* dy, int64_t ld_dy, const void* a, int64_t ld_a, void* da, int64_t ld_da,
