@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(256) gate_qk_rotary_vec_kernel(const T* z, lon
     }
 #pragma unroll
     for (int o = kLanes / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if (r >= rows) break;
+    if (r >= rows) continue;   // (no break: the lanes of the other rows of the warp shuffle again)
     const float inv = 1.f / fmaxf(sqrtf(ss), eps);
     const long long chunk = r / period;
     const int pos = (int)(r - chunk * period);

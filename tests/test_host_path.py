@@ -254,3 +254,17 @@ def test_second_derivative_through_the_block(bidir):
     assert len(res[0]) == len(res[1])
     for a, b in zip(*res):
         assert rel_l2(a, b) < 1e-4
+
+
+@pytest.mark.parametrize("rows", [1, 5, 9, 63, 65])
+@pytest.mark.parametrize("zdim", [64, 128, 256])
+def test_query_key_rows_that_end_inside_a_warp(rows, zdim):
+    """16 bytes per access against the same rows an element off, which take one value per access."""
+    from fairseq_apollo_b200 import ops
+    torch.manual_seed(rows)
+    buf = torch.randn(rows * zdim + 8, device="cuda").bfloat16()
+    g, b = torch.randn(2, zdim, device="cuda"), torch.randn(2, zdim, device="cuda")
+    rot = torch.polar(torch.ones(7, zdim // 2), torch.rand(7, zdim // 2)).cuda()
+    one = buf[1:1 + rows * zdim].view(rows, zdim)
+    for a, c in zip(ops.gate_qk_rotary(one.clone(), g, b, rot, 7), ops.gate_qk_rotary(one, g, b, rot, 7)):
+        assert rel_l2(a, c) < 2.0 ** -9
