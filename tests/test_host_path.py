@@ -268,3 +268,22 @@ def test_query_key_rows_that_end_inside_a_warp(rows, zdim):
     one = buf[1:1 + rows * zdim].view(rows, zdim)
     for a, c in zip(ops.gate_qk_rotary(one.clone(), g, b, rot, 7), ops.gate_qk_rotary(one, g, b, rot, 7)):
         assert rel_l2(a, c) < 2.0 ** -9
+
+
+def test_bidirectional_block_beyond_a_grid_axis():
+    """65536 sequences: more than the relative-bias softmax takes in a launch."""
+    import fairseq_apollo_b200 as M
+    torch.manual_seed(13)
+    blk = M.MovingAverageGatedAttention(8, 8, 16, 4, bidirectional=True, rel_pos_bias='simple', max_positions=4, moving_act='silu').cuda()
+    x = torch.randn(65536, 4, 8, device="cuda")
+    dx, dw = [], []
+    for parts in ((x,), x.split(40000)):
+        blk.zero_grad()
+        got = []
+        for p in parts:
+            p = p.clone().requires_grad_(True)
+            blk(p)[0].square().sum().backward()
+            got.append(p.grad)
+        dx.append(torch.cat(got))
+        dw.append(blk.h_proj.weight.grad.clone())
+    assert rel_l2(*dx) < 1e-5 and rel_l2(*dw) < 1e-4
