@@ -44,7 +44,8 @@ def mode_of(blk, x, padding_mask, attn_mask, need_weights, before_attn_fn):
         ok = _own(blk.rel_pos_bias, "RotaryEmbedding") and _own(blk.efficient_attn, "EfficientAttention") and period <= 8192
         return CAUSAL if ok else None
     if (blk.attention_activation == 'softmax' and blk.attn_softmax is None and period <= 8192
-            and _own(blk.rel_pos_bias, "SimpleRelativePositionalBias") and period <= blk.rel_pos_bias.max_positions):
+            and _own(blk.rel_pos_bias, "SimpleRelativePositionalBias") and period <= blk.rel_pos_bias.max_positions
+            and x.size(0) * (seq // period) <= 65535):   # (chunks that the softmax takes in a launch)
         return _BIAS
     return None
 
