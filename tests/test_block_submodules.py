@@ -13,7 +13,7 @@ class Adapter(torch.nn.Linear):
     """A linear layer with something beside it, as low-rank adapters and quantised layers are built."""
 
     def forward(self, x):
-        return super().forward(x) + 0.5 * x.mean(-1, keepdim=True)
+        return 3.0 * super().forward(x) + 1.0
 
 
 def _adapted(lin):
