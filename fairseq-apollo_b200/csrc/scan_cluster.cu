@@ -488,7 +488,8 @@ bool plan(int dtype, const ScanArgs& a, int& T, int& ranks, double& rounds, doub
 }  // namespace
 
 // From a grid of shapes on one B200: a fixed part, then the longer of what a segment's steps take and what all elements
-// take.  Beyond eight million elements, or in rounds of long segments, the three launches of scan_ema.cu are as fast.
+// take.  Beyond 8.5 million elements (6.5 of complex poles in more than one round, 4.3 walked both ways: where that grid had
+// the two level), or in rounds of long segments, the three launches of scan_ema.cu are as fast.
 double scan_cluster_us(int dtype, const ScanArgs& a) {
   int T = 0, ranks = 1;
   double rounds = 0, steps = 0;

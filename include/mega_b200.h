@@ -372,7 +372,7 @@ MEGA_API int mega_timestep_norm_bwd(const void* dy, const void* x, void* dx, int
  * STARTED with (prev_count, prev_mean, prev_var) instead of saves of every step: nothing has to be kept from
  * mega_timestep_norm_fwd but its arguments.  Channels contiguous (stride 1) in all three tensors, base
  * addresses and the strides of x and dy multiples of 16 bytes, D whole 16-byte pieces, dx distinct from both;
- * MEGA_ERR_UNSUPPORTED otherwise.
+ * MEGA_ERR_UNSUPPORTED otherwise, beyond 65535 sequences, and when the device has no scratch memory to give.
  */
 MEGA_API int mega_timestep_norm_bwd_stats(const void* dy, const void* x, void* dx, int dtype, int B, int L, int D,
                            int64_t gsb, int64_t gsl, int64_t gsd, int64_t xsb, int64_t xsl, int64_t xsd,
