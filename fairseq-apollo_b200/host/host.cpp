@@ -835,8 +835,8 @@ class BlockFn : public torch::autograd::Function<BlockFn> {
     Tensor h_lin = at::mm(gated, wh.t());
     Tensor out = at::empty({bsz, seq, d}, x.options().requires_grad(false));
     check(mega_gate_output(x.data_ptr(), d, u, f, hx, f, h_lin.data_ptr(), d, out.data_ptr(), d, dt, rows, (int)d, w.stream), "gate_output");
-    ctx->save_for_backward({x, xn, mx, wv, wm, wh, ga, bias, rot, v_lin, base, q, k, v3, wgt, attn, gated, h_lin, x_, xn_, mx_, bv, bm,
-                            gamma, beta, rot.defined() ? Tensor() : mask_u8(given(mask_), bsz, seq)});
+    ctx->save_for_backward({x_, xn_, mx_, wv, wm, wh, ga, bias, rot, v_lin, base, q, k, v3, wgt, attn, gated, h_lin, bv, bm, gamma, beta,
+                            rot.defined() ? Tensor() : mask_u8(given(mask_), bsz, seq)});
     ctx->saved_data["period"] = period;
     ctx->saved_data["types"] = std::vector<int64_t>{(int64_t)bv.scalar_type(), (int64_t)bm.scalar_type(), (int64_t)gamma.scalar_type(),
                                                     (int64_t)beta.scalar_type()};
@@ -847,11 +847,11 @@ class BlockFn : public torch::autograd::Function<BlockFn> {
   // functions of the inputs.  (Through aliases of them: an input that another one was computed from gets its own share.)
   static variable_list differentiable(AutogradContext* ctx, const variable_list& sv, Tensor dout) {
     const int64_t period = ctx->saved_data["period"].toInt();
-    std::vector<Tensor> in = {sv[18], sv[19], sv[20], sv[3], sv[21], sv[4], sv[22], sv[5], sv[23], sv[24], sv[7]};
+    std::vector<Tensor> in = {sv[0], sv[1], sv[2], sv[3], sv[18], sv[4], sv[19], sv[5], sv[20], sv[21], sv[7]};
     for (auto& t : in)
       if (t.defined()) t = t.view_as(t);
     const Tensor &x = in[0], &xn = in[1], &mx = in[2], &wv = in[3], &bv = in[4], &wm = in[5], &bm = in[6], &wh = in[7], &gamma = in[8],
-                 &beta = in[9], &bias = in[10], &rot = sv[8], &mask = sv[25];
+                 &beta = in[9], &bias = in[10], &rot = sv[8], &mask = sv[22];
     const int64_t bsz = x.size(0), seq = x.size(1), d = x.size(2), s = gamma.size(1), e = wv.size(0), nb = bsz * seq / period;
     const auto type = x.scalar_type();
     const Tensor v = at::silu(at::linear(xn, wv, bv)).reshape({nb, period, e}), base = at::linear(mx, wm, bm);
@@ -894,7 +894,8 @@ class BlockFn : public torch::autograd::Function<BlockFn> {
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto sv = ctx->get_saved_variables();
     if (at::GradMode::is_enabled()) return differentiable(ctx, sv, grads[0].to(sv[0].scalar_type()));
-    const Tensor &x = sv[0], &xn = sv[1], &mx = sv[2], &wv = sv[3], &wm = sv[4], &wh = sv[5], &ga = sv[6], &bias = sv[7], &rot = sv[8],
+    const Tensor x = sv[0].contiguous(), xn = sv[1].contiguous().flatten(0, 1), mx = sv[2].contiguous().flatten(0, 1);
+    const Tensor &wv = sv[3], &wm = sv[4], &wh = sv[5], &ga = sv[6], &bias = sv[7], &rot = sv[8],
                  &v_lin = sv[9], &base = sv[10], &q = sv[11], &k = sv[12], &v3 = sv[13], &wgt = sv[14], &attn = sv[15], &gated = sv[16],
                  &h_lin = sv[17];
     const Where w(x);

@@ -287,3 +287,29 @@ def test_bidirectional_block_beyond_a_grid_axis():
         dx.append(torch.cat(got))
         dw.append(blk.h_proj.weight.grad.clone())
     assert rel_l2(*dx) < 1e-5 and rel_l2(*dw) < 1e-4
+
+
+def test_saved_tensors_of_a_training_pass():
+    """What hooks on saved tensors see (offloading, compression): every activation once per Function that needs it."""
+    import fairseq_apollo_b200 as M
+    from collections import Counter
+    torch.manual_seed(14)
+    blk = M.MovingAverageGatedAttention(64, 64, 128, 16, efficient_attn=True, rel_pos_bias='rotary', chunk_size=32,
+                                        moving_act='silu').cuda().bfloat16()
+    x = torch.randn(2, 64, 64, device="cuda").bfloat16()
+    grads = []
+    for hooks in (False, True):
+        blk.zero_grad()
+        xx, seen = x.clone().requires_grad_(True), Counter()
+
+        def pack(t):
+            if t.numel() >= x.numel():
+                seen[t.data_ptr()] += 1
+            return t.cpu() if hooks else t
+        with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t.cuda()):
+            y = blk(xx)[0]
+        y.sum().backward()
+        assert max(seen.values()) <= 2      # (the block's input and the norm's output: a Function on either side)
+        grads.append([xx.grad] + [p.grad.clone() for p in blk.parameters() if p.grad is not None])
+    for a, b in zip(*grads):
+        assert rel_l2(a, b) < 1e-2
