@@ -569,6 +569,14 @@ extern "C" int mega_ema_bwd(const void* dy, const void* x, void* dx, int dtype, 
     ca.dp = dp; ca.dq = dq; ca.dg = dgamma_hat; ca.domega = domega;
     if (scan_ema_bwd_try(dtype, ca, xsd, dsd, gsd, s)) return check_launch("ema_bwd(scan)");
   }
+  if (!bidir) {   // states carried in or out (or what the scan does not take)
+    EmaBwdStreamArgs sa{};
+    sa.B = B; sa.L = L; sa.D = D; sa.N = N;
+    sa.p = p; sa.q = q; sa.g = gamma_hat; sa.omega = omega; sa.mask = pad_mask; sa.h_in = h_in; sa.dh_out = dh_out;
+    sa.dp = dp; sa.dq = dq; sa.dg = dgamma_hat; sa.domega = domega; sa.dh_in = dh_in;
+    if (ema_bwd_stream_try(dtype, dy, x, dx, gsb, gsl, gsd, xsb, xsl, xsd, dsb, dsl, dsd, sa, s))
+      return check_launch("ema_bwd(stream)");
+  }
   EmaBwdArgs a{};
   a.dy = dy; a.x = x; a.dx = dx; a.B = B; a.D = D; a.L = L; a.N = N;
   a.gsb = gsb; a.gsd = gsd; a.gsl = gsl; a.xsb = xsb; a.xsd = xsd; a.xsl = xsl;

@@ -1,4 +1,4 @@
-// Interface of the streamed backward of TimestepNorm (stream_bwd.cu) and of its grouped form (group_norm.cu).
+// Interface of the streamed backward of TimestepNorm and of the EMA with states (stream_bwd.cu) and of its grouped form (group_norm.cu).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -13,8 +13,19 @@ struct TsnBwdStreamArgs {
   float *dprev_mean, *dprev_var, *dgamma, *dbeta;
 };
 
-// Returns false, having launched nothing, outside its envelope (channel stride != 1, bases or strides not 16-byte
-// aligned, more than 65535 sequences).
+struct EmaBwdStreamArgs {
+  int B, L, D, N;
+  const float *p, *q, *g, *omega;
+  const unsigned char* mask;
+  const float *h_in, *dh_out;
+  float *dp, *dq, *dg, *domega, *dh_in;
+};
+
+// Each returns false, having launched nothing, outside its envelope (channel stride != 1, bases or strides not 16-byte
+// aligned, more than 65535 sequences, ndim > 16 for the EMA).
+bool ema_bwd_stream_try(int dtype, const void* dy, const void* x, void* dx, long long gsb, long long gsl,
+                        long long gsd, long long xsb, long long xsl, long long xsd, long long dsb, long long dsl,
+                        long long dsd, const EmaBwdStreamArgs& a, cudaStream_t s);
 bool tsn_bwd_stream_try(int dtype, const void* dy, const void* x, void* dx, long long gsb, long long gsl,
                         long long gsd, long long xsb, long long xsl, long long xsd, long long dsb, long long dsl,
                         long long dsd, const float* cummean, const float* cumrstd, const TsnBwdStreamArgs& a,
