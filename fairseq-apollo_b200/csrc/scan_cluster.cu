@@ -156,8 +156,9 @@ __global__ void __launch_bounds__(kW * 32, kC ? 1 : 2) scan_cluster_kernel(Clust
     for (int id = lane; id < n * kPer; id += 32) {
       const int r = id / kPer, c = (id % kPer) * (16 / (int)sizeof(T));
       const bool in = c < left;
+      const int bytes = in ? min(16, (left - c) * (int)sizeof(T)) : 0;   // (nothing behind the last channel is read)
       asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16, %2;" ::"r"(at + id * 16),
-                   "l"(in ? x + (long long)r * a.xsl + c : x), "r"(in ? 16 : 0)
+                   "l"(in ? x + (long long)r * a.xsl + c : x), "r"(bytes)
                    : "memory");
     }
     tile_commit();

@@ -713,7 +713,8 @@ static bool dispatch(int dtype, const ScanArgs& a, cudaStream_t st) {
 }  // namespace
 
 bool scan_ema_fwd_ok(int dtype, const ScanArgs& a, long long xsd, long long ysd) {
-  return g_options[OPT_DISABLE_STREAM].load() == 0 && rows_ok(dtype, a.x, a.xsb, a.xsl, xsd, a.D) && ysd == 1 && a.N <= 16 &&
+  return g_options[OPT_DISABLE_STREAM].load() == 0 && rows_ok(dtype, a.x, a.xsb, a.xsl, xsd) && (!a.prev_count || pieces_ok(dtype, a.D)) &&
+         ysd == 1 && a.N <= 16 &&
          (long long)a.B * (a.bidir ? 2 : 1) <= 65535 && (a.x != a.y || (a.xsb == a.ysb && a.xsl == a.ysl));
 }
 
@@ -724,7 +725,7 @@ bool scan_ema_fwd_try(int dtype, const ScanArgs& a, long long xsd, long long ysd
 }
 
 bool scan_ema_bwd_try(int dtype, const ScanArgs& a, long long xsd, long long ysd, long long gsd, cudaStream_t s) {
-  if (!rows_ok(dtype, a.x, a.xsb, a.xsl, xsd, a.D) || !rows_ok(dtype, a.dy, a.gsb, a.gsl, gsd, a.D) || ysd != 1 || a.h_in ||
+  if (!rows_ok(dtype, a.x, a.xsb, a.xsl, xsd) || !rows_ok(dtype, a.dy, a.gsb, a.gsl, gsd) || ysd != 1 || a.h_in ||
       a.h_out)
     return false;
   return dispatch<true>(dtype, a, s);

@@ -26,7 +26,7 @@ struct ScanArgs {
 };
 
 // Each returns false, having launched nothing, outside its envelope (channel stride other than 1, inputs whose rows
-// are not whole 16-byte pieces, ndim > 16, too many sequences for the grid) or when there is no scratch memory.
+// do not start at 16-byte boundaries (behind a norm: are not whole 16-byte pieces), ndim > 16, too many sequences for the grid) or when there is no scratch memory.
 // The forward may run in place (x == y, same strides): a warp reads its rows ahead of where it writes them.
 bool scan_ema_fwd_ok(int dtype, const ScanArgs& a, long long xsd, long long ysd);   // the envelope alone
 bool scan_ema_fwd_try(int dtype, const ScanArgs& a, long long xsd, long long ysd, cudaStream_t s);

@@ -508,7 +508,7 @@ static bool pairs_ok(int dtype, const ScanNormArgs& a, long long ysd) {
 }
 
 bool scan_norm_fwd_try(int dtype, const ScanNormArgs& a, long long xsd, long long ysd, cudaStream_t s) {
-  if (!rows_ok(dtype, a.x, a.xsb, a.xsl, xsd, a.D) || !pairs_ok(dtype, a, ysd) || a.x == a.y) return false;
+  if (!pieces_ok(dtype, a.D) || !rows_ok(dtype, a.x, a.xsb, a.xsl, xsd) || !pairs_ok(dtype, a, ysd) || a.x == a.y) return false;
   // (every segment's block reads the incoming statistics, the last one's writes the new ones)
   const size_t n = (size_t)a.B * a.D;
   for (const float* out : {a.mean_out, a.var_out})
@@ -517,19 +517,19 @@ bool scan_norm_fwd_try(int dtype, const ScanNormArgs& a, long long xsd, long lon
 }
 
 bool scan_norm_bwd_try(int dtype, const ScanNormArgs& a, long long xsd, long long ysd, long long gsd, cudaStream_t s) {
-  if (!rows_ok(dtype, a.x, a.xsb, a.xsl, xsd, a.D) || !rows_ok(dtype, a.dy, a.gsb, a.gsl, gsd, a.D) ||
+  if (!pieces_ok(dtype, a.D) || !rows_ok(dtype, a.x, a.xsb, a.xsl, xsd) || !rows_ok(dtype, a.dy, a.gsb, a.gsl, gsd) ||
       !pairs_ok(dtype, a, ysd) || a.y == a.x || a.y == a.dy)
     return false;
   return dispatch<true>(dtype, a, s);
 }
 
 bool scan_sqn_fwd_try(int dtype, const ScanNormArgs& a, long long xsd, long long ysd, cudaStream_t s) {
-  if (!rows_ok(dtype, a.x, a.xsb, a.xsl, xsd, a.D) || ysd != 1) return false;
+  if (!pieces_ok(dtype, a.D) || !rows_ok(dtype, a.x, a.xsb, a.xsl, xsd) || ysd != 1) return false;
   return sqn_dispatch(dtype, a, false, s);
 }
 
 bool scan_sqn_bwd_try(int dtype, const ScanNormArgs& a, long long xsd, long long ysd, long long gsd, cudaStream_t s) {
-  if (!rows_ok(dtype, a.x, a.xsb, a.xsl, xsd, a.D) || !rows_ok(dtype, a.dy, a.gsb, a.gsl, gsd, a.D) || ysd != 1 ||
+  if (!pieces_ok(dtype, a.D) || !rows_ok(dtype, a.x, a.xsb, a.xsl, xsd) || !rows_ok(dtype, a.dy, a.gsb, a.gsl, gsd) || ysd != 1 ||
       a.y == a.x || a.y == a.dy)
     return false;
   return sqn_dispatch(dtype, a, true, s);

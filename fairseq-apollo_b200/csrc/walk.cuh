@@ -28,8 +28,8 @@ __device__ __forceinline__ void fetch_tile(uint32_t dst, const T* row, long long
     const int r = id / kPer, c = (id % kPer) * (16 / (int)sizeof(T));
     const bool in = r < rows && c < d_left;
     const T* src = in ? row + (long long)r * stride + c : row;
-    asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16, %2;" ::"r"(dst + id * 16), "l"(src), "r"(in ? 16 : 0)
-                 : "memory");
+    const int bytes = in ? min(16, (d_left - c) * (int)sizeof(T)) : 0;   // (nothing behind the last channel is read)
+    asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16, %2;" ::"r"(dst + id * 16), "l"(src), "r"(bytes) : "memory");
   }
 }
 __device__ __forceinline__ void tile_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
@@ -165,10 +165,12 @@ __device__ __forceinline__ void walk_pairs(const T* x, long long xsl, const T* g
 
 }  // namespace
 
-// channels contiguous, rows in whole 16-byte pieces
-static inline bool rows_ok(int dtype, const void* p, long long sb, long long sl, long long sd, int D) {
+// channels contiguous, rows that start at 16-byte boundaries
+static inline bool rows_ok(int dtype, const void* p, long long sb, long long sl, long long sd) {
   const long long es = elem_size(dtype);
-  return sd == 1 && aligned_to(p, 16) && (sb * es) % 16 == 0 && (sl * es) % 16 == 0 && (D * es) % 16 == 0;
+  return sd == 1 && aligned_to(p, 16) && (sb * es) % 16 == 0 && (sl * es) % 16 == 0;
 }
+// ... and are whole 16-byte pieces (where a lane takes two channels)
+static inline bool pieces_ok(int dtype, int D) { return (D * elem_size(dtype)) % 16 == 0; }
 
 }  // namespace mega
