@@ -283,24 +283,27 @@ __global__ void __launch_bounds__(128) sqn_column_kernel(SqnArgs a) {
 // ---------------------------------------------------------------------------
 // parameters of a norm module in one launch each way (as torch operations: a dozen launches of a few values)
 // ---------------------------------------------------------------------------
-// fp32 effective scale (weight + 1) and bias; with B > 0 also the priors as running statistics of B sequences
+// fp32 effective scale (weight + 1) and bias; with B > 0 also the priors as running statistics of B sequences.  One of these
+// runs in front of every inference call, so it is launched ahead of the end of what comes before it (layer of 16 x 4096 x
+// 1024 bf16: 144 us with it, 139 without).
 template <typename T>
 __global__ void norm_prepare_kernel(const long long* prior_count, const T* prior_mean, const T* prior_logv, const T* weight,
                                     const T* bias, int B, int G, int D, long long* count, float* mean, float* var,
                                     float* gamma, float* beta) {
+  pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < D) {
+  if (i < D && blockIdx.y == 0) {
     gamma[i] = Elem<T>::ld(weight + i) + 1.f;
     beta[i] = Elem<T>::ld(bias + i);
   }
   if (i < G) {
     const float m = Elem<T>::ld(prior_mean + i), v = expf(Elem<T>::ld(prior_logv + i));
-    for (int b = 0; b < B; ++b) {
+    for (int b = blockIdx.y; b < B; b += gridDim.y) {
       mean[(size_t)b * G + i] = m;
       var[(size_t)b * G + i] = v;
     }
   }
-  if (i < B) count[i] = prior_count[0];
+  if (i < B && blockIdx.y == 0) count[i] = prior_count[0];
 }
 // their gradients in the parameters' type: the affine pair converted, the priors' summed over the batch
 template <typename T>
@@ -815,8 +818,10 @@ extern "C" int mega_norm_prepare(const int64_t* prior_count, const void* prior_m
   if (B > 0 && (!prior_count || !prior_mean || !prior_logv || !count || !mean || !var)) return MEGA_ERR_NULL;
   if (!valid_dtype(dtype)) return MEGA_ERR_DTYPE;
   if (D <= 0 || B < 0 || (B > 0 && G <= 0)) return MEGA_ERR_SHAPE;
-  const int n = D > B ? D : B;   // (G <= D)
-  MEGA_DISPATCH_DTYPE(dtype, launch(norm_prepare_kernel<T>, (unsigned)((n + 127) / 128), 128, 0, stream,
+  int n = D > B ? D : B;
+  if (B > 0 && G > n) n = G;
+  const dim3 grid((n + 127) / 128, B > 8 ? 8 : B > 0 ? B : 1);
+  MEGA_DISPATCH_DTYPE(dtype, launch_after(norm_prepare_kernel<T>, grid, dim3(128), 0, stream,
                                     (const long long*)prior_count, (const T*)prior_mean, (const T*)prior_logv,
                                     (const T*)weight, (const T*)bias, B, B > 0 ? G : 0, D, (long long*)count, mean, var, gamma,
                                     beta));
