@@ -6,16 +6,17 @@
 //   local pole states   H = X V      X (S, 32) the row, V (32, poles): q^(31-k), anti-causal q^k
 //   outputs             Y = X T + C E   T (32, 32) the taps between positions of a segment, both directions at once;
 //                                    C (S, poles) the states that enter a segment, E (poles, 32)
-// omega x is added in fp32 beside them.
-// and a scan of the S states per pole (C from H): the run that a lane holds, lanes by shuffles, warps through a table.
+// with omega x added in fp32, and a scan of the S states per pole (C from H): the run that a lane holds, lanes by shuffles,
+// warps through a table.
 // 96 multiply-adds per element bidirectional, 64 causal.  HBM sees the row once in, once out.
 //
 // fp32 on the bf16 tensor pipe: a float is exactly the sum of three bf16 values, and six of the nine products (all
 // but those below 2^-24 of the largest) are accumulated in fp32.  That is 576 bf16 products per element where the packed
 // FMA pipe, at an eleventh of the rate, would spend 96 slots.  The tensor pipe truncates its sums, so what would be large
-// in them stays out: omega x, usually the larger part of an output, and every tile's leading products have fp32 additions
-// of their own.  Against the float64 recurrence: 1.0e-7 bidirectional, 6.1e-8 causal (the fp32 walk: 1.1e-7 and 6.7e-8;
-// omega on T's diagonal, one accumulator and taps summed in fp32: 1.3e-7 and 8.0e-8).
+// in them stays out: omega x, usually the larger part of an output, and the leading products of the outputs, which have an
+// accumulator of their own.  Against the float64 recurrence: 1.0e-7 bidirectional, 6.4e-8 causal (the fp32 walk: 1.0e-7 and
+// 6.8e-8; omega on T's diagonal, one accumulator and taps summed in fp32: 1.2e-7 and 8.3e-8; each tile's leading products
+// added by themselves: 9.3e-8 and 6.1e-8, at 717 us where the case below takes 686).
 //
 // B = 32, D = 256, L = 16384 fp32 bidirectional after the norm: 1310 us as a walk (FMA, one row per SM), 590 us now (650
 // padded by up to half): the tensor pipe is at 45 %, issue slots at 40 %, the rest is latency, 16 warps being what the
@@ -81,27 +82,32 @@ __device__ __forceinline__ Frag load_frag(const unsigned char* block) {
   const int lane = threadIdx.x & 31;
   return {*reinterpret_cast<const uint4*>(block + lane * 16), *reinterpret_cast<const uint2*>(block + 512 + lane * 8)};
 }
-// d = products of K reduction tiles, all but those of the leading parts, smallest first, then those, each tile's on its own:
-// the tensor pipe truncates its sums, the additions here round.  Block of tile k at block + k * stride.
-template <int K>
+// d = products of K reduction tiles, all but those of the leading parts, smallest first, then those.  The tensor pipe truncates
+// its sums: kApart gives the leading products an accumulator of their own, which an fp32 addition joins.  Block of tile k at
+// block + k * stride.
+template <int K, bool kApart>
 __device__ __forceinline__ void products(float (&d)[4], const uint32_t (&a)[K][3][4], const unsigned char* block, int stride) {
+  float l[4] = {0.f, 0.f, 0.f, 0.f};
   d[0] = d[1] = d[2] = d[3] = 0.f;
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     const Frag b = load_frag(block + k * stride);
+    if (kApart) mma(l, a[k][0], b.u.x, b.u.y);
     mma(d, a[k][2], b.u.x, b.u.y);
     mma(d, a[k][0], b.v.x, b.v.y);
     mma(d, a[k][1], b.u.z, b.u.w);
     mma(d, a[k][1], b.u.x, b.u.y);
     mma(d, a[k][0], b.u.z, b.u.w);
   }
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    const uint2 b = *reinterpret_cast<const uint2*>(block + k * stride + (threadIdx.x & 31) * 16);
-    float l[4] = {0.f, 0.f, 0.f, 0.f};
-    mma(l, a[k][0], b.x, b.y);
+  if (kApart) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) d[i] += l[i];
+  } else {
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const uint2 b = *reinterpret_cast<const uint2*>(block + k * stride + (threadIdx.x & 31) * 16);
+      mma(d, a[k][0], b.x, b.y);
+    }
   }
 }
 // zero where the mask's bits say so
@@ -531,7 +537,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) rowres_kernel(RowArgs a) {
         load_x(gr, 1, f[1]);
         auto states = [&] {
 #pragma unroll
-          for (int nt = 0; nt < kStateTiles; ++nt) products<2>(st[gr][nt], f, fv + nt * kBlockBytes, kStateTiles * kBlockBytes);
+          for (int nt = 0; nt < kStateTiles; ++nt) products<2, false>(st[gr][nt], f, fv + nt * kBlockBytes, kStateTiles * kBlockBytes);
         };
         // Causal rows: T's zeros do not keep a NaN or an infinity from the positions before it, and the products would make
         // up to 31 earlier outputs NaN.  A segment with one takes its outputs from the finite values alone, NaN from there
@@ -569,8 +575,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1) rowres_kernel(RowArgs a) {
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
           float y[2][4];
-          products<2>(y[0], f, ft + 2 * half * kBlockBytes, 4 * kBlockBytes);
-          products<2>(y[1], f, ft + (2 * half + 1) * kBlockBytes, 4 * kBlockBytes);
+          products<2, true>(y[0], f, ft + 2 * half * kBlockBytes, 4 * kBlockBytes);
+          products<2, true>(y[1], f, ft + (2 * half + 1) * kBlockBytes, 4 * kBlockBytes);
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             float4* at = reinterpret_cast<float4*>(xs + 4 * piece(seg_of(gr, h), 4 * half + t, rs));
@@ -662,8 +668,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1) rowres_kernel(RowArgs a) {
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         float y[2][4];
-        products<kStateK>(y[0], f, fe + 2 * half * kBlockBytes, 4 * kBlockBytes);
-        products<kStateK>(y[1], f, fe + (2 * half + 1) * kBlockBytes, 4 * kBlockBytes);
+        products<kStateK, true>(y[0], f, fe + 2 * half * kBlockBytes, 4 * kBlockBytes);
+        products<kStateK, true>(y[1], f, fe + (2 * half + 1) * kBlockBytes, 4 * kBlockBytes);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           float4* at = reinterpret_cast<float4*>(xs + 4 * piece(seg_of(gr, h), 4 * half + t, rs));
