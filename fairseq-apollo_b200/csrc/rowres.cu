@@ -18,9 +18,9 @@
 // 6.8e-8; omega on T's diagonal, one accumulator and taps summed in fp32: 1.2e-7 and 8.3e-8; each tile's leading products
 // added by themselves: 9.3e-8 and 6.1e-8, at 717 us where the case below takes 686).
 //
-// B = 32, D = 256, L = 16384 fp32 bidirectional after the norm: 1310 us as a walk (FMA, one row per SM), 590 us now (650
-// padded by up to half): the tensor pipe is at 45 %, issue slots at 40 %, the rest is latency, 16 warps being what the
-// registers allow.  L = 1024, B = 32, D = 128: 37 us.
+// B = 32, D = 256, L = 16384 fp32 bidirectional after the norm: 1310 us as a walk (FMA, one row per SM), 609 us now (691
+// padded by up to half): the tensor pipe is at 48 %, shared memory at 55 %, issue slots at 41 %, the rest is latency, 16
+// warps being what the registers allow.  L = 1024, B = 32, D = 128: 42 us.  (L2 flushed in front of each call.)
 #include <algorithm>
 #include <type_traits>
 
