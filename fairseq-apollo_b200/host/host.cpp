@@ -979,8 +979,8 @@ std::tuple<Tensor, Tensor, Tensor> block_infer(Tensor x, Tensor xn, Tensor mx, c
   x = x.contiguous();
   const Tensor xn2 = xn.contiguous().view({rows, d}), mx2 = mx.contiguous().view({rows, d});
   // (score rows and reduction indices in whole 16-byte pieces: the library's products are several times faster on them;
-  // the positions in between are of no row's causal range, and their values zero.  It takes a launch for each chunk, so at 32 chunks the two
-  // are level: 32 of 500 take 615 us with the pitch, 33 of 500 take 605 without)
+  // the positions in between are of no row's causal range, and their values zero.  It takes a launch for each chunk, so at 32
+  // chunks the two are level: 32 of 500 take 615 us with the pitch, 33 of 500 take 605 without)
   const int64_t pitch = period % 8 && nb <= 32 ? (period + 7) / 8 * 8 : period;
   Tensor v_lin = at::addmm(bv, xn2, wv.t()), v3 = v_lin.view({nb, period, e}), vp = v3;
   if (pitch != period) {
@@ -1023,8 +1023,9 @@ Tensor block_train(const Tensor& x, const Tensor& xn, const Tensor& mx, const Te
 // and the same library call took 6.6 us through the interpreter and ctypes, 2 us here.
 //
 // A plan is everything a step passes to the library, and what it was built from: it holds as long as the parameters
-// (identity, version counters and storage: p.data = t, which is also how a module is moved, leaves the first two alone), the state tensors, the batch, the dtype and the options stay what they were.  The
-// state tensors are updated in place, except the counts: one array is read, another written, and they alternate.
+// (identity, version counters and storage: p.data = t, which is also how a module is moved, leaves the first two alone), the
+// state tensors, the batch, the dtype and the options stay what they were.  The state tensors are updated in place, except
+// the counts: one array is read, another written, and they alternate.
 struct Names {
   PyObject *params, *modules, *groups, *bidirectional, *plan, *block_plan, *count, *mean, *var, *h, *key, *value, *key_mask,
       *forward, *hooks, *pre_hooks;
@@ -1058,6 +1059,7 @@ struct StepPlan {
   py::object nkey, ekey, groups, activation;
   py::object count, count_next, mean, var, h;
   std::vector<Tensor> operands;            // gamma, beta, p, q, g, omega (fp32)
+  bool kept = false;                       // (below)
   Tensor count_t, next_t, mean_t, var_t, h_t;
   int dtype, device, ndim, cplx, normed;
   int64_t batch, dim;
@@ -1092,6 +1094,20 @@ bool params_match(const StepPlan& p, PyObject* dict, size_t from, size_t to) {
 
 // norm_ema_step(norm, move, x, incremental_state, activation, return_normed): the outputs, or None when the layer has
 // no plan for this call
+// A graph that holds a step works on the state's tensors, which whoever replays it has to keep, and on the plan's, which go
+// with the plan: with the next generation, or a change of mode.  Those stay as long as the pole states then.
+void keep_with_state(StepPlan& p) {
+  using Kept = std::unordered_map<PyObject*, std::pair<py::object, std::vector<Tensor>>>;
+  static Kept* const all = new Kept;
+  PyObject* const h = p.h.ptr();
+  auto& kept = (*all)[h];
+  if (!kept.first) kept.first = py::weakref(h, py::cpp_function([h](py::handle) { all->erase(h); }));
+  kept.second.insert(kept.second.end(), p.operands.begin(), p.operands.end());
+  kept.second.push_back(p.count_t);
+  kept.second.push_back(p.next_t);
+  p.kept = true;
+}
+
 PyObject* norm_ema_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
   try {
     if (n != 6) throw py::type_error("norm_ema_step takes 6 arguments");
@@ -1125,6 +1141,7 @@ PyObject* norm_ema_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
     }
     const c10::cuda::CUDAGuard guard((c10::DeviceIndex)p.device);
     void* stream = at::cuda::getCurrentCUDAStream((c10::DeviceIndex)p.device).stream();
+    if (!p.kept && c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) keep_with_state(p);
     auto like = [&] { return Tensor(at::detail::empty_cuda(x.sizes(), x.scalar_type(), x.device(), std::nullopt)); };
     Tensor y = like(), xn = p.normed ? like() : Tensor();
     const auto& o = p.operands;

@@ -92,12 +92,12 @@ def sequence_norm_ema(norm: SequenceNorm, move: MultiHeadEMA, x: Tensor, padding
 
 def _ema_params(move: MultiHeadEMA):
     """(p, q, gamma, omega) of the layer, fp32 and contiguous.  Outside of training they are kept until a parameter
-    changes (identity, version counter, storage), the layer is moved or its mode is set; never across streams, nor from a
-    call that is only being captured."""
+    changes (identity, version counter, storage), the layer is moved or its mode is set; never across streams, nor in a
+    graph that is being captured: it has its own, which stay as long as it does."""
     third = move.theta if move.complex else move.beta
     tensors = (move.alpha, move.delta, third, move.gamma, move.omega)
     key = None
-    if not move.training:
+    if not move.training and not torch.cuda.is_current_stream_capturing():
         key = [_raw_stream(move.alpha.get_device())] + [t._version for t in tensors] + [t.data_ptr() for t in tensors]
         cache = move.__dict__.get("_decode_cache")
         if cache is not None and cache[0] == key and all(a is b for a, b in zip(cache[2], tensors)):
@@ -108,7 +108,7 @@ def _ema_params(move: MultiHeadEMA):
     else:
         p, q, g = ops.ema_coeffs(move.alpha, move.delta, move.beta, move.gamma)
     prm = (p, q, g, move.omega.detach().float().reshape(-1).contiguous())
-    if key is not None and not torch.cuda.is_current_stream_capturing():
+    if key is not None:
         move._decode_cache = (key, prm, tensors)
     return prm
 

@@ -206,3 +206,61 @@ def test_chunk_is_laid_out_as_it_fills():
         got += [blk(x[:, t:t + 1].contiguous(), incremental_state=inc)[0] for t in range(8, 600)]
         want = blk(x)[0]
     assert rel_l2(torch.cat(got, 1), want) < 1e-2
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("length", [1, 24])
+def test_graph_outlives_what_a_layer_keeps(cplx, length):
+    """A captured call replayed after another generation and a change of mode, with what they gave back taken by others."""
+    import fairseq_apollo_b200 as M
+    blk = _block(M, cplx)
+    x = torch.randn(2, length, 64, device="cuda").bfloat16()
+
+    def call(inc):
+        return M.timestep_norm_ema(blk.norm, blk.move, x, None, inc, "silu", True)
+
+    with torch.no_grad():
+        want, inc = {}, {}
+        for _ in range(2):
+            call(want)
+            call(inc)
+        state = {key: dict(own) for key, own in inc.items()}   # (what the graph starts from is the caller's to keep)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = call(inc)
+        for _ in range(2):
+            call({})
+        blk.train()
+        blk.eval()
+        gc.collect()
+        junk = [torch.full((n,), float("nan"), device="cuda") for n in (16, 64, 128, 1024, 2048, 4096) for _ in range(16)]
+        graph.replay()
+        ref = call(want)
+    torch.cuda.synchronize()
+    del junk, state
+    for a, b in zip(got, ref):
+        assert torch.equal(a, b)
+    for name in want:
+        for key, t in want[name].items():
+            assert torch.equal(inc[name][key], t), key
+
+
+def test_what_a_graph_reads_goes_with_the_state():
+    import fairseq_apollo_b200 as M
+    blk = _block(M)
+    x = torch.randn(2, 1, 64, device="cuda").bfloat16()
+    with torch.no_grad():
+        M.timestep_norm_ema(blk.norm, blk.move, x, None, {})
+        gc.collect()
+        before = torch.cuda.memory_allocated()
+        inc = {}
+        M.timestep_norm_ema(blk.norm, blk.move, x, None, inc)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            M.timestep_norm_ema(blk.norm, blk.move, x, None, inc)
+        M.timestep_norm_ema(blk.norm, blk.move, x, None, {})
+        held = torch.cuda.memory_allocated()
+        graph.reset()
+        del graph, inc
+        gc.collect()
+        assert torch.cuda.memory_allocated() < held and torch.cuda.memory_allocated() <= before
