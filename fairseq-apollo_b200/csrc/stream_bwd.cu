@@ -1,8 +1,8 @@
 // Streamed backward kernels for channel-contiguous activations ((B, L, D) memory): the per-feature TimestepNorm from
-// statistics saved by its forward, and the causal EMA with states carried in or out.  Same data movement as the streamed forward kernels: a CTA owns kW adjacent channels of
-// one sequence, tiles of kR timesteps arrive through a TMA ring (cp.async.bulk.tensor + mbarrier) and the input gradient
-// leaves through TMA stores, so HBM sees whole row segments while every thread keeps its channel's recurrences in
-// registers.  The norm walks time backwards once.
+// statistics saved by its forward, and the causal EMA with states carried in or out.  Same data movement as the streamed
+// forward kernels: a CTA owns kW adjacent channels of one sequence, tiles of kR timesteps arrive through a TMA ring
+// (cp.async.bulk.tensor + mbarrier) and the input gradient leaves through TMA stores, so HBM sees whole row segments while
+// every thread keeps its channel's recurrences in registers.  The norm walks time backwards once.
 #include <mutex>
 
 #include "common.cuh"
