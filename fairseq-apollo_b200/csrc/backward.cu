@@ -8,6 +8,7 @@
 // so no state history is stored.  The anti-causal half of a bidirectional layer is the same
 // computation on the reversed sequence, delayed by one step when the kernel is shifted.
 // Four lanes share a (batch, channel) row and split its poles; sums over the batch are atomic adds.
+#include "chunk_ema.cuh"
 #include "common.cuh"
 #include "scan_ema.cuh"
 #include "scan_norm.cuh"
@@ -567,6 +568,7 @@ extern "C" int mega_ema_bwd(const void* dy, const void* x, void* dx, int dtype, 
     ca.bidir = bidir ? 1 : 0;
     ca.shift = (flags & MEGA_EMA_NO_SHIFT) ? 0 : 1;
     ca.dp = dp; ca.dq = dq; ca.dg = dgamma_hat; ca.domega = domega;
+    if (chunk_ema_bwd_try(dtype, ca, xsd, dsd, gsd, s)) return check_launch("ema_bwd(chunk)");
     if (scan_ema_bwd_try(dtype, ca, xsd, dsd, gsd, s)) return check_launch("ema_bwd(scan)");
   }
   if (!bidir) {   // states carried in or out (or what the scan does not take)

@@ -3,6 +3,7 @@
 // h_{n,t}) + omega x_t.  Evaluated as the recurrence itself: O(L) per row, one pass over x, no
 // length cap.  Four lanes share a (batch, channel) row and split its poles; the per-step output is
 // a two-shuffle reduction.
+#include "chunk_ema.cuh"
 #include "common.cuh"
 #include "stream_bwd.cuh"
 #include "stream_cl.cuh"
@@ -657,6 +658,7 @@ extern "C" int mega_cema_fwd(const void* x, void* y, int dtype, int B, int D, in
     ca.bidir = bidir ? 1 : 0;
     ca.shift = (flags & MEGA_EMA_NO_SHIFT) ? 0 : 1;
     ca.silu = (flags & MEGA_EMA_SILU) ? 1 : 0;
+    if (chunk_ema_fwd_try(dtype, dtype, ca, xsd, ysd, (cudaStream_t)stream)) return check_launch("cema_fwd(chunk)");
     if (!bidir && N <= 16 && !scan_cluster_first(dtype, ca, xsd, ysd)) {
       StreamArgs sa{};
       sa.B = B; sa.L = L; sa.D = D; sa.N = N;
@@ -805,6 +807,7 @@ extern "C" int mega_cema_bwd(const void* dy, const void* x, void* dx, int dtype,
     ca.bidir = bidir ? 1 : 0;
     ca.shift = (flags & MEGA_EMA_NO_SHIFT) ? 0 : 1;
     ca.dp = dp; ca.dq = dq; ca.dg = dgamma_hat; ca.domega = domega;
+    if (chunk_ema_bwd_try(dtype, ca, xsd, dsd, gsd, s)) return check_launch("cema_bwd(chunk)");
     if (scan_ema_bwd_try(dtype, ca, xsd, dsd, gsd, s)) return check_launch("cema_bwd(scan)");
   }
   CemaBwdArgs a{};

@@ -1,0 +1,1080 @@
+// The causal EMA and its backward as matrix products of chunks, parallel over time: real or complex poles, channels contiguous.
+//
+// With chunks of 16 positions, h the poles' states and everything below a matrix of the channel,
+//   states   h' = q^16 h + V x         V (16 x poles): q^(15-k)
+//   outputs  y  = T x + G h            T (16 x 16): the taps, omega on its diagonal; G (poles x 16): c q^(j+1)
+// and for the backward, l = sum_j q^j dy_j and w = sum_j j q^(j-1) dy_j of a chunk (V and its derivative U against dy in
+// reversed order), s = dh/dq (s' = q^16 s + 16 q^15 h + U x) and R_k the correlation of x and dy at lag k within chunks,
+//   sum_t dy_t h_t = q A1 + sum_k q^k R_k,          A1 = sum over chunks of l h
+//   sum_t dy_t s_t = q A2 + A1 + sum_k k q^(k-1) R_k,   A2 = sum over chunks of l s + w h,
+// while dx is the layer itself run over dy in reversed time.  So nothing is computed per position and pole: 16 + 16 + 16
+// multiply-adds per element forward (real), 64 + 16 backward beside them, all on the tensor pipe.
+//
+// fp32 on the bf16 tensor pipe: matrices, states and fp32 inputs go in as three bf16 parts, of whose products all but
+// those below 2^-24 are taken (split_mma.cuh); a bf16 input is one part, an fp16 one two.
+//
+// A sequence is cut into segments that run at the same time: (1) every segment but the last folds its inputs into a state
+// of its own, (2) a small launch carries the states over the segments, (3) outputs, and the sums of the parameters'
+// gradients.  A block takes eight segments of 16 (8) adjacent channels in tiles of 64 or 128 positions.  The tile comes with
+// asynchronous copies, is turned into rows along time as bf16 parts, and then a warp owns a channel: the rows of
+// its products are two consecutive chunks of the eight segments, so that states stay in a thread; matrices live in registers
+// (complex: some in shared memory) for the whole segment.  Two buffers let half of the warps turn tiles while the others
+// multiply.
+#include <algorithm>
+#include <cmath>
+#include <type_traits>
+
+#include "chunk_ema.cuh"
+#include "common.cuh"
+#include "scan_cluster.cuh"
+#include "scratch.cuh"
+#include "split_mma.cuh"
+#include "tma.cuh"
+#include "walk.cuh"
+
+namespace mega {
+
+namespace {
+
+enum Mode { kLocal, kLocalSens, kEmit, kGrad };   // local states; with their derivatives; outputs; sums of the gradients
+
+struct ChunkArgs {
+  ScanArgs a;
+  const void* in;           // what is walked, and its strides
+  long long isb, isl;
+  int T, S;                 // steps of a segment (a multiple of 64), segments of a sequence
+  int walked;               // of them, those that this launch takes
+  int rev;                  // time runs backwards
+  int parts, part;          // values per (sequence, segment) in the carry array, first one of this launch
+  float* carry;             // [B][S][parts][D][16]: what a segment starts from (of segment 0: unused)
+  const unsigned char* frag;   // [D][blocks] of kBlockBytes
+  int blocks;
+  const float* pow;         // [D][4][16]: q^16 (re, im), 16 q^15 (re, im)
+};
+
+template <typename T>
+constexpr int kPartsOf = sizeof(T) == 4 ? 3 : std::is_same<T, __half>::value ? 2 : 1;
+
+// blocks of a channel: V, [U], T, G
+template <bool kC>
+struct Blocks {
+  static constexpr int v = kC ? 4 : 2, t = 2, g = kC ? 4 : 2;
+};
+
+template <typename In, typename Out, bool kC, int kMode>
+struct Form {
+  static constexpr int kP = kPartsOf<In>;
+  // positions of a tile (what shared memory holds), and bytes of a row: eight rows hit different banks
+  static constexpr int kTile = (kP == 1 && !(kMode == kGrad && kC)) || (kP == 2 && !kC && kMode != kGrad) ? 128 : 64;
+  static constexpr int kRow = 2 * kTile + 16;
+  static constexpr int kCh = kMode == kGrad && kP == 3 ? 8 : 16;   // channels of a block, and its warps
+  static constexpr int kThreads = 32 * kCh;
+  static constexpr int kIns = kMode == kGrad ? 2 : 1;
+  static constexpr int kPlane = kCh * 8 * kRow;                    // bytes of one part of a tile
+  static constexpr int kBufs = (kMode == kGrad && (kP == 3 || (kP == 2 && kC))) || (kMode == kLocalSens && kP == 3 && kC) ? 1 : 2;
+  static constexpr int kV = Blocks<kC>::v;
+  static constexpr int kRegs = kMode == kEmit ? (kC ? Blocks<kC>::g : 2 * kV + 2) : kMode == kLocal ? kV : kC ? 0 : 2 * kV;
+  static constexpr int kAll = kMode == kEmit ? kV + Blocks<kC>::t + Blocks<kC>::g : kMode == kLocal ? kV : 2 * kV;
+  static constexpr int kShared = kAll - kRegs;                     // matrices in shared memory (the first ones)
+  static constexpr int kE = 16 / (int)sizeof(In), kPos = kTile / (4 * kE);  // channels of a 16-byte piece; positions of a thread
+  static constexpr int kSlot = kIns * kPos * kThreads * 16;        // bytes of a tile as it arrives
+  static constexpr int stage = kBufs * kIns * kP * kPlane;
+  static constexpr int fixed = stage + kShared * kCh * kBlockBytes;
+  static constexpr int kSlots = fixed + 2 * kSlot <= (kCh == 8 ? 112 : 226) * 1024 ? 2 : 1;
+  static constexpr int mats = stage + kSlots * kSlot;
+  static constexpr int total = mats + kShared * kCh * kBlockBytes;
+  static constexpr int kPerSm = kCh == 8 && total <= 112 * 1024 ? 2 : 1;
+  static_assert(total <= 227 * 1024, "a block's shared memory");
+};
+
+// byte offset of (channel, segment, 16-position block): blocks of a row in an order that differs between the channels a
+// warp writes at once
+template <int kRow>
+__device__ __forceinline__ int row_at(int ch, int seg, int blk) { return (ch * 8 + seg) * kRow + ((blk ^ ((ch >> 2) & 3)) << 5); }
+
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+  uint32_t r;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
+  return r;
+}
+__device__ __forceinline__ void ldmatrix(uint32_t (&f)[4], uint32_t at) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(f[0]), "=r"(f[1]), "=r"(f[2]), "=r"(f[3]) : "r"(at) : "memory");
+}
+__device__ __forceinline__ void ldmatrix_t(uint32_t (&f)[4], uint32_t at) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(f[0]), "=r"(f[1]), "=r"(f[2]), "=r"(f[3]) : "r"(at) : "memory");
+}
+
+// the lower bf16 of a pair (as a shift it would become a multiplication, which costs more issue slots)
+__device__ __forceinline__ float lower(uint32_t p) { return __uint_as_float(prmt(p, 0u, 0x1044)); }
+// scalar form of split3: next to other fp32 work a packed operation costs what it saves
+__device__ __forceinline__ void split(float lo, float hi, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
+  p0 = bf16_pair(lo, hi);
+  lo -= lower(p0);
+  hi -= __uint_as_float(p0 & 0xffff0000u);
+  p1 = bf16_pair(lo, hi);
+  p2 = bf16_pair(lo - lower(p1), hi - __uint_as_float(p1 & 0xffff0000u));
+}
+// Product j, smallest first, of those of a (kP parts) with a block: the leading one is the last.  (Callers go through the
+// products of several independent sums in turn, so that none waits for the one before it.)
+template <int kP>
+constexpr int kTerms = kP == 1 ? 3 : kP == 2 ? 5 : 6;
+template <int kP>
+__device__ __forceinline__ void term(int j, bool onto, float (&d)[4], const uint32_t (&a)[kP][4], const Frag& b) {
+  constexpr int kOf[3][6][2] = {{{0, 2}, {0, 1}, {0, 0}}, {{0, 2}, {1, 1}, {1, 0}, {0, 1}, {0, 0}}, {{0, 2}, {2, 0}, {1, 1}, {1, 0}, {0, 1}, {0, 0}}};
+  const int p = kOf[kP - 1][j][0], q = kOf[kP - 1][j][1];
+  const uint32_t b0 = q == 0 ? b.u.x : q == 1 ? b.u.z : b.v.x, b1 = q == 0 ? b.u.y : q == 1 ? b.u.w : b.v.y;
+  if (onto) mma(d, a[p], b0, b1);
+  else mma0(d, a[p], b0, b1);
+}
+
+// A thread's share of the tiles: kPos positions of kE channels of one segment.
+template <typename E, int kCh, int kTile>
+struct Share {
+  static constexpr int kRow = 2 * kTile + 16;
+  static constexpr int kE = 16 / (int)sizeof(E), kPos = kTile / (4 * kE), kCols = kCh / kE, kGroups = kTile / kPos;
+  int left;         // positions of the segment from the share's next piece on (<= 0: none)
+  int at[2];        // where its channels' rows take them: the first four, the others
+  long long step;   // bytes from a position to the next
+  char* next;
+  __device__ __forceinline__ Share(const ChunkArgs& s, int id, const void* base, long long sb, long long sl, bool back) {
+    const int col = id % kCols, pg = id / kCols % kGroups, seg = id / (kCols * kGroups);
+    const int row = blockIdx.y * 8 + seg, c = blockIdx.x * kCh + col * kE;
+    const int b = row / s.walked, first = (row - b * s.walked) * s.T;
+    const bool ok = b < s.a.B && c < s.a.D;
+    const int t = first + pg * kPos, pos = pg * kPos, in = back ? 16 - kPos - (pos & 15) : pos & 15;
+    left = ok ? min(s.T, s.a.L - first) - pos : 0;
+    step = (s.rev ? -sl : sl) * (long long)sizeof(E);
+    next = (char*)base + (ok ? b * sb + (s.rev ? s.a.L - 1 - t : t) * sl + c : 0) * (long long)sizeof(E);
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      at[i] = row_at<kRow>(col * kE + (kE == 8 ? 4 * i : 0), seg, pos >> 4) + in * 2 - (kE == 8 ? 4 * i * 8 * kRow : 0);
+  }
+  __device__ __forceinline__ int row(int j) const { return at[j >> 2] + j * 8 * kRow; }   // of channel j
+  __device__ __forceinline__ void advance() {
+    left -= kTile;
+    next += kTile * step;
+  }
+  // its pieces of a tile on their way (zeros where the segment has ended: nothing is read there)
+  __device__ __forceinline__ void fetch(uint32_t slot) {
+    const char* from = next;
+#pragma unroll
+    for (int k = 0; k < kPos; ++k, from += step)
+      asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16, %2;" ::"r"(slot + k * 32 * kCh * 16), "l"(from), "r"(k < left ? 16 : 0)
+                   : "memory");
+    advance();
+  }
+};
+
+// kPos 16-bit values of a row, kPos / 2 words
+template <int kPos>
+struct alignas(2 * kPos) Words {
+  uint32_t v[kPos / 2];
+};
+
+// A thread's pieces into the rows of the buffer; kBack: the positions of a 16-position block in reversed order.
+template <typename E, int kCh, int kTile, int kP, int kPlane, bool kBack>
+__device__ __forceinline__ void turn(const Share<E, kCh, kTile>& sh, const unsigned char* slot, unsigned char* buf) {
+  constexpr int kPos = Share<E, kCh, kTile>::kPos, kE = Share<E, kCh, kTile>::kE;
+  uint32_t w[kPos][4];
+#pragma unroll
+  for (int k = 0; k < kPos; ++k) {
+    const uint4 v = *reinterpret_cast<const uint4*>(slot + (kBack ? kPos - 1 - k : k) * 32 * kCh * 16);
+    w[k][0] = v.x; w[k][1] = v.y; w[k][2] = v.z; w[k][3] = v.w;
+  }
+#pragma unroll
+  for (int j = 0; j < kE; ++j) {
+    Words<kPos> part[kP];
+#pragma unroll
+    for (int i = 0; i < kPos / 2; ++i) {
+      if constexpr (sizeof(E) == 4) {
+        split(__uint_as_float(w[2 * i][j & 3]), __uint_as_float(w[2 * i + 1][j & 3]), part[0].v[i], part[1 % kP].v[i], part[2 % kP].v[i]);
+      } else {
+        uint32_t v = prmt(w[2 * i][j >> 1], w[2 * i + 1][j >> 1], j & 1 ? 0x7632 : 0x5410);
+        if constexpr (kP == 2) {   // fp16: its leading eight bits, and the rest
+          const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&v));
+          v = bf16_pair(f.x, f.y);
+          part[1].v[i] = bf16_pair(f.x - __uint_as_float(v << 16), f.y - __uint_as_float(v & 0xffff0000u));
+        }
+        part[0].v[i] = v;
+      }
+    }
+#pragma unroll
+    for (int p = 0; p < kP; ++p) *reinterpret_cast<Words<kPos>*>(buf + sh.row(j) + p * kPlane) = part[p];
+  }
+}
+
+// A thread's share of the outputs, from the rows of the buffer (fp32: upper and lower halves in the first two parts).
+template <typename E, int kCh, int kTile, int kPlane>
+__device__ __forceinline__ void put(Share<E, kCh, kTile>& sh, const unsigned char* buf) {
+  constexpr int kPos = Share<E, kCh, kTile>::kPos, kE = Share<E, kCh, kTile>::kE;
+  Words<kPos> hi[kE], lo[sizeof(E) == 4 ? kE : 1];
+#pragma unroll
+  for (int j = 0; j < kE; ++j) {
+    hi[j] = *reinterpret_cast<const Words<kPos>*>(buf + sh.row(j));
+    if constexpr (sizeof(E) == 4) lo[j] = *reinterpret_cast<const Words<kPos>*>(buf + sh.row(j) + kPlane);
+  }
+  char* to = sh.next;
+#pragma unroll
+  for (int k = 0; k < kPos; ++k, to += sh.step) {
+    auto word = [&](int i) {
+      if constexpr (sizeof(E) == 4) return prmt(lo[i].v[k >> 1], hi[i].v[k >> 1], k & 1 ? 0x7632 : 0x5410);
+      else return prmt(hi[2 * i].v[k >> 1], hi[2 * i + 1].v[k >> 1], k & 1 ? 0x7632 : 0x5410);
+    };
+    if (k < sh.left) *reinterpret_cast<uint4*>(to) = make_uint4(word(0), word(1), word(2), word(3));
+  }
+  sh.advance();
+}
+
+// ---- the matrices of a channel --------------------------------------------------------------------------------
+// A warp per channel; powers in double, rounded once.  sens: U behind V; outs: T and G behind those; gain: the input gain p
+// is V's (states as the layer exports them) instead of G's; om: omega on T's diagonal.
+struct PrepArgs {
+  const float *p, *q, *g, *omega;
+  int D, N, sens, outs, gain, om, blocks;
+  unsigned char* frag;
+  float* pow;
+};
+template <bool kC>
+__global__ void __launch_bounds__(128) chunk_prepare_kernel(PrepArgs a) {
+  __shared__ double2 table[4][17][16];
+  __shared__ float taps[4][16];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, d = blockIdx.x * 4 + warp;
+  if (d >= a.D) return;
+  double2(&pw)[17][16] = table[warp];
+  const int n = lane & 15;
+  const size_t at = (size_t)d * a.N + n;
+  const bool live = n < a.N;
+  double qr = 0., qi = 0., wr = 0., wi = 0.;   // pole; output weight p g
+  if (live) {
+    const double p = a.p[at];
+    qr = kC ? a.q[2 * at] : a.q[at];
+    wr = p * (kC ? a.g[2 * at] : a.g[at]);
+    if (kC) {
+      qi = a.q[2 * at + 1];
+      wi = p * a.g[2 * at + 1];
+    }
+  }
+  double vr = 1., vi = 0.;
+  for (int e = 0; e <= 16; ++e) {
+    if (lane < 16) pw[e][n] = make_double2(vr, vi);
+    if (e < 16 && a.outs) {
+      double tap = wr * vr - wi * vi;
+#pragma unroll
+      for (int s = 8; s > 0; s >>= 1) tap += __shfl_xor_sync(0xffffffffu, tap, s);
+      if (lane == 0) taps[warp][e] = (float)(e == 0 && a.om ? tap + a.omega[d] : tap);
+    }
+    const double r = vr * qr - vi * qi;
+    vi = vr * qi + vi * qr;
+    vr = r;
+  }
+  __syncwarp();
+  if (lane < 16) {
+    float* pc = a.pow + (size_t)d * 64 + n;
+    pc[0] = (float)pw[16][n].x;
+    pc[16] = (float)pw[16][n].y;
+    pc[32] = (float)(16. * pw[15][n].x);
+    pc[48] = (float)(16. * pw[15][n].y);
+  }
+  constexpr int kV = Blocks<kC>::v;
+  const int g = lane >> 2, t = lane & 3;
+  const int us = kV, ts = us + (a.sens ? kV : 0), gs = ts + 2;
+  for (int blk = 0; blk < a.blocks; ++blk) {
+    float v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int k = 2 * t + (i & 1) + 8 * (i >> 1);
+      double x;
+      if (blk < ts) {
+        const int nt = blk < us ? blk : blk - us, pole = 8 * (nt & 1) + g, e = 15 - k;
+        const bool sens = blk >= us;
+        const double2 w = pw[sens ? max(e - 1, 0) : e][pole];
+        x = nt < 2 ? w.x : w.y;
+        if (sens) x *= e;
+        if (pole >= a.N) x = 0.;
+        else if (a.gain) x *= a.p[(size_t)d * a.N + pole];
+      } else if (blk < gs) {
+        const int lag = 8 * (blk - ts) + g - k;
+        x = lag >= 0 ? taps[warp][lag] : 0.f;
+      } else {
+        const int kt = (blk - gs) >> 1, j = 8 * ((blk - gs) & 1) + g;
+        const size_t row = (size_t)d * a.N + k;
+        double cr = 0., ci = 0.;
+        if (k < a.N) {
+          const double p = a.gain ? 1. : (double)a.p[row];
+          cr = p * (kC ? a.g[2 * row] : a.g[row]);
+          if (kC) ci = p * a.g[2 * row + 1];
+        }
+        const double2 w = pw[j + 1][k];
+        x = kt == 0 ? cr * w.x - ci * w.y : -(cr * w.y + ci * w.x);
+      }
+      v[i] = (float)x;
+    }
+    store_frag(a.frag + ((size_t)d * a.blocks + blk) * kBlockBytes, v);
+  }
+}
+
+// ---- the walk ----------------------------------------------------------------------------------------------
+template <typename In, typename Out, bool kC, int kMode>
+__global__ void __launch_bounds__(Form<In, Out, kC, kMode>::kThreads, Form<In, Out, kC, kMode>::kPerSm) chunk_kernel(ChunkArgs s) {
+  using F = Form<In, Out, kC, kMode>;
+  constexpr int kP = F::kP, kV = F::kV, kPlane = F::kPlane, kCh = F::kCh, kTile = F::kTile, kRow = F::kRow;
+  constexpr int kRe = kC ? 2 : 1;      // real numbers of a value
+  constexpr bool kSens = kMode == kLocalSens || kMode == kGrad;
+  constexpr bool kApart = kMode == kEmit && sizeof(Out) == 4;   // omega x in fp32: the tensor pipe truncates its sums
+  extern __shared__ __align__(16) unsigned char smem[];
+  const ScanArgs& a = s.a;
+  int tid;
+  asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));   // (read once: it is used in every tile)
+  const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int d = blockIdx.x * kCh + warp, dc = min(d, a.D - 1);
+  Share<In, kCh, kTile> sh(s, tid, s.in, s.isb, s.isl, false);
+  Share<In, kCh, kTile> sg(s, tid, a.dy, a.gsb, a.gsl, true);
+  Share<Out, kCh, kTile> so(s, tid, a.y, a.ysb, a.ysl, false);
+  // the row of this lane's states, and the longest one
+  const int row = blockIdx.y * 8 + g, b = row / s.walked, seg = row - b * s.walked;
+  const bool live = b < a.B && d < a.D;
+  const int len = b < a.B ? min(s.T, a.L - seg * s.T) : 0;
+  const int most = __reduce_max_sync(0xffffffffu, len);
+  const int steps = (most + 31) / 32, tiles = (most + kTile - 1) / kTile;
+
+  const uint32_t stage = smem_u32(smem) + F::stage + tid * 16;
+  auto issue = [&](int tile) {
+    if (tile < tiles) {
+      const uint32_t slot = stage + tile % F::kSlots * F::kSlot;
+      sh.fetch(slot);
+      if constexpr (F::kIns == 2) sg.fetch(slot + F::kSlot / 2);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int i = 0; i < F::kSlots; ++i) issue(i);
+
+  // matrices and powers
+  const unsigned char* mats = s.frag + (size_t)dc * s.blocks * kBlockBytes;
+  const unsigned char* own = smem + F::mats + warp * F::kShared * kBlockBytes;
+  const int skip = kMode == kEmit ? s.blocks - F::kAll : 0;   // (U, where the call has it, lies between V and T)
+  if constexpr (F::kShared > 0) {
+    unsigned char* to = smem + F::mats + warp * F::kShared * kBlockBytes;
+    for (int blk = 0; blk < F::kShared; ++blk) {
+      const unsigned char* from = mats + (blk >= kV ? blk + skip : blk) * kBlockBytes;
+      reinterpret_cast<uint4*>(to + blk * kBlockBytes)[lane] = __ldg(reinterpret_cast<const uint4*>(from) + lane);
+      reinterpret_cast<uint2*>(to + blk * kBlockBytes + 512)[lane] = __ldg(reinterpret_cast<const uint2*>(from + 512) + lane);
+    }
+    __syncwarp();
+  }
+  Frag held[F::kRegs > 0 ? F::kRegs : 1];
+#pragma unroll
+  for (int i = 0; i < F::kRegs; ++i) {
+    const int blk = F::kShared + i, at = blk >= kV ? blk + skip : blk;
+    held[i] = {__ldg(reinterpret_cast<const uint4*>(mats + at * kBlockBytes) + lane),
+               __ldg(reinterpret_cast<const uint2*>(mats + at * kBlockBytes + 512) + lane)};
+  }
+  auto matrix = [&](int blk) -> Frag {   // (blk is a constant wherever this is called)
+    if (blk < F::kShared) return load_frag(own + blk * kBlockBytes);
+    return held[blk - F::kShared];
+  };
+  // poles of a lane: 8 i + 2 t + e
+  float qr[4], qi[kC ? 4 : 1], ur[kSens ? 4 : 1], ui[kSens && kC ? 4 : 1];
+  const float* pw = s.pow + (size_t)dc * 64;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int n = 8 * (i >> 1) + 2 * t + (i & 1);
+    qr[i] = __ldg(pw + n);
+    if (kC) qi[kC ? i : 0] = __ldg(pw + 16 + n);
+    if (kSens) ur[kSens ? i : 0] = __ldg(pw + 32 + n);
+    if (kSens && kC) ui[kSens && kC ? i : 0] = __ldg(pw + 48 + n);
+  }
+  const float om = kApart ? __ldg(a.omega + dc) : 0.f;
+
+  // states that the segment starts from
+  auto carry_at = [&](int at, int part) { return s.carry + (((size_t)(b * s.S + at) * s.parts + s.part + part) * a.D + d) * 16 + 2 * t; };
+  float h[kRe][4], sn[kSens ? kRe : 1][4];
+#pragma unroll
+  for (int c = 0; c < kRe; ++c)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      h[c][i] = 0.f;
+      if (kSens) sn[kSens ? c : 0][i] = 0.f;
+    }
+  if ((kMode == kEmit || kMode == kGrad) && live) {
+    if (seg > 0) {
+#pragma unroll
+      for (int c = 0; c < kRe; ++c)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const float2 v = __ldg(reinterpret_cast<const float2*>(carry_at(seg, c) + 8 * k));
+          h[c][2 * k] = v.x;
+          h[c][2 * k + 1] = v.y;
+          if (kSens) {
+            const float2 u = __ldg(reinterpret_cast<const float2*>(carry_at(seg, kRe + c) + 8 * k));
+            sn[kSens ? c : 0][2 * k] = u.x;
+            sn[kSens ? c : 0][2 * k + 1] = u.y;
+          }
+        }
+    } else if (kMode == kEmit && a.h_in) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int n = 8 * (i >> 1) + 2 * t + (i & 1);
+        const size_t at = ((size_t)b * a.D + d) * a.N + n;
+        if (n < a.N) {
+          h[0][i] = __ldg(a.h_in + kRe * at);
+          if (kC) h[kRe - 1][i] = __ldg(a.h_in + kRe * at + 1);
+        }
+      }
+    }
+  }
+  // q^16 h + v of pole i
+  auto next = [&](int i, float& re, float& im, float vr, float vi) {
+    if (kC) {
+      const float r = fmaf(qr[i], re, fmaf(-qi[kC ? i : 0], im, vr));
+      im = fmaf(qi[kC ? i : 0], re, fmaf(qr[i], im, vi));
+      re = r;
+    } else {
+      re = fmaf(qr[i], re, vr);
+    }
+  };
+  // kGrad: A1 and A2 of the lane's poles, R of its entries
+  float a1[kMode == kGrad ? kRe : 1][4] = {}, a2[kMode == kGrad ? kRe : 1][4] = {}, R[kMode == kGrad ? 8 : 1] = {};
+
+  // eight rows of 16 bytes each: segments, their first or second chunk, lower or upper half of it
+  const int blk_in = (lane >> 3) & 1;
+  const uint32_t frag_row = smem_u32(smem) + (warp * 8 + (lane & 7)) * kRow + (lane >> 4) * 16;
+  const int swz = ((warp >> 2) & 3) << 5;
+  unsigned char* mine = smem + (warp * 8 + g) * kRow + 4 * t;   // (of the rows g and g + 8: outputs)
+  const int final = kMode == kEmit && a.h_out != nullptr && live && seg == s.S - 1 ? (len - 1) / 32 : -1;   // step whose end leaves
+
+  // kStep steps of 32 positions at a time: their products do not wait for each other, only their states do
+  constexpr int kStep = kMode == kGrad && kC ? 1 : 2;
+  auto multiply = [&](int tile) {
+    const int buf = tile % F::kBufs * F::kIns * kP * kPlane;
+    const int n = min(kTile / 32, steps - kTile / 32 * tile), last = final - kTile / 32 * tile;
+#pragma unroll 1
+    for (int s0 = 0; s0 < n; s0 += kStep) {
+      const int first = (s0 << 6) ^ swz;   // of the first step's two blocks; the other one lies 32 bytes up or down
+      auto rows = [&](int st) { return frag_row + buf + ((first ^ (st << 6)) ^ (blk_in << 5)); };
+      uint32_t f[kStep][kP][4];
+#pragma unroll
+      for (int st = 0; st < kStep; ++st)
+#pragma unroll
+        for (int p = 0; p < kP; ++p) ldmatrix(f[st][p], rows(st) + p * kPlane);
+      if constexpr (kMode == kLocal || kMode == kLocalSens) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {   // eight poles at a time
+          float v[kStep][kRe][4], u[kStep][kSens ? kRe : 1][4];
+#pragma unroll
+          for (int j = 0; j < kTerms<kP>; ++j)
+#pragma unroll
+            for (int c = 0; c < kRe; ++c)
+#pragma unroll
+              for (int st = 0; st < kStep; ++st) {
+                term<kP>(j, j > 0, v[st][c], f[st], matrix(2 * c + k));
+                if (kSens) term<kP>(j, j > 0, u[st][kSens ? c : 0], f[st], matrix((kSens ? kV : 0) + 2 * c + k));
+              }
+#pragma unroll
+          for (int m = 0; m < 4 * kStep; ++m) {   // (in the order of time: steps, chunks, for two poles)
+            const int st = m >> 2, i = 2 * k + (m & 1), at = m & 3;
+            if (kSens) {   // s' = q^16 s + 16 q^15 h + U x
+              float xr = u[st][0][at], xi = kC ? u[st][kSens ? kRe - 1 : 0][at] : 0.f;
+              xr = fmaf(ur[kSens ? i : 0], h[0][i], xr);
+              if (kC) {
+                xr = fmaf(-ui[kSens && kC ? i : 0], h[kRe - 1][i], xr);
+                xi = fmaf(ur[kSens ? i : 0], h[kRe - 1][i], fmaf(ui[kSens && kC ? i : 0], h[0][i], xi));
+              }
+              next(i, sn[0][i], sn[kSens ? kRe - 1 : 0][i], xr, xi);
+            }
+            next(i, h[0][i], h[kRe - 1][i], v[st][0][at], v[st][kRe - 1][at]);
+          }
+        }
+      } else if constexpr (kMode == kEmit) {
+        float v[kStep][2][kRe][4];
+        float odd = 0.f;   // NaN where a row holds an infinity or a NaN
+#pragma unroll
+        for (int j = 0; j < kTerms<kP>; ++j)
+#pragma unroll
+          for (int k = 0; k < 2; ++k)
+#pragma unroll
+            for (int c = 0; c < kRe; ++c)
+#pragma unroll
+              for (int st = 0; st < kStep; ++st) term<kP>(j, j > 0, v[st][k][c], f[st], matrix(2 * c + k));
+#pragma unroll
+        for (int st = 0; st < kStep; ++st) {
+          odd = fmaf(v[st][0][0][0], 0.f, fmaf(v[st][0][0][2], 0.f, odd));
+          // (a state that is exported is that of the segment's last position, wherever in a step it lies: position by position)
+          if (s0 + st == last) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int m = 8 * (i >> 1) + 2 * t + (i & 1);
+              const size_t row_n = (size_t)d * a.N + m;
+              if (m >= a.N) continue;
+              const float p = __ldg(a.p + row_n), fr = __ldg(a.q + kRe * row_n), fi = kC ? __ldg(a.q + kRe * row_n + 1) : 0.f;
+              float re = h[0][i], im = h[kRe - 1][i];
+              for (int k = 0; k < len - 32 * final; ++k) {
+                const unsigned char* from = smem + buf + row_at<kRow>(warp, g, 2 * (s0 + st) + (k >> 4)) + (k & 15) * 2;
+                float x = 0.f;
+#pragma unroll
+                for (int pl = kP - 1; pl >= 0; --pl) x += __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(from + pl * kPlane));
+                x *= p;
+                const float r = kC ? fmaf(fr, re, fmaf(-fi, im, x)) : fmaf(fr, re, x);
+                if (kC) im = fmaf(fr, im, fi * re);
+                re = r;
+              }
+              const size_t o = ((size_t)b * a.D + d) * a.N + m;
+              a.h_out[kRe * o] = re;
+              if (kC) a.h_out[kRe * o + 1] = im;
+            }
+          }
+#pragma unroll
+          for (int m = 0; m < 8; ++m) {   // what enters the chunks, in the place of what they add
+            const int i = m & 3, k = i >> 1, at = 2 * (m >> 2) + (i & 1);
+            const float vr = v[st][k][0][at], vi = v[st][k][kRe - 1][at];
+            v[st][k][0][at] = h[0][i];
+            if (kC) v[st][k][kRe - 1][at] = h[kRe - 1][i];
+            next(i, h[0][i], h[kRe - 1][i], vr, vi);
+          }
+        }
+        __syncwarp();
+        const bool any_odd = __any_sync(0xffffffffu, odd != odd);
+#pragma unroll
+        for (int st = 0; st < kStep; ++st) {
+          // entering states: the A operand of G as they stand
+          uint32_t hp[kRe][3][4];
+#pragma unroll
+          for (int c = 0; c < kRe; ++c)
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+#pragma unroll
+              for (int r = 0; r < 2; ++r)
+                split(v[st][k][c][2 * r], v[st][k][c][2 * r + 1], hp[c][0][2 * k + r], hp[c][1][2 * k + r], hp[c][2][2 * k + r]);
+          // T's zeros would carry a NaN or an infinity to the positions before it: such a chunk takes its outputs from the finite
+          // values ahead of the first one, and is NaN from there on (as are all later states)
+          int bad[2];
+          if (any_odd) {
+            bad[0] = bad[1] = 16;
+#pragma unroll
+            for (int i = 3; i >= 0; --i) {   // (rows g, g + 8, then their upper halves)
+#pragma unroll
+              for (int e = 1; e >= 0; --e)
+                if (((f[st][0][i] >> (16 * e)) & 0x7f80u) == 0x7f80u) bad[i & 1] = 8 * (i >> 1) + 2 * t + e;
+            }
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+#pragma unroll
+              for (int m = 1; m < 4; m <<= 1) bad[r] = min(bad[r], __shfl_xor_sync(0xffffffffu, bad[r], m));
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int pos = 8 * (i >> 1) + 2 * t, from = i & 1 ? bad[1] : bad[0];
+              const uint32_t keep = pos + 1 < from ? ~0u : pos < from ? 0xffffu : 0u;
+#pragma unroll
+              for (int p = 0; p < kP; ++p) f[st][p][i] &= keep;
+            }
+          }
+          float y[2][4];
+#pragma unroll
+          for (int j = 0; j < kTerms<kP> - 1; ++j)
+#pragma unroll
+            for (int k = 0; k < 2; ++k) term<kP>(j, j > 0, y[k], f[st], matrix(kV + k));
+#pragma unroll
+          for (int j = 0; j < kTerms<3> - 1; ++j)
+#pragma unroll
+            for (int c = 0; c < kRe; ++c)
+#pragma unroll
+              for (int k = 0; k < 2; ++k) term<3>(j, true, y[k], hp[c], matrix(kV + 2 + 2 * c + k));
+#pragma unroll
+          for (int c = 0; c <= kRe; ++c)
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+              const Frag m = matrix(c < kRe ? kV + 2 + 2 * c + k : kV + k);
+              const uint32_t(&p)[4] = c < kRe ? hp[c < kRe ? c : 0][0] : f[st][0];
+              if (kApart) {   // (by themselves, so that what truncates is small)
+                float l[4];
+                mma0(l, p, m.u.x, m.u.y);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) y[k][i] += l[i];
+              } else {
+                mma(y[k], p, m.u.x, m.u.y);
+              }
+            }
+          if (kApart) {
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+#pragma unroll
+              for (int r = 0; r < 2; ++r) {
+                float x0 = 0.f, x1 = 0.f;
+#pragma unroll
+                for (int p = kP - 1; p >= 0; --p) {
+                  x0 += __uint_as_float(f[st][p][2 * k + r] << 16);
+                  x1 += __uint_as_float(f[st][p][2 * k + r] & 0xffff0000u);
+                }
+                y[k][2 * r] = fmaf(om, x0, y[k][2 * r]);
+                y[k][2 * r + 1] = fmaf(om, x1, y[k][2 * r + 1]);
+              }
+          }
+          if (a.silu) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) y[i >> 2][i & 3] = siluf_(y[i >> 2][i & 3]);
+          }
+          if (any_odd) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              if (8 * (i >> 2) + 2 * t + (i & 1) >= bad[(i >> 1) & 1]) y[i >> 2][i & 3] = __int_as_float(0x7fffffff);
+          }
+#pragma unroll
+          for (int k = 0; k < 2; ++k)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+              const float y0 = y[k][2 * r], y1 = y[k][2 * r + 1];
+              unsigned char* to = mine + buf + ((first ^ (st << 6)) ^ (r << 5)) + 16 * k;
+              if constexpr (sizeof(Out) == 4) {
+                *reinterpret_cast<uint32_t*>(to) = prmt(__float_as_uint(y0), __float_as_uint(y1), 0x7632);
+                *reinterpret_cast<uint32_t*>(to + kPlane) = prmt(__float_as_uint(y0), __float_as_uint(y1), 0x5410);
+              } else if constexpr (std::is_same<Out, __half>::value) {
+                *reinterpret_cast<__half2*>(to) = __floats2half2_rn(y0, y1);
+              } else {
+                *reinterpret_cast<uint32_t*>(to) = bf16_pair(y0, y1);
+              }
+            }
+        }
+        __syncwarp();
+      } else {
+        uint32_t e[kStep][kP][4];
+#pragma unroll
+        for (int st = 0; st < kStep; ++st)
+#pragma unroll
+          for (int p = 0; p < kP; ++p) ldmatrix(e[st][p], rows(st) + (kP + p) * kPlane);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          float v[kStep][kRe][4], u[kStep][kRe][4], l[kStep][kRe][4], w[kStep][kRe][4];
+#pragma unroll
+          for (int c = 0; c < kRe; ++c) {
+            const Frag mv = matrix(2 * c + k), mu = matrix(kV + 2 * c + k);
+#pragma unroll
+            for (int j = 0; j < kTerms<kP>; ++j)
+#pragma unroll
+              for (int st = 0; st < kStep; ++st) {
+                term<kP>(j, j > 0, v[st][c], f[st], mv);
+                term<kP>(j, j > 0, l[st][c], e[st], mv);
+                term<kP>(j, j > 0, u[st][c], f[st], mu);
+                term<kP>(j, j > 0, w[st][c], e[st], mu);
+              }
+          }
+#pragma unroll
+          for (int o = 0; o < 4 * kStep; ++o) {   // (in the order of time: steps, chunks, for two poles)
+            const int st = o >> 2, m = o & 3, i = 2 * k + (o & 1);
+            float &hr = h[0][i], &hi = h[kRe - 1][i], &sr = sn[0][i], &si = sn[kSens ? kRe - 1 : 0][i];
+            const float lr = l[st][0][m], li = l[st][kRe - 1][m], wr = w[st][0][m], wi = w[st][kRe - 1][m];
+            float xr = u[st][0][m], xi = u[st][kRe - 1][m];
+            constexpr int im = kMode == kGrad ? kRe - 1 : 0;
+            if (kC) {
+              a1[0][i] = fmaf(lr, hr, fmaf(-li, hi, a1[0][i]));
+              a1[im][i] = fmaf(lr, hi, fmaf(li, hr, a1[im][i]));
+              a2[0][i] = fmaf(lr, sr, fmaf(-li, si, fmaf(wr, hr, fmaf(-wi, hi, a2[0][i]))));
+              a2[im][i] = fmaf(lr, si, fmaf(li, sr, fmaf(wr, hi, fmaf(wi, hr, a2[im][i]))));
+              xr = fmaf(ur[kSens ? i : 0], hr, fmaf(-ui[kSens && kC ? i : 0], hi, xr));
+              xi = fmaf(ur[kSens ? i : 0], hi, fmaf(ui[kSens && kC ? i : 0], hr, xi));
+            } else {
+              a1[0][i] = fmaf(lr, hr, a1[0][i]);
+              a2[0][i] = fmaf(lr, sr, fmaf(wr, hr, a2[0][i]));
+              xr = fmaf(ur[kSens ? i : 0], hr, xr);
+            }
+            next(i, sr, si, xr, xi);
+            next(i, hr, hi, v[st][0][m], v[st][kRe - 1][m]);
+          }
+        }
+        // x and dy with the 16 chunks as the reduction: entry (i, j) is the sum of x_i dy_(15 - j)
+#pragma unroll
+        for (int st = 0; st < kStep; ++st) {
+#pragma unroll
+          for (int p = 0; p < kP; ++p) {
+            uint32_t m[4];
+            ldmatrix_t(m, rows(st) + p * kPlane);
+            f[st][p][0] = m[0]; f[st][p][1] = m[2]; f[st][p][2] = m[1]; f[st][p][3] = m[3];
+            ldmatrix_t(e[st][p], rows(st) + (kP + p) * kPlane);
+          }
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            float r[4];
+            bool onto = false;
+#pragma unroll
+            for (int o = 2 * kP - 2; o >= 0; --o)   // (products of parts p and o - p: below 2^-24 they are left out)
+#pragma unroll
+              for (int p = 0; p < kP; ++p)
+                if (o <= 2 && o - p >= 0 && o - p < kP) {
+                  if (onto) mma(r, f[st][p], e[st][o - p][2 * k], e[st][o - p][2 * k + 1]);
+                  else mma0(r, f[st][p], e[st][o - p][2 * k], e[st][o - p][2 * k + 1]);
+                  onto = true;
+                }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) R[(kMode == kGrad ? 4 * k + i : 0)] += r[i];   // (in fp32: the tensor pipe truncates its sums)
+          }
+        }
+      }
+    }
+  };
+  auto arrive = [&](int tile) {   // the tile's rows, and the copies of one further on
+    asm volatile("cp.async.wait_group %0;" ::"n"(F::kSlots - 1) : "memory");
+    if (tile < tiles) {
+      const unsigned char* slot = smem + F::stage + tid * 16 + tile % F::kSlots * F::kSlot;
+      unsigned char* buf = smem + tile % F::kBufs * F::kIns * kP * kPlane;
+      turn<In, kCh, kTile, kP, kPlane, false>(sh, slot, buf);
+      if constexpr (F::kIns == 2) turn<In, kCh, kTile, kP, kPlane, true>(sg, slot + F::kSlot / 2, buf + kP * kPlane);
+    }
+    issue(tile + F::kSlots);
+  };
+  auto leave = [&](int tile) {
+    if constexpr (kMode == kEmit)
+      if (tile >= 0) put<Out, kCh, kTile, kPlane>(so, smem + tile % F::kBufs * F::kIns * kP * kPlane);
+  };
+  // (a thread takes outputs from where it puts inputs, unless their types differ in size)
+  constexpr bool kSame = kMode != kEmit || sizeof(In) == sizeof(Out);
+  if constexpr (F::kBufs == 2) {
+    arrive(0);
+    __syncthreads();
+    for (int i = 0; i < tiles; ++i) {
+      if constexpr (kSame) {
+#pragma unroll 1
+        for (int half = 0; half < 2; ++half) {
+          if (((warp >> 2) & 1) == half) {
+            if (d < a.D) multiply(i);
+          } else {
+            leave(i - 1);
+            arrive(i + 1);
+          }
+        }
+      } else {
+        leave(i - 1);
+        __syncthreads();
+        arrive(i + 1);
+        if (d < a.D) multiply(i);
+      }
+      __syncthreads();
+    }
+    leave(tiles - 1);
+  } else {
+    for (int i = 0; i < tiles; ++i) {
+      arrive(i);
+      __syncthreads();
+      if (d < a.D) multiply(i);
+      __syncthreads();
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+
+  if constexpr (kMode == kLocal || kMode == kLocalSens) {   // what the segment behind it starts from
+    if (live) {
+#pragma unroll
+      for (int c = 0; c < kRe; ++c)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          *reinterpret_cast<float2*>(carry_at(seg + 1, c) + 8 * k) = make_float2(h[c][2 * k], h[c][2 * k + 1]);
+          if (kSens)
+            *reinterpret_cast<float2*>(carry_at(seg + 1, kRe + c) + 8 * k) =
+                make_float2(sn[kSens ? c : 0][2 * k], sn[kSens ? c : 0][2 * k + 1]);
+        }
+    }
+  }
+  if constexpr (kMode == kGrad) {   // sums over the rows, then the channel's gradients, a lane per pole
+    __syncthreads();   // (the buffers are free)
+    float* red = reinterpret_cast<float*>(smem) + warp * (16 * 17 + 4 * 16);
+    float* sums = red + 16 * 17;   // [a1, a2][re, im][16]
+#pragma unroll
+    for (int c = 0; c < kRe; ++c)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+#pragma unroll
+        for (int m = 4; m < 32; m <<= 1) {
+          a1[c][i] += __shfl_xor_sync(0xffffffffu, a1[c][i], m);
+          a2[c][i] += __shfl_xor_sync(0xffffffffu, a2[c][i], m);
+        }
+        if (g == 0) {
+          sums[c * 16 + 8 * (i >> 1) + 2 * t + (i & 1)] = a1[c][i];
+          sums[(2 + c) * 16 + 8 * (i >> 1) + 2 * t + (i & 1)] = a2[c][i];
+        }
+      }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      red[(g + 8 * ((i >> 1) & 1)) * 17 + 8 * (i >> 2) + 2 * t + (i & 1)] = R[(kMode == kGrad ? i : 0)];
+    __syncwarp();
+    float lag = 0.f;
+    if (lane < 16)
+      for (int i = 0; i < 16 - lane; ++i) lag += red[i * 17 + 15 - i - lane];
+    const int n = lane & 15;
+    const size_t at = (size_t)dc * a.N + min(n, a.N - 1);
+    const double fr = a.q[kRe * at], fi = kC ? a.q[kRe * at + 1] : 0.;
+    double er = 0., ei = 0., dr = 0., di = 0.;   // sum of q^k R_k and its derivative
+    for (int k = 15; k >= 0; --k) {
+      const double v = __shfl_sync(0xffffffffu, lag, k);
+      const double t0 = dr * fr - di * fi + er, t1 = dr * fi + di * fr + ei;
+      dr = t0;
+      di = t1;
+      const double t2 = er * fr - ei * fi + v;
+      ei = er * fi + ei * fr;
+      er = t2;
+    }
+    if (lane < 16 && n < a.N && d < a.D) {
+      const double s1r = sums[n], s1i = kC ? sums[16 + n] : 0., s2r = sums[32 + n], s2i = kC ? sums[48 + n] : 0.;
+      const float hr = (float)(er + fr * s1r - fi * s1i), sr = (float)(dr + s1r + fr * s2r - fi * s2i);
+      const float p = __ldg(a.p + at);
+      if (kC) {
+        const float hi = (float)(ei + fr * s1i + fi * s1r), si = (float)(di + s1i + fr * s2i + fi * s2r);
+        const float gr = __ldg(a.g + 2 * at), gi = __ldg(a.g + 2 * at + 1);
+        atomicAdd(a.dp + at, gr * hr - gi * hi);
+        atomicAdd(a.dg + 2 * at, p * hr);
+        atomicAdd(a.dg + 2 * at + 1, -p * hi);
+        atomicAdd(a.dq + 2 * at, p * (gr * sr - gi * si));
+        atomicAdd(a.dq + 2 * at + 1, -p * (gi * sr + gr * si));
+      } else {
+        const float gn = __ldg(a.g + at);
+        atomicAdd(a.dp + at, gn * hr);
+        atomicAdd(a.dg + at, p * hr);
+        atomicAdd(a.dq + at, p * gn * sr);
+      }
+    }
+    if (lane == 0 && d < a.D) atomicAdd(a.domega + d, lag);
+  }
+}
+
+// ---- the carry ---------------------------------------------------------------------------------------------
+// A thread per (sequence, channel, pole): what every segment starts from, in the place of what the segment before it adds.
+// blockIdx.z 0: h (and its derivative with kSens); 1: the adjoint.
+template <bool kC, bool kSens>
+__global__ void __launch_bounds__(128) chunk_carry_kernel(ChunkArgs s) {
+  const ScanArgs& a = s.a;
+  constexpr int kRe = kC ? 2 : 1;
+  const int i = blockIdx.x * 128 + threadIdx.x, b = blockIdx.y;   // channel and pole
+  if (i >= a.D * 16) return;
+  const int d = i >> 4, n = i & 15;
+  const bool adjoint = kSens && blockIdx.z == 1, in = n < a.N;
+  const size_t at = (size_t)d * a.N + n;
+  const double qr = in ? (double)a.q[kRe * at] : 0., qi = in && kC ? (double)a.q[kRe * at + 1] : 0.;
+  double ur = 1., ui = 0.;   // q^(T-1)
+  double br = qr, bi = qi;
+  for (int e = s.T - 1; e > 0; e >>= 1) {
+    if (e & 1) {
+      const double r = ur * br - ui * bi;
+      ui = ur * bi + ui * br;
+      ur = r;
+    }
+    const double r = br * br - bi * bi;
+    bi = 2. * br * bi;
+    br = r;
+  }
+  const double wr = ur * qr - ui * qi, wi = ur * qi + ui * qr;
+  const float fr = (float)wr, fi = (float)wi, gr = (float)(s.T * ur), gi = (float)(s.T * ui);
+  const size_t val = (size_t)a.D * 16, step = val * s.parts;
+  float* v = s.carry + ((size_t)b * s.S + 1) * step + (size_t)(adjoint ? 2 * kRe : 0) * val + i;
+  float hr = 0.f, hi = 0.f, sr = 0.f, si = 0.f;
+  if (!kSens && a.h_in && in) {
+    const size_t o = ((size_t)b * a.D + d) * a.N + n;
+    hr = a.h_in[kRe * o];
+    if (kC) hi = a.h_in[kRe * o + 1];
+  }
+  constexpr int kB = 4;   // segments whose loads go out together
+  for (int k0 = 1; k0 < s.S; k0 += kB, v += kB * step) {
+    float lr[kB], li[kB], mr[kB], mi[kB];
+#pragma unroll
+    for (int u = 0; u < kB; ++u) {
+      const float* p = v + (size_t)min(u, s.S - 1 - k0) * step;
+      lr[u] = __ldcg(p);
+      if (kC) li[u] = __ldcg(p + val);
+      if (kSens && !adjoint) {
+        mr[u] = __ldcg(p + kRe * val);
+        if (kC) mi[u] = __ldcg(p + (kRe + 1) * val);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kB; ++u) {
+      if (k0 + u >= s.S) break;
+      float* p = v + (size_t)u * step;
+      if (kSens && !adjoint) {
+        float x = fmaf(gr, hr, mr[u]), y = 0.f;
+        if (kC) {
+          x = fmaf(-gi, hi, x);
+          y = fmaf(gr, hi, fmaf(gi, hr, mi[u]));
+        }
+        const float r = kC ? fmaf(fr, sr, fmaf(-fi, si, x)) : fmaf(fr, sr, x);
+        if (kC) si = fmaf(fi, sr, fmaf(fr, si, y));
+        sr = r;
+        p[kRe * val] = sr;
+        if (kC) p[(kRe + 1) * val] = si;
+      }
+      const float r = kC ? fmaf(fr, hr, fmaf(-fi, hi, lr[u])) : fmaf(fr, hr, lr[u]);
+      if (kC) hi = fmaf(fi, hr, fmaf(fr, hi, li[u]));
+      hr = r;
+      p[0] = hr;
+      if (kC) p[val] = hi;
+    }
+  }
+}
+
+// ---- launches ----------------------------------------------------------------------------------------------
+template <typename In, typename Out, bool kC, int kMode>
+void run(const ChunkArgs& s, cudaStream_t st) {
+  using F = Form<In, Out, kC, kMode>;
+  const dim3 grid((s.a.D + F::kCh - 1) / F::kCh, (unsigned)(((long long)s.a.B * s.walked + 7) / 8));
+  launch(chunk_kernel<In, Out, kC, kMode>, grid, F::kThreads, F::total, (void*)st, s);
+}
+
+// Steps of a segment: a multiple of 64 (two steps of the tensor products) that minimises rounds of blocks over the SMs x
+// (steps + what a block's start and end cost beside them), the launch of the local states counted as 0.45 of the others
+// (measured: 0.4 - 0.5).  Returns that cost.
+double pick(const ScanArgs& a, ChunkArgs& s) {
+  const long long cols = (a.D + 15) / 16;
+  double best = 1e30;
+  for (int S = 1; S <= 1024; ++S) {
+    const int t = (int)((((long long)a.L + S - 1) / S + 63) / 64 * 64);
+    const int n = (int)(((long long)a.L + t - 1) / t);
+    const double rounds = ceil((double)(cols * (((long long)a.B * n + 7) / 8)) / 148.0);
+    const double local = n > 1 ? ceil((double)(cols * (((long long)a.B * (n - 1) + 7) / 8)) / 148.0) : 0.;
+    const double cost = (rounds + 0.45 * local) * (t + 96.0);
+    if (cost < best) {
+      best = cost;
+      s.T = t;
+      s.S = n;
+    }
+    if (t == 64) break;
+  }
+  return best;
+}
+
+bool envelope(int dtype, const ScanArgs& a) {
+  return g_options[OPT_CHUNK].load() != 1 && g_options[OPT_DISABLE_STREAM].load() == 0 && !a.bidir && !a.mask && !a.prev_count && a.N >= 1 &&
+         a.N <= 16 && a.B <= 65535 && a.L >= 1 && a.L < 0x7fffff00 && pieces_ok(dtype, a.D);
+}
+
+// Times in us, fitted to a grid of 38 shapes on one B200 (1 to 64 sequences, 209 to 32768 positions, 128 to 2048 channels), to
+// a fifth.  Here: a part for the launches and the blocks' start, and ns per unit of pick()'s cost by the number of parts of a
+// value and the kind of poles.
+double chunk_us(int dtype, const ScanArgs& a, bool bwd, double cost, bool segmented) {
+  static const double kFwd[2][3] = {{25., 32., 43.}, {44., 54., 76.}}, kBwd[2][3] = {{55., 82., 109.}, {105., 155., 196.}};
+  const int parts = dtype == MEGA_BF16 ? 0 : dtype == MEGA_F16 ? 1 : 2;
+  return (bwd ? (segmented ? 38. : 24.) : (segmented ? 22. : 14.)) +
+         (bwd ? kBwd : kFwd)[a.cplx ? 1 : 0][parts] * 1e-3 * cost * (segmented ? 1. : a.cplx ? 1.14 : 1.07);
+}
+// The form that a call takes otherwise: the scan backward (real bf16 16 x 4096 x 1024: 517 us against 241 here, complex 1481
+// against 459, fp32 539 against 500); forward the cluster kernel, the scan (fp32 complex of that size: 565 against 385; real fp32
+// of 4 sequences 86 against 90), or in bf16 the tensor-core kernel, which walks a sequence as one chain (complex 4 x 4096 x
+// 1024: 219 against 93; real 16 x 4096 x 1024: 100 against 121, 1 x 6606 x 1680: 145 against 56).
+double other_us(int dtype, const ScanArgs& a, bool bwd) {
+  const double L = a.L, n = (double)a.B * a.D * L;
+  if (bwd) return a.cplx ? 59. + n / 47e3 : 40. + n / 125e3;
+  if (dtype == MEGA_BF16 && g_options[OPT_DISABLE_MMA].load() == 0 && !(a.cplx && a.h_out && a.L % 32 != 0))
+    return scan_cluster_first(dtype, a, 1, 1) ? 0.9 * scan_cluster_us(dtype, a)
+                                              : a.cplx ? 95. + std::max(L * 29e-3, n / 700e3) : 6. + std::max(L * 22e-3, n / 1300e3);
+  const double one = scan_cluster_us(dtype, a);
+  return one < 1e29 ? 0.9 * one : std::min(scan_ema_fwd_us(a), a.cplx ? 25. + n / 123e3 : 15. + n / 270e3);
+}
+bool pays(int dtype, const ScanArgs& a, bool bwd, double cost, bool segmented) {
+  if (g_options[OPT_CHUNK].load() == 2) return true;
+  // (a prompt whose state leaves at a length that is no multiple of 32: the tensor-core kernel's head, then a tail)
+  if (dtype == MEGA_BF16 && !a.cplx && a.h_out && a.L % 32 != 0) return false;
+  return g_options[OPT_MMA_TILE].load() == 0 && chunk_us(dtype, a, bwd, cost, segmented) < 0.93 * other_us(dtype, a, bwd);
+}
+
+template <typename In, typename Out, bool kC>
+bool fwd(int dtype, const ScanArgs& a, cudaStream_t st) {
+  ChunkArgs s{};
+  s.a = a;
+  const double cost = pick(a, s);
+  if ((long long)a.B * s.S > 8LL * 65535 || !pays(dtype, a, false, cost, s.S > 1)) return false;
+  const bool state = a.h_in || a.h_out;
+  constexpr int kBlocks = 2 * Blocks<kC>::v + 2;
+  s.blocks = kBlocks;
+  s.parts = kC ? 2 : 1;
+  const size_t frag = (size_t)a.D * kBlocks * kBlockBytes, carry = s.S > 1 ? (size_t)a.B * s.S * s.parts * a.D * 16 : 0;
+  Scratch sc(Scratch::padded(frag) + Scratch::padded((size_t)a.D * 256) + Scratch::padded(carry * 4), st);
+  if (!sc) return false;
+  unsigned char* fr = sc.take<unsigned char>(frag);
+  float* pow = sc.take<float>((size_t)a.D * 64);
+  s.frag = fr;
+  s.pow = pow;
+  s.carry = carry ? sc.take<float>(carry) : nullptr;
+  const PrepArgs p{a.p, a.q, a.g, a.omega, a.D, a.N, 0, 1, state ? 1 : 0, sizeof(Out) == 4 ? 0 : 1, kBlocks, fr, pow};
+  launch(chunk_prepare_kernel<kC>, (unsigned)((a.D + 3) / 4), 128, 0, (void*)st, p);
+  s.in = a.x;
+  s.isb = a.xsb;
+  s.isl = a.xsl;
+  if (s.S > 1) {
+    s.walked = s.S - 1;
+    run<In, In, kC, kLocal>(s, st);
+    launch(chunk_carry_kernel<kC, false>, dim3((a.D * 16 + 127) / 128, a.B), 128, 0, (void*)st, s);
+  }
+  s.walked = s.S;
+  run<In, Out, kC, kEmit>(s, st);
+  g_last_kernel.store("chunk_ema", std::memory_order_relaxed);
+  return true;
+}
+
+template <typename T, bool kC>
+bool bwd(int dtype, const ScanArgs& a, cudaStream_t st) {
+  ChunkArgs s{};
+  s.a = a;
+  const double cost = pick(a, s);
+  if ((long long)a.B * s.S > 8LL * 65535 || !pays(dtype, a, true, cost, s.S > 1)) return false;
+  constexpr int kRe = kC ? 2 : 1, kBlocks = 3 * Blocks<kC>::v + 2;
+  s.blocks = kBlocks;
+  s.parts = 3 * kRe;
+  const size_t frag = (size_t)a.D * kBlocks * kBlockBytes, carry = s.S > 1 ? (size_t)a.B * s.S * s.parts * a.D * 16 : 0;
+  Scratch sc(Scratch::padded(frag) + Scratch::padded((size_t)a.D * 256) + Scratch::padded(carry * 4), st);
+  if (!sc) return false;
+  unsigned char* fr = sc.take<unsigned char>(frag);
+  float* pow = sc.take<float>((size_t)a.D * 64);
+  s.frag = fr;
+  s.pow = pow;
+  s.carry = carry ? sc.take<float>(carry) : nullptr;
+  const PrepArgs p{a.p, a.q, a.g, a.omega, a.D, a.N, 1, 1, 0, sizeof(T) == 4 ? 0 : 1, kBlocks, fr, pow};
+  launch(chunk_prepare_kernel<kC>, (unsigned)((a.D + 3) / 4), 128, 0, (void*)st, p);
+  ChunkArgs x = s, g = s;   // forward over x; backward over dy
+  x.in = a.x;
+  x.isb = a.xsb;
+  x.isl = a.xsl;
+  g.in = a.dy;
+  g.isb = a.gsb;
+  g.isl = a.gsl;
+  g.rev = 1;
+  g.part = 2 * kRe;
+  if (s.S > 1) {
+    x.walked = g.walked = s.S - 1;
+    run<T, T, kC, kLocalSens>(x, st);
+    run<T, T, kC, kLocal>(g, st);
+    launch(chunk_carry_kernel<kC, true>, dim3((a.D * 16 + 127) / 128, a.B, 2), 128, 0, (void*)st, s);
+  }
+  x.walked = g.walked = s.S;
+  run<T, T, kC, kGrad>(x, st);
+  run<T, T, kC, kEmit>(g, st);
+  g_last_kernel.store("chunk_ema", std::memory_order_relaxed);
+  return true;
+}
+
+}  // namespace
+
+// (in place: a block reads a tile before it writes it, and no other block reads it once the local states are there)
+bool chunk_ema_fwd_try(int dtype, int out_dtype, const ScanArgs& a, long long xsd, long long ysd, cudaStream_t s) {
+  if (!envelope(dtype, a) || !pieces_ok(out_dtype, a.D) || !rows_ok(dtype, a.x, a.xsb, a.xsl, xsd) ||
+      !rows_ok(out_dtype, a.y, a.ysb, a.ysl, ysd))
+    return false;
+#define MEGA_FWD(IN, OUT) return a.cplx ? fwd<IN, OUT, true>(dtype, a, s) : fwd<IN, OUT, false>(dtype, a, s)
+  if (dtype == MEGA_F32 && out_dtype == MEGA_BF16) MEGA_FWD(float, __nv_bfloat16);
+  if (dtype == MEGA_F32 && out_dtype == MEGA_F16) MEGA_FWD(float, __half);
+  if (dtype != out_dtype) return false;
+  if (dtype == MEGA_F32) MEGA_FWD(float, float);
+  if (dtype == MEGA_BF16) MEGA_FWD(__nv_bfloat16, __nv_bfloat16);
+  if (dtype == MEGA_F16) MEGA_FWD(__half, __half);
+#undef MEGA_FWD
+  return false;
+}
+
+bool chunk_ema_bwd_try(int dtype, const ScanArgs& a, long long xsd, long long ysd, long long gsd, cudaStream_t s) {
+  if (!envelope(dtype, a) || a.h_in || a.h_out || a.silu || !rows_ok(dtype, a.x, a.xsb, a.xsl, xsd) ||
+      !rows_ok(dtype, a.dy, a.gsb, a.gsl, gsd) || !rows_ok(dtype, a.y, a.ysb, a.ysl, ysd))
+    return false;
+  switch (dtype) {
+    case MEGA_F32: return a.cplx ? bwd<float, true>(dtype, a, s) : bwd<float, false>(dtype, a, s);
+    case MEGA_BF16: return a.cplx ? bwd<__nv_bfloat16, true>(dtype, a, s) : bwd<__nv_bfloat16, false>(dtype, a, s);
+    case MEGA_F16: return a.cplx ? bwd<__half, true>(dtype, a, s) : bwd<__half, false>(dtype, a, s);
+    default: return false;
+  }
+}
+
+}  // namespace mega

@@ -25,8 +25,9 @@
 #include <type_traits>
 
 #include "common.cuh"
-#include "tma.cuh"
 #include "rowres.cuh"
+#include "split_mma.cuh"
+#include "tma.cuh"
 
 namespace mega {
 
@@ -35,7 +36,6 @@ namespace {
 constexpr int kRowNP = 16;    // poles per direction
 constexpr int kSeg = 32;      // positions of a segment
 constexpr int kMaxThreads = 512;
-constexpr int kBlockBytes = 32 * 24;   // a B fragment (16 x 8) in three bf16 parts: uint4 and uint2 per lane
 
 // q^32 of a pole, then q^(32 g R) for g = 0 .. 8, R the segments a lane holds
 constexpr int kQ1 = 0, kQRun = 1, kQRows = 10;
@@ -50,38 +50,6 @@ struct RowSmem {   // byte offsets: the channel's tables first, at addresses tha
   __host__ __device__ static constexpr int total(int nseg) { return mask(nseg) + 2 * nseg * 4; }
 };
 
-__device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
-  uint32_t r;
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
-  return r;
-}
-// two floats as three packed bf16 pairs whose sums they are
-__device__ __forceinline__ void split3(float lo, float hi, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
-  const f32x2 minus = pack2(-1.f, -1.f);
-  f32x2 v = pack2(lo, hi);
-  p0 = bf16_pair(lo, hi);
-  v = fma2(pack2(__uint_as_float(p0 << 16), __uint_as_float(p0 & 0xffff0000u)), minus, v);
-  unpack2(v, lo, hi);
-  p1 = bf16_pair(lo, hi);
-  v = fma2(pack2(__uint_as_float(p1 << 16), __uint_as_float(p1 & 0xffff0000u)), minus, v);
-  unpack2(v, lo, hi);
-  p2 = bf16_pair(lo, hi);
-}
-
-__device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-struct Frag {   // B fragment: parts 0 and 1 in u, part 2 in v
-  uint4 u;
-  uint2 v;
-};
-__device__ __forceinline__ Frag load_frag(const unsigned char* block) {
-  const int lane = threadIdx.x & 31;
-  return {*reinterpret_cast<const uint4*>(block + lane * 16), *reinterpret_cast<const uint2*>(block + 512 + lane * 8)};
-}
 // d = products of K reduction tiles, all but those of the leading parts, smallest first, then those.  The tensor pipe truncates
 // its sums: kApart gives the leading products an accumulator of their own, which an fp32 addition joins.  Block of tile k at
 // block + k * stride.
@@ -216,12 +184,7 @@ __device__ __forceinline__ void prepare_channel(const RowArgs& a, int d, int per
         v[i] = (float)(cp * pw[(pole < 16 ? pos + 1 : (a.shift ? 31 : 32) - pos) * 32 + pole]);
       }
     }
-    uint32_t lo[3], hi[3];
-    split3(v[0], v[1], lo[0], lo[1], lo[2]);
-    split3(v[2], v[3], hi[0], hi[1], hi[2]);
-    unsigned char* dst = smem + o::frag + blk * kBlockBytes;
-    *reinterpret_cast<uint4*>(dst + lane * 16) = make_uint4(lo[0], hi[0], lo[1], hi[1]);
-    *reinterpret_cast<uint2*>(dst + 512 + lane * 8) = make_uint2(lo[2], hi[2]);
+    store_frag(smem + o::frag + blk * kBlockBytes, v);
   }
 }
 

@@ -598,11 +598,11 @@ __global__ void __launch_bounds__(kWarps * 32, kC ? 2 : 3) scan_bwd_kernel(SegAr
 
 // Segments of a call.  A block takes four segments of 32 channels; `resident` blocks of the last kernel fit an SM.
 // The choice minimises (rounds of blocks over the 148 SMs) x (steps of a segment + what its states cost beside
-// them: written, carried and read, 64 steps' worth backward and 40 forward), so that neither a nearly empty last round nor short segments dominate.  Segments
+// them: written, carried and read, 64 steps' worth backward and 40 forward), so that neither a nearly empty last round nor short segments dominate; it is returned.  Segments
 // are at least 32 steps; a bidirectional one keeps its share of the outputs in shared memory, so at most 64: beyond 4096
 // of those the counts start from what the length asks for.
 // One segment per sequence when the channels alone fill the device: no first pass then.
-static void pick_segments(const ScanArgs& a, int resident, bool bwd, SegArgs& s) {
+static double pick_segments(const ScanArgs& a, int resident, bool bwd, SegArgs& s) {
   const long long strips = (long long)((a.D + 31) / 32) * a.B;
   const double slots = 148.0 * resident;
   double best = 1e30;
@@ -631,6 +631,7 @@ static void pick_segments(const ScanArgs& a, int resident, bool bwd, SegArgs& s)
     }
     if (t == 32) break;
   }
+  return best;
 }
 
 template <typename T, bool kC, bool kMask, bool kNorm>
@@ -716,6 +717,12 @@ bool scan_ema_fwd_ok(int dtype, const ScanArgs& a, long long xsd, long long ysd)
   return g_options[OPT_DISABLE_STREAM].load() == 0 && rows_ok(dtype, a.x, a.xsb, a.xsl, xsd) && (!a.prev_count || pieces_ok(dtype, a.D)) &&
          ysd == 1 && a.N <= 16 &&
          (long long)a.B * (a.bidir ? 2 : 1) <= 65535 && (a.x != a.y || (a.xsb == a.ysb && a.xsl == a.ysl));
+}
+
+// (16 x 4096 x 1024: 254 us real, 565 complex; 64 x 256 x 1024: 52 and 110)
+double scan_ema_fwd_us(const ScanArgs& a) {
+  SegArgs s{};
+  return 10. + pick_segments(a, a.cplx || a.prev_count ? 3 : 4, false, s) * (a.cplx ? 0.33 : 0.23);
 }
 
 bool scan_ema_fwd_try(int dtype, const ScanArgs& a, long long xsd, long long ysd, cudaStream_t s) {

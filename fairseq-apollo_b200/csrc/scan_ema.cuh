@@ -30,6 +30,7 @@ struct ScanArgs {
 // The forward may run in place (x == y, same strides): a warp reads its rows ahead of where it writes them.
 bool scan_ema_fwd_ok(int dtype, const ScanArgs& a, long long xsd, long long ysd);   // the envelope alone
 bool scan_ema_fwd_try(int dtype, const ScanArgs& a, long long xsd, long long ysd, cudaStream_t s);
+double scan_ema_fwd_us(const ScanArgs& a);   // predicted time of the scan's launches, causal, no norm in front
 bool scan_ema_bwd_try(int dtype, const ScanArgs& a, long long xsd, long long ysd, long long gsd, cudaStream_t s);
 
 }  // namespace mega

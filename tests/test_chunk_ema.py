@@ -1,0 +1,161 @@
+"""The causal EMA as matrix products of chunks (csrc/chunk_ema.cu), forward and backward, against the recurrence in float64: at
+the edges of its chunks (16), steps (32), tiles (64, 128), segments and blocks of channels (8, 16)."""
+import pytest
+import torch
+
+from _util import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+# y and dx: one rounding of the result (2^-9, 2^-12); fp32: products of three bf16 parts leave 2^-24 of each term of sums of some
+# forty (taps, poles, omega x), 2e-7 in the 2-norm at most.  States: as fp32.  Sums over B L positions: 2^-24 times the square
+# root of the additions of a channel (under 64), in sums that cancel to a tenth
+LIMIT = {torch.float32: 5e-7, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}
+SUMS = 5e-6
+
+
+@pytest.fixture
+def forced():
+    from fairseq_apollo_b200 import _lib
+    _lib.set_option(6, 2)
+    yield _lib
+    _lib.set_option(6, 0)
+
+
+def problem(gen, bsz, length, dim, ndim, dtype, cplx):
+    p = torch.rand(dim, ndim, generator=gen) * 0.9 + 0.05
+    mag = 1 - p * torch.sigmoid(torch.randn(dim, ndim, generator=gen))
+    g = torch.randn(dim, ndim, generator=gen) * 0.25
+    if cplx:
+        mag = torch.polar(mag, torch.rand(dim, ndim, generator=gen) * 6.28)
+        g = torch.complex(g, torch.randn(dim, ndim, generator=gen) * 0.25)
+    omega = torch.randn(dim, generator=gen)
+    x, dy = ((torch.randn(bsz, length, dim, generator=gen) + 0.1).to(dtype) for _ in range(2))
+    return x, dy, p, mag, g, omega
+
+
+def recurrence(x, p, q, g, omega, h=None):
+    """(B, L, D) in double -> outputs, last state"""
+    h = torch.zeros(x.size(0), *p.shape, dtype=q.dtype) if h is None else h
+    out = []
+    for xt in x.unbind(1):
+        h = q * h + p * xt.unsqueeze(-1)
+        y = (g * h).sum(-1)
+        out.append((y.real if y.is_complex() else y) + omega * xt)
+    return torch.stack(out, 1), h
+
+
+def double(t):
+    return t.to(torch.complex128) if t.is_complex() else t.double()
+
+
+SHAPES = [(1, 2, 8, 16), (2, 15, 16, 16), (1, 17, 24, 5), (3, 33, 8, 16), (9, 64, 16, 1), (2, 65, 40, 16), (1, 127, 16, 16),
+          (2, 129, 8, 16), (1, 700, 136, 16), (5, 321, 24, 7)]
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("bsz,length,dim,ndim", SHAPES)
+def test_against_float64(forced, bsz, length, dim, ndim, dtype, cplx):
+    from fairseq_apollo_b200 import ops
+    gen = torch.Generator().manual_seed(length)
+    x, dy, p, q, g, omega = problem(gen, bsz, length, dim, ndim, dtype, cplx)
+    leaves = [double(t).requires_grad_(True) for t in (x, p, q, g, omega)]
+    want, _ = recurrence(*leaves)
+    want.backward(dy.double())
+    fwd, bwd = (ops.cema_forward, ops.cema_backward) if cplx else (ops.ema_forward, ops.ema_backward)
+    c = [t.cuda() for t in (p, q, g, omega)]
+    xc, dyc = x.cuda().transpose(1, 2), dy.cuda().transpose(1, 2)
+    y = fwd(xc, *c)
+    assert forced.last_kernel() == "chunk_ema"
+    assert rel_l2(y.transpose(1, 2), want) < LIMIT[dtype]
+    got = bwd(dyc, xc, *c)
+    assert forced.last_kernel() == "chunk_ema"
+    assert rel_l2(got[0].transpose(1, 2), leaves[0].grad) < LIMIT[dtype]
+    for name, a, b in zip(("p", "q", "g", "omega"), got[1:5], leaves[1:]):
+        b = b.grad
+        if a.is_complex():
+            a, b = torch.view_as_real(a.cpu()), torch.view_as_real(b)
+        assert rel_l2(a, b) < SUMS or (a.cpu().double() - b).norm() < 1e-5, name   # (one position: dq is zero)
+    # with a state, activated
+    h = torch.randn(bsz, dim, ndim, dtype=q.dtype, generator=gen)
+    wanted, last = recurrence(*[double(t) for t in (x, p, q, g, omega)], double(h))
+    y, out = fwd(xc, *c, None, h.cuda(), True, silu=True)
+    assert forced.last_kernel() == "chunk_ema"
+    assert rel_l2(y.transpose(1, 2), torch.nn.functional.silu(wanted)) < LIMIT[dtype]
+    if cplx:
+        out, last = torch.view_as_real(out.cpu()), torch.view_as_real(last)
+    assert rel_l2(out, last) < 5e-7
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_many_segments_and_any_strides(forced, dtype):
+    """Sequences cut into segments, the last one ragged; time-major memory and slices of wider rows."""
+    from fairseq_apollo_b200 import ops
+    gen = torch.Generator().manual_seed(1)
+    x, dy, p, q, g, omega = problem(gen, 2, 5000, 16, 16, dtype, False)
+    c = [t.cuda() for t in (p, q, g, omega)]
+    xc, dyc = x.cuda().transpose(1, 2), dy.cuda().transpose(1, 2)
+    y, grads = ops.ema_forward(xc, *c), ops.ema_backward(dyc, xc, *c)
+    assert forced.last_kernel() == "chunk_ema"
+    xt = x.cuda().transpose(0, 1).contiguous().permute(1, 2, 0)
+    wide = torch.full((2, 5000, 48), float("nan"), dtype=dtype, device="cuda")
+    wide[..., 16:32] = dy.cuda()
+    y2, grads2 = ops.ema_forward(xt, *c), ops.ema_backward(wide[..., 16:32].transpose(1, 2), xt, *c)
+    assert torch.equal(y, y2) and torch.equal(grads[0], grads2[0])
+    forced.set_option(6, 1)
+    y3, grads3 = ops.ema_forward(xc.float(), *c), ops.ema_backward(dyc.float(), xc.float(), *c)
+    assert rel_l2(y, y3) < LIMIT[dtype] and rel_l2(grads[0], grads3[0]) < LIMIT[dtype]
+    for a, b in zip(grads2[1:5], grads3[1:5]):
+        assert rel_l2(a, b) < SUMS
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("at", [0, 15, 16, 40, 99])
+def test_nothing_before_a_non_finite_input(forced, value, dtype, at, cplx):
+    """Outputs ahead of an infinity or a NaN are as without it, and not finite from there on; the input's gradient the other
+    way round in time."""
+    from fairseq_apollo_b200 import ops
+    gen = torch.Generator().manual_seed(at)
+    x, dy, p, q, g, omega = problem(gen, 2, 100, 16, 16, dtype, cplx)
+    fwd, bwd = (ops.cema_forward, ops.cema_backward) if cplx else (ops.ema_forward, ops.ema_backward)
+    c = [t.cuda() for t in (p, q, g, omega)]
+    xc, dyc = x.cuda().transpose(1, 2), dy.cuda().transpose(1, 2)
+    clean, grad = fwd(xc, *c), bwd(dyc, xc, *c)[0]
+    bad, bad_dy = xc.clone(), dyc.clone()
+    bad[1, 3, at] = value
+    bad_dy[1, 3, at] = value
+    y, dx = fwd(bad, *c), bwd(bad_dy, xc, *c)[0]
+    assert forced.last_kernel() == "chunk_ema"
+    assert torch.equal(y[1, 3, :at], clean[1, 3, :at]) and not torch.isfinite(y[1, 3, at:]).any()
+    assert torch.equal(dx[1, 3, at + 1:], grad[1, 3, at + 1:]) and not torch.isfinite(dx[1, 3, :at + 1]).any()
+    keep = torch.ones(16, dtype=torch.bool)
+    keep[3] = False
+    assert torch.equal(y[:, keep], clean[:, keep]) and torch.equal(dx[:, keep], grad[:, keep])
+    assert torch.equal(y[0], clean[0])
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+def test_chosen_calls_agree_with_the_scan(cplx):
+    """A call that the estimate gives to the chunks, against the forms that walk position by position."""
+    from fairseq_apollo_b200 import _lib, ops
+    gen = torch.Generator().manual_seed(4)
+    x, dy, p, q, g, omega = problem(gen, 4, 2048, 512, 16, torch.bfloat16, cplx)
+    bwd = ops.cema_backward if cplx else ops.ema_backward
+    c = [t.cuda() for t in (p, q, g, omega)]
+    xc, dyc = x.cuda().transpose(1, 2), dy.cuda().transpose(1, 2)
+    got = bwd(dyc, xc, *c)
+    assert _lib.last_kernel() == "chunk_ema"
+    _lib.set_option(6, 1)
+    try:
+        want = bwd(dyc, xc, *c)
+        assert _lib.last_kernel() != "chunk_ema"
+    finally:
+        _lib.set_option(6, 0)
+    assert rel_l2(got[0], want[0]) < 2.0 ** -8
+    for a, b in zip(got[1:5], want[1:5]):
+        if a.is_complex():
+            a, b = torch.view_as_real(a), torch.view_as_real(b)
+        assert rel_l2(a, b) < 1e-5   # (the scan's own error: 3e-6)
