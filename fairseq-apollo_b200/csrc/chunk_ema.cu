@@ -116,6 +116,15 @@ __device__ __forceinline__ void split(float lo, float hi, uint32_t& p0, uint32_t
   p1 = bf16_pair(lo, hi);
   p2 = bf16_pair(lo - lower(p1), hi - __uint_as_float(p1 & 0xffff0000u));
 }
+// silu without a division's slow path (inside the walk that cost half of its time: 607 us where this takes 340, 6 x 4999 x 2048
+// complex): the reciprocal to one unit, for fp32 outputs to a half by a Newton step (the clamp keeps that from an infinity)
+template <typename T>
+__device__ __forceinline__ float silu_of(float v) {
+  const float d = sizeof(T) == 4 ? fminf(1.f + __expf(-v), 1e38f) : 1.f + __expf(-v);
+  float r = rcp_approx(d);
+  if (sizeof(T) == 4) r = fmaf(r, fmaf(-d, r, 1.f), r);
+  return v * r;
+}
 // Product j, smallest first, of those of a (kP parts) with a block: the leading one is the last.  (Callers go through the
 // products of several independent sums in turn, so that none waits for the one before it.)
 template <int kP>
@@ -445,7 +454,7 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode>::kThreads, Form<In, O
   const int final = kMode == kEmit && a.h_out != nullptr && live && seg == s.S - 1 ? (len - 1) / 32 : -1;   // step whose end leaves
 
   // kStep steps of 32 positions at a time: their products do not wait for each other, only their states do
-  constexpr int kStep = kMode == kGrad && kC ? 1 : 2;
+  constexpr int kStep = kC && (kMode == kGrad || kP == 3) ? 1 : 2;   // (what registers hold: a spill goes to L2 beside this much shared memory)
   auto multiply = [&](int tile) {
     const int buf = tile % F::kBufs * F::kIns * kP * kPlane;
     const int n = min(kTile / 32, steps - kTile / 32 * tile), last = final - kTile / 32 * tile;
@@ -613,7 +622,7 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode>::kThreads, Form<In, O
           }
           if (a.silu) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) y[i >> 2][i & 3] = siluf_(y[i >> 2][i & 3]);
+            for (int i = 0; i < 8; ++i) y[i >> 2][i & 3] = silu_of<Out>(y[i >> 2][i & 3]);
           }
           if (any_odd) {
 #pragma unroll
@@ -947,7 +956,7 @@ bool envelope(int dtype, const ScanArgs& a) {
 // a fifth.  Here: a part for the launches and the blocks' start, and ns per unit of pick()'s cost by the number of parts of a
 // value and the kind of poles.
 double chunk_us(int dtype, const ScanArgs& a, bool bwd, double cost, bool segmented) {
-  static const double kFwd[2][3] = {{25., 32., 43.}, {44., 54., 76.}}, kBwd[2][3] = {{55., 82., 109.}, {105., 155., 196.}};
+  static const double kFwd[2][3] = {{25., 32., 43.}, {44., 54., 64.}}, kBwd[2][3] = {{55., 82., 109.}, {105., 155., 185.}};
   const int parts = dtype == MEGA_BF16 ? 0 : dtype == MEGA_F16 ? 1 : 2;
   return (bwd ? (segmented ? 38. : 24.) : (segmented ? 22. : 14.)) +
          (bwd ? kBwd : kFwd)[a.cplx ? 1 : 0][parts] * 1e-3 * cost * (segmented ? 1. : a.cplx ? 1.14 : 1.07);
@@ -973,11 +982,11 @@ bool pays(int dtype, const ScanArgs& a, bool bwd, double cost, bool segmented) {
 }
 
 template <typename In, typename Out, bool kC>
-bool fwd(int dtype, const ScanArgs& a, cudaStream_t st) {
+bool fwd(int dtype, const ScanArgs& a, bool asked, cudaStream_t st) {
   ChunkArgs s{};
   s.a = a;
   const double cost = pick(a, s);
-  if ((long long)a.B * s.S > 8LL * 65535 || !pays(dtype, a, false, cost, s.S > 1)) return false;
+  if ((long long)a.B * s.S > 8LL * 65535 || !(asked || pays(dtype, a, false, cost, s.S > 1))) return false;
   const bool state = a.h_in || a.h_out;
   constexpr int kBlocks = 2 * Blocks<kC>::v + 2;
   s.blocks = kBlocks;
@@ -1050,11 +1059,11 @@ bool bwd(int dtype, const ScanArgs& a, cudaStream_t st) {
 }  // namespace
 
 // (in place: a block reads a tile before it writes it, and no other block reads it once the local states are there)
-bool chunk_ema_fwd_try(int dtype, int out_dtype, const ScanArgs& a, long long xsd, long long ysd, cudaStream_t s) {
+bool chunk_ema_fwd_try(int dtype, int out_dtype, const ScanArgs& a, long long xsd, long long ysd, cudaStream_t s, bool asked) {
   if (!envelope(dtype, a) || !pieces_ok(out_dtype, a.D) || !rows_ok(dtype, a.x, a.xsb, a.xsl, xsd) ||
       !rows_ok(out_dtype, a.y, a.ysb, a.ysl, ysd))
     return false;
-#define MEGA_FWD(IN, OUT) return a.cplx ? fwd<IN, OUT, true>(dtype, a, s) : fwd<IN, OUT, false>(dtype, a, s)
+#define MEGA_FWD(IN, OUT) return a.cplx ? fwd<IN, OUT, true>(dtype, a, asked, s) : fwd<IN, OUT, false>(dtype, a, asked, s)
   if (dtype == MEGA_F32 && out_dtype == MEGA_BF16) MEGA_FWD(float, __nv_bfloat16);
   if (dtype == MEGA_F32 && out_dtype == MEGA_F16) MEGA_FWD(float, __half);
   if (dtype != out_dtype) return false;
@@ -1063,6 +1072,13 @@ bool chunk_ema_fwd_try(int dtype, int out_dtype, const ScanArgs& a, long long xs
   if (dtype == MEGA_F16) MEGA_FWD(__half, __half);
 #undef MEGA_FWD
   return false;
+}
+
+double chunk_ema_fwd_us(int dtype, const ScanArgs& a) {
+  if (!envelope(dtype, a)) return 1e30;
+  ChunkArgs s{};
+  const double cost = pick(a, s);
+  return chunk_us(dtype, a, false, cost, s.S > 1);
 }
 
 bool chunk_ema_bwd_try(int dtype, const ScanArgs& a, long long xsd, long long ysd, long long gsd, cudaStream_t s) {

@@ -10,7 +10,9 @@ namespace mega {
 // contiguous in whole 16-byte pieces on every tensor), when another form is predicted to be faster, or without scratch memory.
 // Forward: x of type dtype, y of type out_dtype (the same, or x in fp32 and y of 16 bits); x may be y where the types are the
 // same.  Backward: a.y is dx, which is neither x nor dy.
-bool chunk_ema_fwd_try(int dtype, int out_dtype, const ScanArgs& a, long long xsd, long long ysd, cudaStream_t s);
+// asked: whatever the prediction says.
+bool chunk_ema_fwd_try(int dtype, int out_dtype, const ScanArgs& a, long long xsd, long long ysd, cudaStream_t s, bool asked = false);
+double chunk_ema_fwd_us(int dtype, const ScanArgs& a);   // predicted time, 1e30 outside the envelope
 bool chunk_ema_bwd_try(int dtype, const ScanArgs& a, long long xsd, long long ysd, long long gsd, cudaStream_t s);
 
 }  // namespace mega

@@ -456,8 +456,9 @@ extern "C" int mega_tsn_ema_fwd(const void* x, void* y, void* xn_out, int dtype,
     sa.p = p; sa.q = q; sa.g = gamma_hat; sa.omega = omega; sa.h_in = h_in; sa.h_out = h_out; sa.mask = pad_mask;
     sa.silu = a.silu;
     // (a real layer's ragged state in bf16 keeps the two launches below up to 8192 positions: 6 x 4999 x 2048 with a second
-    // output takes 269 us on them; fewer than four sequences go to the streamed chain instead, 198 ns a position)
-    if (!(dtype == MEGA_BF16 && h_out && L % 32 != 0 && !pad_mask && L < 8192) &&
+    // output takes 269 us on them; with one, fewer than four sequences would go to the streamed chain, 198 ns a position: 1 x
+    // 5731 x 1152 1142 us where the forms parallel over time take 95)
+    if (!(dtype == MEGA_BF16 && h_out && L % 32 != 0 && !pad_mask && L < 8192 && (B >= 4 || !xn_out)) &&
         norm_ema_split_try(dtype, x, y, xn_out, xsb, xsl, xsd, ysb, ysl, ysd, sa, (cudaStream_t)stream))
       return check_launch("tsn_ema_fwd(split)");
     // A state is exported and L is not a multiple of the tensor-core kernel's step of 32 positions (it

@@ -5,11 +5,14 @@
 // normalise their inputs as they read them, and, for bf16, TimestepNorm by itself (scan_norm.cu) followed by the
 // tensor-core kernel alone, which runs in half the time of the fused one; the normalised activations then go to their
 // own output, or through y in place.
+#include "chunk_ema.cuh"
 #include "common.cuh"
 #include "norm_ema_split.cuh"
 #include "scan_cluster.cuh"
 #include "scan_ema.cuh"
 #include "scan_norm.cuh"
+#include "scratch.cuh"
+#include "walk.cuh"
 
 namespace mega {
 
@@ -33,15 +36,18 @@ bool mma_takes(int dtype, const StreamArgs& a, bool want_xn) {
 double fused_us(int dtype, const StreamArgs& a, bool want_xn) {
   const double L = a.L, n = (double)a.B * a.D * a.L;
   if (mma_takes(dtype, a, want_xn)) {
-    const double fixed = a.cplx ? 68.0 : want_xn ? 15.0 : a.mask ? 13.0 : 11.0;
-    const double chain = a.cplx ? (want_xn ? 46.0 : 36.0) : want_xn ? 44.0 : a.mask ? 42.0 : 30.0;
+    const double fixed = a.cplx ? (want_xn ? 100.0 : 95.0) : want_xn ? 15.0 : a.mask ? 13.0 : 11.0;
+    const double chain = a.cplx ? (want_xn ? 41.0 : 38.0) : want_xn ? 44.0 : a.mask ? 42.0 : 30.0;
     const double rate = a.cplx ? (want_xn ? 300e3 : 480e3) : want_xn ? 500e3 : a.mask ? 520e3 : 600e3;
     const double far = L * 1e-3 * (a.cplx ? (want_xn ? 75.0 : 62.0) : want_xn || a.mask ? 50.0 : 34.0);
     const double near = fixed + longer(chain, rate, L, n);
     return near > far ? near : far;
   }
-  // (complex: 254 ns a position with a state, which prompts of 700 to 4999 positions show alike)
-  return a.cplx ? 8.0 + longer(a.h_in || a.h_out ? 254.0 : 171.0, 168e3, L, n) : 6.0 + longer(122.0, want_xn ? 160e3 : 260e3, L, n);
+  // (the streamed chain: 171 to 260 ns a position complex, 150 to 200 real, more where the channels do not fit the SMs at once;
+  // with a second output a third of the rate: 57 x 995 x 632 fp32 163 us and 489)
+  const bool slow = want_xn || a.h_in || a.h_out;
+  return a.cplx ? (slow ? 30.0 + longer(234.0, 70e3, L, n) : 8.0 + longer(171.0, 130e3, L, n))
+                : slow ? 15.0 + longer(185.0, 85e3, L, n) : 6.0 + longer(145.0, 230e3, L, n);
 }
 
 // TimestepNorm, then the tensor-core kernel alone: where the fused call would run on it too (both round the normalised
@@ -56,6 +62,44 @@ double mma_us(int dtype, const StreamArgs& a, bool want_xn) {
 double scan_us(int dtype, const ScanArgs& ea, bool want_xn) {
   const double n = (double)ea.B * ea.D * ea.L, one = scan_cluster_us(dtype, ea);
   return one < 1e29 ? one : 45.0 + n / (ea.cplx ? (want_xn ? 78e3 : 88e3) : (want_xn ? 145e3 : 165e3));
+}
+
+// TimestepNorm in fp32, then the products of chunks (chunk_ema.cu): the normalised activations lie in scratch memory, for fp32
+// calls in xn or, in place, in y.  (moments and normalised activations of 6 x 4999 x 2048 bf16: 125 us)
+constexpr double kWideMost = 62e6;   // elements of scratch memory: what the pool keeps between calls (scratch.cuh)
+double chunk_us(int dtype, const ScanArgs& ea) {
+  ScanArgs a = ea;
+  a.prev_count = nullptr;
+  const double n = (double)a.B * a.D * a.L;
+  if (dtype != MEGA_F32 && n > kWideMost) return 1e30;
+  return 18.0 + n / (dtype == MEGA_F32 ? 480e3 : 540e3) + chunk_ema_fwd_us(MEGA_F32, a);
+}
+bool norm_chunk_try(int dtype, const ScanArgs& ea, long long xsd, long long ysd, cudaStream_t s) {
+  if (!rows_ok(dtype, ea.y, ea.ysb, ea.ysl, ysd) || (ea.xn && !rows_ok(dtype, ea.xn, ea.ysb, ea.ysl, ysd))) return false;
+  ScanNormArgs na{};
+  na.x = ea.x; na.B = ea.B; na.D = ea.D; na.L = ea.L;
+  na.xsb = ea.xsb; na.xsl = ea.xsl; na.ysb = ea.ysb; na.ysl = ea.ysl;
+  na.prev_count = ea.prev_count; na.prev_mean = ea.prev_mean; na.prev_var = ea.prev_var; na.gamma = ea.gamma; na.beta = ea.beta;
+  na.eps = ea.eps; na.count_out = ea.count_out; na.mean_out = ea.mean_out; na.var_out = ea.var_out;
+  ScanArgs a = ea;
+  a.prev_count = nullptr;
+  a.xn = nullptr;
+  if (dtype == MEGA_F32) {
+    na.y = ea.xn ? ea.xn : ea.y;
+    a.x = na.y;
+    a.xsb = ea.ysb;
+    a.xsl = ea.ysl;
+    return scan_norm_fwd_try(dtype, na, xsd, ysd, s) && chunk_ema_fwd_try(dtype, dtype, a, 1, ysd, s, true);
+  }
+  const size_t n = (size_t)ea.B * ea.L * ea.D;
+  Scratch sc(Scratch::padded(n * 4), s);
+  if (!sc) return false;
+  na.wide = sc.take<float>(n);
+  na.y = ea.xn;
+  a.x = na.wide;
+  a.xsb = (long long)ea.L * ea.D;
+  a.xsl = ea.D;
+  return scan_norm_fwd_try(dtype, na, xsd, ysd, s) && chunk_ema_fwd_try(MEGA_F32, dtype, a, 1, ysd, s, true);
 }
 
 }  // namespace
@@ -80,6 +124,11 @@ bool norm_ema_split_try(int dtype, const void* x, void* y, void* xn, long long x
   const bool chunk = dtype == MEGA_BF16 && a.h_out && !a.mask && !a.cplx;
   const double fused = fused_us(dtype, a, xn != nullptr), scan = scan_us(dtype, ea, xn != nullptr) + (chunk ? 25.0 : 0.0),
                mma = mma_us(dtype, a, xn != nullptr) + 25.0;
+  if (forced == 0 && !a.mask) {   // (what stands in mean_out and the like once the norm has run is what the forms below write too)
+    const double chunk = chunk_us(dtype, ea);
+    if ((chunk < 0.88 * (scan < mma ? scan : mma) && chunk < 0.88 * fused) || (chunk < 1e29 && g_options[OPT_CHUNK].load() == 2))
+      if (norm_chunk_try(dtype, ea, xsd, ysd, s)) return true;
+  }
   if (forced == 0 && (scan < mma ? scan : mma) > 0.9 * fused) return false;
   if (mma < scan && forced != 3) {
     void* mid = xn ? xn : y;

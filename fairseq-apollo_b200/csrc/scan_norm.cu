@@ -137,14 +137,17 @@ struct PairRunning {
   }
 };
 
-template <typename T, bool kMask>
+// kWide: the output in fp32 for what follows on it, beside that of type T or in its place.
+template <typename T, bool kMask, bool kWide>
 __global__ void __launch_bounds__(kWarps * 32) norm_emit_kernel(SegNorm s) {
   extern __shared__ __align__(16) unsigned char rings[];
   const ScanNormArgs& a = s.a;
   const PairLane l = pair_lane(s);
   if (!l.active) return;
   const T* x = reinterpret_cast<const T*>(a.x) + l.b * a.xsb + l.d0;
-  T* py = reinterpret_cast<T*>(a.y) + l.b * a.ysb + (long long)l.t0 * a.ysl + l.dc;
+  const bool own = !kWide || a.y != nullptr;
+  T* py = own ? reinterpret_cast<T*>(a.y) + l.b * a.ysb + (long long)l.t0 * a.ysl + l.dc : nullptr;
+  float* pw = kWide ? a.wide + ((size_t)l.b * a.L + l.t0) * a.D + l.dc : nullptr;
   const unsigned char* m = kMask ? a.mask + (size_t)l.b * a.L : nullptr;
   const f32x2 w = ldg2(a.gamma + l.dc), bb = ldg2(a.beta + l.dc);
   const float eps = a.eps;
@@ -160,8 +163,14 @@ __global__ void __launch_bounds__(kWarps * 32) norm_emit_kernel(SegNorm s) {
                                   const f32x2 d = st.step(xv, eps, inv, r);
                                   out = fma2(mul2(sub2(d, st.u), r), w, bb);
                                 }
-                                if (l.ok) pair_st(py, out);
-                                py += a.ysl;
+                                if (kWide) {
+                                  if (l.ok) *reinterpret_cast<f32x2*>(pw) = out;
+                                  pw += a.D;
+                                }
+                                if (own) {
+                                  if (l.ok) pair_st(py, out);
+                                  py += a.ysl;
+                                }
                               });
   if (l.seg == s.S - 1 && l.ok) {
     const bool any = st.n > 0.f;
@@ -416,7 +425,8 @@ static void fwd_launch(const SegNorm& s, cudaStream_t st) {
   const dim3 pairs((s.a.D + 63) / 64, grid.y, grid.z);
   const size_t rings = (size_t)kWarps * kRing * kTileBytes;
   launch(norm_moments_kernel<T, kMask>, grid, block, rings, (void*)st, moments_of(s));
-  launch(norm_emit_kernel<T, kMask>, pairs, block, rings, (void*)st, s);
+  if (s.a.wide) launch(norm_emit_kernel<T, kMask, true>, pairs, block, rings, (void*)st, s);
+  else launch(norm_emit_kernel<T, kMask, false>, pairs, block, rings, (void*)st, s);
 }
 template <typename T, bool kMask>
 static void bwd_launch(const SegNorm& s, cudaStream_t st) {
@@ -508,7 +518,9 @@ static bool pairs_ok(int dtype, const ScanNormArgs& a, long long ysd) {
 }
 
 bool scan_norm_fwd_try(int dtype, const ScanNormArgs& a, long long xsd, long long ysd, cudaStream_t s) {
-  if (!pieces_ok(dtype, a.D) || !rows_ok(dtype, a.x, a.xsb, a.xsl, xsd) || !pairs_ok(dtype, a, ysd) || a.x == a.y) return false;
+  if (!pieces_ok(dtype, a.D) || !rows_ok(dtype, a.x, a.xsb, a.xsl, xsd) || !((a.wide && !a.y) || pairs_ok(dtype, a, ysd)) ||
+      a.x == a.y)
+    return false;
   // (every segment's block reads the incoming statistics, the last one's writes the new ones)
   const size_t n = (size_t)a.B * a.D;
   for (const float* out : {a.mean_out, a.var_out})

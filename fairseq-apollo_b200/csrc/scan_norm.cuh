@@ -7,6 +7,7 @@ namespace mega {
 struct ScanNormArgs {
   const void* x;
   void* y;          // forward: output; backward: input gradient
+  float* wide;      // forward: the output in fp32 too, dense (B, L, D), or null; y may then be null
   const void* dy;
   int B, D, L;
   long long xsb, xsl, ysb, ysl, gsb, gsl;

@@ -159,3 +159,38 @@ def test_chosen_calls_agree_with_the_scan(cplx):
         if a.is_complex():
             a, b = torch.view_as_real(a), torch.view_as_real(b)
         assert rel_l2(a, b) < 1e-5   # (the scan's own error: 3e-6)
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("bsz,length,dim", [(1, 33, 8), (2, 200, 24), (3, 513, 40)])
+@pytest.mark.parametrize("normed", [False, True])
+def test_behind_timestep_norm(forced, bsz, length, dim, dtype, cplx, normed):
+    """TimestepNorm -> EMA with states in and out: the products take the normalised activations in fp32, not as they are
+    rounded for the second output."""
+    from fairseq_apollo_b200 import ops
+    from oracle import mega_oracle as O
+    gen = torch.Generator().manual_seed(length)
+    x, _, p, q, g, omega = problem(gen, bsz, length, dim, 16, dtype, cplx)
+    if dtype == torch.bfloat16 and not cplx and not normed:
+        pytest.skip("another form's call")
+    pc = torch.full((bsz,), 3, dtype=torch.int64)
+    pm, pv = torch.randn(bsz, dim, generator=gen) * 0.1, torch.rand(bsz, dim, generator=gen) + 0.5
+    gamma, beta = torch.randn(dim, generator=gen) * 0.1 + 1, torch.randn(dim, generator=gen) * 0.1
+    h = torch.randn(bsz, dim, 16, dtype=q.dtype, generator=gen)
+    xn, cnt, mean, var = O.timestep_norm(x.double(), pc, pm.double(), pv.double(), gamma.double(), beta.double(), None,
+                                         acc_dtype=torch.float64)[:4]
+    want, last = recurrence(xn, *[double(t) for t in (p, q, g, omega)], double(h))
+    c = [t.cuda() for t in (pc, pm, pv, gamma, beta)]
+    got = ops.tsn_ema_forward(x.cuda(), *c, 1e-5, p.cuda(), q.cuda(), g.cuda(), omega.cuda(), None, h_in=h.cuda(), want_state=True,
+                              want_normed=normed, complex_poles=cplx)
+    assert forced.last_kernel() == "chunk_ema"
+    limit = max(LIMIT[dtype], 4e-6)   # (the statistics: reciprocals and roots to 2^-22, sums of up to 513 deviations)
+    assert rel_l2(got["y"], want) < limit
+    if normed:
+        assert rel_l2(got["xn"], xn) < limit
+    out = got["h"]
+    if cplx:
+        out, last = torch.view_as_real(out.cpu()), torch.view_as_real(last)
+    assert rel_l2(out, last) < 4e-6
+    assert torch.equal(got["count"].cpu(), cnt) and rel_l2(got["mean"], mean) < 4e-6 and rel_l2(got["var"], var) < 4e-6
