@@ -61,7 +61,7 @@ struct Blocks {
   static constexpr int v = kC ? 4 : 2, t = 2, g = kC ? 4 : 2;
 };
 
-template <typename In, typename Out, bool kC, int kMode>
+template <typename In, typename Out, bool kC, int kMode, bool kMask>
 struct Form {
   static constexpr int kP = kPartsOf<In>;
   // positions of a tile (what shared memory holds), and bytes of a row: eight rows hit different banks
@@ -79,10 +79,12 @@ struct Form {
   static constexpr int kE = 16 / (int)sizeof(In), kPos = kTile / (4 * kE);  // channels of a 16-byte piece; positions of a thread
   static constexpr int kSlot = kIns * kPos * kThreads * 16;        // bytes of a tile as it arrives
   static constexpr int stage = kBufs * kIns * kP * kPlane;
-  static constexpr int fixed = stage + kShared * kCh * kBlockBytes;
+  static constexpr int fixed = stage + kShared * kCh * kBlockBytes + (kMask ? 512 : 0);
   static constexpr int kSlots = fixed + 2 * kSlot <= (kCh == 8 ? 112 : 226) * 1024 ? 2 : 1;
   static constexpr int mats = stage + kSlots * kSlot;
-  static constexpr int total = mats + kShared * kCh * kBlockBytes;
+  static constexpr int bits = mats + kShared * kCh * kBlockBytes;  // padded positions: a word for 32 of them, two sets
+  static constexpr int kBits = 8 * kTile / 32;                     // words of a set
+  static constexpr int total = bits + (kMask ? 2 * kBits * 4 : 0);
   static constexpr int kPerSm = kCh == 8 && total <= 112 * 1024 ? 2 : 1;
   static_assert(total <= 227 * 1024, "a block's shared memory");
 };
@@ -325,13 +327,17 @@ __global__ void __launch_bounds__(128) chunk_prepare_kernel(PrepArgs a) {
 }
 
 // ---- the walk ----------------------------------------------------------------------------------------------
-template <typename In, typename Out, bool kC, int kMode>
-__global__ void __launch_bounds__(Form<In, Out, kC, kMode>::kThreads, Form<In, Out, kC, kMode>::kPerSm) chunk_kernel(ChunkArgs s) {
-  using F = Form<In, Out, kC, kMode>;
+// kMask: padded positions are zero to the states (and to the correlations), omega x takes them as they are; in reversed time,
+// where outputs are the input's gradient, it is the outputs at padded positions that are omega dy alone.
+template <typename In, typename Out, bool kC, int kMode, bool kMask>
+__global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask>::kThreads, Form<In, Out, kC, kMode, kMask>::kPerSm)
+    chunk_kernel(ChunkArgs s) {
+  using F = Form<In, Out, kC, kMode, kMask>;
   constexpr int kP = F::kP, kV = F::kV, kPlane = F::kPlane, kCh = F::kCh, kTile = F::kTile, kRow = F::kRow;
   constexpr int kRe = kC ? 2 : 1;      // real numbers of a value
   constexpr bool kSens = kMode == kLocalSens || kMode == kGrad;
-  constexpr bool kApart = kMode == kEmit && sizeof(Out) == 4;   // omega x in fp32: the tensor pipe truncates its sums
+  constexpr bool kWide = kMode == kEmit && sizeof(Out) == 4;   // leading products by themselves: the tensor pipe truncates its sums
+  constexpr bool kApart = kWide || (kMode == kEmit && kMask);   // omega x in fp32
   extern __shared__ __align__(16) unsigned char smem[];
   const ScanArgs& a = s.a;
   int tid;
@@ -446,6 +452,21 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode>::kThreads, Form<In, O
   // kGrad: A1 and A2 of the lane's poles, R of its entries
   float a1[kMode == kGrad ? kRe : 1][4] = {}, a2[kMode == kGrad ? kRe : 1][4] = {}, R[kMode == kGrad ? 8 : 1] = {};
 
+  float beside = 0.f;   // of omega, at padded positions
+  // columns 8 k .. of x and dy with the 16 chunks as the reduction (products of parts below 2^-24 are left out)
+  auto correlate = [](float (&r)[4], const uint32_t (&x)[kP][4], const uint32_t (&y)[kP][4], int k) {
+    bool onto = false;
+#pragma unroll
+    for (int o = 2 * kP - 2; o >= 0; --o)
+#pragma unroll
+      for (int p = 0; p < kP; ++p)
+        if (o <= 2 && o - p >= 0 && o - p < kP) {
+          if (onto) mma(r, x[p], y[o - p][2 * k], y[o - p][2 * k + 1]);
+          else mma0(r, x[p], y[o - p][2 * k], y[o - p][2 * k + 1]);
+          onto = true;
+        }
+  };
+
   // eight rows of 16 bytes each: segments, their first or second chunk, lower or upper half of it
   const int blk_in = (lane >> 3) & 1;
   const uint32_t frag_row = smem_u32(smem) + (warp * 8 + (lane & 7)) * kRow + (lane >> 4) * 16;
@@ -467,6 +488,32 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode>::kThreads, Form<In, O
       for (int st = 0; st < kStep; ++st)
 #pragma unroll
         for (int p = 0; p < kP; ++p) ldmatrix(f[st][p], rows(st) + p * kPlane);
+      // bits of the segment's row in a step; what they leave of the lane's words of a fragment
+      const uint32_t* bits = kMask ? reinterpret_cast<const uint32_t*>(smem + F::bits) + (tile & 1) * F::kBits + s0 : nullptr;
+      auto keep = [&](uint32_t w, int i) {   // word i: rows g and g + 8 (the step's chunks), then their upper halves
+        const uint32_t two = w >> (16 * (i & 1) + 8 * (i >> 1) + 2 * t) & 3u;
+        return (two & 1u ? 0u : 0xffffu) | (two & 2u ? 0u : 0xffff0000u);
+      };
+      uint32_t padded[kStep];
+      bool some = false;
+      if constexpr (kMask) {
+#pragma unroll
+        for (int st = 0; st < kStep; ++st) {
+          padded[st] = bits[g * (kTile / 32) + st];
+          some = some || padded[st] != 0u;
+        }
+        some = __any_sync(0xffffffffu, some);
+      }
+      if (kMask && some && !(kMode == kEmit && s.rev)) {
+#pragma unroll
+        for (int st = 0; st < kStep; ++st)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const uint32_t m = keep(padded[st], i);
+#pragma unroll
+            for (int p = 0; p < kP; ++p) f[st][p][i] &= m;
+          }
+      }
       if constexpr (kMode == kLocal || kMode == kLocalSens) {
 #pragma unroll
         for (int k = 0; k < 2; ++k) {   // eight poles at a time
@@ -523,7 +570,7 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode>::kThreads, Form<In, O
                 float x = 0.f;
 #pragma unroll
                 for (int pl = kP - 1; pl >= 0; --pl) x += __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(from + pl * kPlane));
-                x *= p;
+                x = kMask && (padded[st] >> k & 1u) ? 0.f : x * p;
                 const float r = kC ? fmaf(fr, re, fmaf(-fi, im, x)) : fmaf(fr, re, x);
                 if (kC) im = fmaf(fr, im, fi * re);
                 re = r;
@@ -596,7 +643,7 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode>::kThreads, Form<In, O
             for (int k = 0; k < 2; ++k) {
               const Frag m = matrix(c < kRe ? kV + 2 + 2 * c + k : kV + k);
               const uint32_t(&p)[4] = c < kRe ? hp[c < kRe ? c : 0][0] : f[st][0];
-              if (kApart) {   // (by themselves, so that what truncates is small)
+              if (kWide) {   // (by themselves, so that what truncates is small)
                 float l[4];
                 mma0(l, p, m.u.x, m.u.y);
 #pragma unroll
@@ -606,6 +653,11 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode>::kThreads, Form<In, O
               }
             }
           if (kApart) {
+            uint32_t own_x[kMask ? kP : 1][4];   // as they came
+            if constexpr (kMask) {
+#pragma unroll
+              for (int p = 0; p < kP; ++p) ldmatrix(own_x[p], rows(st) + p * kPlane);
+            }
 #pragma unroll
             for (int k = 0; k < 2; ++k)
 #pragma unroll
@@ -613,8 +665,14 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode>::kThreads, Form<In, O
                 float x0 = 0.f, x1 = 0.f;
 #pragma unroll
                 for (int p = kP - 1; p >= 0; --p) {
-                  x0 += __uint_as_float(f[st][p][2 * k + r] << 16);
-                  x1 += __uint_as_float(f[st][p][2 * k + r] & 0xffff0000u);
+                  const uint32_t w = kMask ? own_x[kMask ? p : 0][2 * k + r] : f[st][p][2 * k + r];
+                  x0 += __uint_as_float(w << 16);
+                  x1 += __uint_as_float(w & 0xffff0000u);
+                }
+                if (kMask && some && s.rev) {
+                  const uint32_t m = keep(padded[st], 2 * k + r);
+                  if (!(m & 0xffffu)) y[k][2 * r] = 0.f;
+                  if (!(m & 0xffff0000u)) y[k][2 * r + 1] = 0.f;
                 }
                 y[k][2 * r] = fmaf(om, x0, y[k][2 * r]);
                 y[k][2 * r + 1] = fmaf(om, x1, y[k][2 * r + 1]);
@@ -627,7 +685,9 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode>::kThreads, Form<In, O
           if (any_odd) {
 #pragma unroll
             for (int i = 0; i < 8; ++i)
-              if (8 * (i >> 2) + 2 * t + (i & 1) >= bad[(i >> 1) & 1]) y[i >> 2][i & 3] = __int_as_float(0x7fffffff);
+              if (8 * (i >> 2) + 2 * t + (i & 1) >= bad[(i >> 1) & 1] &&
+                  !(kMask && s.rev && !(keep(padded[st], 2 * (i >> 2) + ((i >> 1) & 1)) >> (16 * (i & 1)) & 1u)))
+                y[i >> 2][i & 3] = __int_as_float(0x7fffffff);
           }
 #pragma unroll
           for (int k = 0; k < 2; ++k)
@@ -701,19 +761,32 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode>::kThreads, Form<In, O
             f[st][p][0] = m[0]; f[st][p][1] = m[2]; f[st][p][2] = m[1]; f[st][p][3] = m[3];
             ldmatrix_t(e[st][p], rows(st) + (kP + p) * kPlane);
           }
+          if (kMask && some) {   // the padded positions' own products are omega's alone
+            uint32_t only[kP][4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {   // (position g or g + 8 of the chunks of the segments 2t and 2t + 1)
+              const int at = 16 * (i >> 1) + g + 8 * (i & 1);
+              const uint32_t m = (bits[2 * t * (kTile / 32) + st] >> at & 1u ? 0u : 0xffffu) |
+                                 (bits[(2 * t + 1) * (kTile / 32) + st] >> at & 1u ? 0u : 0xffff0000u);
+#pragma unroll
+              for (int p = 0; p < kP; ++p) {
+                only[p][i] = f[st][p][i] & ~m;
+                f[st][p][i] &= m;
+              }
+            }
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+              float r[4];
+              correlate(r, only, e[st], k);
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                if (8 * k + 2 * t + (i & 1) == 15 - g - 8 * (i >> 1)) beside += r[i];
+            }
+          }
 #pragma unroll
           for (int k = 0; k < 2; ++k) {
             float r[4];
-            bool onto = false;
-#pragma unroll
-            for (int o = 2 * kP - 2; o >= 0; --o)   // (products of parts p and o - p: below 2^-24 they are left out)
-#pragma unroll
-              for (int p = 0; p < kP; ++p)
-                if (o <= 2 && o - p >= 0 && o - p < kP) {
-                  if (onto) mma(r, f[st][p], e[st][o - p][2 * k], e[st][o - p][2 * k + 1]);
-                  else mma0(r, f[st][p], e[st][o - p][2 * k], e[st][o - p][2 * k + 1]);
-                  onto = true;
-                }
+            correlate(r, f[st], e[st], k);
 #pragma unroll
             for (int i = 0; i < 4; ++i) R[(kMode == kGrad ? 4 * k + i : 0)] += r[i];   // (in fp32: the tensor pipe truncates its sums)
           }
@@ -721,7 +794,30 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode>::kThreads, Form<In, O
       }
     }
   };
+  // padded positions of a tile: a word for 32 positions of a row, in the order they are walked; read a tile ahead
+  constexpr int kVotes = F::kBits / kCh;   // words of a warp
+  bool pad[kMask ? kVotes : 1];
+  auto look = [&](int tile) {
+    if constexpr (kMask) {
+#pragma unroll
+      for (int i = 0; i < kVotes; ++i) {
+        const int word = warp * kVotes + i, r = blockIdx.y * 8 + word / (kTile / 32), bb = r / s.walked, first = (r - bb * s.walked) * s.T;
+        const int pos = tile * kTile + word % (kTile / 32) * 32 + lane, at = first + pos;
+        pad[i] = bb < a.B && pos < s.T && at < a.L && __ldg(a.mask + (size_t)bb * a.L + (s.rev ? a.L - 1 - at : at)) != 0;
+      }
+    }
+  };
+  look(0);
   auto arrive = [&](int tile) {   // the tile's rows, and the copies of one further on
+    if constexpr (kMask) {
+      uint32_t* bits = reinterpret_cast<uint32_t*>(smem + F::bits) + (tile & 1) * F::kBits;
+#pragma unroll
+      for (int i = 0; i < kVotes; ++i) {
+        const uint32_t v = __ballot_sync(0xffffffffu, pad[i]);
+        if (lane == 0) bits[warp * kVotes + i] = v;
+      }
+      look(tile + 1);
+    }
     asm volatile("cp.async.wait_group %0;" ::"n"(F::kSlots - 1) : "memory");
     if (tile < tiles) {
       const unsigned char* slot = smem + F::stage + tid * 16 + tile % F::kSlots * F::kSlot;
@@ -840,7 +936,11 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode>::kThreads, Form<In, O
         atomicAdd(a.dq + at, p * gn * sr);
       }
     }
-    if (lane == 0 && d < a.D) atomicAdd(a.domega + d, lag);
+    if (kMask) {
+#pragma unroll
+      for (int m = 1; m < 32; m <<= 1) beside += __shfl_xor_sync(0xffffffffu, beside, m);
+    }
+    if (lane == 0 && d < a.D) atomicAdd(a.domega + d, kMask ? lag + beside : lag);
   }
 }
 
@@ -918,11 +1018,11 @@ __global__ void __launch_bounds__(128) chunk_carry_kernel(ChunkArgs s) {
 }
 
 // ---- launches ----------------------------------------------------------------------------------------------
-template <typename In, typename Out, bool kC, int kMode>
+template <typename In, typename Out, bool kC, int kMode, bool kMask>
 void run(const ChunkArgs& s, cudaStream_t st) {
-  using F = Form<In, Out, kC, kMode>;
+  using F = Form<In, Out, kC, kMode, kMask>;
   const dim3 grid((s.a.D + F::kCh - 1) / F::kCh, (unsigned)(((long long)s.a.B * s.walked + 7) / 8));
-  launch(chunk_kernel<In, Out, kC, kMode>, grid, F::kThreads, F::total, (void*)st, s);
+  launch(chunk_kernel<In, Out, kC, kMode, kMask>, grid, F::kThreads, F::total, (void*)st, s);
 }
 
 // Steps of a segment: a multiple of 64 (two steps of the tensor products) that minimises rounds of blocks over the SMs x
@@ -948,7 +1048,7 @@ double pick(const ScanArgs& a, ChunkArgs& s) {
 }
 
 bool envelope(int dtype, const ScanArgs& a) {
-  return g_options[OPT_CHUNK].load() != 1 && g_options[OPT_DISABLE_STREAM].load() == 0 && !a.bidir && !a.mask && !a.prev_count && a.N >= 1 &&
+  return g_options[OPT_CHUNK].load() != 1 && g_options[OPT_DISABLE_STREAM].load() == 0 && !a.bidir && !a.prev_count && a.N >= 1 &&
          a.N <= 16 && a.B <= 65535 && a.L >= 1 && a.L < 0x7fffff00 && pieces_ok(dtype, a.D);
 }
 
@@ -959,7 +1059,8 @@ double chunk_us(int dtype, const ScanArgs& a, bool bwd, double cost, bool segmen
   static const double kFwd[2][3] = {{25., 32., 43.}, {44., 54., 64.}}, kBwd[2][3] = {{55., 82., 109.}, {105., 155., 185.}};
   const int parts = dtype == MEGA_BF16 ? 0 : dtype == MEGA_F16 ? 1 : 2;
   return (bwd ? (segmented ? 38. : 24.) : (segmented ? 22. : 14.)) +
-         (bwd ? kBwd : kFwd)[a.cplx ? 1 : 0][parts] * 1e-3 * cost * (segmented ? 1. : a.cplx ? 1.14 : 1.07);
+         (bwd ? kBwd : kFwd)[a.cplx ? 1 : 0][parts] * 1e-3 * cost * (segmented ? 1. : a.cplx ? 1.14 : 1.07) *
+             (a.mask ? (bwd ? 1.22 : 1.33) : 1.);
 }
 // The form that a call takes otherwise: the scan backward (real bf16 16 x 4096 x 1024: 517 us against 241 here, complex 1481
 // against 459, fp32 539 against 500); forward the cluster kernel, the scan (fp32 complex of that size: 565 against 385; real fp32
@@ -968,9 +1069,9 @@ double chunk_us(int dtype, const ScanArgs& a, bool bwd, double cost, bool segmen
 double other_us(int dtype, const ScanArgs& a, bool bwd) {
   const double L = a.L, n = (double)a.B * a.D * L;
   if (bwd) return a.cplx ? 59. + n / 47e3 : 40. + n / 125e3;
-  if (dtype == MEGA_BF16 && g_options[OPT_DISABLE_MMA].load() == 0 && !(a.cplx && a.h_out && a.L % 32 != 0))
+  if (dtype == MEGA_BF16 && g_options[OPT_DISABLE_MMA].load() == 0 && !(a.cplx && (a.mask || (a.h_out && a.L % 32 != 0))))
     return scan_cluster_first(dtype, a, 1, 1) ? 0.9 * scan_cluster_us(dtype, a)
-                                              : a.cplx ? 95. + std::max(L * 29e-3, n / 700e3) : 6. + std::max(L * 22e-3, n / 1300e3);
+                                              : a.cplx ? 95. + std::max(L * 29e-3, n / 700e3) : 6. + std::max(L * (a.mask ? 42e-3 : 22e-3), n / 1300e3);
   const double one = scan_cluster_us(dtype, a);
   return one < 1e29 ? 0.9 * one : std::min(scan_ema_fwd_us(a), a.cplx ? 25. + n / 123e3 : 15. + n / 270e3);
 }
@@ -981,7 +1082,7 @@ bool pays(int dtype, const ScanArgs& a, bool bwd, double cost, bool segmented) {
   return g_options[OPT_MMA_TILE].load() == 0 && chunk_us(dtype, a, bwd, cost, segmented) < 0.93 * other_us(dtype, a, bwd);
 }
 
-template <typename In, typename Out, bool kC>
+template <typename In, typename Out, bool kC, bool kMask>
 bool fwd(int dtype, const ScanArgs& a, bool asked, cudaStream_t st) {
   ChunkArgs s{};
   s.a = a;
@@ -999,23 +1100,23 @@ bool fwd(int dtype, const ScanArgs& a, bool asked, cudaStream_t st) {
   s.frag = fr;
   s.pow = pow;
   s.carry = carry ? sc.take<float>(carry) : nullptr;
-  const PrepArgs p{a.p, a.q, a.g, a.omega, a.D, a.N, 0, 1, state ? 1 : 0, sizeof(Out) == 4 ? 0 : 1, kBlocks, fr, pow};
+  const PrepArgs p{a.p, a.q, a.g, a.omega, a.D, a.N, 0, 1, state ? 1 : 0, sizeof(Out) == 4 || kMask ? 0 : 1, kBlocks, fr, pow};
   launch(chunk_prepare_kernel<kC>, (unsigned)((a.D + 3) / 4), 128, 0, (void*)st, p);
   s.in = a.x;
   s.isb = a.xsb;
   s.isl = a.xsl;
   if (s.S > 1) {
     s.walked = s.S - 1;
-    run<In, In, kC, kLocal>(s, st);
+    run<In, In, kC, kLocal, kMask>(s, st);
     launch(chunk_carry_kernel<kC, false>, dim3((a.D * 16 + 127) / 128, a.B), 128, 0, (void*)st, s);
   }
   s.walked = s.S;
-  run<In, Out, kC, kEmit>(s, st);
+  run<In, Out, kC, kEmit, kMask>(s, st);
   g_last_kernel.store("chunk_ema", std::memory_order_relaxed);
   return true;
 }
 
-template <typename T, bool kC>
+template <typename T, bool kC, bool kMask>
 bool bwd(int dtype, const ScanArgs& a, cudaStream_t st) {
   ChunkArgs s{};
   s.a = a;
@@ -1032,7 +1133,7 @@ bool bwd(int dtype, const ScanArgs& a, cudaStream_t st) {
   s.frag = fr;
   s.pow = pow;
   s.carry = carry ? sc.take<float>(carry) : nullptr;
-  const PrepArgs p{a.p, a.q, a.g, a.omega, a.D, a.N, 1, 1, 0, sizeof(T) == 4 ? 0 : 1, kBlocks, fr, pow};
+  const PrepArgs p{a.p, a.q, a.g, a.omega, a.D, a.N, 1, 1, 0, sizeof(T) == 4 || kMask ? 0 : 1, kBlocks, fr, pow};
   launch(chunk_prepare_kernel<kC>, (unsigned)((a.D + 3) / 4), 128, 0, (void*)st, p);
   ChunkArgs x = s, g = s;   // forward over x; backward over dy
   x.in = a.x;
@@ -1045,13 +1146,13 @@ bool bwd(int dtype, const ScanArgs& a, cudaStream_t st) {
   g.part = 2 * kRe;
   if (s.S > 1) {
     x.walked = g.walked = s.S - 1;
-    run<T, T, kC, kLocalSens>(x, st);
-    run<T, T, kC, kLocal>(g, st);
+    run<T, T, kC, kLocalSens, kMask>(x, st);
+    run<T, T, kC, kLocal, false>(g, st);
     launch(chunk_carry_kernel<kC, true>, dim3((a.D * 16 + 127) / 128, a.B, 2), 128, 0, (void*)st, s);
   }
   x.walked = g.walked = s.S;
-  run<T, T, kC, kGrad>(x, st);
-  run<T, T, kC, kEmit>(g, st);
+  run<T, T, kC, kGrad, kMask>(x, st);
+  run<T, T, kC, kEmit, kMask>(g, st);
   g_last_kernel.store("chunk_ema", std::memory_order_relaxed);
   return true;
 }
@@ -1063,15 +1164,19 @@ bool chunk_ema_fwd_try(int dtype, int out_dtype, const ScanArgs& a, long long xs
   if (!envelope(dtype, a) || !pieces_ok(out_dtype, a.D) || !rows_ok(dtype, a.x, a.xsb, a.xsl, xsd) ||
       !rows_ok(out_dtype, a.y, a.ysb, a.ysl, ysd))
     return false;
-#define MEGA_FWD(IN, OUT) return a.cplx ? fwd<IN, OUT, true>(dtype, a, asked, s) : fwd<IN, OUT, false>(dtype, a, asked, s)
-  if (dtype == MEGA_F32 && out_dtype == MEGA_BF16) MEGA_FWD(float, __nv_bfloat16);
-  if (dtype == MEGA_F32 && out_dtype == MEGA_F16) MEGA_FWD(float, __half);
+#define MEGA_FWD(IN, OUT, MASK) return a.cplx ? fwd<IN, OUT, true, MASK>(dtype, a, asked, s) : fwd<IN, OUT, false, MASK>(dtype, a, asked, s)
+#define MEGA_FWD_SAME(TY) if (a.mask) MEGA_FWD(TY, TY, true); else MEGA_FWD(TY, TY, false)
+  if (dtype == MEGA_F32 && out_dtype == MEGA_BF16 && !a.mask) MEGA_FWD(float, __nv_bfloat16, false);
+  if (dtype == MEGA_F32 && out_dtype == MEGA_F16 && !a.mask) MEGA_FWD(float, __half, false);
   if (dtype != out_dtype) return false;
-  if (dtype == MEGA_F32) MEGA_FWD(float, float);
-  if (dtype == MEGA_BF16) MEGA_FWD(__nv_bfloat16, __nv_bfloat16);
-  if (dtype == MEGA_F16) MEGA_FWD(__half, __half);
+  switch (dtype) {
+    case MEGA_F32: MEGA_FWD_SAME(float);
+    case MEGA_BF16: MEGA_FWD_SAME(__nv_bfloat16);
+    case MEGA_F16: MEGA_FWD_SAME(__half);
+    default: return false;
+  }
+#undef MEGA_FWD_SAME
 #undef MEGA_FWD
-  return false;
 }
 
 double chunk_ema_fwd_us(int dtype, const ScanArgs& a) {
@@ -1086,9 +1191,13 @@ bool chunk_ema_bwd_try(int dtype, const ScanArgs& a, long long xsd, long long ys
       !rows_ok(dtype, a.dy, a.gsb, a.gsl, gsd) || !rows_ok(dtype, a.y, a.ysb, a.ysl, ysd))
     return false;
   switch (dtype) {
-    case MEGA_F32: return a.cplx ? bwd<float, true>(dtype, a, s) : bwd<float, false>(dtype, a, s);
-    case MEGA_BF16: return a.cplx ? bwd<__nv_bfloat16, true>(dtype, a, s) : bwd<__nv_bfloat16, false>(dtype, a, s);
-    case MEGA_F16: return a.cplx ? bwd<__half, true>(dtype, a, s) : bwd<__half, false>(dtype, a, s);
+#define MEGA_BWD(TY)                                                                                            \
+  return a.mask ? (a.cplx ? bwd<TY, true, true>(dtype, a, s) : bwd<TY, false, true>(dtype, a, s))                \
+                : (a.cplx ? bwd<TY, true, false>(dtype, a, s) : bwd<TY, false, false>(dtype, a, s))
+    case MEGA_F32: MEGA_BWD(float);
+    case MEGA_BF16: MEGA_BWD(__nv_bfloat16);
+    case MEGA_F16: MEGA_BWD(__half);
+#undef MEGA_BWD
     default: return false;
   }
 }

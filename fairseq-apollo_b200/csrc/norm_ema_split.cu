@@ -46,8 +46,8 @@ double fused_us(int dtype, const StreamArgs& a, bool want_xn) {
   // (the streamed chain: 171 to 260 ns a position complex, 150 to 200 real, more where the channels do not fit the SMs at once;
   // with a second output a third of the rate: 57 x 995 x 632 fp32 163 us and 489)
   const bool slow = want_xn || a.h_in || a.h_out;
-  return a.cplx ? (slow ? 30.0 + longer(234.0, 70e3, L, n) : 8.0 + longer(171.0, 130e3, L, n))
-                : slow ? 15.0 + longer(185.0, 85e3, L, n) : 6.0 + longer(145.0, 230e3, L, n);
+  return a.cplx ? (slow ? 25.0 + longer(234.0, 75e3, L, n) : 8.0 + longer(171.0, 130e3, L, n))
+                : slow ? 10.0 + longer(185.0, 100e3, L, n) : 6.0 + longer(145.0, 230e3, L, n);
 }
 
 // TimestepNorm, then the tensor-core kernel alone: where the fused call would run on it too (both round the normalised
@@ -70,6 +70,7 @@ constexpr double kWideMost = 62e6;   // elements of scratch memory: what the poo
 double chunk_us(int dtype, const ScanArgs& ea) {
   ScanArgs a = ea;
   a.prev_count = nullptr;
+  a.mask = nullptr;
   const double n = (double)a.B * a.D * a.L;
   if (dtype != MEGA_F32 && n > kWideMost) return 1e30;
   return 18.0 + n / (dtype == MEGA_F32 ? 480e3 : 540e3) + chunk_ema_fwd_us(MEGA_F32, a);
@@ -80,10 +81,11 @@ bool norm_chunk_try(int dtype, const ScanArgs& ea, long long xsd, long long ysd,
   na.x = ea.x; na.B = ea.B; na.D = ea.D; na.L = ea.L;
   na.xsb = ea.xsb; na.xsl = ea.xsl; na.ysb = ea.ysb; na.ysl = ea.ysl;
   na.prev_count = ea.prev_count; na.prev_mean = ea.prev_mean; na.prev_var = ea.prev_var; na.gamma = ea.gamma; na.beta = ea.beta;
-  na.eps = ea.eps; na.count_out = ea.count_out; na.mean_out = ea.mean_out; na.var_out = ea.var_out;
+  na.eps = ea.eps; na.count_out = ea.count_out; na.mean_out = ea.mean_out; na.var_out = ea.var_out; na.mask = ea.mask;
   ScanArgs a = ea;
   a.prev_count = nullptr;
   a.xn = nullptr;
+  a.mask = nullptr;   // (the norm has zeroed what is padded)
   if (dtype == MEGA_F32) {
     na.y = ea.xn ? ea.xn : ea.y;
     a.x = na.y;
@@ -124,7 +126,7 @@ bool norm_ema_split_try(int dtype, const void* x, void* y, void* xn, long long x
   const bool chunk = dtype == MEGA_BF16 && a.h_out && !a.mask && !a.cplx;
   const double fused = fused_us(dtype, a, xn != nullptr), scan = scan_us(dtype, ea, xn != nullptr) + (chunk ? 25.0 : 0.0),
                mma = mma_us(dtype, a, xn != nullptr) + 25.0;
-  if (forced == 0 && !a.mask) {   // (what stands in mean_out and the like once the norm has run is what the forms below write too)
+  if (forced == 0) {   // (what stands in mean_out and the like once the norm has run is what the forms below write too)
     const double chunk = chunk_us(dtype, ea);
     if ((chunk < 0.88 * (scan < mma ? scan : mma) && chunk < 0.88 * fused) || (chunk < 1e29 && g_options[OPT_CHUNK].load() == 2))
       if (norm_chunk_try(dtype, ea, xsd, ysd, s)) return true;

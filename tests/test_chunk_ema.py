@@ -88,6 +88,50 @@ def test_against_float64(forced, bsz, length, dim, ndim, dtype, cplx):
     assert rel_l2(out, last) < 5e-7
 
 
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("bsz,length,dim,ndim", [(2, 37, 16, 5), (3, 130, 24, 16), (9, 200, 16, 16), (2, 1500, 8, 16)])
+def test_padded_positions(forced, bsz, length, dim, ndim, dtype, cplx):
+    """Zero to the states whatever stands there, NaN included in omega x's own position; their input gradient is omega dy."""
+    from fairseq_apollo_b200 import ops
+    gen = torch.Generator().manual_seed(length)
+    x, dy, p, q, g, omega = problem(gen, bsz, length, dim, ndim, dtype, cplx)
+    mask = torch.rand(bsz, length, generator=gen) < 0.2
+    mask[-1, length // 2:] = True
+    leaves = [double(t).requires_grad_(True) for t in (x, p, q, g, omega)]
+    masked = leaves[0].masked_fill(mask.unsqueeze(-1), 0.)
+    want = recurrence(masked, *leaves[1:4], torch.zeros(dim, dtype=torch.float64))[0] + leaves[4] * leaves[0]
+    want.backward(dy.double())
+    fwd, bwd = (ops.cema_forward, ops.cema_backward) if cplx else (ops.ema_forward, ops.ema_backward)
+    c = [t.cuda() for t in (p, q, g, omega)]
+    xc, dyc, mc = x.cuda().transpose(1, 2), dy.cuda().transpose(1, 2), mask.cuda()
+    y, got = fwd(xc, *c, mc), bwd(dyc, xc, *c, mc)
+    assert forced.last_kernel() == "chunk_ema"
+    assert rel_l2(y.transpose(1, 2), want) < LIMIT[dtype] and rel_l2(got[0].transpose(1, 2), leaves[0].grad) < LIMIT[dtype]
+    for a, b in zip(got[1:5], leaves[1:]):
+        b = b.grad
+        if a.is_complex():
+            a, b = torch.view_as_real(a.cpu()), torch.view_as_real(b)
+        assert rel_l2(a, b) < SUMS
+    h = torch.randn(bsz, dim, ndim, dtype=q.dtype, generator=gen)
+    _, last = recurrence(masked.detach(), *[t.detach() for t in leaves[1:]], double(h))
+    out = fwd(xc, *c, mc, h.cuda(), True)[1]
+    assert forced.last_kernel() == "chunk_ema"
+    if cplx:
+        out, last = torch.view_as_real(out.cpu()), torch.view_as_real(last)
+    assert rel_l2(out, last) < 5e-7
+    bad = xc.clone()
+    bad[-1, :, length - 1] = float("nan")
+    z = fwd(bad, *c, mc)
+    assert torch.equal(z[..., :length - 1], y[..., :length - 1]) and z[-1, :, -1].isnan().all() and torch.equal(z[:-1], y[:-1])
+    bad = dyc.clone()
+    bad[-1, :, length - 1] = float("inf")
+    dx = bwd(bad, xc, *c, mc)[0]
+    there = mask[-1].nonzero().flatten()[:-1].cuda()
+    assert torch.equal(dx[-1][:, there], got[0][-1][:, there]) and not torch.isfinite(dx[-1, :, -1]).any()
+    assert torch.equal(dx[:-1], got[0][:-1])
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_many_segments_and_any_strides(forced, dtype):
     """Sequences cut into segments, the last one ragged; time-major memory and slices of wider rows."""
