@@ -249,8 +249,8 @@ struct PrepArgs {
 };
 template <bool kC>
 __global__ void __launch_bounds__(128) chunk_prepare_kernel(PrepArgs a) {
-  __shared__ double2 table[4][17][16];
-  __shared__ float taps[4][16];
+  __shared__ double2 table[4][17][16], weight[4][16];
+  __shared__ float taps[4][16], gains[4][16];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, d = blockIdx.x * 4 + warp;
   if (d >= a.D) return;
   double2(&pw)[17][16] = table[warp];
@@ -266,6 +266,11 @@ __global__ void __launch_bounds__(128) chunk_prepare_kernel(PrepArgs a) {
       qi = a.q[2 * at + 1];
       wi = p * a.g[2 * at + 1];
     }
+  }
+  // (what the blocks below take from here: read from memory for each of their entries it was half of the kernel's 8.4 us)
+  if (lane < 16) {
+    gains[warp][n] = a.gain && live ? a.p[at] : 1.f;
+    weight[warp][n] = !a.gain || !live ? make_double2(wr, wi) : make_double2(kC ? a.g[2 * at] : a.g[at], kC ? a.g[2 * at + 1] : 0.f);
   }
   double vr = 1., vi = 0.;
   for (int e = 0; e <= 16; ++e) {
@@ -291,6 +296,7 @@ __global__ void __launch_bounds__(128) chunk_prepare_kernel(PrepArgs a) {
   constexpr int kV = Blocks<kC>::v;
   const int g = lane >> 2, t = lane & 3;
   const int us = kV, ts = us + (a.sens ? kV : 0), gs = ts + 2;
+#pragma unroll 2
   for (int blk = 0; blk < a.blocks; ++blk) {
     float v[4];
 #pragma unroll
@@ -303,22 +309,14 @@ __global__ void __launch_bounds__(128) chunk_prepare_kernel(PrepArgs a) {
         const double2 w = pw[sens ? max(e - 1, 0) : e][pole];
         x = nt < 2 ? w.x : w.y;
         if (sens) x *= e;
-        if (pole >= a.N) x = 0.;
-        else if (a.gain) x *= a.p[(size_t)d * a.N + pole];
+        x = pole >= a.N ? 0. : x * gains[warp][pole];
       } else if (blk < gs) {
         const int lag = 8 * (blk - ts) + g - k;
         x = lag >= 0 ? taps[warp][lag] : 0.f;
       } else {
         const int kt = (blk - gs) >> 1, j = 8 * ((blk - gs) & 1) + g;
-        const size_t row = (size_t)d * a.N + k;
-        double cr = 0., ci = 0.;
-        if (k < a.N) {
-          const double p = a.gain ? 1. : (double)a.p[row];
-          cr = p * (kC ? a.g[2 * row] : a.g[row]);
-          if (kC) ci = p * a.g[2 * row + 1];
-        }
-        const double2 w = pw[j + 1][k];
-        x = kt == 0 ? cr * w.x - ci * w.y : -(cr * w.y + ci * w.x);
+        const double2 w = pw[j + 1][k], c = weight[warp][k];
+        x = kt == 0 ? c.x * w.x - c.y * w.y : -(c.x * w.y + c.y * w.x);
       }
       v[i] = (float)x;
     }

@@ -3,7 +3,7 @@
 // The norm pools the statistics of the D / G channels of a group at every step and combines them over the
 // steps.  Only that combination is serial, it is one value per step and group, and it is associative, so
 // a pass is three launches: (1) the moments of every (step, group), a vector of 16 bytes per lane and
-// shuffles inside the group; (2) a scan over the steps, one block per sequence and 8 groups, 128 threads
+// shuffles inside the group; (2) a scan over the steps, one block per sequence and 2 groups, 256 threads
 // along time: each walks its run of steps, the runs are combined across the threads (Chan's rule for
 // counts, means and squared deviations), each walks its run again from what came before; (3) the
 // elementwise part.  The backward is the same with the reverse scan written as plain suffix sums: with
@@ -22,8 +22,11 @@ namespace mega {
 namespace {
 
 constexpr int kRowsPerBlock = 32;   // rows (sequence, step) of a block of the moment and elementwise kernels
-constexpr int kScanG = 8;           // groups per block of the scan
-constexpr int kScanT = 128;         // threads along time per block of the scan
+// Groups per block of the scan, and threads along time: the scan is issue slots and latency, so it goes over as many SMs as
+// there are pairs of groups (8 groups and 128 threads: 16 SMs for 4 sequences of 32 groups, 25 us forward and 41 backward at
+// L = 4096; one group would read a sector of 32 bytes for each float)
+constexpr int kScanG = 2;
+constexpr int kScanT = 256;
 
 template <typename T>
 struct Vec {
@@ -146,7 +149,7 @@ __global__ void __launch_bounds__(kScanG* kScanT) group_scan_kernel(const float*
   }
   part[ti][gi] = r;
   __syncthreads();
-  // inclusive scan over the threads along time (seven rounds)
+  // inclusive scan over the threads along time (eight rounds)
 #pragma unroll
   for (int o = 1; o < kScanT; o <<= 1) {
     Run mine = part[ti][gi];
@@ -322,8 +325,9 @@ __global__ void __launch_bounds__(kScanG* kScanT) group_bwd_scan_kernel(const fl
     cnts[ti] = (float)c;
   }
   __syncthreads();
-  float later = 0.f;
-  for (int i = 0; i < ti; ++i) later += cnts[i];
+  float later = mp ? 0.f : (float)min(L, ti * per);
+  if (mp)
+    for (int i = 0; i < ti; ++i) later += cnts[i];
   const float n_end = (float)count[b];
   const float n_in = n_end - later;   // count after this run's last step (its own steps are counted apart: see the forward)
   auto prev_u = [&](int t) -> float { return t > 0 ? __ldg(cummean + base + (size_t)(t - 1) * G) : prev_mean[(size_t)b * G + g]; };
