@@ -3,12 +3,14 @@
 // With chunks of 16 positions, h the poles' states and everything below a matrix of the channel,
 //   states   h' = q^16 h + V x         V (16 x poles): q^(15-k)
 //   outputs  y  = T x + G h            T (16 x 16): the taps, omega on its diagonal; G (poles x 16): c q^(j+1)
-// and for the backward, l = sum_j q^j dy_j and w = sum_j j q^(j-1) dy_j of a chunk (V and its derivative U against dy in
-// reversed order), s = dh/dq (s' = q^16 s + 16 q^15 h + U x) and R_k the correlation of x and dy at lag k within chunks,
-//   sum_t dy_t h_t = q A1 + sum_k q^k R_k,          A1 = sum over chunks of l h
-//   sum_t dy_t s_t = q A2 + A1 + sum_k k q^(k-1) R_k,   A2 = sum over chunks of l s + w h,
-// while dx is the layer itself run over dy in reversed time.  So nothing is computed per position and pole: 16 + 16 + 16
-// multiply-adds per element forward (real), 64 + 16 backward beside them, all on the tensor pipe.
+// Backward: dx is the layer itself run over dy in reversed time, its states h the adjoint.  Of the parameters' gradients the sums
+// over time sum_t dy_t (state of x)_t are, by adjointness, sum_t x_t h_t, and the same with the derivative s = dh/dq in h's place
+// (s' = q^16 s + 16 q^15 h + U dy, U the derivative of V).  With l = sum_j q^j x_j and w = sum_j j q^(j-1) x_j of a chunk (V and
+// U against x in the other order) and R_k the correlation of x and dy at lag k within chunks,
+//   sum_t x_t h_t = q A1 + sum_k q^k R_k,               A1 = sum over chunks of l h
+//   sum_t x_t s_t = q A2 + A1 + sum_k k q^(k-1) R_k,    A2 = sum over chunks of l s + w h.
+// So nothing is computed per position and pole: 16 + 16 + 16 multiply-adds per element forward (real), 48 + 16 more backward, all
+// on the tensor pipe.
 //
 // fp32 on the bf16 tensor pipe: matrices, states and fp32 inputs go in as three bf16 parts, of whose products all but
 // those below 2^-24 are taken (split_mma.cuh); a bf16 input is one part, an fp16 one two.
@@ -36,16 +38,19 @@ namespace mega {
 
 namespace {
 
-enum Mode { kLocal, kLocalSens, kEmit, kGrad };   // local states; with their derivatives; outputs; sums of the gradients
+// local states; with their derivatives; outputs; sums of the parameters' gradients; those and the outputs (the input's gradient)
+enum Mode { kLocal, kLocalSens, kEmit, kGrad, kBoth };
 
 struct ChunkArgs {
   ScanArgs a;
   const void* in;           // what is walked, and its strides
   long long isb, isl;
+  const void* beside;       // with the sums: what it is correlated with
+  long long bsb, bsl;
   int T, S;                 // steps of a segment (a multiple of 64), segments of a sequence
   int walked;               // of them, those that this launch takes
   int rev;                  // time runs backwards
-  int parts, part;          // values per (sequence, segment) in the carry array, first one of this launch
+  int parts;                // values per (sequence, segment) in the carry array
   float* carry;             // [B][S][parts][D][16]: what a segment starts from (of segment 0: unused)
   const unsigned char* frag;   // [D][blocks] of kBlockBytes
   int blocks;
@@ -65,16 +70,16 @@ template <typename In, typename Out, bool kC, int kMode, bool kMask>
 struct Form {
   static constexpr int kP = kPartsOf<In>;
   // positions of a tile (what shared memory holds), and bytes of a row: eight rows hit different banks
-  static constexpr int kTile = (kP == 1 && !(kMode == kGrad && kC)) || (kP == 2 && !kC && kMode != kGrad) ? 128 : 64;
+  static constexpr int kTile = (kP == 1 && kMode != kBoth && !(kMode == kGrad && kC)) || (kP == 2 && !kC && kMode < kGrad) ? 128 : 64;
   static constexpr int kRow = 2 * kTile + 16;
   static constexpr int kCh = kMode == kGrad && kP == 3 ? 8 : 16;   // channels of a block, and its warps
   static constexpr int kThreads = 32 * kCh;
-  static constexpr int kIns = kMode == kGrad ? 2 : 1;
+  static constexpr int kIns = kMode >= kGrad ? 2 : 1;
   static constexpr int kPlane = kCh * 8 * kRow;                    // bytes of one part of a tile
   static constexpr int kBufs = (kMode == kGrad && (kP == 3 || (kP == 2 && kC))) || (kMode == kLocalSens && kP == 3 && kC) ? 1 : 2;
   static constexpr int kV = Blocks<kC>::v;
-  static constexpr int kRegs = kMode == kEmit ? (kC ? Blocks<kC>::g : 2 * kV + 2) : kMode == kLocal ? kV : kC ? 0 : 2 * kV;
-  static constexpr int kAll = kMode == kEmit ? kV + Blocks<kC>::t + Blocks<kC>::g : kMode == kLocal ? kV : 2 * kV;
+  static constexpr int kRegs = kMode == kBoth ? 2 + Blocks<kC>::g : kMode == kEmit ? (kC ? Blocks<kC>::g : 2 * kV + 2) : kMode == kLocal ? kV : kC ? 0 : 2 * kV;
+  static constexpr int kAll = kMode == kBoth ? 2 * kV + 2 + Blocks<kC>::g : kMode == kEmit ? kV + 2 + Blocks<kC>::g : kMode == kLocal ? kV : 2 * kV;
   static constexpr int kShared = kAll - kRegs;                     // matrices in shared memory (the first ones)
   static constexpr int kE = 16 / (int)sizeof(In), kPos = kTile / (4 * kE);  // channels of a 16-byte piece; positions of a thread
   static constexpr int kSlot = kIns * kPos * kThreads * 16;        // bytes of a tile as it arrives
@@ -333,9 +338,11 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask>::kThreads, For
   using F = Form<In, Out, kC, kMode, kMask>;
   constexpr int kP = F::kP, kV = F::kV, kPlane = F::kPlane, kCh = F::kCh, kTile = F::kTile, kRow = F::kRow;
   constexpr int kRe = kC ? 2 : 1;      // real numbers of a value
-  constexpr bool kSens = kMode == kLocalSens || kMode == kGrad;
-  constexpr bool kWide = kMode == kEmit && sizeof(Out) == 4;   // leading products by themselves: the tensor pipe truncates its sums
-  constexpr bool kApart = kWide || (kMode == kEmit && kMask);   // omega x in fp32
+  constexpr bool kSums = kMode >= kGrad, kOuts = kMode == kEmit || kMode == kBoth;
+  constexpr bool kSens = kMode == kLocalSens || kSums;
+  constexpr int kTs = kMode == kBoth ? 2 * kV : kV;   // T's first block
+  constexpr bool kWide = kOuts && sizeof(Out) == 4;   // leading products by themselves: the tensor pipe truncates its sums
+  constexpr bool kApart = kWide || (kOuts && kMask);   // omega x in fp32
   extern __shared__ __align__(16) unsigned char smem[];
   const ScanArgs& a = s.a;
   int tid;
@@ -343,7 +350,7 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask>::kThreads, For
   const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int d = blockIdx.x * kCh + warp, dc = min(d, a.D - 1);
   Share<In, kCh, kTile> sh(s, tid, s.in, s.isb, s.isl, false);
-  Share<In, kCh, kTile> sg(s, tid, a.dy, a.gsb, a.gsl, true);
+  Share<In, kCh, kTile> sg(s, tid, s.beside, s.bsb, s.bsl, true);
   Share<Out, kCh, kTile> so(s, tid, a.y, a.ysb, a.ysl, false);
   // the row of this lane's states, and the longest one
   const int row = blockIdx.y * 8 + g, b = row / s.walked, seg = row - b * s.walked;
@@ -401,7 +408,7 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask>::kThreads, For
   const float om = kApart ? __ldg(a.omega + dc) : 0.f;
 
   // states that the segment starts from
-  auto carry_at = [&](int at, int part) { return s.carry + (((size_t)(b * s.S + at) * s.parts + s.part + part) * a.D + d) * 16 + 2 * t; };
+  auto carry_at = [&](int at, int part) { return s.carry + (((size_t)(b * s.S + at) * s.parts + part) * a.D + d) * 16 + 2 * t; };
   float h[kRe][4], sn[kSens ? kRe : 1][4];
 #pragma unroll
   for (int c = 0; c < kRe; ++c)
@@ -410,7 +417,7 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask>::kThreads, For
       h[c][i] = 0.f;
       if (kSens) sn[kSens ? c : 0][i] = 0.f;
     }
-  if ((kMode == kEmit || kMode == kGrad) && live) {
+  if ((kOuts || kSums) && live) {
     if (seg > 0) {
 #pragma unroll
       for (int c = 0; c < kRe; ++c)
@@ -447,11 +454,11 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask>::kThreads, For
       re = fmaf(qr[i], re, vr);
     }
   };
-  // kGrad: A1 and A2 of the lane's poles, R of its entries
-  float a1[kMode == kGrad ? kRe : 1][4] = {}, a2[kMode == kGrad ? kRe : 1][4] = {}, R[kMode == kGrad ? 8 : 1] = {};
+  // kSums: A1 and A2 of the lane's poles, R of its entries
+  float a1[kSums ? kRe : 1][4] = {}, a2[kSums ? kRe : 1][4] = {}, R[kSums ? 8 : 1] = {};
 
   float beside = 0.f;   // of omega, at padded positions
-  // columns 8 k .. of x and dy with the 16 chunks as the reduction (products of parts below 2^-24 are left out)
+  // columns 8 k .. of the products of two inputs with the 16 chunks as the reduction (parts' products below 2^-24 left out)
   auto correlate = [](float (&r)[4], const uint32_t (&x)[kP][4], const uint32_t (&y)[kP][4], int k) {
     bool onto = false;
 #pragma unroll
@@ -473,7 +480,7 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask>::kThreads, For
   const int final = kMode == kEmit && a.h_out != nullptr && live && seg == s.S - 1 ? (len - 1) / 32 : -1;   // step whose end leaves
 
   // kStep steps of 32 positions at a time: their products do not wait for each other, only their states do
-  constexpr int kStep = kC && (kMode == kGrad || kP == 3) ? 1 : 2;   // (what registers hold: a spill goes to L2 beside this much shared memory)
+  constexpr int kStep = kMode == kBoth || (kC && (kMode == kGrad || kP == 3)) ? 1 : 2;   // (what registers hold: a spill goes to L2 beside this much shared memory)
   auto multiply = [&](int tile) {
     const int buf = tile % F::kBufs * F::kIns * kP * kPlane;
     const int n = min(kTile / 32, steps - kTile / 32 * tile), last = final - kTile / 32 * tile;
@@ -502,7 +509,7 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask>::kThreads, For
         }
         some = __any_sync(0xffffffffu, some);
       }
-      if (kMask && some && !(kMode == kEmit && s.rev)) {
+      if (kMask && some && !kSums && !(kMode == kEmit && s.rev)) {
 #pragma unroll
         for (int st = 0; st < kStep; ++st)
 #pragma unroll
@@ -512,6 +519,120 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask>::kThreads, For
             for (int p = 0; p < kP; ++p) f[st][p][i] &= m;
           }
       }
+      // outputs of a step, from the states that enter its chunks
+      auto emit = [&](int st, const float (&enter)[2][kRe][4], bool any_odd) {
+        // entering states: the A operand of G as they stand
+        uint32_t hp[kRe][3][4];
+#pragma unroll
+        for (int c = 0; c < kRe; ++c)
+#pragma unroll
+          for (int k = 0; k < 2; ++k)
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+              split(enter[k][c][2 * r], enter[k][c][2 * r + 1], hp[c][0][2 * k + r], hp[c][1][2 * k + r], hp[c][2][2 * k + r]);
+        // T's zeros would carry a NaN or an infinity to the positions before it: such a chunk takes its outputs from the finite
+        // values ahead of the first one, and is NaN from there on (as are all later states)
+        int bad[2];
+        if (any_odd) {
+          bad[0] = bad[1] = 16;
+#pragma unroll
+          for (int i = 3; i >= 0; --i) {   // (rows g, g + 8, then their upper halves)
+#pragma unroll
+            for (int e = 1; e >= 0; --e)
+              if (((f[st][0][i] >> (16 * e)) & 0x7f80u) == 0x7f80u) bad[i & 1] = 8 * (i >> 1) + 2 * t + e;
+          }
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+#pragma unroll
+            for (int m = 1; m < 4; m <<= 1) bad[r] = min(bad[r], __shfl_xor_sync(0xffffffffu, bad[r], m));
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int pos = 8 * (i >> 1) + 2 * t, from = i & 1 ? bad[1] : bad[0];
+            const uint32_t keep = pos + 1 < from ? ~0u : pos < from ? 0xffffu : 0u;
+#pragma unroll
+            for (int p = 0; p < kP; ++p) f[st][p][i] &= keep;
+          }
+        }
+        float y[2][4];
+#pragma unroll
+        for (int j = 0; j < kTerms<kP> - 1; ++j)
+#pragma unroll
+          for (int k = 0; k < 2; ++k) term<kP>(j, j > 0, y[k], f[st], matrix(kTs + k));
+#pragma unroll
+        for (int j = 0; j < kTerms<3> - 1; ++j)
+#pragma unroll
+          for (int c = 0; c < kRe; ++c)
+#pragma unroll
+            for (int k = 0; k < 2; ++k) term<3>(j, true, y[k], hp[c], matrix(kTs + 2 + 2 * c + k));
+#pragma unroll
+        for (int c = 0; c <= kRe; ++c)
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const Frag m = matrix(c < kRe ? kTs + 2 + 2 * c + k : kTs + k);
+            const uint32_t(&p)[4] = c < kRe ? hp[c < kRe ? c : 0][0] : f[st][0];
+            if (kWide) {   // (by themselves, so that what truncates is small)
+              float l[4];
+              mma0(l, p, m.u.x, m.u.y);
+#pragma unroll
+              for (int i = 0; i < 4; ++i) y[k][i] += l[i];
+            } else {
+              mma(y[k], p, m.u.x, m.u.y);
+            }
+          }
+        if (kApart) {
+          uint32_t own_x[kMask ? kP : 1][4];   // as they came
+          if constexpr (kMask) {
+#pragma unroll
+            for (int p = 0; p < kP; ++p) ldmatrix(own_x[p], rows(st) + p * kPlane);
+          }
+#pragma unroll
+          for (int k = 0; k < 2; ++k)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+              float x0 = 0.f, x1 = 0.f;
+#pragma unroll
+              for (int p = kP - 1; p >= 0; --p) {
+                const uint32_t w = kMask ? own_x[kMask ? p : 0][2 * k + r] : f[st][p][2 * k + r];
+                x0 += __uint_as_float(w << 16);
+                x1 += __uint_as_float(w & 0xffff0000u);
+              }
+              if (kMask && some && s.rev) {
+                const uint32_t m = keep(padded[st], 2 * k + r);
+                if (!(m & 0xffffu)) y[k][2 * r] = 0.f;
+                if (!(m & 0xffff0000u)) y[k][2 * r + 1] = 0.f;
+              }
+              y[k][2 * r] = fmaf(om, x0, y[k][2 * r]);
+              y[k][2 * r + 1] = fmaf(om, x1, y[k][2 * r + 1]);
+            }
+        }
+        if (a.silu) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) y[i >> 2][i & 3] = silu_of<Out>(y[i >> 2][i & 3]);
+        }
+        if (any_odd) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            if (8 * (i >> 2) + 2 * t + (i & 1) >= bad[(i >> 1) & 1] &&
+                !(kMask && s.rev && !(keep(padded[st], 2 * (i >> 2) + ((i >> 1) & 1)) >> (16 * (i & 1)) & 1u)))
+              y[i >> 2][i & 3] = __int_as_float(0x7fffffff);
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const float y0 = y[k][2 * r], y1 = y[k][2 * r + 1];
+            unsigned char* to = mine + buf + ((first ^ (st << 6)) ^ (r << 5)) + 16 * k;
+            if constexpr (sizeof(Out) == 4) {
+              *reinterpret_cast<uint32_t*>(to) = prmt(__float_as_uint(y0), __float_as_uint(y1), 0x7632);
+              *reinterpret_cast<uint32_t*>(to + kPlane) = prmt(__float_as_uint(y0), __float_as_uint(y1), 0x5410);
+            } else if constexpr (std::is_same<Out, __half>::value) {
+              *reinterpret_cast<__half2*>(to) = __floats2half2_rn(y0, y1);
+            } else {
+              *reinterpret_cast<uint32_t*>(to) = bf16_pair(y0, y1);
+            }
+          }
+      };
       if constexpr (kMode == kLocal || kMode == kLocalSens) {
 #pragma unroll
         for (int k = 0; k < 2; ++k) {   // eight poles at a time
@@ -590,119 +711,7 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask>::kThreads, For
         __syncwarp();
         const bool any_odd = __any_sync(0xffffffffu, odd != odd);
 #pragma unroll
-        for (int st = 0; st < kStep; ++st) {
-          // entering states: the A operand of G as they stand
-          uint32_t hp[kRe][3][4];
-#pragma unroll
-          for (int c = 0; c < kRe; ++c)
-#pragma unroll
-            for (int k = 0; k < 2; ++k)
-#pragma unroll
-              for (int r = 0; r < 2; ++r)
-                split(v[st][k][c][2 * r], v[st][k][c][2 * r + 1], hp[c][0][2 * k + r], hp[c][1][2 * k + r], hp[c][2][2 * k + r]);
-          // T's zeros would carry a NaN or an infinity to the positions before it: such a chunk takes its outputs from the finite
-          // values ahead of the first one, and is NaN from there on (as are all later states)
-          int bad[2];
-          if (any_odd) {
-            bad[0] = bad[1] = 16;
-#pragma unroll
-            for (int i = 3; i >= 0; --i) {   // (rows g, g + 8, then their upper halves)
-#pragma unroll
-              for (int e = 1; e >= 0; --e)
-                if (((f[st][0][i] >> (16 * e)) & 0x7f80u) == 0x7f80u) bad[i & 1] = 8 * (i >> 1) + 2 * t + e;
-            }
-#pragma unroll
-            for (int r = 0; r < 2; ++r) {
-#pragma unroll
-              for (int m = 1; m < 4; m <<= 1) bad[r] = min(bad[r], __shfl_xor_sync(0xffffffffu, bad[r], m));
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const int pos = 8 * (i >> 1) + 2 * t, from = i & 1 ? bad[1] : bad[0];
-              const uint32_t keep = pos + 1 < from ? ~0u : pos < from ? 0xffffu : 0u;
-#pragma unroll
-              for (int p = 0; p < kP; ++p) f[st][p][i] &= keep;
-            }
-          }
-          float y[2][4];
-#pragma unroll
-          for (int j = 0; j < kTerms<kP> - 1; ++j)
-#pragma unroll
-            for (int k = 0; k < 2; ++k) term<kP>(j, j > 0, y[k], f[st], matrix(kV + k));
-#pragma unroll
-          for (int j = 0; j < kTerms<3> - 1; ++j)
-#pragma unroll
-            for (int c = 0; c < kRe; ++c)
-#pragma unroll
-              for (int k = 0; k < 2; ++k) term<3>(j, true, y[k], hp[c], matrix(kV + 2 + 2 * c + k));
-#pragma unroll
-          for (int c = 0; c <= kRe; ++c)
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-              const Frag m = matrix(c < kRe ? kV + 2 + 2 * c + k : kV + k);
-              const uint32_t(&p)[4] = c < kRe ? hp[c < kRe ? c : 0][0] : f[st][0];
-              if (kWide) {   // (by themselves, so that what truncates is small)
-                float l[4];
-                mma0(l, p, m.u.x, m.u.y);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) y[k][i] += l[i];
-              } else {
-                mma(y[k], p, m.u.x, m.u.y);
-              }
-            }
-          if (kApart) {
-            uint32_t own_x[kMask ? kP : 1][4];   // as they came
-            if constexpr (kMask) {
-#pragma unroll
-              for (int p = 0; p < kP; ++p) ldmatrix(own_x[p], rows(st) + p * kPlane);
-            }
-#pragma unroll
-            for (int k = 0; k < 2; ++k)
-#pragma unroll
-              for (int r = 0; r < 2; ++r) {
-                float x0 = 0.f, x1 = 0.f;
-#pragma unroll
-                for (int p = kP - 1; p >= 0; --p) {
-                  const uint32_t w = kMask ? own_x[kMask ? p : 0][2 * k + r] : f[st][p][2 * k + r];
-                  x0 += __uint_as_float(w << 16);
-                  x1 += __uint_as_float(w & 0xffff0000u);
-                }
-                if (kMask && some && s.rev) {
-                  const uint32_t m = keep(padded[st], 2 * k + r);
-                  if (!(m & 0xffffu)) y[k][2 * r] = 0.f;
-                  if (!(m & 0xffff0000u)) y[k][2 * r + 1] = 0.f;
-                }
-                y[k][2 * r] = fmaf(om, x0, y[k][2 * r]);
-                y[k][2 * r + 1] = fmaf(om, x1, y[k][2 * r + 1]);
-              }
-          }
-          if (a.silu) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) y[i >> 2][i & 3] = silu_of<Out>(y[i >> 2][i & 3]);
-          }
-          if (any_odd) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-              if (8 * (i >> 2) + 2 * t + (i & 1) >= bad[(i >> 1) & 1] &&
-                  !(kMask && s.rev && !(keep(padded[st], 2 * (i >> 2) + ((i >> 1) & 1)) >> (16 * (i & 1)) & 1u)))
-                y[i >> 2][i & 3] = __int_as_float(0x7fffffff);
-          }
-#pragma unroll
-          for (int k = 0; k < 2; ++k)
-#pragma unroll
-            for (int r = 0; r < 2; ++r) {
-              const float y0 = y[k][2 * r], y1 = y[k][2 * r + 1];
-              unsigned char* to = mine + buf + ((first ^ (st << 6)) ^ (r << 5)) + 16 * k;
-              if constexpr (sizeof(Out) == 4) {
-                *reinterpret_cast<uint32_t*>(to) = prmt(__float_as_uint(y0), __float_as_uint(y1), 0x7632);
-                *reinterpret_cast<uint32_t*>(to + kPlane) = prmt(__float_as_uint(y0), __float_as_uint(y1), 0x5410);
-              } else if constexpr (std::is_same<Out, __half>::value) {
-                *reinterpret_cast<__half2*>(to) = __floats2half2_rn(y0, y1);
-              } else {
-                *reinterpret_cast<uint32_t*>(to) = bf16_pair(y0, y1);
-              }
-            }
-        }
+        for (int st = 0; st < kStep; ++st) emit(st, v[st], any_odd);
         __syncwarp();
       } else {
         uint32_t e[kStep][kP][4];
@@ -710,6 +719,18 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask>::kThreads, For
         for (int st = 0; st < kStep; ++st)
 #pragma unroll
           for (int p = 0; p < kP; ++p) ldmatrix(e[st][p], rows(st) + (kP + p) * kPlane);
+        if (kMask && some) {   // (its blocks lie in reversed order)
+#pragma unroll
+          for (int st = 0; st < kStep; ++st)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const uint32_t two = padded[st] >> (16 * (i & 1) + 14 - 8 * (i >> 1) - 2 * t) & 3u;
+              const uint32_t m = (two & 2u ? 0u : 0xffffu) | (two & 1u ? 0u : 0xffff0000u);
+#pragma unroll
+              for (int p = 0; p < kP; ++p) e[st][p][i] &= m;
+            }
+        }
+        float enter[kMode == kBoth ? kStep : 1][2][kRe][4], odd = 0.f;
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
           float v[kStep][kRe][4], u[kStep][kRe][4], l[kStep][kRe][4], w[kStep][kRe][4];
@@ -729,10 +750,15 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask>::kThreads, For
 #pragma unroll
           for (int o = 0; o < 4 * kStep; ++o) {   // (in the order of time: steps, chunks, for two poles)
             const int st = o >> 2, m = o & 3, i = 2 * k + (o & 1);
+            if (kMode == kBoth) {
+              enter[kMode == kBoth ? st : 0][k][0][m] = h[0][i];
+              if (kC) enter[kMode == kBoth ? st : 0][k][kRe - 1][m] = h[kRe - 1][i];
+              if (k == 0 && !(o & 1)) odd = fmaf(v[st][0][m], 0.f, odd);
+            }
             float &hr = h[0][i], &hi = h[kRe - 1][i], &sr = sn[0][i], &si = sn[kSens ? kRe - 1 : 0][i];
             const float lr = l[st][0][m], li = l[st][kRe - 1][m], wr = w[st][0][m], wi = w[st][kRe - 1][m];
             float xr = u[st][0][m], xi = u[st][kRe - 1][m];
-            constexpr int im = kMode == kGrad ? kRe - 1 : 0;
+            constexpr int im = kSums ? kRe - 1 : 0;
             if (kC) {
               a1[0][i] = fmaf(lr, hr, fmaf(-li, hi, a1[0][i]));
               a1[im][i] = fmaf(lr, hi, fmaf(li, hr, a1[im][i]));
@@ -749,33 +775,34 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask>::kThreads, For
             next(i, hr, hi, v[st][0][m], v[st][kRe - 1][m]);
           }
         }
-        // x and dy with the 16 chunks as the reduction: entry (i, j) is the sum of x_i dy_(15 - j)
+        // both with the 16 chunks as the reduction: entry (i, j) is the sum of the products of positions i and 15 - j
 #pragma unroll
         for (int st = 0; st < kStep; ++st) {
+          uint32_t ft[kP][4];
 #pragma unroll
           for (int p = 0; p < kP; ++p) {
             uint32_t m[4];
             ldmatrix_t(m, rows(st) + p * kPlane);
-            f[st][p][0] = m[0]; f[st][p][1] = m[2]; f[st][p][2] = m[1]; f[st][p][3] = m[3];
+            ft[p][0] = m[0]; ft[p][1] = m[2]; ft[p][2] = m[1]; ft[p][3] = m[3];
             ldmatrix_t(e[st][p], rows(st) + (kP + p) * kPlane);
           }
           if (kMask && some) {   // the padded positions' own products are omega's alone
             uint32_t only[kP][4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {   // (position g or g + 8 of the chunks of the segments 2t and 2t + 1)
-              const int at = 16 * (i >> 1) + g + 8 * (i & 1);
+            for (int i = 0; i < 4; ++i) {   // (a position of a chunk of the segments 2t and 2t + 1)
+              const int at = 16 * (i & 1) + 15 - g - 8 * (i >> 1);
               const uint32_t m = (bits[2 * t * (kTile / 32) + st] >> at & 1u ? 0u : 0xffffu) |
                                  (bits[(2 * t + 1) * (kTile / 32) + st] >> at & 1u ? 0u : 0xffff0000u);
 #pragma unroll
               for (int p = 0; p < kP; ++p) {
-                only[p][i] = f[st][p][i] & ~m;
-                f[st][p][i] &= m;
+                only[p][i] = e[st][p][i] & ~m;
+                e[st][p][i] &= m;
               }
             }
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
               float r[4];
-              correlate(r, only, e[st], k);
+              correlate(r, ft, only, k);
 #pragma unroll
               for (int i = 0; i < 4; ++i)
                 if (8 * k + 2 * t + (i & 1) == 15 - g - 8 * (i >> 1)) beside += r[i];
@@ -784,10 +811,17 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask>::kThreads, For
 #pragma unroll
           for (int k = 0; k < 2; ++k) {
             float r[4];
-            correlate(r, f[st], e[st], k);
+            correlate(r, ft, e[st], k);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) R[(kMode == kGrad ? 4 * k + i : 0)] += r[i];   // (in fp32: the tensor pipe truncates its sums)
+            for (int i = 0; i < 4; ++i) R[(kSums ? 4 * k + i : 0)] += r[i];   // (in fp32: the tensor pipe truncates its sums)
           }
+        }
+        if constexpr (kMode == kBoth) {
+          __syncwarp();
+          const bool any_odd = __any_sync(0xffffffffu, odd != odd);
+#pragma unroll
+          for (int st = 0; st < kStep; ++st) emit(st, enter[st], any_odd);
+          __syncwarp();
         }
       }
     }
@@ -826,11 +860,11 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask>::kThreads, For
     issue(tile + F::kSlots);
   };
   auto leave = [&](int tile) {
-    if constexpr (kMode == kEmit)
+    if constexpr (kOuts)
       if (tile >= 0) put<Out, kCh, kTile, kPlane>(so, smem + tile % F::kBufs * F::kIns * kP * kPlane);
   };
   // (a thread takes outputs from where it puts inputs, unless their types differ in size)
-  constexpr bool kSame = kMode != kEmit || sizeof(In) == sizeof(Out);
+  constexpr bool kSame = !kOuts || sizeof(In) == sizeof(Out);
   if constexpr (F::kBufs == 2) {
     arrive(0);
     __syncthreads();
@@ -877,7 +911,7 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask>::kThreads, For
         }
     }
   }
-  if constexpr (kMode == kGrad) {   // sums over the rows, then the channel's gradients, a lane per pole
+  if constexpr (kSums) {   // sums over the rows, then the channel's gradients, a lane per pole
     __syncthreads();   // (the buffers are free)
     float* red = reinterpret_cast<float*>(smem) + warp * (16 * 17 + 4 * 16);
     float* sums = red + 16 * 17;   // [a1, a2][re, im][16]
@@ -897,7 +931,7 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask>::kThreads, For
       }
 #pragma unroll
     for (int i = 0; i < 8; ++i)
-      red[(g + 8 * ((i >> 1) & 1)) * 17 + 8 * (i >> 2) + 2 * t + (i & 1)] = R[(kMode == kGrad ? i : 0)];
+      red[(g + 8 * ((i >> 1) & 1)) * 17 + 8 * (i >> 2) + 2 * t + (i & 1)] = R[(kSums ? i : 0)];
     __syncwarp();
     float lag = 0.f;
     if (lane < 16)
@@ -944,7 +978,7 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask>::kThreads, For
 
 // ---- the carry ---------------------------------------------------------------------------------------------
 // A thread per (sequence, channel, pole): what every segment starts from, in the place of what the segment before it adds.
-// blockIdx.z 0: h (and its derivative with kSens); 1: the adjoint.
+// kSens: its derivative too.
 template <bool kC, bool kSens>
 __global__ void __launch_bounds__(128) chunk_carry_kernel(ChunkArgs s) {
   const ScanArgs& a = s.a;
@@ -952,7 +986,7 @@ __global__ void __launch_bounds__(128) chunk_carry_kernel(ChunkArgs s) {
   const int i = blockIdx.x * 128 + threadIdx.x, b = blockIdx.y;   // channel and pole
   if (i >= a.D * 16) return;
   const int d = i >> 4, n = i & 15;
-  const bool adjoint = kSens && blockIdx.z == 1, in = n < a.N;
+  const bool in = n < a.N;
   const size_t at = (size_t)d * a.N + n;
   const double qr = in ? (double)a.q[kRe * at] : 0., qi = in && kC ? (double)a.q[kRe * at + 1] : 0.;
   double ur = 1., ui = 0.;   // q^(T-1)
@@ -970,7 +1004,7 @@ __global__ void __launch_bounds__(128) chunk_carry_kernel(ChunkArgs s) {
   const double wr = ur * qr - ui * qi, wi = ur * qi + ui * qr;
   const float fr = (float)wr, fi = (float)wi, gr = (float)(s.T * ur), gi = (float)(s.T * ui);
   const size_t val = (size_t)a.D * 16, step = val * s.parts;
-  float* v = s.carry + ((size_t)b * s.S + 1) * step + (size_t)(adjoint ? 2 * kRe : 0) * val + i;
+  float* v = s.carry + ((size_t)b * s.S + 1) * step + i;
   float hr = 0.f, hi = 0.f, sr = 0.f, si = 0.f;
   if (!kSens && a.h_in && in) {
     const size_t o = ((size_t)b * a.D + d) * a.N + n;
@@ -985,7 +1019,7 @@ __global__ void __launch_bounds__(128) chunk_carry_kernel(ChunkArgs s) {
       const float* p = v + (size_t)min(u, s.S - 1 - k0) * step;
       lr[u] = __ldcg(p);
       if (kC) li[u] = __ldcg(p + val);
-      if (kSens && !adjoint) {
+      if (kSens) {
         mr[u] = __ldcg(p + kRe * val);
         if (kC) mi[u] = __ldcg(p + (kRe + 1) * val);
       }
@@ -994,7 +1028,7 @@ __global__ void __launch_bounds__(128) chunk_carry_kernel(ChunkArgs s) {
     for (int u = 0; u < kB; ++u) {
       if (k0 + u >= s.S) break;
       float* p = v + (size_t)u * step;
-      if (kSens && !adjoint) {
+      if (kSens) {
         float x = fmaf(gr, hr, mr[u]), y = 0.f;
         if (kC) {
           x = fmaf(-gi, hi, x);
@@ -1054,14 +1088,14 @@ bool envelope(int dtype, const ScanArgs& a) {
 // a fifth.  Here: a part for the launches and the blocks' start, and ns per unit of pick()'s cost by the number of parts of a
 // value and the kind of poles.
 double chunk_us(int dtype, const ScanArgs& a, bool bwd, double cost, bool segmented) {
-  static const double kFwd[2][3] = {{25., 32., 43.}, {44., 54., 64.}}, kBwd[2][3] = {{55., 82., 109.}, {105., 155., 185.}};
+  static const double kFwd[2][3] = {{25., 32., 43.}, {44., 54., 64.}}, kBwd[2][3] = {{48., 75., 102.}, {97., 140., 168.}};
   const int parts = dtype == MEGA_BF16 ? 0 : dtype == MEGA_F16 ? 1 : 2;
-  return (bwd ? (segmented ? 38. : 24.) : (segmented ? 22. : 14.)) +
+  return (bwd ? (segmented ? 32. : 20.) : (segmented ? 22. : 14.)) +
          (bwd ? kBwd : kFwd)[a.cplx ? 1 : 0][parts] * 1e-3 * cost * (segmented ? 1. : a.cplx ? 1.14 : 1.07) *
              (a.mask ? (bwd ? 1.22 : 1.33) : 1.);
 }
-// The form that a call takes otherwise: the scan backward (real bf16 16 x 4096 x 1024: 517 us against 241 here, complex 1481
-// against 459, fp32 539 against 500); forward the cluster kernel, the scan (fp32 complex of that size: 565 against 385; real fp32
+// The form that a call takes otherwise: the scan backward (real bf16 16 x 4096 x 1024: 517 us against 233 here, complex 1481
+// against 459, fp32 539 against 505); forward the cluster kernel, the scan (fp32 complex of that size: 565 against 385; real fp32
 // of 4 sequences 86 against 90), or in bf16 the tensor-core kernel, which walks a sequence as one chain (complex 4 x 4096 x
 // 1024: 219 against 93; real 16 x 4096 x 1024: 100 against 121, 1 x 6606 x 1680: 145 against 56).
 double other_us(int dtype, const ScanArgs& a, bool bwd) {
@@ -1122,7 +1156,7 @@ bool bwd(int dtype, const ScanArgs& a, cudaStream_t st) {
   if ((long long)a.B * s.S > 8LL * 65535 || !pays(dtype, a, true, cost, s.S > 1)) return false;
   constexpr int kRe = kC ? 2 : 1, kBlocks = 3 * Blocks<kC>::v + 2;
   s.blocks = kBlocks;
-  s.parts = 3 * kRe;
+  s.parts = 2 * kRe;
   const size_t frag = (size_t)a.D * kBlocks * kBlockBytes, carry = s.S > 1 ? (size_t)a.B * s.S * s.parts * a.D * 16 : 0;
   Scratch sc(Scratch::padded(frag) + Scratch::padded((size_t)a.D * 256) + Scratch::padded(carry * 4), st);
   if (!sc) return false;
@@ -1133,24 +1167,27 @@ bool bwd(int dtype, const ScanArgs& a, cudaStream_t st) {
   s.carry = carry ? sc.take<float>(carry) : nullptr;
   const PrepArgs p{a.p, a.q, a.g, a.omega, a.D, a.N, 1, 1, 0, sizeof(T) == 4 || kMask ? 0 : 1, kBlocks, fr, pow};
   launch(chunk_prepare_kernel<kC>, (unsigned)((a.D + 3) / 4), 128, 0, (void*)st, p);
-  ChunkArgs x = s, g = s;   // forward over x; backward over dy
-  x.in = a.x;
-  x.isb = a.xsb;
-  x.isl = a.xsl;
-  g.in = a.dy;
-  g.isb = a.gsb;
-  g.isl = a.gsl;
-  g.rev = 1;
-  g.part = 2 * kRe;
+  s.in = a.dy;   // (walked backwards: its states are the adjoint)
+  s.isb = a.gsb;
+  s.isl = a.gsl;
+  s.beside = a.x;
+  s.bsb = a.xsb;
+  s.bsl = a.xsl;
+  s.rev = 1;
   if (s.S > 1) {
-    x.walked = g.walked = s.S - 1;
-    run<T, T, kC, kLocalSens, kMask>(x, st);
-    run<T, T, kC, kLocal, false>(g, st);
-    launch(chunk_carry_kernel<kC, true>, dim3((a.D * 16 + 127) / 128, a.B, 2), 128, 0, (void*)st, s);
+    s.walked = s.S - 1;
+    run<T, T, kC, kLocalSens, false>(s, st);
+    launch(chunk_carry_kernel<kC, true>, dim3((a.D * 16 + 127) / 128, a.B), 128, 0, (void*)st, s);
   }
-  x.walked = g.walked = s.S;
-  run<T, T, kC, kGrad, kMask>(x, st);
-  run<T, T, kC, kEmit, kMask>(g, st);
+  s.walked = s.S;
+  // (real bf16: one launch reads dy once for both, 16 x 4096 x 1024 241 -> 233 us, 4 x 4096 x 1024 131 -> 109 with the local states
+  // of dy alone)
+  if constexpr (kPartsOf<T> == 1 && !kC) {
+    run<T, T, kC, kBoth, kMask>(s, st);
+  } else {   // (more parts or poles than registers and shared memory hold at once)
+    run<T, T, kC, kGrad, kMask>(s, st);
+    run<T, T, kC, kEmit, kMask>(s, st);
+  }
   g_last_kernel.store("chunk_ema", std::memory_order_relaxed);
   return true;
 }
