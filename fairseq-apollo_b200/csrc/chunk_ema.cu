@@ -1092,7 +1092,7 @@ double chunk_us(int dtype, const ScanArgs& a, bool bwd, double cost, bool segmen
   const int parts = dtype == MEGA_BF16 ? 0 : dtype == MEGA_F16 ? 1 : 2;
   return (bwd ? (segmented ? 32. : 20.) : (segmented ? 22. : 14.)) +
          (bwd ? kBwd : kFwd)[a.cplx ? 1 : 0][parts] * 1e-3 * cost * (segmented ? 1. : a.cplx ? 1.14 : 1.07) *
-             (a.mask ? (bwd ? 1.22 : 1.33) : 1.);
+             (a.mask ? (bwd ? 1.22 : a.cplx ? 1.22 : 1.36) : 1.);
 }
 // The form that a call takes otherwise: the scan backward (real bf16 16 x 4096 x 1024: 517 us against 233 here, complex 1481
 // against 459, fp32 539 against 505); forward the cluster kernel, the scan (fp32 complex of that size: 565 against 385; real fp32

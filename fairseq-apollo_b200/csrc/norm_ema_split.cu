@@ -5,6 +5,8 @@
 // normalise their inputs as they read them, and, for bf16, TimestepNorm by itself (scan_norm.cu) followed by the
 // tensor-core kernel alone, which runs in half the time of the fused one; the normalised activations then go to their
 // own output, or through y in place.
+#include <cmath>
+
 #include "chunk_ema.cuh"
 #include "common.cuh"
 #include "norm_ema_split.cuh"
@@ -43,11 +45,15 @@ double fused_us(int dtype, const StreamArgs& a, bool want_xn) {
     const double near = fixed + longer(chain, rate, L, n);
     return near > far ? near : far;
   }
-  // (the streamed chain: 171 to 260 ns a position complex, 150 to 200 real, more where the channels do not fit the SMs at once;
-  // with a second output a third of the rate: 57 x 995 x 632 fp32 163 us and 489)
-  const bool slow = want_xn || a.h_in || a.h_out;
-  return a.cplx ? (slow ? 25.0 + longer(234.0, 75e3, L, n) : 8.0 + longer(171.0, 130e3, L, n))
-                : slow ? 10.0 + longer(185.0, 100e3, L, n) : 6.0 + longer(145.0, 230e3, L, n);
+  // The streamed chain: ns a position by the blocks (128 channels of a sequence) that share an SM.  With a second output 16 x 4096 x
+  // 1024 fp32 755 us, 31 x 2094 x 624 673, 58 x 530 x 960 fp16 163; without 58 x 530 x 960 114, 27 x 1781 x 1296 with a state 309.
+  const double per = ceil((double)a.B * ((a.D + 127) / 128) / 148.0), wide = dtype == MEGA_F32 ? 1.35 : 1.0;
+  const bool state = a.h_in || a.h_out;
+  double ns;
+  if (a.cplx) ns = want_xn ? (per < 2 ? (state ? 254.0 : 234.0) : per < 3 ? 440.0 : 123.0 * per * wide)
+                           : (per < 2 ? (state ? 254.0 : 171.0) : per < 3 ? 250.0 : 92.0 * per * wide);
+  else ns = want_xn ? (per < 2 ? 185.0 : per < 3 ? 335.0 : 100.0 * per * wide) : per < 3 ? 148.0 : 54.0 * per * wide;
+  return 8.0 + L * ns * 1e-3;
 }
 
 // TimestepNorm, then the tensor-core kernel alone: where the fused call would run on it too (both round the normalised
@@ -73,7 +79,7 @@ double chunk_us(int dtype, const ScanArgs& ea) {
   a.mask = nullptr;
   const double n = (double)a.B * a.D * a.L;
   if (dtype != MEGA_F32 && n > kWideMost) return 1e30;
-  return 18.0 + n / (dtype == MEGA_F32 ? 480e3 : 540e3) + chunk_ema_fwd_us(MEGA_F32, a);
+  return 28.0 + n / (dtype == MEGA_F32 ? 480e3 : 540e3) + chunk_ema_fwd_us(MEGA_F32, a);
 }
 bool norm_chunk_try(int dtype, const ScanArgs& ea, long long xsd, long long ysd, cudaStream_t s) {
   if (!rows_ok(dtype, ea.y, ea.ysb, ea.ysl, ysd) || (ea.xn && !rows_ok(dtype, ea.xn, ea.ysb, ea.ysl, ysd))) return false;
