@@ -22,6 +22,10 @@
 // its products are two consecutive chunks of the eight segments, so that states stay in a thread; matrices live in registers
 // (complex: some in shared memory) for the whole segment.  Two buffers let half of the warps turn tiles while the others
 // multiply.
+//
+// bf16 calls that would otherwise go to the tensor-core kernel take the leading parts alone, as that one does (lean_call).
+// What bounds it: the tensor pipe is busy 45 % of the time, the rest is issue slots and the latency of a turn at 16 warps per
+// SM; DRAM stays below a third of its rate.
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
@@ -66,7 +70,7 @@ struct Blocks {
   static constexpr int v = kC ? 4 : 2, t = 2, g = kC ? 4 : 2;
 };
 
-template <typename In, typename Out, bool kC, int kMode, bool kMask>
+template <typename In, typename Out, bool kC, int kMode, bool kMask, bool kLean = false>
 struct Form {
   static constexpr int kP = kPartsOf<In>;
   // positions of a tile (what shared memory holds), and bytes of a row: eight rows hit different banks
@@ -78,7 +82,7 @@ struct Form {
   static constexpr int kPlane = kCh * 8 * kRow;                    // bytes of one part of a tile
   static constexpr int kBufs = (kMode == kGrad && (kP == 3 || (kP == 2 && kC))) || (kMode == kLocalSens && kP == 3 && kC) ? 1 : 2;
   static constexpr int kV = Blocks<kC>::v;
-  static constexpr int kRegs = kMode == kBoth ? 2 + Blocks<kC>::g : kMode == kEmit ? (kC ? Blocks<kC>::g : 2 * kV + 2) : kMode == kLocal ? kV : kC ? 0 : 2 * kV;
+  static constexpr int kRegs = kLean ? (kMode == kEmit ? kV + 2 + Blocks<kC>::g : kV) : kMode == kBoth ? 2 + Blocks<kC>::g : kMode == kEmit ? (kC ? Blocks<kC>::g : 2 * kV + 2) : kMode == kLocal ? kV : kC ? 0 : 2 * kV;
   static constexpr int kAll = kMode == kBoth ? 2 * kV + 2 + Blocks<kC>::g : kMode == kEmit ? kV + 2 + Blocks<kC>::g : kMode == kLocal ? kV : 2 * kV;
   static constexpr int kShared = kAll - kRegs;                     // matrices in shared memory (the first ones)
   static constexpr int kE = 16 / (int)sizeof(In), kPos = kTile / (4 * kE);  // channels of a 16-byte piece; positions of a thread
@@ -332,10 +336,12 @@ __global__ void __launch_bounds__(128) chunk_prepare_kernel(PrepArgs a) {
 // ---- the walk ----------------------------------------------------------------------------------------------
 // kMask: padded positions are zero to the states (and to the correlations), omega x takes them as they are; in reversed time,
 // where outputs are the input's gradient, it is the outputs at padded positions that are omega dy alone.
-template <typename In, typename Out, bool kC, int kMode, bool kMask>
-__global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask>::kThreads, Form<In, Out, kC, kMode, kMask>::kPerSm)
+// kLean: leading parts alone (bf16 forward: what the tensor-core kernel that walks a sequence as one chain takes too).
+template <typename In, typename Out, bool kC, int kMode, bool kMask, bool kLean>
+__global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask, kLean>::kThreads, Form<In, Out, kC, kMode, kMask, kLean>::kPerSm)
     chunk_kernel(ChunkArgs s) {
-  using F = Form<In, Out, kC, kMode, kMask>;
+  using F = Form<In, Out, kC, kMode, kMask, kLean>;
+  constexpr int kFrom = kLean ? kTerms<kPartsOf<In>> - 1 : 0, kFromH = kLean ? kTerms<3> - 1 : 0;   // first products taken
   constexpr int kP = F::kP, kV = F::kV, kPlane = F::kPlane, kCh = F::kCh, kTile = F::kTile, kRow = F::kRow;
   constexpr int kRe = kC ? 2 : 1;      // real numbers of a value
   constexpr bool kSums = kMode >= kGrad, kOuts = kMode == kEmit || kMode == kBoth;
@@ -529,7 +535,8 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask>::kThreads, For
           for (int k = 0; k < 2; ++k)
 #pragma unroll
             for (int r = 0; r < 2; ++r)
-              split(enter[k][c][2 * r], enter[k][c][2 * r + 1], hp[c][0][2 * k + r], hp[c][1][2 * k + r], hp[c][2][2 * k + r]);
+              if (kLean) hp[c][0][2 * k + r] = bf16_pair(enter[k][c][2 * r], enter[k][c][2 * r + 1]);
+              else split(enter[k][c][2 * r], enter[k][c][2 * r + 1], hp[c][0][2 * k + r], hp[c][1][2 * k + r], hp[c][2][2 * k + r]);
         // T's zeros would carry a NaN or an infinity to the positions before it: such a chunk takes its outputs from the finite
         // values ahead of the first one, and is NaN from there on (as are all later states)
         int bad[2];
@@ -556,11 +563,11 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask>::kThreads, For
         }
         float y[2][4];
 #pragma unroll
-        for (int j = 0; j < kTerms<kP> - 1; ++j)
+        for (int j = kFrom; j < kTerms<kP> - 1; ++j)
 #pragma unroll
-          for (int k = 0; k < 2; ++k) term<kP>(j, j > 0, y[k], f[st], matrix(kTs + k));
+          for (int k = 0; k < 2; ++k) term<kP>(j, j > kFrom, y[k], f[st], matrix(kTs + k));
 #pragma unroll
-        for (int j = 0; j < kTerms<3> - 1; ++j)
+        for (int j = kFromH; j < kTerms<3> - 1; ++j)
 #pragma unroll
           for (int c = 0; c < kRe; ++c)
 #pragma unroll
@@ -576,6 +583,8 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask>::kThreads, For
               mma0(l, p, m.u.x, m.u.y);
 #pragma unroll
               for (int i = 0; i < 4; ++i) y[k][i] += l[i];
+            } else if (kLean && c == 0) {
+              mma0(y[k], p, m.u.x, m.u.y);
             } else {
               mma(y[k], p, m.u.x, m.u.y);
             }
@@ -638,12 +647,12 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask>::kThreads, For
         for (int k = 0; k < 2; ++k) {   // eight poles at a time
           float v[kStep][kRe][4], u[kStep][kSens ? kRe : 1][4];
 #pragma unroll
-          for (int j = 0; j < kTerms<kP>; ++j)
+          for (int j = kFrom; j < kTerms<kP>; ++j)
 #pragma unroll
             for (int c = 0; c < kRe; ++c)
 #pragma unroll
               for (int st = 0; st < kStep; ++st) {
-                term<kP>(j, j > 0, v[st][c], f[st], matrix(2 * c + k));
+                term<kP>(j, j > kFrom, v[st][c], f[st], matrix(2 * c + k));
                 if (kSens) term<kP>(j, j > 0, u[st][kSens ? c : 0], f[st], matrix((kSens ? kV : 0) + 2 * c + k));
               }
 #pragma unroll
@@ -665,13 +674,13 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask>::kThreads, For
         float v[kStep][2][kRe][4];
         float odd = 0.f;   // NaN where a row holds an infinity or a NaN
 #pragma unroll
-        for (int j = 0; j < kTerms<kP>; ++j)
+        for (int j = kFrom; j < kTerms<kP>; ++j)
 #pragma unroll
           for (int k = 0; k < 2; ++k)
 #pragma unroll
             for (int c = 0; c < kRe; ++c)
 #pragma unroll
-              for (int st = 0; st < kStep; ++st) term<kP>(j, j > 0, v[st][k][c], f[st], matrix(2 * c + k));
+              for (int st = 0; st < kStep; ++st) term<kP>(j, j > kFrom, v[st][k][c], f[st], matrix(2 * c + k));
 #pragma unroll
         for (int st = 0; st < kStep; ++st) {
           odd = fmaf(v[st][0][0][0], 0.f, fmaf(v[st][0][0][2], 0.f, odd));
@@ -1050,11 +1059,11 @@ __global__ void __launch_bounds__(128) chunk_carry_kernel(ChunkArgs s) {
 }
 
 // ---- launches ----------------------------------------------------------------------------------------------
-template <typename In, typename Out, bool kC, int kMode, bool kMask>
+template <typename In, typename Out, bool kC, int kMode, bool kMask, bool kLean = false>
 void run(const ChunkArgs& s, cudaStream_t st) {
-  using F = Form<In, Out, kC, kMode, kMask>;
+  using F = Form<In, Out, kC, kMode, kMask, kLean>;
   const dim3 grid((s.a.D + F::kCh - 1) / F::kCh, (unsigned)(((long long)s.a.B * s.walked + 7) / 8));
-  launch(chunk_kernel<In, Out, kC, kMode, kMask>, grid, F::kThreads, F::total, (void*)st, s);
+  launch(chunk_kernel<In, Out, kC, kMode, kMask, kLean>, grid, F::kThreads, F::total, (void*)st, s);
 }
 
 // Steps of a segment: a multiple of 64 (two steps of the tensor products) that minimises rounds of blocks over the SMs x
@@ -1087,39 +1096,56 @@ bool envelope(int dtype, const ScanArgs& a) {
 // Times in us, fitted to a grid of 38 shapes on one B200 (1 to 64 sequences, 209 to 32768 positions, 128 to 2048 channels), to
 // a fifth.  Here: a part for the launches and the blocks' start, and ns per unit of pick()'s cost by the number of parts of a
 // value and the kind of poles.
-double chunk_us(int dtype, const ScanArgs& a, bool bwd, double cost, bool segmented) {
+double chunk_us(int dtype, const ScanArgs& a, bool bwd, bool lean, double cost, bool segmented) {
   static const double kFwd[2][3] = {{25., 32., 43.}, {44., 54., 64.}}, kBwd[2][3] = {{48., 75., 102.}, {97., 140., 168.}};
-  const int parts = dtype == MEGA_BF16 ? 0 : dtype == MEGA_F16 ? 1 : 2;
+  static const double kLeanFwd[2] = {17.5, 22.5};
+  const int parts = dtype == MEGA_BF16 ? 0 : dtype == MEGA_F16 ? 1 : 2, c = a.cplx ? 1 : 0;
   return (bwd ? (segmented ? 32. : 20.) : (segmented ? 22. : 14.)) +
-         (bwd ? kBwd : kFwd)[a.cplx ? 1 : 0][parts] * 1e-3 * cost * (segmented ? 1. : a.cplx ? 1.14 : 1.07) *
+         (lean ? kLeanFwd[c] : bwd ? kBwd[c][parts] : kFwd[c][parts]) * 1e-3 * cost * (segmented ? 1. : a.cplx ? 1.14 : 1.07) *
              (a.mask ? (bwd ? 1.22 : a.cplx ? 1.22 : 1.36) : 1.);
+}
+// bf16 calls without states or mask that are too long for a cluster go to the tensor-core kernel, which takes leading parts alone
+// and walks a sequence as one chain: here they take leading parts alone too (lean), in a quarter of the products and the same
+// distance from float64 (2.8e-3 before the outputs are rounded): real 16 x 4096 x 1024 102 us as a chain, 90 here (123 in all
+// parts); 32 x 2048 x 1024 164 and 95; 8 x 8192 x 1024 186 and 137; complex 4 x 4096 x 1024 219 and 60.
+bool chain_takes(const ScanArgs& a) { return a.L < (1 << 24) && (!a.cplx || a.B >= 4); }   // (mma_cl_try)
+bool lean_call(int dtype, const ScanArgs& a) {
+  return dtype == MEGA_BF16 && !a.mask && !a.h_in && !a.h_out && g_options[OPT_DISABLE_MMA].load() == 0 &&
+         (g_options[OPT_CHUNK].load() == 3 || (g_options[OPT_CHUNK].load() == 0 && chain_takes(a) && !scan_cluster_first(dtype, a, 1, 1)));
+}
+double chain_us(const ScanArgs& a) {
+  const double L = a.L, n = (double)a.B * a.D * L, tiles = ((a.D + 15) / 16) * (double)((a.B + 7) / 8);
+  if (a.cplx) return 95. + std::max(L * 29e-3, n / 700e3);
+  if (a.mask) return 6. + std::max(L * 42e-3, n / 1300e3);
+  // (the pipelined form while each of its tiles has an SM; between that and the segmented form 80 - 170 ns a position)
+  const double ns = tiles > 148. && tiles <= 600. ? 0.28 * tiles : 22.;
+  return 6. + std::max(L * ns * 1e-3, n / 1300e3);
 }
 // The form that a call takes otherwise: the scan backward (real bf16 16 x 4096 x 1024: 517 us against 233 here, complex 1481
 // against 459, fp32 539 against 505); forward the cluster kernel, the scan (fp32 complex of that size: 565 against 385; real fp32
-// of 4 sequences 86 against 90), or in bf16 the tensor-core kernel, which walks a sequence as one chain (complex 4 x 4096 x
-// 1024: 219 against 93; real 16 x 4096 x 1024: 100 against 121, 1 x 6606 x 1680: 145 against 56).
+// of 4 sequences 86 against 90), or in bf16 the tensor-core kernel, which walks a sequence as one chain.
 double other_us(int dtype, const ScanArgs& a, bool bwd) {
   const double L = a.L, n = (double)a.B * a.D * L;
   if (bwd) return a.cplx ? 59. + n / 47e3 : 40. + n / 125e3;
-  if (dtype == MEGA_BF16 && g_options[OPT_DISABLE_MMA].load() == 0 && !(a.cplx && (a.mask || (a.h_out && a.L % 32 != 0))))
-    return scan_cluster_first(dtype, a, 1, 1) ? 0.9 * scan_cluster_us(dtype, a)
-                                              : a.cplx ? 95. + std::max(L * 29e-3, n / 700e3) : 6. + std::max(L * (a.mask ? 42e-3 : 22e-3), n / 1300e3);
+  if (dtype == MEGA_BF16 && g_options[OPT_DISABLE_MMA].load() == 0 && chain_takes(a) &&
+      !(a.cplx && (a.mask || (a.h_out && a.L % 32 != 0))))
+    return scan_cluster_first(dtype, a, 1, 1) ? 0.9 * scan_cluster_us(dtype, a) : chain_us(a);
   const double one = scan_cluster_us(dtype, a);
   return one < 1e29 ? 0.9 * one : std::min(scan_ema_fwd_us(a), a.cplx ? 25. + n / 123e3 : 15. + n / 270e3);
 }
-bool pays(int dtype, const ScanArgs& a, bool bwd, double cost, bool segmented) {
-  if (g_options[OPT_CHUNK].load() == 2) return true;
+bool pays(int dtype, const ScanArgs& a, bool bwd, bool lean, double cost, bool segmented) {
+  if (g_options[OPT_CHUNK].load() >= 2) return true;
   // (a prompt whose state leaves at a length that is no multiple of 32: the tensor-core kernel's head, then a tail)
   if (dtype == MEGA_BF16 && !a.cplx && a.h_out && a.L % 32 != 0) return false;
-  return g_options[OPT_MMA_TILE].load() == 0 && chunk_us(dtype, a, bwd, cost, segmented) < 0.93 * other_us(dtype, a, bwd);
+  return g_options[OPT_MMA_TILE].load() == 0 && chunk_us(dtype, a, bwd, lean, cost, segmented) < 0.93 * other_us(dtype, a, bwd);
 }
 
-template <typename In, typename Out, bool kC, bool kMask>
+template <typename In, typename Out, bool kC, bool kMask, bool kLean = false>
 bool fwd(int dtype, const ScanArgs& a, bool asked, cudaStream_t st) {
   ChunkArgs s{};
   s.a = a;
   const double cost = pick(a, s);
-  if ((long long)a.B * s.S > 8LL * 65535 || !(asked || pays(dtype, a, false, cost, s.S > 1))) return false;
+  if ((long long)a.B * s.S > 8LL * 65535 || !(asked || pays(dtype, a, false, kLean, cost, s.S > 1))) return false;
   const bool state = a.h_in || a.h_out;
   constexpr int kBlocks = 2 * Blocks<kC>::v + 2;
   s.blocks = kBlocks;
@@ -1139,11 +1165,11 @@ bool fwd(int dtype, const ScanArgs& a, bool asked, cudaStream_t st) {
   s.isl = a.xsl;
   if (s.S > 1) {
     s.walked = s.S - 1;
-    run<In, In, kC, kLocal, kMask>(s, st);
+    run<In, In, kC, kLocal, kMask, kLean>(s, st);
     launch(chunk_carry_kernel<kC, false>, dim3((a.D * 16 + 127) / 128, a.B), 128, 0, (void*)st, s);
   }
   s.walked = s.S;
-  run<In, Out, kC, kEmit, kMask>(s, st);
+  run<In, Out, kC, kEmit, kMask, kLean>(s, st);
   g_last_kernel.store("chunk_ema", std::memory_order_relaxed);
   return true;
 }
@@ -1153,7 +1179,7 @@ bool bwd(int dtype, const ScanArgs& a, cudaStream_t st) {
   ChunkArgs s{};
   s.a = a;
   const double cost = pick(a, s);
-  if ((long long)a.B * s.S > 8LL * 65535 || !pays(dtype, a, true, cost, s.S > 1)) return false;
+  if ((long long)a.B * s.S > 8LL * 65535 || !pays(dtype, a, true, false, cost, s.S > 1)) return false;
   constexpr int kRe = kC ? 2 : 1, kBlocks = 3 * Blocks<kC>::v + 2;
   s.blocks = kBlocks;
   s.parts = 2 * kRe;
@@ -1206,7 +1232,11 @@ bool chunk_ema_fwd_try(int dtype, int out_dtype, const ScanArgs& a, long long xs
   if (dtype != out_dtype) return false;
   switch (dtype) {
     case MEGA_F32: MEGA_FWD_SAME(float);
-    case MEGA_BF16: MEGA_FWD_SAME(__nv_bfloat16);
+    case MEGA_BF16:
+      if (lean_call(dtype, a))
+        return a.cplx ? fwd<__nv_bfloat16, __nv_bfloat16, true, false, true>(dtype, a, asked, s)
+                      : fwd<__nv_bfloat16, __nv_bfloat16, false, false, true>(dtype, a, asked, s);
+      MEGA_FWD_SAME(__nv_bfloat16);
     case MEGA_F16: MEGA_FWD_SAME(__half);
     default: return false;
   }
@@ -1218,7 +1248,7 @@ double chunk_ema_fwd_us(int dtype, const ScanArgs& a) {
   if (!envelope(dtype, a)) return 1e30;
   ChunkArgs s{};
   const double cost = pick(a, s);
-  return chunk_us(dtype, a, false, cost, s.S > 1);
+  return chunk_us(dtype, a, false, lean_call(dtype, a), cost, s.S > 1);
 }
 
 bool chunk_ema_bwd_try(int dtype, const ScanArgs& a, long long xsd, long long ysd, long long gsd, cudaStream_t s) {

@@ -435,7 +435,7 @@ extern "C" int mega_ema_fwd(const void* x, void* y, int dtype, int B, int D, int
   ca.bidir = bidir ? 1 : 0;
   ca.shift = (flags & MEGA_EMA_NO_SHIFT) ? 0 : 1;
   ca.silu = (flags & MEGA_EMA_SILU) ? 1 : 0;
-  if (chunk_ema_fwd_try(dtype, dtype, ca, xsd, ysd, (cudaStream_t)stream)) return check_launch("ema_fwd(chunk)");
+  if (x != y && chunk_ema_fwd_try(dtype, dtype, ca, xsd, ysd, (cudaStream_t)stream)) return check_launch("ema_fwd(chunk)");
   if (!bidir && x != y && !scan_cluster_first(dtype, ca, xsd, ysd)) {
     StreamArgs sa{};
     sa.B = B; sa.L = L; sa.D = D; sa.N = N;

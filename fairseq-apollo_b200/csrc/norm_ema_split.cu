@@ -3,8 +3,9 @@
 // The fused kernels move every element once, but a sequence is one chain of steps to them: with few sequences and
 // channels they leave the SMs idle.  Two ways fill the SMs whatever the shape: the scan (scan_ema.cu), whose walks
 // normalise their inputs as they read them, and, for bf16, TimestepNorm by itself (scan_norm.cu) followed by the
-// tensor-core kernel alone, which runs in half the time of the fused one; the normalised activations then go to their
-// own output, or through y in place.
+// tensor-core kernel alone, which runs in half the time of the fused one, or by the products of chunks (chunk_ema.cu; in bf16
+// 14 x 3140 x 712 with the second output 250 us as a chain, 154 so); the normalised activations then go to their own output, or
+// through y in place.
 #include <cmath>
 
 #include "chunk_ema.cuh"
@@ -47,15 +48,25 @@ double fused_us(int dtype, const StreamArgs& a, bool want_xn) {
   }
   // The streamed chain: ns a position by the blocks (128 channels of a sequence) that share an SM.  With a second output 16 x 4096 x
   // 1024 fp32 755 us, 31 x 2094 x 624 673, 58 x 530 x 960 fp16 163; without 58 x 530 x 960 114, 27 x 1781 x 1296 with a state 309.
-  const double per = ceil((double)a.B * ((a.D + 127) / 128) / 148.0), wide = dtype == MEGA_F32 ? 1.35 : 1.0;
+  const double per = ceil((double)a.B * ((a.D + 127) / 128) / 148.0 - 0.1), wide = dtype == MEGA_F32 ? 1.35 : 1.0;
   const bool state = a.h_in || a.h_out;
   double ns;
   if (a.cplx) ns = want_xn ? (per < 2 ? (state ? 254.0 : 234.0) : per < 3 ? 440.0 : 123.0 * per * wide)
                            : (per < 2 ? (state ? 254.0 : 171.0) : per < 3 ? 250.0 : 92.0 * per * wide);
-  else ns = want_xn ? (per < 2 ? 185.0 : per < 3 ? 335.0 : 100.0 * per * wide) : per < 3 ? 148.0 : 54.0 * per * wide;
+  else ns = want_xn ? (per < 2 ? 185.0 : per < 3 ? 335.0 : 100.0 * per) : per < 2 ? 138.0 : per < 3 ? 148.0 : 54.0 * per * wide;
   return 8.0 + L * ns * 1e-3;
 }
 
+// The EMA of the normalised activations where TimestepNorm has left them.
+ScanArgs behind_norm(const ScanArgs& ea, const void* mid) {
+  ScanArgs a = ea;
+  a.x = mid;
+  a.xsb = ea.ysb;
+  a.xsl = ea.ysl;
+  a.xn = nullptr;
+  a.prev_count = nullptr;
+  return a;
+}
 // TimestepNorm, then the tensor-core kernel alone: where the fused call would run on it too (both round the normalised
 // activations to bf16), without a mask (that form gains little) and at lengths that it can stop at
 double mma_us(int dtype, const StreamArgs& a, bool want_xn) {
@@ -129,12 +140,17 @@ bool norm_ema_split_try(int dtype, const void* x, void* y, void* xn, long long x
   // (the margins: two more launches for the norm by itself, on a host that is not ahead of the device; the fixed 45 us of
   // the scan's launches hold one; the models are good to a tenth)
   // (a prompt that comes in chunks keeps to the tensor-core kernel, and its rounding, unless much is gained)
-  const bool chunk = dtype == MEGA_BF16 && a.h_out && !a.mask && !a.cplx;
-  const double fused = fused_us(dtype, a, xn != nullptr), scan = scan_us(dtype, ea, xn != nullptr) + (chunk ? 25.0 : 0.0),
-               mma = mma_us(dtype, a, xn != nullptr) + 25.0;
+  const bool prompt = dtype == MEGA_BF16 && a.h_out && !a.mask && !a.cplx;
+  const double fused = fused_us(dtype, a, xn != nullptr), scan = scan_us(dtype, ea, xn != nullptr) + (prompt ? 25.0 : 0.0),
+               chain = mma_us(dtype, a, xn != nullptr) + 25.0;
+  // The products of chunks behind TimestepNorm in bf16: for calls that would run on the tensor-core kernel in one of its two ways,
+  // whose roundings these are too (complex 4 x 4096 x 1024 263 us fused, 103 so; real 142 and 94).
+  const bool rounds = chain < 1e29 && (scan > 0.9 * fused || chain < scan);
+  const double chunks = rounds ? 35.0 + (double)a.B * a.D * a.L / 700e3 + chunk_ema_fwd_us(dtype, behind_norm(ea, ea.y)) : 1e30;
+  const double mma = chunks < chain ? chunks : chain;
   if (forced == 0) {   // (what stands in mean_out and the like once the norm has run is what the forms below write too)
-    const double chunk = chunk_us(dtype, ea);
-    if ((chunk < 0.88 * (scan < mma ? scan : mma) && chunk < 0.88 * fused) || (chunk < 1e29 && g_options[OPT_CHUNK].load() == 2))
+    const double chunk = chunk_us(dtype, ea), by_scan = scan - (prompt ? 25.0 : 0.0);
+    if ((chunk < 0.88 * (by_scan < mma ? by_scan : mma) && chunk < 0.88 * fused) || (chunk < 1e29 && g_options[OPT_CHUNK].load() == 2))
       if (norm_chunk_try(dtype, ea, xsd, ysd, s)) return true;
   }
   if (forced == 0 && (scan < mma ? scan : mma) > 0.9 * fused) return false;
@@ -146,7 +162,8 @@ bool norm_ema_split_try(int dtype, const void* x, void* y, void* xn, long long x
     na.prev_count = a.prev_count; na.prev_mean = a.prev_mean; na.prev_var = a.prev_var; na.gamma = a.gamma;
     na.beta = a.beta; na.eps = a.eps; na.count_out = a.count_out; na.mean_out = a.mean_out; na.var_out = a.var_out;
     if (scan_norm_fwd_try(dtype, na, xsd, ysd, s) &&
-        mma_cl_try(dtype, mid, y, nullptr, ysb, ysl, ysd, ysb, ysl, ysd, false, a, s))
+        ((chunks < chain && chunk_ema_fwd_try(dtype, dtype, behind_norm(ea, mid), 1, ysd, s, true)) ||
+         mma_cl_try(dtype, mid, y, nullptr, ysb, ysl, ysd, ysb, ysl, ysd, false, a, s)))
       return true;   // (were the second one refused, the next form starts from x again)
   }
   return scan_ema_fwd_try(dtype, ea, xsd, ysd, s);

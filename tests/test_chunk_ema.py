@@ -182,6 +182,22 @@ def test_nothing_before_a_non_finite_input(forced, value, dtype, at, cplx):
 
 
 @pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("bsz,length,dim,ndim", SHAPES)
+def test_leading_parts(forced, bsz, length, dim, ndim, cplx):
+    """bf16 in leading parts alone: matrices, states and outputs are rounded once each (2^-9), which adds up to 2^-8."""
+    from fairseq_apollo_b200 import ops
+    gen = torch.Generator().manual_seed(length)
+    x, _, p, q, g, omega = problem(gen, bsz, length, dim, ndim, torch.bfloat16, cplx)
+    want, _ = recurrence(*[double(t) for t in (x, p, q, g, omega)])
+    fwd = ops.cema_forward if cplx else ops.ema_forward
+    c = [t.cuda() for t in (p, q, g, omega)]
+    forced.set_option(6, 3)
+    y = fwd(x.cuda().transpose(1, 2), *c, silu=True)
+    assert forced.last_kernel() == "chunk_ema"
+    assert rel_l2(y.transpose(1, 2), torch.nn.functional.silu(want)) < 1.5 * 2.0 ** -8
+
+
+@pytest.mark.parametrize("cplx", [False, True])
 def test_chosen_calls_agree_with_the_scan(cplx):
     """A call that the estimate gives to the chunks, against the forms that walk position by position."""
     from fairseq_apollo_b200 import _lib, ops
