@@ -39,6 +39,8 @@ bool mma_takes(int dtype, const StreamArgs& a, bool want_xn) {
 double fused_us(int dtype, const StreamArgs& a, bool want_xn) {
   const double L = a.L, n = (double)a.B * a.D * a.L;
   if (mma_takes(dtype, a, want_xn)) {
+    // (both a mask and the second output: 11 x 1894 x 464 153 us, 6 x 4999 x 2048 387, 16 x 4096 x 1024 257)
+    if (a.mask && want_xn) return 15.0 + longer(65.0, 290e3, L, n);
     const double fixed = a.cplx ? (want_xn ? 100.0 : 95.0) : want_xn ? 15.0 : a.mask ? 13.0 : 11.0;
     const double chain = a.cplx ? (want_xn ? 41.0 : 38.0) : want_xn ? 44.0 : a.mask ? 42.0 : 30.0;
     const double rate = a.cplx ? (want_xn ? 300e3 : 480e3) : want_xn ? 500e3 : a.mask ? 520e3 : 600e3;
@@ -78,7 +80,10 @@ double mma_us(int dtype, const StreamArgs& a, bool want_xn) {
 // (in one launch, or as the scan's five)
 double scan_us(int dtype, const ScanArgs& ea, bool want_xn) {
   const double n = (double)ea.B * ea.D * ea.L, one = scan_cluster_us(dtype, ea);
-  return one < 1e29 ? one : 45.0 + n / (ea.cplx ? (want_xn ? 78e3 : 88e3) : (want_xn ? 145e3 : 165e3));
+  // (padding masks: 33 x 1282 x 456 fp32 199 us, 16 x 4096 x 1024 fp16 475, with the second output 5 x 4079 x 536 201, complex
+  // 1 x 9084 x 728 152)
+  const double masked = !ea.mask ? 1.0 : ea.cplx ? 1.15 : want_xn ? 1.45 : dtype == MEGA_F32 ? 1.2 : 1.1;
+  return one < 1e29 ? one : 45.0 + masked * n / (ea.cplx ? (want_xn ? 78e3 : 88e3) : (want_xn ? 145e3 : 165e3));
 }
 
 // TimestepNorm in fp32, then the products of chunks (chunk_ema.cu): the normalised activations lie in scratch memory, for fp32
