@@ -24,8 +24,8 @@
 // multiply.
 //
 // bf16 calls that would otherwise go to the tensor-core kernel take the leading parts alone, as that one does (lean_call).
-// What bounds it: the tensor pipe is busy 45 % of the time, the rest is issue slots and the latency of a turn at 16 warps per
-// SM; DRAM stays below a third of its rate.
+// What bounds it (backward of 16 x 4096 x 1024 bf16, 225 us for both of its walks in one): the tensor pipe is busy 47 % of the
+// time, issue slots 45 %, shared memory 32 %, DRAM 21 %; 16 warps per SM at 128 registers do not hide the chain of products.
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
@@ -1098,11 +1098,11 @@ bool envelope(int dtype, const ScanArgs& a) {
 // value and the kind of poles.
 double chunk_us(int dtype, const ScanArgs& a, bool bwd, bool lean, double cost, bool segmented) {
   static const double kFwd[2][3] = {{25., 32., 43.}, {44., 54., 64.}}, kBwd[2][3] = {{48., 75., 102.}, {97., 140., 168.}};
-  static const double kLeanFwd[2] = {17.5, 22.5};
+  static const double kLeanFwd[2] = {17., 22.5};
   const int parts = dtype == MEGA_BF16 ? 0 : dtype == MEGA_F16 ? 1 : 2, c = a.cplx ? 1 : 0;
   return (bwd ? (segmented ? 32. : 20.) : (segmented ? 22. : 14.)) +
          (lean ? kLeanFwd[c] : bwd ? kBwd[c][parts] : kFwd[c][parts]) * 1e-3 * cost * (segmented ? 1. : a.cplx ? 1.14 : 1.07) *
-             (a.mask ? (bwd ? 1.22 : a.cplx ? 1.22 : 1.36) : 1.);
+             (a.mask ? (bwd ? 1.22 : a.cplx ? 1.22 : 1.36) : 1.) * (lean && a.D % 16 ? 1.2 : 1.);   // (16 channels in two sectors)
 }
 // bf16 calls without states or mask that are too long for a cluster go to the tensor-core kernel, which takes leading parts alone
 // and walks a sequence as one chain: here they take leading parts alone too (lean), in a quarter of the products and the same
@@ -1117,8 +1117,8 @@ double chain_us(const ScanArgs& a) {
   const double L = a.L, n = (double)a.B * a.D * L, tiles = ((a.D + 15) / 16) * (double)((a.B + 7) / 8);
   if (a.cplx) return 95. + std::max(L * 29e-3, n / 700e3);
   if (a.mask) return 6. + std::max(L * 42e-3, n / 1300e3);
-  // (the pipelined form while each of its tiles has an SM; between that and the segmented form 80 - 170 ns a position)
-  const double ns = tiles > 148. && tiles <= 600. ? 0.28 * tiles : 22.;
+  // (16-channel tiles while each of them has an SM: 16 x 4096 x 1024 101 us, 14 x 3140 x 712 81; between that and the segmented form 80 - 170 ns a position)
+  const double ns = tiles > 148. && tiles <= 600. ? 0.28 * tiles : 23.2;
   return 6. + std::max(L * ns * 1e-3, n / 1300e3);
 }
 // The form that a call takes otherwise: the scan backward (real bf16 16 x 4096 x 1024: 517 us against 233 here, complex 1481
