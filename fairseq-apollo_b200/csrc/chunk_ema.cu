@@ -55,7 +55,7 @@ struct ChunkArgs {
   int walked;               // of them, those that this launch takes
   int rev;                  // time runs backwards
   int parts;                // values per (sequence, segment) in the carry array
-  float* carry;             // [B][S][parts][D][16]: what a segment starts from (of segment 0: unused)
+  float* carry;             // [B][S][parts][D][16]: what a segment starts from (of segment 0: a state that comes in, or unused)
   const unsigned char* frag;   // [D][blocks] of kBlockBytes
   int blocks;
   const float* pow;         // [D][4][16]: q^16 (re, im), 16 q^15 (re, im)
@@ -424,7 +424,9 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask, kLean>::kThrea
       if (kSens) sn[kSens ? c : 0][i] = 0.f;
     }
   if ((kOuts || kSums) && live) {
-    if (seg > 0) {
+    // (of several segments also the first one's: h_out may be h_in, which the last segment's block writes at any time)
+    const bool given = kMode == kEmit && a.h_in != nullptr;
+    if (seg > 0 || (given && s.S > 1)) {
 #pragma unroll
       for (int c = 0; c < kRe; ++c)
 #pragma unroll
@@ -438,14 +440,14 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask, kLean>::kThrea
             sn[kSens ? c : 0][2 * k + 1] = u.y;
           }
         }
-    } else if (kMode == kEmit && a.h_in) {
+    } else if (given) {   // (the lane that writes them to h_out reads them, and not as what nothing writes)
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int n = 8 * (i >> 1) + 2 * t + (i & 1);
         const size_t at = ((size_t)b * a.D + d) * a.N + n;
         if (n < a.N) {
-          h[0][i] = __ldg(a.h_in + kRe * at);
-          if (kC) h[kRe - 1][i] = __ldg(a.h_in + kRe * at + 1);
+          h[0][i] = __ldcg(a.h_in + kRe * at);
+          if (kC) h[kRe - 1][i] = __ldcg(a.h_in + kRe * at + 1);
         }
       }
     }
@@ -986,7 +988,8 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask, kLean>::kThrea
 }
 
 // ---- the carry ---------------------------------------------------------------------------------------------
-// A thread per (sequence, channel, pole): what every segment starts from, in the place of what the segment before it adds.
+// A thread per (sequence, channel, pole): what every segment starts from, in the place of what the segment before it adds;
+// of the first one a state that comes in.
 // kSens: its derivative too.
 template <bool kC, bool kSens>
 __global__ void __launch_bounds__(128) chunk_carry_kernel(ChunkArgs s) {
@@ -1015,10 +1018,15 @@ __global__ void __launch_bounds__(128) chunk_carry_kernel(ChunkArgs s) {
   const size_t val = (size_t)a.D * 16, step = val * s.parts;
   float* v = s.carry + ((size_t)b * s.S + 1) * step + i;
   float hr = 0.f, hi = 0.f, sr = 0.f, si = 0.f;
-  if (!kSens && a.h_in && in) {
+  if (!kSens && a.h_in) {
     const size_t o = ((size_t)b * a.D + d) * a.N + n;
-    hr = a.h_in[kRe * o];
-    if (kC) hi = a.h_in[kRe * o + 1];
+    if (in) {
+      hr = __ldcg(a.h_in + kRe * o);
+      if (kC) hi = __ldcg(a.h_in + kRe * o + 1);
+    }
+    float* first = v - step;
+    first[0] = hr;
+    if (kC) first[val] = hi;
   }
   constexpr int kB = 4;   // segments whose loads go out together
   for (int k0 = 1; k0 < s.S; k0 += kB, v += kB * step) {

@@ -137,8 +137,8 @@ MEGA_API int mega_ema_bias(const float* q, const float* gamma_hat, const float* 
  * The EMA layer forward: y = conv(k, x*(1-mask)) [+ carried-state term] + omega*x [then SiLU].
  * x, y: activations (B,D,L) by strides.  p, q, gamma_hat: (K,N) with K = D, or 2*D when
  * MEGA_EMA_BIDIRECTIONAL.  omega (D).  pad_mask NULL or (B,L).  h_in NULL or (B,D,N): state
- * carried in; h_out NULL or (B,D,N): state after the last position (ema_hidden).  States are
- * rejected for bidirectional calls.  truncation <= 0 or >= L: full-length kernel; otherwise
+ * carried in; h_out NULL or (B,D,N): state after the last position (ema_hidden), h_in itself or
+ * apart from it (as wherever a call takes both).  States are rejected for bidirectional calls.  truncation <= 0 or >= L: full-length kernel; otherwise
  * the kernel support is its first `truncation` taps (bidirectional only, as in the reference).
  * Replaces: BaseMovingLayer.forward (fairseq/modules/base_moving_average.py:120-172) with
  * fftconv / bidirectional_fftconv (fairseq/modules/fused_ops/fftconv.py:13-27,85-100),

@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 def option():
     from fairseq_apollo_b200 import _lib
     yield _lib.set_option
-    for key in (1, 5):
+    for key in (1, 5, 6):
         _lib.set_option(key, 0)
 
 
@@ -192,3 +192,50 @@ def test_variance_of_long_segments(option):
     var = (2 + xd.pow(2).sum(1)) / n - mean.pow(2)
     assert rel_l2(res["mean"], mean) < 8e-7
     assert rel_l2(res["var"], var) < 8e-7
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("normed", [None, False, True])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("length", [40, 64 * 11 + 1])
+def test_pole_states_in_place(cplx, normed, dtype, length, option):
+    """h_out is h_in (C interface): one segment, and more segments than a block of the chunks takes, the last of one position."""
+    from fairseq_apollo_b200 import _lib
+    gen = torch.Generator().manual_seed(length)
+    bsz, dim, ndim, code = 3, 24, 16, {torch.float32: 0, torch.bfloat16: 1}[dtype]
+    x = torch.randn(bsz, length, dim, generator=gen).to(dtype).cuda()
+    pc, pm, pv = torch.full((bsz,), 2).cuda(), torch.zeros(bsz, dim).cuda(), torch.ones(bsz, dim).cuda()
+    ga, be = torch.ones(dim).cuda(), torch.zeros(dim).cuda()
+    two = (2,) if cplx else ()
+    p, om = torch.rand(dim, ndim, generator=gen).cuda(), torch.randn(dim, generator=gen).cuda()
+    q = (torch.rand(dim, ndim, *two, generator=gen) * 0.3 + (0.3 if cplx else 0.6)).cuda()
+    g = torch.randn(dim, ndim, *two, generator=gen).cuda()
+    start = torch.randn(bsz, dim, ndim, *two, generator=gen).cuda()
+    P = lambda t: None if t is None else t.data_ptr()
+    sb, sl, sd = x.stride()
+    lib = _lib.lib()
+
+    def run(h_in, h_out):
+        y, xn = torch.empty_like(x), torch.empty_like(x) if normed else None
+        cnt, mean, var = torch.empty_like(pc), torch.empty_like(pm), torch.empty_like(pv)
+        stream = torch.cuda.current_stream().cuda_stream
+        if normed is None:
+            rc = (lib.mega_cema_fwd if cplx else lib.mega_ema_fwd)(
+                P(x), P(y), code, bsz, dim, length, sb, sd, sl, sb, sd, sl, P(p), P(q), P(g), P(om), ndim, None, P(h_in), P(h_out), 0, 0,
+                stream)
+        else:
+            rc = (lib.mega_tsn_cema_fwd if cplx else lib.mega_tsn_ema_fwd)(
+                P(x), P(y), P(xn), code, bsz, length, dim, sb, sl, sd, sb, sl, sd, P(pc), P(pm), P(pv), P(ga), P(be), 1e-5, P(cnt),
+                P(mean), P(var), P(p), P(q), P(g), P(om), ndim, None, P(h_in), P(h_out), 0, stream)
+        assert rc == 0
+        return y
+
+    for form in (2, 0):
+        option(6, form)
+        apart, own = torch.empty_like(start), start.clone()
+        want = run(start, apart)
+        for _ in range(3):
+            own.copy_(start)
+            y = run(own, own)   # (not every form takes both: bf16 operands differ by 2^-9, a wrong start by its whole size)
+            limit = 1e-5 if dtype == torch.float32 else 2.0 ** -7
+            assert rel_l2(y, want) < limit and rel_l2(own, apart) < limit
