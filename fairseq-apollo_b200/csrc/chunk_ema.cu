@@ -58,7 +58,7 @@ struct ChunkArgs {
   float* carry;             // [B][S][parts][D][16]: what a segment starts from (of segment 0: a state that comes in, or unused)
   const unsigned char* frag;   // [D][blocks] of kBlockBytes
   int blocks;
-  const float* pow;         // [D][4][16]: q^16 (re, im), 16 q^15 (re, im)
+  const float* pow;         // [D][6][16]: q^16 (re, im), 16 q^15 (re, im), what rounding took from q^16 relative to it (re, im)
 };
 
 template <typename T>
@@ -88,12 +88,14 @@ struct Form {
   static constexpr int kE = 16 / (int)sizeof(In), kPos = kTile / (4 * kE);  // channels of a 16-byte piece; positions of a thread
   static constexpr int kSlot = kIns * kPos * kThreads * 16;        // bytes of a tile as it arrives
   static constexpr int stage = kBufs * kIns * kP * kPlane;
-  static constexpr int fixed = stage + kShared * kCh * kBlockBytes + (kMask ? 512 : 0);
+  static constexpr int kRests = kLean ? 0 : kCh * 16 * (kC ? 8 : 4);  // of q^16
+  static constexpr int fixed = stage + kShared * kCh * kBlockBytes + (kMask ? 512 : 0) + kRests;
   static constexpr int kSlots = fixed + 2 * kSlot <= (kCh == 8 ? 112 : 226) * 1024 ? 2 : 1;
   static constexpr int mats = stage + kSlots * kSlot;
   static constexpr int bits = mats + kShared * kCh * kBlockBytes;  // padded positions: a word for 32 of them, two sets
   static constexpr int kBits = 8 * kTile / 32;                     // words of a set
-  static constexpr int total = bits + (kMask ? 2 * kBits * 4 : 0);
+  static constexpr int rests = bits + (kMask ? 2 * kBits * 4 : 0);
+  static constexpr int total = rests + kRests;
   static constexpr int kPerSm = kCh == 8 && total <= 112 * 1024 ? 2 : 1;
   static_assert(total <= 227 * 1024, "a block's shared memory");
 };
@@ -296,11 +298,17 @@ __global__ void __launch_bounds__(128) chunk_prepare_kernel(PrepArgs a) {
   }
   __syncwarp();
   if (lane < 16) {
-    float* pc = a.pow + (size_t)d * 64 + n;
-    pc[0] = (float)pw[16][n].x;
-    pc[16] = (float)pw[16][n].y;
+    float* pc = a.pow + (size_t)d * 96 + n;
+    const double2 w = pw[16][n];
+    const float r = (float)w.x, i = (float)w.y;
+    pc[0] = r;
+    pc[16] = i;
     pc[32] = (float)(16. * pw[15][n].x);
     pc[48] = (float)(16. * pw[15][n].y);
+    const double m = (double)r * r + (double)i * i;   // (w - v) / v, v = r + i I; none for poles that forget sooner than they are corrected
+    const bool some = m > 0.81;
+    pc[64] = some ? (float)(((w.x - r) * r + (w.y - i) * i) / m) : 0.f;
+    pc[80] = some ? (float)(((w.y - i) * r - (w.x - r) * i) / m) : 0.f;
   }
   constexpr int kV = Blocks<kC>::v;
   const int g = lane >> 2, t = lane & 3;
@@ -402,7 +410,7 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask, kLean>::kThrea
   };
   // poles of a lane: 8 i + 2 t + e
   float qr[4], qi[kC ? 4 : 1], ur[kSens ? 4 : 1], ui[kSens && kC ? 4 : 1];
-  const float* pw = s.pow + (size_t)dc * 64;
+  const float* pw = s.pow + (size_t)dc * 96;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int n = 8 * (i >> 1) + 2 * t + (i & 1);
@@ -412,6 +420,17 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask, kLean>::kThrea
     if (kSens && kC) ui[kSens && kC ? i : 0] = __ldg(pw + 48 + n);
   }
   const float om = kApart ? __ldg(a.omega + dc) : 0.f;
+  // q^16 rounded to fp32 is off by the same 2^-25 in every chunk, which adds up to 2^-25 / (1 - q^16) of a state; so every
+  // 512 positions the states get what it lacks, for the 32 chunks to come at once (a pole at 0.9999: 6e-6 from float64 without, a
+  // recurrence in fp32 1.4e-6, so 4e-7; at each tile of 64 it cost a backward 5 %)
+  if constexpr (!kLean) {
+    if (lane < 16) {
+      float* rest = reinterpret_cast<float*>(smem + F::rests) + warp * 16 * kRe;
+      rest[kRe * lane] = __ldg(pw + 64 + lane);
+      if (kC) rest[kRe * lane + kRe - 1] = __ldg(pw + 80 + lane);
+    }
+    __syncwarp();
+  }
 
   // states that the segment starts from
   auto carry_at = [&](int at, int part) { return s.carry + (((size_t)(b * s.S + at) * s.parts + part) * a.D + d) * 16 + 2 * t; };
@@ -460,6 +479,30 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask, kLean>::kThrea
       re = r;
     } else {
       re = fmaf(qr[i], re, vr);
+    }
+  };
+  auto settle = [&](float chunks) {
+    int id;   // (read again, and the loads volatile: nothing of this is kept in a register beside the products)
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(id));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t at = smem_u32(smem) + F::rests + ((id >> 5) * 16 + 8 * (i >> 1) + 2 * (id & 3) + (i & 1)) * (4 * kRe);
+      float er, ei = 0.f;
+      if (kC) asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(er), "=f"(ei) : "r"(at));
+      else asm volatile("ld.shared.f32 %0, [%1];" : "=f"(er) : "r"(at));
+      er *= chunks;
+      ei *= chunks;
+      auto more = [&](float& re, float& im) {
+        if (kC) {
+          const float r = re;
+          re = fmaf(er, r, fmaf(-ei, im, r));
+          im = fmaf(er, im, fmaf(ei, r, im));
+        } else {
+          re = fmaf(er, re, re);
+        }
+      };
+      more(h[0][i], h[kRe - 1][i]);
+      if (kSens) more(sn[0][i], sn[kSens ? kRe - 1 : 0][i]);
     }
   };
   // kSums: A1 and A2 of the lane's poles, R of its entries
@@ -880,6 +923,8 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask, kLean>::kThrea
     arrive(0);
     __syncthreads();
     for (int i = 0; i < tiles; ++i) {
+      if constexpr (!kLean)
+        if (i % (512 / kTile) == 0) settle(2 * min(16, steps - kTile / 32 * i));
       if constexpr (kSame) {
 #pragma unroll 1
         for (int half = 0; half < 2; ++half) {
@@ -901,6 +946,8 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask, kLean>::kThrea
     leave(tiles - 1);
   } else {
     for (int i = 0; i < tiles; ++i) {
+      if constexpr (!kLean)
+        if (i % (512 / kTile) == 0) settle(2 * min(16, steps - kTile / 32 * i));
       arrive(i);
       __syncthreads();
       if (d < a.D) multiply(i);
@@ -1015,6 +1062,7 @@ __global__ void __launch_bounds__(128) chunk_carry_kernel(ChunkArgs s) {
   }
   const double wr = ur * qr - ui * qi, wi = ur * qi + ui * qr;
   const float fr = (float)wr, fi = (float)wi, gr = (float)(s.T * ur), gi = (float)(s.T * ui);
+  const float er = (float)(wr - fr), ei = (float)(wi - fi);   // (the same rounding in every segment: see settle())
   const size_t val = (size_t)a.D * 16, step = val * s.parts;
   float* v = s.carry + ((size_t)b * s.S + 1) * step + i;
   float hr = 0.f, hi = 0.f, sr = 0.f, si = 0.f;
@@ -1051,14 +1099,16 @@ __global__ void __launch_bounds__(128) chunk_carry_kernel(ChunkArgs s) {
           x = fmaf(-gi, hi, x);
           y = fmaf(gr, hi, fmaf(gi, hr, mi[u]));
         }
+        x = fmaf(er, sr, kC ? fmaf(-ei, si, x) : x);
         const float r = kC ? fmaf(fr, sr, fmaf(-fi, si, x)) : fmaf(fr, sr, x);
-        if (kC) si = fmaf(fi, sr, fmaf(fr, si, y));
+        if (kC) si = fmaf(fi, sr, fmaf(fr, si, fmaf(ei, sr, fmaf(er, si, y))));
         sr = r;
         p[kRe * val] = sr;
         if (kC) p[(kRe + 1) * val] = si;
       }
-      const float r = kC ? fmaf(fr, hr, fmaf(-fi, hi, lr[u])) : fmaf(fr, hr, lr[u]);
-      if (kC) hi = fmaf(fi, hr, fmaf(fr, hi, li[u]));
+      const float x = fmaf(er, hr, kC ? fmaf(-ei, hi, lr[u]) : lr[u]);
+      const float r = kC ? fmaf(fr, hr, fmaf(-fi, hi, x)) : fmaf(fr, hr, x);
+      if (kC) hi = fmaf(fi, hr, fmaf(fr, hi, fmaf(ei, hr, fmaf(er, hi, li[u]))));
       hr = r;
       p[0] = hr;
       if (kC) p[val] = hi;
@@ -1159,10 +1209,10 @@ bool fwd(int dtype, const ScanArgs& a, bool asked, cudaStream_t st) {
   s.blocks = kBlocks;
   s.parts = kC ? 2 : 1;
   const size_t frag = (size_t)a.D * kBlocks * kBlockBytes, carry = s.S > 1 ? (size_t)a.B * s.S * s.parts * a.D * 16 : 0;
-  Scratch sc(Scratch::padded(frag) + Scratch::padded((size_t)a.D * 256) + Scratch::padded(carry * 4), st);
+  Scratch sc(Scratch::padded(frag) + Scratch::padded((size_t)a.D * 96 * 4) + Scratch::padded(carry * 4), st);
   if (!sc) return false;
   unsigned char* fr = sc.take<unsigned char>(frag);
-  float* pow = sc.take<float>((size_t)a.D * 64);
+  float* pow = sc.take<float>((size_t)a.D * 96);
   s.frag = fr;
   s.pow = pow;
   s.carry = carry ? sc.take<float>(carry) : nullptr;
@@ -1192,10 +1242,10 @@ bool bwd(int dtype, const ScanArgs& a, cudaStream_t st) {
   s.blocks = kBlocks;
   s.parts = 2 * kRe;
   const size_t frag = (size_t)a.D * kBlocks * kBlockBytes, carry = s.S > 1 ? (size_t)a.B * s.S * s.parts * a.D * 16 : 0;
-  Scratch sc(Scratch::padded(frag) + Scratch::padded((size_t)a.D * 256) + Scratch::padded(carry * 4), st);
+  Scratch sc(Scratch::padded(frag) + Scratch::padded((size_t)a.D * 96 * 4) + Scratch::padded(carry * 4), st);
   if (!sc) return false;
   unsigned char* fr = sc.take<unsigned char>(frag);
-  float* pow = sc.take<float>((size_t)a.D * 64);
+  float* pow = sc.take<float>((size_t)a.D * 96);
   s.frag = fr;
   s.pow = pow;
   s.carry = carry ? sc.take<float>(carry) : nullptr;

@@ -254,3 +254,32 @@ def test_behind_timestep_norm(forced, bsz, length, dim, dtype, cplx, normed):
         out, last = torch.view_as_real(out.cpu()), torch.view_as_real(last)
     assert rel_l2(out, last) < 4e-6
     assert torch.equal(got["count"].cpu(), cnt) and rel_l2(got["mean"], mean) < 4e-6 and rel_l2(got["var"], var) < 4e-6
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("slow", [1e-3, 1e-4])
+def test_slow_poles(forced, slow, cplx):
+    """Poles near the unit circle over many chunks: a power of a pole that is rounded alike in every chunk or segment would add up
+    to 2^-25 / (1 - q^16), 6e-6 at 1e-4.  What is left is the rounding of each chunk's sum, of either sign: 2^-25 times the square
+    root of the 1 / (32 slow) that a state holds, and 2^-25 for each of the 16 chunks, on average, between the corrections."""
+    from fairseq_apollo_b200 import ops
+    gen = torch.Generator().manual_seed(2)
+    bsz, length, dim, ndim = 2, 16384 - 5, 16, 4
+    x, dy, p, _, g, omega = problem(gen, bsz, length, dim, ndim, torch.float32, cplx)
+    q = 1 - slow * (torch.rand(dim, ndim, generator=gen) + 0.5)
+    if cplx:
+        q = torch.polar(q, torch.rand(dim, ndim, generator=gen) * 6.28)
+    h = torch.randn(bsz, dim, ndim, dtype=q.dtype, generator=gen)
+    args = [double(t) for t in (p, q, g, omega)]
+    want, last = recurrence(x.double(), *args, double(h))
+    dx = recurrence(dy.double().flip(1), *args)[0].flip(1)
+    fwd, bwd = (ops.cema_forward, ops.cema_backward) if cplx else (ops.ema_forward, ops.ema_backward)
+    c = [t.cuda() for t in (p, q, g, omega)]
+    y, out = fwd(x.cuda().transpose(1, 2), *c, None, h.cuda(), True)
+    assert forced.last_kernel() == "chunk_ema"
+    grad = bwd(dy.cuda().transpose(1, 2), x.cuda().transpose(1, 2), *c)[0]
+    assert forced.last_kernel() == "chunk_ema"
+    if cplx:
+        out, last = torch.view_as_real(out.cpu()), torch.view_as_real(last)
+    limit = 2.0 ** -25 * ((1 / (32 * slow)) ** 0.5 + 16)
+    assert rel_l2(out, last) < limit and rel_l2(y.transpose(1, 2), want) < limit and rel_l2(grad.transpose(1, 2), dx) < limit
