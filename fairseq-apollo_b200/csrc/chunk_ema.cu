@@ -341,6 +341,74 @@ __global__ void __launch_bounds__(128) chunk_prepare_kernel(PrepArgs a) {
   }
 }
 
+// ---- what the products cannot give -----------------------------------------------------------------------------
+// An infinity, a NaN or a value that bf16 rounds to an infinity makes NaN of all products that it enters, where the recurrence
+// leaves finite states and outputs, or infinite ones, as they follow.  Here it is, position by position in fp32: n positions from
+// `first` on (in the order they are walked) of the row of a quad (none where n is 0), from and to the states of a lane's poles;
+// each(k, y) for outputs from the first such value on.  The whole warp takes part, for `most` positions.
+template <typename In, bool kC, bool kSens, int kRe, typename Each>
+__device__ __forceinline__ void one_by_one(const ChunkArgs& s, int b, int d, int first, int n, int most, float (&h)[kRe][4],
+                                           float (*sens)[4], Each each) {
+  const ScanArgs& a = s.a;
+  const int t = threadIdx.x & 3;
+  const bool gain = a.h_in || a.h_out;   // (the states are the layer's own then: see chunk_prepare_kernel)
+  float fr[4], fi[4], u[4], c[4], ci[4], z = 0.f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {   // (poles there are not: states and weights of zero)
+    const int m = 8 * (i >> 1) + 2 * t + (i & 1);
+    const size_t at = (size_t)d * a.N + min(m, a.N - 1);
+    const float p = __ldg(a.p + at);
+    fr[i] = m < a.N ? __ldg(a.q + kRe * at) : 0.f;
+    fi[i] = kC && m < a.N ? __ldg(a.q + kRe * at + 1) : 0.f;
+    u[i] = gain ? p : 1.f;
+    c[i] = m < a.N ? (gain ? 1.f : p) * __ldg(a.g + kRe * at) : 0.f;
+    ci[i] = kC && m < a.N ? (gain ? 1.f : p) * __ldg(a.g + kRe * at + 1) : 0.f;
+    z = fmaf(h[0][i], 0.f, fmaf(h[kRe - 1][i], 0.f, z));
+  }
+  const unsigned quad = 15u << (threadIdx.x & 28);
+  bool on = (__ballot_sync(0xffffffffu, z != z) & quad) != 0u;
+  const float om = __ldg(a.omega + d);
+  const long long step = s.rev ? -s.isl : s.isl;
+  const In* x = reinterpret_cast<const In*>(s.in) + b * s.isb + (long long)(s.rev ? a.L - 1 - first : first) * s.isl + d;
+  const unsigned char* pad = a.mask ? a.mask + (size_t)b * a.L + (s.rev ? a.L - 1 - first : first) : nullptr;
+#pragma unroll 1
+  for (int k0 = 0; k0 < most; k0 += 8) {
+    float v[8];
+    bool skip[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int at = k0 + k;
+      v[k] = at < n ? Elem<In>::ld(x + at * step) : 0.f;
+      skip[k] = pad && at < n && __ldg(pad + (s.rev ? -at : at)) != 0;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const bool in_row = k0 + k < n;
+      const float in = skip[k] && !s.rev ? 0.f : v[k];
+      on = on || (bf16_pair(in, in) & 0x7f80u) == 0x7f80u;
+      float out = 0.f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (!in_row || 8 * (i >> 1) + 2 * t + (i & 1) >= a.N) continue;
+        float &re = h[0][i], &im = h[kRe - 1][i];
+        if (kSens) {
+          float &sr = sens[0][i], &si = sens[kRe - 1][i];
+          const float r = kC ? fmaf(fr[i], sr, fmaf(-fi[i], si, re)) : fmaf(fr[i], sr, re);
+          if (kC) si = fmaf(fr[i], si, fmaf(fi[i], sr, im));
+          sr = r;
+        }
+        const float w = u[i] * in, r = kC ? fmaf(fr[i], re, fmaf(-fi[i], im, w)) : fmaf(fr[i], re, w);
+        if (kC) im = fmaf(fr[i], im, fi[i] * re);
+        re = r;
+        out = fmaf(c[i], re, kC ? fmaf(-ci[i], im, out) : out);
+      }
+#pragma unroll
+      for (int m = 1; m < 4; m <<= 1) out += __shfl_xor_sync(0xffffffffu, out, m);
+      if (on && in_row) each(k0 + k, fmaf(om, v[k], skip[k] && s.rev ? 0.f : out));
+    }
+  }
+}
+
 // ---- the walk ----------------------------------------------------------------------------------------------
 // kMask: padded positions are zero to the states (and to the correlations), omega x takes them as they are; in reversed time,
 // where outputs are the input's gradient, it is the outputs at padded positions that are omega dy alone.
@@ -435,17 +503,18 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask, kLean>::kThrea
   // states that the segment starts from
   auto carry_at = [&](int at, int part) { return s.carry + (((size_t)(b * s.S + at) * s.parts + part) * a.D + d) * 16 + 2 * t; };
   float h[kRe][4], sn[kSens ? kRe : 1][4];
+  auto start = [&]() {
 #pragma unroll
-  for (int c = 0; c < kRe; ++c)
+    for (int c = 0; c < kRe; ++c)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      h[c][i] = 0.f;
-      if (kSens) sn[kSens ? c : 0][i] = 0.f;
-    }
-  if ((kOuts || kSums) && live) {
-    // (of several segments also the first one's: h_out may be h_in, which the last segment's block writes at any time)
+      for (int i = 0; i < 4; ++i) {
+        h[c][i] = 0.f;
+        if (kSens) sn[kSens ? c : 0][i] = 0.f;
+      }
+    if (!(kOuts || kSums) || !live) return;
+    // (the first segment's too lies with the others, of one segment where h_out is h_in: that is written while this is read)
     const bool given = kMode == kEmit && a.h_in != nullptr;
-    if (seg > 0 || (given && s.S > 1)) {
+    if (seg > 0 || (given && s.carry)) {
 #pragma unroll
       for (int c = 0; c < kRe; ++c)
 #pragma unroll
@@ -459,18 +528,19 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask, kLean>::kThrea
             sn[kSens ? c : 0][2 * k + 1] = u.y;
           }
         }
-    } else if (given) {   // (the lane that writes them to h_out reads them, and not as what nothing writes)
+    } else if (given) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int n = 8 * (i >> 1) + 2 * t + (i & 1);
         const size_t at = ((size_t)b * a.D + d) * a.N + n;
         if (n < a.N) {
-          h[0][i] = __ldcg(a.h_in + kRe * at);
-          if (kC) h[kRe - 1][i] = __ldcg(a.h_in + kRe * at + 1);
+          h[0][i] = __ldg(a.h_in + kRe * at);
+          if (kC) h[kRe - 1][i] = __ldg(a.h_in + kRe * at + 1);
         }
       }
     }
-  }
+  };
+  start();
   // q^16 h + v of pole i
   auto next = [&](int i, float& re, float& im, float vr, float vi) {
     if (kC) {
@@ -583,7 +653,7 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask, kLean>::kThrea
               if (kLean) hp[c][0][2 * k + r] = bf16_pair(enter[k][c][2 * r], enter[k][c][2 * r + 1]);
               else split(enter[k][c][2 * r], enter[k][c][2 * r + 1], hp[c][0][2 * k + r], hp[c][1][2 * k + r], hp[c][2][2 * k + r]);
         // T's zeros would carry a NaN or an infinity to the positions before it: such a chunk takes its outputs from the finite
-        // values ahead of the first one, and is NaN from there on (as are all later states)
+        // values ahead of the first one, and is NaN from there on, as are all later states (until one_by_one())
         int bad[2];
         if (any_odd) {
           bad[0] = bad[1] = 16;
@@ -956,7 +1026,37 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask, kLean>::kThrea
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 
+  // (a state that is not finite stays so: such a row is gone through once more)
+  float z = 0.f;
+#pragma unroll
+  for (int i = 0; i < 4 * kRe; ++i) z = fmaf(h[i >> 2][i & 3], 0.f, z);
+  const unsigned odd = __ballot_sync(0xffffffffu, z != z);   // (of all lanes, also those without a row)
+  const bool odd_row = live && (odd >> (lane & 28) & 15u) != 0u;
+  const bool again = kMode != kGrad && __any_sync(0xffffffffu, odd_row);
+  if constexpr (kOuts) {
+    __syncthreads();   // (the block's outputs are there)
+    if (again && s.in != a.y) {   // (in place the inputs are gone: NaN from there on)
+      const int first = seg * s.T;
+      Out* y = reinterpret_cast<Out*>(a.y) + b * a.ysb + d;
+      if (odd_row) start();
+      one_by_one<In, kC, false>(s, b, d, first, odd_row ? len : 0, most, h, sn, [&](int k, float v) {
+        if (a.silu) v = silu_of<Out>(v);
+        if ((k & 3) == t) Elem<Out>::st(y + (s.rev ? a.L - 1 - first - k : first + k) * a.ysl, v);
+      });
+      if (odd_row && final >= 0) {
+#pragma unroll
+        for (int i = 0; i < 4 * kRe; ++i) {
+          const int m = 8 * ((i >> 1) & 1) + 2 * t + (i & 1);
+          if (m < a.N) a.h_out[kRe * (((size_t)b * a.D + d) * a.N + m) + (i >> 2)] = h[i >> 2][i & 3];
+        }
+      }
+    }
+  }
   if constexpr (kMode == kLocal || kMode == kLocalSens) {   // what the segment behind it starts from
+    if (again) {
+      if (odd_row) start();
+      one_by_one<In, kC, kSens>(s, b, d, seg * s.T, odd_row ? len : 0, most, h, sn, [](int, float) {});
+    }
     if (live) {
 #pragma unroll
       for (int c = 0; c < kRe; ++c)
@@ -1107,7 +1207,8 @@ __global__ void __launch_bounds__(128) chunk_carry_kernel(ChunkArgs s) {
         if (kC) p[(kRe + 1) * val] = si;
       }
       const float x = fmaf(er, hr, kC ? fmaf(-ei, hi, lr[u]) : lr[u]);
-      const float r = kC ? fmaf(fr, hr, fmaf(-fi, hi, x)) : fmaf(fr, hr, x);
+      float r = kC ? fmaf(fr, hr, fmaf(-fi, hi, x)) : fmaf(fr, hr, x);
+      if (!kC && fabsf(hr) == INFINITY && qr != 0.) r = hr + lr[u];   // (whatever is left of q^T: T is even)
       if (kC) hi = fmaf(fi, hr, fmaf(fr, hi, fmaf(ei, hr, fmaf(er, hi, li[u]))));
       hr = r;
       p[0] = hr;
@@ -1208,7 +1309,8 @@ bool fwd(int dtype, const ScanArgs& a, bool asked, cudaStream_t st) {
   constexpr int kBlocks = 2 * Blocks<kC>::v + 2;
   s.blocks = kBlocks;
   s.parts = kC ? 2 : 1;
-  const size_t frag = (size_t)a.D * kBlocks * kBlockBytes, carry = s.S > 1 ? (size_t)a.B * s.S * s.parts * a.D * 16 : 0;
+  const bool slots = s.S > 1 || (a.h_in && a.h_in == a.h_out);
+  const size_t frag = (size_t)a.D * kBlocks * kBlockBytes, carry = slots ? (size_t)a.B * s.S * s.parts * a.D * 16 : 0;
   Scratch sc(Scratch::padded(frag) + Scratch::padded((size_t)a.D * 96 * 4) + Scratch::padded(carry * 4), st);
   if (!sc) return false;
   unsigned char* fr = sc.take<unsigned char>(frag);
@@ -1224,8 +1326,8 @@ bool fwd(int dtype, const ScanArgs& a, bool asked, cudaStream_t st) {
   if (s.S > 1) {
     s.walked = s.S - 1;
     run<In, In, kC, kLocal, kMask, kLean>(s, st);
-    launch(chunk_carry_kernel<kC, false>, dim3((a.D * 16 + 127) / 128, a.B), 128, 0, (void*)st, s);
   }
+  if (slots) launch(chunk_carry_kernel<kC, false>, dim3((a.D * 16 + 127) / 128, a.B), 128, 0, (void*)st, s);
   s.walked = s.S;
   run<In, Out, kC, kEmit, kMask, kLean>(s, st);
   g_last_kernel.store("chunk_ema", std::memory_order_relaxed);

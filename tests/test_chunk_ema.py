@@ -283,3 +283,72 @@ def test_slow_poles(forced, slow, cplx):
         out, last = torch.view_as_real(out.cpu()), torch.view_as_real(last)
     limit = 2.0 ** -25 * ((1 / (32 * slow)) ** 0.5 + 16)
     assert rel_l2(out, last) < limit and rel_l2(y.transpose(1, 2), want) < limit and rel_l2(grad.transpose(1, 2), dx) < limit
+
+
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("state", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("at", [0, 15, 40, 70, 191])
+def test_infinities_are_the_recurrences(forced, dtype, at, state, masked):
+    """From an infinite input on, outputs and states are infinite where the recurrence's are (weights of one sign), not NaN, in
+    later segments too and for poles that forget within a chunk; the input's gradient the other way round in time."""
+    from fairseq_apollo_b200 import ops
+    gen = torch.Generator().manual_seed(at)
+    bsz, length, dim, ndim = 2, 300, 16, 5
+    x, dy, p, q, g, omega = problem(gen, bsz, length, dim, ndim, dtype, False)
+    q[:, 0] = 1e-4
+    g, omega = g.abs() + 0.1, omega.abs() + 0.1
+    mask = None
+    if masked:
+        mask = torch.rand(bsz, length, generator=gen) < 0.2
+        mask[1, at] = False
+    c = [t.cuda() for t in (p, q, g, omega)]
+    bad, bad_dy = x.clone(), dy.clone()
+    bad[1, at, 3], bad_dy[1, at, 3] = float("inf"), float("-inf")
+    mc = None if mask is None else mask.cuda()
+    h = torch.randn(bsz, dim, ndim, generator=gen) if state else None
+    out = ops.ema_forward(bad.cuda().transpose(1, 2), *c, mc, None if h is None else h.cuda(), state)
+    assert forced.last_kernel() == "chunk_ema"
+    keep = torch.ones(bsz, length, 1) if mask is None else (~mask).double().unsqueeze(-1)
+    args = [t.double() for t in (p, q, g, omega)]
+    want, last = recurrence(torch.where(keep > 0, bad.double(), 0.0), *args, None if h is None else h.double())
+    want = want + omega.double() * torch.where(keep > 0, 0.0, x.double())
+    y = (out[0] if state else out).transpose(1, 2).cpu().double()
+    assert torch.equal(y.isinf(), want.isinf()) and not y.isnan().any() and y[1, at:, 3].isinf().all()
+    fine = ~want.isinf()
+    assert rel_l2(y[fine], want[fine]) < LIMIT[dtype]
+    if state:
+        assert torch.equal(out[1].isinf().cpu(), last.isinf()) and last[1, 3].isinf().all()
+        fine = ~last.isinf()
+        assert rel_l2(out[1].cpu()[fine], last[fine]) < 5e-7
+        return
+    got = ops.ema_backward(bad_dy.cuda().transpose(1, 2), x.cuda().transpose(1, 2), *c, mc)
+    assert forced.last_kernel() == "chunk_ema"
+    back = recurrence(bad_dy.double().flip(1), *args)[0].flip(1)
+    want = torch.where(keep > 0, back, omega.double() * dy.double())
+    dx = got[0].transpose(1, 2).cpu().double()
+    assert torch.equal(dx.isinf(), want.isinf()) and not dx.isnan().any()
+    fine = ~want.isinf()
+    assert rel_l2(dx[fine], want[fine]) < LIMIT[dtype]
+    assert not any(torch.isfinite(t[3]).any() for t in got[1:5])
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+def test_values_that_bf16_takes_for_infinite(forced, cplx):
+    """fp32 values above bf16's largest: finite, as the recurrence has them."""
+    from fairseq_apollo_b200 import ops
+    gen = torch.Generator().manual_seed(3)
+    x, dy, p, q, g, omega = problem(gen, 2, 300, 16, 5, torch.float32, cplx)
+    g, omega = g * 0.1, omega.clamp(-0.4, 0.4)
+    x[1, 37, 3], dy[0, 250, 5] = 3.4e38, -3.4e38
+    args = [double(t) for t in (p, q, g, omega)]
+    want, back = recurrence(x.double(), *args)[0], recurrence(dy.double().flip(1), *args)[0].flip(1)
+    c = [t.cuda() for t in (p, q, g, omega)]
+    fwd, bwd = (ops.cema_forward, ops.cema_backward) if cplx else (ops.ema_forward, ops.ema_backward)
+    y = fwd(x.cuda().transpose(1, 2), *c).transpose(1, 2).cpu().double()
+    dx = bwd(dy.cuda().transpose(1, 2), x.cuda().transpose(1, 2), *c)[0].transpose(1, 2).cpu().double()
+    for a, b, row, ch in ((y, want, 1, 3), (dx, back, 0, 5)):
+        assert torch.isfinite(a).all()
+        there = torch.zeros_like(a, dtype=torch.bool)
+        there[row, :, ch] = True
+        assert rel_l2(a[there] * 2.0 ** -64, b[there] * 2.0 ** -64) < 5e-7 and rel_l2(a[~there], b[~there]) < 5e-7
