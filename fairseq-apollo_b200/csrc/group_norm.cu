@@ -3,8 +3,8 @@
 // The norm pools the statistics of the D / G channels of a group at every step and combines them over the
 // steps.  Only that combination is serial, it is one value per step and group, and it is associative, so
 // a pass is three launches: (1) the moments of every (step, group), a vector of 16 bytes per lane and
-// shuffles inside the group; (2) a scan over the steps, one block per sequence and 2 groups, 256 threads
-// along time: each walks its run of steps, the runs are combined across the threads (Chan's rule for
+// shuffles inside the group; (2) a scan over the steps, one block per sequence and 2 or 8 groups, 256 or 128
+// threads along time: each walks its run of steps, the runs are combined across the threads (Chan's rule for
 // counts, means and squared deviations), each walks its run again from what came before; (3) the
 // elementwise part.  The backward is the same with the reverse scan written as plain suffix sums: with
 // V = dL/dvar / n and U = dL/dmean / n at count n the recurrence of the reference
@@ -22,11 +22,12 @@ namespace mega {
 namespace {
 
 constexpr int kRowsPerBlock = 32;   // rows (sequence, step) of a block of the moment and elementwise kernels
-// Groups per block of the scan, and threads along time: the scan is issue slots and latency, so it goes over as many SMs as
-// there are pairs of groups (8 groups and 128 threads: 16 SMs for 4 sequences of 32 groups, 25 us forward and 41 backward at
-// L = 4096; one group would read a sector of 32 bytes for each float)
-constexpr int kScanG = 2;
-constexpr int kScanT = 256;
+// The scan's blocks take 2 groups with 256 threads along time while there are no more of them than SMs, else 8 with 128: it is
+// issue slots and latency, so it goes over as many SMs as there are pairs (4 sequences of 32 groups at L = 4096: 36 us forward
+// and 20 backward against 48 + 12 and 23 + 21; one group would read a sector of 32 bytes for each float), but beyond the SMs half
+// of a sector is read twice (forward and backward of 10 sequences of 12 groups at L = 2805: 174 us against 186; of 27 of 24 at
+// 1256 218 against 195).
+bool by_pairs(int B, int G) { return (long long)B * ((G + 1) / 2) <= 148; }
 
 template <typename T>
 struct Vec {
@@ -102,6 +103,7 @@ __device__ __forceinline__ Run combine(Run a, Run b) {
   return {n, fmaf(d, w, a.m), a.s + b.s + d * d * a.n * w};
 }
 
+template <int kScanG, int kScanT>
 __global__ void __launch_bounds__(kScanG* kScanT) group_scan_kernel(const float* gm, const float* gv, int L, int G,
                                                                     const long long* prev_count, const float* prev_mean,
                                                                     const float* prev_var, const unsigned char* mask,
@@ -149,7 +151,7 @@ __global__ void __launch_bounds__(kScanG* kScanT) group_scan_kernel(const float*
   }
   part[ti][gi] = r;
   __syncthreads();
-  // inclusive scan over the threads along time (eight rounds)
+  // inclusive scan over the threads along time (seven or eight rounds)
 #pragma unroll
   for (int o = 1; o < kScanT; o <<= 1) {
     Run mine = part[ti][gi];
@@ -298,6 +300,7 @@ __device__ __forceinline__ Map compose(Map late, Map early) {
   return {late.n + early.n, late.sv + early.sv, late.su + early.su + early.sw * late.sv, late.sw + early.sw};
 }
 
+template <int kScanG, int kScanT>
 __global__ void __launch_bounds__(kScanG* kScanT) group_bwd_scan_kernel(const float* ds, const float* db, int L, int G,
                                                                         const float* cummean, const float* cumrstd,
                                                                         const float* group_mean, const float* prev_mean,
@@ -472,12 +475,13 @@ bool group_norm_try(int dtype, const void* x, void* y, long long xsb, long long 
   float* cm = save ? a.cummean : sc.take<float>(n);
   float* cr = save ? a.cumrstd : sc.take<float>(n);
   const unsigned grid_m = (unsigned)((rows + kRowsPerBlock - 1) / kRowsPerBlock);
-  const dim3 grid_s((a.G + kScanG - 1) / kScanG, a.B);
+  const bool pairs = by_pairs(a.B, a.G);
+  const dim3 grid_s(pairs ? (a.G + 1) / 2 : (a.G + 7) / 8, a.B);
   switch (dtype) {
 #define MEGA_GROUP_CASE(DT, TY)                                                                                       \
   case DT:                                                                                                            \
     launch(group_moments_kernel<TY>, grid_m, 256, 0, (void*)s, (const TY*)x, xsb, xsl, a.L, a.D, a.G, rows, gm, gv);   \
-    launch(group_scan_kernel, grid_s, kScanG * kScanT, 0, (void*)s, gm, gv, a.L, a.G, a.prev_count, a.prev_mean,       \
+    launch(pairs ? group_scan_kernel<2, 256> : group_scan_kernel<8, 128>, grid_s, pairs ? 512 : 1024, 0, (void*)s, gm, gv, a.L, a.G, a.prev_count, a.prev_mean,       \
            a.prev_var, a.mask, a.eps, cm, cr, a.count_out, a.mean_out, a.var_out);                                     \
     launch(group_apply_kernel<TY>, apply_grid(rows * (a.D / Vec<TY>::kN)), 256, 0, (void*)s, (const TY*)x, (TY*)y, xsb, \
            xsl, ysb, ysl, a.L, a.D, a.G, rows, cm, cr, a.gamma, a.beta, a.mask);                                       \
@@ -502,7 +506,8 @@ bool group_norm_bwd_try(int dtype, const void* dy, const void* x, void* dx, long
   Scratch sc(Scratch::padded(n * sizeof(float)) * 4, s);
   if (!sc) return false;
   float *ds = sc.take<float>(n), *db = sc.take<float>(n), *dux = sc.take<float>(n), *dvx = sc.take<float>(n);
-  const dim3 grid_s((a.G + kScanG - 1) / kScanG, a.B);
+  const bool pairs = by_pairs(a.B, a.G);
+  const dim3 grid_s(pairs ? (a.G + 1) / 2 : (a.G + 7) / 8, a.B);
   switch (dtype) {
 #define MEGA_GROUP_CASE(DT, TY)                                                                                        \
   case DT: {                                                                                                           \
@@ -510,7 +515,7 @@ bool group_norm_bwd_try(int dtype, const void* dy, const void* x, void* dx, long
                       (unsigned)((a.D / Vec<TY>::kN + 31) / 32));                                                      \
     launch(group_bwd_sums_kernel<TY>, grid_m, 256, 0, (void*)s, (const TY*)dy, (const TY*)x, gsb, gsl, xsb, xsl, a.L,  \
            a.D, a.G, rows, a.cummean, a.cumrstd, a.gamma, a.mask, ds, db, a.dgamma, a.dbeta);                          \
-    launch(group_bwd_scan_kernel, grid_s, kScanG * kScanT, 0, (void*)s, ds, db, a.L, a.G, a.cummean, a.cumrstd,        \
+    launch(pairs ? group_bwd_scan_kernel<2, 256> : group_bwd_scan_kernel<8, 128>, grid_s, pairs ? 512 : 1024, 0, (void*)s, ds, db, a.L, a.G, a.cummean, a.cumrstd,        \
            a.group_mean, a.prev_mean, a.count, a.dmean, a.dvar, a.mask, dux, dvx, a.dprev_mean, a.dprev_var);          \
     launch(group_bwd_apply_kernel<TY>, apply_grid(rows * (a.D / Vec<TY>::kN)), 256, 0, (void*)s, (const TY*)dy,        \
            (const TY*)x, (TY*)dx, gsb, gsl, xsb, xsl, dsb, dsl, a.L, a.D, a.G, rows, a.cumrstd, a.group_mean, dux, dvx, \

@@ -1,5 +1,5 @@
 """TimestepNorm, per feature and per group, forward and backward, and SequenceNorm at the edges of their splits over time:
-segments of at least 64 steps, tiles of 8 or 16 steps, 64 channels of a warp, 128 threads along time of a group.
+segments of at least 64 steps, tiles of 8 or 16 steps, 64 channels of a warp, 256 or 128 threads along time of a group.
 
 Reference: the running statistics written out in float64 as cumulative sums, and autograd through them.  fp32: sums of L
 values about a centre, a handful of approximate reciprocals and square roots (2^-22 each) per step: 1e-5 relative 2-norm;
@@ -36,6 +36,12 @@ def _reference(x, mask, count, mean, logv, weight, bias, groups, eps):
     (127, 2, 64, 4, torch.float32, False),         # fewer steps than threads along time
     (129, 1, 96, 3, torch.float32, True),
     (1100, 2, 128, 2, torch.bfloat16, False),      # nine steps per thread: a batch of loads and one over
+    (2200, 2, 128, 2, torch.bfloat16, False),      # the same with 256 threads along time
+    (255, 1, 64, 4, torch.float32, False),
+    (257, 1, 96, 3, torch.float32, True),
+    (127, 40, 64, 8, torch.float32, False),        # more pairs of groups than SMs: eight to a block, 128 threads along time
+    (129, 50, 96, 6, torch.float32, True),         # eight to a block, two of them there are not
+    (1100, 75, 64, 4, torch.bfloat16, False),
 ])
 def test_timestep_norm_tiles(length, bsz, dim, groups, dtype, masked):
     import fairseq_apollo_b200 as M

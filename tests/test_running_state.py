@@ -128,7 +128,7 @@ def _norm_call(form, gen, bsz, length, dim, count):
 
 @pytest.mark.parametrize("form,length,bsz,dim,split", [
     ("norm", 700, 2, 72, 0),          # several segments of at least 64 steps
-    ("group", 700, 2, 128, 0),        # 128 threads along time, the last ones without steps
+    ("group", 700, 2, 128, 0),        # 256 threads along time, the last ones without steps
     ("fused", 700, 2, 72, 3),         # a cluster of blocks
     ("fused", 100, 1, 32, 3),         # one block
     ("fused", 2200, 64, 96, 3),       # the scan of several launches
