@@ -34,29 +34,35 @@ bool mma_takes(int dtype, const StreamArgs& a, bool want_xn) {
          !(a.cplx && a.h_out && a.L % 32 != 0);   // (it cannot stop a state in mid-step; a real layer's head still runs there)
 }
 
-// (a part for the launch and, on the tensor-core kernel with complex poles, for filling the pipeline of its tiles; long
-// chains of the forms with a second output or a mask fall behind the short ones' rate)
+// (a part for the launch and, on the tensor-core kernel with complex poles, for its coefficients; long chains of the forms with
+// a second output or a mask fall behind the short ones' rate)
 double fused_us(int dtype, const StreamArgs& a, bool want_xn) {
   const double L = a.L, n = (double)a.B * a.D * a.L;
   if (mma_takes(dtype, a, want_xn)) {
     // (both a mask and the second output: 11 x 1894 x 464 153 us, 6 x 4999 x 2048 387, 16 x 4096 x 1024 257)
     if (a.mask && want_xn) return 15.0 + longer(65.0, 290e3, L, n);
-    const double fixed = a.cplx ? (want_xn ? 100.0 : 95.0) : want_xn ? 15.0 : a.mask ? 13.0 : 11.0;
-    const double chain = a.cplx ? (want_xn ? 41.0 : 38.0) : want_xn ? 44.0 : a.mask ? 42.0 : 30.0;
+    // (complex: 34 x 185 x 480 with the second output 76 us, 13 x 319 x 320 76, 9 x 2831 x 136 with it 205)
+    const double fixed = a.cplx ? 68.0 : want_xn ? 15.0 : a.mask ? 13.0 : 11.0;
+    const double chain = a.cplx ? (want_xn ? 46.0 : 36.0) : want_xn ? 44.0 : a.mask ? 42.0 : 30.0;
     const double rate = a.cplx ? (want_xn ? 300e3 : 480e3) : want_xn ? 500e3 : a.mask ? 520e3 : 600e3;
     const double far = L * 1e-3 * (a.cplx ? (want_xn ? 75.0 : 62.0) : want_xn || a.mask ? 50.0 : 34.0);
     const double near = fixed + longer(chain, rate, L, n);
-    return near > far ? near : far;
+    // (complex, once not every tile of 16 channels and 8 sequences has an SM: 26 x 443 x 1464 with the second output 217 us,
+    // 9 x 3282 x 1944 279)
+    const double tiles = ((a.D + 15) / 16) * (double)((a.B + 7) / 8);
+    const double crowd = a.cplx && tiles > 148.0 ? 66.0 + L * 1e-3 * (tiles > 300.0 ? 0.8 * tiles : want_xn ? 90.0 : 65.0) : 0.0;
+    return fmax(near, fmax(far, crowd));
   }
-  // The streamed chain: ns a position by the blocks (128 channels of a sequence) that share an SM.  With a second output 16 x 4096 x
-  // 1024 fp32 755 us, 31 x 2094 x 624 673, 58 x 530 x 960 fp16 163; without 58 x 530 x 960 114, 27 x 1781 x 1296 with a state 309.
-  const double per = ceil((double)a.B * ((a.D + 127) / 128) / 148.0 - 0.1), wide = dtype == MEGA_F32 ? 1.35 : 1.0;
-  const bool state = a.h_in || a.h_out;
-  double ns;
-  if (a.cplx) ns = want_xn ? (per < 2 ? (state ? 254.0 : 234.0) : per < 3 ? 440.0 : 123.0 * per * wide)
-                           : (per < 2 ? (state ? 254.0 : 171.0) : per < 3 ? 250.0 : 92.0 * per * wide);
-  else ns = want_xn ? (per < 2 ? 185.0 : per < 3 ? 335.0 : 100.0 * per) : per < 2 ? 138.0 : per < 3 ? 148.0 : 54.0 * per * wide;
-  return 8.0 + L * ns * 1e-3;
+  // The streamed chain: ns a position by the blocks (128 channels of a sequence) that share an SM, from 310 shapes of 36 to 885
+  // blocks and 64 to 3000 positions, to a tenth up to two blocks: 17 x 190 x 1024 fp32 27 us, 5 x 139 x 2000 fp16 with a state and
+  // the second output 24, 28 x 1486 x 488 fp32 with the second output 190; complex 41 x 335 x 128 64, 24 x 1213 x 976 301.
+  const double blocks = (double)a.B * ((a.D + 127) / 128) / 148.0, per = blocks <= 1.0 ? 1.0 : fmax(2.0, ceil(blocks - 0.2));
+  double ns = a.cplx ? (per < 2 ? 175.0 : per < 3 ? 250.0 : per < 4 ? 340.0 : 130.0 * per)
+                     : (per < 2 ? 125.0 : per < 3 ? 150.0 : per < 4 ? 195.0 : 78.0 * per);
+  if (a.h_in || a.h_out) ns *= 1.09;
+  if (a.mask) ns *= 1.03;
+  if (dtype == MEGA_F32 && want_xn && blocks > 1.5) ns *= 1.4;
+  return 4.0 * per + L * ns * 1e-3;
 }
 
 // The EMA of the normalised activations where TimestepNorm has left them.
@@ -83,7 +89,8 @@ double scan_us(int dtype, const ScanArgs& ea, bool want_xn) {
   // (padding masks: 33 x 1282 x 456 fp32 199 us, 16 x 4096 x 1024 fp16 475, with the second output 5 x 4079 x 536 201, complex
   // 1 x 9084 x 728 152)
   const double masked = !ea.mask ? 1.0 : ea.cplx ? 1.15 : want_xn ? 1.45 : dtype == MEGA_F32 ? 1.2 : 1.1;
-  return one < 1e29 ? one : 45.0 + masked * n / (ea.cplx ? (want_xn ? 78e3 : 88e3) : (want_xn ? 145e3 : 165e3));
+  // (real: 10 x 985 x 1200 fp16 87 us, 60 x 2033 x 344 fp32 with the second output 268)
+  return one < 1e29 ? one : (ea.cplx ? 45.0 : 38.0) + masked * n / (ea.cplx ? (want_xn ? 78e3 : 88e3) : (want_xn ? 160e3 : 165e3));
 }
 
 // TimestepNorm in fp32, then the products of chunks (chunk_ema.cu): the normalised activations lie in scratch memory, for fp32
@@ -95,7 +102,7 @@ double chunk_us(int dtype, const ScanArgs& ea) {
   a.mask = nullptr;
   const double n = (double)a.B * a.D * a.L;
   if (dtype != MEGA_F32 && n > kWideMost) return 1e30;
-  return 28.0 + n / (dtype == MEGA_F32 ? 480e3 : 540e3) + chunk_ema_fwd_us(MEGA_F32, a);
+  return 12.0 + n / (dtype == MEGA_F32 ? 480e3 : 540e3) + chunk_ema_fwd_us(MEGA_F32, a);
 }
 bool norm_chunk_try(int dtype, const ScanArgs& ea, long long xsd, long long ysd, cudaStream_t s) {
   if (!rows_ok(dtype, ea.y, ea.ysb, ea.ysl, ysd) || (ea.xn && !rows_ok(dtype, ea.xn, ea.ysb, ea.ysl, ysd))) return false;
@@ -142,23 +149,26 @@ bool norm_ema_split_try(int dtype, const void* x, void* y, void* xn, long long x
   ea.cplx = a.cplx; ea.silu = a.silu;
   ea.prev_count = a.prev_count; ea.prev_mean = a.prev_mean; ea.prev_var = a.prev_var; ea.gamma = a.gamma; ea.beta = a.beta;
   ea.eps = a.eps; ea.count_out = a.count_out; ea.mean_out = a.mean_out; ea.var_out = a.var_out;
-  // (the margins: two more launches for the norm by itself, on a host that is not ahead of the device; the fixed 45 us of
-  // the scan's launches hold one; the models are good to a tenth)
+  // (the margins: more launches on a host that is not ahead of the device; the fixed parts of the forms in several launches hold
+  // some 10 us for it too; the models are good to a tenth: over 900 shapes this takes the fastest form or one within 3 % of that
+  // of the models before it in all but 9)
   // (a prompt that comes in chunks keeps to the tensor-core kernel, and its rounding, unless much is gained)
-  const bool prompt = dtype == MEGA_BF16 && a.h_out && !a.mask && !a.cplx;
+  const bool prompt = dtype == MEGA_BF16 && a.h_out && !a.mask && !a.cplx && mma_takes(dtype, a, xn != nullptr);
   const double fused = fused_us(dtype, a, xn != nullptr), scan = scan_us(dtype, ea, xn != nullptr) + (prompt ? 25.0 : 0.0),
                chain = mma_us(dtype, a, xn != nullptr) + 25.0;
   // The products of chunks behind TimestepNorm in bf16: for calls that would run on the tensor-core kernel in one of its two ways,
   // whose roundings these are too (complex 4 x 4096 x 1024 263 us fused, 103 so; real 142 and 94).
   const bool rounds = chain < 1e29 && (scan > 0.9 * fused || chain < scan);
-  const double chunks = rounds ? 35.0 + (double)a.B * a.D * a.L / 700e3 + chunk_ema_fwd_us(dtype, behind_norm(ea, ea.y)) : 1e30;
+  const double chunks = rounds ? 15.0 + (double)a.B * a.D * a.L / 700e3 + chunk_ema_fwd_us(dtype, behind_norm(ea, ea.y)) : 1e30;
   const double mma = chunks < chain ? chunks : chain;
   if (forced == 0) {   // (what stands in mean_out and the like once the norm has run is what the forms below write too)
     const double chunk = chunk_us(dtype, ea), by_scan = scan - (prompt ? 25.0 : 0.0);
     if ((chunk < 0.88 * (by_scan < mma ? by_scan : mma) && chunk < 0.88 * fused) || (chunk < 1e29 && g_options[OPT_CHUNK].load() == 2))
       if (norm_chunk_try(dtype, ea, xsd, ysd, s)) return true;
   }
-  if (forced == 0 && (scan < mma ? scan : mma) > 0.9 * fused) return false;
+  // (a scan in one launch is worth its estimate where that is a launch's fixed part: 28 x 66 x 88 fp32 9.2 us, as a chain 11.4)
+  const double n = (double)a.B * a.D * a.L, margin = n < 4e5 && scan < 45.0 ? 1.0 : 0.9;
+  if (forced == 0 && (scan < mma ? scan : mma) > margin * fused) return false;
   if (mma < scan && forced != 3) {
     void* mid = xn ? xn : y;
     ScanNormArgs na{};
