@@ -64,17 +64,19 @@ struct ChunkArgs {
 template <typename T>
 constexpr int kPartsOf = sizeof(T) == 4 ? 3 : std::is_same<T, __half>::value ? 2 : 1;
 
-// blocks of a channel: V, [U], T, G
+// blocks of a channel: V, [U], T (two), G
 template <bool kC>
 struct Blocks {
-  static constexpr int v = kC ? 4 : 2, t = 2, g = kC ? 4 : 2;
+  static constexpr int v = kC ? 4 : 2, g = kC ? 4 : 2;
 };
 
 template <typename In, typename Out, bool kC, int kMode, bool kMask, bool kLean = false>
 struct Form {
   static constexpr int kP = kPartsOf<In>;
+  static_assert(kMode != kBoth || (kP == 1 && !kC), "the sums and the outputs in one: what registers and shared memory hold");
+  static_assert(kMode != kGrad || kP > 1 || kC, "real one-part sums come with the outputs");
   // positions of a tile (what shared memory holds), and bytes of a row: eight rows hit different banks
-  static constexpr int kTile = (kP == 1 && kMode != kBoth && !(kMode == kGrad && kC)) || (kP == 2 && !kC && kMode < kGrad) ? 128 : 64;
+  static constexpr int kTile = kMode < kGrad && (kP == 1 || (kP == 2 && !kC)) ? 128 : 64;
   static constexpr int kRow = 2 * kTile + 16;
   static constexpr int kCh = kMode == kGrad && kP == 3 ? 8 : 16;   // channels of a block, and its warps
   static constexpr int kThreads = 32 * kCh;
@@ -876,7 +878,6 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask, kLean>::kThrea
             const int st = o >> 2, m = o & 3, i = 2 * k + (o & 1);
             if (kMode == kBoth) {
               enter[kMode == kBoth ? st : 0][k][0][m] = h[0][i];
-              if (kC) enter[kMode == kBoth ? st : 0][k][kRe - 1][m] = h[kRe - 1][i];
               if (k == 0 && !(o & 1)) odd = fmaf(v[st][0][m], 0.f, odd);
             }
             float &hr = h[0][i], &hi = h[kRe - 1][i], &sr = sn[0][i], &si = sn[kSens ? kRe - 1 : 0][i];
