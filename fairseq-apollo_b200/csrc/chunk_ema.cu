@@ -436,11 +436,23 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask, kLean>::kThrea
   Share<In, kCh, kTile> sh(s, tid, s.in, s.isb, s.isl, false);
   Share<In, kCh, kTile> sg(s, tid, s.beside, s.bsb, s.bsl, true);
   Share<Out, kCh, kTile> so(s, tid, a.y, a.ysb, a.ysl, false);
-  // the row of this lane's states, and the longest one
-  const int row = blockIdx.y * 8 + g, b = row / s.walked, seg = row - b * s.walked;
-  const bool live = b < a.B && d < a.D;
-  const int len = b < a.B ? min(s.T, a.L - seg * s.T) : 0;
-  const int most = __reduce_max_sync(0xffffffffu, len);
+  // the row of this lane's states (found again where it is asked for: that leaves registers to the walk), and the longest one
+  struct Row {
+    int b, seg, len;
+    bool live;
+  };
+  auto own_row = [&]() -> Row {
+    int y;
+    asm volatile("mov.u32 %0, %%ctaid.y;" : "=r"(y));
+    Row r;
+    r.b = (y * 8 + g) / s.walked;
+    r.seg = y * 8 + g - r.b * s.walked;
+    r.live = r.b < a.B && d < a.D;
+    r.len = r.b < a.B ? min(s.T, a.L - r.seg * s.T) : 0;
+    return r;
+  };
+  const Row row0 = own_row();
+  const int most = __reduce_max_sync(0xffffffffu, row0.len);
   const int steps = (most + 31) / 32, tiles = (most + kTile - 1) / kTile;
 
   const uint32_t stage = smem_u32(smem) + F::stage + tid * 16;
@@ -503,9 +515,10 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask, kLean>::kThrea
   }
 
   // states that the segment starts from
-  auto carry_at = [&](int at, int part) { return s.carry + (((size_t)(b * s.S + at) * s.parts + part) * a.D + d) * 16 + 2 * t; };
+  auto carry_at = [&](int b, int at, int part) { return s.carry + (((size_t)(b * s.S + at) * s.parts + part) * a.D + d) * 16 + 2 * t; };
   float h[kRe][4], sn[kSens ? kRe : 1][4];
-  auto start = [&]() {
+  auto start = [&](const Row& r) {
+    const int b = r.b, seg = r.seg;
 #pragma unroll
     for (int c = 0; c < kRe; ++c)
 #pragma unroll
@@ -513,7 +526,7 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask, kLean>::kThrea
         h[c][i] = 0.f;
         if (kSens) sn[kSens ? c : 0][i] = 0.f;
       }
-    if (!(kOuts || kSums) || !live) return;
+    if (!(kOuts || kSums) || !r.live) return;
     // (the first segment's too lies with the others, of one segment where h_out is h_in: that is written while this is read)
     const bool given = kMode == kEmit && a.h_in != nullptr;
     if (seg > 0 || (given && s.carry)) {
@@ -521,11 +534,11 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask, kLean>::kThrea
       for (int c = 0; c < kRe; ++c)
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-          const float2 v = __ldg(reinterpret_cast<const float2*>(carry_at(seg, c) + 8 * k));
+          const float2 v = __ldg(reinterpret_cast<const float2*>(carry_at(b, seg, c) + 8 * k));
           h[c][2 * k] = v.x;
           h[c][2 * k + 1] = v.y;
           if (kSens) {
-            const float2 u = __ldg(reinterpret_cast<const float2*>(carry_at(seg, kRe + c) + 8 * k));
+            const float2 u = __ldg(reinterpret_cast<const float2*>(carry_at(b, seg, kRe + c) + 8 * k));
             sn[kSens ? c : 0][2 * k] = u.x;
             sn[kSens ? c : 0][2 * k + 1] = u.y;
           }
@@ -542,7 +555,7 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask, kLean>::kThrea
       }
     }
   };
-  start();
+  start(row0);
   // q^16 h + v of pole i
   auto next = [&](int i, float& re, float& im, float vr, float vi) {
     if (kC) {
@@ -600,10 +613,10 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask, kLean>::kThrea
   const uint32_t frag_row = smem_u32(smem) + (warp * 8 + (lane & 7)) * kRow + (lane >> 4) * 16;
   const int swz = ((warp >> 2) & 3) << 5;
   unsigned char* mine = smem + (warp * 8 + g) * kRow + 4 * t;   // (of the rows g and g + 8: outputs)
-  const int final = kMode == kEmit && a.h_out != nullptr && live && seg == s.S - 1 ? (len - 1) / 32 : -1;   // step whose end leaves
+  const int final = kMode == kEmit && a.h_out != nullptr && row0.live && row0.seg == s.S - 1 ? (row0.len - 1) / 32 : -1;   // step whose end leaves
 
   // kStep steps of 32 positions at a time: their products do not wait for each other, only their states do
-  constexpr int kStep = kMode == kBoth || (kC && (kMode == kGrad || kP == 3)) ? 1 : 2;   // (what registers hold: a spill goes to L2 beside this much shared memory)
+  constexpr int kStep = kMode == kBoth || (kC && (kMode == kGrad || kP == 3)) ? 1 : 2;   // (what registers hold; at the cap of 128, 21 of the 50 forms spill 4 to 116 bytes all the same)
   auto multiply = [&](int tile) {
     const int buf = tile % F::kBufs * F::kIns * kP * kPlane;
     const int n = min(kTile / 32, steps - kTile / 32 * tile), last = final - kTile / 32 * tile;
@@ -803,6 +816,8 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask, kLean>::kThrea
           odd = fmaf(v[st][0][0][0], 0.f, fmaf(v[st][0][0][2], 0.f, odd));
           // (a state that is exported is that of the segment's last position, wherever in a step it lies: position by position)
           if (s0 + st == last) {
+            const Row r = own_row();
+            const int b = r.b, len = r.len;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               const int m = 8 * (i >> 1) + 2 * t + (i & 1);
@@ -1032,14 +1047,16 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask, kLean>::kThrea
 #pragma unroll
   for (int i = 0; i < 4 * kRe; ++i) z = fmaf(h[i >> 2][i & 3], 0.f, z);
   const unsigned odd = __ballot_sync(0xffffffffu, z != z);   // (of all lanes, also those without a row)
-  const bool odd_row = live && (odd >> (lane & 28) & 15u) != 0u;
+  const Row end = own_row();
+  const int b = end.b, seg = end.seg, len = end.len;
+  const bool odd_row = end.live && (odd >> (lane & 28) & 15u) != 0u;
   const bool again = kMode != kGrad && __any_sync(0xffffffffu, odd_row);
   if constexpr (kOuts) {
     __syncthreads();   // (the block's outputs are there)
     if (again && s.in != a.y) {   // (in place the inputs are gone: NaN from there on)
       const int first = seg * s.T;
       Out* y = reinterpret_cast<Out*>(a.y) + b * a.ysb + d;
-      if (odd_row) start();
+      if (odd_row) start(end);
       one_by_one<In, kC, false>(s, b, d, first, odd_row ? len : 0, most, h, sn, [&](int k, float v) {
         if (a.silu) v = silu_of<Out>(v);
         if ((k & 3) == t) Elem<Out>::st(y + (s.rev ? a.L - 1 - first - k : first + k) * a.ysl, v);
@@ -1055,17 +1072,17 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask, kLean>::kThrea
   }
   if constexpr (kMode == kLocal || kMode == kLocalSens) {   // what the segment behind it starts from
     if (again) {
-      if (odd_row) start();
+      if (odd_row) start(end);
       one_by_one<In, kC, kSens>(s, b, d, seg * s.T, odd_row ? len : 0, most, h, sn, [](int, float) {});
     }
-    if (live) {
+    if (end.live) {
 #pragma unroll
       for (int c = 0; c < kRe; ++c)
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-          *reinterpret_cast<float2*>(carry_at(seg + 1, c) + 8 * k) = make_float2(h[c][2 * k], h[c][2 * k + 1]);
+          *reinterpret_cast<float2*>(carry_at(b, seg + 1, c) + 8 * k) = make_float2(h[c][2 * k], h[c][2 * k + 1]);
           if (kSens)
-            *reinterpret_cast<float2*>(carry_at(seg + 1, kRe + c) + 8 * k) =
+            *reinterpret_cast<float2*>(carry_at(b, seg + 1, kRe + c) + 8 * k) =
                 make_float2(sn[kSens ? c : 0][2 * k], sn[kSens ? c : 0][2 * k + 1]);
         }
     }
@@ -1253,9 +1270,10 @@ bool envelope(int dtype, const ScanArgs& a) {
          a.N <= 16 && a.B <= 65535 && a.L >= 1 && a.L < 0x7fffff00 && pieces_ok(dtype, a.D);
 }
 
-// Times in us, fitted to a grid of 38 shapes on one B200 (1 to 64 sequences, 209 to 32768 positions, 128 to 2048 channels), to
-// a fifth.  Here: a part for the launches and the blocks' start, and ns per unit of pick()'s cost by the number of parts of a
-// value and the kind of poles.
+// Times in us, fitted to a grid of 38 shapes on one B200 (1 to 64 sequences, 209 to 32768 positions, 128 to 2048 channels).  Here:
+// a part for the launches and the blocks' start, some 10 us more of it than the device takes, for a host that is not far ahead;
+// and ns per unit of pick()'s cost by the number of parts of a value and the kind of poles, which over 600 more shapes is 4 to
+// 12 % off (standard deviation, by form).  So near a border the choice is between forms that differ by a tenth.
 double chunk_us(int dtype, const ScanArgs& a, bool bwd, bool lean, double cost, bool segmented) {
   static const double kFwd[2][3] = {{25., 32., 43.}, {44., 54., 64.}}, kBwd[2][3] = {{48., 75., 102.}, {97., 140., 168.}};
   static const double kLeanFwd[2] = {17., 22.5};
