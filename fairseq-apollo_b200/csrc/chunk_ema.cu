@@ -1249,8 +1249,7 @@ void run(const ChunkArgs& s, cudaStream_t st) {
 double pick(const ScanArgs& a, ChunkArgs& s) {
   const long long cols = (a.D + 15) / 16;
   double best = 1e30;
-  for (int S = 1; S <= 1024; ++S) {
-    const int t = (int)((((long long)a.L + S - 1) / S + 63) / 64 * 64);
+  auto consider = [&](int t) {
     const int n = (int)(((long long)a.L + t - 1) / t);
     const double rounds = ceil((double)(cols * (((long long)a.B * n + 7) / 8)) / 148.0);
     const double local = n > 1 ? ceil((double)(cols * (((long long)a.B * (n - 1) + 7) / 8)) / 148.0) : 0.;
@@ -1260,6 +1259,14 @@ double pick(const ScanArgs& a, ChunkArgs& s) {
       s.T = t;
       s.S = n;
     }
+  };
+  if (const int asked = g_options[OPT_CHUNK_STEPS].load(); asked > 0) {
+    consider((std::min(asked, 1 << 24) + 63) / 64 * 64);
+    return best;
+  }
+  for (int S = 1; S <= 1024; ++S) {
+    const int t = (int)((((long long)a.L + S - 1) / S + 63) / 64 * 64);
+    consider(t);
     if (t == 64) break;
   }
   return best;

@@ -18,7 +18,7 @@ namespace mega {
 extern std::atomic<uint64_t> g_launches;
 extern thread_local char g_cuda_err[256];
 extern std::atomic<int> g_options[8];
-enum { OPT_DISABLE_STREAM = 0, OPT_DISABLE_MMA = 1, OPT_MMA_TILE = 2, OPT_WAIT_LIMIT = 3, OPT_WITHHOLD_LOAD = 4, OPT_SPLIT = 5, OPT_CHUNK = 6 };
+enum { OPT_DISABLE_STREAM = 0, OPT_DISABLE_MMA = 1, OPT_MMA_TILE = 2, OPT_WAIT_LIMIT = 3, OPT_WITHHOLD_LOAD = 4, OPT_SPLIT = 5, OPT_CHUNK = 6, OPT_CHUNK_STEPS = 7 };
 // Name of the kernel family of the most recent launch (test aid): launch() sets "other", the
 // launchers of the named families overwrite it right after.
 extern std::atomic<const char*> g_last_kernel;

@@ -96,6 +96,7 @@ MEGA_API uint64_t mega_launch_count(void);
 #define MEGA_OPT_CHUNK 6 /* causal EMA and its backward as matrix products of chunks: 1: never, 2: wherever that form applies (3: bf16
                             forward in leading parts alone),
                             0: where it is estimated to be faster */
+#define MEGA_OPT_CHUNK_STEPS 7 /* steps of a segment of that form, rounded up to a multiple of 64; 0: as estimated */
 MEGA_API int mega_set_option(int key, int value);
 /*
  * Test aid: name of the kernel family of this process's most recent launch ("tsn_ema_mma tile=7 pipe=1",

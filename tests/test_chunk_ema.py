@@ -7,11 +7,16 @@ from _util import rel_l2
 
 pytestmark = pytest.mark.gpu
 
-# y and dx: one rounding of the result (2^-9, 2^-12); fp32: products of three bf16 parts leave 2^-24 of each term of sums of some
-# forty (taps, poles, omega x), 2e-7 in the 2-norm at most.  States: as fp32.  Sums over B L positions: 2^-24 times the square
-# root of the additions of a channel (under 64), in sums that cancel to a tenth
-LIMIT = {torch.float32: 5e-7, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}
+# y and dx: one rounding of the result (2^-8 or 2^-11 of a value at most, 1.7e-3 or 2.1e-4 in the 2-norm of many, so 2^-9 and 2^-12
+# beyond 1000 of them; leading parts alone are 3.3e-3 off in bf16 and would not pass); fp32: products of three bf16 parts leave 2^-24 of each term of sums of some forty (taps, poles, omega x), 2e-7 in the 2-norm for poles
+# that forget within the 512 positions between the corrections of q^16 (test_slow_poles: the others).  States: as fp32.  Sums over
+# B L positions: 2^-24 times the square root of the additions of a channel (under 64), in sums that cancel to a tenth
+LIMIT = {torch.float32: 5e-7, torch.bfloat16: 2.0 ** -9, torch.float16: 2.0 ** -12}
 SUMS = 5e-6
+
+
+def limit_of(dtype, values):
+    return LIMIT[dtype] * (2 if dtype != torch.float32 and values.numel() < 1000 else 1)
 
 
 @pytest.fixture
@@ -20,6 +25,7 @@ def forced():
     _lib.set_option(6, 2)
     yield _lib
     _lib.set_option(6, 0)
+    _lib.set_option(7, 0)
 
 
 def problem(gen, bsz, length, dim, ndim, dtype, cplx):
@@ -68,21 +74,21 @@ def test_against_float64(forced, bsz, length, dim, ndim, dtype, cplx):
     xc, dyc = x.cuda().transpose(1, 2), dy.cuda().transpose(1, 2)
     y = fwd(xc, *c)
     assert forced.last_kernel() == "chunk_ema"
-    assert rel_l2(y.transpose(1, 2), want) < LIMIT[dtype]
+    assert rel_l2(y.transpose(1, 2), want) < limit_of(dtype, x)
     got = bwd(dyc, xc, *c)
     assert forced.last_kernel() == "chunk_ema"
-    assert rel_l2(got[0].transpose(1, 2), leaves[0].grad) < LIMIT[dtype]
+    assert rel_l2(got[0].transpose(1, 2), leaves[0].grad) < limit_of(dtype, x)
     for name, a, b in zip(("p", "q", "g", "omega"), got[1:5], leaves[1:]):
         b = b.grad
         if a.is_complex():
             a, b = torch.view_as_real(a.cpu()), torch.view_as_real(b)
-        assert rel_l2(a, b) < SUMS or (a.cpu().double() - b).norm() < 1e-5, name   # (one position: dq is zero)
+        assert rel_l2(a, b) < SUMS, name
     # with a state, activated
     h = torch.randn(bsz, dim, ndim, dtype=q.dtype, generator=gen)
     wanted, last = recurrence(*[double(t) for t in (x, p, q, g, omega)], double(h))
     y, out = fwd(xc, *c, None, h.cuda(), True, silu=True)
     assert forced.last_kernel() == "chunk_ema"
-    assert rel_l2(y.transpose(1, 2), torch.nn.functional.silu(wanted)) < LIMIT[dtype]
+    assert rel_l2(y.transpose(1, 2), torch.nn.functional.silu(wanted)) < limit_of(dtype, x)
     if cplx:
         out, last = torch.view_as_real(out.cpu()), torch.view_as_real(last)
     assert rel_l2(out, last) < 5e-7
@@ -258,12 +264,14 @@ def test_behind_timestep_norm(forced, bsz, length, dim, dtype, cplx, normed):
 
 @pytest.mark.parametrize("cplx", [False, True])
 @pytest.mark.parametrize("slow", [1e-3, 1e-4])
-def test_slow_poles(forced, slow, cplx):
+@pytest.mark.parametrize("steps", [0, 4096, 16384])
+def test_slow_poles(forced, slow, cplx, steps):
     """Poles near the unit circle over many chunks: a power of a pole that is rounded alike in every chunk or segment would add up
     to 2^-25 / (1 - q^16), 6e-6 at 1e-4.  What is left is the rounding of each chunk's sum, of either sign: 2^-25 times the square
     root of the 1 / (32 slow) that a state holds, and 2^-25 for each of the 16 chunks, on average, between the corrections."""
     from fairseq_apollo_b200 import ops
     gen = torch.Generator().manual_seed(2)
+    forced.set_option(7, steps)
     bsz, length, dim, ndim = 2, 16384 - 5, 16, 4
     x, dy, p, _, g, omega = problem(gen, bsz, length, dim, ndim, torch.float32, cplx)
     q = 1 - slow * (torch.rand(dim, ndim, generator=gen) + 0.5)
@@ -352,3 +360,149 @@ def test_values_that_bf16_takes_for_infinite(forced, cplx):
         there = torch.zeros_like(a, dtype=torch.bool)
         there[row, :, ch] = True
         assert rel_l2(a[there] * 2.0 ** -64, b[there] * 2.0 ** -64) < 5e-7 and rel_l2(a[~there], b[~there]) < 5e-7
+
+
+# Long segments: from five tiles of 128 (or ten of 64) positions on, and a last one of a few positions or tiles
+LONG = [(192, 2, 1000, 24, 16), (640, 3, 1283, 16, 16), (704, 1, 1500, 40, 5), (1536, 9, 1536 - 7, 16, 16), (1088, 2, 1089, 8, 16)]
+
+
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("steps,bsz,length,dim,ndim", LONG)
+def test_many_tiles_of_a_segment(forced, steps, bsz, length, dim, ndim, dtype, cplx, masked):
+    """Slots, buffers and padding bits used again from the third tile on, outputs that leave while the next tile arrives, a state
+    exported from a late tile; forward with a state, and backward."""
+    from fairseq_apollo_b200 import ops
+    gen = torch.Generator().manual_seed(length)
+    x, dy, p, q, g, omega = problem(gen, bsz, length, dim, ndim, dtype, cplx)
+    mask = None
+    if masked:
+        mask = torch.rand(bsz, length, generator=gen) < 0.15
+        mask[-1, length - length // 3:] = True
+    forced.set_option(7, steps)
+    leaves = [double(t).requires_grad_(True) for t in (x, p, q, g, omega)]
+    seen = leaves[0] if mask is None else leaves[0].masked_fill(mask.unsqueeze(-1), 0.)
+    want = recurrence(seen, *leaves[1:4], torch.zeros(dim, dtype=torch.float64))[0] + leaves[4] * leaves[0]
+    want.backward(dy.double())
+    fwd, bwd = (ops.cema_forward, ops.cema_backward) if cplx else (ops.ema_forward, ops.ema_backward)
+    c = [t.cuda() for t in (p, q, g, omega)]
+    xc, dyc, mc = x.cuda().transpose(1, 2), dy.cuda().transpose(1, 2), None if mask is None else mask.cuda()
+    y = fwd(xc, *c, mc)
+    assert forced.last_kernel() == "chunk_ema"
+    assert rel_l2(y.transpose(1, 2), want) < LIMIT[dtype]
+    got = bwd(dyc, xc, *c, mc)
+    assert forced.last_kernel() == "chunk_ema"
+    assert rel_l2(got[0].transpose(1, 2), leaves[0].grad) < LIMIT[dtype]
+    for a, b in zip(got[1:5], leaves[1:]):
+        b = b.grad
+        if a.is_complex():
+            a, b = torch.view_as_real(a.cpu()), torch.view_as_real(b)
+        assert rel_l2(a, b) < SUMS
+    h = torch.randn(bsz, dim, ndim, dtype=q.dtype, generator=gen)
+    extra, last = recurrence(torch.zeros_like(seen), *[t.detach() for t in leaves[1:]], double(h))
+    _, own = recurrence(seen.detach(), *[t.detach() for t in leaves[1:]])
+    y, out = fwd(xc, *c, mc, h.cuda(), True)
+    assert forced.last_kernel() == "chunk_ema"
+    assert rel_l2(y.transpose(1, 2), want.detach() + extra) < LIMIT[dtype]
+    out, last = out.cpu(), last + own
+    if cplx:
+        out, last = torch.view_as_real(out), torch.view_as_real(last)
+    assert rel_l2(out, last) < (1e-6 if masked else 5e-7)   # (a state that only decays: 2^-25 for each of 32 chunks)
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+def test_many_tiles_in_leading_parts(forced, cplx):
+    from fairseq_apollo_b200 import ops
+    gen = torch.Generator().manual_seed(8)
+    x, _, p, q, g, omega = problem(gen, 3, 1500, 24, 16, torch.bfloat16, cplx)
+    want, _ = recurrence(*[double(t) for t in (x, p, q, g, omega)])
+    c = [t.cuda() for t in (p, q, g, omega)]
+    forced.set_option(6, 3)
+    forced.set_option(7, 704)
+    y = (ops.cema_forward if cplx else ops.ema_forward)(x.cuda().transpose(1, 2), *c)
+    assert forced.last_kernel() == "chunk_ema"
+    assert rel_l2(y.transpose(1, 2), want) < 1.5 * 2.0 ** -8
+
+
+def _normed_problem(gen, bsz, length, dim, mask):
+    from oracle import mega_oracle as O
+    pc = torch.full((bsz,), 3, dtype=torch.int64)
+    pm, pv = torch.randn(bsz, dim, generator=gen) * 0.1, torch.rand(bsz, dim, generator=gen) + 0.5
+    gamma, beta = torch.randn(dim, generator=gen) * 0.1 + 1, torch.randn(dim, generator=gen) * 0.1
+    norm = lambda x: O.timestep_norm(x.double(), pc, pm.double(), pv.double(), gamma.double(), beta.double(), mask,
+                                     acc_dtype=torch.float64)
+    return [t.cuda() for t in (pc, pm, pv, gamma, beta)], norm
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("normed", [False, True])
+@pytest.mark.parametrize("masked", [False, True])
+def test_many_tiles_behind_timestep_norm(forced, dtype, cplx, normed, masked):
+    """TimestepNorm with padding in the middle and at the end, which the products then know nothing of; long segments from fp32
+    scratch memory into each type."""
+    from fairseq_apollo_b200 import ops
+    gen = torch.Generator().manual_seed(17)
+    bsz, length, dim = 3, 1283, 40
+    x, _, p, q, g, omega = problem(gen, bsz, length, dim, 16, dtype, cplx)
+    mask = None
+    if masked:
+        mask = torch.rand(bsz, length, generator=gen) < 0.1
+        mask[-1, length - length // 4:] = True
+    if dtype == torch.bfloat16 and not cplx and not normed and not masked:
+        pytest.skip("another form's call")
+    stats, norm = _normed_problem(gen, bsz, length, dim, mask)
+    xn, cnt, mean, var = norm(x)[:4]
+    want, last = recurrence(xn, *[double(t) for t in (p, q, g, omega)])
+    forced.set_option(7, 704)
+    got = ops.tsn_ema_forward(x.cuda(), *stats, 1e-5, *[t.cuda() for t in (p, q, g, omega)], None if mask is None else mask.cuda(),
+                              want_state=not masked, want_normed=normed, complex_poles=cplx)
+    assert forced.last_kernel() == "chunk_ema"
+    limit = max(LIMIT[dtype], 4e-6)   # (the statistics: reciprocals and roots to 2^-22, sums of up to 1283 deviations)
+    assert rel_l2(got["y"], want) < limit
+    if normed:
+        assert rel_l2(got["xn"], xn) < limit
+    if not masked:
+        out = got["h"].cpu()
+        if cplx:
+            out, last = torch.view_as_real(out), torch.view_as_real(last)
+        assert rel_l2(out, last) < 4e-6
+    assert torch.equal(got["count"].cpu(), cnt) and rel_l2(got["mean"], mean) < 4e-6 and rel_l2(got["var"], var) < 4e-6
+
+
+def test_leading_parts_behind_timestep_norm():
+    """A bf16 call without a state that would run on the tensor cores: TimestepNorm in bf16, then the leading parts.  Its roundings:
+    the normalised activations (2^-9), matrices, states and outputs."""
+    from fairseq_apollo_b200 import _lib, ops
+    gen = torch.Generator().manual_seed(21)
+    bsz, length, dim = 22, 129, 1176
+    x, _, p, q, g, omega = problem(gen, bsz, length, dim, 16, torch.bfloat16, True)
+    stats, norm = _normed_problem(gen, bsz, length, dim, None)
+    xn = norm(x)[0]
+    want, _ = recurrence(xn, *[double(t) for t in (p, q, g, omega)])
+    got = ops.tsn_ema_forward(x.cuda(), *stats, 1e-5, *[t.cuda() for t in (p, q, g, omega)], None, want_normed=True, complex_poles=True)
+    assert _lib.last_kernel() == "chunk_ema"
+    assert rel_l2(got["y"], want) < 2 * 2.0 ** -8 and rel_l2(got["xn"], xn) < 2.0 ** -9
+
+
+@pytest.mark.parametrize("steps", [64, 1024])
+def test_complex_poles_over_many_segments(forced, steps):
+    """No mask, sequences cut into up to 47 segments, time-major memory: against the forms that walk position by position."""
+    from fairseq_apollo_b200 import ops
+    gen = torch.Generator().manual_seed(1)
+    x, dy, p, q, g, omega = problem(gen, 2, 3000, 16, 16, torch.float32, True)
+    forced.set_option(7, steps)
+    c = [t.cuda() for t in (p, q, g, omega)]
+    xt, dyc = x.cuda().transpose(0, 1).contiguous().permute(1, 2, 0), dy.cuda().transpose(1, 2)
+    y, grads = ops.cema_forward(xt, *c), ops.cema_backward(dyc, xt, *c)
+    assert forced.last_kernel() == "chunk_ema"
+    leaves = [double(t).requires_grad_(True) for t in (x, p, q, g, omega)]
+    want, _ = recurrence(*leaves)
+    want.backward(dy.double())
+    assert rel_l2(y.transpose(1, 2), want) < LIMIT[torch.float32] and rel_l2(grads[0].transpose(1, 2), leaves[0].grad) < LIMIT[torch.float32]
+    for a, b in zip(grads[1:5], leaves[1:]):
+        b = b.grad
+        if a.is_complex():
+            a, b = torch.view_as_real(a.cpu()), torch.view_as_real(b)
+        assert rel_l2(a, b) < SUMS
