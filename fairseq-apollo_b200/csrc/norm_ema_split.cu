@@ -150,8 +150,8 @@ bool norm_ema_split_try(int dtype, const void* x, void* y, void* xn, long long x
   ea.prev_count = a.prev_count; ea.prev_mean = a.prev_mean; ea.prev_var = a.prev_var; ea.gamma = a.gamma; ea.beta = a.beta;
   ea.eps = a.eps; ea.count_out = a.count_out; ea.mean_out = a.mean_out; ea.var_out = a.var_out;
   // (the margins: more launches on a host that is not ahead of the device; the fixed parts of the forms in several launches hold
-  // some 10 us for it too; the models are good to a tenth: over 900 shapes this takes the fastest form or one within 3 % of that
-  // of the models before it in all but 9)
+  // some 10 us for it too; the models are good to a tenth: of 900 shapes 6 take a form more than 3 % slower than
+  // the one they took before there were products of chunks)
   // (a prompt that comes in chunks keeps to the tensor-core kernel, and its rounding, unless much is gained)
   const bool prompt = dtype == MEGA_BF16 && a.h_out && !a.mask && !a.cplx && mma_takes(dtype, a, xn != nullptr);
   const double fused = fused_us(dtype, a, xn != nullptr), scan = scan_us(dtype, ea, xn != nullptr) + (prompt ? 25.0 : 0.0),
