@@ -3,8 +3,19 @@
 // allocation that suits their step loop (ptxas --register-usage-level) does not suit the others; for the
 // same reason the forms with tiles narrower than 56 channels are launched from mma_cl_narrow.cu.
 #include "mma_cl_kernel.cuh"
+#include "tmem_ema.cuh"
 
 namespace mega {
+
+// us of the fused pair with real poles as this kernel's chain, from 100 timings (4 to 64 sequences, 128 to 4096 positions, 256 to 2048
+// channels on one B200): ns a position by the tiles of 16 channels and 8 sequences.
+double mma_chain_us(const StreamArgs& a, bool xn) {
+  const double tiles = ((a.D + 15) / 16) * (double)((a.B + kSeq - 1) / kSeq);
+  const int v = (xn ? 1 : 0) + (a.mask ? 2 : 0);
+  static const double kFew[4] = {32., 49., 45., 58.}, kMore[4] = {53., 69., 70., 87.}, kMany[4] = {1., 1.35, 1.2, 1.55};
+  const double ns = tiles <= 148. ? kFew[v] : tiles <= 296. ? kMore[v] : 0.158 * tiles * kMany[v];
+  return (tiles <= 296. ? 11. : 25. + 0.03 * tiles) + a.L * ns * 1e-3 * (a.silu && !xn && !a.mask ? 1.04 : 1.);
+}
 
 // Envelope: bf16, channel stride 1, ndim <= 16, a padding mask only with real poles, a
 // normalised-copy output (strided like y) only together with the normalisation and distinct from x
@@ -37,6 +48,15 @@ bool mma_cl_try(int dtype, const void* x, void* y, void* xn, long long xsb, long
     return false;
   if (a_in.h_out && (a_in.L % kStep) != 0) return false;
   if ((a_in.B + kSeq - 1) / kSeq > 65535) return false;
+  // TimestepNorm -> EMA with real poles: statistics by scalar arithmetic and accumulators in tensor memory (16 x 4096 x 1024 92 us
+  // against 140, with the second output 110 against 208, masked 111 against 195), or this kernel's chain (64 x 32768 x 2048, where
+  // the power cap slows the other: 5.2 ms both)
+  if (norm && ema && !a_in.cplx) {
+    const int runs = forced == 162 ? 2 : forced == 164 ? 4 : forced == 168 ? 8 : 0;
+    if ((forced == 16 || runs > 0 || (forced == 0 && tmem_ema_us(a_in, want_xn) < 0.97 * mma_chain_us(a_in, want_xn))) &&
+        tmem_ema_try(dtype, x, y, xn, xsb, xsl, ysb, ysl, a_in, s, runs))
+      return true;
+  }
   // Tile width.  Large problems: 64 channels, or 56 when that fills the 148 SMs in fewer or
   // fuller waves (one CTA per SM; e.g. D = 2048 with 64 sequences: 37 x 8 = 296 CTAs = two full
   // waves).  Problems too small to give every SM a wide tile: 32 or 16 channels per CTA, so
@@ -153,6 +173,8 @@ cudaError_t mma_cl_read_device_error(int* v, bool reset) {
   int v2 = 0;
   cudaError_t e = read_device_error(v, reset);
   if (e == cudaSuccess) e = mma_cl_seg_read_device_error(&v2, reset);
+  if (e == cudaSuccess && *v == 0) *v = v2;
+  if (e == cudaSuccess) e = tmem_ema_read_device_error(&v2, reset);
   if (e == cudaSuccess && *v == 0) *v = v2;
   if (e == cudaSuccess) e = mma_cl_narrow_read_device_error(&v2, reset);
   if (e == cudaSuccess && *v == 0) *v = v2;

@@ -1,0 +1,821 @@
+// Fused TimestepNorm -> causal EMA for bf16 activations with contiguous channels and real poles: the statistics in plain fp32, a thread
+// per channel of a sequence, the EMA in tcgen05 products with accumulators in tensor memory.
+//
+// A block walks 16 channels of 8 sequences in tiles of 256 positions = 16 chunks of 16.  For one channel the (sequence, chunk) pairs
+// of a tile are the 128 rows of its products; with h the states that enter a chunk and everything else a matrix of the channel,
+//   local  v = V x         V (16 poles x 16): p q^(15-k)
+//   carry  h' = q^16 h + v
+//   output y = T x + G h   T (16 x 16): the taps, omega on the diagonal; G (16 x 16 poles): g q^(j+1)
+//   - the normalised rows go to shared memory as 16-byte pieces along time (K-major), which serve as A of T x and as B of V x;
+//   - V x is taken the other way round, poles on the rows: eight channels share an accumulator of 128 rows x 128
+//     columns, each channel's V (in tensor memory) being zero but for its own 16 rows.  So a thread holds one pole and reads a
+//     sequence's chunks as columns in the order of time: the carry stays inside it, one multiply-add per chunk;
+//   - the states go back as bf16, eight chunks to a 16-byte piece (MN-major), over the rows of x that are no longer needed, and G h is
+//     added to T x;
+//   - an output's thread holds a (sequence, chunk) row, reads two positions of the 16 channels at a time and writes 32 bytes each.
+// The statistics are a chain along time, 12 to 13 instructions a position.  One warp to a scheduler issues 0.4 of them a cycle (41 cycles
+// a position), so three groups of warps take the parts of 32 positions in turn: a group sums its part about a centre of its own before
+// the state of the part before is there, hands the state on, and normalises (28 cycles).  Warps: 12 of the statistics (ahead by up to
+// two tiles), 4 of states, 4 of outputs (8 with SiLU), one that fetches x (TMA), one that issues products, 2 for the normalised
+// activations as an output.  Everything is exchanged over mbarriers, the statistics over named barriers of two warps.
+//
+// What bounds it (16 x 4096 x 1024, 92 us against 140 in the forms of mma_cl_kernel.cuh; 67 without anything but the statistics): issue
+// slots and latency at 22 warps, 0.65 instructions per scheduler and cycle; the products' reads of shared memory 12 us, the outputs 4.
+// Two things that cost much: outputs that may stay in L1 (103 us; no_allocate), and code that does not fit the instruction cache (the
+// same walk in 250 KB of code 512 us; what is rare is out of line).  Over all SMs for long the power cap takes 12 % of the clock.
+//
+// What is not finite stays in its channel: a normalised value that is an infinity or a NaN (and whatever follows it) would make NaN of
+// the other seven channels' states, so it goes to the products as zero and the outputs from there on are written as NaN.
+#include <algorithm>
+#include <cmath>
+#include <type_traits>
+
+#include "common.cuh"
+#include "scratch.cuh"
+#include "split_mma.cuh"
+#include "stream_cl.cuh"
+#include "tma.cuh"
+#include "tmem_ema.cuh"
+#include "umma.cuh"
+
+namespace mega {
+
+namespace {
+
+constexpr int kQ = 8, kCh = 16, kTile = 256, kChunk = 16, kPart = 32;   // kPart: positions of a stage of x
+constexpr int kStages = 4, kStageBytes = 2 * kPart * kQ * kCh * 2;   // a stage: two parts
+constexpr int kPlane = 4096 + 16, kBuf = kCh * kPlane;   // rows of a channel (16 bytes on: eight channels hit different banks); of a tile
+constexpr int kMat = 1024;                               // T and G of a channel
+enum { kOffX = 0, kOffOp = kOffX + kStages * kStageBytes, kOffMat = kOffOp + 2 * kBuf, kOffInv = kOffMat + kCh * kMat,
+       kOffMail = kOffInv + 16 * 64 * 4, kOffTaps = kOffMail + 4 * 32 * 8, kOffBad = kOffTaps + kCh * 16 * 4, kOffBar = kOffBad + kQ * kCh * 4,
+       kOffEnd = kOffBar + 40 * 8 + 16 };
+// barriers
+enum { kXFull = 0, kXEmpty = kStages, kOpFull = 2 * kStages, kOpEmpty = kOpFull + 2, kHDone = kOpEmpty + 2, kHRead, kTDone, kYDone, kYRead, kReady, kEnd, kXnRead, kBars = kXnRead + 2 };
+static_assert(kBars <= 40, "barriers");
+// columns of tensor memory: V of 16 channels, two accumulators of local states, outputs
+constexpr int kColV = 0, kColH = 128, kColY = 256;
+// Warps: four of the states, four (with SiLU eight) of the outputs, kGroups times four of the statistics, x, products, and two for the
+// normalised activations where they are an output.
+constexpr int kGroups = 3;
+template <bool kSilu, bool kXn>
+struct Roles {
+  static constexpr int kOut = 4, kOuts = kSilu ? 2 : 1, kStats = kOut + 4 * kOuts, kLoad = kStats + 4 * kGroups, kMma = kLoad + 1, kCopy = kMma + 1;
+  static constexpr int kThreads = 32 * (kCopy + (kXn ? 2 : 0));
+};
+static_assert(kGroups == 3, "what a run leaves: a mean of each group");
+
+struct TmemArgs {
+  StreamArgs a;
+  __nv_bfloat16 *y, *xn;
+  long long ysb, ysl;
+  int wide;   // outputs: 32-byte pieces
+  // Sequences in runs: a work item is (run, group of sequences, tile of channels); blocks draw items in that order, and one starts
+  // from what the item of the run before has left behind its flag.
+  int tiles_d, per_run, runs, run_len;   // run_len: whole tiles
+  int* sched;                            // the next item; flags of the items (1: its state is there, 2: it gave up)
+  float4* state;                         // [B][D] the means behind the last three parts, squared deviations
+  float* h;                              // [B][D][16]
+};
+
+__device__ __forceinline__ bool tried(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok != 0;
+}
+// A wait that gives up raises `gone`; from then on no wait lasts, and everything runs out on whatever the buffers hold.
+// (out of line: the roles' code together has to stay within the instruction cache, about 32 KB)
+__device__ __noinline__ void wait_on(uint32_t bar, uint32_t parity, long long limit, volatile int* gone) {
+  const long long start = clock64();
+  while (!*gone) {
+#pragma unroll 1
+    for (int i = 0; i < 32; ++i) {   // (polling takes issue slots and shared memory from the other warps)
+      __nanosleep(40);
+      if (tried(bar, parity)) return;
+    }
+    if (clock64() - start > limit) {
+      g_device_error = 1;
+      *gone = 1;
+    }
+  }
+}
+__device__ __forceinline__ void arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ float minus_bf16(unsigned short x, float c) {   // x - c
+  float d;
+  asm("sub.f32.bf16 %0, %1, %2;" : "=f"(d) : "h"(x), "f"(c));
+  return d;
+}
+template <int N>
+__device__ __forceinline__ void landed(float (&v)[N]) {   // (the registers of a load from tensor memory, once it has been waited for)
+#pragma unroll
+  for (int i = 0; i < N; ++i) asm volatile("" : "+f"(v[i]));
+}
+__device__ __forceinline__ void store32(void* to, const uint32_t (&w)[8]) {
+  asm volatile("st.global.L1::no_allocate.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(to), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]),
+               "r"(w[5]), "r"(w[6]), "r"(w[7])
+               : "memory");
+}
+// 16 channels of a position, or eight where the others are not there
+__device__ __forceinline__ void store_channels(__nv_bfloat16* to, bool wide, bool both, const uint32_t (&w)[8]) {
+  if (wide) {
+    store32(to, w);
+    return;
+  }
+  asm volatile("st.global.L1::no_allocate.v4.b32 [%0], {%1,%2,%3,%4};" ::"l"(to), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
+  if (both)
+    asm volatile("st.global.L1::no_allocate.v4.b32 [%0], {%1,%2,%3,%4};" ::"l"(to + 8), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
+}
+__device__ __forceinline__ float ex2_approx(float v) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r;
+}
+// silu of two values: 1 + exp(-v) by way of a power of two, and the reciprocal to one unit
+__device__ __forceinline__ uint32_t silu_pair(float a, float b) {
+  const f32x2 v = pack2(a, b), x = mul2(v, pack2(-1.44269504f, -1.44269504f));
+  float xa, xb, da, db;
+  unpack2(x, xa, xb);
+  unpack2(add2(pack2(ex2_approx(xa), ex2_approx(xb)), pack2(1.f, 1.f)), da, db);
+  unpack2(mul2(v, pack2(rcp_approx(da), rcp_approx(db))), a, b);
+  return bf16_pair(a, b);
+}
+
+// byte of row (sequence, chunk) in a plane; a row's second eight values lie 128 bytes on
+__device__ __forceinline__ int row_of(int s, int chunk) { return (2 * s + (chunk >> 3)) * 256 + (chunk & 7) * 16; }
+
+// one position of a channel, dev from some c: the sums about c with it, and its normalised value
+__device__ __forceinline__ float normed(float dev, float inv, float eps, float w, float bb, float& s1, float& s2) {
+  s1 += dev;
+  s2 = fmaf(dev, dev, s2);
+  const float u = s1 * inv, v = fmaxf(fmaf(-u, u, fmaf(s2, inv, eps)), eps);
+  return fmaf(dev - u, rsqrt_approx(v) * w, bb);
+}
+// two positions, the later one's sums behind the earlier one's; what does not depend on the order in packed arithmetic
+__device__ __forceinline__ void normed2(float dev_a, float dev_b, f32x2 inv, float eps, f32x2 eps2, f32x2 w, f32x2 bb, float& s1, float& s2,
+                                        float& out_a, float& out_b) {
+  const float s1a = s1 + dev_a, s2a = fmaf(dev_a, dev_a, s2);
+  s1 = s1a + dev_b;
+  s2 = fmaf(dev_b, dev_b, s2a);
+  const f32x2 u = mul2(pack2(s1a, s1), inv), q = fma2(pack2(s2a, s2), inv, eps2);
+  float ua, ub, va, vb;
+  unpack2(u, ua, ub);
+  const f32x2 v = fma2(pack2(-ua, -ub), u, q);
+  unpack2(v, va, vb);
+  const f32x2 r = mul2(pack2(rsqrt_approx(fmaxf(va, eps)), rsqrt_approx(fmaxf(vb, eps))), w);
+  unpack2(fma2(sub2(pack2(dev_a, dev_b), u), r, bb), out_a, out_b);
+}
+// A part with padded positions (bits of pad; nothing but zeros comes of them) or without a mean to begin with (fresh: its first
+// value is the centre).  Returns the mean and the squared deviations behind it.
+__device__ __noinline__ float2 few(const unsigned char* from, const float* invs, unsigned char* to, unsigned pad, bool fresh, float c, float s2,
+                                   float eps, float w, float bb) {
+  float s1 = 0.f, u = 0.f;
+#pragma unroll 1
+  for (int i = 0; i < kPart; ++i) {
+    float out = 0.f;
+    if (!(pad >> i & 1u)) {
+      const unsigned short v = *reinterpret_cast<const unsigned short*>(from + i * (kQ * kCh * 2));
+      if (fresh) c = __uint_as_float((uint32_t)v << 16);
+      fresh = false;
+      out = normed(minus_bf16(v, c), invs[i], eps, w, bb, s1, s2);
+      u = s1 * invs[i];
+    }
+    *reinterpret_cast<__nv_bfloat16*>(to + (i >> 4) * 16 + (i >> 3 & 1) * 128 + (i & 7) * 2) = __float2bfloat16_rn(out);
+  }
+  return make_float2(c + u, fmaf(-u, s1, s2));
+}
+// What is not finite among a part's values: zero to the products, and noted.
+__device__ __noinline__ void odd_values(unsigned char* rows, int t0, bool live, int* first, volatile int* any) {
+#pragma unroll 1
+  for (int i = 0; i < kPart; ++i) {
+    unsigned short* at = reinterpret_cast<unsigned short*>(rows + (i >> 4) * 16 + (i >> 3 & 1) * 128) + (i & 7);
+    if ((*at & 0x7f80u) != 0x7f80u) continue;
+    *at = 0;
+    if (live) {
+      atomicMin(first, t0 + i);
+      *any = 1;
+    }
+  }
+}
+__device__ __forceinline__ void zero_row(unsigned char* to) {
+  *reinterpret_cast<uint4*>(to) = make_uint4(0u, 0u, 0u, 0u);
+  *reinterpret_cast<uint4*>(to + 128) = make_uint4(0u, 0u, 0u, 0u);
+}
+// What a channel's statistics leave behind: of the call, or for the next run (slot: of the group's mean).  Out of line, as are the others
+// above: nothing of it is held in registers beside the walk.
+__device__ __noinline__ void finish(const TmemArgs& t, int b, int d, float mean, float dev2, int seen) {
+  const StreamArgs& a = t.a;
+  const size_t at = (size_t)b * a.D + d;
+  const long long count = a.prev_count[b] + a.count_offset + seen;
+  a.mean_out[at] = seen > 0 ? mean : a.prev_mean[at];
+  a.var_out[at] = seen > 0 ? not_negative(dev2 / (float)count) : a.prev_var[at];
+  if (d == 0) a.count_out[b] = count;
+}
+__device__ __noinline__ void hand_on(const TmemArgs& t, int b, int d, int slot, float mean, float dev2) {   // (whole tiles: slots 0, 1, 2)
+  float* to = reinterpret_cast<float*>(t.state + (size_t)b * t.a.D + d);
+  to[slot] = mean;
+  if (slot == kGroups - 1) to[3] = dev2;
+}
+
+template <bool kSilu, bool kXn, bool kMask>
+__global__ void __launch_bounds__(Roles<kSilu, kXn>::kThreads, 1) tsn_ema_tmem_kernel(const __grid_constant__ CUtensorMap tx, const __grid_constant__ TmemArgs t) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  using R = Roles<kSilu, kXn>;
+  const StreamArgs& a = t.a;
+  const uint32_t base = smem_u32(smem);
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  int* bad = reinterpret_cast<int*>(smem + kOffBad);   // [sequence][channel]: first position that is not finite
+  volatile int* gone = reinterpret_cast<volatile int*>(smem + kOffBar + kBars * 8);
+  volatile int* any_bad = gone + 1;
+  uint32_t* tm_slot = reinterpret_cast<uint32_t*>(smem + kOffBar + kBars * 8 + 8);
+  auto bar = [&](int i) { return base + kOffBar + i * 8; };
+  const long long limit = a.wait_limit;
+  auto wait = [&](int i, int phase) {
+    if (!tried(bar(i), phase & 1)) wait_on(bar(i), phase & 1, limit, gone);
+  };
+  auto wait_all = [&](int i, int phase) {   // (a whole warp)
+    wait(i, phase);
+    __syncwarp();
+  };
+
+  int* drawn = reinterpret_cast<int*>(smem + kOffBar + kBars * 8 + 12);
+  if (tid == 0) *drawn = t.runs > 1 ? atomicAdd(t.sched, 1) : (int)blockIdx.x;
+  if (warp == 0) tm_alloc(smem_u32(tm_slot), 512);
+  if (tid == 32) {
+    auto init = [&](int i, int n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar(i)), "r"(n) : "memory"); };
+    for (int i = 0; i < kStages; ++i) {
+      init(kXFull + i, 1);
+      init(kXEmpty + i, 8);   // (two parts of four warps)
+    }
+    for (int i = 0; i < 2; ++i) {
+      init(kOpFull + i, 4 * kGroups);
+      init(kOpEmpty + i, 1);
+      init(kXnRead + i, 2);
+    }
+    init(kHDone, 1);
+    init(kHRead, 4);
+    init(kTDone, 1);
+    init(kYDone, 1);
+    init(kYRead, 4 * R::kOuts);
+    init(kReady, 4);
+    init(kEnd, 1);
+    *gone = 0;
+    *any_bad = 0;
+    mbar_fence_init();
+  }
+  if (tid < kQ * kCh) bad[tid] = 0x7fffffff;
+  tm_before();
+  __syncthreads();
+  tm_after();
+  const uint32_t tm = __shfl_sync(0xffffffffu, *tm_slot, 0);   // (uniform to the compiler: what issues products needs it in uniform registers)
+  const int item = *drawn, run = item / t.per_run, place = item - run * t.per_run;
+  const int d0 = place % t.tiles_d * kCh, b0 = place / t.tiles_d * kQ;
+  const int begin = run * t.run_len, len = min(a.L - begin, t.run_len);   // the block's positions
+  const int tiles = (len + kTile - 1) / kTile, parts = (len + kPart - 1) / kPart;
+  if (run > 0) {
+    if (tid == 0) {
+      const long long start = clock64();
+      int flag = 0;
+      while (true) {
+        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(flag) : "l"(t.sched + 1 + item - t.per_run) : "memory");
+        if (flag != 0) break;
+        __nanosleep(200);
+        if (clock64() - start > limit) {
+          g_device_error = 1;
+          break;
+        }
+      }
+      if (flag != 1) *gone = 1;
+    }
+    __syncthreads();
+  }
+
+  if (warp >= R::kStats && warp < R::kLoad) {
+    // ---- statistics: four threads per channel of a sequence, which take every fourth part ---------------------------
+    const int nw = warp & 3, own = (warp - R::kStats) >> 2, ch = lane & 15, s = 2 * nw + (lane >> 4), d = d0 + ch, b = b0 + s;
+    const bool live = d < a.D && b < a.B;
+    const float eps = a.eps, w = live ? __ldg(a.gamma + d) : 0.f, bb = live ? __ldg(a.beta + d) : 0.f;
+    const float n0 = b < a.B ? (float)(a.prev_count[b] + a.count_offset) : 1.f;
+    // the mean and the squared deviations so far, as handed from part to part
+    const size_t at = live ? (size_t)b * a.D + d : 0;
+    float mean = live ? a.prev_mean[at] : 0.f, dev2 = (live ? a.prev_var[at] : 1.f) * n0;
+    float c = mean;   // what deviations are taken from
+    if (run > 0 && live) {   // (so that the bits are those of one run)
+      const float4 m = __ldcg(t.state + at);
+      mean = m.z;
+      dev2 = m.w;
+      c = own == 0 ? m.x : own == 1 ? m.y : m.z;
+    }
+    // values that are not finite come with sums that are not, unless the parameters make them
+    bool odd = live && !(eps >= 1e-12f && fabsf(w) <= 1e10f && fabsf(bb) <= 1e37f);
+    float* tab = reinterpret_cast<float*>(smem + kOffInv) + (4 * own + nw) * 64 + (lane >> 4) * 32;
+    float2* mail = reinterpret_cast<float2*>(smem + kOffMail) + nw * 32 + lane;
+    const unsigned char* from = smem + kOffX + nw * 64 + lane * 2;
+    const unsigned char* mrow = kMask && b < a.B ? a.mask + (size_t)b * a.L : nullptr;
+    auto mask_at = [&](int part) -> unsigned {   // bit i: the part's position i is padded, of the lane's sequence
+      const int t0 = part * kPart;
+      if constexpr (kMask) {
+        const int p = t0 + ch;
+        const unsigned lo = __ballot_sync(0xffffffffu, mrow == nullptr || p >= len || __ldg(mrow + p) != 0);
+        const unsigned hi = __ballot_sync(0xffffffffu, mrow == nullptr || p + 16 >= len || __ldg(mrow + p + 16) != 0);
+        return lane & 16 ? __byte_perm(lo, hi, 0x7632) : __byte_perm(lo, hi, 0x5410);
+      } else {
+        return len - t0 >= 32 ? 0u : ~((1u << max(len - t0, 0)) - 1u);
+      }
+    };
+    const f32x2 eps2 = pack2(eps, eps), w2 = pack2(w, w), bb2 = pack2(bb, bb);
+    int seen = 0;
+    if (kMask)
+      for (int i = 0; i < own; ++i) seen += 32 - __popc(mask_at(i));
+    const int plain = kMask ? 0 : len / kPart;   // parts that are whole
+    // the mean and the squared deviations go from a part to the next by shared memory and a barrier of the two warps (every wait of
+    // theirs that could last is bounded, so both come)
+    const int mine = 1 + 4 * own + nw, theirs = 1 + 4 * ((own + 1) % kGroups) + nw;
+    int part = own;
+#pragma unroll 1
+    for (int tile = 0; tile < tiles; ++tile) {
+      if (tile >= 2) wait_all(kOpEmpty + (tile & 1), (tile >> 1) - 1);
+      unsigned char* plane = smem + kOffOp + (tile & 1) * kBuf + ch * kPlane + row_of(s, 0);
+      const int first = part, end = min(8 * tile + 8, parts);
+#pragma unroll 1
+      for (; part < end; part += kGroups) {
+        if (!kMask) seen = begin + part * kPart;
+        const unsigned pad = mask_at(part);
+        // 1 / count of the part's positions, for the whole warp
+        tab[ch] = rcp_approx(n0 + (float)(seen + __popc(~pad & ((2u << ch) - 1u))));
+        tab[ch + 16] = rcp_approx(n0 + (float)(seen + __popc(~pad & (~0u >> (15 - ch)))));
+        const float n = n0 + (float)seen;
+        wait_all(kXFull + (part >> 1) % kStages, (part >> 1) / kStages);
+        const unsigned char* v = from + (part & (2 * kStages - 1)) * (kStageBytes / 2);
+        unsigned char* to = plane + (part & 4) * 64 + (part & 3) * 32;
+        auto take = [&]() {   // the state that the part before left
+          if (part == 0) return;
+          asm volatile("bar.sync %0, 64;" ::"r"(mine) : "memory");
+          const float2 m = *mail;
+          mean = m.x;
+          dev2 = m.y;
+        };
+        auto give = [&]() {
+          if (part == parts - 1) return;
+          *mail = make_float2(mean, dev2);
+          asm volatile("bar.arrive %0, 64;" ::"r"(theirs) : "memory");
+        };
+        auto whole = [&](auto some) {   // some: positions are padded (zeros; the counts know of them)
+          constexpr bool kSome = decltype(some)::value;
+          // (the first time: any value of the channel is as good a centre as its mean)
+          if (!kSome && part < kGroups && run == 0) c = __uint_as_float((uint32_t)*reinterpret_cast<const unsigned short*>(v) << 16);
+          float dev[kPart], t1[2] = {0.f, 0.f}, t2[2] = {0.f, 0.f};
+#pragma unroll
+          for (int i = 0; i < kPart; ++i) {
+            dev[i] = minus_bf16(*reinterpret_cast<const unsigned short*>(v + i * (kQ * kCh * 2)), c);
+            if (kSome && (pad >> i & 1u)) dev[i] = 0.f;
+            t1[i & 1] += dev[i];
+            t2[i & 1] = fmaf(dev[i], dev[i], t2[i & 1]);
+          }
+          take();
+          const float off = mean - c;
+          float s1 = n * off, s2 = fmaf(s1, off, dev2);
+          const float e1 = s1 + (t1[0] + t1[1]), ue = e1 * tab[kPart - 1];
+          mean = c + ue;
+          dev2 = fmaf(-e1, ue, s2 + (t2[0] + t2[1]));
+          give();
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            float out[8];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              const ulonglong2 inv = reinterpret_cast<const ulonglong2*>(tab)[2 * q + j];
+#pragma unroll
+              for (int i = 0; i < 2; ++i) {
+                const int at = 8 * q + 4 * j + 2 * i;
+                normed2(dev[at], dev[at + 1], i ? inv.y : inv.x, eps, eps2, w2, bb2, s1, s2, out[4 * j + 2 * i], out[4 * j + 2 * i + 1]);
+                if (kSome && (pad >> at & 1u)) out[4 * j + 2 * i] = 0.f;
+                if (kSome && (pad >> at & 2u)) out[4 * j + 2 * i + 1] = 0.f;
+              }
+            }
+            *reinterpret_cast<uint4*>(to + (q >> 1) * 16 + (q & 1) * 128) =
+                make_uint4(bf16_pair(out[0], out[1]), bf16_pair(out[2], out[3]), bf16_pair(out[4], out[5]), bf16_pair(out[6], out[7]));
+          }
+        };
+        if (kMask ? !__any_sync(0xffffffffu, pad != 0u || n == 0.f) : part < plain && (part > 0 || !__any_sync(0xffffffffu, n == 0.f))) {
+          whole(std::false_type{});
+        } else if (kMask && !__any_sync(0xffffffffu, n == 0.f)) {
+          whole(std::true_type{});
+        } else {
+          take();
+          const float2 after = few(v, tab, to, pad, n == 0.f, mean, dev2, eps, w, bb);
+          mean = after.x;
+          dev2 = after.y;
+          give();
+        }
+        c = mean;
+        if (kMask) {
+          seen += 32 - __popc(pad);
+          if (part == parts - 1 && live && !*gone) finish(t, b, d, mean, dev2, seen);
+#pragma unroll 1
+          for (int i = 1; i < kGroups; ++i) seen += 32 - __popc(mask_at(part + i));
+        }
+        __syncwarp();
+        if (lane == 0) arrive(bar(kXEmpty + (part >> 1) % kStages));
+      }
+      if (odd || !(fabsf(dev2) < 3e38f)) {
+#pragma unroll 1
+        for (int i = first; i < part; i += kGroups) odd_values(plane + (i & 4) * 64 + (i & 3) * 32, i * kPart, live, bad + s * kCh + ch, any_bad);
+      }
+      if (!kMask && end == parts && run < t.runs - 1 && live && !*gone) hand_on(t, b, d, part - parts, c, dev2);
+      if (end == parts && part - kGroups == parts - 1) {   // (behind the end: zeros)
+        if (!kMask && run == t.runs - 1 && live && !*gone) finish(t, b, d, mean, dev2, a.L);
+#pragma unroll 1
+        for (int r = 2 * ((parts - 1) & 7) + 2; r < 16; ++r) zero_row(plane + (r >> 3) * 256 + (r & 7) * 16);
+      }
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) arrive(bar(kOpFull + (tile & 1)));
+    }
+  } else if (warp < 4) {
+    // ---- states and outputs -------------------------------------------------------------------------------------
+    const int half = lane >> 4, pole = lane & 15;
+    const uint32_t quarter = tm + ((uint32_t)warp << 21);
+    // states of channel 2 warp + half, sequences 0 - 3 and 4 - 7, then of channel 8 + that: they take turns as the first of four
+    float q16 = 0.f, q16_other = 0.f, h[4][4];
+    auto turn_states = [&]() {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float v = h[0][i];
+        h[0][i] = h[1][i];
+        h[1][i] = h[2][i];
+        h[2][i] = h[3][i];
+        h[3][i] = v;
+      }
+    };
+    auto turn_pole = [&]() {
+      const float q = q16;
+      q16 = q16_other;
+      q16_other = q;
+    };
+#pragma unroll 1
+    for (int g = 0; g < 2; ++g) {   // the matrices of channel 8 g + 2 warp + half, from this lane's pole
+      const int ch = 8 * g + 2 * warp + half, d = d0 + ch;
+      const bool in = d < a.D && pole < a.N;
+      const size_t o = in ? (size_t)d * a.N + pole : 0;
+      const float p = in ? __ldg(a.p + o) : 0.f, q = in ? __ldg(a.q + o) : 0.f, gm = in ? __ldg(a.g + o) : 0.f;
+      double q2 = (double)q * q;
+      q2 *= q2;
+      q2 *= q2;
+      q16 = (float)(q2 * q2);
+      unsigned char* mat = smem + kOffMat + ch * kMat;
+      float* taps = reinterpret_cast<float*>(smem + kOffTaps) + ch * 16;
+      float pw = 1.f, vk[16];
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        vk[15 - e] = p * pw;
+        float tap = p * gm * pw;
+#pragma unroll
+        for (int m = 8; m > 0; m >>= 1) tap += __shfl_xor_sync(0xffffffffu, tap, m);
+        if (pole == e) taps[e] = e == 0 && d < a.D ? tap + __ldg(a.omega + d) : tap;
+        pw *= q;
+        *reinterpret_cast<__nv_bfloat16*>(mat + 512 + (e >> 3) * 256 + (pole >> 3) * 128 + (e & 7) * 16 + (pole & 7) * 2) =
+            __float2bfloat16_rn(gm * pw);
+      }
+      uint32_t words[8], mine[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) words[i] = bf16_pair(vk[2 * i], vk[2 * i + 1]);
+#pragma unroll 1
+      for (int j = 0; j < 8; ++j) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) mine[i] = j == 2 * warp + half ? words[i] : 0u;
+        tm_st8(quarter + kColV + 8 * (8 * g + j), mine);
+      }
+      __syncwarp();
+      float row[16];   // row `pole` of T
+#pragma unroll
+      for (int k = 0; k < 16; ++k) row[k] = k <= pole ? taps[max(pole - k, 0)] : 0.f;
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        *reinterpret_cast<uint4*>(mat + (pole >> 3) * 256 + i * 128 + (pole & 7) * 16) =
+            make_uint4(bf16_pair(row[8 * i], row[8 * i + 1]), bf16_pair(row[8 * i + 2], row[8 * i + 3]),
+                       bf16_pair(row[8 * i + 4], row[8 * i + 5]), bf16_pair(row[8 * i + 6], row[8 * i + 7]));
+#pragma unroll 1
+      for (int hf = 0; hf < 2; ++hf) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int sq = b0 + 4 * hf + i;
+          const size_t o = (size_t)sq * a.D + d;
+          h[0][i] = !in || sq >= a.B ? 0.f : run > 0 ? __ldcg(t.h + o * 16 + pole) : a.h_in ? a.h_in[o * a.N + pole] : 0.f;
+        }
+        turn_states();
+      }
+      turn_pole();
+    }
+    tm_wait_st();
+    tm_before();
+    fence_proxy_async();
+    __syncwarp();
+    if (lane == 0) arrive(bar(kReady));
+
+#pragma unroll 1
+    for (int tile = 0; tile < tiles; ++tile) {
+      unsigned char* op = smem + kOffOp + (tile & 1) * kBuf;
+      const int last = min(15, (len - tile * kTile + kChunk - 1) / kChunk - 1);   // the tile's last chunk
+#pragma unroll 1
+      for (int unit = 0; unit < 4; ++unit) {
+        const int g = unit >> 1, hf = unit & 1, ch = 8 * g + 2 * warp + half;
+        if (hf == 0) {
+          wait_all(kHDone, g);
+          tm_after();
+        }
+        unsigned char* to = op + ch * kPlane + (pole >> 3) * 128 + (pole & 7) * 16 + hf * 2048;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          float v[32];
+          tm_ld32(quarter + kColH + 64 * hf + 32 * j, v);
+          tm_wait_ld();
+          landed(v);
+          if (j == 0 && unit == 0) {   // (x is still read until then)
+            wait_all(kTDone, tile);
+            if (kXn) wait_all(kXnRead + (tile & 1), tile >> 1);
+          }
+          auto carry = [&](auto stops) {   // stops: chunks behind the last one, whose local states are zero, leave the states as they are
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              uint32_t w[8];
+              float hs = h[0][2 * j + i], enter = 0.f;
+#pragma unroll
+              for (int c = 0; c < 16; ++c) {
+                if (c & 1) w[c >> 1] = bf16_pair(enter, hs);
+                else enter = hs;
+                hs = fmaf(decltype(stops)::value && c > last ? 1.f : q16, hs, v[16 * i + c]);
+              }
+              h[0][2 * j + i] = hs;
+              *reinterpret_cast<uint4*>(to + (2 * j + i) * 512) = make_uint4(w[0], w[1], w[2], w[3]);
+              *reinterpret_cast<uint4*>(to + (2 * j + i) * 512 + 256) = make_uint4(w[4], w[5], w[6], w[7]);
+            }
+          };
+          if (last < 15) carry(std::true_type{});
+          else carry(std::false_type{});
+        }
+        if (hf) {
+          fence_proxy_async();
+          tm_before();
+          __syncwarp();
+          if (lane == 0) arrive(bar(kHRead));
+        }
+        turn_states();
+        if (hf) turn_pole();
+      }
+    }
+    const bool on = run < t.runs - 1;
+    if ((on || a.h_out) && !*gone) {
+#pragma unroll 1
+      for (int unit = 0; unit < 4; ++unit) {
+        const int ch = 8 * (unit >> 1) + 2 * warp + half, d = d0 + ch;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int s = 4 * (unit & 1) + i;
+          const size_t o = (size_t)(b0 + s) * a.D + d;
+          if (d < a.D && pole < a.N && b0 + s < a.B) {
+            if (on) t.h[o * 16 + pole] = h[0][i];
+            else a.h_out[o * a.N + pole] = bad[s * kCh + ch] < len ? __int_as_float(0x7fffffff) : h[0][i];
+          }
+        }
+        turn_states();
+      }
+    }
+  } else if (warp < R::kStats) {
+    // ---- outputs: a thread per sequence and chunk ----------------------------------------------------------------
+    const int half = lane >> 4, chunk = lane & 15, s_out = 2 * (warp & 3) + half, b = b0 + s_out;
+    const uint32_t quarter = tm + ((uint32_t)(warp & 3) << 21);
+    const int first = ((warp - R::kOut) >> 2) * (8 / R::kOuts);   // pairs of positions
+#pragma unroll 1
+    for (int tile = 0; tile < tiles; ++tile) {
+      const int t0 = tile * kTile + chunk * kChunk;
+      const long long row = (long long)b * t.ysb + (long long)(begin + t0) * t.ysl + d0;
+      wait_all(kYDone, tile);
+      tm_after();
+      const int rows = *gone ? 0 : a.B;   // (nothing is stored once a wait has run out)
+      const bool full = t.wide != 0 && b0 + kQ <= rows && (tile + 1) * kTile <= len;
+      __nv_bfloat16* to = t.y + row + 2 * first * t.ysl;
+#pragma unroll 1
+      for (int i = first; i < first + 8 / R::kOuts; ++i) {
+        float v[2 * kCh];
+#pragma unroll
+        for (int c = 0; c < kCh; ++c) tm_ld2(quarter + kColY + 16 * c + 2 * i, v + 2 * c);
+        tm_wait_ld();
+        landed(v);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          uint32_t w[8];
+#pragma unroll
+          for (int c = 0; c < 8; ++c) w[c] = kSilu ? silu_pair(v[4 * c + k], v[4 * c + 2 + k]) : bf16_pair(v[4 * c + k], v[4 * c + 2 + k]);
+          if (full) store32(to, w);
+          else if (b < rows && t0 + 2 * i + k < len) store_channels(to, t.wide != 0, d0 + 8 < a.D, w);
+          to += t.ysl;
+        }
+      }
+      tm_before();
+      __syncwarp();
+      if (lane == 0) arrive(bar(kYRead));
+      if (*any_bad && b < rows) {
+        for (int c = 0; c < kCh && d0 + c < a.D; ++c)
+          for (int k = max(bad[s_out * kCh + c] - t0, 2 * first); k < 2 * first + kChunk / R::kOuts && t0 + k < len; ++k) {
+            t.y[row + k * t.ysl + c] = __ushort_as_bfloat16(0x7fff);
+            if (kXn) t.xn[row + k * t.ysl + c] = __ushort_as_bfloat16(0x7fff);
+          }
+      }
+    }
+  } else if (warp == R::kLoad) {
+    // ---- x ------------------------------------------------------------------------------------------------------
+    if (lane == 0) {
+      prefetch_tensormap(&tx);
+      const int stages = (parts + 1) / 2;
+      int k = 0;
+      for (; k < stages; ++k) {
+        const int st = k % kStages;
+        if (k >= kStages) wait(kXEmpty + st, k / kStages - 1);
+        if (*gone) break;
+        uint64_t* full = reinterpret_cast<uint64_t*>(smem + kOffBar) + kXFull + st;
+        mbar_expect_tx(full, kStageBytes);
+        if (k != a.withhold_step) tma_load_3d(smem + kOffX + st * kStageBytes, &tx, d0, b0, begin + k * 2 * kPart, full);
+      }
+      if (*gone)   // (left early: what is on its way arrives first)
+        for (int i = max(k - kStages, 0); i < k; ++i)
+          if (i != a.withhold_step) {
+            const long long start = clock64();
+            while (!tried(bar(kXFull + i % kStages), i / kStages & 1) && clock64() - start < 2 * limit + 100000) {}
+          }
+    }
+  } else if (warp >= R::kCopy) {
+    // ---- the normalised activations as an output, before states take their place --------------------------------------
+    const int chunk = lane & 15;
+#pragma unroll 1
+    for (int tile = 0; kXn && tile < tiles; ++tile) {
+      const int t0 = tile * kTile + chunk * kChunk;
+      wait_all(kOpFull + (tile & 1), tile >> 1);
+      const int rows = *gone ? 0 : a.B;
+      const bool full = t.wide != 0 && b0 + kQ <= rows && (tile + 1) * kTile <= len;
+#pragma unroll 1
+      for (int i = 0; i < 8; ++i) {   // two sequences, four of their 16 positions
+        const int s = 4 * (warp & 1) + 2 * (i >> 2) + (lane >> 4), b = b0 + s, k0 = 4 * (i & 3);
+        const unsigned char* from = smem + kOffOp + (tile & 1) * kBuf + row_of(s, chunk) + (k0 >> 3) * 128 + (k0 & 4) * 2;
+        uint2 v[kCh];
+#pragma unroll
+        for (int c = 0; c < kCh; ++c) v[c] = *reinterpret_cast<const uint2*>(from + c * kPlane);
+        __nv_bfloat16* to = t.xn + (long long)b * t.ysb + (long long)(begin + t0 + k0) * t.ysl + d0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          uint32_t w[8];
+#pragma unroll
+          for (int c = 0; c < 8; ++c) w[c] = __byte_perm(k < 2 ? v[2 * c].x : v[2 * c].y, k < 2 ? v[2 * c + 1].x : v[2 * c + 1].y, k & 1 ? 0x7632 : 0x5410);
+          if (full) store32(to, w);
+          else if (b < rows && t0 + k0 + k < len) store_channels(to, t.wide != 0, d0 + 8 < a.D, w);
+          to += t.ysl;
+        }
+      }
+      __syncwarp();
+      if (lane == 0) arrive(bar(kXnRead + (tile & 1)));
+    }
+  } else if (umma_elect()) {
+    // ---- products -----------------------------------------------------------------------------------------------
+    constexpr uint32_t kLocal = umma_idesc(128, 128, false), kTaps = umma_idesc(128, 16, false), kStates = umma_idesc(128, 16, true);
+    wait(kReady, 0);
+    tm_after();
+    const uint64_t rows0 = umma_desc(base + kOffOp, 128, 256), mats0 = umma_desc(base + kOffMat, 128, 256);
+    auto local = [&](uint64_t op, int g) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) umma_tm(tm + kColH, tm + kColV + 64 * g + 8 * j, op + (8 * g + j) * kPlane / 16, kLocal, j > 0);
+      umma_commit(bar(kHDone));
+    };
+    auto outs = [&](uint64_t op, int g) {   // G h
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        umma(tm + kColY + 128 * g + 16 * j, op + (8 * g + j) * kPlane / 16, mats0 + ((8 * g + j) * kMat + 512) / 16, kStates, true);
+    };
+#pragma unroll 1
+    for (int tile = 0; tile < tiles; ++tile) {
+      const uint64_t op = rows0 + (tile & 1) * (kBuf / 16);
+      wait(kOpFull + (tile & 1), tile >> 1);
+      tm_after();
+      local(op, 0);
+      if (tile > 0) wait(kYRead, tile - 1);
+      tm_after();
+#pragma unroll
+      for (int j = 0; j < kCh; ++j) umma(tm + kColY + 16 * j, op + j * kPlane / 16, mats0 + j * kMat / 16, kTaps, false);
+      umma_commit(bar(kTDone));
+      wait(kHRead, 0);
+      tm_after();
+      local(op, 1);
+      outs(op, 0);
+      wait(kHRead, 1);
+      tm_after();
+      outs(op, 1);
+      umma_commit(bar(kYDone));
+      umma_commit(bar(kOpEmpty + (tile & 1)));
+    }
+    // (nothing may be under way when the block ends)
+    umma_commit(bar(kEnd));
+    const long long start = clock64();
+    while (!tried(bar(kEnd), 0) && clock64() - start < 2 * limit + 100000) {}
+  }
+  __syncwarp();
+  tm_before();
+  __syncthreads();
+  tm_after();
+  if (warp == 0) tm_free(tm, 512);
+  if (run < t.runs - 1 && tid == 0) {
+    __threadfence();
+    asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(t.sched + 1 + item), "r"(*gone ? 2 : 1) : "memory");
+  }
+}
+
+template <bool kSilu, bool kXn, bool kMask>
+void launch_form(const CUtensorMap& tx, const TmemArgs& t, cudaStream_t s) {
+  const unsigned grid = (unsigned)(t.per_run * t.runs);
+  launch(tsn_ema_tmem_kernel<kSilu, kXn, kMask>, grid, Roles<kSilu, kXn>::kThreads, kOffEnd, (void*)s, tx, t);
+}
+
+}  // namespace
+
+namespace {
+
+// us of a call in so many runs, from 200 timings (1 to 64 sequences, 128 to 32768 positions, 256 to 2048 channels on one B200): a
+// block's start and end 6, then ns a position whatever the block's share of the 128 pairs, and rounds of blocks over the SMs (several
+// of them: at the clock that the power cap leaves).
+double runs_us(const StreamArgs& a, bool xn, int runs) {
+  const double tiles = (double)((a.D + kCh - 1) / kCh) * ((a.B + kQ - 1) / kQ) * runs;
+  const int len = ((a.L + kTile - 1) / kTile + runs - 1) / runs * kTile;
+  double ns = a.silu ? (xn ? 31.5 : 28.) : xn ? 26. : 20.;
+  if (a.mask) ns += 4.5;
+  if (a.D % kCh) ns = std::max(ns, xn ? 41. : 28.5);   // (outputs in 16-byte pieces: 24 x 1500 x 1000 103 us, with the second one 138)
+  const double rounds = std::ceil(tiles / 148.);
+  return 4. + rounds * (6. + len * ns * (rounds > 2. ? 1.125e-3 : 1e-3));
+}
+// runs: what balances the blocks' rounds (16 x 8192 x 5120 in two: 4.5 rounds of the sequence for 5)
+int runs_of(const StreamArgs& a, bool xn) {
+  int best = 1;
+  if (a.mask) return best;   // (the positions that count are known to the run before alone)
+  double least = 0.95 * runs_us(a, xn, 1);
+  for (int n = 2; n <= 8; n *= 2)
+    if (const double us = runs_us(a, xn, n); a.L >= 1024 * n && us < least) {
+      least = us;
+      best = n;
+    }
+  return best;
+}
+
+}  // namespace
+
+double tmem_ema_us(const StreamArgs& a, bool xn) { return runs_us(a, xn, runs_of(a, xn)); }
+
+bool tmem_ema_try(int dtype, const void* x, void* y, void* xn, long long xsb, long long xsl, long long ysb, long long ysl,
+                  const StreamArgs& a, cudaStream_t s, int asked) {
+  if (dtype != MEGA_BF16 || a.cplx || a.N < 1 || a.N > 16 || a.D % 8 != 0 || (a.h_out && a.L % kChunk != 0) || a.L >= (1 << 24)) return false;
+  if (!aligned_to(y, 16) || (xn && !aligned_to(xn, 16)) || ysb % 8 != 0 || ysl % 8 != 0) return false;
+  const long long per_run = (long long)((a.D + kCh - 1) / kCh) * ((a.B + kQ - 1) / kQ);
+  if (per_run > (1 << 24)) return false;
+  CUtensorMap tx;
+  if (!make_tensor_map_3d(&tx, dtype, x, a.D, a.B, a.L, xsb, xsl, kCh, kQ, 2 * kPart, CU_TENSOR_MAP_SWIZZLE_NONE)) return false;
+  TmemArgs t{};
+  t.a = a;
+  t.y = reinterpret_cast<__nv_bfloat16*>(y);
+  t.xn = reinterpret_cast<__nv_bfloat16*>(xn);
+  t.ysb = ysb;
+  t.ysl = ysl;
+  t.wide = a.D % 16 == 0 && ysb % 16 == 0 && ysl % 16 == 0 && aligned_to(y, 32) && (!xn || aligned_to(xn, 32));
+  t.tiles_d = (a.D + kCh - 1) / kCh;
+  t.per_run = (int)per_run;
+  t.runs = asked > 0 && !a.mask ? asked : runs_of(a, xn != nullptr);
+  const int tiles = (a.L + kTile - 1) / kTile, run_tiles = (tiles + t.runs - 1) / t.runs;
+  t.runs = (tiles + run_tiles - 1) / run_tiles;
+  t.run_len = run_tiles * kTile;
+  auto go = [&]() {
+#define MEGA_TMEM(SILU, XN) (a.mask ? launch_form<SILU, XN, true>(tx, t, s) : launch_form<SILU, XN, false>(tx, t, s))
+    if (a.silu) xn ? MEGA_TMEM(true, true) : MEGA_TMEM(true, false);
+    else xn ? MEGA_TMEM(false, true) : MEGA_TMEM(false, false);
+#undef MEGA_TMEM
+  };
+  if (t.runs == 1) {
+    go();
+  } else {
+    const size_t flags = 1 + (size_t)per_run * t.runs, rows = (size_t)a.B * a.D;
+    Scratch sc(Scratch::padded(flags * 4) + Scratch::padded(rows * 16) + Scratch::padded(rows * 64), s);
+    if (!sc) return false;
+    t.sched = sc.take<int>(flags);
+    t.state = sc.take<float4>(rows);
+    t.h = sc.take<float>(rows * 16);
+    if (cudaMemsetAsync(t.sched, 0, flags * 4, s) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    go();
+  }
+  static const char* const kNames[9] = {"", "tsn_ema_mma tmem", "tsn_ema_mma tmem segmented runs=2", "tsn_ema_mma tmem segmented runs=3",
+                                        "tsn_ema_mma tmem segmented runs=4", "tsn_ema_mma tmem segmented runs=5", "tsn_ema_mma tmem segmented runs=6",
+                                        "tsn_ema_mma tmem segmented runs=7", "tsn_ema_mma tmem segmented runs=8"};
+  g_last_kernel.store(a.mask ? "tsn_ema_mma tmem mask" : kNames[std::min(t.runs, 8)], std::memory_order_relaxed);
+  return true;
+}
+
+cudaError_t tmem_ema_read_device_error(int* v, bool reset) { return read_device_error(v, reset); }
+
+}  // namespace mega

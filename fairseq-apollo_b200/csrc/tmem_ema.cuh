@@ -1,0 +1,17 @@
+// Interface of the fused TimestepNorm -> EMA kernel with accumulators in tensor memory (tmem_ema.cu).
+#pragma once
+#include <cuda_runtime.h>
+
+#include "stream_cl.cuh"
+
+namespace mega {
+
+// bf16, channel stride 1 (whole 16-byte pieces), real poles, ndim <= 16, L a multiple of 16 where a state is exported.  False, nothing
+// launched, outside of that.  runs: pieces of the sequence, taken one after the other by different blocks (0: as estimated).
+bool tmem_ema_try(int dtype, const void* x, void* y, void* xn, long long xsb, long long xsl, long long ysb, long long ysl,
+                  const StreamArgs& a, cudaStream_t s, int runs = 0);
+// Its estimated time.
+double tmem_ema_us(const StreamArgs& a, bool xn);
+cudaError_t tmem_ema_read_device_error(int* v, bool reset);
+
+}  // namespace mega

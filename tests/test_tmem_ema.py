@@ -1,0 +1,154 @@
+"""Fused TimestepNorm -> EMA with accumulators in tensor memory (bf16, real poles): edges of its tiles (16 channels, 8 sequences, 256
+positions in chunks of 16 and parts of 32), runs of a sequence, padding, values that are not finite, waits that run out."""
+import time
+
+import pytest
+import torch
+
+from _util import make_ema_params, rel_l2, right_pad_mask
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def option():
+    from fairseq_apollo_b200 import _lib
+    yield _lib.set_option
+    for key in (2, 3, 4):
+        _lib.set_option(key, 0)
+
+
+def _case(bsz, length, dim, ndim, state, masked, seed=0):
+    gen = torch.Generator().manual_seed(seed + length)
+    prm = make_ema_params(gen, dim, ndim)
+    x = (torch.randn(bsz, length, dim, generator=gen) * 1.1 - 0.3).to(torch.bfloat16)
+    count = torch.full((bsz,), 2, dtype=torch.int64)
+    count[0] = 0
+    stats = (count, torch.randn(bsz, dim, generator=gen) * 0.1 - 0.3, torch.rand(bsz, dim, generator=gen) + 0.5,
+             torch.randn(dim, generator=gen) * 0.1 + 1, torch.randn(dim, generator=gen) * 0.1)
+    h0 = torch.randn(bsz, dim, ndim, generator=gen) * 0.3 if state else None
+    mask = None
+    if masked:
+        mask = right_pad_mask(gen, bsz, length, 0.5)
+        mask[0, :min(3, length)] = True
+        mask[-1, min(70, length // 2):min(130, length)] = True
+    return x, stats, prm, h0, mask
+
+
+def _run(x, stats, prm, h0, mask, **kw):
+    from fairseq_apollo_b200 import ops
+    dev = lambda t: None if t is None else t.cuda()
+    p, q, g = ops.ema_coeffs(*[t.cuda() for t in prm[:4]])
+    return ops.tsn_ema_forward(x.cuda(), *[t.cuda() for t in stats], 1e-5, p, q, g, prm[4].cuda(), dev(mask), h_in=dev(h0), **kw)
+
+
+# Outputs: operands are bf16 (2^-9 each), sums fp32; the statistics are plain fp32 sums (1e-6 of the variance and less).
+@pytest.mark.parametrize("bsz,length,dim,ndim,state,normed,silu,masked,tile", [
+    (8, 256, 16, 16, False, False, False, False, 16),     # one whole tile
+    (8, 257, 16, 16, False, True, False, False, 16),      # one position of another one
+    (5, 31, 72, 16, False, False, True, False, 16),       # parts, channels and sequences that are not whole
+    (4, 33, 8, 1, False, True, True, False, 16),          # half a tile of channels, one pole
+    (9, 544, 40, 16, True, True, True, False, 16),        # states in and out
+    (4, 777, 24, 5, False, True, False, False, 16),
+    (8, 1, 16, 16, False, False, False, False, 16),
+    (16, 1024, 208, 16, True, False, False, False, 16),
+    (8, 1000, 64, 16, False, False, False, True, 16),     # padding
+    (6, 512, 40, 16, True, True, True, True, 16),
+    (5, 96, 24, 16, False, False, True, True, 16),
+    (8, 1024, 48, 16, True, False, False, False, 162),    # runs
+    (20, 2048 + 96, 40, 16, True, True, True, False, 164),
+    (9, 2048 + 17, 64, 7, False, False, True, False, 168),
+])
+def test_against_oracle(option, bsz, length, dim, ndim, state, normed, silu, masked, tile):
+    from fairseq_apollo_b200 import _lib
+    from oracle import mega_oracle as O
+    x, stats, prm, h0, mask = _case(bsz, length, dim, ndim, state, masked)
+    want = state and length % 32 == 0
+    option(2, tile)
+    r = _run(x, stats, prm, h0, mask, want_state=want, want_normed=normed, silu=silu)
+    name = _lib.last_kernel()
+    assert "tmem" in name and ("segmented" in name) == (tile > 100)
+    xn, cnt, mean, var = O.timestep_norm(x.float(), *stats, mask, acc_dtype=torch.float64)[:4]
+    y, h = O.ema_forward_recurrence(xn.transpose(1, 2), *prm, mask, h=h0, return_state=True, silu=silu)
+    assert rel_l2(r["y"].float(), y.transpose(1, 2)) < 6e-3
+    assert torch.equal(r["count"].cpu(), cnt)
+    assert rel_l2(r["mean"], mean) < 2e-6 and rel_l2(r["var"], var) < 2e-6
+    if want:
+        assert rel_l2(r["h"], h) < 6e-3
+    if normed:
+        assert rel_l2(r["xn"].float(), xn) < 4e-3
+        if masked:
+            assert (r["xn"].cpu()[mask] == 0).all()
+    assert _lib.device_error() == 0
+
+
+@pytest.mark.parametrize("tile", [16, 162])
+def test_long_sequence_far_from_zero(option, tile):
+    """Values about 100 with a deviation of 1: the statistics keep their accuracy over 16384 positions."""
+    from fairseq_apollo_b200 import _lib
+    from oracle import mega_oracle as O
+    x, stats, prm, h0, mask = _case(8, 16384, 16, 16, False, False, seed=5)
+    x = (x.float() + 100).to(torch.bfloat16)
+    stats[0].fill_(2)
+    option(2, tile)
+    r = _run(x, stats, prm, None, None, want_normed=True)
+    xn, _, mean, var = O.timestep_norm(x.float(), *stats, None, acc_dtype=torch.float64)[:4]
+    assert rel_l2(r["mean"], mean) < 1e-6 and rel_l2(r["var"], var) < 2e-5
+    assert rel_l2(r["xn"].float(), xn) < 4e-3
+    assert _lib.device_error() == 0
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), float("-inf")])
+@pytest.mark.parametrize("tile,at", [(16, 300), (16, 0), (162, 511)])
+def test_not_finite_stays_in_its_channel(option, value, tile, at):
+    option(2, tile)
+    x, stats, prm, h0, mask = _case(8, 1024, 48, 16, True, False, seed=2)
+    clean = _run(x, stats, prm, h0, mask, want_state=True, want_normed=True)
+    x[2, at, 21] = value
+    r = _run(x, stats, prm, h0, mask, want_state=True, want_normed=True)
+    rest = torch.ones(8, 48, dtype=torch.bool)
+    rest[2, 21] = False
+    for k in ("y", "xn"):
+        a, b = r[k].cpu().transpose(1, 2), clean[k].cpu().transpose(1, 2)
+        assert torch.equal(a[rest], b[rest]) and torch.equal(a[2, 21, :at], b[2, 21, :at])
+        assert not torch.isfinite(a[2, 21, at:].float()).any()
+    for k in ("h", "mean", "var"):
+        assert torch.equal(r[k].cpu()[rest], clean[k].cpu()[rest])
+    assert not torch.isfinite(r["h"][2, 21]).any() and not torch.isfinite(r["mean"][2, 21])
+
+
+@pytest.mark.parametrize("tile", [16, 164])
+def test_wait_that_runs_out(option, tile):
+    """x of 64 positions never arrives: the kernel gives up, says so, and the next call is as always."""
+    from fairseq_apollo_b200 import _lib
+    x, stats, prm, h0, mask = _case(8, 4096, 64, 16, False, False)
+    assert _lib.device_error(reset=True) == 0
+    option(2, tile)
+    good = _run(x, stats, prm, h0, mask)["y"]
+    option(3, 2_000_000)   # SM cycles, about a millisecond
+    option(4, 5)
+    start = time.time()
+    _run(x, stats, prm, h0, mask)
+    torch.cuda.synchronize()
+    assert time.time() - start < 5.0
+    assert _lib.device_error(reset=True) != 0
+    option(3, 0)
+    option(4, 0)
+    assert torch.equal(_run(x, stats, prm, h0, mask)["y"], good)
+    assert _lib.device_error() == 0
+
+
+def test_strides_and_views(option):
+    """Rows that are not 32-byte aligned, a time-major view, and outputs written over the inputs give what contiguous tensors give."""
+    from fairseq_apollo_b200 import _lib, ops
+    x, stats, prm, h0, mask = _case(8, 320, 32, 16, False, False)
+    option(2, 16)
+    want = _run(x, stats, prm, None, None)["y"]
+    wide = torch.zeros(8, 320, 40, dtype=torch.bfloat16)
+    wide[:, :, 8:] = x
+    major = x.transpose(0, 1).contiguous()
+    p, q, g = ops.ema_coeffs(*[t.cuda() for t in prm[:4]])
+    for v in (wide.cuda()[:, :, 8:], major.cuda().transpose(0, 1)):
+        r = ops.tsn_ema_forward(v, *[t.cuda() for t in stats], 1e-5, p, q, g, prm[4].cuda())["y"]
+        assert "tmem" in _lib.last_kernel()
+        assert torch.equal(r, want)
