@@ -52,9 +52,9 @@ bool mma_cl_try(int dtype, const void* x, void* y, void* xn, long long xsb, long
   // against 140, with the second output 110 against 208, masked 111 against 195), or this kernel's chain (64 x 32768 x 2048, where
   // the power cap slows the other: 5.2 ms both)
   if (norm && ema && !a_in.cplx) {
-    const int runs = forced == 162 ? 2 : forced == 164 ? 4 : forced == 168 ? 8 : 0;
-    if ((forced == 16 || runs > 0 || (forced == 0 && tmem_ema_us(a_in, want_xn) < 0.97 * mma_chain_us(a_in, want_xn))) &&
-        tmem_ema_try(dtype, x, y, xn, xsb, xsl, ysb, ysl, a_in, s, runs))
+    const int asked = forced == 14 ? 4 : forced == 16 ? 9 : forced == 162 ? 10 : forced == 164 ? 12 : forced == 168 ? 16 : 0;
+    if ((asked > 0 || (forced == 0 && tmem_ema_us(a_in, want_xn) < 0.97 * mma_chain_us(a_in, want_xn))) &&
+        tmem_ema_try(dtype, x, y, xn, xsb, xsl, ysb, ysl, a_in, s, asked))
       return true;
   }
   // Tile width.  Large problems: 64 channels, or 56 when that fills the 148 SMs in fewer or

@@ -36,19 +36,23 @@ bool mma_takes(int dtype, const StreamArgs& a, bool want_xn) {
 }
 
 // (a part for the launch and, on the tensor-core kernel with complex poles, for its coefficients; long chains of the forms with
-// a second output or a mask fall behind the short ones' rate)
+// a second output or a mask fall behind the short ones' rate.  With real poles mma_cl_try has a faster form since (tmem_ema.cu), whose
+// roundings are the same: these times are left to say which calls round their operands to bf16, the others' results stay)
 double fused_us(int dtype, const StreamArgs& a, bool want_xn) {
   const double L = a.L, n = (double)a.B * a.D * a.L;
-  if (mma_takes(dtype, a, want_xn) && !a.cplx) {
-    const double tmem = tmem_ema_us(a, want_xn), chain = mma_chain_us(a, want_xn);
-    return tmem < 0.97 * chain ? tmem : chain;   // (mma_cl_try)
-  }
   if (mma_takes(dtype, a, want_xn)) {
+    // (both a mask and the second output: 11 x 1894 x 464 153 us, 6 x 4999 x 2048 387, 16 x 4096 x 1024 257)
+    if (a.mask && want_xn) return 15.0 + longer(65.0, 290e3, L, n);
     // (complex: 34 x 185 x 480 with the second output 76 us, 13 x 319 x 320 76, 9 x 2831 x 136 with it 205)
-    const double near = 68.0 + longer(want_xn ? 46.0 : 36.0, want_xn ? 300e3 : 480e3, L, n), far = L * 1e-3 * (want_xn ? 75.0 : 62.0);
-    // (once not every tile of 16 channels and 8 sequences has an SM: 26 x 443 x 1464 with the second output 217 us, 9 x 3282 x 1944 279)
+    const double fixed = a.cplx ? 68.0 : want_xn ? 15.0 : a.mask ? 13.0 : 11.0;
+    const double chain = a.cplx ? (want_xn ? 46.0 : 36.0) : want_xn ? 44.0 : a.mask ? 42.0 : 30.0;
+    const double rate = a.cplx ? (want_xn ? 300e3 : 480e3) : want_xn ? 500e3 : a.mask ? 520e3 : 600e3;
+    const double far = L * 1e-3 * (a.cplx ? (want_xn ? 75.0 : 62.0) : want_xn || a.mask ? 50.0 : 34.0);
+    const double near = fixed + longer(chain, rate, L, n);
+    // (complex, once not every tile of 16 channels and 8 sequences has an SM: 26 x 443 x 1464 with the second output 217 us,
+    // 9 x 3282 x 1944 279)
     const double tiles = ((a.D + 15) / 16) * (double)((a.B + 7) / 8);
-    const double crowd = tiles > 148.0 ? 66.0 + L * 1e-3 * (tiles > 300.0 ? 0.8 * tiles : want_xn ? 90.0 : 65.0) : 0.0;
+    const double crowd = a.cplx && tiles > 148.0 ? 66.0 + L * 1e-3 * (tiles > 300.0 ? 0.8 * tiles : want_xn ? 90.0 : 65.0) : 0.0;
     return fmax(near, fmax(far, crowd));
   }
   // The streamed chain: ns a position by the blocks (128 channels of a sequence) that share an SM, from 310 shapes of 36 to 885
@@ -159,6 +163,9 @@ bool norm_ema_split_try(int dtype, const void* x, void* y, void* xn, long long x
   const bool rounds = chain < 1e29 && (scan > 0.9 * fused || chain < scan);
   const double chunks = rounds ? 15.0 + (double)a.B * a.D * a.L / 700e3 + chunk_ema_fwd_us(dtype, behind_norm(ea, ea.y)) : 1e30;
   const double mma = chunks < chain ? chunks : chain;
+  // (of what rounds to bf16 the fused kernel with accumulators in tensor memory, where it is the faster one: 8 x 8192 x 1024 with the
+  // second output and SiLU 253 us as norm and products of chunks, 199 so)
+  const bool whole = !a.cplx && mma_takes(dtype, a, xn != nullptr) && tmem_ema_us(a, xn != nullptr) < 0.95 * mma;
   if (forced == 0) {   // (what stands in mean_out and the like once the norm has run is what the forms below write too)
     const double chunk = chunk_us(dtype, ea), by_scan = scan - (prompt ? 25.0 : 0.0);
     if ((chunk < 0.88 * (by_scan < mma ? by_scan : mma) && chunk < 0.88 * fused) || (chunk < 1e29 && g_options[OPT_CHUNK].load() == 2))
@@ -167,6 +174,7 @@ bool norm_ema_split_try(int dtype, const void* x, void* y, void* xn, long long x
   // (a scan in one launch is worth its estimate where that is a launch's fixed part: 28 x 66 x 88 fp32 9.2 us, as a chain 11.4)
   const double n = (double)a.B * a.D * a.L, margin = n < 4e5 && scan < 45.0 ? 1.0 : 0.9;
   if (forced == 0 && (scan < mma ? scan : mma) > margin * fused) return false;
+  if (forced == 0 && mma < scan && whole) return false;
   if (mma < scan && forced != 3) {
     void* mid = xn ? xn : y;
     ScanNormArgs na{};

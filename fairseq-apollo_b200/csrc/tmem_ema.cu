@@ -1,7 +1,7 @@
 // Fused TimestepNorm -> causal EMA for bf16 activations with contiguous channels and real poles: the statistics in plain fp32, a thread
 // per channel of a sequence, the EMA in tcgen05 products with accumulators in tensor memory.
 //
-// A block walks 16 channels of 8 sequences in tiles of 256 positions = 16 chunks of 16.  For one channel the (sequence, chunk) pairs
+// A block walks 16 channels of 8 (4) sequences in tiles of 256 positions = 16 chunks of 16.  For one channel the (sequence, chunk) pairs
 // of a tile are the 128 rows of its products; with h the states that enter a chunk and everything else a matrix of the channel,
 //   local  v = V x         V (16 poles x 16): p q^(15-k)
 //   carry  h' = q^16 h + v
@@ -42,27 +42,28 @@ namespace mega {
 
 namespace {
 
-constexpr int kQ = 8, kCh = 16, kTile = 256, kChunk = 16, kPart = 32;   // kPart: positions of a stage of x
-constexpr int kStages = 4, kStageBytes = 2 * kPart * kQ * kCh * 2;   // a stage: two parts
+constexpr int kMostQ = 8, kCh = 16, kTile = 256, kChunk = 16, kPart = 32;   // kPart: positions of a stage of x
+constexpr int kStages = 4;   // of x, two parts each
 constexpr int kPlane = 4096 + 16, kBuf = kCh * kPlane;   // rows of a channel (16 bytes on: eight channels hit different banks); of a tile
 constexpr int kMat = 1024;                               // T and G of a channel
-enum { kOffX = 0, kOffOp = kOffX + kStages * kStageBytes, kOffMat = kOffOp + 2 * kBuf, kOffInv = kOffMat + kCh * kMat,
-       kOffMail = kOffInv + 16 * 64 * 4, kOffTaps = kOffMail + 4 * 32 * 8, kOffBad = kOffTaps + kCh * 16 * 4, kOffBar = kOffBad + kQ * kCh * 4,
+enum { kOffX = 0, kOffOp = kOffX + kStages * 2 * kPart * kMostQ * kCh * 2, kOffMat = kOffOp + 2 * kBuf, kOffInv = kOffMat + kCh * kMat,
+       kOffMail = kOffInv + 16 * 64 * 4, kOffTaps = kOffMail + 4 * 32 * 8, kOffBad = kOffTaps + kCh * 16 * 4, kOffBar = kOffBad + kMostQ * kCh * 4,
        kOffEnd = kOffBar + 40 * 8 + 16 };
 // barriers
 enum { kXFull = 0, kXEmpty = kStages, kOpFull = 2 * kStages, kOpEmpty = kOpFull + 2, kHDone = kOpEmpty + 2, kHRead, kTDone, kYDone, kYRead, kReady, kEnd, kXnRead, kBars = kXnRead + 2 };
 static_assert(kBars <= 40, "barriers");
 // columns of tensor memory: V of 16 channels, two accumulators of local states, outputs
 constexpr int kColV = 0, kColH = 128, kColY = 256;
-// Warps: four of the states, four (with SiLU eight) of the outputs, kGroups times four of the statistics, x, products, and two for the
-// normalised activations where they are an output.
-constexpr int kGroups = 3;
-template <bool kSilu, bool kXn>
+// kQ: sequences of a block, eight or (few of them: more blocks, each with half of the work) four.
+// Warps: four of the states, four or (SiLU; four sequences, of which half of the warps have rows) eight of the outputs, twelve of the
+// statistics in groups, x, products, and two for the normalised activations where they are an output.
+template <int kQ, bool kSilu, bool kXn>
 struct Roles {
-  static constexpr int kOut = 4, kOuts = kSilu ? 2 : 1, kStats = kOut + 4 * kOuts, kLoad = kStats + 4 * kGroups, kMma = kLoad + 1, kCopy = kMma + 1;
+  static constexpr int kPer = kQ / 2, kGroups = 12 / kPer;   // warps of a group of the statistics (two sequences each), groups
+  static constexpr int kOut = 4, kOuts = kSilu || kQ == 4 ? 2 : 1, kStats = kOut + 4 * kOuts, kLoad = kStats + 12, kMma = kLoad + 1, kCopy = kMma + 1;
   static constexpr int kThreads = 32 * (kCopy + (kXn ? 2 : 0));
+  static constexpr int kStep = kQ * kCh * 2, kStageBytes = 2 * kPart * kStep;   // bytes from a position of x to the next; of a stage
 };
-static_assert(kGroups == 3, "what a run leaves: a mean of each group");
 
 struct TmemArgs {
   StreamArgs a;
@@ -168,14 +169,14 @@ __device__ __forceinline__ void normed2(float dev_a, float dev_b, f32x2 inv, flo
 }
 // A part with padded positions (bits of pad; nothing but zeros comes of them) or without a mean to begin with (fresh: its first
 // value is the centre).  Returns the mean and the squared deviations behind it.
-__device__ __noinline__ float2 few(const unsigned char* from, const float* invs, unsigned char* to, unsigned pad, bool fresh, float c, float s2,
+__device__ __noinline__ float2 few(const unsigned char* from, int step, const float* invs, unsigned char* to, unsigned pad, bool fresh, float c, float s2,
                                    float eps, float w, float bb) {
   float s1 = 0.f, u = 0.f;
 #pragma unroll 1
   for (int i = 0; i < kPart; ++i) {
     float out = 0.f;
     if (!(pad >> i & 1u)) {
-      const unsigned short v = *reinterpret_cast<const unsigned short*>(from + i * (kQ * kCh * 2));
+      const unsigned short v = *reinterpret_cast<const unsigned short*>(from + i * step);
       if (fresh) c = __uint_as_float((uint32_t)v << 16);
       fresh = false;
       out = normed(minus_bf16(v, c), invs[i], eps, w, bb, s1, s2);
@@ -212,16 +213,17 @@ __device__ __noinline__ void finish(const TmemArgs& t, int b, int d, float mean,
   a.var_out[at] = seen > 0 ? not_negative(dev2 / (float)count) : a.prev_var[at];
   if (d == 0) a.count_out[b] = count;
 }
-__device__ __noinline__ void hand_on(const TmemArgs& t, int b, int d, int slot, float mean, float dev2) {   // (whole tiles: slots 0, 1, 2)
+__device__ __noinline__ void hand_on(const TmemArgs& t, int b, int d, int slot, float mean, float dev2) {   // (whole tiles, three groups: slots 0, 1, 2)
   float* to = reinterpret_cast<float*>(t.state + (size_t)b * t.a.D + d);
   to[slot] = mean;
-  if (slot == kGroups - 1) to[3] = dev2;
+  if (slot == 2) to[3] = dev2;
 }
 
-template <bool kSilu, bool kXn, bool kMask>
-__global__ void __launch_bounds__(Roles<kSilu, kXn>::kThreads, 1) tsn_ema_tmem_kernel(const __grid_constant__ CUtensorMap tx, const __grid_constant__ TmemArgs t) {
+template <int kQ, bool kSilu, bool kXn, bool kMask>
+__global__ void __launch_bounds__(Roles<kQ, kSilu, kXn>::kThreads, 1) tsn_ema_tmem_kernel(const __grid_constant__ CUtensorMap tx, const __grid_constant__ TmemArgs t) {
   extern __shared__ __align__(128) unsigned char smem[];
-  using R = Roles<kSilu, kXn>;
+  using R = Roles<kQ, kSilu, kXn>;
+  constexpr int kGroups = R::kGroups, kPer = R::kPer, kStep = R::kStep;
   const StreamArgs& a = t.a;
   const uint32_t base = smem_u32(smem);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
@@ -246,10 +248,10 @@ __global__ void __launch_bounds__(Roles<kSilu, kXn>::kThreads, 1) tsn_ema_tmem_k
     auto init = [&](int i, int n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar(i)), "r"(n) : "memory"); };
     for (int i = 0; i < kStages; ++i) {
       init(kXFull + i, 1);
-      init(kXEmpty + i, 8);   // (two parts of four warps)
+      init(kXEmpty + i, 2 * kPer);   // (two parts)
     }
     for (int i = 0; i < 2; ++i) {
-      init(kOpFull + i, 4 * kGroups);
+      init(kOpFull + i, 12);
       init(kOpEmpty + i, 1);
       init(kXnRead + i, 2);
     }
@@ -257,7 +259,7 @@ __global__ void __launch_bounds__(Roles<kSilu, kXn>::kThreads, 1) tsn_ema_tmem_k
     init(kHRead, 4);
     init(kTDone, 1);
     init(kYDone, 1);
-    init(kYRead, 4 * R::kOuts);
+    init(kYRead, kPer * R::kOuts);
     init(kReady, 4);
     init(kEnd, 1);
     *gone = 0;
@@ -293,7 +295,7 @@ __global__ void __launch_bounds__(Roles<kSilu, kXn>::kThreads, 1) tsn_ema_tmem_k
 
   if (warp >= R::kStats && warp < R::kLoad) {
     // ---- statistics: four threads per channel of a sequence, which take every fourth part ---------------------------
-    const int nw = warp & 3, own = (warp - R::kStats) >> 2, ch = lane & 15, s = 2 * nw + (lane >> 4), d = d0 + ch, b = b0 + s;
+    const int nw = (warp - R::kStats) % kPer, own = (warp - R::kStats) / kPer, ch = lane & 15, s = 2 * nw + (lane >> 4), d = d0 + ch, b = b0 + s;
     const bool live = d < a.D && b < a.B;
     const float eps = a.eps, w = live ? __ldg(a.gamma + d) : 0.f, bb = live ? __ldg(a.beta + d) : 0.f;
     const float n0 = b < a.B ? (float)(a.prev_count[b] + a.count_offset) : 1.f;
@@ -309,7 +311,7 @@ __global__ void __launch_bounds__(Roles<kSilu, kXn>::kThreads, 1) tsn_ema_tmem_k
     }
     // values that are not finite come with sums that are not, unless the parameters make them
     bool odd = live && !(eps >= 1e-12f && fabsf(w) <= 1e10f && fabsf(bb) <= 1e37f);
-    float* tab = reinterpret_cast<float*>(smem + kOffInv) + (4 * own + nw) * 64 + (lane >> 4) * 32;
+    float* tab = reinterpret_cast<float*>(smem + kOffInv) + (kPer * own + nw) * 64 + (lane >> 4) * 32;
     float2* mail = reinterpret_cast<float2*>(smem + kOffMail) + nw * 32 + lane;
     const unsigned char* from = smem + kOffX + nw * 64 + lane * 2;
     const unsigned char* mrow = kMask && b < a.B ? a.mask + (size_t)b * a.L : nullptr;
@@ -331,7 +333,7 @@ __global__ void __launch_bounds__(Roles<kSilu, kXn>::kThreads, 1) tsn_ema_tmem_k
     const int plain = kMask ? 0 : len / kPart;   // parts that are whole
     // the mean and the squared deviations go from a part to the next by shared memory and a barrier of the two warps (every wait of
     // theirs that could last is bounded, so both come)
-    const int mine = 1 + 4 * own + nw, theirs = 1 + 4 * ((own + 1) % kGroups) + nw;
+    const int mine = 1 + kPer * own + nw, theirs = 1 + kPer * ((own + 1) % kGroups) + nw;
     int part = own;
 #pragma unroll 1
     for (int tile = 0; tile < tiles; ++tile) {
@@ -347,7 +349,7 @@ __global__ void __launch_bounds__(Roles<kSilu, kXn>::kThreads, 1) tsn_ema_tmem_k
         tab[ch + 16] = rcp_approx(n0 + (float)(seen + __popc(~pad & (~0u >> (15 - ch)))));
         const float n = n0 + (float)seen;
         wait_all(kXFull + (part >> 1) % kStages, (part >> 1) / kStages);
-        const unsigned char* v = from + (part & (2 * kStages - 1)) * (kStageBytes / 2);
+        const unsigned char* v = from + (part & (2 * kStages - 1)) * (R::kStageBytes / 2);
         unsigned char* to = plane + (part & 4) * 64 + (part & 3) * 32;
         auto take = [&]() {   // the state that the part before left
           if (part == 0) return;
@@ -368,7 +370,7 @@ __global__ void __launch_bounds__(Roles<kSilu, kXn>::kThreads, 1) tsn_ema_tmem_k
           float dev[kPart], t1[2] = {0.f, 0.f}, t2[2] = {0.f, 0.f};
 #pragma unroll
           for (int i = 0; i < kPart; ++i) {
-            dev[i] = minus_bf16(*reinterpret_cast<const unsigned short*>(v + i * (kQ * kCh * 2)), c);
+            dev[i] = minus_bf16(*reinterpret_cast<const unsigned short*>(v + i * kStep), c);
             if (kSome && (pad >> i & 1u)) dev[i] = 0.f;
             t1[i & 1] += dev[i];
             t2[i & 1] = fmaf(dev[i], dev[i], t2[i & 1]);
@@ -404,7 +406,7 @@ __global__ void __launch_bounds__(Roles<kSilu, kXn>::kThreads, 1) tsn_ema_tmem_k
           whole(std::true_type{});
         } else {
           take();
-          const float2 after = few(v, tab, to, pad, n == 0.f, mean, dev2, eps, w, bb);
+          const float2 after = few(v, R::kStep, tab, to, pad, n == 0.f, mean, dev2, eps, w, bb);
           mean = after.x;
           dev2 = after.y;
           give();
@@ -437,16 +439,15 @@ __global__ void __launch_bounds__(Roles<kSilu, kXn>::kThreads, 1) tsn_ema_tmem_k
     // ---- states and outputs -------------------------------------------------------------------------------------
     const int half = lane >> 4, pole = lane & 15;
     const uint32_t quarter = tm + ((uint32_t)warp << 21);
-    // states of channel 2 warp + half, sequences 0 - 3 and 4 - 7, then of channel 8 + that: they take turns as the first of four
-    float q16 = 0.f, q16_other = 0.f, h[4][4];
+    // states of channel 2 warp + half, four sequences at a time, then of channel 8 + that: they take turns as the first set
+    float q16 = 0.f, q16_other = 0.f, h[kQ / 2][4];
     auto turn_states = [&]() {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const float v = h[0][i];
-        h[0][i] = h[1][i];
-        h[1][i] = h[2][i];
-        h[2][i] = h[3][i];
-        h[3][i] = v;
+#pragma unroll
+        for (int k = 1; k < kQ / 2; ++k) h[k - 1][i] = h[k][i];
+        h[kQ / 2 - 1][i] = v;
       }
     };
     auto turn_pole = [&]() {
@@ -497,7 +498,7 @@ __global__ void __launch_bounds__(Roles<kSilu, kXn>::kThreads, 1) tsn_ema_tmem_k
             make_uint4(bf16_pair(row[8 * i], row[8 * i + 1]), bf16_pair(row[8 * i + 2], row[8 * i + 3]),
                        bf16_pair(row[8 * i + 4], row[8 * i + 5]), bf16_pair(row[8 * i + 6], row[8 * i + 7]));
 #pragma unroll 1
-      for (int hf = 0; hf < 2; ++hf) {
+      for (int hf = 0; hf < kQ / 4; ++hf) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int sq = b0 + 4 * hf + i;
@@ -519,8 +520,8 @@ __global__ void __launch_bounds__(Roles<kSilu, kXn>::kThreads, 1) tsn_ema_tmem_k
       unsigned char* op = smem + kOffOp + (tile & 1) * kBuf;
       const int last = min(15, (len - tile * kTile + kChunk - 1) / kChunk - 1);   // the tile's last chunk
 #pragma unroll 1
-      for (int unit = 0; unit < 4; ++unit) {
-        const int g = unit >> 1, hf = unit & 1, ch = 8 * g + 2 * warp + half;
+      for (int unit = 0; unit < kQ / 2; ++unit) {
+        const int g = unit / (kQ / 4), hf = unit % (kQ / 4), ch = 8 * g + 2 * warp + half;
         if (hf == 0) {
           wait_all(kHDone, g);
           tm_after();
@@ -555,24 +556,24 @@ __global__ void __launch_bounds__(Roles<kSilu, kXn>::kThreads, 1) tsn_ema_tmem_k
           if (last < 15) carry(std::true_type{});
           else carry(std::false_type{});
         }
-        if (hf) {
+        if (hf == kQ / 4 - 1) {
           fence_proxy_async();
           tm_before();
           __syncwarp();
           if (lane == 0) arrive(bar(kHRead));
         }
         turn_states();
-        if (hf) turn_pole();
+        if (hf == kQ / 4 - 1) turn_pole();
       }
     }
     const bool on = run < t.runs - 1;
     if ((on || a.h_out) && !*gone) {
 #pragma unroll 1
-      for (int unit = 0; unit < 4; ++unit) {
-        const int ch = 8 * (unit >> 1) + 2 * warp + half, d = d0 + ch;
+      for (int unit = 0; unit < kQ / 2; ++unit) {
+        const int ch = 8 * (unit / (kQ / 4)) + 2 * warp + half, d = d0 + ch;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const int s = 4 * (unit & 1) + i;
+          const int s = 4 * (unit % (kQ / 4)) + i;
           const size_t o = (size_t)(b0 + s) * a.D + d;
           if (d < a.D && pole < a.N && b0 + s < a.B) {
             if (on) t.h[o * 16 + pole] = h[0][i];
@@ -588,7 +589,7 @@ __global__ void __launch_bounds__(Roles<kSilu, kXn>::kThreads, 1) tsn_ema_tmem_k
     const uint32_t quarter = tm + ((uint32_t)(warp & 3) << 21);
     const int first = ((warp - R::kOut) >> 2) * (8 / R::kOuts);   // pairs of positions
 #pragma unroll 1
-    for (int tile = 0; tile < tiles; ++tile) {
+    for (int tile = 0; (warp & 3) < kPer && tile < tiles; ++tile) {
       const int t0 = tile * kTile + chunk * kChunk;
       const long long row = (long long)b * t.ysb + (long long)(begin + t0) * t.ysl + d0;
       wait_all(kYDone, tile);
@@ -635,8 +636,8 @@ __global__ void __launch_bounds__(Roles<kSilu, kXn>::kThreads, 1) tsn_ema_tmem_k
         if (k >= kStages) wait(kXEmpty + st, k / kStages - 1);
         if (*gone) break;
         uint64_t* full = reinterpret_cast<uint64_t*>(smem + kOffBar) + kXFull + st;
-        mbar_expect_tx(full, kStageBytes);
-        if (k != a.withhold_step) tma_load_3d(smem + kOffX + st * kStageBytes, &tx, d0, b0, begin + k * 2 * kPart, full);
+        mbar_expect_tx(full, R::kStageBytes);
+        if (k != a.withhold_step) tma_load_3d(smem + kOffX + st * R::kStageBytes, &tx, d0, b0, begin + k * 2 * kPart, full);
       }
       if (*gone)   // (left early: what is on its way arrives first)
         for (int i = max(k - kStages, 0); i < k; ++i)
@@ -655,8 +656,8 @@ __global__ void __launch_bounds__(Roles<kSilu, kXn>::kThreads, 1) tsn_ema_tmem_k
       const int rows = *gone ? 0 : a.B;
       const bool full = t.wide != 0 && b0 + kQ <= rows && (tile + 1) * kTile <= len;
 #pragma unroll 1
-      for (int i = 0; i < 8; ++i) {   // two sequences, four of their 16 positions
-        const int s = 4 * (warp & 1) + 2 * (i >> 2) + (lane >> 4), b = b0 + s, k0 = 4 * (i & 3);
+      for (int i = 0; i < kQ; ++i) {   // two sequences, four of their 16 positions
+        const int s = kPer * (warp & 1) + 2 * (i >> 2) + (lane >> 4), b = b0 + s, k0 = 4 * (i & 3);
         const unsigned char* from = smem + kOffOp + (tile & 1) * kBuf + row_of(s, chunk) + (k0 >> 3) * 128 + (k0 & 4) * 2;
         uint2 v[kCh];
 #pragma unroll
@@ -677,7 +678,7 @@ __global__ void __launch_bounds__(Roles<kSilu, kXn>::kThreads, 1) tsn_ema_tmem_k
     }
   } else if (umma_elect()) {
     // ---- products -----------------------------------------------------------------------------------------------
-    constexpr uint32_t kLocal = umma_idesc(128, 128, false), kTaps = umma_idesc(128, 16, false), kStates = umma_idesc(128, 16, true);
+    constexpr uint32_t kLocal = umma_idesc(128, 16 * kQ, false), kTaps = umma_idesc(128, 16, false), kStates = umma_idesc(128, 16, true);
     wait(kReady, 0);
     tm_after();
     const uint64_t rows0 = umma_desc(base + kOffOp, 128, 256), mats0 = umma_desc(base + kOffMat, 128, 256);
@@ -728,10 +729,10 @@ __global__ void __launch_bounds__(Roles<kSilu, kXn>::kThreads, 1) tsn_ema_tmem_k
   }
 }
 
-template <bool kSilu, bool kXn, bool kMask>
+template <int kQ, bool kSilu, bool kXn, bool kMask>
 void launch_form(const CUtensorMap& tx, const TmemArgs& t, cudaStream_t s) {
   const unsigned grid = (unsigned)(t.per_run * t.runs);
-  launch(tsn_ema_tmem_kernel<kSilu, kXn, kMask>, grid, Roles<kSilu, kXn>::kThreads, kOffEnd, (void*)s, tx, t);
+  launch(tsn_ema_tmem_kernel<kQ, kSilu, kXn, kMask>, grid, Roles<kQ, kSilu, kXn>::kThreads, kOffEnd, (void*)s, tx, t);
 }
 
 }  // namespace
@@ -741,22 +742,26 @@ namespace {
 // us of a call in so many runs, from 200 timings (1 to 64 sequences, 128 to 32768 positions, 256 to 2048 channels on one B200): a
 // block's start and end 6, then ns a position whatever the block's share of the 128 pairs, and rounds of blocks over the SMs (several
 // of them: at the clock that the power cap leaves).
-double runs_us(const StreamArgs& a, bool xn, int runs) {
-  const double tiles = (double)((a.D + kCh - 1) / kCh) * ((a.B + kQ - 1) / kQ) * runs;
+double runs_us(const StreamArgs& a, bool xn, int runs, int q) {
+  const double tiles = (double)((a.D + kCh - 1) / kCh) * ((a.B + q - 1) / q) * runs;
   const int len = ((a.L + kTile - 1) / kTile + runs - 1) / runs * kTile;
-  double ns = a.silu ? (xn ? 31.5 : 28.) : xn ? 26. : 20.;
-  if (a.mask) ns += 4.5;
-  if (a.D % kCh) ns = std::max(ns, xn ? 41. : 28.5);   // (outputs in 16-byte pieces: 24 x 1500 x 1000 103 us, with the second one 138)
-  const double rounds = std::ceil(tiles / 148.);
+  double ns = q == 4 ? (a.silu ? (xn ? 23.3 : 22.2) : xn ? 14.7 : 12.4) : a.silu ? (xn ? 31.5 : 28.) : xn ? 26. : 20.;
+  if (a.mask) ns += q == 4 ? 3.4 : 4.5;
+  // (outputs in 16-byte pieces: 24 x 1500 x 1000 103 us, with the second one 138, padded too 160)
+  if (a.D % kCh) ns = std::max(ns, (xn ? (a.mask ? 50. : 41.) : 28.5) * (q == 4 ? 0.7 : 1.));
+  const double rounds = std::max(std::ceil(tiles / 148.), (double)runs);   // (a sequence's runs follow one another)
   return 4. + rounds * (6. + len * ns * (rounds > 2. ? 1.125e-3 : 1e-3));
 }
+// sequences of a block: four where that gives all blocks an SM at once (a position takes 12 - 23 ns for 20 - 32: 8 x 8192 x 1024 112 us
+// against 176, 4 x 4096 x 1024 60 against 88; in two rounds 16 x 4096 x 1024 118 against 91)
+int sequences_of(const StreamArgs& a) { return (long long)((a.D + kCh - 1) / kCh) * ((a.B + 3) / 4) <= 148 ? 4 : 8; }
 // runs: what balances the blocks' rounds (16 x 8192 x 5120 in two: 4.5 rounds of the sequence for 5)
 int runs_of(const StreamArgs& a, bool xn) {
   int best = 1;
   if (a.mask) return best;   // (the positions that count are known to the run before alone)
-  double least = 0.95 * runs_us(a, xn, 1);
+  double least = 0.95 * runs_us(a, xn, 1, 8);
   for (int n = 2; n <= 8; n *= 2)
-    if (const double us = runs_us(a, xn, n); a.L >= 1024 * n && us < least) {
+    if (const double us = runs_us(a, xn, n, 8); a.L >= 1024 * n && us < least) {
       least = us;
       best = n;
     }
@@ -765,16 +770,20 @@ int runs_of(const StreamArgs& a, bool xn) {
 
 }  // namespace
 
-double tmem_ema_us(const StreamArgs& a, bool xn) { return runs_us(a, xn, runs_of(a, xn)); }
+double tmem_ema_us(const StreamArgs& a, bool xn) {
+  const int q = sequences_of(a);
+  return runs_us(a, xn, q == 8 ? runs_of(a, xn) : 1, q);
+}
 
 bool tmem_ema_try(int dtype, const void* x, void* y, void* xn, long long xsb, long long xsl, long long ysb, long long ysl,
                   const StreamArgs& a, cudaStream_t s, int asked) {
   if (dtype != MEGA_BF16 || a.cplx || a.N < 1 || a.N > 16 || a.D % 8 != 0 || (a.h_out && a.L % kChunk != 0) || a.L >= (1 << 24)) return false;
   if (!aligned_to(y, 16) || (xn && !aligned_to(xn, 16)) || ysb % 8 != 0 || ysl % 8 != 0) return false;
-  const long long per_run = (long long)((a.D + kCh - 1) / kCh) * ((a.B + kQ - 1) / kQ);
+  const int q = asked == 4 ? 4 : asked > 0 ? 8 : sequences_of(a);
+  const long long per_run = (long long)((a.D + kCh - 1) / kCh) * ((a.B + q - 1) / q);
   if (per_run > (1 << 24)) return false;
   CUtensorMap tx;
-  if (!make_tensor_map_3d(&tx, dtype, x, a.D, a.B, a.L, xsb, xsl, kCh, kQ, 2 * kPart, CU_TENSOR_MAP_SWIZZLE_NONE)) return false;
+  if (!make_tensor_map_3d(&tx, dtype, x, a.D, a.B, a.L, xsb, xsl, kCh, q, 2 * kPart, CU_TENSOR_MAP_SWIZZLE_NONE)) return false;
   TmemArgs t{};
   t.a = a;
   t.y = reinterpret_cast<__nv_bfloat16*>(y);
@@ -784,15 +793,17 @@ bool tmem_ema_try(int dtype, const void* x, void* y, void* xn, long long xsb, lo
   t.wide = a.D % 16 == 0 && ysb % 16 == 0 && ysl % 16 == 0 && aligned_to(y, 32) && (!xn || aligned_to(xn, 32));
   t.tiles_d = (a.D + kCh - 1) / kCh;
   t.per_run = (int)per_run;
-  t.runs = asked > 0 && !a.mask ? asked : runs_of(a, xn != nullptr);
+  t.runs = q == 4 || a.mask ? 1 : asked > 0 ? asked - 8 : runs_of(a, xn != nullptr);
   const int tiles = (a.L + kTile - 1) / kTile, run_tiles = (tiles + t.runs - 1) / t.runs;
   t.runs = (tiles + run_tiles - 1) / run_tiles;
   t.run_len = run_tiles * kTile;
   auto go = [&]() {
-#define MEGA_TMEM(SILU, XN) (a.mask ? launch_form<SILU, XN, true>(tx, t, s) : launch_form<SILU, XN, false>(tx, t, s))
+#define MEGA_TMEM_OF(Q, SILU, XN) (a.mask ? launch_form<Q, SILU, XN, true>(tx, t, s) : launch_form<Q, SILU, XN, false>(tx, t, s))
+#define MEGA_TMEM(SILU, XN) (q == 4 ? MEGA_TMEM_OF(4, SILU, XN) : MEGA_TMEM_OF(8, SILU, XN))
     if (a.silu) xn ? MEGA_TMEM(true, true) : MEGA_TMEM(true, false);
     else xn ? MEGA_TMEM(false, true) : MEGA_TMEM(false, false);
 #undef MEGA_TMEM
+#undef MEGA_TMEM_OF
   };
   if (t.runs == 1) {
     go();

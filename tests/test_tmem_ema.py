@@ -55,6 +55,10 @@ def _run(x, stats, prm, h0, mask, **kw):
     (8, 1000, 64, 16, False, False, False, True, 16),     # padding
     (6, 512, 40, 16, True, True, True, True, 16),
     (5, 96, 24, 16, False, False, True, True, 16),
+    (8, 256, 16, 16, False, False, False, False, 14),     # four sequences to a block
+    (5, 290, 72, 16, False, True, True, False, 14),
+    (7, 544, 40, 16, True, False, False, False, 14),
+    (6, 1000, 24, 5, False, True, True, True, 14),
     (8, 1024, 48, 16, True, False, False, False, 162),    # runs
     (20, 2048 + 96, 40, 16, True, True, True, False, 164),
     (9, 2048 + 17, 64, 7, False, False, True, False, 168),
@@ -82,7 +86,7 @@ def test_against_oracle(option, bsz, length, dim, ndim, state, normed, silu, mas
     assert _lib.device_error() == 0
 
 
-@pytest.mark.parametrize("tile", [16, 162])
+@pytest.mark.parametrize("tile", [14, 16, 162])
 def test_long_sequence_far_from_zero(option, tile):
     """Values about 100 with a deviation of 1: the statistics keep their accuracy over 16384 positions."""
     from fairseq_apollo_b200 import _lib
@@ -99,7 +103,7 @@ def test_long_sequence_far_from_zero(option, tile):
 
 
 @pytest.mark.parametrize("value", [float("nan"), float("inf"), float("-inf")])
-@pytest.mark.parametrize("tile,at", [(16, 300), (16, 0), (162, 511)])
+@pytest.mark.parametrize("tile,at", [(14, 300), (16, 300), (16, 0), (162, 511)])
 def test_not_finite_stays_in_its_channel(option, value, tile, at):
     option(2, tile)
     x, stats, prm, h0, mask = _case(8, 1024, 48, 16, True, False, seed=2)
@@ -117,7 +121,7 @@ def test_not_finite_stays_in_its_channel(option, value, tile, at):
     assert not torch.isfinite(r["h"][2, 21]).any() and not torch.isfinite(r["mean"][2, 21])
 
 
-@pytest.mark.parametrize("tile", [16, 164])
+@pytest.mark.parametrize("tile", [14, 16, 164])
 def test_wait_that_runs_out(option, tile):
     """x of 64 positions never arrives: the kernel gives up, says so, and the next call is as always."""
     from fairseq_apollo_b200 import _lib
