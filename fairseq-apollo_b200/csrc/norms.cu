@@ -9,6 +9,7 @@
 #include "scan_norm.cuh"
 #include "stream_bwd.cuh"
 #include "stream_cl.cuh"
+#include "tmem_ema.cuh"
 
 namespace mega {
 
@@ -572,16 +573,19 @@ static int tsn_fwd_common(const void* x, void* y, int dtype, int B, int L, int D
       sa.beta = beta; sa.eps = (float)eps; sa.count_out = a.count_out; sa.mean_out = mean_out; sa.var_out = var_out;
       sa.mask = pad_mask;
       sa.cummean = cummean; sa.cumrstd = cumrstd;
-      // The scan takes its statistics in fp32 (variances 1e-6 off), the tensor-core form from bf16 and tf32 operands (3e-4).
-      // Measured, scan against that form: 16 x 4096 x 1024 102 / 142 us, 16 x 32768 x 2048 1179 / 1433, 32 x 8192 x 2048
-      // 592 / 620; with 64 sequences of 2048 channels it is up to 15 % behind (32768 positions: 4969 / 4305 us), and stays for
-      // its precision.
+      // The walk of tmem_ema.cu (bf16, where there are enough sequences and channels: 16 x 4096 x 1024 68 us, 64 x 4096 x 2048 469) and
+      // the scan (105, 614) take their statistics in fp32 (variances 1e-6 off), the tensor-core form from bf16 and tf32 operands
+      // (3e-4; 142, and 4305 us at 64 x 32768 x 2048 where the scan takes 4969).
       if (!cummean && g_options[OPT_MMA_TILE].load() == 0 && g_options[OPT_DISABLE_MMA].load() == 0) {
         ScanNormArgs na{};
         na.x = x; na.y = y; na.B = B; na.D = D; na.L = L;
         na.xsb = xsb; na.xsl = xsl; na.ysb = ysb; na.ysl = ysl;
         na.prev_count = a.prev_count; na.prev_mean = prev_mean; na.prev_var = prev_var; na.gamma = gamma; na.beta = beta;
         na.mask = pad_mask; na.eps = (float)eps; na.count_out = a.count_out; na.mean_out = mean_out; na.var_out = var_out;
+        const int form = g_options[OPT_SPLIT].load();
+        if (xsd == 1 && ysd == 1 && form != 3 && (form == 4 || tmem_norm_us(sa) < 0.9 * scan_norm_us(na)) &&
+            tmem_norm_try(dtype, x, y, xsb, xsl, ysb, ysl, sa, (cudaStream_t)stream))
+          return check_launch("timestep_norm_fwd(tmem)");
         if (scan_norm_fwd_try(dtype, na, xsd, ysd, (cudaStream_t)stream)) return check_launch("timestep_norm_fwd(scan)");
       }
       // (statistics updated in place, a form of the tensor-core kernel asked for by name, or the streamed kernel)

@@ -517,6 +517,9 @@ static bool pairs_ok(int dtype, const ScanNormArgs& a, long long ysd) {
   return ysd == 1 && aligned_to(a.y, 2 * elem_size(dtype)) && a.ysb % 2 == 0 && a.ysl % 2 == 0;
 }
 
+// (us, from 15 shapes of 2 to 67 M elements to 4 %; 537 M are 614)
+double scan_norm_us(const ScanNormArgs& a) { return (14.0 + (double)a.B * a.D * a.L / 740e3) * (a.mask ? 1.32 : 1.0); }
+
 bool scan_norm_fwd_try(int dtype, const ScanNormArgs& a, long long xsd, long long ysd, cudaStream_t s) {
   if (!pieces_ok(dtype, a.D) || !rows_ok(dtype, a.x, a.xsb, a.xsl, xsd) || !((a.wide && !a.y) || pairs_ok(dtype, a, ysd)) ||
       a.x == a.y)

@@ -25,6 +25,7 @@ struct ScanNormArgs {
 // Each returns false, having launched nothing, outside its envelope (channels not contiguous, rows that are not
 // whole 16-byte pieces, too many sequences for the grid, statistics updated in place) or when there is no scratch memory.
 bool scan_norm_fwd_try(int dtype, const ScanNormArgs& a, long long xsd, long long ysd, cudaStream_t s);
+double scan_norm_us(const ScanNormArgs& a);   // of the forward
 bool scan_norm_bwd_try(int dtype, const ScanNormArgs& a, long long xsd, long long ysd, long long gsd, cudaStream_t s);
 
 // Per-channel SequenceNorm: var_out receives rstd; the backward takes the forward's count, mean and rstd as

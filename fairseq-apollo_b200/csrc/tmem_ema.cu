@@ -57,11 +57,13 @@ constexpr int kColV = 0, kColH = 128, kColY = 256;
 // kQ: sequences of a block, eight or (few of them: more blocks, each with half of the work) four.
 // Warps: four of the states, four or (SiLU; four sequences, of which half of the warps have rows) eight of the outputs, twelve of the
 // statistics in groups, x, products, and two for the normalised activations where they are an output.
-template <int kQ, bool kSilu, bool kXn>
+// TimestepNorm by itself (kEma false) has the statistics' warps, x, and four (two) that write what they leave.
+template <int kQ, bool kSilu, bool kXn, bool kEma>
 struct Roles {
   static constexpr int kPer = kQ / 2, kGroups = 12 / kPer;   // warps of a group of the statistics (two sequences each), groups
-  static constexpr int kOut = 4, kOuts = kSilu || kQ == 4 ? 2 : 1, kStats = kOut + 4 * kOuts, kLoad = kStats + 12, kMma = kLoad + 1, kCopy = kMma + 1;
-  static constexpr int kThreads = 32 * (kCopy + (kXn ? 2 : 0));
+  static constexpr int kOut = 4, kOuts = kSilu || kQ == 4 ? 2 : 1, kStats = kEma ? kOut + 4 * kOuts : 0, kLoad = kStats + 12;
+  static constexpr int kMma = kLoad + 1, kCopy = kMma + (kEma ? 1 : 0), kCopies = !kXn ? 0 : kEma || kQ == 4 ? 2 : 4;
+  static constexpr int kThreads = 32 * (kCopy + kCopies);
   static constexpr int kStep = kQ * kCh * 2, kStageBytes = 2 * kPart * kStep;   // bytes from a position of x to the next; of a stage
 };
 
@@ -219,10 +221,10 @@ __device__ __noinline__ void hand_on(const TmemArgs& t, int b, int d, int slot, 
   if (slot == 2) to[3] = dev2;
 }
 
-template <int kQ, bool kSilu, bool kXn, bool kMask>
-__global__ void __launch_bounds__(Roles<kQ, kSilu, kXn>::kThreads, 1) tsn_ema_tmem_kernel(const __grid_constant__ CUtensorMap tx, const __grid_constant__ TmemArgs t) {
+template <int kQ, bool kSilu, bool kXn, bool kMask, bool kEma>
+__global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kEma>::kThreads, 1) tsn_ema_tmem_kernel(const __grid_constant__ CUtensorMap tx, const __grid_constant__ TmemArgs t) {
   extern __shared__ __align__(128) unsigned char smem[];
-  using R = Roles<kQ, kSilu, kXn>;
+  using R = Roles<kQ, kSilu, kXn, kEma>;
   constexpr int kGroups = R::kGroups, kPer = R::kPer, kStep = R::kStep;
   const StreamArgs& a = t.a;
   const uint32_t base = smem_u32(smem);
@@ -243,7 +245,7 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn>::kThreads, 1) tsn_ema_tm
 
   int* drawn = reinterpret_cast<int*>(smem + kOffBar + kBars * 8 + 12);
   if (tid == 0) *drawn = t.runs > 1 ? atomicAdd(t.sched, 1) : (int)blockIdx.x;
-  if (warp == 0) tm_alloc(smem_u32(tm_slot), 512);
+  if (kEma && warp == 0) tm_alloc(smem_u32(tm_slot), 512);
   if (tid == 32) {
     auto init = [&](int i, int n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar(i)), "r"(n) : "memory"); };
     for (int i = 0; i < kStages; ++i) {
@@ -252,7 +254,7 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn>::kThreads, 1) tsn_ema_tm
     }
     for (int i = 0; i < 2; ++i) {
       init(kOpFull + i, 12);
-      init(kOpEmpty + i, 1);
+      init(kOpEmpty + i, kEma ? 1 : R::kCopies);
       init(kXnRead + i, 2);
     }
     init(kHDone, 1);
@@ -270,7 +272,7 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn>::kThreads, 1) tsn_ema_tm
   tm_before();
   __syncthreads();
   tm_after();
-  const uint32_t tm = __shfl_sync(0xffffffffu, *tm_slot, 0);   // (uniform to the compiler: what issues products needs it in uniform registers)
+  const uint32_t tm = kEma ? __shfl_sync(0xffffffffu, *tm_slot, 0) : 0u;   // (uniform to the compiler: what issues products needs it in uniform registers)
   const int item = *drawn, run = item / t.per_run, place = item - run * t.per_run;
   const int d0 = place % t.tiles_d * kCh, b0 = place / t.tiles_d * kQ;
   const int begin = run * t.run_len, len = min(a.L - begin, t.run_len);   // the block's positions
@@ -421,11 +423,11 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn>::kThreads, 1) tsn_ema_tm
         __syncwarp();
         if (lane == 0) arrive(bar(kXEmpty + (part >> 1) % kStages));
       }
-      if (odd || !(fabsf(dev2) < 3e38f)) {
+      if (kEma && (odd || !(fabsf(dev2) < 3e38f))) {
 #pragma unroll 1
         for (int i = first; i < part; i += kGroups) odd_values(plane + (i & 4) * 64 + (i & 3) * 32, i * kPart, live, bad + s * kCh + ch, any_bad);
       }
-      if (!kMask && end == parts && run < t.runs - 1 && live && !*gone) hand_on(t, b, d, part - parts, c, dev2);
+      if (kEma && !kMask && end == parts && run < t.runs - 1 && live && !*gone) hand_on(t, b, d, part - parts, c, dev2);
       if (end == parts && part - kGroups == parts - 1) {   // (behind the end: zeros)
         if (!kMask && run == t.runs - 1 && live && !*gone) finish(t, b, d, mean, dev2, a.L);
 #pragma unroll 1
@@ -435,7 +437,7 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn>::kThreads, 1) tsn_ema_tm
       __syncwarp();
       if (lane == 0) arrive(bar(kOpFull + (tile & 1)));
     }
-  } else if (warp < 4) {
+  } else if (kEma && warp < 4) {
     // ---- states and outputs -------------------------------------------------------------------------------------
     const int half = lane >> 4, pole = lane & 15;
     const uint32_t quarter = tm + ((uint32_t)warp << 21);
@@ -583,7 +585,7 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn>::kThreads, 1) tsn_ema_tm
         turn_states();
       }
     }
-  } else if (warp < R::kStats) {
+  } else if (kEma && warp < R::kStats) {
     // ---- outputs: a thread per sequence and chunk ----------------------------------------------------------------
     const int half = lane >> 4, chunk = lane & 15, s_out = 2 * (warp & 3) + half, b = b0 + s_out;
     const uint32_t quarter = tm + ((uint32_t)(warp & 3) << 21);
@@ -656,8 +658,8 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn>::kThreads, 1) tsn_ema_tm
       const int rows = *gone ? 0 : a.B;
       const bool full = t.wide != 0 && b0 + kQ <= rows && (tile + 1) * kTile <= len;
 #pragma unroll 1
-      for (int i = 0; i < kQ; ++i) {   // two sequences, four of their 16 positions
-        const int s = kPer * (warp & 1) + 2 * (i >> 2) + (lane >> 4), b = b0 + s, k0 = 4 * (i & 3);
+      for (int i = 0; i < 2 * kQ / R::kCopies; ++i) {   // two sequences, four of their 16 positions
+        const int s = kQ / R::kCopies * (warp - R::kCopy) + 2 * (i >> 2) + (lane >> 4), b = b0 + s, k0 = 4 * (i & 3);
         const unsigned char* from = smem + kOffOp + (tile & 1) * kBuf + row_of(s, chunk) + (k0 >> 3) * 128 + (k0 & 4) * 2;
         uint2 v[kCh];
 #pragma unroll
@@ -674,9 +676,9 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn>::kThreads, 1) tsn_ema_tm
         }
       }
       __syncwarp();
-      if (lane == 0) arrive(bar(kXnRead + (tile & 1)));
+      if (lane == 0) arrive(bar((kEma ? kXnRead : kOpEmpty) + (tile & 1)));
     }
-  } else if (umma_elect()) {
+  } else if (kEma && umma_elect()) {
     // ---- products -----------------------------------------------------------------------------------------------
     constexpr uint32_t kLocal = umma_idesc(128, 16 * kQ, false), kTaps = umma_idesc(128, 16, false), kStates = umma_idesc(128, 16, true);
     wait(kReady, 0);
@@ -722,17 +724,17 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn>::kThreads, 1) tsn_ema_tm
   tm_before();
   __syncthreads();
   tm_after();
-  if (warp == 0) tm_free(tm, 512);
+  if (kEma && warp == 0) tm_free(tm, 512);
   if (run < t.runs - 1 && tid == 0) {
     __threadfence();
     asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(t.sched + 1 + item), "r"(*gone ? 2 : 1) : "memory");
   }
 }
 
-template <int kQ, bool kSilu, bool kXn, bool kMask>
+template <int kQ, bool kSilu, bool kXn, bool kMask, bool kEma = true>
 void launch_form(const CUtensorMap& tx, const TmemArgs& t, cudaStream_t s) {
   const unsigned grid = (unsigned)(t.per_run * t.runs);
-  launch(tsn_ema_tmem_kernel<kQ, kSilu, kXn, kMask>, grid, Roles<kQ, kSilu, kXn>::kThreads, kOffEnd, (void*)s, tx, t);
+  launch(tsn_ema_tmem_kernel<kQ, kSilu, kXn, kMask, kEma>, grid, Roles<kQ, kSilu, kXn, kEma>::kThreads, kOffEnd, (void*)s, tx, t);
 }
 
 }  // namespace
@@ -751,6 +753,13 @@ double runs_us(const StreamArgs& a, bool xn, int runs, int q) {
   if (a.D % kCh) ns = std::max(ns, (xn ? (a.mask ? 50. : 41.) : 28.5) * (q == 4 ? 0.7 : 1.));
   const double rounds = std::max(std::ceil(tiles / 148.), (double)runs);   // (a sequence's runs follow one another)
   return 4. + rounds * (6. + len * ns * (rounds > 2. ? 1.125e-3 : 1e-3));
+}
+// with the limit of its waits, and the load that a test withholds
+StreamArgs bounded(StreamArgs a) {
+  const int limit = g_options[OPT_WAIT_LIMIT].load(), withheld = g_options[OPT_WITHHOLD_LOAD].load();
+  a.wait_limit = limit > 0 ? (long long)limit : 4000000000LL;
+  a.withhold_step = withheld > 0 ? withheld : -1;
+  return a;
 }
 // sequences of a block: four where that gives all blocks an SM at once (a position takes 12 - 23 ns for 20 - 32: 8 x 8192 x 1024 112 us
 // against 176, 4 x 4096 x 1024 60 against 88; in two rounds 16 x 4096 x 1024 118 against 91)
@@ -785,7 +794,7 @@ bool tmem_ema_try(int dtype, const void* x, void* y, void* xn, long long xsb, lo
   CUtensorMap tx;
   if (!make_tensor_map_3d(&tx, dtype, x, a.D, a.B, a.L, xsb, xsl, kCh, q, 2 * kPart, CU_TENSOR_MAP_SWIZZLE_NONE)) return false;
   TmemArgs t{};
-  t.a = a;
+  t.a = bounded(a);
   t.y = reinterpret_cast<__nv_bfloat16*>(y);
   t.xn = reinterpret_cast<__nv_bfloat16*>(xn);
   t.ysb = ysb;
@@ -824,6 +833,40 @@ bool tmem_ema_try(int dtype, const void* x, void* y, void* xn, long long xsb, lo
                                         "tsn_ema_mma tmem segmented runs=4", "tsn_ema_mma tmem segmented runs=5", "tsn_ema_mma tmem segmented runs=6",
                                         "tsn_ema_mma tmem segmented runs=7", "tsn_ema_mma tmem segmented runs=8"};
   g_last_kernel.store(a.mask ? "tsn_ema_mma tmem mask" : kNames[std::min(t.runs, 8)], std::memory_order_relaxed);
+  return true;
+}
+
+// (16 x 4096 x 1024 68 us, masked 95; 8 x 8192 x 1024 82 and 116; 64 x 4096 x 2048 469 and 626; 24 x 1500 x 1000 77 and 93)
+double tmem_norm_us(const StreamArgs& a) {
+  const int q = sequences_of(a);
+  const double tiles = (double)((a.D + kCh - 1) / kCh) * ((a.B + q - 1) / q), rounds = std::ceil(tiles / 148.);
+  const int len = (a.L + kTile - 1) / kTile * kTile;
+  const double ns = ((q == 4 ? 8.5 : 14.8) + (a.mask ? (q == 4 ? 4.5 : 6.) : 0.)) * (a.D % kCh ? 1.35 : 1.);
+  return 4. + rounds * (5. + len * ns * 1e-3);
+}
+
+bool tmem_norm_try(int dtype, const void* x, void* y, long long xsb, long long xsl, long long ysb, long long ysl, const StreamArgs& a,
+                   cudaStream_t s) {
+  if (dtype != MEGA_BF16 || a.D % 8 != 0 || a.L >= (1 << 24) || x == y) return false;
+  if (!aligned_to(y, 16) || ysb % 8 != 0 || ysl % 8 != 0) return false;
+  const int q = sequences_of(a);
+  const long long blocks = (long long)((a.D + kCh - 1) / kCh) * ((a.B + q - 1) / q);
+  if (blocks > (1 << 24)) return false;
+  CUtensorMap tx;
+  if (!make_tensor_map_3d(&tx, dtype, x, a.D, a.B, a.L, xsb, xsl, kCh, q, 2 * kPart, CU_TENSOR_MAP_SWIZZLE_NONE)) return false;
+  TmemArgs t{};
+  t.a = bounded(a);
+  t.xn = reinterpret_cast<__nv_bfloat16*>(y);
+  t.ysb = ysb;
+  t.ysl = ysl;
+  t.wide = a.D % 16 == 0 && ysb % 16 == 0 && ysl % 16 == 0 && aligned_to(y, 32);
+  t.tiles_d = (a.D + kCh - 1) / kCh;
+  t.per_run = (int)blocks;
+  t.runs = 1;
+  t.run_len = (a.L + kTile - 1) / kTile * kTile;
+  if (q == 4) a.mask ? launch_form<4, false, true, true, false>(tx, t, s) : launch_form<4, false, true, false, false>(tx, t, s);
+  else a.mask ? launch_form<8, false, true, true, false>(tx, t, s) : launch_form<8, false, true, false, false>(tx, t, s);
+  g_last_kernel.store("tsn_ema_mma tmem norm", std::memory_order_relaxed);
   return true;
 }
 

@@ -14,6 +14,10 @@ bool tmem_ema_try(int dtype, const void* x, void* y, void* xn, long long xsb, lo
                   const StreamArgs& a, cudaStream_t s, int asked = 0);
 // Its estimated time.
 double tmem_ema_us(const StreamArgs& a, bool xn);
+// TimestepNorm by itself in the same way (bf16, x and y distinct), and its estimated time.
+bool tmem_norm_try(int dtype, const void* x, void* y, long long xsb, long long xsl, long long ysb, long long ysl, const StreamArgs& a,
+                   cudaStream_t s);
+double tmem_norm_us(const StreamArgs& a);
 cudaError_t tmem_ema_read_device_error(int* v, bool reset);
 
 }  // namespace mega

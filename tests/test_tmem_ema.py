@@ -156,3 +156,41 @@ def test_strides_and_views(option):
         r = ops.tsn_ema_forward(v, *[t.cuda() for t in stats], 1e-5, p, q, g, prm[4].cuda())["y"]
         assert "tmem" in _lib.last_kernel()
         assert torch.equal(r, want)
+
+
+@pytest.mark.parametrize("bsz,length,dim,masked", [(8, 256, 16, False), (5, 290, 72, False), (4, 33, 8, True), (16, 1000, 40, True),
+                                                   (20, 2048, 1100 // 4 * 8, False), (9, 1, 24, False)])
+def test_norm_alone(option, bsz, length, dim, masked):
+    from fairseq_apollo_b200 import _lib, ops
+    from oracle import mega_oracle as O
+    x, stats, _, _, mask = _case(bsz, length, dim, 1, False, masked)
+    _lib.set_option(5, 4)
+    try:
+        r = ops.timestep_norm_fwd(x.cuda(), *[t.cuda() for t in stats], None if mask is None else mask.cuda())
+        assert _lib.last_kernel() == "tsn_ema_mma tmem norm"
+    finally:
+        _lib.set_option(5, 0)
+    ref = O.timestep_norm(x.float(), *stats, mask, acc_dtype=torch.float64)
+    assert rel_l2(r[0].float(), ref[0]) < 4e-3 and torch.equal(r[1].cpu(), ref[1])
+    assert rel_l2(r[2], ref[2]) < 2e-6 and rel_l2(r[3], ref[3]) < 2e-6
+    if masked:
+        assert (r[0].cpu()[mask] == 0).all()
+    assert _lib.device_error() == 0
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_norm_alone_not_finite(option, value):
+    """As in the scan: such a value's channel is not finite from there on, the others know nothing of it."""
+    from fairseq_apollo_b200 import _lib, ops
+    x, stats, _, _, _ = _case(8, 600, 16, 1, False, False)
+    clean = x.clone()
+    x[3, 270, 5] = value
+    _lib.set_option(5, 4)
+    try:
+        a, b = [ops.timestep_norm_fwd(v.cuda(), *[t.cuda() for t in stats])[0].cpu() for v in (x, clean)]
+    finally:
+        _lib.set_option(5, 0)
+    rest = torch.ones(8, 16, dtype=torch.bool)
+    rest[3, 5] = False
+    assert torch.equal(a.transpose(1, 2)[rest], b.transpose(1, 2)[rest]) and torch.equal(a[3, :270, 5], b[3, :270, 5])
+    assert not torch.isfinite(a[3, 270:, 5].float()).any()
