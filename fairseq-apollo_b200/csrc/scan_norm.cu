@@ -29,6 +29,11 @@ namespace mega {
 
 namespace {
 
+// Tiles in flight of the walks that read x and dy: with three of a 16-bit type a fourth block fits an SM (16 x 4096 x 1024 bf16 with
+// the moments 230 us -> 226, 32 x 2048 x 512 136 -> 128); in fp32, at the rate of memory, four (285 us, three 304).
+template <typename T>
+constexpr int kRingTwo = sizeof(T) == 4 ? kRing : 3;
+
 struct SegNorm {
   ScanNormArgs a;
   int T, S;
@@ -85,7 +90,6 @@ __device__ __forceinline__ PairLane pair_lane(const SegNorm& s) {
 }
 __device__ __forceinline__ f32x2 ldg2(const float* p) { return pack2(__ldg(p), __ldg(p + 1)); }
 __device__ __forceinline__ f32x2 both(float v) { return pack2(v, v); }
-__device__ __forceinline__ f32x2 neg2(f32x2 v) { return mul2(v, both(-1.f)); }
 
 // What a segment starts from: the prior and the segments before it (for two channels).
 __device__ __forceinline__ void pair_before(const SegNorm& s, const PairLane& l, Run (&r)[2]) {
@@ -108,20 +112,31 @@ __device__ __forceinline__ void pair_before(const SegNorm& s, const PairLane& l,
   r[0].n = r[1].n = n0 + seen;
 }
 
-// Running (norm_run.cuh) for two channels.
+// Running (norm_run.cuh) for two channels.  Its walks are bound by the FMA pipe, in which a packed instruction takes two cycles: so
+// no sign is turned in packed arithmetic, and what all steps of a walk share is a factor of its sums.  (16 x 4096 x 1024 bf16,
+// with 26, 23 and 11 packed instructions a step the map 103 us, the gradients 113, the outputs 67; with 18, 19 and 9
+// 88, 98 and 63.)
 struct PairRunning {
-  f32x2 c, s1, s2, in_s, u;
-  float n0, seen, n;
-  __device__ __forceinline__ void start(const Run (&r)[2]) {
+  f32x2 c, s1, s2, in_s, u, eps2;
+  float n0, seen, n, eps;
+  // x: the segment's first step of the lane's channels (one that counts is the centre where nothing came in)
+  template <typename T>
+  __device__ __forceinline__ void start(const Run (&r)[2], float e, const T* x, long long xsl, const unsigned char* m, int t0, int t1) {
     c = pack2(r[0].m, r[1].m);
     s1 = s2 = u = both(0.f);
     n0 = n = r[0].n;
     seen = 0.f;
     in_s = pack2(r[0].s, r[1].s);
+    eps = e;
+    eps2 = both(e);
+    if (n0 == 0.f) {
+      int t = t0;
+      while (m && t < t1 && m[t]) ++t;
+      if (t < t1) c = pack2(Elem<T>::ld(x + t * xsl), Elem<T>::ld(x + t * xsl + 1));
+    }
   }
   // returns x - c; inv = 1 / n, r = 1 / sqrt(var + eps)
-  __device__ __forceinline__ f32x2 step(f32x2 x, float eps, f32x2& inv, f32x2& r) {
-    if (n == 0.f) c = x;
+  __device__ __forceinline__ f32x2 step(f32x2 x, f32x2& inv, f32x2& r) {
     const f32x2 d = sub2(x, c);
     s1 = add2(s1, d);
     s2 = fma2(d, d, s2);
@@ -129,10 +144,11 @@ struct PairRunning {
     n = n0 + seen;
     inv = both(rcp_approx(n));
     u = mul2(s1, inv);
-    const f32x2 v = fma2(neg2(u), u, mul2(add2(in_s, s2), inv));
-    float a, b;
-    unpack2(v, a, b);
-    r = pack2(rsqrt_approx(fmaxf(a, 0.f) + eps), rsqrt_approx(fmaxf(b, 0.f) + eps));
+    const f32x2 q = fma2(add2(in_s, s2), inv, eps2);
+    float a, b, ua, ub;
+    unpack2(q, a, b);
+    unpack2(u, ua, ub);
+    r = pack2(rsqrt_approx(fmaxf(fmaf(-ua, ua, a), eps)), rsqrt_approx(fmaxf(fmaf(-ub, ub, b), eps)));
     return d;
   }
 };
@@ -150,17 +166,16 @@ __global__ void __launch_bounds__(kWarps * 32) norm_emit_kernel(SegNorm s) {
   float* pw = kWide ? a.wide + ((size_t)l.b * a.L + l.t0) * a.D + l.dc : nullptr;
   const unsigned char* m = kMask ? a.mask + (size_t)l.b * a.L : nullptr;
   const f32x2 w = ldg2(a.gamma + l.dc), bb = ldg2(a.beta + l.dc);
-  const float eps = a.eps;
   Run in[2];
   pair_before(s, l, in);
   PairRunning st;
-  st.start(in);
+  st.start(in, a.eps, x + (l.dc - l.d0), a.xsl, m, l.t0, l.t1);
   walk_pairs<T, false, kMask>(x, a.xsl, x, 0, m, l.t0, l.t1, l.left, rings + (size_t)l.warp * kRing * kTileBytes,
                               [&](f32x2 xv, f32x2, bool pad) {
                                 f32x2 out = both(0.f);
                                 if (!(kMask && pad)) {
                                   f32x2 inv, r;
-                                  const f32x2 d = st.step(xv, eps, inv, r);
+                                  const f32x2 d = st.step(xv, inv, r);
                                   out = fma2(mul2(sub2(d, st.u), r), w, bb);
                                 }
                                 if (kWide) {
@@ -206,32 +221,31 @@ __global__ void __launch_bounds__(kWarps * 32) norm_bwd_map_kernel(SegNorm s) {
     const T* x = reinterpret_cast<const T*>(a.x) + l.b * a.xsb + l.d0;
     const T* g = reinterpret_cast<const T*>(a.dy) + l.b * a.gsb + l.d0;
     const unsigned char* m = kMask ? a.mask + (size_t)l.b * a.L : nullptr;
-    const f32x2 w = ldg2(a.gamma + l.dc), wh = mul2(w, both(-0.5f));
-    const float eps = a.eps;
+    const f32x2 w = ldg2(a.gamma + l.dc);
     Run in[2];
     pair_before(s, l, in);
     PairRunning st;
-    st.start(in);
-    f32x2 sv = both(0.f), su = sv, se = sv;   // (su with its sign turned)
-    walk_pairs<T, true, kMask>(x, a.xsl, g, a.gsl, m, l.t0, l.t1, l.left, rings + (size_t)l.warp * 2 * kRing * kTileBytes,
+    st.start(in, a.eps, x + (l.dc - l.d0), a.xsl, m, l.t0, l.t1);
+    // sums whose factors -w / 2 (sv), w (su) and 2 (se) follow; se with its sign turned
+    f32x2 sv = both(0.f), su = sv, se = sv;
+    walk_pairs<T, true, kMask, kRingTwo<T>>(x, a.xsl, g, a.gsl, m, l.t0, l.t1, l.left, rings + (size_t)l.warp * 2 * kRingTwo<T> * kTileBytes,
                                [&](f32x2 xv, f32x2 gv, bool pad) {
                                  if (kMask && pad) return;
                                  const f32x2 up = st.u;
                                  f32x2 inv, r;
-                                 const f32x2 d = st.step(xv, eps, inv, r);
-                                 const f32x2 gr = mul2(gv, r), gx = mul2(gr, sub2(d, st.u));
-                                 se = fma2(mul2(sub2(d, up), both(2.f)), inv, se);
-                                 const f32x2 b = mul2(mul2(gx, mul2(r, r)), mul2(wh, inv));
-                                 sv = add2(sv, b);
-                                 su = add2(su, fma2(b, se, mul2(gr, mul2(w, inv))));
+                                 const f32x2 d = st.step(xv, inv, r);
+                                 const f32x2 gr = mul2(gv, r), gx = mul2(gr, sub2(d, st.u)), b = mul2(gx, mul2(r, r));
+                                 se = fma2(sub2(up, d), inv, se);
+                                 sv = fma2(b, inv, sv);
+                                 su = fma2(fma2(b, se, gr), inv, su);
                                  dg = add2(dg, gx);
                                  db = add2(db, gv);
                                });
     if (l.ok) {
       const size_t i = ((size_t)l.b * s.S + l.seg) * a.D + l.d;
-      *reinterpret_cast<f32x2*>(s.sv + i) = sv;
-      *reinterpret_cast<f32x2*>(s.su + i) = neg2(su);
-      *reinterpret_cast<f32x2*>(s.sw + i) = neg2(se);
+      *reinterpret_cast<f32x2*>(s.sv + i) = mul2(sv, mul2(w, both(-0.5f)));
+      *reinterpret_cast<f32x2*>(s.su + i) = mul2(su, mul2(w, both(-1.f)));
+      *reinterpret_cast<f32x2*>(s.sw + i) = add2(se, se);
     }
   }
   __syncthreads();
@@ -258,8 +272,7 @@ __global__ void __launch_bounds__(kWarps * 32) norm_bwd_emit_kernel(SegNorm s) {
   const T* g = reinterpret_cast<const T*>(a.dy) + l.b * a.gsb + l.d0;
   T* pd = reinterpret_cast<T*>(a.y) + l.b * a.ysb + (long long)l.t0 * a.ysl + l.dc;
   const unsigned char* m = kMask ? a.mask + (size_t)l.b * a.L : nullptr;
-  const f32x2 w = ldg2(a.gamma + l.dc), wh = mul2(w, both(0.5f));
-  const float eps = a.eps;
+  const f32x2 w = ldg2(a.gamma + l.dc);
   const size_t row = (size_t)l.b * a.D + l.dc;
   const float n0 = (float)a.prev_count[l.b];
   float total = 0.f;   // unmasked steps of the call
@@ -288,22 +301,23 @@ __global__ void __launch_bounds__(kWarps * 32) norm_bwd_emit_kernel(SegNorm s) {
       a.dprev_var[row + k] = any ? n0 * vv[k] : (a.dvar ? a.dvar[row + k] : 0.f);
     }
   }
+  f32x2 V2 = add2(V, V);
   Run in[2];
   pair_before(s, l, in);
   PairRunning st;
-  st.start(in);
-  walk_pairs<T, true, kMask>(x, a.xsl, g, a.gsl, m, l.t0, l.t1, l.left, rings + (size_t)l.warp * 2 * kRing * kTileBytes,
+  st.start(in, a.eps, x + (l.dc - l.d0), a.xsl, m, l.t0, l.t1);
+  walk_pairs<T, true, kMask, kRingTwo<T>>(x, a.xsl, g, a.gsl, m, l.t0, l.t1, l.left, rings + (size_t)l.warp * 2 * kRingTwo<T> * kTileBytes,
                              [&](f32x2 xv, f32x2 gv, bool pad) {
                                f32x2 out = both(0.f);
                                if (!(kMask && pad)) {
                                  const f32x2 up = st.u;
                                  f32x2 inv, r;
-                                 const f32x2 d = st.step(xv, eps, inv, r);
-                                 const f32x2 xu = sub2(d, st.u), gr = mul2(gv, r), gx = mul2(gr, xu), V2 = add2(V, V);
+                                 const f32x2 d = st.step(xv, inv, r);
+                                 const f32x2 xu = sub2(d, st.u), gr = mul2(gv, r), wi = mul2(w, inv);
                                  const f32x2 h = fma2(mul2(sub2(d, up), inv), V2, W);   // W + e V
                                  out = fma2(gr, w, fma2(xu, V2, h));
-                                 W = fma2(gr, mul2(w, inv), h);                         // W - (a - e V) with a = -gr w / n
-                                 V = fma2(mul2(gx, mul2(r, r)), mul2(wh, inv), V);      // V - b
+                                 W = fma2(gr, wi, h);                                   // W - (a - e V) with a = -gr w / n
+                                 V2 = fma2(mul2(mul2(gr, xu), mul2(r, r)), wi, V2);     // V - b
                                }
                                if (l.ok) pair_st(pd, out);
                                pd += a.ysl;
@@ -432,10 +446,10 @@ template <typename T, bool kMask>
 static void bwd_launch(const SegNorm& s, cudaStream_t st) {
   const dim3 grid((s.a.D + 31) / 32, (s.S + kWarps - 1) / kWarps, s.a.B), block(kWarps * 32);
   const dim3 pairs((s.a.D + 63) / 64, grid.y, grid.z);
-  const size_t rings = (size_t)kWarps * kRing * kTileBytes;
+  const size_t rings = (size_t)kWarps * kRing * kTileBytes, two = (size_t)kWarps * 2 * kRingTwo<T> * kTileBytes;
   launch(norm_moments_kernel<T, kMask>, grid, block, rings, (void*)st, moments_of(s));
-  launch(norm_bwd_map_kernel<T, kMask>, pairs, block, 2 * rings, (void*)st, s);
-  launch(norm_bwd_emit_kernel<T, kMask>, pairs, block, 2 * rings, (void*)st, s);
+  launch(norm_bwd_map_kernel<T, kMask>, pairs, block, two, (void*)st, s);
+  launch(norm_bwd_emit_kernel<T, kMask>, pairs, block, two, (void*)st, s);
 }
 
 template <typename T, bool kMask>
@@ -480,7 +494,7 @@ static bool dispatch(int dtype, const ScanNormArgs& a, cudaStream_t st) {
   if (g_options[OPT_DISABLE_STREAM].load() != 0 || a.B > 65535) return false;
   SegNorm s{};
   s.a = a;
-  pick_segments(a, kBwd ? 3 : 6, 64, s);
+  pick_segments(a, !kBwd ? 6 : dtype == MEGA_F32 ? 3 : 4, 64, s);   // (resident blocks)
   const size_t n = (size_t)a.B * s.S * a.D;
   Scratch sc(Scratch::padded(n * 4) * (kBwd ? 5 : 2) + Scratch::padded((size_t)a.B * s.S * 4), st);
   if (!sc) return false;

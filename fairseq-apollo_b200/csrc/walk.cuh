@@ -118,8 +118,8 @@ __device__ __forceinline__ void pair_st(T* p, f32x2 v) {
   }
 }
 
-// walk() in time order for 64 channels: f(v, g, pad) sees the pairs of every step.
-template <typename T, bool kTwo, bool kMask, typename F>
+// walk() in time order for 64 channels, rings of kSlots tiles: f(v, g, pad) sees the pairs of every step.
+template <typename T, bool kTwo, bool kMask, int kSlots = kRing, typename F>
 __device__ __forceinline__ void walk_pairs(const T* x, long long xsl, const T* g, long long gsl, const unsigned char* m, int t0, int t1,
                                            int d_left, unsigned char* ring, F&& f) {
   constexpr int kR = kTileBytes / (64 * (int)sizeof(T));
@@ -129,9 +129,9 @@ __device__ __forceinline__ void walk_pairs(const T* x, long long xsl, const T* g
   const uint32_t rs = smem_u32(ring);
   auto issue = [&](int j) {
     if (j < tiles) {
-      const int slot = j % kRing;
+      const int slot = j % kSlots;
       fetch_tile<T, 64>(rs + slot * kTileBytes, px + (long long)(j * kR) * xsl, xsl, n - j * kR, d_left, lane);
-      if (kTwo) fetch_tile<T, 64>(rs + (kRing + slot) * kTileBytes, pg + (long long)(j * kR) * gsl, gsl, n - j * kR, d_left, lane);
+      if (kTwo) fetch_tile<T, 64>(rs + (kSlots + slot) * kTileBytes, pg + (long long)(j * kR) * gsl, gsl, n - j * kR, d_left, lane);
     }
     tile_commit();
   };
@@ -141,16 +141,16 @@ __device__ __forceinline__ void walk_pairs(const T* x, long long xsl, const T* g
     return __ballot_sync(0xffffffffu, lane < kR && k < n && __ldg(m + t0 + k) != 0);
   };
 #pragma unroll
-  for (int j = 0; j < kRing - 1; ++j) issue(j);
+  for (int j = 0; j < kSlots - 1; ++j) issue(j);
   unsigned next = flags(0);
   for (int j = 0; j < tiles; ++j) {
-    tile_wait<kRing - 2>();
+    tile_wait<kSlots - 2>();
     __syncwarp();
-    issue(j + kRing - 1);
+    issue(j + kSlots - 1);
     const unsigned bits = next;
     if (j + 1 < tiles) next = flags(j + 1);
-    const T* tx = reinterpret_cast<const T*>(ring + (j % kRing) * kTileBytes) + 2 * lane;
-    const T* tg = reinterpret_cast<const T*>(ring + (kRing + j % kRing) * kTileBytes) + 2 * lane;
+    const T* tx = reinterpret_cast<const T*>(ring + (j % kSlots) * kTileBytes) + 2 * lane;
+    const T* tg = reinterpret_cast<const T*>(ring + (kSlots + j % kSlots) * kTileBytes) + 2 * lane;
     const int rows = min(kR, n - j * kR);
     int r0 = 0;
     for (; r0 + kU <= rows; r0 += kU) {

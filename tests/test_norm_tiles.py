@@ -132,3 +132,37 @@ def test_norm_ema_forms_agree(bsz, length, dim, cplx, xn):
         assert torch.equal(r["count"], res[0]["count"])
         if xn:
             assert rel_l2(r["xn"].float(), res[0]["xn"].float()) < 2.0 ** -7
+
+
+# The first step has no variance: its terms, of size eps^-1/2 = 316, cancel against what the later steps carry back, and leave what
+# approximate roots and reciprocals (2^-22) and sums of a handful of such terms leave: 316 x 2^-20 of gradients of size one.  16 bits:
+# the rounding of the output beside that.
+@pytest.mark.parametrize("dtype,rounding", [(torch.float32, 0.0), (torch.bfloat16, 2.0 ** -9), (torch.float16, 2.0 ** -12)])
+@pytest.mark.parametrize("length,dim,lead", [(64, 8, 0), (300, 72, 70), (1111, 136, 3)])
+def test_backward_without_a_prior(dtype, rounding, length, dim, lead):
+    """Nothing came in and the first steps (a whole segment of 64 and more) are padded: the first step that counts is the centre."""
+    from fairseq_apollo_b200 import ops
+    gen = torch.Generator().manual_seed(length)
+    bsz = 3
+    x = (torch.randn(bsz, length, dim, generator=gen) + 100.0).to(dtype)
+    dy = torch.randn(bsz, length, dim, generator=gen).to(dtype)
+    gamma, dmean, dvar = torch.randn(dim, generator=gen), torch.randn(bsz, dim, generator=gen), torch.randn(bsz, dim, generator=gen)
+    mask = torch.zeros(bsz, length, dtype=torch.bool)
+    mask[1, :lead] = True
+    mask[2, length // 2:length // 2 + 9] = True
+    zero = torch.zeros(bsz, dim)
+    got = ops.timestep_norm_bwd_stats(*[t.cuda() for t in (dy, dmean, dvar, x, torch.zeros(bsz, dtype=torch.int64), zero, zero + 1, gamma, mask)])
+    xd, gd = x.double().requires_grad_(True), gamma.double().requires_grad_(True)
+    keep = (~mask).double()[..., None]
+    count = keep.cumsum(1).clamp(min=1)
+    about = torch.stack([xd.detach()[b, int((~mask[b]).nonzero()[0])] for b in range(bsz)])[:, None]
+    dev = (xd - about) * keep
+    mean = dev.cumsum(1) / count
+    var = (dev * dev).cumsum(1) / count - mean * mean
+    y = (dev - mean) * (var.clamp(min=0) + 1e-5).rsqrt() * gd * keep
+    total = (y * dy.double()).sum() + (mean[:, -1] * dmean.double()).sum() + (var[:, -1] * dvar.double()).sum()
+    dx, dgamma = torch.autograd.grad(total, (xd, gd))
+    assert rel_l2(got[0].float(), dx) < 316 * 2.0 ** -20 + rounding
+    assert rel_l2(got[3], dgamma) < 1e-5
+    assert rel_l2(got[4], (dy.double() * keep).sum((0, 1))) < 1e-5
+    assert (got[0].cpu()[mask] == 0).all()
