@@ -26,7 +26,8 @@
 // bf16 calls that would otherwise go to the tensor-core kernel take the leading parts alone, as that one does (lean_call).
 // What bounds it (backward of 16 x 4096 x 1024 bf16, 227 us for both of its walks in one): the tensor pipe is busy 47 % of the
 // time, issue slots 45 %, shared memory 32 %, DRAM 21 %; 16 warps per SM at 128 registers do not hide the chain of products.
-// Complex outputs of fp32 inputs (6 x 4999 x 2048, 374 us): 46, 47, 35 and 12 %.
+// Complex outputs of fp32 inputs (6 x 4999 x 2048, 344 us; 374 under the profiler before half of the warps turned while others
+// multiplied): 46, 47, 35 and 12 %.
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
@@ -1012,21 +1013,18 @@ __global__ void __launch_bounds__(Form<In, Out, kC, kMode, kMask, kLean>::kThrea
     for (int i = 0; i < tiles; ++i) {
       if constexpr (!kLean)
         if (i % (512 / kTile) == 0) settle(2 * min(16, steps - kTile / 32 * i));
-      if constexpr (kSame) {
-#pragma unroll 1
-        for (int half = 0; half < 2; ++half) {
-          if (((warp >> 2) & 1) == half) {
-            if (d < a.D) multiply(i);
-          } else {
-            leave(i - 1);
-            arrive(i + 1);
-          }
-        }
-      } else {
+      if constexpr (!kSame) {   // (and half and half from there on: complex 6 x 4999 x 2048 from fp32 344 us, all turning first 359)
         leave(i - 1);
         __syncthreads();
-        arrive(i + 1);
-        if (d < a.D) multiply(i);
+      }
+#pragma unroll 1
+      for (int half = 0; half < 2; ++half) {
+        if (((warp >> 2) & 1) == half) {
+          if (d < a.D) multiply(i);
+        } else {
+          if constexpr (kSame) leave(i - 1);
+          arrive(i + 1);
+        }
       }
       __syncthreads();
     }
