@@ -48,7 +48,7 @@ bool mma_cl_try(int dtype, const void* x, void* y, void* xn, long long xsb, long
     return false;
   if (a_in.h_out && (a_in.L % kStep) != 0) return false;
   if ((a_in.B + kSeq - 1) / kSeq > 65535) return false;
-  // TimestepNorm -> EMA with real poles: statistics by scalar arithmetic and accumulators in tensor memory (16 x 4096 x 1024 92 us
+  // TimestepNorm -> EMA with real poles: statistics by scalar arithmetic and accumulators in tensor memory (16 x 4096 x 1024 90 us
   // against 140, with the second output 110 against 208, masked 111 against 195), or this kernel's chain (64 x 32768 x 2048, where
   // the power cap slows the other: 5.2 ms both)
   if (norm && ema && !a_in.cplx) {

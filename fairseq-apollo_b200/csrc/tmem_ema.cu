@@ -8,18 +8,22 @@
 //   output y = T x + G h   T (16 x 16): the taps, omega on the diagonal; G (16 x 16 poles): g q^(j+1)
 //   - the normalised rows go to shared memory as 16-byte pieces along time (K-major), which serve as A of T x and as B of V x;
 //   - V x is taken the other way round, poles on the rows: eight channels share an accumulator of 128 rows x 128
-//     columns, each channel's V (in tensor memory) being zero but for its own 16 rows.  So a thread holds one pole and reads a
-//     sequence's chunks as columns in the order of time: the carry stays inside it, one multiply-add per chunk;
+//     columns, and V's of eight channels under each other are one operand, of whose products with a channel's rows only the channel's
+//     own 16 rows are written.  So a thread holds one pole and reads a sequence's chunks as columns in the order of time: the carry
+//     stays inside it, one multiply-add per chunk;
 //   - the states go back as bf16, eight chunks to a 16-byte piece (MN-major), over the rows of x that are no longer needed, and G h is
 //     added to T x;
-//   - an output's thread holds a (sequence, chunk) row, reads two positions of the 16 channels at a time and writes 32 bytes each.
+//   - an output's thread holds a (sequence, chunk) row, reads two positions of the 16 channels at a time and writes 32 bytes each;
+//   - the outputs of eight channels have one of two places, with SiLU, whose outputs take long, one of three: T x of the next tile's
+//     first eight does not wait for them then (16 x 4096 x 1024 126 -> 112 us, 8 x 8192 x 1024 192 -> 174, with the second output 200 ->
+//     178).  Tensor memory has room for that where V is in shared memory, from where it costs the plain form 89 -> 98 us.
 // The statistics are a chain along time, 12 to 13 instructions a position.  One warp to a scheduler issues 0.4 of them a cycle (41 cycles
 // a position), so three groups of warps take the parts of 32 positions in turn: a group sums its part about a centre of its own before
 // the state of the part before is there, hands the state on, and normalises (28 cycles).  Warps: 12 of the statistics (ahead by up to
 // two tiles), 4 of states, 4 of outputs (8 with SiLU), one that fetches x (TMA), one that issues products, 2 for the normalised
 // activations as an output.  Everything is exchanged over mbarriers, the statistics over named barriers of two warps.
 //
-// What bounds it (16 x 4096 x 1024, 92 us against 140 in the forms of mma_cl_kernel.cuh; 67 without anything but the statistics): issue
+// What bounds it (16 x 4096 x 1024, 90 us against 140 in the forms of mma_cl_kernel.cuh; 67 without anything but the statistics): issue
 // slots and latency at 22 warps, 0.65 instructions per scheduler and cycle; the products' reads of shared memory 12 us, the outputs 4.
 // Two things that cost much: outputs that may stay in L1 (103 us; no_allocate), and code that does not fit the instruction cache (the
 // same walk in 250 KB of code 512 us; what is rare is out of line).  Over all SMs for long the power cap takes 12 % of the clock.
@@ -48,12 +52,13 @@ constexpr int kPlane = 4096 + 16, kBuf = kCh * kPlane;   // rows of a channel (1
 constexpr int kMat = 1024;                               // T and G of a channel
 enum { kOffX = 0, kOffOp = kOffX + kStages * 2 * kPart * kMostQ * kCh * 2, kOffMat = kOffOp + 2 * kBuf, kOffInv = kOffMat + kCh * kMat,
        kOffMail = kOffInv + 16 * 64 * 4, kOffTaps = kOffMail + 4 * 32 * 8, kOffBad = kOffTaps + kCh * 16 * 4, kOffBar = kOffBad + kMostQ * kCh * 4,
-       kOffEnd = kOffBar + 40 * 8 + 16 };
+       kOffV = kOffBar + 40 * 8 + 32, kOffEnd = kOffV + 2 * 4096 };   // kOffV: V of 8 channels under each other, twice
+static_assert(kOffV % 16 == 0 && kOffEnd <= 227 * 1024, "shared memory");
 // barriers
-enum { kXFull = 0, kXEmpty = kStages, kOpFull = 2 * kStages, kOpEmpty = kOpFull + 2, kHDone = kOpEmpty + 2, kHRead, kTDone, kYDone, kYRead, kReady, kEnd, kXnRead, kBars = kXnRead + 2 };
+enum { kXFull = 0, kXEmpty = kStages, kOpFull = 2 * kStages, kOpEmpty = kOpFull + 2, kHDone = kOpEmpty + 2, kHRead, kTDone, kYDone = kTDone + 2, kYRead, kReady, kEnd, kXnRead, kBars = kXnRead + 2 };
 static_assert(kBars <= 40, "barriers");
-// columns of tensor memory: V of 16 channels, two accumulators of local states, outputs
-constexpr int kColV = 0, kColH = 128, kColY = 256;
+// columns of tensor memory: local states of eight channels; outputs of eight channels, two or three times (and V)
+constexpr int kColH = 0, kColY = 128;
 // kQ: sequences of a block, eight or (few of them: more blocks, each with half of the work) four.
 // Warps: four of the states, four or (SiLU; four sequences, of which half of the warps have rows) eight of the outputs, twelve of the
 // statistics in groups, x, products, and two for the normalised activations where they are an output.
@@ -226,6 +231,8 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kEma>::kThreads, 1) tsn_
   extern __shared__ __align__(128) unsigned char smem[];
   using R = Roles<kQ, kSilu, kXn, kEma>;
   constexpr int kGroups = R::kGroups, kPer = R::kPer, kStep = R::kStep;
+  constexpr bool kThree = kSilu, kVShared = kThree && kQ == 8;   // places of the outputs; V in shared memory
+  constexpr int kColV = kQ == 4 ? 64 : 384;
   const StreamArgs& a = t.a;
   const uint32_t base = smem_u32(smem);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
@@ -260,6 +267,7 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kEma>::kThreads, 1) tsn_
     init(kHDone, 1);
     init(kHRead, 4);
     init(kTDone, 1);
+    init(kTDone + 1, 1);
     init(kYDone, 1);
     init(kYRead, kPer * R::kOuts);
     init(kReady, 4);
@@ -481,14 +489,17 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kEma>::kThreads, 1) tsn_
         *reinterpret_cast<__nv_bfloat16*>(mat + 512 + (e >> 3) * 256 + (pole >> 3) * 128 + (e & 7) * 16 + (pole & 7) * 2) =
             __float2bfloat16_rn(gm * pw);
       }
-      uint32_t words[8], mine[8];
+      if constexpr (kVShared) {
+        unsigned char* v = smem + kOffV + g * 4096 + (2 * warp + half) * 512 + (pole >> 3) * 256 + (pole & 7) * 16;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) words[i] = bf16_pair(vk[2 * i], vk[2 * i + 1]);
-#pragma unroll 1
-      for (int j = 0; j < 8; ++j) {
+        for (int i = 0; i < 2; ++i)
+          *reinterpret_cast<uint4*>(v + i * 128) = make_uint4(bf16_pair(vk[8 * i], vk[8 * i + 1]), bf16_pair(vk[8 * i + 2], vk[8 * i + 3]),
+                                                              bf16_pair(vk[8 * i + 4], vk[8 * i + 5]), bf16_pair(vk[8 * i + 6], vk[8 * i + 7]));
+      } else {
+        uint32_t words[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) mine[i] = j == 2 * warp + half ? words[i] : 0u;
-        tm_st8(quarter + kColV + 8 * (8 * g + j), mine);
+        for (int i = 0; i < 8; ++i) words[i] = bf16_pair(vk[2 * i], vk[2 * i + 1]);
+        tm_st8(quarter + kColV + 8 * g, words);
       }
       __syncwarp();
       float row[16];   // row `pole` of T
@@ -511,8 +522,10 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kEma>::kThreads, 1) tsn_
       }
       turn_pole();
     }
-    tm_wait_st();
-    tm_before();
+    if (!kVShared) {
+      tm_wait_st();
+      tm_before();
+    }
     fence_proxy_async();
     __syncwarp();
     if (lane == 0) arrive(bar(kReady));
@@ -535,9 +548,9 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kEma>::kThreads, 1) tsn_
           tm_ld32(quarter + kColH + 64 * hf + 32 * j, v);
           tm_wait_ld();
           landed(v);
-          if (j == 0 && unit == 0) {   // (x is still read until then)
-            wait_all(kTDone, tile);
-            if (kXn) wait_all(kXnRead + (tile & 1), tile >> 1);
+          if (j == 0 && hf == 0) {   // (x is still read until then)
+            wait_all(kTDone + g, tile);
+            if (kXn && g == 0) wait_all(kXnRead + (tile & 1), tile >> 1);
           }
           auto carry = [&](auto stops) {   // stops: chunks behind the last one, whose local states are zero, leave the states as they are
 #pragma unroll
@@ -599,11 +612,12 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kEma>::kThreads, 1) tsn_
       const int rows = *gone ? 0 : a.B;   // (nothing is stored once a wait has run out)
       const bool full = t.wide != 0 && b0 + kQ <= rows && (tile + 1) * kTile <= len;
       __nv_bfloat16* to = t.y + row + 2 * first * t.ysl;
+      const uint32_t y0 = 128 * (kThree ? 2 * tile % 3 : 0), y1 = 128 * (kThree ? (2 * tile + 1) % 3 : 1);
 #pragma unroll 1
       for (int i = first; i < first + 8 / R::kOuts; ++i) {
         float v[2 * kCh];
 #pragma unroll
-        for (int c = 0; c < kCh; ++c) tm_ld2(quarter + kColY + 16 * c + 2 * i, v + 2 * c);
+        for (int c = 0; c < kCh; ++c) tm_ld2(quarter + kColY + (c < 8 ? y0 : y1) + 16 * (c & 7) + 2 * i, v + 2 * c);
         tm_wait_ld();
         landed(v);
 #pragma unroll
@@ -658,7 +672,7 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kEma>::kThreads, 1) tsn_
       const int rows = *gone ? 0 : a.B;
       const bool full = t.wide != 0 && b0 + kQ <= rows && (tile + 1) * kTile <= len;
 #pragma unroll 1
-      for (int i = 0; i < 2 * kQ / R::kCopies; ++i) {   // two sequences, four of their 16 positions
+      for (int i = 0; i < 2 * kQ / (kXn ? R::kCopies : 1); ++i) {   // two sequences, four of their 16 positions
         const int s = kQ / R::kCopies * (warp - R::kCopy) + 2 * (i >> 2) + (lane >> 4), b = b0 + s, k0 = 4 * (i & 3);
         const unsigned char* from = smem + kOffOp + (tile & 1) * kBuf + row_of(s, chunk) + (k0 >> 3) * 128 + (k0 & 4) * 2;
         uint2 v[kCh];
@@ -684,34 +698,50 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kEma>::kThreads, 1) tsn_
     wait(kReady, 0);
     tm_after();
     const uint64_t rows0 = umma_desc(base + kOffOp, 128, 256), mats0 = umma_desc(base + kOffMat, 128, 256);
+    const uint64_t v0 = umma_desc(base + kOffV, 128, 256);
     auto local = [&](uint64_t op, int g) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) umma_tm(tm + kColH, tm + kColV + 64 * g + 8 * j, op + (8 * g + j) * kPlane / 16, kLocal, j > 0);
+      for (int j = 0; j < 8; ++j) {
+        if constexpr (kVShared) umma_16_rows(tm + kColH, v0 + g * (4096 / 16), op + (8 * g + j) * kPlane / 16, kLocal, j);
+        else umma_16_rows(tm + kColH, tm + kColV + 8 * g, op + (8 * g + j) * kPlane / 16, kLocal, j);
+      }
       umma_commit(bar(kHDone));
     };
-    auto outs = [&](uint64_t op, int g) {   // G h
+    auto taps = [&](uint64_t op, int g, uint32_t y) {   // T x
+#pragma unroll
+      for (int j = 0; j < 8; ++j) umma(y + 16 * j, op + (8 * g + j) * kPlane / 16, mats0 + (8 * g + j) * kMat / 16, kTaps, false);
+      umma_commit(bar(kTDone + g));
+    };
+    auto outs = [&](uint64_t op, int g, uint32_t y) {   // G h
 #pragma unroll
       for (int j = 0; j < 8; ++j)
-        umma(tm + kColY + 128 * g + 16 * j, op + (8 * g + j) * kPlane / 16, mats0 + ((8 * g + j) * kMat + 512) / 16, kStates, true);
+        umma(y + 16 * j, op + (8 * g + j) * kPlane / 16, mats0 + ((8 * g + j) * kMat + 512) / 16, kStates, true);
     };
 #pragma unroll 1
     for (int tile = 0; tile < tiles; ++tile) {
       const uint64_t op = rows0 + (tile & 1) * (kBuf / 16);
+      const uint32_t y0 = tm + kColY + 128 * (kThree ? 2 * tile % 3 : 0), y1 = tm + kColY + 128 * (kThree ? (2 * tile + 1) % 3 : 1);
       wait(kOpFull + (tile & 1), tile >> 1);
       tm_after();
       local(op, 0);
-      if (tile > 0) wait(kYRead, tile - 1);
-      tm_after();
-#pragma unroll
-      for (int j = 0; j < kCh; ++j) umma(tm + kColY + 16 * j, op + j * kPlane / 16, mats0 + j * kMat / 16, kTaps, false);
-      umma_commit(bar(kTDone));
+      if (!kThree) {
+        if (tile > 0) wait(kYRead, tile - 1);
+        tm_after();
+      }
+      taps(op, 0, y0);   // (three places: of two tiles ago, whose outputs the tile before has waited for)
+      if (!kThree) taps(op, 1, y1);
       wait(kHRead, 0);
       tm_after();
       local(op, 1);
-      outs(op, 0);
+      if (kThree) {
+        if (tile > 0) wait(kYRead, tile - 1);
+        tm_after();
+        taps(op, 1, y1);
+      }
+      outs(op, 0, y0);
       wait(kHRead, 1);
       tm_after();
-      outs(op, 1);
+      outs(op, 1, y1);
       umma_commit(bar(kYDone));
       umma_commit(bar(kOpEmpty + (tile & 1)));
     }
@@ -747,7 +777,7 @@ namespace {
 double runs_us(const StreamArgs& a, bool xn, int runs, int q) {
   const double tiles = (double)((a.D + kCh - 1) / kCh) * ((a.B + q - 1) / q) * runs;
   const int len = ((a.L + kTile - 1) / kTile + runs - 1) / runs * kTile;
-  double ns = q == 4 ? (a.silu ? (xn ? 23.3 : 22.2) : xn ? 14.7 : 12.4) : a.silu ? (xn ? 31.5 : 28.) : xn ? 26. : 20.;
+  double ns = q == 4 ? (a.silu ? (xn ? 20.4 : 19.8) : xn ? 14.7 : 12.4) : a.silu ? (xn ? 27.8 : 24.6) : xn ? 26. : 20.;
   if (a.mask) ns += q == 4 ? 3.4 : 4.5;
   // (outputs in 16-byte pieces: 24 x 1500 x 1000 103 us, with the second one 138, padded too 160)
   if (a.D % kCh) ns = std::max(ns, (xn ? (a.mask ? 50. : 41.) : 28.5) * (q == 4 ? 0.7 : 1.));

@@ -22,17 +22,22 @@ __device__ __forceinline__ bool umma_elect() {
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
   return one != 0;
 }
-// d (+)= a b for k = 16; a from shared memory, or from tensor memory
+// d (+)= a b for k = 16
 __device__ __forceinline__ void umma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool onto) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
                "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)onto)
                : "memory");
 }
-__device__ __forceinline__ void umma_tm(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, bool onto) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
-               "r"(a), "l"(b), "r"(idesc), "r"((uint32_t)onto)
-               : "memory");
-}
+// d = a b, of which rows 16 j to 16 j + 15 alone are written; a from shared memory, or from tensor memory
+#define MEGA_UMMA_16_ROWS(A, TY)                                                                                                       \
+  const uint32_t off = j & 1 ? 0x0000ffffu : 0xffff0000u; /* (a bit per row: not written) */                                           \
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, 0, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], " A ", %2, %3, {%4, %5, %6, %7}, p;\n\t}" \
+               ::"r"(d), TY(a), "l"(b), "r"(idesc), "r"(j >> 1 == 0 ? off : ~0u), "r"(j >> 1 == 1 ? off : ~0u),                        \
+               "r"(j >> 1 == 2 ? off : ~0u), "r"(j >> 1 == 3 ? off : ~0u)                                                              \
+               : "memory")
+__device__ __forceinline__ void umma_16_rows(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, int j) { MEGA_UMMA_16_ROWS("%1", "l"); }
+__device__ __forceinline__ void umma_16_rows(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, int j) { MEGA_UMMA_16_ROWS("[%1]", "r"); }
+#undef MEGA_UMMA_16_ROWS
 // the barrier completes when all products issued so far by this thread have
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -40,13 +45,18 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
 __device__ __forceinline__ void tm_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tm_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tm_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tm_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tm_alloc(uint32_t to, int columns) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(to), "r"(columns) : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
 }
 __device__ __forceinline__ void tm_free(uint32_t at, int columns) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(at), "r"(columns) : "memory");
+}
+__device__ __forceinline__ void tm_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tm_st8(uint32_t at, const uint32_t* v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(at), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+               "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
 }
 // lane i of a warp: row i of its quarter, consecutive columns
 __device__ __forceinline__ void tm_ld2(uint32_t at, float* v) {
@@ -63,10 +73,4 @@ __device__ __forceinline__ void tm_ld32(uint32_t at, float* v) {
       : "r"(at)
       : "memory");
 }
-__device__ __forceinline__ void tm_st8(uint32_t at, const uint32_t* v) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(at), "r"(v[0]), "r"(v[1]), "r"(v[2]),
-               "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
-               : "memory");
-}
-
 }  // namespace mega
