@@ -16,7 +16,7 @@
 //   - an output's thread holds a (sequence, chunk) row, reads two positions of the 16 channels at a time and writes 32 bytes each;
 //   - the outputs of eight channels have one of two places, with SiLU, whose outputs take long, one of three: T x of the next tile's
 //     first eight does not wait for them then (16 x 4096 x 1024 126 -> 112 us, 8 x 8192 x 1024 192 -> 174, with the second output 200 ->
-//     178).  Tensor memory has room for that where V is in shared memory, from where it costs the plain form 89 -> 98 us.
+//     178; a place is free once its last values are in registers: 109, 159 and 161).  Tensor memory has room for that where V is in shared memory, from where it costs the plain form 89 -> 98 us.
 // The statistics are a chain along time, 12 to 13 instructions a position.  One warp to a scheduler issues 0.4 of them a cycle (41 cycles
 // a position), so three groups of warps take the parts of 32 positions in turn: a group sums its part about a centre of its own before
 // the state of the part before is there, hands the state on, and normalises (28 cycles).  Warps: 12 of the statistics (ahead by up to
@@ -620,6 +620,11 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kEma>::kThreads, 1) tsn_
         for (int c = 0; c < kCh; ++c) tm_ld2(quarter + kColY + (c < 8 ? y0 : y1) + 16 * (c & 7) + 2 * i, v + 2 * c);
         tm_wait_ld();
         landed(v);
+        if (i == first + 8 / R::kOuts - 1) {   // (the next products need not wait for what is on its way to memory)
+          tm_before();
+          __syncwarp();
+          if (lane == 0) arrive(bar(kYRead));
+        }
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
           uint32_t w[8];
@@ -630,9 +635,6 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kEma>::kThreads, 1) tsn_
           to += t.ysl;
         }
       }
-      tm_before();
-      __syncwarp();
-      if (lane == 0) arrive(bar(kYRead));
       if (*any_bad && b < rows) {
         for (int c = 0; c < kCh && d0 + c < a.D; ++c)
           for (int k = max(bad[s_out * kCh + c] - t0, 2 * first); k < 2 * first + kChunk / R::kOuts && t0 + k < len; ++k) {
@@ -777,7 +779,7 @@ namespace {
 double runs_us(const StreamArgs& a, bool xn, int runs, int q) {
   const double tiles = (double)((a.D + kCh - 1) / kCh) * ((a.B + q - 1) / q) * runs;
   const int len = ((a.L + kTile - 1) / kTile + runs - 1) / runs * kTile;
-  double ns = q == 4 ? (a.silu ? (xn ? 20.4 : 19.8) : xn ? 14.7 : 12.4) : a.silu ? (xn ? 27.8 : 24.6) : xn ? 26. : 20.;
+  double ns = q == 4 ? (a.silu ? (xn ? 18.3 : 18.1) : xn ? 14.7 : 12.4) : a.silu ? (xn ? 27.6 : 23.9) : xn ? 26. : 20.;
   if (a.mask) ns += q == 4 ? 3.4 : 4.5;
   // (outputs in 16-byte pieces: 24 x 1500 x 1000 103 us, with the second one 138, padded too 160)
   if (a.D % kCh) ns = std::max(ns, (xn ? (a.mask ? 50. : 41.) : 28.5) * (q == 4 ? 0.7 : 1.));
