@@ -37,7 +37,9 @@
 #include "scan_cluster.cuh"
 #include "scratch.cuh"
 #include "split_mma.cuh"
+#include "stream_cl.cuh"
 #include "tma.cuh"
+#include "tmem_ema.cuh"
 #include "walk.cuh"
 
 namespace mega {
@@ -1297,23 +1299,26 @@ bool lean_call(int dtype, const ScanArgs& a) {
   return dtype == MEGA_BF16 && !a.mask && !a.h_in && !a.h_out && g_options[OPT_DISABLE_MMA].load() == 0 &&
          (g_options[OPT_CHUNK].load() == 3 || (g_options[OPT_CHUNK].load() == 0 && chain_takes(a) && !scan_cluster_first(dtype, a, 1, 1)));
 }
-double chain_us(const ScanArgs& a) {
-  const double L = a.L, n = (double)a.B * a.D * L, tiles = ((a.D + 15) / 16) * (double)((a.B + 7) / 8);
-  if (a.cplx) return 95. + std::max(L * 29e-3, n / 700e3);
-  if (a.mask) return 6. + std::max(L * 42e-3, n / 1300e3);
-  // (16-channel tiles while each of them has an SM: 16 x 4096 x 1024 101 us, 14 x 3140 x 712 81; between that and the segmented form 80 - 170 ns a position)
-  const double ns = tiles > 148. && tiles <= 600. ? 0.28 * tiles : 23.2;
-  return 6. + std::max(L * ns * 1e-3, n / 1300e3);
+double chain_us(const ScanArgs& a, bool lean) {
+  StreamArgs t{};
+  t.B = a.B; t.L = a.L; t.D = a.D; t.N = a.N;
+  t.mask = a.mask;
+  t.cplx = a.cplx;
+  t.silu = a.silu;
+  const double us = mma_ema_chain_us(t);
+  // (what takes leading parts alone may as well do so with accumulators in tensor memory: 16 x 4096 x 1024 74 us for 90, 8 x 8192 x 1024
+  // 95 for 135; a call with states, which is here in all parts, keeps to those)
+  return lean && !a.cplx ? std::min(us, 1.05 * tmem_ema_us(t, false, false)) : us;
 }
 // The form that a call takes otherwise: the scan backward (real bf16 16 x 4096 x 1024: 517 us against 233 here, complex 1481
 // against 459, fp32 539 against 505); forward the cluster kernel, the scan (fp32 complex of that size: 565 against 385; real fp32
 // of 4 sequences 86 against 90), or in bf16 the tensor-core kernel, which walks a sequence as one chain.
-double other_us(int dtype, const ScanArgs& a, bool bwd) {
+double other_us(int dtype, const ScanArgs& a, bool bwd, bool lean) {
   const double L = a.L, n = (double)a.B * a.D * L;
   if (bwd) return a.cplx ? 59. + n / 47e3 : 40. + n / 125e3;
   if (dtype == MEGA_BF16 && g_options[OPT_DISABLE_MMA].load() == 0 && chain_takes(a) &&
       !(a.cplx && (a.mask || (a.h_out && a.L % 32 != 0))))
-    return scan_cluster_first(dtype, a, 1, 1) ? 0.9 * scan_cluster_us(dtype, a) : chain_us(a);
+    return scan_cluster_first(dtype, a, 1, 1) ? 0.9 * scan_cluster_us(dtype, a) : chain_us(a, lean);
   const double one = scan_cluster_us(dtype, a);
   return one < 1e29 ? 0.9 * one : std::min(scan_ema_fwd_us(a), a.cplx ? 25. + n / 123e3 : 15. + n / 270e3);
 }
@@ -1321,7 +1326,7 @@ bool pays(int dtype, const ScanArgs& a, bool bwd, bool lean, double cost, bool s
   if (g_options[OPT_CHUNK].load() >= 2) return true;
   // (a prompt whose state leaves at a length that is no multiple of 32: the tensor-core kernel's head, then a tail)
   if (dtype == MEGA_BF16 && !a.cplx && a.h_out && a.L % 32 != 0) return false;
-  return g_options[OPT_MMA_TILE].load() == 0 && chunk_us(dtype, a, bwd, lean, cost, segmented) < 0.93 * other_us(dtype, a, bwd);
+  return g_options[OPT_MMA_TILE].load() == 0 && chunk_us(dtype, a, bwd, lean, cost, segmented) < 0.93 * other_us(dtype, a, bwd, lean);
 }
 
 template <typename In, typename Out, bool kC, bool kMask, bool kLean = false>

@@ -17,6 +17,16 @@ double mma_chain_us(const StreamArgs& a, bool xn) {
   return (tiles <= 296. ? 11. : 25. + 0.03 * tiles) + a.L * ns * 1e-3 * (a.silu && !xn && !a.mask ? 1.04 : 1.);
 }
 
+// ... and of the EMA by itself: 16-channel tiles while each of them has an SM (16 x 4096 x 1024 101 us, 14 x 3140 x 712 81); between
+// that and the segmented form 80 - 170 ns a position.
+double mma_ema_chain_us(const StreamArgs& a) {
+  const double L = a.L, n = (double)a.B * a.D * L, tiles = ((a.D + 15) / 16) * (double)((a.B + 7) / 8);
+  if (a.cplx) return 95. + std::max(L * 29e-3, n / 700e3);
+  if (a.mask) return 6. + std::max(L * 42e-3, n / 1300e3);
+  const double ns = tiles > 148. && tiles <= 600. ? 0.28 * tiles : 23.2;
+  return 6. + std::max(L * ns * 1e-3, n / 1300e3);
+}
+
 // Envelope: bf16, channel stride 1, ndim <= 16, a padding mask only with real poles, a
 // normalised-copy output (strided like y) only together with the normalisation and distinct from x
 // and y, B >= 4 (rows of the MMAs are sequences) unless the pipelined form applies, L < 2^24, and L
@@ -51,10 +61,11 @@ bool mma_cl_try(int dtype, const void* x, void* y, void* xn, long long xsb, long
   // TimestepNorm -> EMA with real poles: statistics by scalar arithmetic and accumulators in tensor memory (16 x 4096 x 1024 90 us
   // against 140, with the second output 110 against 208, masked 111 against 195), or this kernel's chain (64 x 32768 x 2048, where
   // the power cap slows the other: 5.2 ms both)
-  if (norm && ema && !a_in.cplx) {
+  // The EMA by itself: 16 x 4096 x 1024 74 us (98 here), 8 x 2000 x 1024 30 (52), 64 x 4096 x 2048 540 (471).
+  if (ema && !a_in.cplx && (norm || !masked)) {
     const int asked = forced == 14 ? 4 : forced == 16 ? 9 : forced == 162 ? 10 : forced == 164 ? 12 : forced == 168 ? 16 : 0;
-    if ((asked > 0 || (forced == 0 && tmem_ema_us(a_in, want_xn) < 0.97 * mma_chain_us(a_in, want_xn))) &&
-        tmem_ema_try(dtype, x, y, xn, xsb, xsl, ysb, ysl, a_in, s, asked))
+    const bool better = forced == 0 && tmem_ema_us(a_in, norm, want_xn) < 0.97 * (norm ? mma_chain_us(a_in, want_xn) : mma_ema_chain_us(a_in));
+    if ((asked > 0 || better) && tmem_ema_try(dtype, x, y, xn, xsb, xsl, ysb, ysl, norm, a_in, s, asked))
       return true;
   }
   // Tile width.  Large problems: 64 channels, or 56 when that fills the 148 SMs in fewer or

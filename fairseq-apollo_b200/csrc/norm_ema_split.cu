@@ -165,7 +165,7 @@ bool norm_ema_split_try(int dtype, const void* x, void* y, void* xn, long long x
   const double mma = chunks < chain ? chunks : chain;
   // (of what rounds to bf16 the fused kernel with accumulators in tensor memory, where it is the faster one: 8 x 8192 x 1024 with the
   // second output and SiLU 253 us as norm and products of chunks, 161 so)
-  const bool whole = !a.cplx && mma_takes(dtype, a, xn != nullptr) && tmem_ema_us(a, xn != nullptr) < 0.95 * mma;
+  const bool whole = !a.cplx && mma_takes(dtype, a, xn != nullptr) && tmem_ema_us(a, true, xn != nullptr) < 0.95 * mma;
   if (forced == 0) {   // (what stands in mean_out and the like once the norm has run is what the forms below write too)
     const double chunk = chunk_us(dtype, ea), by_scan = scan - (prompt ? 25.0 : 0.0);
     if ((chunk < 0.88 * (by_scan < mma ? by_scan : mma) && chunk < 0.88 * fused) || (chunk < 1e29 && g_options[OPT_CHUNK].load() == 2))

@@ -43,6 +43,8 @@ bool stream_cl_try(int dtype, const void* x, void* y, void* xn, long long xsb, l
 // stated at the definition).  Same contract as stream_cl_try.
 bool mma_cl_try(int dtype, const void* x, void* y, void* xn, long long xsb, long long xsl, long long xsd,
                 long long ysb, long long ysl, long long ysd, bool norm, const StreamArgs& a, cudaStream_t s);
+// The estimated time of its chain for the EMA by itself.
+double mma_ema_chain_us(const StreamArgs& a);
 // Estimated time of the fused pair with real poles in the forms of mma_cl_kernel.cuh.
 double mma_chain_us(const StreamArgs& a, bool xn);
 // The segmented form of the tensor-core path with the given number of runs (2, 4 or 8), or false

@@ -1,5 +1,5 @@
-// Fused TimestepNorm -> causal EMA for bf16 activations with contiguous channels and real poles: the statistics in plain fp32, a thread
-// per channel of a sequence, the EMA in tcgen05 products with accumulators in tensor memory.
+// TimestepNorm -> causal EMA, and either by itself, for bf16 activations with contiguous channels and real poles: the statistics in plain
+// fp32, a thread per channel of a sequence, the EMA in tcgen05 products with accumulators in tensor memory.
 //
 // A block walks 16 channels of 8 (4) sequences in tiles of 256 positions = 16 chunks of 16.  For one channel the (sequence, chunk) pairs
 // of a tile are the 128 rows of its products; with h the states that enter a chunk and everything else a matrix of the channel,
@@ -28,8 +28,13 @@
 // Two things that cost much: outputs that may stay in L1 (103 us; no_allocate), and code that does not fit the instruction cache (the
 // same walk in 250 KB of code 512 us; what is rare is out of line).  Over all SMs for long the power cap takes 12 % of the clock.
 //
-// What is not finite stays in its channel: a normalised value that is an infinity or a NaN (and whatever follows it) would make NaN of
-// the other seven channels' states, so it goes to the products as zero and the outputs from there on are written as NaN.
+// The EMA by itself (x turned into rows in the statistics' place) takes 74 us there, 98 as a chain of mma_cl_kernel.cuh and 83 as products
+// of chunks with their matrices; 8 x 8192 x 1024 95 for 135.  What is left is the chain from products to states to products to outputs
+// of a tile; without its outputs, or without its states, it takes a fifth less each.  Without states of the layer the input gain is
+// G's, as in the products of chunks, whose distance from float64 this has (2.296e-3; 2.304e-3 with the gain in V, as in the chain).
+//
+// An infinity or a NaN among a chunk's rows would make NaN of the outputs ahead of it too: it goes to the products as zero, and the
+// outputs from there on are written as NaN (the EMA by itself: as the recurrence has them).
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
@@ -46,6 +51,7 @@ namespace mega {
 
 namespace {
 
+enum Form { kPair, kNormOnly, kEmaOnly };   // TimestepNorm -> EMA; either by itself
 constexpr int kMostQ = 8, kCh = 16, kTile = 256, kChunk = 16, kPart = 32;   // kPart: positions of a stage of x
 constexpr int kStages = 4;   // of x, two parts each
 constexpr int kPlane = 4096 + 16, kBuf = kCh * kPlane;   // rows of a channel (16 bytes on: eight channels hit different banks); of a tile
@@ -62,11 +68,14 @@ constexpr int kColH = 0, kColY = 128;
 // kQ: sequences of a block, eight or (few of them: more blocks, each with half of the work) four.
 // Warps: four of the states, four or (SiLU; four sequences, of which half of the warps have rows) eight of the outputs, twelve of the
 // statistics in groups, x, products, and two for the normalised activations where they are an output.
-// TimestepNorm by itself (kEma false) has the statistics' warps, x, and four (two) that write what they leave.
-template <int kQ, bool kSilu, bool kXn, bool kEma>
+// TimestepNorm by itself has the statistics' warps, x, and four (two) that write what they leave; the EMA by itself eight that turn x into
+// rows in the place of the statistics'.
+template <int kQ, bool kSilu, bool kXn, int kForm>
 struct Roles {
-  static constexpr int kPer = kQ / 2, kGroups = 12 / kPer;   // warps of a group of the statistics (two sequences each), groups
-  static constexpr int kOut = 4, kOuts = kSilu || kQ == 4 ? 2 : 1, kStats = kEma ? kOut + 4 * kOuts : 0, kLoad = kStats + 12;
+  static constexpr bool kEma = kForm != kNormOnly;
+  static constexpr int kWarps = kForm == kEmaOnly ? 8 : 12;           // that write rows
+  static constexpr int kPer = kQ / 2, kGroups = kWarps / kPer;           // of a group (two sequences each); groups
+  static constexpr int kOut = 4, kOuts = kForm == kEmaOnly ? 4 : kSilu || kQ == 4 ? 2 : 1, kStats = kEma ? kOut + 4 * kOuts : 0, kLoad = kStats + kWarps;
   static constexpr int kMma = kLoad + 1, kCopy = kMma + (kEma ? 1 : 0), kCopies = !kXn ? 0 : kEma || kQ == 4 ? 2 : 4;
   static constexpr int kThreads = 32 * (kCopy + kCopies);
   static constexpr int kStep = kQ * kCh * 2, kStageBytes = 2 * kPart * kStep;   // bytes from a position of x to the next; of a stage
@@ -76,6 +85,8 @@ struct TmemArgs {
   StreamArgs a;
   __nv_bfloat16 *y, *xn;
   long long ysb, ysl;
+  const __nv_bfloat16* x;   // (beside the tensor map: for values that are not finite)
+  long long xsb, xsl;
   int wide;   // outputs: 32-byte pieces
   // Sequences in runs: a work item is (run, group of sequences, tile of channels); blocks draw items in that order, and one starts
   // from what the item of the run before has left behind its flag.
@@ -226,10 +237,54 @@ __device__ __noinline__ void hand_on(const TmemArgs& t, int b, int d, int slot, 
   if (slot == 2) to[3] = dev2;
 }
 
-template <int kQ, bool kSilu, bool kXn, bool kMask, bool kEma>
-__global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kEma>::kThreads, 1) tsn_ema_tmem_kernel(const __grid_constant__ CUtensorMap tx, const __grid_constant__ TmemArgs t) {
+// The EMA by itself: outputs from an infinity or a NaN on, and the state, are the recurrence's, position by position in fp32 (in place,
+// where the inputs are gone: NaN); so are those of a row whose state is not finite to begin with or in the end.  first: the first of the
+// block's positions to be written.
+__device__ __noinline__ void one_by_one(const TmemArgs& t, int run, int begin, int len, int b, int d, int first, bool silu) {
+  const StreamArgs& a = t.a;
+  if (b >= a.B || d >= a.D || first >= len) return;
+  const bool in_place = t.x == t.y;
+  const size_t o = (size_t)b * a.D + d;
+  float h[16], p[16], q[16], g[16];
+#pragma unroll
+  for (int n = 0; n < 16; ++n) {
+    const bool in = n < a.N;
+    const size_t c = (size_t)d * a.N + (in ? n : 0);
+    const bool apart = !a.h_in && !a.h_out;   // (as the states of the runs are)
+    p[n] = !in ? 0.f : apart ? 1.f : a.p[c];
+    q[n] = in ? a.q[c] : 0.f;
+    g[n] = !in ? 0.f : apart ? a.p[c] * a.g[c] : a.g[c];
+    h[n] = !in ? 0.f : run > 0 ? __ldcg(t.h + o * 16 + n) : a.h_in ? a.h_in[o * a.N + n] : 0.f;
+  }
+  const float om = a.omega[d];
+  const __nv_bfloat16* x = t.x + b * t.xsb + (long long)begin * t.xsl + d;
+  __nv_bfloat16* y = t.y + b * t.ysb + (long long)begin * t.ysl + d;
+#pragma unroll 1
+  for (int i = 0; i < len; ++i) {
+    const float v = in_place ? __int_as_float(0x7fffffff) : __bfloat162float(x[i * t.xsl]);
+    float out = om * v;
+#pragma unroll
+    for (int n = 0; n < 16; ++n) {
+      if (n >= a.N) break;
+      h[n] = fmaf(q[n], h[n], p[n] * v);
+      out = fmaf(g[n], h[n], out);
+    }
+    if (i >= first) y[i * t.ysl] = __float2bfloat16_rn(silu ? siluf_(out) : out);
+  }
+  float* to = run < t.runs - 1 ? t.h : a.h_out;
+  const int pitch = run < t.runs - 1 ? 16 : a.N;
+  if (to)
+#pragma unroll
+    for (int n = 0; n < 16; ++n)
+      if (n < a.N) to[o * pitch + n] = h[n];
+}
+
+template <int kQ, bool kSilu, bool kXn, bool kMask, int kForm>
+__global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kForm>::kThreads, 1) tsn_ema_tmem_kernel(const __grid_constant__ CUtensorMap tx, const __grid_constant__ TmemArgs t) {
   extern __shared__ __align__(128) unsigned char smem[];
-  using R = Roles<kQ, kSilu, kXn, kEma>;
+  using R = Roles<kQ, kSilu, kXn, kForm>;
+  constexpr bool kEma = R::kEma;
+  static_assert(kForm != kEmaOnly || (!kXn && !kMask), "x as it is, whole");
   constexpr int kGroups = R::kGroups, kPer = R::kPer, kStep = R::kStep;
   constexpr bool kThree = kSilu, kVShared = kThree && kQ == 8;   // places of the outputs; V in shared memory
   constexpr int kColV = kQ == 4 ? 64 : 384;
@@ -260,7 +315,7 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kEma>::kThreads, 1) tsn_
       init(kXEmpty + i, 2 * kPer);   // (two parts)
     }
     for (int i = 0; i < 2; ++i) {
-      init(kOpFull + i, 12);
+      init(kOpFull + i, R::kWarps);
       init(kOpEmpty + i, kEma ? 1 : R::kCopies);
       init(kXnRead + i, 2);
     }
@@ -303,7 +358,44 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kEma>::kThreads, 1) tsn_
     __syncthreads();
   }
 
-  if (warp >= R::kStats && warp < R::kLoad) {
+  if (kForm == kEmaOnly && warp >= R::kStats && warp < R::kLoad) {
+    // ---- x into rows: a thread per channel of a sequence, the groups' warps take the parts in turn -----------------------------
+    const int nw = (warp - R::kStats) % kPer, own = (warp - R::kStats) / kPer, ch = lane & 15, s = 2 * nw + (lane >> 4);
+    const bool live = d0 + ch < a.D && b0 + s < a.B;
+    const unsigned char* from = smem + kOffX + nw * 64 + lane * 2;
+    int part = own;
+#pragma unroll 1
+    for (int tile = 0; tile < tiles; ++tile) {
+      if (tile >= 2) wait_all(kOpEmpty + (tile & 1), (tile >> 1) - 1);
+      unsigned char* plane = smem + kOffOp + (tile & 1) * kBuf + ch * kPlane + row_of(s, 0);
+      const int end = min(8 * tile + 8, parts);
+#pragma unroll 1
+      for (; part < end; part += kGroups) {
+        wait_all(kXFull + (part >> 1) % kStages, (part >> 1) / kStages);
+        const unsigned char* v = from + (part & (2 * kStages - 1)) * (R::kStageBytes / 2);
+        unsigned char* to = plane + (part & 4) * 64 + (part & 3) * 32;
+        uint32_t w[kPart / 2], odd = 0u;
+#pragma unroll
+        for (int i = 0; i < kPart / 2; ++i) {
+          w[i] = __byte_perm(*reinterpret_cast<const unsigned short*>(v + 2 * i * kStep), *reinterpret_cast<const unsigned short*>(v + (2 * i + 1) * kStep), 0x5410);
+          odd |= (w[i] & 0x7f807f80u) + 0x00800080u;   // (bits 15 and 31: an exponent of ones)
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          *reinterpret_cast<uint4*>(to + (q >> 1) * 16 + (q & 1) * 128) = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+        if (odd & 0x80008000u) odd_values(to, part * kPart, live, bad + s * kCh + ch, any_bad);
+        __syncwarp();
+        if (lane == 0) arrive(bar(kXEmpty + (part >> 1) % kStages));
+      }
+      if (end == parts && part - kGroups == parts - 1) {   // (behind the end: zeros)
+#pragma unroll 1
+        for (int r = 2 * ((parts - 1) & 7) + 2; r < 16; ++r) zero_row(plane + (r >> 3) * 256 + (r & 7) * 16);
+      }
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) arrive(bar(kOpFull + (tile & 1)));
+    }
+  } else if (kForm != kEmaOnly && warp >= R::kStats && warp < R::kLoad) {
     // ---- statistics: four threads per channel of a sequence, which take every fourth part ---------------------------
     const int nw = (warp - R::kStats) % kPer, own = (warp - R::kStats) / kPer, ch = lane & 15, s = 2 * nw + (lane >> 4), d = d0 + ch, b = b0 + s;
     const bool live = d < a.D && b < a.B;
@@ -470,7 +562,9 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kEma>::kThreads, 1) tsn_
       const int ch = 8 * g + 2 * warp + half, d = d0 + ch;
       const bool in = d < a.D && pole < a.N;
       const size_t o = in ? (size_t)d * a.N + pole : 0;
-      const float p = in ? __ldg(a.p + o) : 0.f, q = in ? __ldg(a.q + o) : 0.f, gm = in ? __ldg(a.g + o) : 0.f;
+      const float gain = in ? __ldg(a.p + o) : 0.f, q = in ? __ldg(a.q + o) : 0.f;
+      const bool apart = kForm == kEmaOnly && !a.h_in && !a.h_out;   // the input gain is G's
+      const float p = apart ? (in ? 1.f : 0.f) : gain, gm = !in ? 0.f : apart ? gain * __ldg(a.g + o) : __ldg(a.g + o);
       double q2 = (double)q * q;
       q2 *= q2;
       q2 *= q2;
@@ -517,6 +611,11 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kEma>::kThreads, 1) tsn_
           const int sq = b0 + 4 * hf + i;
           const size_t o = (size_t)sq * a.D + d;
           h[0][i] = !in || sq >= a.B ? 0.f : run > 0 ? __ldcg(t.h + o * 16 + pole) : a.h_in ? a.h_in[o * a.N + pole] : 0.f;
+          if (kForm == kEmaOnly && !(fabsf(h[0][i]) <= 3.4e38f)) {   // (one_by_one)
+            h[0][i] = 0.f;
+            bad[(4 * hf + i) * kCh + ch] = 0;
+            *any_bad = 1;
+          }
         }
         turn_states();
       }
@@ -582,7 +681,7 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kEma>::kThreads, 1) tsn_
       }
     }
     const bool on = run < t.runs - 1;
-    if ((on || a.h_out) && !*gone) {
+    if ((on || a.h_out || kForm == kEmaOnly) && !*gone) {
 #pragma unroll 1
       for (int unit = 0; unit < kQ / 2; ++unit) {
         const int ch = 8 * (unit / (kQ / 4)) + 2 * warp + half, d = d0 + ch;
@@ -590,9 +689,20 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kEma>::kThreads, 1) tsn_
         for (int i = 0; i < 4; ++i) {
           const int s = 4 * (unit % (kQ / 4)) + i;
           const size_t o = (size_t)(b0 + s) * a.D + d;
-          if (d < a.D && pole < a.N && b0 + s < a.B) {
+          bool redo = false;
+          if constexpr (kForm == kEmaOnly) {   // (one_by_one; in place only where an input was the reason)
+            const unsigned odd = __ballot_sync(0xffffffffu, !(fabsf(h[0][i]) <= 3.4e38f));
+            redo = bad[s * kCh + ch] < len;
+            if (!redo && t.x != t.y && (odd >> (16 * half) & 0xffffu)) {
+              redo = true;
+              if (pole == 0) bad[s * kCh + ch] = 0;
+              *any_bad = 1;
+            }
+            __syncwarp();
+          }
+          if (d < a.D && pole < a.N && b0 + s < a.B && !redo) {
             if (on) t.h[o * 16 + pole] = h[0][i];
-            else a.h_out[o * a.N + pole] = bad[s * kCh + ch] < len ? __int_as_float(0x7fffffff) : h[0][i];
+            else if (a.h_out) a.h_out[o * a.N + pole] = bad[s * kCh + ch] < len ? __int_as_float(0x7fffffff) : h[0][i];
           }
         }
         turn_states();
@@ -602,7 +712,8 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kEma>::kThreads, 1) tsn_
     // ---- outputs: a thread per sequence and chunk ----------------------------------------------------------------
     const int half = lane >> 4, chunk = lane & 15, s_out = 2 * (warp & 3) + half, b = b0 + s_out;
     const uint32_t quarter = tm + ((uint32_t)(warp & 3) << 21);
-    const int first = ((warp - R::kOut) >> 2) * (8 / R::kOuts);   // pairs of positions
+    constexpr int kMine = kChunk / R::kOuts;   // positions
+    const int first = ((warp - R::kOut) >> 2) * kMine;
 #pragma unroll 1
     for (int tile = 0; (warp & 3) < kPer && tile < tiles; ++tile) {
       const int t0 = tile * kTile + chunk * kChunk;
@@ -611,33 +722,33 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kEma>::kThreads, 1) tsn_
       tm_after();
       const int rows = *gone ? 0 : a.B;   // (nothing is stored once a wait has run out)
       const bool full = t.wide != 0 && b0 + kQ <= rows && (tile + 1) * kTile <= len;
-      __nv_bfloat16* to = t.y + row + 2 * first * t.ysl;
+      __nv_bfloat16* to = t.y + row + first * t.ysl;
       const uint32_t y0 = 128 * (kThree ? 2 * tile % 3 : 0), y1 = 128 * (kThree ? (2 * tile + 1) % 3 : 1);
 #pragma unroll 1
-      for (int i = first; i < first + 8 / R::kOuts; ++i) {
+      for (int i = first; i < first + kMine; i += 2) {
         float v[2 * kCh];
+        uint32_t w[2][8];
 #pragma unroll
-        for (int c = 0; c < kCh; ++c) tm_ld2(quarter + kColY + (c < 8 ? y0 : y1) + 16 * (c & 7) + 2 * i, v + 2 * c);
+        for (int c = 0; c < kCh; ++c) tm_ld2(quarter + kColY + (c < 8 ? y0 : y1) + 16 * (c & 7) + i, v + 2 * c);
         tm_wait_ld();
         landed(v);
-        if (i == first + 8 / R::kOuts - 1) {   // (the next products need not wait for what is on its way to memory)
+        if (i == first + kMine - 2) {   // (the next products need not wait for what is on its way to memory)
           tm_before();
           __syncwarp();
           if (lane == 0) arrive(bar(kYRead));
         }
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-          uint32_t w[8];
 #pragma unroll
-          for (int c = 0; c < 8; ++c) w[c] = kSilu ? silu_pair(v[4 * c + k], v[4 * c + 2 + k]) : bf16_pair(v[4 * c + k], v[4 * c + 2 + k]);
-          if (full) store32(to, w);
-          else if (b < rows && t0 + 2 * i + k < len) store_channels(to, t.wide != 0, d0 + 8 < a.D, w);
+          for (int c = 0; c < 8; ++c) w[k][c] = kSilu ? silu_pair(v[4 * c + k], v[4 * c + 2 + k]) : bf16_pair(v[4 * c + k], v[4 * c + 2 + k]);
+          if (full) store32(to, w[k]);
+          else if (b < rows && t0 + i + k < len) store_channels(to, t.wide != 0, d0 + 8 < a.D, w[k]);
           to += t.ysl;
         }
       }
-      if (*any_bad && b < rows) {
+      if (kForm != kEmaOnly && *any_bad && b < rows) {
         for (int c = 0; c < kCh && d0 + c < a.D; ++c)
-          for (int k = max(bad[s_out * kCh + c] - t0, 2 * first); k < 2 * first + kChunk / R::kOuts && t0 + k < len; ++k) {
+          for (int k = max(bad[s_out * kCh + c] - t0, first); k < first + kMine && t0 + k < len; ++k) {
             t.y[row + k * t.ysl + c] = __ushort_as_bfloat16(0x7fff);
             if (kXn) t.xn[row + k * t.ysl + c] = __ushort_as_bfloat16(0x7fff);
           }
@@ -752,6 +863,10 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kEma>::kThreads, 1) tsn_
     const long long start = clock64();
     while (!tried(bar(kEnd), 0) && clock64() - start < 2 * limit + 100000) {}
   }
+  if constexpr (kForm == kEmaOnly) {   // what the products cannot give
+    __syncthreads();
+    if (*any_bad && !*gone && tid < kQ * kCh) one_by_one(t, run, begin, len, b0 + tid / kCh, d0 + tid % kCh, bad[tid], kSilu);
+  }
   __syncwarp();
   tm_before();
   __syncthreads();
@@ -763,10 +878,10 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kEma>::kThreads, 1) tsn_
   }
 }
 
-template <int kQ, bool kSilu, bool kXn, bool kMask, bool kEma = true>
+template <int kQ, bool kSilu, bool kXn, bool kMask, int kForm = kPair>
 void launch_form(const CUtensorMap& tx, const TmemArgs& t, cudaStream_t s) {
   const unsigned grid = (unsigned)(t.per_run * t.runs);
-  launch(tsn_ema_tmem_kernel<kQ, kSilu, kXn, kMask, kEma>, grid, Roles<kQ, kSilu, kXn, kEma>::kThreads, kOffEnd, (void*)s, tx, t);
+  launch(tsn_ema_tmem_kernel<kQ, kSilu, kXn, kMask, kForm>, grid, Roles<kQ, kSilu, kXn, kForm>::kThreads, kOffEnd, (void*)s, tx, t);
 }
 
 }  // namespace
@@ -774,17 +889,18 @@ void launch_form(const CUtensorMap& tx, const TmemArgs& t, cudaStream_t s) {
 namespace {
 
 // us of a call in so many runs, from 200 timings (1 to 64 sequences, 128 to 32768 positions, 256 to 2048 channels on one B200): a
-// block's start and end 6, then ns a position whatever the block's share of the 128 pairs, and rounds of blocks over the SMs (several
-// of them: at the clock that the power cap leaves).
-double runs_us(const StreamArgs& a, bool xn, int runs, int q) {
+// block's start and end 6 (13 with states of the layer behind an EMA by itself), then ns a position whatever the block's share of the
+// 128 pairs, and rounds of blocks over the SMs (several of them: at the clock that the power cap leaves).
+double runs_us(const StreamArgs& a, bool norm, bool xn, int runs, int q) {
   const double tiles = (double)((a.D + kCh - 1) / kCh) * ((a.B + q - 1) / q) * runs;
   const int len = ((a.L + kTile - 1) / kTile + runs - 1) / runs * kTile;
   double ns = q == 4 ? (a.silu ? (xn ? 18.3 : 18.1) : xn ? 14.7 : 12.4) : a.silu ? (xn ? 27.6 : 23.9) : xn ? 26. : 20.;
+  if (!norm) ns = q == 4 ? (a.silu ? 13.4 : 10.5) : a.silu ? 18.3 : 15.9;
   if (a.mask) ns += q == 4 ? 3.4 : 4.5;
   // (outputs in 16-byte pieces: 24 x 1500 x 1000 103 us, with the second one 138, padded too 160)
   if (a.D % kCh) ns = std::max(ns, (xn ? (a.mask ? 50. : 41.) : 28.5) * (q == 4 ? 0.7 : 1.));
   const double rounds = std::max(std::ceil(tiles / 148.), (double)runs);   // (a sequence's runs follow one another)
-  return 4. + rounds * (6. + len * ns * (rounds > 2. ? 1.125e-3 : 1e-3));
+  return 4. + rounds * ((!norm && (a.h_in || a.h_out) ? 13. : 6.) + len * ns * (rounds > 2. ? 1.125e-3 : 1e-3));
 }
 // with the limit of its waits, and the load that a test withholds
 StreamArgs bounded(StreamArgs a) {
@@ -797,12 +913,12 @@ StreamArgs bounded(StreamArgs a) {
 // against 176, 4 x 4096 x 1024 60 against 88; in two rounds 16 x 4096 x 1024 118 against 91)
 int sequences_of(const StreamArgs& a) { return (long long)((a.D + kCh - 1) / kCh) * ((a.B + 3) / 4) <= 148 ? 4 : 8; }
 // runs: what balances the blocks' rounds (16 x 8192 x 5120 in two: 4.5 rounds of the sequence for 5)
-int runs_of(const StreamArgs& a, bool xn) {
+int runs_of(const StreamArgs& a, bool norm, bool xn) {
   int best = 1;
   if (a.mask) return best;   // (the positions that count are known to the run before alone)
-  double least = 0.95 * runs_us(a, xn, 1, 8);
+  double least = 0.95 * runs_us(a, norm, xn, 1, 8);
   for (int n = 2; n <= 8; n *= 2)
-    if (const double us = runs_us(a, xn, n, 8); a.L >= 1024 * n && us < least) {
+    if (const double us = runs_us(a, norm, xn, n, 8); a.L >= 1024 * n && us < least) {
       least = us;
       best = n;
     }
@@ -811,13 +927,14 @@ int runs_of(const StreamArgs& a, bool xn) {
 
 }  // namespace
 
-double tmem_ema_us(const StreamArgs& a, bool xn) {
+double tmem_ema_us(const StreamArgs& a, bool norm, bool xn) {
   const int q = sequences_of(a);
-  return runs_us(a, xn, q == 8 ? runs_of(a, xn) : 1, q);
+  return runs_us(a, norm, xn, q == 8 ? runs_of(a, norm, xn) : 1, q);
 }
 
-bool tmem_ema_try(int dtype, const void* x, void* y, void* xn, long long xsb, long long xsl, long long ysb, long long ysl,
+bool tmem_ema_try(int dtype, const void* x, void* y, void* xn, long long xsb, long long xsl, long long ysb, long long ysl, bool norm,
                   const StreamArgs& a, cudaStream_t s, int asked) {
+  if (!norm && (a.mask || xn)) return false;
   if (dtype != MEGA_BF16 || a.cplx || a.N < 1 || a.N > 16 || a.D % 8 != 0 || (a.h_out && a.L % kChunk != 0) || a.L >= (1 << 24)) return false;
   if (!aligned_to(y, 16) || (xn && !aligned_to(xn, 16)) || ysb % 8 != 0 || ysl % 8 != 0) return false;
   const int q = asked == 4 ? 4 : asked > 0 ? 8 : sequences_of(a);
@@ -827,6 +944,9 @@ bool tmem_ema_try(int dtype, const void* x, void* y, void* xn, long long xsb, lo
   if (!make_tensor_map_3d(&tx, dtype, x, a.D, a.B, a.L, xsb, xsl, kCh, q, 2 * kPart, CU_TENSOR_MAP_SWIZZLE_NONE)) return false;
   TmemArgs t{};
   t.a = bounded(a);
+  t.x = reinterpret_cast<const __nv_bfloat16*>(x);
+  t.xsb = xsb;
+  t.xsl = xsl;
   t.y = reinterpret_cast<__nv_bfloat16*>(y);
   t.xn = reinterpret_cast<__nv_bfloat16*>(xn);
   t.ysb = ysb;
@@ -834,11 +954,16 @@ bool tmem_ema_try(int dtype, const void* x, void* y, void* xn, long long xsb, lo
   t.wide = a.D % 16 == 0 && ysb % 16 == 0 && ysl % 16 == 0 && aligned_to(y, 32) && (!xn || aligned_to(xn, 32));
   t.tiles_d = (a.D + kCh - 1) / kCh;
   t.per_run = (int)per_run;
-  t.runs = q == 4 || a.mask ? 1 : asked > 0 ? asked - 8 : runs_of(a, xn != nullptr);
+  t.runs = q == 4 || a.mask ? 1 : asked > 0 ? asked - 8 : runs_of(a, norm, xn != nullptr);
   const int tiles = (a.L + kTile - 1) / kTile, run_tiles = (tiles + t.runs - 1) / t.runs;
   t.runs = (tiles + run_tiles - 1) / run_tiles;
   t.run_len = run_tiles * kTile;
   auto go = [&]() {
+    if (!norm) {
+      if (q == 4) a.silu ? launch_form<4, true, false, false, kEmaOnly>(tx, t, s) : launch_form<4, false, false, false, kEmaOnly>(tx, t, s);
+      else a.silu ? launch_form<8, true, false, false, kEmaOnly>(tx, t, s) : launch_form<8, false, false, false, kEmaOnly>(tx, t, s);
+      return;
+    }
 #define MEGA_TMEM_OF(Q, SILU, XN) (a.mask ? launch_form<Q, SILU, XN, true>(tx, t, s) : launch_form<Q, SILU, XN, false>(tx, t, s))
 #define MEGA_TMEM(SILU, XN) (q == 4 ? MEGA_TMEM_OF(4, SILU, XN) : MEGA_TMEM_OF(8, SILU, XN))
     if (a.silu) xn ? MEGA_TMEM(true, true) : MEGA_TMEM(true, false);
@@ -864,7 +989,7 @@ bool tmem_ema_try(int dtype, const void* x, void* y, void* xn, long long xsb, lo
   static const char* const kNames[9] = {"", "tsn_ema_mma tmem", "tsn_ema_mma tmem segmented runs=2", "tsn_ema_mma tmem segmented runs=3",
                                         "tsn_ema_mma tmem segmented runs=4", "tsn_ema_mma tmem segmented runs=5", "tsn_ema_mma tmem segmented runs=6",
                                         "tsn_ema_mma tmem segmented runs=7", "tsn_ema_mma tmem segmented runs=8"};
-  g_last_kernel.store(a.mask ? "tsn_ema_mma tmem mask" : kNames[std::min(t.runs, 8)], std::memory_order_relaxed);
+  g_last_kernel.store(!norm ? "ema_mma tmem" : a.mask ? "tsn_ema_mma tmem mask" : kNames[std::min(t.runs, 8)], std::memory_order_relaxed);
   return true;
 }
 
@@ -896,8 +1021,8 @@ bool tmem_norm_try(int dtype, const void* x, void* y, long long xsb, long long x
   t.per_run = (int)blocks;
   t.runs = 1;
   t.run_len = (a.L + kTile - 1) / kTile * kTile;
-  if (q == 4) a.mask ? launch_form<4, false, true, true, false>(tx, t, s) : launch_form<4, false, true, false, false>(tx, t, s);
-  else a.mask ? launch_form<8, false, true, true, false>(tx, t, s) : launch_form<8, false, true, false, false>(tx, t, s);
+  if (q == 4) a.mask ? launch_form<4, false, true, true, kNormOnly>(tx, t, s) : launch_form<4, false, true, false, kNormOnly>(tx, t, s);
+  else a.mask ? launch_form<8, false, true, true, kNormOnly>(tx, t, s) : launch_form<8, false, true, false, kNormOnly>(tx, t, s);
   g_last_kernel.store("tsn_ema_mma tmem norm", std::memory_order_relaxed);
   return true;
 }

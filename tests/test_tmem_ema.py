@@ -1,5 +1,6 @@
-"""Fused TimestepNorm -> EMA with accumulators in tensor memory (bf16, real poles): edges of its tiles (16 channels, 8 sequences, 256
-positions in chunks of 16 and parts of 32), runs of a sequence, padding, values that are not finite, waits that run out."""
+"""TimestepNorm -> EMA, and either by itself, with accumulators in tensor memory (bf16, real poles): edges of the tiles (16 channels,
+8 sequences, 256 positions in chunks of 16 and parts of 32), runs of a sequence, padding, values that are not finite, waits that run
+out."""
 import time
 
 import pytest
@@ -119,6 +120,80 @@ def test_not_finite_stays_in_its_channel(option, value, tile, at):
     for k in ("h", "mean", "var"):
         assert torch.equal(r[k].cpu()[rest], clean[k].cpu()[rest])
     assert not torch.isfinite(r["h"][2, 21]).any() and not torch.isfinite(r["mean"][2, 21])
+
+
+def _ema(x, prm, h0, tile, option, **kw):
+    from fairseq_apollo_b200 import _lib, ops
+    p, q, g = ops.ema_coeffs(*[t.cuda() for t in prm[:4]])
+    option(2, tile)
+    r = ops.ema_forward(x.cuda().transpose(1, 2), p, q, g, prm[4].cuda(), h_in=None if h0 is None else h0.cuda(), **kw)
+    assert "ema_mma tmem" == _lib.last_kernel()
+    y, h = r if isinstance(r, tuple) else (r, None)
+    return y.float().cpu(), None if h is None else h.cpu()
+
+
+# As above: operands and outputs are bf16 (2^-9 each), sums fp32.
+@pytest.mark.parametrize("bsz,length,dim,ndim,state,silu,tile", [
+    (8, 256, 16, 16, False, False, 16),
+    (5, 257, 72, 16, False, True, 16),
+    (9, 544, 40, 16, True, True, 16),
+    (4, 31, 24, 5, False, False, 16),
+    (8, 17, 16, 1, False, False, 16),
+    (7, 544, 40, 16, True, False, 14),
+    (6, 1000, 24, 5, False, True, 14),
+    (4, 33, 8, 16, False, False, 14),
+    (8, 1024, 48, 16, True, False, 162),
+    (9, 2048 + 17, 64, 7, False, True, 168),
+])
+def test_ema_by_itself(option, bsz, length, dim, ndim, state, silu, tile):
+    from oracle import mega_oracle as O
+    x, _, prm, h0, _ = _case(bsz, length, dim, ndim, state, False)
+    y, h = _ema(x, prm, h0, tile, option, want_state=state, silu=silu)
+    want, last = O.ema_forward_recurrence(x.double().transpose(1, 2), *prm, None, h=h0, return_state=True, silu=silu)
+    assert rel_l2(y, want) < 6e-3
+    if state:
+        assert rel_l2(h, last) < 6e-3
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), float("-inf")])
+@pytest.mark.parametrize("tile,at", [(14, 300), (16, 0), (16, 1023), (162, 511), (162, 512)])
+@pytest.mark.parametrize("state", [False, True])
+def test_ema_by_itself_not_finite(option, value, tile, at, state):
+    """From such an input on its row is the recurrence's (weights of one sign: infinite, not NaN), in the state too; a state that comes in
+    infinite makes an infinite row; the other rows know nothing of it."""
+    x, _, prm, h0, _ = _case(8, 1024, 48, 16, True, False, seed=3)
+    prm = [prm[0], prm[1], prm[2].abs(), prm[3].abs(), prm[4].abs()]   # p, g and omega of one sign
+    h0 = h0 if state else None
+    clean, last = _ema(x, prm, h0, tile, option, want_state=state)
+    x[2, at, 21] = value
+    if state:
+        h0[5, 7, 3] = float("inf")
+    y, h = _ema(x, prm, h0, tile, option, want_state=state)
+    rest = torch.ones(8, 48, dtype=torch.bool)
+    rest[2, 21] = False
+    rest[5, 7] = not state
+    assert torch.equal(y[rest], clean[rest]) and torch.equal(y[2, 21, :at], clean[2, 21, :at])
+    same = (lambda t: t.isnan()) if value != value else (lambda t: t == value)
+    assert same(y[2, 21, at:]).all()
+    if state:
+        assert torch.equal(h[rest], last[rest]) and same(h[2, 21]).all()
+        assert (y[5, 7] == float("inf")).all() and h[5, 7, 3] == float("inf") and torch.isfinite(h[5, 7, :3]).all()
+
+
+@pytest.mark.parametrize("bsz,length,dim,silu,state", [(8, 2000, 1024, False, False), (16, 4096, 1024, True, False), (8, 4096, 1024, False, True)])
+def test_ema_by_itself_is_chosen(option, bsz, length, dim, silu, state):
+    """Against the form in the same roundings that walks a sequence as one chain: both are 2.3e-3 from float64 (5e-3 apart at most)."""
+    from fairseq_apollo_b200 import _lib, ops
+    x, _, prm, h0, _ = _case(bsz, length, dim, 16, state, False)
+    y, h = _ema(x, prm, h0, 0, option, want_state=state, silu=silu)
+    p, q, g = ops.ema_coeffs(*[t.cuda() for t in prm[:4]])
+    option(2, 2)
+    r = ops.ema_forward(x.cuda().transpose(1, 2), p, q, g, prm[4].cuda(), h_in=None if h0 is None else h0.cuda(), want_state=state, silu=silu)
+    assert "tmem" not in _lib.last_kernel()
+    want, last = r if isinstance(r, tuple) else (r, None)
+    assert rel_l2(y, want.float()) < 5e-3
+    if state:
+        assert rel_l2(h, last) < 5e-3
 
 
 @pytest.mark.parametrize("tile", [14, 16, 164])
