@@ -1307,7 +1307,7 @@ double chain_us(const ScanArgs& a, bool lean) {
   t.silu = a.silu;
   const double us = mma_ema_chain_us(t);
   // (what takes leading parts alone may as well do so with accumulators in tensor memory: 16 x 4096 x 1024 74 us for 90, 8 x 8192 x 1024
-  // 95 for 135; a call with states, which is here in all parts, keeps to those)
+  // 87 for 135; a call with states, which is here in all parts, keeps to those)
   return lean && !a.cplx ? std::min(us, 1.05 * tmem_ema_us(t, false, false)) : us;
 }
 // The form that a call takes otherwise: the scan backward (real bf16 16 x 4096 x 1024: 517 us against 233 here, complex 1481

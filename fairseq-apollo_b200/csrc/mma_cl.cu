@@ -61,7 +61,7 @@ bool mma_cl_try(int dtype, const void* x, void* y, void* xn, long long xsb, long
   // TimestepNorm -> EMA with real poles: statistics by scalar arithmetic and accumulators in tensor memory (16 x 4096 x 1024 90 us
   // against 140, with the second output 110 against 208, masked 111 against 195), or this kernel's chain (64 x 32768 x 2048, where
   // the power cap slows the other: 5.2 ms both)
-  // The EMA by itself: 16 x 4096 x 1024 74 us (98 here), 8 x 2000 x 1024 30 (52), 64 x 4096 x 2048 540 (471).
+  // The EMA by itself: 16 x 4096 x 1024 74 us (98 here), 8 x 2000 x 1024 28 (52), 64 x 4096 x 2048 540 (471).
   if (ema && !a_in.cplx && (norm || !masked)) {
     const int asked = forced == 14 ? 4 : forced == 16 ? 9 : forced == 162 ? 10 : forced == 164 ? 12 : forced == 168 ? 16 : 0;
     const bool better = forced == 0 && tmem_ema_us(a_in, norm, want_xn) < 0.97 * (norm ? mma_chain_us(a_in, want_xn) : mma_ema_chain_us(a_in));

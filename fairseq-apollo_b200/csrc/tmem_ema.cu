@@ -29,7 +29,8 @@
 // same walk in 250 KB of code 512 us; what is rare is out of line).  Over all SMs for long the power cap takes 12 % of the clock.
 //
 // The EMA by itself (x turned into rows in the statistics' place) takes 74 us there, 98 as a chain of mma_cl_kernel.cuh and 83 as products
-// of chunks with their matrices; 8 x 8192 x 1024 95 for 135.  What is left is the chain from products to states to products to outputs
+// of chunks with their matrices; 8 x 8192 x 1024 87 for 135 (95 with two places of outputs; eight sequences to a
+// block gain nothing from the third).  What is left is the chain from products to states to products to outputs
 // of a tile; without its outputs, or without its states, it takes a fifth less each.  Without states of the layer the input gain is
 // G's, as in the products of chunks, whose distance from float64 this has (2.296e-3; 2.304e-3 with the gain in V, as in the chain).
 //
@@ -286,7 +287,7 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kForm>::kThreads, 1) tsn
   constexpr bool kEma = R::kEma;
   static_assert(kForm != kEmaOnly || (!kXn && !kMask), "x as it is, whole");
   constexpr int kGroups = R::kGroups, kPer = R::kPer, kStep = R::kStep;
-  constexpr bool kThree = kSilu, kVShared = kThree && kQ == 8;   // places of the outputs; V in shared memory
+  constexpr bool kThree = kSilu || (kForm == kEmaOnly && kQ == 4), kVShared = kThree && kQ == 8;   // places of the outputs; V in shared memory
   constexpr int kColV = kQ == 4 ? 64 : 384;
   const StreamArgs& a = t.a;
   const uint32_t base = smem_u32(smem);
@@ -895,7 +896,7 @@ double runs_us(const StreamArgs& a, bool norm, bool xn, int runs, int q) {
   const double tiles = (double)((a.D + kCh - 1) / kCh) * ((a.B + q - 1) / q) * runs;
   const int len = ((a.L + kTile - 1) / kTile + runs - 1) / runs * kTile;
   double ns = q == 4 ? (a.silu ? (xn ? 18.3 : 18.1) : xn ? 14.7 : 12.4) : a.silu ? (xn ? 27.6 : 23.9) : xn ? 26. : 20.;
-  if (!norm) ns = q == 4 ? (a.silu ? 13.4 : 10.5) : a.silu ? 18.3 : 15.9;
+  if (!norm) ns = q == 4 ? (a.silu ? 13.4 : 9.6) : a.silu ? 18.3 : 15.9;
   if (a.mask) ns += q == 4 ? 3.4 : 4.5;
   // (outputs in 16-byte pieces: 24 x 1500 x 1000 103 us, with the second one 138, padded too 160)
   if (a.D % kCh) ns = std::max(ns, (xn ? (a.mask ? 50. : 41.) : 28.5) * (q == 4 ? 0.7 : 1.));
