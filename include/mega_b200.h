@@ -84,8 +84,8 @@ MEGA_API uint64_t mega_launch_count(void);
                                   with two warps per 16-byte column; 222, 224, 422, 124: forms pipelined along the
                                   sequence (channels / 8, warps per column, depth); 82, 84, 88: the segmented
                                   64-channel form in 2, 4, 8 runs; 71: running state in shared memory;
-                                  16: the fused pair with accumulators in tensor memory, eight sequences to a
-                                  block (14: four; 162, 164, 168: in 2, 4, 8 runs);
+                                  16: the fused pair, or the EMA alone, with accumulators in tensor memory, eight
+                                  sequences to a block (14: four; 162, 164, 168: in 2, 4, 8 runs);
                                   0: automatic.  A form that does not apply to a call falls back to automatic */
 #define MEGA_OPT_WAIT_LIMIT 3    /* > 0: SM cycles after which a bounded device-side wait gives up (default ~2 s) */
 #define MEGA_OPT_WITHHOLD_LOAD 4 /* test aid, value k > 0: the tensor-core kernel never issues the TMA load of its
