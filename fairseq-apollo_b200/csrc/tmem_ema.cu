@@ -32,7 +32,8 @@
 // of chunks with their matrices; 8 x 8192 x 1024 87 for 135 (95 with two places of outputs; eight sequences to a
 // block gain nothing from the third).  What is left is the chain from products to states to products to outputs
 // of a tile; without its outputs, or without its states, it takes a fifth less each.  Without states of the layer the input gain is
-// G's, as in the products of chunks, whose distance from float64 this has (2.296e-3; 2.304e-3 with the gain in V, as in the chain).
+// G's, as in the products of chunks, whose distance from float64 this has (2.296e-3; 2.304e-3 with the gain in V, as in the chain;
+// behind the norm 2.865e-3 and 2.871e-3, the chain 2.869e-3).
 //
 // An infinity or a NaN among a chunk's rows would make NaN of the outputs ahead of it too: it goes to the products as zero, and the
 // outputs from there on are written as NaN (the EMA by itself: as the recurrence has them).
@@ -564,7 +565,7 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kForm>::kThreads, 1) tsn
       const bool in = d < a.D && pole < a.N;
       const size_t o = in ? (size_t)d * a.N + pole : 0;
       const float gain = in ? __ldg(a.p + o) : 0.f, q = in ? __ldg(a.q + o) : 0.f;
-      const bool apart = kForm == kEmaOnly && !a.h_in && !a.h_out;   // the input gain is G's
+      const bool apart = !a.h_in && !a.h_out;   // the input gain is G's
       const float p = apart ? (in ? 1.f : 0.f) : gain, gm = !in ? 0.f : apart ? gain * __ldg(a.g + o) : __ldg(a.g + o);
       double q2 = (double)q * q;
       q2 *= q2;
