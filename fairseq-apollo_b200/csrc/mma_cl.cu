@@ -7,11 +7,25 @@
 
 namespace mega {
 
-// us of the fused pair with real poles as this kernel's chain, from 100 timings (4 to 64 sequences, 128 to 4096 positions, 256 to 2048
-// channels on one B200): ns a position by the tiles of 16 channels and 8 sequences.
+// us of the fused pair with real poles as this kernel's chain, from 130 timings (4 to 64 sequences, 128 to 32768 positions, 256 to 2048
+// channels on one B200): ns a position by the tiles of 16 channels and 8 sequences, of the wide tiles by waves of them (64 x 8192 x 2048
+// 1.48 ms, with SiLU 1.82, with the second output too 2.02; 40 x 8192 x 2048 1.06, 1.29 and 2.02).
 double mma_chain_us(const StreamArgs& a, bool xn) {
-  const double tiles = ((a.D + 15) / 16) * (double)((a.B + kSeq - 1) / kSeq);
+  const double groups = (a.B + kSeq - 1) / kSeq, tiles = ((a.D + 15) / 16) * groups, wide = ((a.D + 63) / 64) * groups, less = ((a.D + 55) / 56) * groups;
   const int v = (xn ? 1 : 0) + (a.mask ? 2 : 0);
+  if (wide >= 148. || less >= 148.) {
+    static const double kWave[4] = {83., 112., 97., 125.};
+    const double waves = std::min(std::ceil(wide / 148.), std::ceil(less / 148.));
+    const int nsteps = (a.L + kStep - 1) / kStep;
+    double us = 56. + a.L * waves * kWave[v] * (a.silu ? 1.07 : 1.) * 1e-3, best = waves * 0.96;
+    if (v == 0 && wide > 148.)   // in runs, where mma_cl_try takes them
+      for (int n = 2; n <= 8; n *= 2)
+        if (const double cost = std::ceil(wide * n / 148.) / n; nsteps % n == 0 && nsteps / n >= 64 && cost * 1.02 < best) {
+          best = cost * 1.02;
+          us = 60. + a.L * cost * (a.silu ? 117. : 93.) * 1e-3;
+        }
+    return us;
+  }
   static const double kFew[4] = {32., 49., 45., 58.}, kMore[4] = {53., 69., 70., 87.}, kMany[4] = {1., 1.35, 1.2, 1.55};
   const double ns = tiles <= 148. ? kFew[v] : tiles <= 296. ? kMore[v] : 0.158 * tiles * kMany[v];
   return (tiles <= 296. ? 11. : 25. + 0.03 * tiles) + a.L * ns * 1e-3 * (a.silu && !xn && !a.mask ? 1.04 : 1.);
@@ -59,8 +73,9 @@ bool mma_cl_try(int dtype, const void* x, void* y, void* xn, long long xsb, long
   if (a_in.h_out && (a_in.L % kStep) != 0) return false;
   if ((a_in.B + kSeq - 1) / kSeq > 65535) return false;
   // TimestepNorm -> EMA with real poles: statistics by scalar arithmetic and accumulators in tensor memory (16 x 4096 x 1024 90 us
-  // against 140, with the second output 110 against 208, masked 111 against 195), or this kernel's chain (64 x 32768 x 2048, where
-  // the power cap slows the other: 5.2 ms both)
+  // against 140, with the second output 110 against 208, masked 110 against 195; 64 x 8192 x 2048 1.17 ms against 1.48, with SiLU 1.41
+  // against 1.82), or this kernel's chain (some ragged or short shapes; 64 x 32768 x 2048, where the power cap slows the other,
+  // 4.5 ms in a burst and 5.1 for long against 5.1 and 5.2).
   // The EMA by itself: 16 x 4096 x 1024 74 us (98 here), 8 x 2000 x 1024 28 (52), 64 x 4096 x 2048 540 (471).
   if (ema && !a_in.cplx && (norm || !masked)) {
     const int asked = forced == 14 ? 4 : forced == 16 ? 9 : forced == 162 ? 10 : forced == 164 ? 12 : forced == 168 ? 16 : 0;

@@ -902,7 +902,7 @@ double runs_us(const StreamArgs& a, bool norm, bool xn, int runs, int q) {
   // (outputs in 16-byte pieces: 24 x 1500 x 1000 103 us, with the second one 138, padded too 160)
   if (a.D % kCh) ns = std::max(ns, (xn ? (a.mask ? 50. : 41.) : 28.5) * (q == 4 ? 0.7 : 1.));
   const double rounds = std::max(std::ceil(tiles / 148.), (double)runs);   // (a sequence's runs follow one another)
-  return 4. + rounds * ((!norm && (a.h_in || a.h_out) ? 13. : 6.) + len * ns * (rounds > 2. ? 1.125e-3 : 1e-3));
+  return 4. + rounds * ((!norm && (a.h_in || a.h_out) ? 13. : 6.) + len * ns * (rounds > 2. ? 1.04e-3 : 1e-3));
 }
 // with the limit of its waits, and the load that a test withholds
 StreamArgs bounded(StreamArgs a) {
