@@ -182,12 +182,13 @@ bool norm_ema_split_try(int dtype, const void* x, void* y, void* xn, long long x
     na.xsb = xsb; na.xsl = xsl; na.ysb = ysb; na.ysl = ysl;
     na.prev_count = a.prev_count; na.prev_mean = a.prev_mean; na.prev_var = a.prev_var; na.gamma = a.gamma;
     na.beta = a.beta; na.eps = a.eps; na.count_out = a.count_out; na.mean_out = a.mean_out; na.var_out = a.var_out;
-    const bool normed = (xsd == 1 && ysd == 1 && tmem_norm_us(a) < 0.9 * scan_norm_us(na) && tmem_norm_try(dtype, x, mid, xsb, xsl, ysb, ysl, a, s)) ||
+    // (not where the incoming statistics are gone once it has run: were the second launch refused, the next form starts from x again)
+    const bool normed = (xsd == 1 && ysd == 1 && !stats_in_place(na) && tmem_norm_us(a) < 0.9 * scan_norm_us(na) && tmem_norm_try(dtype, x, mid, xsb, xsl, ysb, ysl, a, s)) ||
                         scan_norm_fwd_try(dtype, na, xsd, ysd, s);
     if (normed &&
         ((chunks < chain && chunk_ema_fwd_try(dtype, dtype, behind_norm(ea, mid), 1, ysd, s, true)) ||
          mma_cl_try(dtype, mid, y, nullptr, ysb, ysl, ysd, ysb, ysl, ysd, false, a, s)))
-      return true;   // (were the second one refused, the next form starts from x again)
+      return true;
   }
   return scan_ema_fwd_try(dtype, ea, xsd, ysd, s);
 }

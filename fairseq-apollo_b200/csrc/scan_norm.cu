@@ -534,14 +534,18 @@ static bool pairs_ok(int dtype, const ScanNormArgs& a, long long ysd) {
 // (us, from 15 shapes of 2 to 67 M elements to 4 %; 537 M are 614)
 double scan_norm_us(const ScanNormArgs& a) { return (14.0 + (double)a.B * a.D * a.L / 740e3) * (a.mask ? 1.32 : 1.0); }
 
+bool stats_in_place(const ScanNormArgs& a) {
+  const size_t n = (size_t)a.B * a.D;
+  for (const float* out : {a.mean_out, a.var_out})
+    if (overlap(out, a.prev_mean, n) || overlap(out, a.prev_var, n)) return true;
+  return false;
+}
+
 bool scan_norm_fwd_try(int dtype, const ScanNormArgs& a, long long xsd, long long ysd, cudaStream_t s) {
   if (!pieces_ok(dtype, a.D) || !rows_ok(dtype, a.x, a.xsb, a.xsl, xsd) || !((a.wide && !a.y) || pairs_ok(dtype, a, ysd)) ||
       a.x == a.y)
     return false;
-  // (every segment's block reads the incoming statistics, the last one's writes the new ones)
-  const size_t n = (size_t)a.B * a.D;
-  for (const float* out : {a.mean_out, a.var_out})
-    if (overlap(out, a.prev_mean, n) || overlap(out, a.prev_var, n)) return false;
+  if (stats_in_place(a)) return false;   // (every segment's block reads the incoming statistics, the last one's writes the new ones)
   return dispatch<false>(dtype, a, s);
 }
 

@@ -26,6 +26,7 @@ struct ScanNormArgs {
 // whole 16-byte pieces, too many sequences for the grid, statistics updated in place) or when there is no scratch memory.
 bool scan_norm_fwd_try(int dtype, const ScanNormArgs& a, long long xsd, long long ysd, cudaStream_t s);
 double scan_norm_us(const ScanNormArgs& a);   // of the forward
+bool stats_in_place(const ScanNormArgs& a);   // whether the new statistics go where the incoming ones are
 bool scan_norm_bwd_try(int dtype, const ScanNormArgs& a, long long xsd, long long ysd, long long gsd, cudaStream_t s);
 
 // Per-channel SequenceNorm: var_out receives rstd; the backward takes the forward's count, mean and rstd as

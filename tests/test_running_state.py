@@ -144,6 +144,41 @@ def test_statistics_updated_in_place(form, length, bsz, dim, split, option):
     assert rel_l2(pm, want[2]) < 1e-5 and rel_l2(pv, want[3]) < 1e-5
 
 
+def _pair_call(bsz, length, dim, gen, shift, in_place, normed=True):
+    """mega_tsn_ema_fwd in bf16, its first output `shift` elements behind a 16-byte boundary; count, mean and variance before and after"""
+    from fairseq_apollo_b200 import _lib
+    rnd = lambda *s: torch.rand(*s, generator=gen, device="cuda")   # noqa: E731
+    x = (torch.randn(bsz, length, dim, generator=gen, device="cuda") * 1.1 + 0.2).bfloat16()
+    y, xn = torch.empty(x.numel() + 8, dtype=x.dtype, device="cuda")[shift:shift + x.numel()].view_as(x), torch.empty_like(x)
+    pc, pm, pv = torch.full((bsz,), 5, device="cuda"), rnd(bsz, dim) * 0.3, rnd(bsz, dim) + 0.5
+    ga, be, prm = rnd(dim) + 0.5, rnd(dim), (rnd(dim, 16) * 0.2, rnd(dim, 16) * 0.5 + 0.4, rnd(dim, 16) - 0.5, rnd(dim))
+    before = [t.clone() for t in (pc, pm, pv, ga, be)]
+    mean, var, cnt = (pm, pv, torch.empty_like(pc)) if in_place else (torch.empty_like(pm), torch.empty_like(pv), torch.empty_like(pc))
+    s, P = x.stride(), lambda t: t.data_ptr()
+    rc = _lib.lib().mega_tsn_ema_fwd(P(x), P(y), P(xn) if normed else None, 1, bsz, length, dim, *s, *s, P(pc), P(pm), P(pv), P(ga), P(be), 1e-5,
+                                     P(cnt), P(mean), P(var), *(P(t) for t in prm), 16, None, None, None, 0,
+                                     torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    return x, y, xn, before, (cnt, mean, var)
+
+
+@pytest.mark.parametrize("split", [2, 0])
+@pytest.mark.parametrize("shift", [0, 4])
+def test_statistics_in_place_where_the_second_launch_is_refused(split, shift, option):
+    """bf16: TimestepNorm could run by itself, but the EMA behind it takes no output off the 16-byte boundaries.  What runs in their
+    place starts from the statistics that came in.  (Outputs are bf16; the variance may come from tf32 products.)"""
+    from oracle import mega_oracle as O
+    option(5, split)
+    x, y, xn, before, after = _pair_call(8, 1024, 2048, torch.Generator(device="cuda").manual_seed(3), shift, True)
+    want = O.timestep_norm(x[:, :, ::64].cpu().double(), before[0].cpu(), *(t[..., ::64].cpu().double() for t in before[1:]), None,
+                           acc_dtype=torch.float64)
+    assert rel_l2(xn[:, :, ::64].float(), want[0]) < 2.0 ** -8
+    assert torch.equal(after[0].cpu(), want[1])
+    assert rel_l2(after[1][:, ::64], want[2]) < 1e-4 and rel_l2(after[2][:, ::64], want[3]) < 1e-3
+    _, apart, _, _, _ = _pair_call(8, 1024, 2048, torch.Generator(device="cuda").manual_seed(3), shift, False)
+    assert rel_l2(y.float(), apart.float()) < 2.0 ** -7
+
+
 @pytest.mark.parametrize("form,length,bsz,dim,split", [
     ("norm", 700, 2, 72, 0), ("group", 700, 2, 128, 0), ("fused", 700, 2, 72, 3), ("fused", 1, 1, 32, 3), ("fused", 2200, 64, 96, 3),
     ("norm", 1, 2, 64, 0),
