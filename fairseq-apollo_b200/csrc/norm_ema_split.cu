@@ -164,8 +164,10 @@ bool norm_ema_split_try(int dtype, const void* x, void* y, void* xn, long long x
   const double chunks = rounds ? 15.0 + (double)a.B * a.D * a.L / 700e3 + chunk_ema_fwd_us(dtype, behind_norm(ea, ea.y)) : 1e30;
   const double mma = chunks < chain ? chunks : chain;
   // (of what rounds to bf16 the fused kernel with accumulators in tensor memory, where it is the faster one: 8 x 8192 x 1024 with the
-  // second output and SiLU 253 us as norm and products of chunks, 161 so)
-  const bool whole = !a.cplx && mma_takes(dtype, a, xn != nullptr) && tmem_ema_us(a, true, xn != nullptr) < 0.95 * mma;
+  // second output and SiLU 253 us as norm and products of chunks, 161 so).  It writes 16-byte pieces, as does what follows on
+  // TimestepNorm by itself; for other outputs there is the scan (8 x 8192 x 1024 with SiLU 370 us; a thread per row 2046)
+  const bool pieces = rows_ok(dtype, y, ysb, ysl, ysd) && (!xn || rows_ok(dtype, xn, ysb, ysl, ysd));
+  const bool whole = pieces && !a.cplx && mma_takes(dtype, a, xn != nullptr) && tmem_ema_us(a, true, xn != nullptr) < 0.95 * mma;
   if (forced == 0) {   // (what stands in mean_out and the like once the norm has run is what the forms below write too)
     const double chunk = chunk_us(dtype, ea), by_scan = scan - (prompt ? 25.0 : 0.0);
     if ((chunk < 0.88 * (by_scan < mma ? by_scan : mma) && chunk < 0.88 * fused) || (chunk < 1e29 && g_options[OPT_CHUNK].load() == 2))
@@ -175,7 +177,7 @@ bool norm_ema_split_try(int dtype, const void* x, void* y, void* xn, long long x
   const double n = (double)a.B * a.D * a.L, margin = n < 4e5 && scan < 45.0 ? 1.0 : 0.9;
   if (forced == 0 && (scan < mma ? scan : mma) > margin * fused) return false;
   if (forced == 0 && mma < scan && whole) return false;
-  if (mma < scan && forced != 3) {
+  if (mma < scan && forced != 3 && pieces) {
     void* mid = xn ? xn : y;
     ScanNormArgs na{};
     na.x = x; na.y = mid; na.B = a.B; na.D = a.D; na.L = a.L;
