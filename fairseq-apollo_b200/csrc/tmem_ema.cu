@@ -752,7 +752,7 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kForm>::kThreads, 1) tsn
         for (int c = 0; c < kCh && d0 + c < a.D; ++c)
           for (int k = max(bad[s_out * kCh + c] - t0, first); k < first + kMine && t0 + k < len; ++k) {
             t.y[row + k * t.ysl + c] = __ushort_as_bfloat16(0x7fff);
-            if (kXn) t.xn[row + k * t.ysl + c] = __ushort_as_bfloat16(0x7fff);
+            if (kXn && !(kMask && __ldg(a.mask + (size_t)b * a.L + t0 + k))) t.xn[row + k * t.ysl + c] = __ushort_as_bfloat16(0x7fff);   // (padded: zero)
           }
       }
     }

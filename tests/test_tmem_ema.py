@@ -122,6 +122,23 @@ def test_not_finite_stays_in_its_channel(option, value, tile, at):
     assert not torch.isfinite(r["h"][2, 21]).any() and not torch.isfinite(r["mean"][2, 21])
 
 
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("tile", [14, 16])
+def test_not_finite_ahead_of_padding(option, value, tile):
+    """The normalised activations of padded positions are zero, behind such a value too; at the others its channel is not finite."""
+    option(2, tile)
+    x, stats, prm, _, _ = _case(8, 700, 48, 16, False, False, seed=4)
+    mask = torch.zeros(8, 700, dtype=torch.bool)
+    mask[2, 310:340] = True
+    mask[2, 512:] = True
+    x[2, 300, 21] = value
+    xn = _run(x, stats, prm, None, mask, want_normed=True)["xn"].cpu()
+    assert (xn[mask] == 0).all()
+    late = ~mask[2]
+    late[:300] = False
+    assert not torch.isfinite(xn[2, late, 21].float()).any()
+
+
 def _ema(x, prm, h0, tile, option, **kw):
     from fairseq_apollo_b200 import _lib, ops
     p, q, g = ops.ema_coeffs(*[t.cuda() for t in prm[:4]])
