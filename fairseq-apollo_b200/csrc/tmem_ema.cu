@@ -302,6 +302,10 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kForm>::kThreads, 1) tsn
   auto wait = [&](int i, int phase) {
     if (!tried(bar(i), phase & 1)) wait_on(bar(i), phase & 1, limit, gone);
   };
+  auto settle = [&](int i, int phase) {   // what the block itself has under way: however short the limit of the other waits is
+    const long long start = clock64();
+    while (!tried(bar(i), phase & 1) && clock64() - start < 2 * limit + 4000000) {}
+  };
   auto wait_all = [&](int i, int phase) {   // (a whole warp)
     wait(i, phase);
     __syncwarp();
@@ -770,12 +774,9 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kForm>::kThreads, 1) tsn
         mbar_expect_tx(full, R::kStageBytes);
         if (k != a.withhold_step) tma_load_3d(smem + kOffX + st * R::kStageBytes, &tx, d0, b0, begin + k * 2 * kPart, full);
       }
-      if (*gone)   // (left early: what is on its way arrives first)
-        for (int i = max(k - kStages, 0); i < k; ++i)
-          if (i != a.withhold_step) {
-            const long long start = clock64();
-            while (!tried(bar(kXFull + i % kStages), i / kStages & 1) && clock64() - start < 2 * limit + 100000) {}
-          }
+      // (what is on its way arrives before the block ends, also where others leave without having waited for it)
+      for (int i = max(k - kStages, 0); i < k; ++i)
+        if (i != a.withhold_step) settle(kXFull + i % kStages, i / kStages);
     }
   } else if (warp >= R::kCopy) {
     // ---- the normalised activations as an output, before states take their place --------------------------------------
@@ -833,7 +834,7 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kForm>::kThreads, 1) tsn
         umma(y + 16 * j, op + (8 * g + j) * kPlane / 16, mats0 + ((8 * g + j) * kMat + 512) / 16, kStates, true);
     };
 #pragma unroll 1
-    for (int tile = 0; tile < tiles; ++tile) {
+    for (int tile = 0; tile < tiles && !*gone; ++tile) {   // (once a wait has run out no more are issued: what is under way ends soon)
       const uint64_t op = rows0 + (tile & 1) * (kBuf / 16);
       const uint32_t y0 = tm + kColY + 128 * (kThree ? 2 * tile % 3 : 0), y1 = tm + kColY + 128 * (kThree ? (2 * tile + 1) % 3 : 1);
       wait(kOpFull + (tile & 1), tile >> 1);
@@ -862,8 +863,7 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kForm>::kThreads, 1) tsn
     }
     // (nothing may be under way when the block ends)
     umma_commit(bar(kEnd));
-    const long long start = clock64();
-    while (!tried(bar(kEnd), 0) && clock64() - start < 2 * limit + 100000) {}
+    settle(kEnd, 0);
   }
   if constexpr (kForm == kEmaOnly) {   // what the products cannot give
     __syncthreads();

@@ -234,6 +234,28 @@ def test_wait_that_runs_out(option, tile):
     assert _lib.device_error() == 0
 
 
+@pytest.mark.parametrize("tile,step", [(14, 5), (16, 62), (164, 5), (164, 14)])   # (of 64 loads, of 16 of a run)
+@pytest.mark.parametrize("alone", [False, True])
+def test_waits_that_run_out_at_once(option, tile, step, alone):
+    """The same with a limit below what a copy takes: whoever waits leaves at once, and what is under way is still waited for, also once
+    the last load has been issued."""
+    from fairseq_apollo_b200 import _lib
+    x, stats, prm, h0, mask = _case(8, 4096, 64, 16, False, False)
+    assert _lib.device_error(reset=True) == 0
+    call = lambda: _ema(x, prm, None, tile, option)[0] if alone else _run(x, stats, prm, h0, mask)["y"]   # noqa: E731
+    option(2, tile)
+    good = call()
+    option(3, 1)
+    option(4, step)
+    for _ in range(3):
+        call()
+    assert _lib.device_error(reset=True) != 0
+    option(3, 0)
+    option(4, 0)
+    assert torch.equal(call(), good)
+    assert _lib.device_error() == 0
+
+
 def test_strides_and_views(option):
     """Rows that are not 32-byte aligned, a time-major view, and outputs written over the inputs give what contiguous tensors give."""
     from fairseq_apollo_b200 import _lib, ops
