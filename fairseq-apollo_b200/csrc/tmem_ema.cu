@@ -313,6 +313,7 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kForm>::kThreads, 1) tsn
 
   int* drawn = reinterpret_cast<int*>(smem + kOffBar + kBars * 8 + 12);
   if (tid == 0) *drawn = t.runs > 1 ? atomicAdd(t.sched, 1) : (int)blockIdx.x;
+  __syncwarp();   // (lane 0 comes from a branch of its own)
   if (kEma && warp == 0) tm_alloc(smem_u32(tm_slot), 512);
   if (tid == 32) {
     auto init = [&](int i, int n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar(i)), "r"(n) : "memory"); };
@@ -865,11 +866,12 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kForm>::kThreads, 1) tsn
     umma_commit(bar(kEnd));
     settle(kEnd, 0);
   }
+  __syncwarp();   // (one lane has issued products, or fetched x: barriers are for warps that are together again)
   if constexpr (kForm == kEmaOnly) {   // what the products cannot give
     __syncthreads();
     if (*any_bad && !*gone && tid < kQ * kCh) one_by_one(t, run, begin, len, b0 + tid / kCh, d0 + tid % kCh, bad[tid], kSilu);
+    __syncwarp();
   }
-  __syncwarp();
   tm_before();
   __syncthreads();
   tm_after();
