@@ -139,7 +139,7 @@ bool norm_chunk_try(int dtype, const ScanArgs& ea, long long xsd, long long ysd,
 
 bool norm_ema_split_try(int dtype, const void* x, void* y, void* xn, long long xsb, long long xsl, long long xsd,
                         long long ysb, long long ysl, long long ysd, const StreamArgs& a, cudaStream_t s) {
-  const int forced = g_options[OPT_SPLIT].load();
+  const int asked = g_options[OPT_SPLIT].load(), forced = asked == 4 ? 0 : asked;   // (4 is about TimestepNorm by itself)
   if (forced == 1 || g_options[OPT_DISABLE_STREAM].load() != 0 || g_options[OPT_DISABLE_MMA].load() != 0 ||
       g_options[OPT_MMA_TILE].load() != 0)   // (a kernel asked for by name)
     return false;

@@ -95,7 +95,7 @@ MEGA_API uint64_t mega_launch_count(void);
 #define MEGA_OPT_SPLIT 5 /* TimestepNorm -> EMA calls: 1: only the kernels that walk a sequence as one chain, 2: the forms
                             parallel over time wherever they apply (3: the scan among them), 0: whichever is estimated
                             to be faster.  TimestepNorm by itself: 3: the scan, 4: the form without tensor cores that
-                            walks a sequence as one chain */
+                            walks a sequence as one chain (the pair then as with 0) */
 #define MEGA_OPT_CHUNK 6 /* causal EMA and its backward as matrix products of chunks: 1: never, 2: wherever that form applies (3: bf16
                             forward in leading parts alone),
                             0: where it is estimated to be faster */

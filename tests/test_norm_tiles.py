@@ -134,6 +134,25 @@ def test_norm_ema_forms_agree(bsz, length, dim, cplx, xn):
             assert rel_l2(r["xn"].float(), res[0]["xn"].float()) < 2.0 ** -7
 
 
+def test_form_of_the_norm_alone_leaves_the_pair():
+    """The form asked for of TimestepNorm by itself (4) is none of the pair, which runs as always."""
+    from fairseq_apollo_b200 import _lib, ops
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    rnd = lambda *s: torch.rand(*s, generator=gen, device="cuda")   # noqa: E731
+    bsz, length, dim = 8, 1024, 2048
+    x = torch.randn(bsz, length, dim, generator=gen, device="cuda").bfloat16()
+    args = (x, torch.full((bsz,), 2, device="cuda"), rnd(bsz, dim) - 0.5, rnd(bsz, dim) + 0.5, rnd(dim) + 0.5, rnd(dim), 1e-5,
+            rnd(dim, 16), rnd(dim, 16) * 0.5 + 0.45, rnd(dim, 16) - 0.5, rnd(dim))
+    res = []
+    for form in (0, 4):
+        _lib.set_option(5, form)
+        try:
+            res.append((ops.tsn_ema_forward(*args)["y"], _lib.last_kernel()))
+        finally:
+            _lib.set_option(5, 0)
+    assert res[0][1] == res[1][1] and torch.equal(res[0][0], res[1][0])
+
+
 # The first step has no variance: its terms, of size eps^-1/2 = 316, cancel against what the later steps carry back, and leave what
 # approximate roots and reciprocals (2^-22) and sums of a handful of such terms leave: 316 x 2^-20 of gradients of size one.  16 bits:
 # the rounding of the output beside that.
