@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 def option():
     from fairseq_apollo_b200 import _lib
     yield _lib.set_option
-    for key in (1, 5, 6):
+    for key in (1, 2, 5, 6):
         _lib.set_option(key, 0)
 
 
@@ -190,6 +190,40 @@ def test_outputs_off_the_boundaries():
     assert _lib.launch_count() - before > 1
     assert rel_l2(y.float(), want.float()) < 2.0 ** -7
     assert rel_l2(after[1], mean) < 1e-4 and rel_l2(after[2], var) < 1e-3
+
+
+@pytest.mark.parametrize("bsz,length,dim,tile", [(8, 1088, 48, 14), (9, 1088, 48, 16), (8, 31, 48, 16), (9, 2144, 40, 164)])
+def test_statistics_in_place_in_bf16(bsz, length, dim, tile, option):
+    """In tensor memory, four and eight sequences to a block, in one and four runs: to the bit what new arrays receive."""
+    from fairseq_apollo_b200 import _lib
+    option(2, tile)
+    run = lambda own: _pair_call(bsz, length, dim, torch.Generator(device="cuda").manual_seed(5), 0, own)   # noqa: E731
+    _, y, xn, _, own = run(True)
+    assert "tmem" in _lib.last_kernel()
+    _, yn, xnn, _, new = run(False)
+    assert torch.equal(y, yn) and torch.equal(xn, xnn) and all(torch.equal(a, b) for a, b in zip(own, new))
+
+
+@pytest.mark.parametrize("bsz,dim", [(8, 64), (16, 1024)])   # four and eight sequences to a block
+@pytest.mark.parametrize("masked", [False, True])
+def test_norm_alone_in_place_in_bf16(bsz, dim, masked, option):
+    from fairseq_apollo_b200 import _lib
+    gen = torch.Generator(device="cuda").manual_seed(dim)
+    rnd = lambda *s: torch.rand(*s, generator=gen, device="cuda")   # noqa: E731
+    x, length = (torch.randn(bsz, 610, dim, generator=gen, device="cuda") + 0.2).bfloat16(), 610
+    mask = torch.zeros(bsz, length, dtype=torch.bool, device="cuda")
+    mask[0], mask[1, 40:77] = True, True
+    pc, pm, pv, ga, be = torch.full((bsz,), 5, device="cuda"), rnd(bsz, dim), rnd(bsz, dim) + 0.5, rnd(dim) + 0.5, rnd(dim)
+    s, P, res = x.stride(), lambda t: t.data_ptr(), []
+    option(5, 4)
+    for own in (False, True):
+        y, cnt, mean, var = torch.empty_like(x), torch.empty_like(pc), pm if own else torch.empty_like(pm), pv if own else torch.empty_like(pv)
+        assert _lib.lib().mega_timestep_norm_fwd(P(x), P(y), 1, bsz, length, dim, *s, *s, P(pc), P(pm), P(pv), P(ga), P(be),
+                                                 P(mask) if masked else None, dim, 1e-5, P(cnt), P(mean), P(var),
+                                                 torch.cuda.current_stream().cuda_stream) == 0
+        assert _lib.last_kernel() == "tsn_ema_mma tmem norm"
+        res.append((y, cnt, mean, var))
+    assert all(torch.equal(a, b) for a, b in zip(*res))
 
 
 @pytest.mark.parametrize("form,length,bsz,dim,split", [

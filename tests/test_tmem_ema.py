@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 def option():
     from fairseq_apollo_b200 import _lib
     yield _lib.set_option
-    for key in (2, 3, 4):
+    for key in (2, 3, 4, 5, 6):
         _lib.set_option(key, 0)
 
 
@@ -197,14 +197,15 @@ def test_ema_by_itself_not_finite(option, value, tile, at, state):
         assert (y[5, 7] == float("inf")).all() and h[5, 7, 3] == float("inf") and torch.isfinite(h[5, 7, :3]).all()
 
 
-@pytest.mark.parametrize("bsz,length,dim,silu,state", [(8, 2000, 1024, False, False), (16, 4096, 1024, True, False), (8, 4096, 1024, False, True)])
+@pytest.mark.parametrize("bsz,length,dim,silu,state", [(8, 2000, 1024, False, False), (16, 4096, 1024, True, False), (8, 4096, 1024, False, True),
+                                                       (3, 4096, 2048, False, False)])
 def test_ema_by_itself_is_chosen(option, bsz, length, dim, silu, state):
     """Against the form in the same roundings that walks a sequence as one chain: both are 2.3e-3 from float64 (5e-3 apart at most)."""
     from fairseq_apollo_b200 import _lib, ops
     x, _, prm, h0, _ = _case(bsz, length, dim, 16, state, False)
     y, h = _ema(x, prm, h0, 0, option, want_state=state, silu=silu)
     p, q, g = ops.ema_coeffs(*[t.cuda() for t in prm[:4]])
-    option(2, 2)
+    option(2, 224)
     r = ops.ema_forward(x.cuda().transpose(1, 2), p, q, g, prm[4].cuda(), h_in=None if h0 is None else h0.cuda(), want_state=state, silu=silu)
     assert "tmem" not in _lib.last_kernel()
     want, last = r if isinstance(r, tuple) else (r, None)
@@ -257,7 +258,7 @@ def test_waits_that_run_out_at_once(option, tile, step, alone):
 
 
 def test_strides_and_views(option):
-    """Rows that are not 32-byte aligned, a time-major view, and outputs written over the inputs give what contiguous tensors give."""
+    """Rows that are not 32-byte aligned and a time-major view give what contiguous tensors give."""
     from fairseq_apollo_b200 import _lib, ops
     x, stats, prm, h0, mask = _case(8, 320, 32, 16, False, False)
     option(2, 16)
@@ -270,6 +271,54 @@ def test_strides_and_views(option):
         r = ops.tsn_ema_forward(v, *[t.cuda() for t in stats], 1e-5, p, q, g, prm[4].cuda())["y"]
         assert "tmem" in _lib.last_kernel()
         assert torch.equal(r, want)
+
+
+@pytest.mark.parametrize("value", [None, float("nan"), float("inf")])
+def test_ema_over_its_inputs(option, value):
+    """Behind TimestepNorm by itself, whose outputs lie where the EMA's go: what it gives from a place of their own.  From a value that is
+    not finite on its row is NaN, in the state too, and the other rows know nothing of it."""
+    from fairseq_apollo_b200 import _lib
+    x, stats, prm, h0, _ = _case(8, 4096, 1024, 16, True, False, seed=6)
+    if value is not None:
+        x[2, 300, 21] = value
+    option(5, 2)
+    option(6, 1)
+    apart = _run(x, stats, prm, h0, None, want_state=True, want_normed=True)
+    assert _lib.last_kernel() == "ema_mma tmem"
+    over = _run(x, stats, prm, h0, None, want_state=True)
+    assert _lib.last_kernel() == "ema_mma tmem"
+    a, b = over["y"].transpose(1, 2), apart["y"].transpose(1, 2)
+    rest = torch.ones(8, 1024, dtype=torch.bool)
+    rest[2, 21] = value is None
+    assert torch.equal(a[rest], b[rest]) and torch.equal(over["h"][rest], apart["h"][rest])
+    assert torch.equal(a[2, 21, :300], b[2, 21, :300])
+    if value is not None:
+        assert a[2, 21, 300:].isnan().all() and over["h"][2, 21].isnan().all()
+
+
+# What a call takes by itself, real poles, against the other form.  The two are apart by no more than their distances from float64
+# together, which their own tests bound by 6e-3 (above) and 1e-2 (the chain: test_tensor_core_path_with_padding_mask).
+@pytest.mark.parametrize("bsz,length,dim,masked,normed,name", [
+    (16, 4096, 1024, False, False, "tsn_ema_mma tmem"),
+    (16, 4096, 1024, True, False, "tsn_ema_mma tmem mask"),
+    (8, 1024, 2048, False, True, "tsn_ema_mma tmem"),
+    (8, 1024, 2048, True, True, "tsn_ema_mma tmem mask"),
+    (3, 4096, 2048, False, False, "tsn_ema_mma tmem"),      # fewer than four sequences
+    (16, 100, 1024, False, False, "tsn_ema_mma tile=2 warps_per_column=2 pipe=4 norm ema"),      # the chain of mma.sync
+    (24, 1500, 1000, False, False, "tsn_ema_mma tile=2 warps_per_column=2 pipe=1 norm ema"),
+])
+def test_pair_is_chosen(option, bsz, length, dim, masked, normed, name):
+    from fairseq_apollo_b200 import _lib
+    x, stats, prm, _, mask = _case(bsz, length, dim, 16, False, masked)
+    r = _run(x, stats, prm, None, mask, want_normed=normed)
+    assert _lib.last_kernel() == name
+    option(2, 16 if "tile" in name else 22 if masked or normed else 224)
+    other = _run(x, stats, prm, None, mask, want_normed=normed)
+    assert ("tmem" in _lib.last_kernel()) == ("tile" in name)
+    assert rel_l2(r["y"].float(), other["y"].float()) < 1.6e-2
+    assert rel_l2(r["mean"], other["mean"]) < 1e-4 and rel_l2(r["var"], other["var"]) < 2e-3
+    if normed:
+        assert rel_l2(r["xn"].float(), other["xn"].float()) < 1.4e-2   # (4e-3 and 1e-2)
 
 
 @pytest.mark.parametrize("bsz,length,dim,masked", [(8, 256, 16, False), (5, 290, 72, False), (4, 33, 8, True), (16, 1000, 40, True),
