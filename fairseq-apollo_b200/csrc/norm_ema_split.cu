@@ -165,9 +165,16 @@ bool norm_ema_split_try(int dtype, const void* x, void* y, void* xn, long long x
   const double mma = chunks < chain ? chunks : chain;
   // (of what rounds to bf16 the fused kernel with accumulators in tensor memory, where it is the faster one: 8 x 8192 x 1024 with the
   // second output and SiLU 253 us as norm and products of chunks, 161 so).  It writes 16-byte pieces, as does what follows on
-  // TimestepNorm by itself; for other outputs there is the scan (8 x 8192 x 1024 with SiLU 370 us; a thread per row 2046)
-  const bool pieces = rows_ok(dtype, y, ysb, ysl, ysd) && (!xn || rows_ok(dtype, xn, ysb, ysl, ysd));
-  const bool whole = pieces && !a.cplx && mma_takes(dtype, a, xn != nullptr) && tmem_ema_us(a, true, xn != nullptr) < 0.95 * mma;
+  // TimestepNorm by itself; for other outputs there is the scan (8 x 8192 x 1024 370 us; a thread per row 2046).
+  // Statistics updated in place: TimestepNorm by itself may not overwrite them before the EMA behind it has been taken, so these calls
+  // are the scan's too, in fp32 throughout.
+  ScanNormArgs na{};
+  na.x = x; na.y = xn ? xn : y; na.B = a.B; na.D = a.D; na.L = a.L;
+  na.xsb = xsb; na.xsl = xsl; na.ysb = ysb; na.ysl = ysl;
+  na.prev_count = a.prev_count; na.prev_mean = a.prev_mean; na.prev_var = a.prev_var; na.gamma = a.gamma;
+  na.beta = a.beta; na.eps = a.eps; na.count_out = a.count_out; na.mean_out = a.mean_out; na.var_out = a.var_out;
+  const bool parts = rows_ok(dtype, y, ysb, ysl, ysd) && (!xn || rows_ok(dtype, xn, ysb, ysl, ysd)) && !stats_in_place(na);
+  const bool whole = parts && !a.cplx && mma_takes(dtype, a, xn != nullptr) && tmem_ema_us(a, true, xn != nullptr) < 0.95 * mma;
   if (forced == 0) {   // (what stands in mean_out and the like once the norm has run is what the forms below write too)
     const double chunk = chunk_us(dtype, ea), by_scan = scan - (prompt ? 25.0 : 0.0);
     if ((chunk < 0.88 * (by_scan < mma ? by_scan : mma) && chunk < 0.88 * fused) || (chunk < 1e29 && g_options[OPT_CHUNK].load() == 2))
@@ -177,20 +184,14 @@ bool norm_ema_split_try(int dtype, const void* x, void* y, void* xn, long long x
   const double n = (double)a.B * a.D * a.L, margin = n < 4e5 && scan < 45.0 ? 1.0 : 0.9;
   if (forced == 0 && (scan < mma ? scan : mma) > margin * fused) return false;
   if (forced == 0 && mma < scan && whole) return false;
-  if (mma < scan && forced != 3 && pieces) {
+  if (mma < scan && forced != 3 && parts) {
     void* mid = xn ? xn : y;
-    ScanNormArgs na{};
-    na.x = x; na.y = mid; na.B = a.B; na.D = a.D; na.L = a.L;
-    na.xsb = xsb; na.xsl = xsl; na.ysb = ysb; na.ysl = ysl;
-    na.prev_count = a.prev_count; na.prev_mean = a.prev_mean; na.prev_var = a.prev_var; na.gamma = a.gamma;
-    na.beta = a.beta; na.eps = a.eps; na.count_out = a.count_out; na.mean_out = a.mean_out; na.var_out = a.var_out;
-    // (not where the incoming statistics are gone once it has run: were the second launch refused, the next form starts from x again)
-    const bool normed = (xsd == 1 && ysd == 1 && !stats_in_place(na) && tmem_norm_us(a) < 0.9 * scan_norm_us(na) && tmem_norm_try(dtype, x, mid, xsb, xsl, ysb, ysl, a, s)) ||
+    const bool normed = (xsd == 1 && ysd == 1 && tmem_norm_us(a) < 0.9 * scan_norm_us(na) && tmem_norm_try(dtype, x, mid, xsb, xsl, ysb, ysl, a, s)) ||
                         scan_norm_fwd_try(dtype, na, xsd, ysd, s);
     if (normed &&
         ((chunks < chain && chunk_ema_fwd_try(dtype, dtype, behind_norm(ea, mid), 1, ysd, s, true)) ||
          mma_cl_try(dtype, mid, y, nullptr, ysb, ysl, ysd, ysb, ysl, ysd, false, a, s)))
-      return true;
+      return true;   // (were the second one refused, the next form starts from x again)
   }
   return scan_ema_fwd_try(dtype, ea, xsd, ysd, s);
 }
