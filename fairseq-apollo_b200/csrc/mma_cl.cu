@@ -8,16 +8,17 @@
 namespace mega {
 
 // us of the fused pair with real poles as this kernel's chain, from 130 timings (4 to 64 sequences, 128 to 32768 positions, 256 to 2048
-// channels on one B200): ns a position by the tiles of 16 channels and 8 sequences, of the wide tiles by waves of them (64 x 8192 x 2048
-// 1.48 ms, with SiLU 1.82, with the second output too 2.02; 40 x 8192 x 2048 1.06, 1.29 and 2.02).
+// channels on one B200) and 4300 of up to 67 M elements (20 to 6000 positions; these to 0.86 - 1.06 of the time, one in twenty outside):
+// a block's start and end, then ns a position by the tiles of 16 channels and 8 sequences, of the wide tiles by waves of them (40 x 94 x
+// 1736 with SiLU 38 us, 25 x 1621 x 1528 197; 64 x 8192 x 2048 1.41 ms in a row, with SiLU 1.52).
 double mma_chain_us(const StreamArgs& a, bool xn) {
   const double groups = (a.B + kSeq - 1) / kSeq, tiles = ((a.D + 15) / 16) * groups, wide = ((a.D + 63) / 64) * groups, less = ((a.D + 55) / 56) * groups;
   const int v = (xn ? 1 : 0) + (a.mask ? 2 : 0);
   if (wide >= 148. || less >= 148.) {
     static const double kWave[4] = {83., 112., 97., 125.};
-    const double waves = std::min(std::ceil(wide / 148.), std::ceil(less / 148.));
+    const double w7 = std::ceil(less / 148.), waves = v != 0 ? w7 : std::min(std::ceil(wide / 148.), w7);   // (masks and xn: 56 channels alone)
     const int nsteps = (a.L + kStep - 1) / kStep;
-    double us = 56. + a.L * waves * kWave[v] * (a.silu ? 1.07 : 1.) * 1e-3, best = waves * 0.96;
+    double us = waves * (27. + a.L * kWave[v] * (waves < 2. ? 1.1 : 1.) * (a.silu ? 1.07 : 1.) * 1e-3), best = waves * 0.96;
     if (v == 0 && wide > 148.)   // in runs, where mma_cl_try takes them
       for (int n = 2; n <= 8; n *= 2)
         if (const double cost = std::ceil(wide * n / 148.) / n; nsteps % n == 0 && nsteps / n >= 64 && cost * 1.02 < best) {
@@ -26,9 +27,9 @@ double mma_chain_us(const StreamArgs& a, bool xn) {
         }
     return us;
   }
-  static const double kFew[4] = {32., 49., 45., 58.}, kMore[4] = {53., 69., 70., 87.}, kMany[4] = {1., 1.35, 1.2, 1.55};
-  const double ns = tiles <= 148. ? kFew[v] : tiles <= 296. ? kMore[v] : 0.158 * tiles * kMany[v];
-  return (tiles <= 296. ? 11. : 25. + 0.03 * tiles) + a.L * ns * 1e-3 * (a.silu && !xn && !a.mask ? 1.04 : 1.);
+  static const double kFew[4] = {31.3, 48.5, 49., 64.}, kMore[4] = {51., 67.5, 62.5, 81.}, kMany[4] = {1., 1.28, 1.17, 1.53};
+  if (tiles <= 148.) return (v == 0 ? 11. : 14.3) + a.L * kFew[v] * 1e-3;
+  return tiles <= 296. ? 15.4 + a.L * kMore[v] * 1e-3 : 20.4 + a.L * std::min(0.3 * tiles, 109.) * kMany[v] * 1e-3;
 }
 
 // ... and of the EMA by itself: 16-channel tiles while each of them has an SM (16 x 4096 x 1024 101 us, 14 x 3140 x 712 81); between
@@ -79,7 +80,7 @@ bool mma_cl_try(int dtype, const void* x, void* y, void* xn, long long xsb, long
   // The EMA by itself: 16 x 4096 x 1024 74 us (98 here), 8 x 2000 x 1024 28 (52), 64 x 4096 x 2048 540 (471).
   if (ema && !a_in.cplx && (norm || !masked)) {
     const int asked = forced == 14 ? 4 : forced == 16 ? 9 : forced == 162 ? 10 : forced == 164 ? 12 : forced == 168 ? 16 : 0;
-    const bool better = forced == 0 && tmem_ema_us(a_in, norm, want_xn) < 0.97 * (norm ? mma_chain_us(a_in, want_xn) : mma_ema_chain_us(a_in));
+    const bool better = forced == 0 && tmem_ema_us(a_in, norm, want_xn) < (norm ? 0.95 * mma_chain_us(a_in, want_xn) : 0.97 * mma_ema_chain_us(a_in));
     if ((asked > 0 || better) && tmem_ema_try(dtype, x, y, xn, xsb, xsl, ysb, ysl, norm, a_in, s, asked))
       return true;
   }

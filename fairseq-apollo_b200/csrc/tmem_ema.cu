@@ -892,19 +892,25 @@ void launch_form(const CUtensorMap& tx, const TmemArgs& t, cudaStream_t s) {
 
 namespace {
 
-// us of a call in so many runs, from 200 timings (1 to 64 sequences, 128 to 32768 positions, 256 to 2048 channels on one B200): a
-// block's start and end 6 (13 with states of the layer behind an EMA by itself), then ns a position whatever the block's share of the
-// 128 pairs, and rounds of blocks over the SMs (several of them: at the clock that the power cap leaves).
+// us of a call in so many runs, from 200 timings (1 to 64 sequences, 128 to 32768 positions, 256 to 2048 channels on one B200) and, of
+// the pair, 4300 of 20 to 6000 positions (to 0.9 - 1.1 of the time, one in ten outside): a block's start and end, then ns a position, and
+// rounds of blocks over the SMs.  A tile that is not whole takes some part of a whole one's time.
 double runs_us(const StreamArgs& a, bool norm, bool xn, int runs, int q) {
   const double tiles = (double)((a.D + kCh - 1) / kCh) * ((a.B + q - 1) / q) * runs;
   const int len = ((a.L + kTile - 1) / kTile + runs - 1) / runs * kTile;
-  double ns = q == 4 ? (a.silu ? (xn ? 18.3 : 18.1) : xn ? 14.7 : 12.4) : a.silu ? (xn ? 27.6 : 23.9) : xn ? 26. : 20.;
-  if (!norm) ns = q == 4 ? (a.silu ? 13.4 : 9.6) : a.silu ? 18.3 : 15.9;
-  if (a.mask) ns += q == 4 ? 3.4 : 4.5;
-  // (outputs in 16-byte pieces: 24 x 1500 x 1000 103 us, with the second one 138, padded too 160)
-  if (a.D % kCh) ns = std::max(ns, (xn ? (a.mask ? 50. : 41.) : 28.5) * (q == 4 ? 0.7 : 1.));
   const double rounds = std::max(std::ceil(tiles / 148.), (double)runs);   // (a sequence's runs follow one another)
-  return 4. + rounds * ((!norm && (a.h_in || a.h_out) ? 13. : 6.) + len * ns * (rounds > 2. ? 1.04e-3 : 1e-3));
+  if (!norm) {   // (13 with states of the layer; several rounds at the clock that the power cap leaves)
+    double ns = q == 4 ? (a.silu ? 13.4 : 9.6) : a.silu ? 18.3 : 15.9;
+    if (a.D % kCh) ns = std::max(ns, 28.5 * (q == 4 ? 0.7 : 1.));
+    return 4. + rounds * ((a.h_in || a.h_out ? 13. : 6.) + len * ns * (rounds > 2. ? 1.04e-3 : 1e-3));
+  }
+  // [sequences of a block][outputs in 32- or 16-byte pieces][SiLU + 2 second output]; with masks that pad something
+  // (16 x 4096 x 1024 88 us, SiLU 107, second output 107, both 124; 8 x 8192 x 1024 112, 159 with SiLU; 24 x 1500 x 1000 103 and 138)
+  static const double kNs[2][2][4] = {{{12.2, 18.1, 14.7, 18.5}, {16., 18.3, 22., 24.3}}, {{18.7, 23.3, 23.5, 27.4}, {25.5, 28.4, 38., 40.}}};
+  const bool pieces = a.D % kCh != 0;
+  const double ns = kNs[q == 8][pieces][(a.silu ? 1 : 0) + (xn ? 2 : 0)] + (!a.mask ? 0. : q == 4 ? 3. : pieces ? 6.5 : 5.);
+  const double steps = runs > 1 ? len : 0.5 * (a.L + len);
+  return 3.5 + rounds * (7.5 + (a.silu ? 1. : 0.) + (xn ? 2. : 0.) - (a.mask ? 1. : 0.) + steps * ns * 1e-3);
 }
 // with the limit of its waits, and the load that a test withholds
 StreamArgs bounded(StreamArgs a) {
@@ -933,7 +939,8 @@ int runs_of(const StreamArgs& a, bool norm, bool xn) {
 
 double tmem_ema_us(const StreamArgs& a, bool norm, bool xn) {
   const int q = sequences_of(a);
-  return runs_us(a, norm, xn, q == 8 ? runs_of(a, norm, xn) : 1, q);
+  const double us = runs_us(a, norm, xn, q == 8 ? runs_of(a, norm, xn) : 1, q);
+  return norm && us > 400. ? 1.06 * us : us;   // (at the clock that the power cap leaves: 64 x 8192 x 2048 1.25 ms in a row, one at a time 1.17)
 }
 
 bool tmem_ema_try(int dtype, const void* x, void* y, void* xn, long long xsb, long long xsl, long long ysb, long long ysl, bool norm,

@@ -306,6 +306,8 @@ def test_ema_over_its_inputs(option, value):
     (3, 4096, 2048, False, False, "tsn_ema_mma tmem"),      # fewer than four sequences
     (16, 100, 1024, False, False, "tsn_ema_mma tile=2 warps_per_column=2 pipe=4 norm ema"),      # the chain of mma.sync
     (24, 1500, 1000, False, False, "tsn_ema_mma tile=2 warps_per_column=2 pipe=1 norm ema"),
+    (58, 96, 1096, False, False, "tsn_ema_mma tile=8 warps_per_column=1 pipe=1 norm ema"),      # (37 us, in tensor memory 49)
+    (37, 154, 1120, False, True, "tsn_ema_mma tile=2 warps_per_column=2 pipe=1 norm ema xn"),   # (43, 54)
 ])
 def test_pair_is_chosen(option, bsz, length, dim, masked, normed, name):
     from fairseq_apollo_b200 import _lib
