@@ -434,7 +434,7 @@ __global__ void __launch_bounds__(kWarps * 32) sqn_bwd_emit_kernel(SegNorm s) {
 
 // Segments: enough blocks of four for the SMs (about six of them resident each) in few rounds, at least 64 steps
 // each and at most 64 of them, since every segment combines those before it.
-static void pick_segments(const ScanNormArgs& a, int resident, int width, SegNorm& s) {
+static double pick_segments(const ScanNormArgs& a, int resident, int width, SegNorm& s) {
   const long long strips = (long long)((a.D + width - 1) / width) * a.B;
   const double slots = 148.0 * resident;
   double best = 1e30;
@@ -450,6 +450,7 @@ static void pick_segments(const ScanNormArgs& a, int resident, int width, SegNor
     }
     if (t == 64) break;
   }
+  return best;
 }
 
 template <typename T, bool kMask>
@@ -513,7 +514,15 @@ static bool dispatch(int dtype, const ScanNormArgs& a, cudaStream_t st) {
   if (g_options[OPT_DISABLE_STREAM].load() != 0 || a.B > 65535) return false;
   SegNorm s{};
   s.a = a;
-  pick_segments(a, !kBwd ? 6 : dtype == MEGA_F32 ? 3 : 4, 64, s);   // (resident blocks)
+  // Resident blocks.  Backward: a fourth shares the FMA pipe with the others, so in one round it has to make the walks a good deal shorter
+  // (32 x 2048 x 512 136 us with three, 128 with four; 50 x 273 x 288 36 and 42; in two rounds 38 x 1706 x 480 142 and 125).
+  const double cost = pick_segments(a, kBwd ? 3 : 6, 64, s);
+  if (kBwd && dtype != MEGA_F32) {
+    SegNorm four = s;
+    const double least = pick_segments(a, 4, 64, four);
+    const bool rounds = (long long)((a.D + 63) / 64) * a.B * ((four.S + kWarps - 1) / kWarps) > 4 * 148;
+    if (least < (rounds ? 1. : 0.85) * cost) s = four;
+  }
   const size_t n = (size_t)a.B * s.S * a.D;
   Scratch sc(Scratch::padded(n * 4) * (kBwd ? 5 : 2) + Scratch::padded((size_t)a.B * s.S * 4), st);
   if (!sc) return false;
