@@ -263,6 +263,28 @@ __device__ __forceinline__ uint32_t vec_off(int seq, int t, int cg) {
   return (uint32_t)(row * (kCg * 16) + (cg << 4));
 }
 
+// The first position of a sequence that counts, 32 at a time by the four lanes that share it (L: none; all lanes of a warp come).  Out of
+// line, like the value there (prev: instead of one that is not finite): nothing of them is held in registers beside the step loop.
+__device__ __noinline__ int first_counted(const unsigned char* row, int L, bool wanted, int q) {
+  int at = L;
+  for (int t0 = 0; t0 < L && __any_sync(0xffffffffu, wanted && at == L); t0 += 32) {
+    int m = L;
+#pragma unroll
+    for (int u = 7; u >= 0; --u) {
+      const int t = t0 + 4 * u + q;
+      if (__ldg(row + min(t, L - 1)) == 0 && t < L) m = t;
+    }
+    m = min(m, __shfl_xor_sync(0xffffffffu, m, 1));
+    m = min(m, __shfl_xor_sync(0xffffffffu, m, 2));
+    at = min(at, m);
+  }
+  return wanted ? at : L;
+}
+__device__ __noinline__ float first_value(const __nv_bfloat16* x, const float* prev) {
+  const float v = __bfloat162float(*x);
+  return fabsf(v) <= 3.4e38f ? v : *prev;
+}
+
 // kWs = warps per column group: 1 (a warp owns the 8 channels of its 16-byte column) or 2 (a warp
 // owns 4 of them: half the per-thread state and tile registers, so more warps fit an SM).
 // kEma = false: TimestepNorm alone (y = the normalised activations; no pole matrices, no states).
@@ -587,6 +609,22 @@ __global__ void __launch_bounds__(kCg * kWs * kWp * 32, 1)
   // ---- running state of this thread: sequence b0 + g, channels 8*warp + e ----------------------
   const int bseq = b0 + g;
   const bool seq_ok = bseq < a.B;
+  // A sequence of which nothing has counted so far has no mean to take squares about, and about zero their tf32 roundings are larger than
+  // the variance of its first few values (40 x 94 x 1736, mean 3: outputs 0.22 off, so 2.8e-3): its first value stands in for one.
+  int t_first = -1;
+  if constexpr (kNorm) {
+    const bool none = seq_ok && (!kPs || seg == 0) && a.prev_count[bseq] == 0;
+    if constexpr (kMask) {
+      const int at = first_counted(a.mask + (size_t)(seq_ok ? bseq : 0) * L, L, none, q);
+      if (at < L) t_first = at;
+    } else if (none) {
+      t_first = 0;
+    }
+  }
+  auto start_mean = [&](int d) -> float {
+    const float* prev = a.prev_mean + (size_t)bseq * a.D + d;
+    return t_first < 0 ? *prev : first_value(reinterpret_cast<const __nv_bfloat16*>(a.x) + bseq * a.xsb + t_first * a.xsl + d, prev);
+  };
   // kWp == 1: the running quantities live in registers from step to step.  kWp > 1: they arrive
   // through the mailbox at every step; a warp only keeps its latest mean per channel (mu_run), the
   // centre of its next sums of squares.
@@ -600,7 +638,7 @@ __global__ void __launch_bounds__(kCg * kWs * kWp * 32, 1)
     const int d = d0 + cbase + e;
     const bool ok = seq_ok && d < a.D;
     if constexpr (kMail) {
-      mu_run[e] = (kNorm && ok) ? a.prev_mean[(size_t)bseq * a.D + d] : 0.f;
+      mu_run[e] = (kNorm && ok) ? start_mean(d) : 0.f;
       // The warps of the last group put the call's initial statistics and pole states into their
       // mailboxes, where step 0 (first group) looks for what "step -1" left (it does not wait: the
       // barrier before the loop orders these writes).
@@ -650,7 +688,7 @@ __global__ void __launch_bounds__(kCg * kWs * kWp * 32, 1)
           m2_run[e] = sm2.y;
         } else {
           const float c0 = (float)a.prev_count[bseq];
-          const float mu = a.prev_mean[(size_t)bseq * a.D + d], vv = a.prev_var[(size_t)bseq * a.D + d];
+          const float mu = start_mean(d), vv = a.prev_var[(size_t)bseq * a.D + d];
           mu_run[e] = mu;
           m2_run[e] = c0 * vv;
           s1_run[e] = c0 * mu;
@@ -1227,8 +1265,12 @@ __global__ void __launch_bounds__(kCg * kWs * kWp * 32, 1)
 template <bool kNorm, int kCg, bool kSilu, int kWs = 1, bool kXn = false, bool kEma = true, bool kCplx = false,
           int kWp = 1, bool kMask = false, bool kSm = false>
 static bool launch_variant(int dtype, const void* x, void* y, long long xsb, long long xsl, long long ysb,
-                           long long ysl, const StreamArgs& a, cudaStream_t s, void* xn = nullptr,
+                           long long ysl, const StreamArgs& a_in, cudaStream_t s, void* xn = nullptr,
                            long long nsb = 0, long long nsl = 0) {
+  StreamArgs a = a_in;
+  a.x = x;
+  a.xsb = xsb;
+  a.xsl = xsl;
   using C = Cfg<kCg, kXn, kCplx, kWs, kWp, kSm>;
   const CUtensorMapSwizzle sw = kCg == 8 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE;
   CUtensorMap tx, ty, tn;

@@ -72,6 +72,9 @@ static bool launch_segmented(int dtype, const void* x, void* y, long long xsb, l
   constexpr int kCg = 8;
   using C = Cfg<kCg, false, false, 1, 1, false>;
   StreamArgs a = a_in;
+  a.x = x;
+  a.xsb = xsb;
+  a.xsl = xsl;
   const int nsteps = (a.L + kStep - 1) / kStep;
   if ((n_seg != 2 && n_seg != 4 && n_seg != 8) || nsteps % n_seg != 0) return false;
   a.n_seg = n_seg;

@@ -20,6 +20,8 @@ struct StreamArgs {
   float *cummean, *cumrstd;  // training saves of the norm-only mode, (B, L, D) fp32 contiguous, or NULL
   int cplx;  // complex poles: q, g are interleaved (re, im) (K, N, 2); states (B, D, N, 2)
   // set by the tensor-core path itself (callers leave them alone)
+  const void* x;         // beside the tensor map
+  long long xsb, xsl;
   long long wait_limit;  // SM cycles after which a bounded wait gives up
   int withhold_step;     // test aid: step whose tile is never loaded, or -1
   long long count_offset;  // added to prev_count (a call that continues another call's positions)

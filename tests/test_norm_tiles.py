@@ -134,6 +134,58 @@ def test_norm_ema_forms_agree(bsz, length, dim, cplx, xn):
             assert rel_l2(r["xn"].float(), res[0]["xn"].float()) < 2.0 ** -7
 
 
+# Operands are bf16 (2^-9 each), squares about the first value tf32 (2^-10 of a variance): as with a prior.
+@pytest.mark.parametrize("tile,cplx,masked", [
+    (2, False, False), (4, False, False), (7, False, False), (8, False, False), (22, False, False), (71, False, False), (222, False, False),
+    (224, False, False), (422, False, False), (124, False, False), (84, False, False), (16, False, False), (14, False, False),
+    (7, False, True), (22, False, True), (16, False, True), (0, True, False)])
+@pytest.mark.parametrize("normed", [False, True])
+def test_first_values_without_a_prior(tile, cplx, masked, normed):
+    """bf16, no count to begin with (the module's default), values far from zero: variances of the first few values, whose squares are
+    large, and nothing counted ahead of them."""
+    from fairseq_apollo_b200 import _lib, ops
+    from oracle import mega_oracle as O
+    gen = torch.Generator().manual_seed(tile + 1)
+    bsz, length, dim = 9, 128 * 2 if tile == 84 else 96, 72
+    rnd = lambda *s: torch.rand(*s, generator=gen)   # noqa: E731
+    x = (torch.randn(bsz, length, dim, generator=gen) + 3.0).bfloat16()
+    count = torch.zeros(bsz, dtype=torch.int64)
+    count[4] = 2
+    mean, var, gamma, beta = 3.0 * (count > 0).float()[:, None].expand(bsz, dim).contiguous(), torch.ones(bsz, dim), rnd(dim) + 0.5, rnd(dim) - 0.5
+    mask = None
+    if masked:
+        mask = torch.zeros(bsz, length, dtype=torch.bool)
+        mask[0, :41] = True
+        mask[1, :5] = True
+        mask[2, 30:] = True
+        mask[3] = True
+    p, q, g, om = rnd(dim, 16) * 0.2, rnd(dim, 16) * 0.5 + 0.45, rnd(dim, 16) - 0.5, rnd(dim)
+    if cplx:
+        q, g = torch.polar(q, rnd(dim, 16) * 3.0), torch.complex(g, g.flip(1))
+    args = [t.cuda() for t in (x, count, mean, var, gamma, beta)] + [1e-5] + [t.cuda() for t in (p, q, g, om)]
+    _lib.set_option(2, tile)
+    _lib.set_option(5, 1)
+    try:
+        r = ops.tsn_ema_forward(*args, None if mask is None else mask.cuda(), want_normed=normed, **({"complex_poles": True} if cplx else {}))
+        assert "tsn_ema_mma" in _lib.last_kernel()
+        alone = ops.timestep_norm_fwd(*args[:6], None if mask is None else mask.cuda())
+    finally:
+        _lib.set_option(2, 0)
+        _lib.set_option(5, 0)
+    xn, cnt, mean, var = O.timestep_norm(x.double(), count, mean.double(), var.double(), gamma.double(), beta.double(), mask, acc_dtype=torch.float64)[:4]
+    h, ys = torch.zeros(bsz, dim, 16, dtype=torch.complex128), []
+    for t in range(length):
+        h = q.to(torch.complex128) * h + p.double() * xn[:, t, :, None]
+        ys.append((h * g.to(torch.complex128)).real.sum(-1) + om.double() * xn[:, t])
+    assert rel_l2(r["y"].float(), torch.stack(ys, 1)) < 1e-2
+    if normed:
+        assert rel_l2(r["xn"].float(), xn) < 6e-3
+    assert rel_l2(alone[0].float(), xn) < 6e-3
+    assert torch.equal(r["count"].cpu(), cnt) and torch.equal(alone[1].cpu(), cnt)
+    for m, v in ((r["mean"], r["var"]), alone[2:4]):
+        assert rel_l2(m, mean) < 1e-4 and rel_l2(v, var) < 2e-3
+
+
 def test_form_of_the_norm_alone_leaves_the_pair():
     """The form asked for of TimestepNorm by itself (4) is none of the pair, which runs as always."""
     from fairseq_apollo_b200 import _lib, ops
