@@ -583,12 +583,7 @@ static int tsn_fwd_common(const void* x, void* y, int dtype, int B, int L, int D
         na.prev_count = a.prev_count; na.prev_mean = prev_mean; na.prev_var = prev_var; na.gamma = gamma; na.beta = beta;
         na.mask = pad_mask; na.eps = (float)eps; na.count_out = a.count_out; na.mean_out = mean_out; na.var_out = var_out;
         const int form = g_options[OPT_SPLIT].load();
-        // (statistics updated in place the scan does not take: what is left is a chain, 13 x 53 x 32 7 us for 10, 20 x 234 x 472 13 for
-        // 14, 39 x 123 x 1912 29 for 41; without the pair's matrices a block has started at once)
-        StreamArgs start = sa;
-        start.L = 0;
-        const double other = !stats_in_place(na) ? scan_norm_us(na) : B < 4 ? 3. + 0.1 * L : 5. + mma_chain_us(sa, false) - mma_chain_us(start, false);
-        if (xsd == 1 && ysd == 1 && form != 3 && (form == 4 || tmem_norm_us(sa) < 0.9 * other) &&
+        if (xsd == 1 && ysd == 1 && form != 3 && (form == 4 || tmem_norm_us(sa) < 0.9 * scan_norm_us(na)) &&
             tmem_norm_try(dtype, x, y, xsb, xsl, ysb, ysl, sa, (cudaStream_t)stream))
           return check_launch("timestep_norm_fwd(tmem)");
         if (scan_norm_fwd_try(dtype, na, xsd, ysd, (cudaStream_t)stream)) return check_launch("timestep_norm_fwd(scan)");
