@@ -263,8 +263,7 @@ __device__ __forceinline__ uint32_t vec_off(int seq, int t, int cg) {
   return (uint32_t)(row * (kCg * 16) + (cg << 4));
 }
 
-// The first position of a sequence that counts, 32 at a time by the four lanes that share it (L: none; all lanes of a warp come).  Out of
-// line, like the value there (prev: instead of one that is not finite): nothing of them is held in registers beside the step loop.
+// The first position of a sequence that counts, 32 at a time by the four lanes that share it (L: none; all lanes of a warp come).
 __device__ __noinline__ int first_counted(const unsigned char* row, int L, bool wanted, int q) {
   int at = L;
   for (int t0 = 0; t0 < L && __any_sync(0xffffffffu, wanted && at == L); t0 += 32) {
@@ -279,10 +278,6 @@ __device__ __noinline__ int first_counted(const unsigned char* row, int L, bool 
     at = min(at, m);
   }
   return wanted ? at : L;
-}
-__device__ __noinline__ float first_value(const __nv_bfloat16* x, const float* prev) {
-  const float v = __bfloat162float(*x);
-  return fabsf(v) <= 3.4e38f ? v : *prev;
 }
 
 // kWs = warps per column group: 1 (a warp owns the 8 channels of its 16-byte column) or 2 (a warp
@@ -621,9 +616,10 @@ __global__ void __launch_bounds__(kCg * kWs * kWp * 32, 1)
       t_first = 0;
     }
   }
-  auto start_mean = [&](int d) -> float {
-    const float* prev = a.prev_mean + (size_t)bseq * a.D + d;
-    return t_first < 0 ? *prev : first_value(reinterpret_cast<const __nv_bfloat16*>(a.x) + bseq * a.xsb + t_first * a.xsl + d, prev);
+  auto start_mean = [&](int d) -> float {   // (both are loaded, so that neither waits for the count)
+    const float prev = a.prev_mean[(size_t)bseq * a.D + d];
+    const float v = __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(a.x)[bseq * a.xsb + max(t_first, 0) * a.xsl + d]);
+    return t_first >= 0 && fabsf(v) <= 3.4e38f ? v : prev;
   };
   // kWp == 1: the running quantities live in registers from step to step.  kWp > 1: they arrive
   // through the mailbox at every step; a warp only keeps its latest mean per channel (mu_run), the
