@@ -80,9 +80,8 @@ bool mma_cl_try(int dtype, const void* x, void* y, void* xn, long long xsb, long
   // The EMA by itself: 16 x 4096 x 1024 74 us (98 here), 8 x 2000 x 1024 28 (52), 64 x 4096 x 2048 540 (471).
   if (ema && !a_in.cplx && (norm || !masked)) {
     const int asked = forced == 14 ? 4 : forced == 16 ? 9 : forced == 162 ? 10 : forced == 164 ? 12 : forced == 168 ? 16 : 0;
-    // (a state that leaves takes its statistics along, whose variance is 2e-7 off there and 3e-4 here)
-    const double chain = forced != 0 ? 0. : norm ? (a_in.h_out ? 1.25 : 0.95) * mma_chain_us(a_in, want_xn) : 0.97 * mma_ema_chain_us(a_in);
-    const bool better = forced == 0 && tmem_ema_us(a_in, norm, want_xn) < chain;
+    // (of two that take about as long the one whose variance is 2e-7 off, here 3e-4)
+    const bool better = forced == 0 && tmem_ema_us(a_in, norm, want_xn) < (norm ? mma_chain_us(a_in, want_xn) : 0.97 * mma_ema_chain_us(a_in));
     if ((asked > 0 || better) && tmem_ema_try(dtype, x, y, xn, xsb, xsl, ysb, ysl, norm, a_in, s, asked))
       return true;
   }

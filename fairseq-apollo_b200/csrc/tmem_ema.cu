@@ -910,7 +910,7 @@ double runs_us(const StreamArgs& a, bool norm, bool xn, int runs, int q) {
   const bool pieces = a.D % kCh != 0;
   const double ns = kNs[q == 8][pieces][(a.silu ? 1 : 0) + (xn ? 2 : 0)] + (!a.mask ? 0. : q == 4 ? 3. : pieces ? 6.5 : 5.);
   const double steps = runs > 1 ? len : 0.5 * (a.L + len);
-  return 3.5 + rounds * (7.5 + (a.silu ? 1. : 0.) + (xn ? 2. : 0.) - (a.mask ? 1. : 0.) + steps * ns * 1e-3);
+  return (runs > 1 ? 6. : 3.5) + rounds * (7.5 + (a.silu ? 1. : 0.) + (xn ? 2. : 0.) - (a.mask ? 1. : 0.) + steps * ns * 1e-3);
 }
 // with the limit of its waits, and the load that a test withholds
 StreamArgs bounded(StreamArgs a) {
@@ -922,11 +922,11 @@ StreamArgs bounded(StreamArgs a) {
 // sequences of a block: four where that gives all blocks an SM at once (a position takes 12 - 23 ns for 20 - 32: 8 x 8192 x 1024 112 us
 // against 176, 4 x 4096 x 1024 60 against 88; in two rounds 16 x 4096 x 1024 118 against 91)
 int sequences_of(const StreamArgs& a) { return (long long)((a.D + kCh - 1) / kCh) * ((a.B + 3) / 4) <= 148 ? 4 : 8; }
-// runs: what balances the blocks' rounds (16 x 8192 x 5120 in two: 4.5 rounds of the sequence for 5)
+// runs: what balances the blocks' rounds (16 x 8192 x 5120 in two: 4.5 rounds of the sequence for 5; 26 x 2208 x 640 97 us, in one 106)
 int runs_of(const StreamArgs& a, bool norm, bool xn) {
   int best = 1;
   if (a.mask) return best;   // (the positions that count are known to the run before alone)
-  double least = 0.95 * runs_us(a, norm, xn, 1, 8);
+  double least = (norm ? 0.98 : 0.95) * runs_us(a, norm, xn, 1, 8);
   for (int n = 2; n <= 8; n *= 2)
     if (const double us = runs_us(a, norm, xn, n, 8); a.L >= 1024 * n && us < least) {
       least = us;

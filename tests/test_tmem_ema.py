@@ -304,7 +304,7 @@ def test_ema_over_its_inputs(option, value):
     (8, 1024, 2048, False, True, "tsn_ema_mma tmem"),
     (8, 1024, 2048, True, True, "tsn_ema_mma tmem mask"),
     (3, 4096, 2048, False, False, "tsn_ema_mma tmem"),      # fewer than four sequences
-    (16, 100, 1024, False, False, "tsn_ema_mma tile=2 warps_per_column=2 pipe=4 norm ema"),      # the chain of mma.sync
+    (16, 60, 1024, False, False, "tsn_ema_mma tile=2 warps_per_column=2 pipe=4 norm ema"),      # the chain of mma.sync
     (24, 1500, 1000, False, False, "tsn_ema_mma tile=2 warps_per_column=2 pipe=1 norm ema"),
     (58, 96, 1096, False, False, "tsn_ema_mma tile=8 warps_per_column=1 pipe=1 norm ema"),      # (37 us, in tensor memory 49)
     (37, 154, 1120, False, True, "tsn_ema_mma tile=2 warps_per_column=2 pipe=1 norm ema xn"),   # (43, 54)
@@ -321,20 +321,6 @@ def test_pair_is_chosen(option, bsz, length, dim, masked, normed, name):
     assert rel_l2(r["mean"], other["mean"]) < 1e-4 and rel_l2(r["var"], other["var"]) < 2e-3
     if normed:
         assert rel_l2(r["xn"].float(), other["xn"].float()) < 1.4e-2   # (4e-3 and 1e-2)
-
-
-def test_statistics_that_leave_with_a_state(option):
-    """Of two forms that take about as long the one with fp32 statistics."""
-    from fairseq_apollo_b200 import _lib
-    from oracle import mega_oracle as O
-    x, stats, prm, h0, _ = _case(37, 160, 1120, 16, True, False)
-    _run(x, stats, prm, None, None, want_normed=True)
-    assert "tile=" in _lib.last_kernel()
-    r = _run(x, stats, prm, h0, None, want_state=True, want_normed=True)
-    assert _lib.last_kernel() == "tsn_ema_mma tmem"
-    ds = slice(None, None, 32)
-    var = O.timestep_norm(x[..., ds].float(), stats[0], *(t[..., ds] for t in stats[1:]), None, acc_dtype=torch.float64)[3]
-    assert rel_l2(r["var"][:, ds], var) < 2e-6
 
 
 @pytest.mark.parametrize("bsz,length,dim,masked", [(8, 256, 16, False), (5, 290, 72, False), (4, 33, 8, True), (16, 1000, 40, True),
