@@ -73,11 +73,11 @@ bool mma_cl_try(int dtype, const void* x, void* y, void* xn, long long xsb, long
     return false;
   if (a_in.h_out && (a_in.L % kStep) != 0) return false;
   if ((a_in.B + kSeq - 1) / kSeq > 65535) return false;
-  // TimestepNorm -> EMA with real poles: statistics by scalar arithmetic and accumulators in tensor memory (16 x 4096 x 1024 90 us
-  // against 140, with the second output 110 against 208, masked 110 against 195; 64 x 8192 x 2048 1.17 ms against 1.48, with SiLU 1.41
-  // against 1.82), or this kernel's chain (some ragged or short shapes; 64 x 32768 x 2048, where the power cap slows the other,
-  // 4.5 ms in a burst and 5.1 for long against 5.1 and 5.2).
-  // The EMA by itself: 16 x 4096 x 1024 74 us (98 here), 8 x 2000 x 1024 28 (52), 64 x 4096 x 2048 540 (471).
+  // TimestepNorm -> EMA with real poles: statistics by scalar arithmetic and accumulators in tensor memory (16 x 4096 x 1024 88 us
+  // against 142, with the second output 107 against 208, masked 106 against 195; 64 x 8192 x 2048 in a row 1.25 ms against 1.41, with
+  // SiLU 1.47 against 1.52), or this kernel's chain (some ragged or short shapes).  The power cap takes most of the gain back where
+  // all SMs are busy for long: 64 x 32768 x 2048 4.7 ms in a run of 20 launches, 5.1 to 5.2 in a long loop, the chain 5.15 and 5.2.
+  // The EMA by itself: 16 x 4096 x 1024 74 us (98 here), 8 x 2000 x 1024 27 (51), 64 x 4096 x 2048 531 (468).
   if (ema && !a_in.cplx && (norm || !masked)) {
     const int asked = forced == 14 ? 4 : forced == 16 ? 9 : forced == 162 ? 10 : forced == 164 ? 12 : forced == 168 ? 16 : 0;
     // (of two that take about as long the one whose variance is 2e-7 off, here 3e-4)

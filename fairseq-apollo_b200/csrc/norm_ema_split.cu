@@ -37,8 +37,8 @@ bool mma_takes(int dtype, const StreamArgs& a, bool want_xn) {
 
 // (a part for the launch and, on the tensor-core kernel with complex poles, for its coefficients; long chains of the forms with
 // a second output or a mask fall behind the short ones' rate.  With real poles mma_cl_try has a faster form since (tmem_ema.cu), whose
-// roundings are the same: these times are left to say which calls round their operands to bf16, the others' results stay)
-double fused_us(int dtype, const StreamArgs& a, bool want_xn) {
+// roundings are the same: these times of the chain are left to say which calls round their operands to bf16, the others' results stay)
+double fused_chain_us(int dtype, const StreamArgs& a, bool want_xn) {
   const double L = a.L, n = (double)a.B * a.D * a.L;
   if (mma_takes(dtype, a, want_xn)) {
     // (both a mask and the second output: 11 x 1894 x 464 153 us, 6 x 4999 x 2048 387, 16 x 4096 x 1024 257)
@@ -156,7 +156,7 @@ bool norm_ema_split_try(int dtype, const void* x, void* y, void* xn, long long x
   // the one they took before there were products of chunks)
   // (a prompt that comes in chunks keeps to the tensor-core kernel, and its rounding, unless much is gained)
   const bool prompt = dtype == MEGA_BF16 && a.h_out && !a.mask && !a.cplx && mma_takes(dtype, a, xn != nullptr);
-  const double fused = fused_us(dtype, a, xn != nullptr), scan = scan_us(dtype, ea, xn != nullptr) + (prompt ? 25.0 : 0.0),
+  const double fused = fused_chain_us(dtype, a, xn != nullptr), scan = scan_us(dtype, ea, xn != nullptr) + (prompt ? 25.0 : 0.0),
                chain = mma_us(dtype, a, xn != nullptr) + 25.0;
   // The products of chunks behind TimestepNorm in bf16: for calls that would run on the tensor-core kernel in one of its two ways,
   // whose roundings these are too (complex 4 x 4096 x 1024 263 us fused, 103 so; real 142 and 94).

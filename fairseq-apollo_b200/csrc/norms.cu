@@ -573,8 +573,8 @@ static int tsn_fwd_common(const void* x, void* y, int dtype, int B, int L, int D
       sa.beta = beta; sa.eps = (float)eps; sa.count_out = a.count_out; sa.mean_out = mean_out; sa.var_out = var_out;
       sa.mask = pad_mask;
       sa.cummean = cummean; sa.cumrstd = cumrstd;
-      // The walk of tmem_ema.cu (bf16, where there are enough sequences and channels: 16 x 4096 x 1024 68 us, 64 x 4096 x 2048 469) and
-      // the scan (105, 614) take their statistics in fp32 (variances 1e-6 off), the tensor-core form from bf16 and tf32 operands
+      // The walk of tmem_ema.cu (bf16, where there are enough sequences and channels: 16 x 4096 x 1024 67 us, 64 x 4096 x 2048 518) and
+      // the scan (97, 641) take their statistics in fp32 (variances 1e-6 off), the tensor-core form from bf16 and tf32 operands
       // (3e-4; 142, and 4305 us at 64 x 32768 x 2048 where the scan takes 4969).
       if (!cummean && g_options[OPT_MMA_TILE].load() == 0 && g_options[OPT_DISABLE_MMA].load() == 0) {
         ScanNormArgs na{};
@@ -590,7 +590,8 @@ static int tsn_fwd_common(const void* x, void* y, int dtype, int B, int L, int D
           return check_launch("timestep_norm_fwd(tmem)");
         if (scan_norm_fwd_try(dtype, na, xsd, ysd, (cudaStream_t)stream)) return check_launch("timestep_norm_fwd(scan)");
       }
-      // (statistics updated in place, a form of the tensor-core kernel asked for by name, or the streamed kernel)
+      // (statistics updated in place where the walk of tmem_ema.cu, which may do so, is not the faster one; a form of the tensor-core
+      // kernel asked for by name; or the streamed kernel)
       if (!cummean && mma_cl_try(dtype, x, y, nullptr, xsb, xsl, xsd, ysb, ysl, ysd, true, sa, (cudaStream_t)stream))
         return check_launch("timestep_norm_fwd(mma)");
       if (stream_cl_try(dtype, x, y, nullptr, xsb, xsl, xsd, ysb, ysl, ysd, false, sa, (cudaStream_t)stream))

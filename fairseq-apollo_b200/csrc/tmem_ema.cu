@@ -23,7 +23,7 @@
 // two tiles), 4 of states, 4 of outputs (8 with SiLU), one that fetches x (TMA), one that issues products, 2 for the normalised
 // activations as an output.  Everything is exchanged over mbarriers, the statistics over named barriers of two warps.
 //
-// What bounds it (16 x 4096 x 1024, 90 us against 140 in the forms of mma_cl_kernel.cuh; 67 without anything but the statistics): issue
+// What bounds it (16 x 4096 x 1024, 88 us against 142 in the forms of mma_cl_kernel.cuh; 67 for the statistics by themselves): issue
 // slots and latency at 22 warps, 0.65 instructions per scheduler and cycle; the products' reads of shared memory 12 us, the outputs 4.
 // Two things that cost much: outputs that may stay in L1 (103 us; no_allocate), and code that does not fit the instruction cache (the
 // same walk in 250 KB of code 512 us; what is rare is out of line).  Over all SMs for long the power cap takes 12 % of the clock.
@@ -403,7 +403,7 @@ __global__ void __launch_bounds__(Roles<kQ, kSilu, kXn, kForm>::kThreads, 1) tsn
       if (lane == 0) arrive(bar(kOpFull + (tile & 1)));
     }
   } else if (kForm != kEmaOnly && warp >= R::kStats && warp < R::kLoad) {
-    // ---- statistics: four threads per channel of a sequence, which take every fourth part ---------------------------
+    // ---- statistics: three (four sequences to a block: six) threads per channel of a sequence, which take the parts in turn ---------
     const int nw = (warp - R::kStats) % kPer, own = (warp - R::kStats) / kPer, ch = lane & 15, s = 2 * nw + (lane >> 4), d = d0 + ch, b = b0 + s;
     const bool live = d < a.D && b < a.B;
     const float eps = a.eps, w = live ? __ldg(a.gamma + d) : 0.f, bb = live ? __ldg(a.beta + d) : 0.f;
@@ -1004,7 +1004,8 @@ bool tmem_ema_try(int dtype, const void* x, void* y, void* xn, long long xsb, lo
   return true;
 }
 
-// (16 x 4096 x 1024 68 us, masked 95; 8 x 8192 x 1024 82 and 116; 64 x 4096 x 2048 469 and 626; 24 x 1500 x 1000 77 and 93)
+// (16 x 4096 x 1024 67 us, masked 93; 8 x 8192 x 1024 82 and 115; 64 x 4096 x 2048 469 and 626, in a row 518 and 632; 24 x 1500 x 1000
+// 76 and 92)
 double tmem_norm_us(const StreamArgs& a) {
   const int q = sequences_of(a);
   const double tiles = (double)((a.D + kCh - 1) / kCh) * ((a.B + q - 1) / q), rounds = std::ceil(tiles / 148.);
