@@ -76,7 +76,7 @@ bool mma_cl_try(int dtype, const void* x, void* y, void* xn, long long xsb, long
   // TimestepNorm -> EMA with real poles: statistics by scalar arithmetic and accumulators in tensor memory (16 x 4096 x 1024 88 us
   // against 142, with the second output 107 against 208, masked 106 against 195; 64 x 8192 x 2048 in a row 1.25 ms against 1.41, with
   // SiLU 1.47 against 1.52), or this kernel's chain (some ragged or short shapes).  The power cap takes most of the gain back where
-  // all SMs are busy for long: 64 x 32768 x 2048 4.7 ms in a run of 20 launches, 5.1 to 5.2 in a long loop, the chain 5.15 and 5.2.
+  // all SMs are busy for long: 64 x 32768 x 2048 4.6 to 4.7 ms in a run of 20 launches, 5.1 to 5.2 in a long loop, the chain 5.15 and 5.2.
   // The EMA by itself: 16 x 4096 x 1024 74 us (98 here), 8 x 2000 x 1024 27 (51), 64 x 4096 x 2048 531 (468).
   if (ema && !a_in.cplx && (norm || !masked)) {
     const int asked = forced == 14 ? 4 : forced == 16 ? 9 : forced == 162 ? 10 : forced == 164 ? 12 : forced == 168 ? 16 : 0;
